@@ -18,6 +18,8 @@ using torch::Tensor;
 inline cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 inline void check(cudaError_t e, const char* what) { TORCH_CHECK(e == cudaSuccess, what, ": ", cudaGetErrorString(e)); }
 
+inline int num_sms() { return at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
+
 inline const float* f32(const Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kFloat32, name, " must be a CUDA float tensor");
   TORCH_CHECK(t.dim() == 0 || t.stride(-1) == 1, name, " must have unit inner stride");
@@ -236,6 +238,28 @@ void window_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
     TORCH_CHECK(!kv_shared, "window_attention: a float result over bf16 pages is not available with shared key / value rows");
     md.out_float = out.data_ptr<float>();
     md.out_float_stride = out.stride(0);
+  }
+  // Prompt portions over bf16 pages at head size 128: the tcgen05 kernel (impl 4) in every step that is not all single tokens.  It was the
+  // faster one at each size measured, 16 heads over 4: 8192 tokens in portions of 4 behind 1000 keys 1147 us against 1374 (mma.sync),
+  // portions of 32 190 against 493, 16 x 2048 tokens with window 1024 344 against 1460, one portion of 77 tokens 15 against 19, and steps
+  // that mix 64 single tokens with a 4096-token portion 1344 against 1663.
+  const int64_t rows_k = k_cache.size(0) * Hkv * 16, rows_v = v_cache.size(0) * v_cache.size(1) * 16;
+  const bool tc_fits = k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.is_contiguous() &&
+                       v_cache.is_contiguous() && window >= 1 && rows_k < (int64_t{1} << 31) - 16 && rows_v < (int64_t{1} << 31) - 16 &&
+                       (float_out || out.scalar_type() == at::kBFloat16) && q.scalar_type() == at::kFloat && !head_major &&
+                       q.stride(1) == 1 && out.stride(1) == 1 &&
+                       nrl_window_attention_tc_fits(q.data_ptr<float>(), q.stride(0), out.data_ptr(), out.stride(0), T, Hq, Hkv, D, Dv, page,
+                                                    static_cast<float>(scale), &md) != 0;
+  TORCH_CHECK(impl != 4 || tc_fits, "window_attention: the tcgen05 kernel does not take this call");
+  if (tc_fits && (impl == 4 || (impl == 0 && !single_token))) {
+    const CUtensorMap tmk = nrl::make_tma_2d(k_cache.data_ptr(), rows_k, 128, 256, 16, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
+    const CUtensorMap tmv = nrl::make_tma_2d(v_cache.data_ptr(), rows_v, 128, 256, 16, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
+    check(nrl_window_attention_tc(&tmk, &tmv, static_cast<int>(rows_k), static_cast<int>(rows_v), f32(q, "q"), q.stride(0),
+                                  i32(block_table, "block_table"), static_cast<int>(block_table.size(1)), i32(tok_entry, "tok_entry"),
+                                  i32(pos, "pos"), static_cast<int>(window), static_cast<float>(scale), static_cast<float>(out_scale),
+                                  out.data_ptr(), out.stride(0), T, Hq, Hkv, &md, num_sms(), cur_stream()),
+          "window_attention");
+    return;
   }
   // steps of single tokens on bf16 pages: cut the key walk into parts so that few sequences still fill the GPU
   int nsplit = 0;

@@ -8,6 +8,7 @@
 // Storage types: `f32` flags select float (1) or bf16 (0) for a typed operand; everything that is accumulated,
 // normalised, exponentiated or carried from token to token is float.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -198,7 +199,7 @@ cudaError_t nrl_window_attention(const float* q, long sq, const void* k_cache, c
 // `nsplit` >= 1 with `part` float [T, Hq, 4 nsplit, Dv + 2] (steps of single tokens over bf16 pages): every warp of nsplit
 // blocks per (token, key/value head) walks its own pages and a second launch merges the parts; nrl_window_attention_splits
 // proposes the count (0: the shape does not fit).
-// `impl`: 0 picks by shape and step kind, 1 the scalar tile kernel, 2 one block per (token, head), 3 the tensor-core kernel.
+// `impl`: 0 picks by shape and step kind, 1 the scalar tile kernel, 2 one block per (token, head), 3 the mma.sync kernels.
 
 // Latent attention on the tensor cores (attention_latent_mma.cu): causal attention of H absorbed queries per token (q float
 // [T, H * D]) over bf16 pages [pages, 1, 16, D] whose rows are key and, in their first Dv columns, value of every head; sink
@@ -210,6 +211,15 @@ cudaError_t nrl_latent_attention_mma(const float* q, long sq, const void* cache,
                                      const int* tok_entry, const int* pos, float scale, float out_scale, void* out, long so, int T, int H,
                                      int D, int Dv, int page, int single_token, int nsplit, float* part, const NrlAttnMods* mods,
                                      cudaStream_t s);
+
+// tcgen05 kernel for prompt portions over bf16 pages (attention_window_tc.cu): head size 128; tmK / tmV are TMA maps of the page pools as
+// [pages * heads * 16][128] rows with boxes of 16 rows x 64 columns, oob_k / oob_v row coordinates behind them (read as zeros).
+int nrl_window_attention_tc_fits(const float* q, long sq, const void* out, long so, long T, int Hq, int Hkv, int D, int Dv, int page, float scale,
+                                 const NrlAttnMods* md);
+cudaError_t nrl_window_attention_tc(const CUtensorMap* tmK, const CUtensorMap* tmV, int oob_k, int oob_v, const float* q, long sq,
+                                    const int* block_table, int max_blocks, const int* tok_entry, const int* pos, int window, float scale,
+                                    float out_scale, void* out, long so, int T, int Hq, int Hkv, const NrlAttnMods* md, int num_sms,
+                                    cudaStream_t s);
 
 // Tensor-core kernel for prompt portions over bf16 pages of 16 tokens (attention_window_mma.cu); `_fits` says whether the
 // shapes and the output's alignment allow it.

@@ -1,5 +1,5 @@
 """Op layer of hybrid (attention + recurrent-state) decoders: thin, launch-counting wrappers over the sm_100a kernels of
-``csrc/stream_ops.cu``, ``csrc/recurrent.cu``, ``csrc/lightning.cu``, ``csrc/attention_window.cu`` / ``attention_window_mma.cu`` /
+``csrc/stream_ops.cu``, ``csrc/recurrent.cu``, ``csrc/lightning.cu``, ``csrc/attention_window.cu`` / ``attention_window_mma.cu`` / ``attention_window_tc.cu`` /
 ``attention_latent_mma.cu`` and ``csrc/moe.cu``
 (with the grouped form of ``csrc/gemm_tc.cu``).
 
@@ -72,14 +72,14 @@ def qknorm_kv_write(q, k, v, qw, kw, eps, k_cache, v_cache, plan):
     _ext().qknorm_kv_write(q, k, v, qw, kw, eps, k_cache, v_cache, plan.kv_slot)
 
 
-WINDOW_IMPLS = {"auto": 0, "tile": 1, "simple": 2, "mma": 3}
+WINDOW_IMPLS = {"auto": 0, "tile": 1, "simple": 2, "mma": 3, "tc": 4}
 
 
 def window_attention(q, k_cache, v_cache, plan, window, scale, out_scale, out, impl: str = "auto", chunked: bool = False,
                      head_scale=None, head_slope=None, gate=None, head_sink=None, value_size: int = 0, softcap: float = 0.0,
                      keep_first: int = 0, dist_bias=None, v_div: int = 1):
-    """``impl``: "auto" (tensor cores for prompt portions over bf16 pages, the scalar tile kernel otherwise) or one kernel by
-    name; a kernel that does not fit the shapes raises.  ``chunked``: keys of the query's own chunk of ``window`` positions
+    """``impl``: "auto" (tensor cores for prompt portions over bf16 pages: tcgen05 ("tc") at head size 128, else mma.sync; the scalar tile
+    kernel otherwise) or one kernel by name; a kernel that does not fit the shapes raises.  ``chunked``: keys of the query's own chunk of ``window`` positions
     instead of the last ``window`` keys.  ``head_scale`` / ``head_slope`` [heads]: per-head score multiplier and linear distance
     penalty; ``gate`` [T, heads] or [T, heads * value size]: the head's output (or every column) is multiplied by sigmoid(gate); ``head_sink`` [heads]: the softmax denominator
     also holds exp(sink).  ``value_size`` > 0 (with ``v_cache is k_cache``): the values are the first ``value_size`` columns of the
