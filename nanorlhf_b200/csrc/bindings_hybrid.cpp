@@ -152,7 +152,7 @@ void delta_scan(const Tensor& qkv, int64_t col_k, int64_t col_v, const c10::opti
   TORCH_CHECK(qkv.dim() == 2 && col_v + heads * Dv <= qkv.size(1) && o.is_contiguous() && o.size(-1) == heads * Dv, "delta_scan: shapes");
   check(nrl_delta_scan(f32(qkv, "qkv"), qkv.stride(0), static_cast<int>(col_k), static_cast<int>(col_v), beta.has_value() ? f32(*beta, "beta") : nullptr,
                        f32(decay, "decay"), f32w(state, "state"), f32w(o, "o"), i32(cu, "cu"), i32(start, "start"),
-                       i32(state_slot, "state_slot"), E, heads, static_cast<int>(kv_heads), D, Dv, per_channel ? 1 : 0,
+                       i32(state_slot, "state_slot"), E, static_cast<int>(qkv.size(0)), heads, static_cast<int>(kv_heads), D, Dv, per_channel ? 1 : 0,
                        static_cast<int>(impl), cur_stream()),
         "delta_scan");
 }

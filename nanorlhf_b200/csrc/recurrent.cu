@@ -676,6 +676,305 @@ delta_scan_col_kernel(const float* __restrict__ qkv, long sq, int col_k, int col
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// Delta rule (or plain accumulation) of prompt portions, four tokens at a time, all arithmetic float.  With g_i the decays, c_i = g_1 .. g_i
+// and G(i, j) = g_{j+1} .. g_i (products, nothing is divided), tokens 1..4 of a chunk over the state S before it give
+//   u_i = beta_i (v_i - S^T (c_i k_i) - sum_{j<i} (k_i . G(i,j) k_j) u_j)          (no delta: u_i = v_i)
+//   o_i = S^T (c_i q_i) + sum_{j<=i} (q_i . G(i,j) k_j) u_j
+//   S  <- c_4 S + sum_j (G(4,j) k_j) u_j^T
+// so an element of the state costs three multiply-adds per token (and one product per chunk) and every vector value that is read from
+// shared memory serves four or eight columns.  The column-resident kernels wait for their vectors and two sums once per token: 16 x 2048
+// tokens, 16 heads of 128 x 128: 4350 us there, 2310 us here (950 us at the float32 multiply-add rate).  What bounds it now is latency: 128 rows
+// x 8 columns take 254 registers, so eight warps per SM issue 0.38 instructions per clock and scheduler, stalled on shared-memory reads,
+// shuffles and fixed latencies.  Inputs come by cp.async three chunks ahead and a chunk's vectors are prepared while the one before is
+// computed (2520 us with loads one chunk ahead); 64 registers of state per thread over twice the warps took 2730 us.
+//
+// Lane = (one of four column groups, one of eight row groups): a thread keeps 2 PIECES rows x CT columns of the state in registers, rows
+// 16 p + 2 rg + {0, 1}, columns in pairs for the packed multiply-add; the shared vectors are stored with every value twice, so that
+// a 16-byte read is two ready operands and serves 2 x CT columns.  Sums over the row groups go by reduce-scatter shuffles: register a of a
+// thread is column a ^ x of its group (x: the column the lane will own), which makes "the half to send" the same registers in every lane.
+// Columns are independent: a state's columns are cut over blocks of two warps, 8 CT columns each.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int kBlkTok = 4;
+constexpr int kBlkWarps = 2;
+
+__device__ __forceinline__ void cp_async_f32(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_f32x4(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// r[i] = sum over all rows of S[., column x] * v_i: `vec` holds four padded vectors with every value twice
+template <int PIECES, int CT>
+__device__ __forceinline__ void blk_product(const f32x2 (&S)[2 * PIECES][CT / 2], const float2* vec, int rg, float (&r)[kBlkTok]) {
+  constexpr int DP = 16 * PIECES;
+  f32x2 acc[CT / 2][kBlkTok];
+#pragma unroll
+  for (int a = 0; a < CT / 2; ++a)
+#pragma unroll
+    for (int i = 0; i < kBlkTok; ++i) acc[a][i] = 0;
+#pragma unroll
+  for (int pc = 0; pc < PIECES; ++pc)
+#pragma unroll
+    for (int i = 0; i < kBlkTok; ++i) {
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(vec + i * DP + pc * 16 + rg * 2);
+#pragma unroll
+      for (int a = 0; a < CT / 2; ++a) acc[a][i] = fma2(S[2 * pc][a], w.x, acc[a][i]);
+#pragma unroll
+      for (int a = 0; a < CT / 2; ++a) acc[a][i] = fma2(S[2 * pc + 1][a], w.y, acc[a][i]);
+    }
+#pragma unroll
+  for (int i = 0; i < kBlkTok; ++i) {
+    float f[CT];
+#pragma unroll
+    for (int a = 0; a < CT / 2; ++a) unpack2(acc[a][i], f[2 * a], f[2 * a + 1]);
+    if (CT == 8) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) f[a] += __shfl_xor_sync(0xffffffffu, f[(a + 4) % CT], 4);
+#pragma unroll
+      for (int a = 0; a < 2; ++a) f[a] += __shfl_xor_sync(0xffffffffu, f[a + 2], 2);
+      r[i] = f[0] + __shfl_xor_sync(0xffffffffu, f[1], 1);
+    } else {
+#pragma unroll
+      for (int a = 0; a < 2; ++a) f[a] += __shfl_xor_sync(0xffffffffu, f[a + 2], 4);
+      f[0] += __shfl_xor_sync(0xffffffffu, f[1], 2);
+      r[i] = f[0] + __shfl_xor_sync(0xffffffffu, f[0], 1);
+    }
+  }
+}
+
+// shared memory of a block: the inputs of four chunks (three on their way) and the prepared vectors of two
+template <int DP, int COLS>
+struct BlkSmem {
+  struct In {
+    float raw[kBlkTok][3][DP];                 // k, q, decay (when per channel)
+    float v[kBlkTok][COLS];
+    float beta[kBlkTok], g[kBlkTok];
+  } in[4];
+  struct Vec {
+    float2 k[kBlkTok][DP], q[kBlkTok][DP], h[kBlkTok][DP], c[DP];      // c_i k_i, c_i q_i, G(4,i) k_i, c_4, every value twice
+    float gram[kBlkWarps][16];                 // k_i . G k_j for j < i: index i (i - 1) / 2 + j; q_i . G k_j for j <= i: 6 + i (i + 1) / 2 + j
+  } vec[2];
+};
+
+template <int PIECES, int CT, bool DELTA, bool WIDE>      // 16 PIECES padded rows (64 or 128); WIDE: 16-byte loads of q, k, decay
+__global__ void __launch_bounds__(32 * kBlkWarps, PIECES * CT == 64 ? 4 : 6)
+delta_scan_blk_kernel(const float* __restrict__ qkv, long sq, int col_k, int col_v, const float* __restrict__ beta,
+                      const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ o, const int* __restrict__ cu,
+                      const int* __restrict__ start, const int* __restrict__ state_slot, int heads, int kv_heads, int D, int Dv,
+                      int per_channel) {
+  constexpr int DP = 16 * PIECES, COLS = 4 * CT * kBlkWarps, NT = 32 * kBlkWarps, PER = DP / NT;      // PER: vector entries a thread prepares
+  using Sm = BlkSmem<DP, COLS>;
+  extern __shared__ __align__(16) unsigned char blk_smem[];
+  Sm& sm = *reinterpret_cast<Sm*>(blk_smem);
+  const int e = blockIdx.x, h = blockIdx.y, g = h / (heads / kv_heads);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rg = lane & 7, x = CT == 8 ? rg : rg >> 1;
+  const int cb0 = blockIdx.z * COLS, cw = warp * 4 * CT + (lane >> 3) * CT, c0 = cb0 + cw;      // first column: block, group in it, group
+  float* gS = state + (static_cast<long>(state_slot[e]) * heads + h) * D * Dv;
+  const bool carried = start[e] > 0;
+  const int t0 = cu[e], t1 = cu[e + 1];
+  const int nd = per_channel ? heads * D : heads;
+
+  // inputs of the chunk that begins at token t; behind the last token: k = q = v = beta = 0, decay 1
+  auto fetch = [&](int t, typename Sm::In& in) {
+    constexpr int kLanes = DP / 4, kRows = NT / kLanes;          // a warp (128 rows) or half a warp (64) per (token, vector)
+    const int d = (tid % kLanes) * 4;
+#pragma unroll
+    for (int s = 0; s < 3 * kBlkTok / kRows; ++s) {
+      const int row = s * kRows + tid / kLanes, i = (row * 11) >> 5, part = row - 3 * i;       // row / 3 for rows below 12
+      if (part == 2 && !per_channel) continue;
+      float* dst = &in.raw[i][part][d];
+      const float* src = part < 2 ? qkv + static_cast<long>(t + i) * sq + (part == 0 ? col_k : 0) + g * D + d
+                                  : decay + static_cast<long>(t + i) * nd + h * D + d;
+      const float fill = part < 2 ? 0.f : 1.f;
+      if (WIDE) {
+        if (t + i < t1 && d < D) cp_async_f32x4(dst, src);
+        else *reinterpret_cast<float4*>(dst) = make_float4(fill, fill, fill, fill);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (t + i < t1 && d + j < D) cp_async_f32(dst + j, src + j);
+          else dst[j] = fill;
+        }
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < kBlkTok * COLS / NT; ++s) {
+      const int i = (s * NT + tid) / COLS, c = (s * NT + tid) % COLS;
+      if (t + i < t1 && cb0 + c < Dv) cp_async_f32(&in.v[i][c], qkv + static_cast<long>(t + i) * sq + col_v + h * Dv + cb0 + c);
+      else in.v[i][c] = 0.f;
+    }
+    if (tid < kBlkTok) {
+      if (DELTA && t + tid < t1) cp_async_f32(&in.beta[tid], beta + static_cast<long>(t + tid) * heads + h);
+      else in.beta[tid] = 0.f;
+    } else if (tid < 2 * kBlkTok && !per_channel) {
+      const int i = tid - kBlkTok;
+      if (t + i < t1) cp_async_f32(&in.g[i], decay + static_cast<long>(t + i) * nd + h);
+      else in.g[i] = 1.f;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto prepare = [&](const typename Sm::In& in, typename Sm::Vec& vec) {
+    float dots[16] = {};
+#pragma unroll
+    for (int s = 0; s < PER; ++s) {
+      const int d = tid + s * NT;
+      float w[kBlkTok], c = 1.f;
+#pragma unroll
+      for (int i = 0; i < kBlkTok; ++i) {
+        const float ki = in.raw[i][0][d], qi = in.raw[i][1][d], gi = per_channel ? in.raw[i][2][d] : in.g[i];
+        c *= gi;
+#pragma unroll
+        for (int j = 0; j < i; ++j) {
+          w[j] *= gi;
+          if (DELTA) dots[i * (i - 1) / 2 + j] += ki * w[j];
+          dots[6 + i * (i + 1) / 2 + j] += qi * w[j];
+        }
+        w[i] = ki;
+        dots[6 + i * (i + 1) / 2 + i] += qi * ki;
+        if (DELTA) vec.k[i][d] = make_float2(c * ki, c * ki);
+        vec.q[i][d] = make_float2(c * qi, c * qi);
+      }
+#pragma unroll
+      for (int i = 0; i < kBlkTok; ++i) vec.h[i][d] = make_float2(w[i], w[i]);
+      vec.c[d] = make_float2(c, c);
+    }
+    // sixteen sums over the warp: halves are exchanged, lane l ends with entry l >> 1
+#pragma unroll
+    for (int m = 8; m >= 1; m >>= 1)
+#pragma unroll
+      for (int a = 0; a < m; ++a) {
+        const bool up = (lane & (2 * m)) != 0;
+        const float keep = up ? dots[a + m] : dots[a], send = up ? dots[a] : dots[a + m];
+        dots[a] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * m);
+      }
+    dots[0] += __shfl_xor_sync(0xffffffffu, dots[0], 1);
+    if ((lane & 1) == 0) vec.gram[warp][lane >> 1] = dots[0];
+  };
+
+  if (t0 < t1) {
+    fetch(t0, sm.in[0]);
+    fetch(t0 + kBlkTok, sm.in[1]);
+    fetch(t0 + 2 * kBlkTok, sm.in[2]);
+  }
+  f32x2 S[2 * PIECES][CT / 2];
+#pragma unroll
+  for (int r = 0; r < 2 * PIECES; ++r)
+#pragma unroll
+    for (int a = 0; a < CT / 2; ++a) {
+      const int d = (r >> 1) * 16 + rg * 2 + (r & 1), ca = c0 + ((2 * a) ^ x), cb = c0 + ((2 * a + 1) ^ x);
+      const bool ok = carried && d < D;
+      S[r][a] = pack2(ok && ca < Dv ? gS[static_cast<long>(d) * Dv + ca] : 0.f, ok && cb < Dv ? gS[static_cast<long>(d) * Dv + cb] : 0.f);
+    }
+  if (t0 < t1) {
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncthreads();
+    prepare(sm.in[0], sm.vec[0]);
+  }
+  const int c_own = c0 + x;
+  for (int t = t0, n = 0; t < t1; t += kBlkTok, ++n) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");         // this thread's part of chunk n + 1
+    __syncthreads();                               // vectors of chunk n and inputs of n + 1 are here; everyone is done with n - 1
+    fetch(t + 3 * kBlkTok, sm.in[(n + 3) & 3]);
+    prepare(sm.in[(n + 1) & 3], sm.vec[(n + 1) & 1]);
+    const typename Sm::Vec& vec = sm.vec[n & 1];
+    const typename Sm::In& in = sm.in[n & 3];
+    float u[kBlkTok], r[kBlkTok];
+#pragma unroll
+    for (int i = 0; i < kBlkTok; ++i) u[i] = in.v[i][cw + x];
+    if (DELTA) {
+      blk_product<PIECES, CT>(S, &vec.k[0][0], rg, r);
+#pragma unroll
+      for (int i = 0; i < kBlkTok; ++i) {
+        float z = u[i] - r[i];
+#pragma unroll
+        for (int j = 0; j < i; ++j) z -= (vec.gram[0][i * (i - 1) / 2 + j] + vec.gram[1][i * (i - 1) / 2 + j]) * u[j];
+        u[i] = in.beta[i] * z;
+      }
+    }
+    blk_product<PIECES, CT>(S, &vec.q[0][0], rg, r);
+#pragma unroll
+    for (int i = 0; i < kBlkTok; ++i) {
+#pragma unroll
+      for (int j = 0; j <= i; ++j) r[i] += (vec.gram[0][6 + i * (i + 1) / 2 + j] + vec.gram[1][6 + i * (i + 1) / 2 + j]) * u[j];
+      if ((CT == 8 || (rg & 1) == (i >> 1)) && t + i < t1 && c_own < Dv) o[(static_cast<long>(t + i) * heads + h) * Dv + c_own] = r[i];
+    }
+    // state: the columns' u come from the lanes that own them
+#pragma unroll
+    for (int pc = 0; pc < PIECES; ++pc) {
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&vec.c[pc * 16 + rg * 2]);
+#pragma unroll
+      for (int a = 0; a < CT / 2; ++a) {
+        S[2 * pc][a] = mul2(S[2 * pc][a], w.x);
+        S[2 * pc + 1][a] = mul2(S[2 * pc + 1][a], w.y);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kBlkTok; ++i) {
+      f32x2 ua[CT / 2];
+#pragma unroll
+      for (int a = 0; a < CT / 2; ++a) {
+        const int la = (lane & 24) + ((2 * a) ^ x) * (8 / CT), lb = (lane & 24) + ((2 * a + 1) ^ x) * (8 / CT);
+        const float ux = __shfl_sync(0xffffffffu, u[i], la), uy = __shfl_sync(0xffffffffu, u[i], lb);
+        ua[a] = pack2(ux, uy);
+      }
+#pragma unroll
+      for (int pc = 0; pc < PIECES; ++pc) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&vec.h[i][pc * 16 + rg * 2]);
+#pragma unroll
+        for (int a = 0; a < CT / 2; ++a) {
+          S[2 * pc][a] = fma2(w.x, ua[a], S[2 * pc][a]);
+          S[2 * pc + 1][a] = fma2(w.y, ua[a], S[2 * pc + 1][a]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 2 * PIECES; ++r)
+#pragma unroll
+    for (int a = 0; a < CT / 2; ++a) {
+      const int d = (r >> 1) * 16 + rg * 2 + (r & 1), ca = c0 + ((2 * a) ^ x), cb = c0 + ((2 * a + 1) ^ x);
+      float fa, fb;
+      unpack2(S[r][a], fa, fb);
+      if (d < D && ca < Dv) gS[static_cast<long>(d) * Dv + ca] = fa;
+      if (d < D && cb < Dv) gS[static_cast<long>(d) * Dv + cb] = fb;
+    }
+}
+
+template <int PIECES, int CT, bool DELTA, bool WIDE>
+cudaError_t launch_delta_blk(dim3 grid, const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
+                             float* o, const int* cu, const int* start, const int* state_slot, int heads, int kv_heads, int D, int Dv,
+                             int per_channel, cudaStream_t s) {
+  auto kern = delta_scan_blk_kernel<PIECES, CT, DELTA, WIDE>;
+  constexpr int smem = sizeof(BlkSmem<16 * PIECES, 4 * CT * kBlkWarps>);
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  kern<<<grid, 32 * kBlkWarps, smem, s>>>(qkv, sq, col_k, col_v, beta, decay, state, o, cu, start, state_slot, heads, kv_heads, D, Dv, per_channel);
+  return cudaGetLastError();
+}
+
 // template sizes and block size of the column-resident kernels for a state of `rows` x `cols`; false when they do not fit
 bool pick_col_layout(int cols, int rows, int* rows_t, int* split_out, int* threads_out) {
   if (rows > 128 || cols < 1 || cols > 256) return false;
@@ -1000,10 +1299,29 @@ cudaError_t nrl_gla_prep(float* qkv, long sq, const float* a_raw, long sa, const
 }
 
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
-                           float* o, const int* cu, const int* start, const int* state_slot, int E, int heads, int kv_heads, int D,
-                           int Dv, int per_channel, int impl, cudaStream_t s) {
+                           float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
+                           int D, int Dv, int per_channel, int impl, cudaStream_t s) {
   if (E <= 0) return cudaSuccess;
-  if (Dv > 512 || heads % kv_heads != 0 || impl < 0 || impl > 3) return cudaErrorInvalidValue;
+  if (Dv > 512 || heads % kv_heads != 0 || impl < 0 || impl > 4) return cudaErrorInvalidValue;
+  // Steps of prompt portions: four tokens at a time.  The line lies at twelve tokens an entry because a thread's state is not read in
+  // whole lines: 64 entries x 16 heads of 128 x 128, portions of 2: 95 us against 50 (column-resident), 4: 97 / 65, 8: 111 / about 97; 16 entries of
+  // 2048: 2310 / 4350, one of 2048: 1564 / 2164, one of 70 with 8 heads of 64 x 64: 33 / 66.
+  if (D >= 1 && D <= 128 && Dv >= 1 && (impl == 4 || (impl == 0 && T >= 12L * E))) {
+    const bool wide = D % 4 == 0 && sq % 4 == 0 && col_k % 4 == 0 && reinterpret_cast<uintptr_t>(qkv) % 16 == 0 &&
+                     reinterpret_cast<uintptr_t>(decay) % 16 == 0;
+    // eight columns per thread unless that leaves SMs without a block (one entry of 2048, 16 heads: four columns 1564 us, eight 1816; 16 entries:
+    // 3730 / 2310)
+    const int ct = static_cast<long>(E) * heads * ((Dv + 63) / 64) >= 148 ? 8 : 4;
+    const dim3 grid(E, heads, (Dv + 8 * ct - 1) / (8 * ct));
+#define NRL_DELTAB(P_, C_, B_)                                                                                                   \
+  if ((D <= 64 ? 4 : 8) == P_ && ct == C_ && (beta != nullptr) == B_)                                                              \
+    return (wide ? launch_delta_blk<P_, C_, B_, true> : launch_delta_blk<P_, C_, B_, false>)(                                      \
+        grid, qkv, sq, col_k, col_v, beta, decay, state, o, cu, start, state_slot, heads, kv_heads, D, Dv, per_channel, s);
+    NRL_DELTAB(4, 4, true) NRL_DELTAB(4, 4, false) NRL_DELTAB(4, 8, true) NRL_DELTAB(4, 8, false)
+    NRL_DELTAB(8, 4, true) NRL_DELTAB(8, 4, false) NRL_DELTAB(8, 8, true) NRL_DELTAB(8, 8, false)
+#undef NRL_DELTAB
+  }
+  if (impl == 4) return cudaErrorInvalidValue;
   if (impl == 0 || impl == 1) {
     int rt, split, threads;
     if (pick_col_layout(Dv, D, &rt, &split, &threads)) {
