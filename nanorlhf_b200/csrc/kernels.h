@@ -30,9 +30,11 @@ cudaError_t nrl_gae_scan(const float* rewards, const float* values, float* adv, 
                          float gamma, float lam, cudaStream_t s);
 cudaError_t nrl_policy_loss(const float* new_lp, const float* old_lp, const float* adv, const uint8_t* mask,
                             const float* ref_lp, float cliprange, float kl_coef, long n, float* grad_unnorm,
-                            float* acc, cudaStream_t s);
+                            float* loss, float* stats, double* scratch, cudaStream_t s);
 cudaError_t nrl_value_loss(const float* vpred, const float* vold, const float* ret, const uint8_t* mask, float clip,
-                           long n, float* grad_unnorm, float* acc, cudaStream_t s);
+                           long n, float* grad_unnorm, float* loss, float* stats, double* scratch, cudaStream_t s);
+long nrl_loss_scratch_doubles(long n);     // doubles of scratch that a loss over n tokens needs (0: none)
+cudaError_t nrl_loss_grad(const float* grad_unnorm, const float* g_loss, const float* denom, long n, float* out, cudaStream_t s);
 cudaError_t nrl_adamw_flat(void* param, const void* grad, void* m, void* v, float* master, long n, int moments_bf16,
                            nrl::AdamHyper h, cudaStream_t s);
 

@@ -234,59 +234,25 @@ def gae_scan(rewards, values, gamma, lam):
     return adv, ret
 
 
-class _PolicyLossFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, new_lp, old_lp, adv, mask, ref_lp, cliprange, kl_coef):
-        _count()
-        grad, acc = ext().policy_loss(new_lp.contiguous(), old_lp.contiguous(), adv.contiguous(), mask.contiguous(),
-                                      None if ref_lp is None else ref_lp.contiguous(), cliprange, kl_coef)
-        denom = acc[1]
-        ctx.save_for_backward(grad, denom)
-        ctx.shape = new_lp.shape
-        ctx.mark_non_differentiable(acc)
-        return acc[0] / denom, acc
-
-    @staticmethod
-    def backward(ctx, g_loss, _g_acc):
-        grad, denom = ctx.saved_tensors
-        return (grad * (g_loss / denom)).view(ctx.shape), None, None, None, None, None, None
+def _count_loss(x):
+    _count(2 if x.requires_grad and torch.is_grad_enabled() else 1)          # forward and, later, backward
 
 
 def policy_loss_token(new_logp, old_logp, adv, mask, cliprange, ref_logp=None, kl_coef=0.0):
-    loss, acc = _PolicyLossFn.apply(new_logp.float(), old_logp.float(), adv.float(), mask, None if ref_logp is None
-                                    else ref_logp.float(), float(cliprange), float(kl_coef))
-    n = float(new_logp.numel())
-    with torch.no_grad():
-        d = acc[1]
-        stats = {"clipfrac": acc[2] / d, "approxkl_masked": 0.5 * acc[3] / d, "approxkl_all": 0.5 * acc[4] / n,
-                 "ratio_mean_all": acc[5] / n, "ratio_mean_masked": acc[6] / d}
-        if ref_logp is not None:
-            stats["refkl_all"] = acc[7] / n
-            stats["refkl_masked"] = acc[8] / d
-    return loss, stats
-
-
-class _ValueLossFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, vpred, vold, ret, mask, clip):
-        _count()
-        grad, acc = ext().value_loss(vpred.contiguous(), vold.contiguous(), ret.contiguous(), mask.contiguous(), clip)
-        ctx.save_for_backward(grad, acc[1])
-        ctx.shape = vpred.shape
-        ctx.mark_non_differentiable(acc)
-        return 0.5 * acc[0] / acc[1], acc
-
-    @staticmethod
-    def backward(ctx, g_loss, _g):
-        grad, denom = ctx.saved_tensors
-        return (grad * (g_loss / denom)).view(ctx.shape), None, None, None, None
+    _count_loss(new_logp)
+    loss, stats = ext().policy_loss(new_logp, old_logp, adv, mask, ref_logp, float(cliprange), float(kl_coef))
+    _, clipfrac, kl_masked, kl_all, ratio_all, ratio_masked, ref_all, ref_masked = stats
+    out = {"clipfrac": clipfrac, "approxkl_masked": kl_masked, "approxkl_all": kl_all, "ratio_mean_all": ratio_all,
+           "ratio_mean_masked": ratio_masked}
+    if ref_logp is not None:
+        out["refkl_all"], out["refkl_masked"] = ref_all, ref_masked
+    return loss, out
 
 
 def value_loss(vpred, values_old, returns, mask, cliprange_value):
-    loss, acc = _ValueLossFn.apply(vpred.float(), values_old.float(), returns.float(), mask, float(cliprange_value))
-    with torch.no_grad():
-        clipfrac = acc[2] / acc[1]
-    return loss, clipfrac
+    _count_loss(vpred)
+    loss, stats = ext().value_loss(vpred, values_old, returns, mask, float(cliprange_value))
+    return loss, stats[1]
 
 
 def adamw_flat(param, grad, m, v, lr, beta1, beta2, eps, wd, step, scale=1.0, master=None):
