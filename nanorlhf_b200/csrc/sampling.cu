@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(kSampThreads) sample_top_p_kernel(const T* __r
 // a serial read-modify-write chain per thread (ncu: IPC 1.0 at 8 warps per SM when ported as is).  This kernel needs no
 // histogram: it draws a token from the FULL softmax (per-thread partial sums -> owner thread walks its elements), then
 // verifies the nucleus condition for that token alone with one more streaming pass -- the token is kept iff the mass of the
-// strictly more probable tokens is < top_p (exactly torch's `(cumsum - p) < top_p` rule, with no 1.1 % cut-off resolution); a
+// strictly more probable tokens is < top_p (exactly torch's `(cumsum - p) < top_p` rule, with no 1.1 % cut-off resolution; both sides of
+// the comparison are the same multiply-add, so tokens that tie with the drawn one never count as more probable); a
 // rejected draw (probability ~ 1 - top_p) is redrawn from the next Philox offset, reusing the partial sums.
 NRL_DEVICE uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 NRL_DEVICE uint32_t cluster_nctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
@@ -297,6 +298,10 @@ constexpr int kSmemPerLane = kSmemThreads / 32;
 constexpr int kSliceBytesMax = 216 * 1024;
 constexpr int kMaxAttempts = 32;                                  // P(32 rejections) <= (1 - top_p)^32; dispatch keeps top_p >= 0.5
 constexpr int kXSlots = 6;                                        // max, mass, and (candidate, mass above) x attempt parity
+constexpr int kPieceVecs = 2 * kSmemThreads;                      // a slice arrives in pieces of two vectors per thread (16 KB)
+constexpr int kPiecesMax = (kSliceBytesMax / 16 + kPieceVecs - 1) / kPieceVecs;
+constexpr int kWalkMax = (kSliceBytesMax / 16 + kSmemThreads - 1) / kSmemThreads;      // vectors of one thread at most
+static_assert(kWalkMax <= 32, "a lane per vector of the drawn thread");
 
 // every CTA of the cluster publishes `n` floats into slot [my rank] of `dst` in every CTA; after the cluster barrier all CTAs hold
 // all contributions and combine them in rank order (identical result everywhere).  A CTA can run at most one cluster barrier
@@ -315,34 +320,51 @@ NRL_DEVICE uint4 lds_v4(uint32_t saddr) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(saddr));
   return r;
 }
-// visit the slice: thread t owns 16-byte vectors t, t + T, t + 2T, ... (ascending), four loads in flight
-template <typename F>
-NRL_DEVICE void slice_for_each(const __nv_bfloat16* zs, int nvec, F&& f) {
-  constexpr int U = 4;
-  const uint32_t zb = smem_u32(zs);
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * kSmemThreads) {
-    uint4 raw[U];
+// largest of the eight bf16 of a vector (NaN is ignored, as by fmaxf)
+NRL_DEVICE float vec_max(const uint4& raw) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const float2 f = __bfloat1622float2(__hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+  return fmaxf(f.x, f.y);
+}
+NRL_DEVICE float vec_min(const uint4& raw) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const float2 f = __bfloat1622float2(__hmin2(__hmin2(h[0], h[1]), __hmin2(h[2], h[3])));
+  return fminf(f.x, f.y);
+}
+NRL_DEVICE uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+NRL_DEVICE uint64_t make_pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+// the vector's eight x * sc + off
+NRL_DEVICE void vec_affine(const uint4& raw, float sc, float off, float (&e)[8]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  const uint64_t s2 = make_pair(sc, sc), o2 = make_pair(off, off);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int v = v0 + u * kSmemThreads;
-      raw[u] = lds_v4(zb + static_cast<uint32_t>(min(v, nvec - 1)) * 16u);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int v = v0 + u * kSmemThreads;
-      if (v < nvec) {
-        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 x = unpack_bf16x2(w[j]);
-          f(v * 8 + 2 * j, x.x);
-          f(v * 8 + 2 * j + 1, x.y);
-        }
-      }
-    }
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16x2(w[j]);
+    const uint64_t r = fma_pair(make_pair(f.x, f.y), s2, o2);
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(e[2 * j]), "=f"(e[2 * j + 1]) : "l"(r));
   }
 }
+NRL_DEVICE float vec_elem(const uint4& raw, int j) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  const float2 f = unpack_bf16x2(w[j >> 1]);
+  return (j & 1) ? f.y : f.x;
+}
 
+// Thread t owns the 16-byte vectors t, t + 512, ... of the slice; the draw's order is (CTA, thread, vector, element), and every sum that
+// decides a draw is formed in that order from the row's maximum, so that a (seed, row, step) names one token for good.
+// The maximum is taken piece by piece as the bulk copies arrive and the first uniform number is drawn meanwhile; the drawn thread's
+// exponentials are formed by a warp and only added in turn; the verification skips vectors without a more probable token.
+// 1024 x 151 936: 201 us (230 with a maximum pass behind the whole copy and a one-thread walk); the floors are 47 us of reads and about
+// 70 us of 2^x on the special-function unit, the rest waits at the row's exchanges.  One pass for maximum and mass (189 us) and half
+// slices on top of it (180 us) change the sums' last bits and with them 1 to 3 tokens in 1024.
 __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(const __nv_bfloat16* __restrict__ logits, long row_stride,
                                                                             int V, int slice, float inv_temp, float top_p,
                                                                             unsigned long long seed, unsigned long long step,
@@ -350,12 +372,12 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
                                                                             const int* __restrict__ row_steps,
                                                                             int* __restrict__ out_tokens) {
   extern __shared__ __align__(128) unsigned char s_dyn[];
-  const __nv_bfloat16* zs = reinterpret_cast<const __nv_bfloat16*>(s_dyn);      // this CTA's slice of the row
-  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ __align__(8) uint64_t s_bar[kPiecesMax];
   __shared__ float red[32];
   __shared__ float s_pub[2];
   __shared__ float s_x[kXSlots][kMaxCluster][2];           // exchange slots, written by the peers
   __shared__ float chunk_sum[kSmemThreads];
+  __shared__ __align__(16) float s_walk[kWalkMax][8];
   __shared__ float s_resid, s_u;
   __shared__ int s_owner;
   const uint32_t crank = cluster_ctarank(), csize = cluster_nctarank();
@@ -365,29 +387,47 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
   const int Vl = max(0, min(slice, V - e0));                                     // tokens in the slice (multiple of 8)
   const int nvec = Vl / 8;
   const float sc = inv_temp * 1.4426950408889634f;                               // logits -> log2 domain
+  const uint32_t zb = smem_u32(s_dyn);                                           // this CTA's slice of the row
+  auto load = [&](int v) { return lds_v4(zb + static_cast<uint32_t>(v) * 16u); };
 
   // A CTA's shared memory may only be written by its peers once it is known to be running: arrive now, wait right before the
   // first exchange (the load and the first pass hide the barrier).
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   // ---- the only global read of the row: 1/C of it, as a few bulk async copies ----
   if (tid == 0) {
-    mbar_init(&s_bar, 1);
+    const int pieces = (nvec + kPieceVecs - 1) / kPieceVecs;
+    for (int i = 0; i < pieces; ++i) mbar_init(&s_bar[i], 1);
     fence_mbar_init();
-    const uint32_t bytes = static_cast<uint32_t>(Vl) * 2u;
-    if (bytes > 0) {
-      mbar_arrive_expect_tx(&s_bar, bytes);
-      const unsigned char* src = reinterpret_cast<const unsigned char*>(logits + static_cast<long>(row) * row_stride + e0);
-      for (uint32_t off = 0; off < bytes; off += 32768u) bulk_load_1d(s_dyn + off, src + off, min(32768u, bytes - off), &s_bar);
-    } else {
-      mbar_arrive(&s_bar);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(logits + static_cast<long>(row) * row_stride + e0);
+    for (int i = 0; i < pieces; ++i) {
+      const uint32_t off = static_cast<uint32_t>(i) * kPieceVecs * 16u, bytes = min(kPieceVecs * 16u, static_cast<uint32_t>(Vl) * 2u - off);
+      mbar_arrive_expect_tx(&s_bar[i], bytes);
+      bulk_load_1d(s_dyn + off, src + off, bytes, &s_bar[i]);
     }
   }
-  __syncthreads();                                         // the barrier is initialised before anyone polls it
-  mbar_wait(&s_bar, 0);
+  const unsigned long long rid = static_cast<unsigned long long>(row_ids ? row_ids[row] : row);
+  const unsigned long long off0 = (step + (row_steps ? static_cast<unsigned long long>(row_steps[row]) : 0ull)) * kMaxAttempts;
+  auto draw = [&](int attempt) {                           // uniform in (0, 1], a function of (seed, row id, tokens generated, attempt)
+    curandStatePhilox4_32_10_t st;                         // only: every CTA of the cluster derives the same draw
+    curand_init(seed, rid, off0 + attempt, &st);
+    return curand_uniform(&st);
+  };
+  if (tid == 32) s_u = draw(0);
+  __syncthreads();                                         // the barriers are initialised before anyone polls them
 
   // ---- pass 1: row maximum ----
   float mx = -INFINITY;
-  slice_for_each(zs, nvec, [&](int, float x) { mx = fmaxf(mx, x * sc); });
+  for (int v0 = tid, piece = 0; v0 < nvec; v0 += kPieceVecs, ++piece) {
+    mbar_wait(&s_bar[piece], 0);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int v = v0 + k * kSmemThreads;
+      if (v < nvec) {
+        const uint4 raw = load(v);
+        mx = fmaxf(mx, (sc >= 0.f ? vec_max(raw) : vec_min(raw)) * sc);
+      }
+    }
+  }
   mx = block_reduce_max(mx, red);
   if (tid == 0) s_pub[0] = mx;
   __syncthreads();
@@ -398,7 +438,13 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
 
   // ---- pass 2: un-normalised probability mass per thread, per CTA, per row ----
   float mine = 0.f;
-  slice_for_each(zs, nvec, [&](int, float x) { mine += exp2f(x * sc - mx); });
+#pragma unroll 4
+  for (int v = tid; v < nvec; v += kSmemThreads) {
+    float e[8];
+    vec_affine(load(v), sc, -mx, e);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mine += exp2f(e[j]);
+  }
   chunk_sum[tid] = mine;
   const float cta_mass = block_reduce_sum(mine, red);      // (its barriers also publish chunk_sum)
   if (tid == 0) s_pub[0] = cta_mass;
@@ -411,18 +457,13 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
     Z += s_x[1][r][0];
     if (s_x[1][r][0] > 0.f) last_with_mass = static_cast<int>(r);
   }
-  const unsigned long long rid = static_cast<unsigned long long>(row_ids ? row_ids[row] : row);
-  const unsigned long long off0 = (step + (row_steps ? static_cast<unsigned long long>(row_steps[row]) : 0ull)) * kMaxAttempts;
-
 #pragma unroll 1
   for (int attempt = 0; attempt < kMaxAttempts; ++attempt) {
-    if (tid == 0) {
-      curandStatePhilox4_32_10_t st;                       // a function of (seed, row id, tokens generated, attempt) only:
-      curand_init(seed, rid, off0 + attempt, &st);         // every CTA of the cluster derives the same draw
-      s_u = curand_uniform(&st) * Z;                       // (0, Z]
+    if (attempt > 0) {
+      if (tid == 0) s_u = draw(attempt);
+      __syncthreads();
     }
-    __syncthreads();
-    const float u = s_u;
+    const float u = s_u * Z;                               // (0, Z]
     int owner_cta = last_with_mass;
     {
       float acc = 0.f;
@@ -467,45 +508,57 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
           s_resid = resid;
         }
       }
-      __syncthreads();
-      if (tid == s_owner) {                                // walk this thread's elements in the order pass 2 summed them
-        const float resid = s_resid;
-        const uint32_t zb = smem_u32(zs);
-        float acc2 = 0.f, d_tok = 0.f, d_last = 0.f;
-        int tok = -1, last = 0;
-        for (int v = tid; v < nvec && tok < 0; v += kSmemThreads) {
-          const uint4 raw = lds_v4(zb + static_cast<uint32_t>(v) * 16u);
-          const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+      if (tid < 32) {
+        __syncwarp();
+        // the owner's elements in the order pass 2 summed them: lane k forms the exponentials of its k-th vector, lane 0 adds them up
+        const int owner = s_owner, vk = owner + tid * kSmemThreads;
+        if (vk < nvec) {
+          float e[8];
+          vec_affine(load(vk), sc, -mx, e);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float2 xx = unpack_bf16x2(w[j >> 1]);
-            const float e = ((j & 1) ? xx.y : xx.x) * sc - mx;
-            if (tok < 0) {
-              acc2 += exp2f(e);
-              last = v * 8 + j;
-              d_last = -e;
-              if (acc2 >= resid) { tok = last; d_tok = -e; }
+          for (int j = 0; j < 8; ++j) s_walk[tid][j] = exp2f(e[j]);
+        }
+        __syncwarp();
+        if (tid == 0) {
+          const float resid = s_resid;
+          float acc2 = 0.f;
+          int tok = -1, last = 0;
+          for (int k = 0; tok < 0 && owner + k * kSmemThreads < nvec; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(&s_walk[k][0]), c = *reinterpret_cast<const float4*>(&s_walk[k][4]);
+            const float e[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+            last = (owner + k * kSmemThreads) * 8 + 7;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              acc2 += e[j];
+              if (tok < 0 && acc2 >= resid) tok = last - 7 + j;
             }
           }
+          if (tok < 0) tok = last;
+          s_pub[0] = __int_as_float(e0 + tok);
+          s_pub[1] = fmaf(vec_elem(load(tok >> 3), tok & 7), sc, -mx);     // octaves above the row maximum (at most 0)
         }
-        if (tok < 0) { tok = last; d_tok = d_last; }
-        s_pub[0] = __int_as_float(e0 + tok);
-        s_pub[1] = d_tok;                                  // octaves below the row maximum
       }
     }
     __syncthreads();
     float (*slot)[2] = s_x[2 + 2 * (attempt & 1)];
     cluster_publish(slot, s_pub, 2, crank, csize);         // only the owner's entry is read
     const int tok = __float_as_int(slot[owner_cta][0]);
-    const float d_tok = slot[owner_cta][1];
+    const float e_tok = slot[owner_cta][1];
     bool accept = top_p >= 1.f || attempt == kMaxAttempts - 1;
     if (!accept) {
       // ---- verification pass: mass of the strictly more probable tokens ----
       float above = 0.f;
-      slice_for_each(zs, nvec, [&](int, float x) {
-        const float d = mx - x * sc;
-        above += (d < d_tok) ? exp2f(-d) : 0.f;
-      });
+#pragma unroll 4
+      for (int v = tid; v < nvec; v += kSmemThreads) {
+        const uint4 raw = load(v);
+        if (fmaf(sc >= 0.f ? vec_max(raw) : vec_min(raw), sc, -mx) > e_tok) {
+          float e[8];
+          vec_affine(raw, sc, -mx, e);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (e[j] > e_tok) above += exp2f(e[j]);
+        }
+      }
       above = block_reduce_sum(above, red);
       if (tid == 0) s_pub[0] = above;
       __syncthreads();
