@@ -237,7 +237,7 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
   maps[1] = map_b(b);
   maps[2] = K2 > 0 ? map_a(*a2) : maps[0];
   maps[3] = K2 > 0 ? map_b(*b2) : maps[1];
-  maps[4] = f32 ? maps[0] : nrl::make_tma_2d(out.data_ptr(), M, N, out.stride(0) * 2, 128, 64, BF, 2);
+  maps[4] = f32 ? maps[0] : nrl::make_tma_2d(out.data_ptr(), M, N, out.stride(0) * 2, 32, 64, BF, 2);
   nrl::tc::TcParams p{};
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K); p.K2 = static_cast<int>(K2);
   p.alpha = static_cast<float>(alpha);
@@ -282,7 +282,7 @@ torch::Tensor gemm_tc_batched(const torch::Tensor& a, const torch::Tensor& b, c1
   CUtensorMap maps[3];
   maps[0] = nrl::make_tma_3d(a.data_ptr(), B, M, K, a.stride(1) * 2, a.stride(0) * 2, 128, 64, BF, 2);
   maps[1] = nrl::make_tma_3d(b.data_ptr(), B, N, K, b.stride(1) * 2, b.stride(0) * 2, ch.bn / ch.cg, 64, BF, 2);
-  maps[2] = nrl::make_tma_3d(out.data_ptr(), B, M, N, out.stride(1) * 2, out.stride(0) * 2, 128, 64, BF, 2);
+  maps[2] = nrl::make_tma_3d(out.data_ptr(), B, M, N, out.stride(1) * 2, out.stride(0) * 2, 32, 64, BF, 2);
   nrl::tc::TcParams p{};
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K); p.alpha = 1.f; p.batch = static_cast<int>(B);
   check(nrl_gemm_tc_batched(maps, &p, ch.cg, ch.bn, num_sms(), cur_stream()), "gemm_tc_batched");
@@ -311,7 +311,7 @@ torch::Tensor gemm_tc_swiglu(const torch::Tensor& a, const torch::Tensor& w_inte
   maps[1] = nrl::make_tma_2d(w_interleaved.data_ptr(), N2, K, w_interleaved.stride(0) * 2, ch.bn / ch.cg, 64, BF, 2);
   maps[2] = maps[0];
   maps[3] = maps[1];
-  maps[4] = nrl::make_tma_2d(out.data_ptr(), M, N2 / 2, out.stride(0) * 2, 128, 64, BF, 2);
+  maps[4] = nrl::make_tma_2d(out.data_ptr(), M, N2 / 2, out.stride(0) * 2, 32, 64, BF, 2);
   nrl::tc::TcParams p{};
   p.M = static_cast<int>(M); p.N = static_cast<int>(N2); p.K = static_cast<int>(K); p.alpha = 1.f;
   check(nrl_gemm_tc(maps, &p, ch.cg, ch.bn, 0, 0, nrl::tc::EPI_SWIGLU, num_sms(), cur_stream()), "gemm_tc_swiglu");
@@ -406,7 +406,7 @@ torch::Tensor gemm_tc_fp8(const torch::Tensor& aq, const torch::Tensor& a_scale,
   CUtensorMap maps[3];
   maps[0] = nrl::make_tma_2d(aq.data_ptr(), M, K, aq.stride(0), 128, 128, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1);
   maps[1] = nrl::make_tma_2d(bq.data_ptr(), N, K, bq.stride(0), ch.bn / ch.cg, 128, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1);
-  maps[2] = nrl::make_tma_2d(out.data_ptr(), M, No, out.stride(0) * 2, 128, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
+  maps[2] = nrl::make_tma_2d(out.data_ptr(), M, No, out.stride(0) * 2, 32, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
   nrl::tc::TcParams p{};
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K); p.alpha = 1.f;
   p.row_scale = a_scale.data_ptr<float>();

@@ -22,9 +22,13 @@
 //   * epilogues       EPI_BF16: alpha, bias, exact GELU -> bf16 through swizzled smem + TMA store;
 //                     EPI_F32 : fp32 row-major out (+)= alpha * acc  (weight-gradient accumulation, lm-head dW).
 //
-// Pipeline (per CTA, 192 threads): warp 0 = TMA producer, warp 1 = MMA issuer (+ TMEM allocator), warps 2-5 = epilogue;
+// Pipeline (per CTA, 320 threads): warp 0 = TMA producer, warp 1 = MMA issuer (+ TMEM allocator), warps 2-9 = epilogue;
 // smem ring of kStages k-blocks behind full/empty mbarriers, two TMEM accumulators so the epilogue of tile i overlaps the
 // main loop of tile i+1, persistent grid with a grouped (L2-friendly) tile order.
+// An epilogue warp owns 32 rows of every other 64-column chunk and stages and stores them on its own (4 KB slab, one TMA store), so no
+// barrier joins the warps.  With four warps that met at two barriers per chunk and read the bias value by value, a 128 x 256 tile's
+// epilogue took longer than a main loop of K = 1024: the six linears of a reward layer (24 571 tokens) 742 -> 429 us, its bias tables
+// (K = 64) 235 -> 92 us each; nothing changes above K = 4096.
 #include "common.cuh"
 #include "gemm_tc.h"
 
@@ -34,11 +38,13 @@ namespace tc {
 constexpr int BLOCK_M = 128;        // rows per CTA (a CTA pair covers 256)
 constexpr int BLOCK_K = 64;         // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int kThreads = 192;
-constexpr int kEpiThreads = 128;
+constexpr int kEpiWarps = 8;        // two per TMEM lane quadrant
+constexpr int kEpiThreads = 32 * kEpiWarps;
+constexpr int kThreads = 64 + kEpiThreads;
 constexpr int kABytes = BLOCK_M * BLOCK_K * 2;      // 16 KB
 constexpr int kPanelBytes = 64 * 128;               // one [64 x 64] bf16 panel of an MN-major operand
-constexpr int kStagingBytes = BLOCK_M * 128;        // 128 rows x 64 bf16 output slab
+constexpr int kSlabBytes = 32 * 128;                // 32 rows x 64 bf16 output slab of an epilogue warp
+constexpr int kStagingBytes = kEpiWarps * kSlabBytes;
 constexpr int kSmemBudget = 227 * 1024;
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;         // clears the CTA-pair peer bit of a shared::cluster address
 constexpr int GROUP_M = 8;                          // tile rows per L2 super-row
@@ -51,10 +57,10 @@ struct Cfg {
   static constexpr int kBPanels = (kBRows + 63) / 64;
   static constexpr int kBBytes = B_MN ? kBPanels * kPanelBytes : kBRows * BLOCK_K * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStagesFit = (kSmemBudget - 2 * kStagingBytes - 1024) / kStageBytes;
+  static constexpr int kStagesFit = (kSmemBudget - kStagingBytes - 1024) / kStageBytes;
   static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
   static constexpr int kStagingOff = kStages * kStageBytes;
-  static constexpr int kBarOff = kStagingOff + 2 * kStagingBytes;
+  static constexpr int kBarOff = kStagingOff + kStagingBytes;
   static constexpr int kTotal = kBarOff + 512;
   static constexpr uint32_t kTmemCols = (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;
   static_assert(kStageBytes % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
@@ -224,7 +230,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);                      // one (multicast) commit
-      mbar_init(&tmem_empty[i], CG * kEpiThreads / 32); // the epilogue warps (of both CTAs)
+      mbar_init(&tmem_empty[i], CG * kEpiWarps); // the epilogue warps (of both CTAs)
     }
     fence_mbar_init();
   }
@@ -328,11 +334,36 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     // ================================ epilogue (every CTA: its own 128 rows) ================================
     const int quad = warp & 3;                          // TMEM lane quadrant this warp may read
     const int row_in_tile = quad * 32 + lane;
-    const int epi_tid = threadIdx.x - 64;
+    const int epi_tid = threadIdx.x - 64, group = (warp - 2) >> 2;      // the two warps of a quadrant take alternate chunks
     int acc = 0;
     uint32_t acc_phase = 0;
-    uint8_t* staging = smem + C::kStagingOff;
-    int store_buf = 0;
+    uint8_t* slab = smem + C::kStagingOff + (warp - 2) * kSlabBytes;
+    const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+    // the accumulator has been read by this warp
+    auto release_acc = [&]() {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_leader(&tmem_empty[acc]);
+        else mbar_arrive(&tmem_empty[acc]);
+      }
+    };
+    // 64 packed columns of this thread's row -> slab -> global
+    auto store_slab = [&](const uint32_t (&pk)[32], int col, int row0, int b) {
+      if (lane == 0) tma_store_wait_read<0>();                          // the warp's previous store has drained
+      __syncwarp();
+      uint8_t* rowp = slab + lane * 128;
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8)
+        *reinterpret_cast<uint4*>(rowp + ((q8 ^ (lane & 7)) * 16)) = make_uint4(pk[q8 * 4], pk[q8 * 4 + 1], pk[q8 * 4 + 2], pk[q8 * 4 + 3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (BATCH) tma_store_3d(&tmD, slab, col, row0, b);
+        else tma_store_2d(&tmD, slab, col, row0);
+        tma_store_commit();
+      }
+    };
     for (int w = unit; w < num_work; w += num_units) {
       const int tile_id = BATCH ? w % tiles_per_batch : w / splits;
       const int bidx = BATCH ? w / tiles_per_batch : 0;
@@ -359,15 +390,11 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         // bytes, for the partial stores here and for the reduction's loads below
         float* mine = p.ws + (static_cast<long>(w % splits) * (num_m * num_n) + tile_id) * tile_elems + row_in_tile * 4;
 #pragma unroll 1
-        for (int ch = 0; ch < BN / 32; ++ch) {
+        for (int ch = group; ch < BN / 32; ch += 2) {
           uint32_t v[32];
           tmem_ld_32x32b_x32(t_acc + ch * 32, v);
           tmem_ld_wait();
-          if (ch == BN / 32 - 1) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-          }
+          if (ch + 2 >= BN / 32) release_acc();
 #pragma unroll
           for (int j = 0; j < 32; j += 4)
             __stcg(reinterpret_cast<float4*>(mine + (ch * 8 + (j >> 2)) * (BLOCK_M * 4)),
@@ -388,7 +415,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           const long split_stride = static_cast<long>(num_m * num_n) * tile_elems;
           __nv_bfloat16* orow = p.out_bf16 + static_cast<long>(row) * p.out_stride + c.n_blk * BN;
 #pragma unroll 1
-          for (int c0 = 0; c0 < BN; c0 += 32) {
+          for (int c0 = group * 32; c0 < BN; c0 += 64) {
             if (c.n_blk * BN + c0 >= p.N) break;
             float acc[32];
 #pragma unroll
@@ -429,19 +456,18 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         continue;
       }
 #pragma unroll 1
-      for (int ch = 0; ch < BN / 64; ++ch) {
+      for (int it = 0;; ++it) {
+        // SwiGLU: two neighbouring chunks make one output slab and stay with one warp
+        const int ch = EPI == EPI_SWIGLU ? (it >> 1) * 4 + group * 2 + (it & 1) : it * 2 + group;
+        if (ch >= BN / 64) {
+          if (it == 0) release_acc();                   // no chunk for this warp
+          break;
+        }
         uint32_t v[2][32];
         tmem_ld_32x32b_x32(t_acc + ch * 64, v[0]);
         tmem_ld_32x32b_x32(t_acc + ch * 64 + 32, v[1]);
         tmem_ld_wait();
-        if (ch == BN / 64 - 1) {                        // every TMEM read of this accumulator has retired
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (CG == 2) mbar_arrive_leader(&tmem_empty[acc]);
-            else mbar_arrive(&tmem_empty[acc]);
-          }
-        }
+        if ((EPI == EPI_SWIGLU ? ((it + 1) >> 1) * 4 + group * 2 + ((it + 1) & 1) : ch + 2) >= BN / 64) release_acc();      // its last one
         const int col0 = c.n_blk * BN + ch * 64;
         if (EPI == EPI_F32 && GROUPED && p.out_bf16 != nullptr && p.act == 2) {
           // grouped up projection with the squared ReLU formed here: a chunk yields 64 activations of this row
@@ -521,67 +547,51 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             if ((ch & 1) == 0) sw_packed[j / 2] = pk;     // static indices: the array stays in registers
             else sw_packed[16 + j / 2] = pk;
           }
-          if (ch & 1) {
-            uint8_t* buf = staging + store_buf * kStagingBytes;
-            if (epi_tid == 0) tma_store_wait_read<1>();
-            named_barrier_sync(1, kEpiThreads);
-            uint8_t* rowp = buf + row_in_tile * 128;
-#pragma unroll
-            for (int q8 = 0; q8 < 8; ++q8)
-              *reinterpret_cast<uint4*>(rowp + ((q8 ^ (row_in_tile & 7)) * 16)) =
-                  make_uint4(sw_packed[q8 * 4], sw_packed[q8 * 4 + 1], sw_packed[q8 * 4 + 2], sw_packed[q8 * 4 + 3]);
-            fence_proxy_async_smem();
-            named_barrier_sync(2, kEpiThreads);
-            if (epi_tid == 0) {
-              tma_store_2d(&tmD, buf, c.n_blk * (BN / 2) + (ch >> 1) * 64, m_blk * BLOCK_M);
-              tma_store_commit();
-            }
-            store_buf ^= 1;
-          }
+          if ((ch & 1) && c.n_blk * (BN / 2) + (ch >> 1) * 64 < p.N / 2 && m_blk * BLOCK_M + quad * 32 < p.M)
+            store_slab(sw_packed, c.n_blk * (BN / 2) + (ch >> 1) * 64, m_blk * BLOCK_M + quad * 32, 0);
         } else {
-          uint8_t* buf = staging + store_buf * kStagingBytes;
-          if (epi_tid == 0) tma_store_wait_read<1>();   // the store that last used `buf` has drained
-          named_barrier_sync(1, kEpiThreads);
           uint32_t packed[32];
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
+          for (int j = 0; j < 64; j += 8) {
+            const int col = col0 + j;
+            float x[8];
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              float x0 = __uint_as_float(v[h][j]) * p.alpha, x1 = __uint_as_float(v[h][j + 1]) * p.alpha;
-              const int col = col0 + h * 32 + j;
-              if (FP8) {
-                const float rs = row_ok ? p.row_scale[row] : 0.f;
-                x0 *= rs * ((col < p.N) ? p.col_scale[col] : 0.f);
-                x1 *= rs * ((col + 1 < p.N) ? p.col_scale[col + 1] : 0.f);
-              }
-              if (p.bias != nullptr) {
-                if (col < p.N) x0 += __bfloat162float(p.bias[col]);
-                if (col + 1 < p.N) x1 += __bfloat162float(p.bias[col + 1]);
-              }
-              if (p.act == 1) {
-                x0 = gelu_erf_tc(x0);
-                x1 = gelu_erf_tc(x1);
-              }
-              packed[h * 16 + j / 2] = pack_bf16x2(x0, x1);
+            for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[j >> 5][(j & 31) + e]) * p.alpha;
+            if (FP8) {
+              const float rs = row_ok ? p.row_scale[row] : 0.f;
+#pragma unroll
+              for (int e = 0; e < 8; ++e) x[e] *= rs * ((col + e < p.N) ? p.col_scale[col + e] : 0.f);
             }
-          uint8_t* rowp = buf + row_in_tile * 128;
+            if (p.bias != nullptr && col < p.N) {         // N % 8 == 0
+              uint32_t bw[4];
+              if (bias_vec) {
+                const uint4 bv = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
+                bw[0] = bv.x; bw[1] = bv.y; bw[2] = bv.z; bw[3] = bv.w;
+              } else {
+                const uint16_t* b16 = reinterpret_cast<const uint16_t*>(p.bias + col);
 #pragma unroll
-          for (int q8 = 0; q8 < 8; ++q8)
-            *reinterpret_cast<uint4*>(rowp + ((q8 ^ (row_in_tile & 7)) * 16)) =
-                make_uint4(packed[q8 * 4], packed[q8 * 4 + 1], packed[q8 * 4 + 2], packed[q8 * 4 + 3]);
-          fence_proxy_async_smem();
-          named_barrier_sync(2, kEpiThreads);
-          if (epi_tid == 0) {
-            if (BATCH) tma_store_3d(&tmD, buf, col0, m_blk * BLOCK_M, bidx);
-            else tma_store_2d(&tmD, buf, col0, m_blk * BLOCK_M);
-            tma_store_commit();
+                for (int e = 0; e < 4; ++e) bw[e] = b16[2 * e] | (static_cast<uint32_t>(b16[2 * e + 1]) << 16);
+              }
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 bf = unpack_bf16x2(bw[e]);
+                x[2 * e] += bf.x;
+                x[2 * e + 1] += bf.y;
+              }
+            }
+            if (p.act == 1) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) x[e] = gelu_erf_tc(x[e]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) packed[j / 2 + e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
           }
-          store_buf ^= 1;
+          if (col0 < p.N && m_blk * BLOCK_M + quad * 32 < p.M) store_slab(packed, col0, m_blk * BLOCK_M + quad * 32, bidx);
         }
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
-    if (EPI != EPI_F32 && !SPLIT && epi_tid == 0) tma_store_wait<0>();
+    if (EPI != EPI_F32 && !SPLIT && lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -823,7 +833,7 @@ extern "C" cudaError_t nrl_gemm_tc_splitk(const CUtensorMap* maps, const nrl::tc
 }
 
 // maps = {A, B, A2, B2, D}; operand boxes (tma_host.h): K-major operand [rows, K]: box {rows = 128 (A) | BN/CG (B), 64};
-// MN-major operand [K, cols]: box {64, 64}; D: box {128, 64}.  Unused maps may repeat a valid one.
+// MN-major operand [K, cols]: box {64, 64}; D: box {32, 64}.  Unused maps may repeat a valid one.
 extern "C" cudaError_t nrl_gemm_tc(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int a_mn, int b_mn,
                                    int epi, int num_sms, cudaStream_t stream) {
   using namespace nrl::tc;
