@@ -1,52 +1,26 @@
 // tcgen05 / TMEM / TMA flash-attention FORWARD (causal, packed varlen, GQA, head_dim 128) for sm_100a.
 //
-// One CTA = 256 query rows of one head as TWO 128-row tiles (A, B) that share one K/V ring, so every K/V byte
-// fetched from L2 feeds two tiles and the two softmax warpgroups hide each other's latencies (2 warps per SMSP).
-// KV is streamed in blocks of 64 keys.
-//   warp 0       TMA producer : Q tiles once, then K_j / V_j (3-stage ring), 128B-swizzled panels of 64 dims
-//   warp 1       MMA issuer   : S_X,j = Q_X K_j^T  (8 x tcgen05.mma 128x64x16, both operands K-major) -> TMEM S_X[j%2]
-//                               O_X  += P_X,j V_j  (4 x tcgen05.mma 128x128x16, A = P in smem K-major, B = V MN-major)
-//   warps 2..5   softmax of tile A, warps 6..9 softmax of tile B: thread i owns query row i (TMEM lane i):
-//                               tcgen05.ld S -> mask -> online max with lazy (2^8) rescale -> exp2 -> bf16 P into
-//                               swizzled smem; rescales O in TMEM when needed; final O / l and LSE go straight to HBM
-// TMEM (512 cols): S_A[2] 0..127, S_B[2] 128..255, O_A 256..383, O_B 384..511.
-// SMEM: Q 64 KB + 3 x (K 16 KB + V 16 KB) + P 2 tiles x 2 buffers x 16 KB = 224 KB.
-// The softmax never waits for the tensor pipe on the common path: P is double buffered (pv_done[X][b] guards reuse) and O is
-// only rescaled - which needs PV of the previous block retired - when a row maximum grew by more than 2^8.
+// Work item: 256 query rows of one head as TWO 128-row tiles (A, B) that share one K/V ring, walking the keys in blocks of 128.
+//   warp 0       TMA producer : Q tiles, then K_0, V_0, K_1, V_1 ... into a ring of four 32 KB tiles (128B-swizzled panels of 64 dims)
+//   warp 1       MMA issuer   : S_X = Q_X K_j^T, then per block O_X += P_X V_j and at once the next S_X, tiles alternating, so that the
+//                               tensor pipe works on one tile while the other is in its softmax
+//   warp 2       finds the next item (which sequence, which rows) while the current one is computed
+//   warps 4..11  one thread per query row: scores from TMEM, mask, online softmax (attention_tc.cuh), P as bf16 back into TMEM over its
+//                scores, where it is the A operand of P V; O / l and LSE at the end.  The next item's queries and first keys arrive meanwhile.
+// One persistent CTA per SM (TMEM 512 columns, 193 KB of shared memory).  Items go from the most to the fewest key blocks over all
+// sequences, heads varying fastest, and are dealt to the CTAs forwards and backwards in turn, so that their shares come out even.
+// The bound is the tensor pipe and, equally, 2^x on the special-function unit (see attention_window_tc.cu).
+// The earlier form (blocks of 64 keys, P through swizzled shared memory, a CTA per item) spent its time on the shared-memory round trip of
+// P and between CTAs: 28 heads over 4, 2 x 6005 tokens 648 -> 467 us (1.1 PFLOP/s).
 // Backward: attention_bwd_tc.cu.  Oracle: the mma.sync kernels in attention_varlen.cu.  Together they replace flash-attn-2
-// (attn_implementation="flash_attention_2", /root/reference/GRPO/grpo.py:219) on the training, log-prob and prefill paths.
-#include <cstdlib>
-
-#include "common.cuh"
+// (attn_implementation="flash_attention_2", GRPO/grpo.py:219) on the training, log-prob and prefill paths.
+#include "attention_tc.cuh"
 #include "kernels.h"
 
 namespace nrl {
 
-constexpr int kTcD = 128;                 // head dim
-constexpr int kTcBM = 256;                // query rows per CTA (two tiles of 128)
-constexpr int kTcBN = 64;                 // keys per block
-constexpr int kQPanel = 128 * 128;        // [128 rows][64 x bf16] swizzled panel (16 KB)
-constexpr int kQTile = 2 * kQPanel;       // one 128 x 128 Q tile (32 KB)
-constexpr int kKVPanel = 64 * 128;        // [64 keys][64 x bf16] (8 KB)
-constexpr int kKVTile = 2 * kKVPanel;     // [64 keys][128 dims] (16 KB)
-constexpr int kPTile = 128 * 128;         // [128 rows][64 keys] bf16 (16 KB)
-constexpr int kStages = 3;
-constexpr int kTcThreads = 320;
-
-// Cycle accounting / knock-out experiments (bench/attn_prof.py) are compiled in only with -DNRL_ATTN_PROFILE
-// (NRL_ATTN_PROFILE=1 python -m nanorlhf_b200.csrc.build); production builds carry neither clock reads nor tests.
-#ifdef NRL_ATTN_PROFILE
-#define NRL_TWAIT(slot, ...)                                              \
-  do {                                                                   \
-    const long long t_ = clock64();                                     \
-    mbar_wait(__VA_ARGS__);                                             \
-    tw[slot] += clock64() - t_;                                         \
-  } while (0)
-#define NRL_DBG(bit) (p.dbg & (bit))
-#else
-#define NRL_TWAIT(slot, ...) mbar_wait(__VA_ARGS__)
-#define NRL_DBG(bit) false
-#endif
+constexpr int kTcBM = 256;                 // query rows per item (two tiles of 128)
+constexpr int kTcSlots = 4;                // ring of K and V tiles
 
 struct AttnTcParams {
   const int* cu_seqlens;
@@ -55,85 +29,67 @@ struct AttnTcParams {
   long o_stride_t;
   int num_seqs, total_tokens, Hq, G;
   float scale_log2;
-  long long* prof;            // optional [grid][40] cycle counters (NRL_ATTN_PROFILE builds, bench/attn_prof.py)
-  int dbg;                    // timing experiments only (NRL_ATTN_DBG): 1 skip S MMAs, 2 skip PV MMAs, 4 skip exps, 8 skip K/V loads
 };
 
 struct AttnTcSmem {
   static constexpr int kQ = 0;                                   // 2 tiles
-  static constexpr int kK = 2 * kQTile;                          // kStages
-  static constexpr int kV = kK + kStages * kKVTile;              // kStages
-  static constexpr int kP = kV + kStages * kKVTile;              // [tile][buf]
-  static constexpr int kBar = kP + 4 * kPTile;
-  static constexpr int kTotal = kBar + 256;
+  static constexpr int kRing = 2 * kAtTile;                      // kTcSlots tiles
+  static constexpr int kBar = kRing + kTcSlots * kAtTile;        // mbarriers, TMEM pointer
+  static constexpr int kTab = kBar + 256;                        // two items: head (-1: none left), q0, first token, length
+  static constexpr int kTotal = kTab + 2 * 16;
 };
 
-__device__ bool tc_locate_block(const int* cu, int num_seqs, int blk, int& m_blk, int& seq_start, int& seq_len) {
-  __shared__ int s_info[4];
-  if (threadIdx.x == 0) {
-    int acc = 0, found = 0;
-    for (int s = 0; s < num_seqs; ++s) {
-      const int a = cu[s], b = cu[s + 1];
-      const int nb = (b - a + kTcBM - 1) / kTcBM;
-      if (blk < acc + nb) {
-        s_info[0] = 1; s_info[1] = blk - acc; s_info[2] = a; s_info[3] = b - a;
-        found = 1;
-        break;
-      }
-      acc += nb;
-    }
-    if (!found) s_info[0] = 0;
+struct AttnItem {
+  int head, q0, start, len;
+  NRL_DEVICE int blocks(int x) const {     // key blocks that tile x walks; tile B may lie entirely behind the end of the sequence
+    return q0 + x * 128 < len ? q0 / 128 + 1 + x : 0;
   }
-  __syncthreads();
-  if (!s_info[0]) return false;
-  m_blk = s_info[1]; seq_start = s_info[2]; seq_len = s_info[3];
-  return true;
+};
+NRL_DEVICE AttnItem attn_item(const uint8_t* smem, uint64_t* tab_full, uint32_t k) {
+  mbar_wait(&tab_full[k & 1], (k >> 1) & 1);
+  const volatile int* t = reinterpret_cast<const volatile int*>(smem + AttnTcSmem::kTab + (k & 1) * 16);
+  return {t[0], t[1], t[2], t[3]};
 }
 
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kAtThreads, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                   const __grid_constant__ CUtensorMap tmV, AttnTcParams p) {
+                   const __grid_constant__ CUtensorMap tmV, const AttnTcParams p) {
   using L = AttnTcSmem;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + L::kBar);
-  uint64_t* kv_full = q_full + 1;              // [kStages]
-  uint64_t* kv_empty = kv_full + kStages;      // [kStages]
-  uint64_t* s_full = kv_empty + kStages;       // [tile][2]
-  uint64_t* p_ready = s_full + 4;              // [tile][2]
-  uint64_t* pv_done = p_ready + 4;             // [tile][2]  PV_X of a block with parity b retired: P_X[b] reusable, O_X current
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(pv_done + 4);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::kBar);      // [kTcSlots]
+  uint64_t* empty = full + kTcSlots;           // [kTcSlots]
+  uint64_t* q_full = empty + kTcSlots;         // [tile]
+  uint64_t* q_empty = q_full + 2;              // [tile]
+  uint64_t* s_full = q_empty + 2;              // [tile]
+  uint64_t* p_ready = s_full + 2;              // [tile]
+  uint64_t* o_done = p_ready + 2;              // [tile]
+  uint64_t* tab_full = o_done + 2;             // [2]
+  uint64_t* tab_empty = tab_full + 2;          // [2]
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tab_empty + 2);
 
-  int m_blk, seq_start, seq_len;
-  // heaviest (latest) query blocks are launched first: longest-processing-time order trims the causal tail
-  if (!tc_locate_block(p.cu_seqlens, p.num_seqs, gridDim.x - 1 - blockIdx.x, m_blk, seq_start, seq_len)) return;
-  const int head = blockIdx.y, kvh = head / p.G;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = m_blk * kTcBM;
-  const int kv_blocks = (seq_len + kTcBN - 1) / kTcBN;
-  // number of KV blocks each tile visits (causal); tile B may lie entirely behind the end of the sequence
-  const int nA = min(kv_blocks, (q0 + 128 + kTcBN - 1) / kTcBN);
-  const int nB = (q0 + 128 < seq_len) ? min(kv_blocks, (q0 + 256 + kTcBN - 1) / kTcBN) : 0;
-  const int n_blocks = max(nA, nB);
-
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
   }
-  if (warp == 1 && lane == 0) {
-    mbar_init(q_full, 1);
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
-    }
-    for (int i = 0; i < 4; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_ready[i], 4);        // one arrive per softmax warp of the tile
-      mbar_init(&pv_done[i], 1);
-    }
-    fence_mbar_init();
-  }
   if (warp == 1) {
+    if (lane == 0) {
+      for (int i = 0; i < kTcSlots; ++i) {
+        mbar_init(&full[i], 1);
+        mbar_init(&empty[i], 1);
+      }
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&q_full[i], 1);
+        mbar_init(&q_empty[i], 1);
+        mbar_init(&s_full[i], 1);
+        mbar_init(&p_ready[i], 4);             // one arrive per softmax warp of the tile
+        mbar_init(&o_done[i], 1);
+        mbar_init(&tab_full[i], 1);
+        mbar_init(&tab_empty[i], 10);          // producer, MMA issuer, eight softmax warps
+      }
+      fence_mbar_init();
+    }
     __syncwarp();
     tmem_alloc(tmem_ptr, 512);
   }
@@ -141,223 +97,189 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
-#ifdef NRL_ATTN_PROFILE
-  long long tw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const long long t_begin = clock64();
-#endif
 
-  if (warp == 0) {
-    // ============================== TMA producer ==============================
-    if (elect_one()) {
-      mbar_arrive_expect_tx(q_full, 2 * kQTile);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        tma_load_2d(smem + L::kQ + t * kQTile, &tmQ, q_full, head * kTcD, seq_start + q0 + t * 128);
-        tma_load_2d(smem + L::kQ + t * kQTile + kQPanel, &tmQ, q_full, head * kTcD + 64, seq_start + q0 + t * 128);
-      }
-      int st = 0;
-      uint32_t phase = 0;
-      for (int j = 0; j < n_blocks; ++j) {
-        NRL_TWAIT(0, &kv_empty[st], phase ^ 1);
-        uint8_t* sk = smem + L::kK + st * kKVTile;
-        uint8_t* sv = smem + L::kV + st * kKVTile;
-        if (NRL_DBG(8)) {
-          mbar_arrive(&kv_full[st]);
-          if (++st == kStages) { st = 0; phase ^= 1; }
-          continue;
-        }
-        mbar_arrive_expect_tx(&kv_full[st], 2 * kKVTile);
-        const int row = seq_start + j * kTcBN;
-        tma_load_2d(sk, &tmK, &kv_full[st], kvh * kTcD, row);
-        tma_load_2d(sk + kKVPanel, &tmK, &kv_full[st], kvh * kTcD + 64, row);
-        tma_load_2d(sv, &tmV, &kv_full[st], kvh * kTcD, row);
-        tma_load_2d(sv + kKVPanel, &tmV, &kv_full[st], kvh * kTcD + 64, row);
-        if (++st == kStages) { st = 0; phase ^= 1; }
-      }
-    }
-  } else if (warp == 1) {
-    // ============================== MMA issuer ==============================
-    // elect.sync (not `lane == 0`) lets the compiler prove single-thread execution; otherwise every tcgen05.mma is
-    // wrapped in an ELECT/branch loop whose latency exceeds these short (32-64 cycle) MMAs
-    if (elect_one()) {
-      constexpr uint32_t idesc_s = make_idesc(128, kTcBN, 1, 1);        // Q K^T : both K-major
-      constexpr uint32_t idesc_o = make_idesc_bmn(128, kTcD);          // P V   : B = V is MN-major
-      NRL_TWAIT(1, q_full, 0);
-      tc_fence_after();
-      int st_s = 0;                       // ring stage of the block whose S is issued next
-      uint32_t ph_s = 0;
-      auto issue_s = [&](int j) {
-        NRL_TWAIT(2, &kv_full[st_s], ph_s);
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(smem + L::kK + st_s * kKVTile);
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (j < (t == 0 ? nA : nB)) {
-            const uint32_t q_addr = smem_u32(smem + L::kQ + t * kQTile);
-            const uint32_t t_s = tmem_base + t * 128 + (j & 1) * kTcBN;
-#pragma unroll
-            for (int k = 0; k < 8; ++k)        // 8 x 16 dims; dims 0-63 in panel 0, 64-127 in panel 1
-              if (!NRL_DBG(1)) umma_f16(t_s, make_smem_desc_sw128(q_addr + (k >> 2) * kQPanel + (k & 3) * 32),
-                       make_smem_desc_sw128(k_addr + (k >> 2) * kKVPanel + (k & 3) * 32), idesc_s, k != 0 ? 1u : 0u);
-            umma_commit(&s_full[t * 2 + (j & 1)]);
+  if (warp < 4) {
+    attn_regs_issue();
+    if (warp == 0) {
+      // ============================== TMA producer ==============================
+      if (elect_one()) {
+        int slot = 0;
+        uint32_t phase = 0, n_q[2] = {0, 0};
+        auto load = [&](const CUtensorMap* tm, int col, int row) {
+          mbar_wait(&empty[slot], phase ^ 1);
+          uint8_t* dst = smem + L::kRing + slot * kAtTile;
+          mbar_arrive_expect_tx(&full[slot], kAtTile);
+          tma_load_2d(dst, tm, &full[slot], col, row);
+          tma_load_2d(dst + kAtPanel, tm, &full[slot], col + 64, row);
+          if (++slot == kTcSlots) { slot = 0; phase ^= 1; }
+        };
+        for (uint32_t k = 0;; ++k) {
+          const AttnItem it = attn_item(smem, tab_full, k);
+          mbar_arrive(&tab_empty[k & 1]);
+          if (it.head < 0) break;
+          const int kvc = it.head / p.G * kAtD, n = max(it.blocks(0), it.blocks(1));
+          for (int x = 0; x < 2; ++x) {
+            if (it.blocks(x) == 0) continue;
+            mbar_wait(&q_empty[x], (n_q[x] & 1) ^ 1);
+            ++n_q[x];
+            uint8_t* dst = smem + L::kQ + x * kAtTile;
+            mbar_arrive_expect_tx(&q_full[x], kAtTile);
+            tma_load_2d(dst, &tmQ, &q_full[x], it.head * kAtD, it.start + it.q0 + x * 128);
+            tma_load_2d(dst + kAtPanel, &tmQ, &q_full[x], it.head * kAtD + 64, it.start + it.q0 + x * 128);
+          }
+          for (int j = 0; j < n; ++j) {
+            load(&tmK, kvc, it.start + j * kAtBN);
+            load(&tmV, kvc, it.start + j * kAtBN);
           }
         }
-        if (++st_s == kStages) { st_s = 0; ph_s ^= 1; }
-      };
-      issue_s(0);
-      int st = 0;
-      for (int j = 0; j < n_blocks; ++j) {
-        if (j + 1 < n_blocks) issue_s(j + 1);               // overlaps the softmax of block j
-        const uint32_t v_addr = smem_u32(smem + L::kV + st * kKVTile);
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (j < (t == 0 ? nA : nB)) {
-            NRL_TWAIT(3, &p_ready[t * 2 + (j & 1)], (j >> 1) & 1);         // P_X,j in smem, O_X rescaled
-            tc_fence_after();
-            const uint32_t p_addr = smem_u32(smem + L::kP + (t * 2 + (j & 1)) * kPTile);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)        // 4 x 16 keys
-              if (!NRL_DBG(2)) umma_f16(tmem_base + 256 + t * 128, make_smem_desc_sw128(p_addr + k * 32),
-                       make_smem_desc_sw128_mn(v_addr + k * 16 * 128, kKVPanel), idesc_o, (j | k) != 0 ? 1u : 0u);
-            umma_commit(&pv_done[t * 2 + (j & 1)]);
-          }
-        }
-        umma_commit(&kv_empty[st]);            // K_j / V_j smem reusable
-        if (++st == kStages) st = 0;
       }
-    }
-    __syncwarp();
-  } else {
-    // ============================== softmax / correction / epilogue ==============================
-    const int tile = (warp - 2) >> 2;                         // 0 = A, 1 = B
-    const int n_mine = tile == 0 ? nA : nB;
-    const int quad = warp & 3;
-    const int r = quad * 32 + lane;                          // row in tile == TMEM lane
-    const int row0 = q0 + tile * 128;                        // first row of the tile (within the sequence)
-    const int row = row0 + r;
-    const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t t_o = tmem_base + 256 + tile * 128 + lane_off;
-    float m_run = -INFINITY, l_run = 0.f;
-    for (int j = 0; j < n_mine; ++j) {
-      const int b = j & 1;
-      NRL_TWAIT(4, &s_full[tile * 2 + b], (j >> 1) & 1);
-      tc_fence_after();
-      const uint32_t t_s = tmem_base + tile * 128 + b * kTcBN + lane_off;
-      uint32_t sv[2][32];
-      tmem_ld_32x32b_x32(t_s, sv[0]);
-      tmem_ld_32x32b_x32(t_s + 32, sv[1]);
-      tmem_ld_wait();
-      const int key0 = j * kTcBN;
-      // only blocks on the diagonal of this tile and a ragged last block need masking (warpgroup-uniform test)
-      if (key0 + kTcBN - 1 > row0 || key0 + kTcBN > seq_len) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key = key0 + c * 32 + i;
-            if (key >= seq_len || key > row) sv[c][i] = 0xff800000u;      // -inf
-          }
-      }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};         // 4 independent chains
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[c][i]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
-      // lazy rescale: keep the stale maximum while the new one is < 2^8 above it (p <= 256 is harmless in bf16 and
-      // l / O stay consistent with m_run); key 0 is live for every row so m_new is finite from block 0 on
-      const float m_new = (mx - m_run > 8.f) ? mx : m_run;
-      const float corr = exp2f(m_run - m_new);
-      float ps4[4] = {0.f, 0.f, 0.f, 0.f};
-      if (!NRL_DBG(4))
-      // exponentials (in place: sv[c][i/2] <- bf16x2(p_i, p_i+1)); the wait below overlaps them
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[c][i]), p.scale_log2, -m_new));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[c][i + 1]), p.scale_log2, -m_new));
-          ps4[(i >> 1) & 3] += p0 + p1;
-          sv[c][i / 2] = pack_bf16x2(p0, p1);
-        }
-      const float ps = (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
-      // P_X[b] was last read by PV_X(j-2).  pv_done[X][b] completes once per two blocks and cannot run ahead of this
-      // thread (its next completion needs our p_ready), so the parity wait is unambiguous.
-      if (j >= 2) {
-        NRL_TWAIT(5, &pv_done[tile * 2 + b], ((j >> 1) - 1) & 1);
-        tc_fence_after();
-      }
-      uint8_t* rowp = smem + L::kP + (tile * 2 + b) * kPTile + r * 128;
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const int ch = c * 4 + q4;           // 16-byte chunk of the 128-byte (64-key) row
-          *reinterpret_cast<uint4*>(rowp + ((ch ^ (r & 7)) << 4)) =
-              make_uint4(sv[c][q4 * 4], sv[c][q4 * 4 + 1], sv[c][q4 * 4 + 2], sv[c][q4 * 4 + 3]);
-        }
-      l_run = l_run * corr + ps;
-      // ---- rescale O in TMEM when this row's maximum moved (rare with the lazy threshold; skipped warp-wide) ----
-      // only then does this block depend on PV_X(j-1) having retired: the softmax never waits for the tensor pipe
-      // on the common path
-      const bool need = (j > 0) && (corr != 1.f);
-      if (__any_sync(0xffffffffu, need)) {
-        NRL_TWAIT(6, &pv_done[tile * 2 + (b ^ 1)], ((j - 1) >> 1) & 1);
-        tc_fence_after();
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t ov[32];
-          tmem_ld_32x32b_x32(t_o + c * 32, ov);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
-          tmem_st_32x32b_x32(t_o + c * 32, ov);
-        }
-        tmem_st_wait();
-      }
-      m_run = m_new;
-      fence_proxy_async_smem();              // P writes visible to the tensor-core (async) proxy
-      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_ready[tile * 2 + b]);
+    } else if (warp == 1) {
+      // ============================== MMA issuer ==============================
+      // elect.sync (not `lane == 0`) lets the compiler prove single-thread execution; otherwise every tcgen05.mma is wrapped in an
+      // ELECT/branch loop whose latency exceeds these short MMAs
+      if (elect_one()) {
+        int slot = 0;                            // ring slot of the next tile in load order
+        uint32_t phase = 0, n_p[2] = {0, 0}, n_q[2] = {0, 0};
+        auto ring_next = [&]() {
+          if (++slot == kTcSlots) { slot = 0; phase ^= 1; }
+        };
+        const uint32_t q_addr = smem_u32(smem + L::kQ), ring = smem_u32(smem + L::kRing);
+        for (uint32_t k = 0;; ++k) {
+          const AttnItem it = attn_item(smem, tab_full, k);
+          mbar_arrive(&tab_empty[k & 1]);
+          if (it.head < 0) break;
+          const int nx[2] = {it.blocks(0), it.blocks(1)}, n = max(nx[0], nx[1]);
+          auto issue_s = [&](int x, int j, int s) {
+            attn_issue_s(tmem_base + x * kAtBN, q_addr + x * kAtTile, ring + s * kAtTile);
+            umma_commit(&s_full[x]);
+            if (j == nx[x] - 1) umma_commit(&q_empty[x]);
+          };
+          mbar_wait(&full[slot], phase);
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            if (nx[x] > 0) {
+              mbar_wait(&q_full[x], n_q[x] & 1);
+              ++n_q[x];
+              tc_fence_after();
+              issue_s(x, 0, slot);
+            }
+          umma_commit(&empty[slot]);
+          ring_next();
+          for (int j = 0; j < n; ++j) {
+            const int v_slot = slot;             // load order is K_0, V_0, K_1 ...: the next K sits behind this V
+            mbar_wait(&full[v_slot], phase);
+            ring_next();
+            const int k_slot = slot;
+            if (j + 1 < n) {
+              mbar_wait(&full[k_slot], phase);
+              ring_next();
+            }
+            // keys behind the end of the sequence belong to another one: their P is 0, their V stays out
+            const int steps = min(8, (it.len - j * kAtBN + 15) / 16);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              if (j < nx[x]) {
+                mbar_wait(&p_ready[x], n_p[x] & 1);
+                ++n_p[x];
+                tc_fence_after();
+                attn_issue_pv(tmem_base + kAtTmemO + x * kAtD, tmem_base + x * kAtBN, ring + v_slot * kAtTile, j == 0, steps);
+                if (j == nx[x] - 1) umma_commit(&o_done[x]);
+              }
+              if (j + 1 < nx[x]) issue_s(x, j + 1, k_slot);
+            }
+            umma_commit(&empty[v_slot]);
+            if (j + 1 < n) umma_commit(&empty[k_slot]);
+          }
+        }
+      }
+      __syncwarp();
+    } else if (warp == 2) {
+      // ============================== items ==============================
+      const int* cu = p.cu_seqlens;
+      int level = 0;
+      for (int s = lane; s < p.num_seqs; s += 32) level = max(level, (cu[s + 1] - cu[s] + kTcBM - 1) / kTcBM);
+      level = __reduce_max_sync(0xffffffffu, level);                 // blocks of the longest sequence
+      int above = 0, upto = 0;                                       // row blocks with an index > level, >= level
+      for (uint32_t k = 0;; ++k) {
+        const int at = (k & 1) ? (k + 1) * gridDim.x - 1 - blockIdx.x : k * gridDim.x + blockIdx.x;
+        const int rank = at / p.Hq;
+        while (level > 0 && rank >= upto) {
+          --level;
+          above = upto;
+          upto = attn_blocks_from<kTcBM>(cu, p.num_seqs, level, lane);
+        }
+        int4 it = make_int4(-1, 0, 0, 0);
+        if (rank < upto) {
+          const int src = attn_nth_sequence<kTcBM>(cu, p.num_seqs, level, rank - above, lane);
+          it = make_int4(at - rank * p.Hq, level * kTcBM, cu[src], cu[src + 1] - cu[src]);
+        }
+        mbar_wait(&tab_empty[k & 1], ((k >> 1) & 1) ^ 1);
+        if (lane == 0) {
+          *reinterpret_cast<int4*>(smem + L::kTab + (k & 1) * 16) = it;
+          mbar_arrive(&tab_full[k & 1]);
+        }
+        __syncwarp();
+        if (it.x < 0) break;
+      }
     }
-    // ---- epilogue: O / l -> bf16, LSE ----
-    if (n_mine > 0) {
-      NRL_TWAIT(7, &pv_done[tile * 2 + ((n_mine - 1) & 1)], ((n_mine - 1) >> 1) & 1);
+  } else {
+    // ============================== softmax, epilogue ==============================
+    attn_regs_softmax();
+    const int x = (warp - 4) >> 2, quad = warp & 3;
+    const int r = quad * 32 + lane;                            // row of the tile == TMEM lane
+    const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t t_s = tmem_base + x * kAtBN + lane_off, t_o = tmem_base + kAtTmemO + x * kAtD + lane_off;
+    uint32_t n_s = 0, n_o = 0;
+    for (uint32_t k = 0;; ++k) {
+      const AttnItem it = attn_item(smem, tab_full, k);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tab_empty[k & 1]);
+      if (it.head < 0) break;
+      const int n = it.blocks(x), row0 = it.q0 + x * 128, row = row0 + r;
+      if (n == 0) continue;
+      float m_run = -INFINITY, l_run = 0.f;
+      for (int j = 0; j < n; ++j) {
+        mbar_wait(&s_full[x], n_s & 1);
+        ++n_s;
+        tc_fence_after();
+        uint32_t sv[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(t_s + c * 32, sv[c]);
+        tmem_ld_wait();
+        const int key0 = j * kAtBN;
+        // only the block on the diagonal needs a mask: the others end before the tile's first row
+        if (j == n - 1) attn_mask_block(sv, 0, min(row, it.len - 1) - key0, 0);
+        attn_softmax_block(sv, p.scale_log2, t_s, t_o, j == 0, m_run, l_run);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[x]);
+      }
+      // ---- O / l -> bf16, LSE ----
+      mbar_wait(&o_done[x], n_o & 1);
+      ++n_o;
       tc_fence_after();
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      const bool row_ok = row < seq_len;
-      __nv_bfloat16* orow = p.out + static_cast<long>(seq_start + row) * p.o_stride_t + head * kTcD;
+      const float inv = 1.f / l_run;                           // every row sees its own key; 0 or NaN only from non-finite scores
+      const bool row_ok = row < it.len;
+      const long t = it.start + row;
+      __nv_bfloat16* orow = p.out + t * p.o_stride_t + it.head * kAtD;
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         uint32_t ov[32];
         tmem_ld_32x32b_x32(t_o + c * 32, ov);
         tmem_ld_wait();
-        if (row_ok) {
+        if (!row_ok) continue;
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            uint4 o4;
-            o4.x = pack_bf16x2(__uint_as_float(ov[q4 * 8]) * inv, __uint_as_float(ov[q4 * 8 + 1]) * inv);
-            o4.y = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 2]) * inv, __uint_as_float(ov[q4 * 8 + 3]) * inv);
-            o4.z = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 4]) * inv, __uint_as_float(ov[q4 * 8 + 5]) * inv);
-            o4.w = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 6]) * inv, __uint_as_float(ov[q4 * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + c * 32 + q4 * 8) = o4;
-          }
-        }
+        for (int i = 0; i < 16; ++i) ov[i] = pack_bf16x2(__uint_as_float(ov[2 * i]) * inv, __uint_as_float(ov[2 * i + 1]) * inv);
+        stg_v8(orow + c * 32, ov);
+        stg_v8(orow + c * 32 + 16, ov + 8);
       }
       if (row_ok && p.lse != nullptr)
-        p.lse[static_cast<long>(head) * p.total_tokens + seq_start + row] = (m_run + log2f(l_run)) * 0.6931471805599453f;
+        p.lse[static_cast<long>(it.head) * p.total_tokens + t] = (m_run + log2f(l_run)) * 0.6931471805599453f;
+      tc_fence_before();                                       // the next item's first P V follows this thread's next p_ready
+      __syncwarp();
     }
   }
-
-#ifdef NRL_ATTN_PROFILE
-  if (p.prof != nullptr && lane == 0 && (warp == 0 || warp == 1 || warp == 2 || warp == 6)) {
-    long long* dst = p.prof + (static_cast<long>(blockIdx.y) * gridDim.x + blockIdx.x) * 40 + (warp == 0 ? 0 : warp == 1 ? 10 : warp == 2 ? 20 : 30);
-    for (int i = 0; i < 8; ++i) dst[i] = tw[i];
-    dst[8] = clock64() - t_begin;
-    dst[9] = n_blocks;
-  }
-#endif
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -370,23 +292,20 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
 extern "C" cudaError_t nrl_attn_fwd_tc(const CUtensorMap* tmQ, const CUtensorMap* tmK, const CUtensorMap* tmV, void* out,
                                        float* lse, long o_stride_t, const int* cu, int num_seqs, int total, int Hq, int Hkv,
-                                       float scale, cudaStream_t s, long long* prof) {
+                                       float scale, int num_sms, cudaStream_t s) {
   using namespace nrl;
   if (total == 0) return cudaSuccess;
   AttnTcParams p;
   p.cu_seqlens = cu; p.out = static_cast<__nv_bfloat16*>(out); p.lse = lse; p.o_stride_t = o_stride_t;
   p.num_seqs = num_seqs; p.total_tokens = total; p.Hq = Hq; p.G = Hq / Hkv;
   p.scale_log2 = scale * 1.4426950408889634f;
-  static const int dbg = getenv("NRL_ATTN_DBG") ? atoi(getenv("NRL_ATTN_DBG")) : 0;
-  p.dbg = dbg;
-  p.prof = prof;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnTcSmem::kTotal);
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  dim3 grid(total / kTcBM + num_seqs, Hq);
-  attn_fwd_tc_kernel<<<grid, kTcThreads, AttnTcSmem::kTotal, s>>>(*tmQ, *tmK, *tmV, p);
+  const long most = static_cast<long>(total / kTcBM + num_seqs) * Hq;
+  attn_fwd_tc_kernel<<<static_cast<int>(most < num_sms ? most : num_sms), kAtThreads, AttnTcSmem::kTotal, s>>>(*tmQ, *tmK, *tmV, p);
   return cudaGetLastError();
 }

@@ -37,6 +37,47 @@ NRL_DEVICE uint64_t add_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 
+NRL_DEVICE uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Packed sequences cut into blocks of BM rows, put in order by the number of blocks in front of (or behind) them: how many blocks have
+// `level` or more of them, and the n-th sequence that has more than `level` blocks (both by a whole warp).
+template <int BM>
+NRL_DEVICE int attn_blocks_from(const int* cu, int num_seqs, int level, int lane) {
+  int n = 0;
+  for (int s = lane; s < num_seqs; s += 32) n += max(0, (cu[s + 1] - cu[s] + BM - 1) / BM - level);
+  return __reduce_add_sync(0xffffffffu, n);
+}
+template <int BM>
+NRL_DEVICE int attn_nth_sequence(const int* cu, int num_seqs, int level, int n, int lane) {
+  for (int s0 = 0; s0 < num_seqs; s0 += 32) {
+    const int s = s0 + lane;
+    const bool has = s < num_seqs && (cu[s + 1] - cu[s] + BM - 1) / BM > level;
+    const uint32_t m = __ballot_sync(0xffffffffu, has);
+    if (n < __popc(m)) return s0 + __fns(m, 0, n + 1);
+    n -= __popc(m);
+  }
+  return 0;                                    // not reached for n below their number
+}
+
+NRL_DEVICE void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+NRL_DEVICE void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
 // 32-byte global accesses (one full sector per lane); addresses are multiples of 32
 NRL_DEVICE void ldg_v8(const float* a, float (&f)[8]) {
   asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -66,12 +107,12 @@ NRL_DEVICE void attn_issue_s(uint32_t t_s, uint32_t q_addr, uint32_t k_addr) {
     umma_f16(t_s, make_smem_desc_sw128(q_addr + (k >> 2) * kAtPanel + (k & 3) * 32),
              make_smem_desc_sw128(k_addr + (k >> 2) * kAtPanel + (k & 3) * 32), idesc, k != 0 ? 1u : 0u);
 }
-// O_X (+)= P_X V: P from TMEM, V in place as an MN-major operand
-NRL_DEVICE void attn_issue_pv(uint32_t t_o, uint32_t t_p, uint32_t v_addr, bool first) {
+// O_X (+)= P_X V: P from TMEM, V in place as an MN-major operand; the first `steps` groups of 16 keys
+NRL_DEVICE void attn_issue_pv(uint32_t t_o, uint32_t t_p, uint32_t v_addr, bool first, int steps = 8) {
   constexpr uint32_t idesc = make_idesc_bmn(128, kAtD);
 #pragma unroll
   for (int k = 0; k < 8; ++k)
-    umma_f16_ts(t_o, t_p + k * 8, make_smem_desc_sw128_mn(v_addr + k * 16 * 128, kAtPanel), idesc, (first && k == 0) ? 0u : 1u);
+    if (k < steps) umma_f16_ts(t_o, t_p + k * 8, make_smem_desc_sw128_mn(v_addr + k * 16 * 128, kAtPanel), idesc, (first && k == 0) ? 0u : 1u);
 }
 
 // scores outside columns [lo, hi] of this block and not below `keep` become -inf (a bit per column)

@@ -28,8 +28,6 @@ CPP_SOURCES = ["bindings.cpp", "runtime.cpp", "bindings_hybrid.cpp"]
 PRECISE_SOURCES = {"stream_ops.cu", "recurrent.cu", "attention_window.cu", "attention_window_mma.cu", "attention_window_tc.cu", "attention_latent_mma.cu", "moe.cu", "lightning.cu"}
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
-if os.environ.get("NRL_ATTN_PROFILE") == "1":       # cycle accounting build of attention_fwd_tc.cu (bench/attn_prof.py)
-    NVCC_FLAGS.append("-DNRL_ATTN_PROFILE")
 
 
 def _stamp(path: str, extra: str) -> str:

@@ -73,7 +73,7 @@ cudaError_t nrl_attn_varlen_bwd(const void* dout, const void* q, const void* k, 
 // tcgen05 forward (attention_fwd_tc.cu): causal, head_dim 128, q/k/v addressed through TMA maps over [T, H*D]
 cudaError_t nrl_attn_fwd_tc(const CUtensorMap* tmQ, const CUtensorMap* tmK, const CUtensorMap* tmV, void* out, float* lse,
                             long o_stride_t, const int* cu, int num_seqs, int total, int Hq, int Hkv, float scale,
-                            cudaStream_t s, long long* prof = nullptr);
+                            int num_sms, cudaStream_t s);
 // TMA-fed DeBERTa disentangled attention (attention_varlen.cu); maps = {Q, K, V, relA, relB}
 cudaError_t nrl_deberta_attn_fwd(const CUtensorMap* maps, void* out, float* lse, long os, const int* cu, int num_seqs,
                                  int total, int Hq, float scale, const short* lut, int lut_center, int NB, int bn, cudaStream_t s);
