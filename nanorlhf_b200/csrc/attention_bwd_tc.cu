@@ -4,28 +4,34 @@
 //   delta   : delta[h, t] = sum_d dO * O                                   (one warp per (token, head))
 //   dK / dV : one CTA per (128-key block, kv head).  K_j, V_j stay in smem; the CTA streams (q head of the group,
 //             64-row query block) pairs:   S^T = K_j Q_i^T,  dP^T = V_j dO_i^T          (tcgen05, TMEM lanes = keys)
-//             P^T = exp2(S^T*c - lse_i),  dS^T = P^T o (dP^T - delta_i) * scale         (softmax warps, one key row each)
+//             P^T = exp2(S^T*c - lse_i),  dS^T = P^T o (dP^T - delta_i)                   (softmax warps, one key row each)
 //             dV_j += P^T dO_i,  dK_j += dS^T Q_i                                         (tcgen05, accumulators in TMEM)
 //   dQ      : one CTA per (128-row query block, q head).  Q_i, dO_i stay in smem; the CTA streams 64-key blocks:
-//             S = Q_i K_j^T,  dP = dO_i V_j^T  ->  dS = P o (dP - delta) * scale  ->  dQ_i += dS K_j
-// Shared structure: warp 0 = TMA producer (3-stage ring), warp 1 = single-thread MMA issuer, warps 2..5 and 6..9 = two
-// elementwise warpgroups that take alternate blocks (each owns one S/dP TMEM buffer and one P/dS smem buffer), so
-// the exp2/convert work of block n overlaps the MMAs of block n+1.  The operands that must be read "transposed"
-// (dO_i, Q_i for dV/dK; K_j for dQ) are consumed in place as MN-major UMMA operands - nothing is transposed in smem.
+//             S = Q_i K_j^T,  dP = dO_i V_j^T  ->  dS = P o (dP - delta)  ->  dQ_i += dS K_j
+// (the scale of the scores is applied to the float accumulators of dK and dQ at the end).
+// Shared structure: warp 0 = TMA producer (4-stage ring), warp 1 = single-thread MMA issuer, warps 2..17 = four
+// elementwise warpgroups: two that share the columns of a block take alternate blocks (each pair owns one S/dP TMEM buffer), so
+// the exp2/convert work of block n overlaps the MMAs of block n+1.  P and dS go back as bf16 into the TMEM columns of their S and dP and are the A
+// operand of the next MMA from there.  The operands that must be read "transposed" (dO_i, Q_i for dV/dK; K_j for dQ) are
+// consumed in place as MN-major UMMA operands - nothing is transposed in smem.
+// Blocks start from the most work to the least over all sequences: a key block in front of a long sequence is up to a whole
+// SM's share of the work, and one that starts late is waited for by the rest of the chip.
+// Before (P and dS through shared memory, one warpgroup per block, blocks in the order of their position) each block waited for one warp per
+// scheduler and the store's round trip, and the last key blocks of a launch ran alone: 28 heads over 4, 2 x 6005 tokens
+// dK / dV 1672 -> 915 us, dQ 1130 -> 728 us (1.1 PFLOP/s).
 // Replaces the flash-attn-2 backward the reference reaches through HF (attn_implementation="flash_attention_2",
-// /root/reference/GRPO/grpo.py:219; training step /root/reference/GRPO/grpo_trainer.py:652).
-#include "common.cuh"
+// GRPO/grpo.py:219; training step GRPO/grpo_trainer.py:652).
+#include "attention_tc.cuh"
 #include "kernels.h"
 
 namespace nrl {
 
-constexpr int kBwdThreads = 320;
+constexpr int kBwdThreads = 576;     // TMA, MMA, and four elementwise warpgroups: block parity x half of its columns
 constexpr int kP128 = 128 * 128;     // [128 rows][64 x bf16] swizzled panel (16 KB)
 constexpr int kT128 = 2 * kP128;     // 128 x 128 bf16 tile (32 KB)
 constexpr int kP64 = 64 * 128;       // [64 rows][64 x bf16] panel (8 KB)
 constexpr int kT64 = 2 * kP64;       // 64 x 128 bf16 tile (16 KB)
-constexpr int kPS = 128 * 128;       // [128 rows][64 x bf16] P / dS tile (16 KB)
-constexpr int kRing = 3;
+constexpr int kRing = 4;
 
 struct AttnBwdParams {
   const int* cu_seqlens;
@@ -37,36 +43,48 @@ struct AttnBwdParams {
   float scale, scale_log2;
 };
 
-// (sequence, block) lookup for packed sequences; result broadcast through `info` (dynamic smem, 4 ints)
-template <int BM>
-NRL_DEVICE bool bwd_locate(const int* cu, int num_seqs, int blk, int* info, int& m_blk, int& seq_start, int& seq_len) {
-  if (threadIdx.x == 0) {
-    int acc = 0, found = 0;
-    for (int s = 0; s < num_seqs; ++s) {
-      const int a = cu[s], b = cu[s + 1];
-      const int nb = (b - a + BM - 1) / BM;
-      if (blk < acc + nb) {
-        info[0] = 1; info[1] = blk - acc; info[2] = a; info[3] = b - a;
-        found = 1;
-        break;
-      }
-      acc += nb;
+// The `rank`-th block of 128 rows in the order of descending work: `level` counts the blocks of its sequence on the side where its work
+// lies (behind it for keys, in front of it for queries).  Result through `info` (4 ints of shared memory).
+NRL_DEVICE bool bwd_locate(const int* cu, int num_seqs, int rank, int* info, int& level, int& blocks, int& seq_start, int& seq_len) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int hi = 0, above = 0;                                     // blocks of the longest sequence; blocks with a level >= hi
+    for (int s = lane; s < num_seqs; s += 32) hi = max(hi, (cu[s + 1] - cu[s] + 127) / 128);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    int lo = 0;
+    bool found = rank < attn_blocks_from<128>(cu, num_seqs, 0, lane);
+    while (found && hi - lo > 1) {
+      const int mid = (lo + hi) >> 1, n = attn_blocks_from<128>(cu, num_seqs, mid, lane);
+      if (rank < n) { lo = mid; } else { hi = mid; above = n; }
     }
-    if (!found) info[0] = 0;
+    const int src = found ? attn_nth_sequence<128>(cu, num_seqs, lo, rank - above, lane) : 0;
+    if (lane == 0) { info[0] = found; info[1] = lo; info[2] = cu[src]; info[3] = cu[src + 1] - cu[src]; }
   }
   __syncthreads();
   if (!info[0]) return false;
-  m_blk = info[1]; seq_start = info[2]; seq_len = info[3];
+  level = info[1]; seq_start = info[2]; seq_len = info[3];
+  blocks = (seq_len + 127) / 128;
   return true;
 }
 
-// 32 fp32 values (as bit patterns) -> 16 packed bf16x2, written in place into the low half
-NRL_DEVICE void store_row_chunk(uint8_t* row_base, int r, int c32, const uint32_t (&pk)[16]) {
-  // columns c32*32 .. +31 of a 64-column (128-byte) row: 16-byte chunks c32*4 .. +3, 128B-swizzled by row
+// 16 columns of one row: P = 2^(S * c - lse), dS = P (dP - delta) as bf16 pairs.  nl(i), nd(i): -lse and -delta of columns i, i + 1;
+// MASK: columns without their bit in `see` are 0.
+template <bool MASK, bool WANT_P, class NL, class ND>
+NRL_DEVICE void bwd_chunk(const uint32_t (&sv)[16], const uint32_t (&dv)[16], uint64_t sc2, NL nl, ND nd, uint32_t see, uint32_t* pk,
+                          uint32_t* dk) {
 #pragma unroll
-  for (int q4 = 0; q4 < 4; ++q4) {
-    const int ch = c32 * 4 + q4;
-    *reinterpret_cast<uint4*>(row_base + ((ch ^ (r & 7)) << 4)) = make_uint4(pk[q4 * 4], pk[q4 * 4 + 1], pk[q4 * 4 + 2], pk[q4 * 4 + 3]);
+  for (int i = 0; i < 16; i += 2) {
+    float p0, p1, d0, d1;
+    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sc2, nl(i)), p0, p1);
+    p0 = ex2_approx(p0);
+    p1 = ex2_approx(p1);
+    if (MASK) {
+      if (!(see & (1u << i))) p0 = 0.f;
+      if (!(see & (2u << i))) p1 = 0.f;
+    }
+    unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), add_f32x2(pack_f32x2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), nd(i))), d0, d1);
+    if (WANT_P) pk[i / 2] = pack_bf16x2(p0, p1);
+    dk[i / 2] = pack_bf16x2(d0, d1);
   }
 }
 
@@ -93,10 +111,8 @@ struct DkdvSmem {
   static constexpr int kV = kT128;
   static constexpr int kQ = 2 * kT128;                     // ring
   static constexpr int kDO = kQ + kRing * kT64;            // ring
-  static constexpr int kP = kDO + kRing * kT64;            // [wg]
-  static constexpr int kDS = kP + 2 * kPS;                 // [wg]
-  static constexpr int kLD = kDS + 2 * kPS;                // [wg][parity][lse2 x 64 | delta x 64] floats
-  static constexpr int kBar = kLD + 2 * 2 * 128 * 4;
+  static constexpr int kLD = kDO + kRing * kT64;           // [wg][parity][-lse2 x 32 | -delta x 32] floats
+  static constexpr int kBar = kLD + 4 * 2 * 64 * 4;
   static constexpr int kTotal = kBar + 256;
 };
 
@@ -108,16 +124,16 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint64_t* kv_full = reinterpret_cast<uint64_t*>(smem + L::kBar);
   uint64_t* qdo_full = kv_full + 1;            // [kRing]
   uint64_t* qdo_empty = qdo_full + kRing;      // [kRing]
-  uint64_t* s_full = qdo_empty + kRing;        // [wg]  S^T and dP^T of the block are in TMEM
-  uint64_t* pds_ready = s_full + 2;            // [wg]  P^T / dS^T of the block are in smem
-  uint64_t* pds_free = pds_ready + 2;          // [wg]  the dV / dK MMAs that read them retired
-  uint64_t* done_bar = pds_free + 2;
+  uint64_t* s_full = qdo_empty + kRing;        // [parity]  S^T and dP^T of the block are in TMEM
+  uint64_t* pds_ready = s_full + 2;            // [parity]  P^T / dS^T of the block have replaced them
+  uint64_t* done_bar = pds_ready + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done_bar + 1);
   int* info = reinterpret_cast<int*>(tmem_ptr + 4);      // its own 16-byte slot: tcgen05.alloc writes next to it
 
-  int kb, seq_start, seq_len;
-  if (!bwd_locate<128>(p.cu_seqlens, p.num_seqs, blockIdx.x, info, kb, seq_start, seq_len)) return;
-  const int kvh = blockIdx.y;
+  int behind, blocks, seq_start, seq_len;
+  const int rank = blockIdx.x / (p.Hq / p.G), kvh = blockIdx.x - rank * (p.Hq / p.G);
+  if (!bwd_locate(p.cu_seqlens, p.num_seqs, rank, info, behind, blocks, seq_start, seq_len)) return;
+  const int kb = blocks - 1 - behind;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int key0 = kb * 128;
   const int i_begin = key0 / 64;                                   // first 64-row query block that sees these keys
@@ -130,7 +146,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   if (warp == 1 && lane == 0) {
     mbar_init(kv_full, 1);
     for (int i = 0; i < kRing; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&pds_ready[i], 4); mbar_init(&pds_free[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&pds_ready[i], 8); }
     mbar_init(done_bar, 1);
     fence_mbar_init();
   }
@@ -139,7 +155,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
-  // TMEM columns: S^T[wg] 0/64, dP^T[wg] 128/192, dV 256..383, dK 384..511
+  // TMEM columns: S^T[parity] 0/64, dP^T[parity] 128/192, dV 256..383, dK 384..511
 
   if (warp == 0) {
     // ============================== TMA producer ==============================
@@ -151,9 +167,9 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       tma_load_2d(smem + L::kV + kP128, &tmV, kv_full, kvh * 128 + 64, seq_start + key0);
       int st = 0;
       uint32_t phase = 0;
+      int head = kvh * p.G, qi = 0;
       for (int it = 0; it < n_iter; ++it) {
-        const int head = kvh * p.G + it / n_qb;
-        const int row = seq_start + (i_begin + it % n_qb) * 64;
+        const int row = seq_start + (i_begin + qi) * 64;
         mbar_wait(&qdo_empty[st], phase ^ 1);
         mbar_arrive_expect_tx(&qdo_full[st], 2 * kT64);
         uint8_t* sq = smem + L::kQ + st * kT64;
@@ -162,6 +178,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tma_load_2d(sq + kP64, &tmQ, &qdo_full[st], head * 128 + 64, row);
         tma_load_2d(sd, &tmDO, &qdo_full[st], head * 128, row);
         tma_load_2d(sd + kP64, &tmDO, &qdo_full[st], head * 128 + 64, row);
+        if (++qi == n_qb) { qi = 0; ++head; }
         if (++st == kRing) { st = 0; phase ^= 1; }
       }
     }
@@ -199,20 +216,17 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         if (it + 1 < n_iter) issue_sdp(it + 1);             // overlaps the elementwise work of block it
         mbar_wait(&pds_ready[b], (it >> 1) & 1);
         tc_fence_after();
-        const uint32_t p_addr = smem_u32(smem + L::kP + b * kPS);
-        const uint32_t ds_addr = smem_u32(smem + L::kDS + b * kPS);
         const uint32_t q_addr = smem_u32(smem + L::kQ + st * kT64);
         const uint32_t do_addr = smem_u32(smem + L::kDO + st * kT64);
 #pragma unroll
         for (int k = 0; k < 4; ++k)            // 4 x 16 query rows
-          umma_f16(tmem_base + 256, make_smem_desc_sw128(p_addr + k * 32),
-                   make_smem_desc_sw128_mn(do_addr + k * 16 * 128, kP64), idesc_g, (it | k) != 0 ? 1u : 0u);
+          umma_f16_ts(tmem_base + 256, tmem_base + b * 64 + (k >> 1) * 32 + (k & 1) * 8, make_smem_desc_sw128_mn(do_addr + k * 16 * 128, kP64), idesc_g,
+                      (it | k) != 0 ? 1u : 0u);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          umma_f16(tmem_base + 384, make_smem_desc_sw128(ds_addr + k * 32),
-                   make_smem_desc_sw128_mn(q_addr + k * 16 * 128, kP64), idesc_g, (it | k) != 0 ? 1u : 0u);
+          umma_f16_ts(tmem_base + 384, tmem_base + 128 + b * 64 + (k >> 1) * 32 + (k & 1) * 8, make_smem_desc_sw128_mn(q_addr + k * 16 * 128, kP64), idesc_g,
+                      (it | k) != 0 ? 1u : 0u);
         umma_commit(&qdo_empty[st]);
-        umma_commit(&pds_free[b]);
         if (++st == kRing) st = 0;
       }
       umma_commit(done_bar);
@@ -220,92 +234,72 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     __syncwarp();
   } else {
     // ============================== elementwise warpgroups ==============================
-    const int wg = (warp - 2) >> 2;
+    const int wg = (warp - 2) >> 2, par = wg & 1, half = wg >> 1;        // blocks of one parity, 32 of their 64 query columns
     const int quad = warp & 3;
     const int r = quad * 32 + lane;                          // key row in tile == TMEM lane
     const int t128 = (warp - 2 - wg * 4) * 32 + lane;        // 0..127 within the warpgroup
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
     const int kk = key0 + r;
-    float* ld_base = reinterpret_cast<float*>(smem + L::kLD) + wg * 256;
+    float* ld_base = reinterpret_cast<float*>(smem + L::kLD) + wg * 128;
+    int head = kvh * p.G, qi = par;                          // of the block that is fetched next
     auto load_ld = [&](int it) -> float {
-      // threads 0..63 fetch lse (in log2 units), 64..127 fetch delta, of query row (t128 & 63) of block `it`
-      if (it >= n_iter) return 0.f;
-      const int head = kvh * p.G + it / n_qb;
-      const int qq = (i_begin + it % n_qb) * 64 + (t128 & 63);
-      if (qq >= seq_len) return t128 < 64 ? INFINITY : 0.f;          // lse = +inf  =>  P = 0 for rows past the end
+      // threads 0..31 fetch -lse (in log2 units), 32..63 fetch -delta, of the columns' query rows of block `it`
+      if (it >= n_iter || t128 >= 64) return 0.f;
+      const int qq = (i_begin + qi) * 64 + half * 32 + (t128 & 31);
+      if (qq >= seq_len) return t128 < 32 ? -INFINITY : 0.f;         // lse = +inf  =>  P = 0 for rows past the end
       const long off = static_cast<long>(head) * p.total_tokens + seq_start + qq;
-      return t128 < 64 ? p.lse[off] * 1.4426950408889634f : p.delta[off];
+      return t128 < 32 ? p.lse[off] * -1.4426950408889634f : -p.delta[off];
     };
-    float ld_next = load_ld(wg);
-    for (int it = wg; it < n_iter; it += 2) {
+    const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    const uint32_t t_s = tmem_base + par * 64 + half * 32 + lane_off, t_dp = t_s + 128;
+    while (qi >= n_qb) { qi -= n_qb; ++head; }
+    float ld_next = load_ld(par);
+    for (int it = par; it < n_iter; it += 2) {
       const int n = it >> 1;
-      float* ldbuf = ld_base + (n & 1) * 128;
-      ldbuf[t128] = ld_next;
+      float* ldbuf = ld_base + (n & 1) * 64;
+      if (t128 < 64) ldbuf[t128] = ld_next;
+      const int q0 = (i_begin + qi) * 64 + half * 32;
       named_barrier_sync(1 + wg, 128);
+      for (qi += 2; qi >= n_qb; qi -= n_qb) ++head;
       ld_next = load_ld(it + 2);
-      const int q0 = (i_begin + it % n_qb) * 64;
-      const bool diag = q0 < key0 + 127;                     // some (key, query) pairs of the block are masked
-      mbar_wait(&s_full[wg], n & 1);
+      mbar_wait(&s_full[par], n & 1);
       tc_fence_after();
-      uint32_t pk[2][16], dk_[2][16];
+      uint32_t pk[16], dk[16];
+      const uint64_t* ld = reinterpret_cast<const uint64_t*>(ldbuf);
 #pragma unroll
-      for (int c32 = 0; c32 < 2; ++c32) {
-        uint32_t sv[32], dv_[32];
-        tmem_ld_32x32b_x32(tmem_base + wg * 64 + c32 * 32 + lane_off, sv);
-        tmem_ld_32x32b_x32(tmem_base + 128 + wg * 64 + c32 * 32 + lane_off, dv_);
+      for (int c = 0; c < 2; ++c) {
+        uint32_t sv[16], dv[16];
+        tmem_ld_32x32b_x16(t_s + c * 16, sv);
+        tmem_ld_32x32b_x16(t_dp + c * 16, dv);
         tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float2 l2 = *reinterpret_cast<const float2*>(ldbuf + c32 * 32 + i);
-          const float2 dl = *reinterpret_cast<const float2*>(ldbuf + 64 + c32 * 32 + i);
-          float p0 = exp2f(fmaf(__uint_as_float(sv[i]), p.scale_log2, -l2.x));
-          float p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), p.scale_log2, -l2.y));
-          if (diag) {
-            if (q0 + c32 * 32 + i < kk) p0 = 0.f;
-            if (q0 + c32 * 32 + i + 1 < kk) p1 = 0.f;
-          }
-          const float d0 = p0 * (__uint_as_float(dv_[i]) - dl.x) * p.scale;
-          const float d1 = p1 * (__uint_as_float(dv_[i + 1]) - dl.y) * p.scale;
-          pk[c32][i / 2] = pack_bf16x2(p0, p1);
-          dk_[c32][i / 2] = pack_bf16x2(d0, d1);
-        }
+        auto nl = [&](int i) { return ld[c * 8 + i / 2]; };
+        auto nd = [&](int i) { return ld[16 + c * 8 + i / 2]; };
+        if (q0 < key0 + 127) bwd_chunk<true, true>(sv, dv, sc2, nl, nd, mask_from(kk - q0 - c * 16), pk + c * 8, dk + c * 8);
+        else bwd_chunk<false, true>(sv, dv, sc2, nl, nd, 0u, pk + c * 8, dk + c * 8);
       }
-      // the dV / dK MMAs of this warpgroup's previous block (it-2) must be done with P^T / dS^T
-      if (it >= 2) {
-        mbar_wait(&pds_free[wg], (n - 1) & 1);
-        tc_fence_after();
-      }
-      uint8_t* prow = smem + L::kP + wg * kPS + r * 128;
-      uint8_t* drow = smem + L::kDS + wg * kPS + r * 128;
-      store_row_chunk(prow, r, 0, pk[0]);
-      store_row_chunk(prow, r, 1, pk[1]);
-      store_row_chunk(drow, r, 0, dk_[0]);
-      store_row_chunk(drow, r, 1, dk_[1]);
-      fence_proxy_async_smem();
+      tmem_st_32x32b_x16(t_s, pk);
+      tmem_st_32x32b_x16(t_dp, dk);
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&pds_ready[wg]);
+      if (lane == 0) mbar_arrive(&pds_ready[par]);
     }
-    // ---- epilogue: warpgroup 0 writes dV, warpgroup 1 writes dK ----
+    // ---- epilogue: parity 0 writes dV, parity 1 writes dK, each warpgroup 64 columns ----
     mbar_wait(done_bar, 0);
     tc_fence_after();
     const bool row_ok = kk < seq_len;
-    __nv_bfloat16* dst = (wg == 0 ? p.dv : p.dk) + static_cast<long>(seq_start + kk) * p.dkv_stride_t + kvh * 128;
+    const float f = par == 0 ? 1.f : p.scale;
+    __nv_bfloat16* dst = (par == 0 ? p.dv : p.dk) + static_cast<long>(seq_start + kk) * p.dkv_stride_t + kvh * 128 + half * 64;
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 2; ++c) {
       uint32_t ov[32];
-      tmem_ld_32x32b_x32(tmem_base + 256 + wg * 128 + c * 32 + lane_off, ov);     // warp-converged (.sync.aligned)
+      tmem_ld_32x32b_x32(tmem_base + 256 + par * 128 + half * 64 + c * 32 + lane_off, ov);     // warp-converged (.sync.aligned)
       tmem_ld_wait();
       if (row_ok) {
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          uint4 o4;
-          o4.x = pack_bf16x2(__uint_as_float(ov[q4 * 8]), __uint_as_float(ov[q4 * 8 + 1]));
-          o4.y = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 2]), __uint_as_float(ov[q4 * 8 + 3]));
-          o4.z = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 4]), __uint_as_float(ov[q4 * 8 + 5]));
-          o4.w = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 6]), __uint_as_float(ov[q4 * 8 + 7]));
-          *reinterpret_cast<uint4*>(dst + c * 32 + q4 * 8) = o4;
-        }
+        for (int i = 0; i < 16; ++i) ov[i] = pack_bf16x2(__uint_as_float(ov[2 * i]) * f, __uint_as_float(ov[2 * i + 1]) * f);
+        stg_v8(dst + c * 32, ov);
+        stg_v8(dst + c * 32 + 16, ov + 8);
       }
     }
   }
@@ -322,8 +316,7 @@ struct DqSmem {
   static constexpr int kDO = kT128;
   static constexpr int kK = 2 * kT128;                     // ring
   static constexpr int kV = kK + kRing * kT64;             // ring
-  static constexpr int kDS = kV + kRing * kT64;            // [wg]
-  static constexpr int kBar = kDS + 2 * kPS;
+  static constexpr int kBar = kV + kRing * kT64;
   static constexpr int kTotal = kBar + 256;
 };
 
@@ -337,15 +330,13 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint64_t* kv_empty = kv_full + kRing;        // [kRing]
   uint64_t* s_full = kv_empty + kRing;         // [wg]
   uint64_t* ds_ready = s_full + 2;             // [wg]
-  uint64_t* ds_free = ds_ready + 2;            // [wg]
-  uint64_t* done_bar = ds_free + 2;
+  uint64_t* done_bar = ds_ready + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done_bar + 1);
   int* info = reinterpret_cast<int*>(tmem_ptr + 4);      // its own 16-byte slot: tcgen05.alloc writes next to it
 
-  int mb, seq_start, seq_len;
-  // latest (longest) query blocks first
-  if (!bwd_locate<128>(p.cu_seqlens, p.num_seqs, gridDim.x - 1 - blockIdx.x, info, mb, seq_start, seq_len)) return;
-  const int head = blockIdx.y, kvh = head / p.G;
+  int mb, blocks, seq_start, seq_len;
+  const int rank = blockIdx.x / p.Hq, head = blockIdx.x - rank * p.Hq, kvh = head / p.G;
+  if (!bwd_locate(p.cu_seqlens, p.num_seqs, rank, info, mb, blocks, seq_start, seq_len)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q0 = mb * 128;
   const int n_kb = min((seq_len + 63) / 64, (q0 + 128 + 63) / 64);
@@ -356,7 +347,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (warp == 1 && lane == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < kRing; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&ds_ready[i], 4); mbar_init(&ds_free[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&ds_ready[i], 8); }
     mbar_init(done_bar, 1);
     fence_mbar_init();
   }
@@ -365,7 +356,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
-  // TMEM columns: S[wg] 0/64, dP[wg] 128/192, dQ 256..383
+  // TMEM columns: S[parity] 0/64, dP[parity] 128/192, dQ 256..383
 
   if (warp == 0) {
     if (elect_one()) {
@@ -422,21 +413,19 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (j + 1 < n_kb) issue_sdp(j + 1);
         mbar_wait(&ds_ready[b], (j >> 1) & 1);
         tc_fence_after();
-        const uint32_t ds_addr = smem_u32(smem + L::kDS + b * kPS);
         const uint32_t k_addr = smem_u32(smem + L::kK + st * kT64);
 #pragma unroll
         for (int k = 0; k < 4; ++k)            // 4 x 16 keys
-          umma_f16(tmem_base + 256, make_smem_desc_sw128(ds_addr + k * 32),
-                   make_smem_desc_sw128_mn(k_addr + k * 16 * 128, kP64), idesc_g, (j | k) != 0 ? 1u : 0u);
+          umma_f16_ts(tmem_base + 256, tmem_base + 128 + b * 64 + (k >> 1) * 32 + (k & 1) * 8, make_smem_desc_sw128_mn(k_addr + k * 16 * 128, kP64), idesc_g,
+                      (j | k) != 0 ? 1u : 0u);
         umma_commit(&kv_empty[st]);
-        umma_commit(&ds_free[b]);
         if (++st == kRing) st = 0;
       }
       umma_commit(done_bar);
     }
     __syncwarp();
   } else {
-    const int wg = (warp - 2) >> 2;
+    const int wg = (warp - 2) >> 2, par = wg & 1, half = wg >> 1;        // blocks of one parity, 32 of their 64 keys
     const int quad = warp & 3;
     const int r = quad * 32 + lane;                          // query row in tile == TMEM lane
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
@@ -445,65 +434,44 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const long loff = static_cast<long>(head) * p.total_tokens + seq_start + row;
     const float lse2 = row_ok ? p.lse[loff] * 1.4426950408889634f : INFINITY;     // +inf => P = 0
     const float dl = row_ok ? p.delta[loff] : 0.f;
-    for (int j = wg; j < n_kb; j += 2) {
+    const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), nl2 = pack_f32x2(-lse2, -lse2), nd2 = pack_f32x2(-dl, -dl);
+    const uint32_t t_s = tmem_base + par * 64 + half * 32 + lane_off, t_dp = t_s + 128;
+    auto nl = [&](int) { return nl2; };
+    auto nd = [&](int) { return nd2; };
+    for (int j = par; j < n_kb; j += 2) {
       const int n = j >> 1;
-      const int key0 = j * 64;
-      const bool edge = (key0 + 63 > q0) || (key0 + 64 > seq_len);
-      mbar_wait(&s_full[wg], n & 1);
+      const int key0 = j * 64 + half * 32;
+      const int hi = min(row, seq_len - 1) - key0;             // last visible key of these columns
+      mbar_wait(&s_full[par], n & 1);
       tc_fence_after();
-      uint32_t dk_[2][16];
+      uint32_t dk[16];
 #pragma unroll
-      for (int c32 = 0; c32 < 2; ++c32) {
-        uint32_t sv[32], dv_[32];
-        tmem_ld_32x32b_x32(tmem_base + wg * 64 + c32 * 32 + lane_off, sv);
-        tmem_ld_32x32b_x32(tmem_base + 128 + wg * 64 + c32 * 32 + lane_off, dv_);
+      for (int c = 0; c < 2; ++c) {
+        uint32_t sv[16], dv[16];
+        tmem_ld_32x32b_x16(t_s + c * 16, sv);
+        tmem_ld_32x32b_x16(t_dp + c * 16, dv);
         tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float p0 = exp2f(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse2));
-          float p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), p.scale_log2, -lse2));
-          if (edge) {
-            const int key = key0 + c32 * 32 + i;
-            if (key > row || key >= seq_len) p0 = 0.f;
-            if (key + 1 > row || key + 1 >= seq_len) p1 = 0.f;
-          }
-          const float d0 = p0 * (__uint_as_float(dv_[i]) - dl) * p.scale;
-          const float d1 = p1 * (__uint_as_float(dv_[i + 1]) - dl) * p.scale;
-          dk_[c32][i / 2] = pack_bf16x2(d0, d1);
-        }
+        if (key0 + 31 > q0 || key0 + 32 > seq_len) bwd_chunk<true, false>(sv, dv, sc2, nl, nd, ~mask_from(hi + 1 - c * 16), nullptr, dk + c * 8);
+        else bwd_chunk<false, false>(sv, dv, sc2, nl, nd, 0u, nullptr, dk + c * 8);
       }
-      if (j >= 2) {
-        mbar_wait(&ds_free[wg], (n - 1) & 1);
-        tc_fence_after();
-      }
-      uint8_t* drow = smem + L::kDS + wg * kPS + r * 128;
-      store_row_chunk(drow, r, 0, dk_[0]);
-      store_row_chunk(drow, r, 1, dk_[1]);
-      fence_proxy_async_smem();
+      tmem_st_32x32b_x16(t_dp, dk);
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ds_ready[wg]);
+      if (lane == 0) mbar_arrive(&ds_ready[par]);
     }
-    // ---- epilogue: each warpgroup writes 64 of the 128 dQ columns ----
+    // ---- epilogue: each warpgroup writes 32 of the 128 dQ columns ----
     mbar_wait(done_bar, 0);
     tc_fence_after();
-    __nv_bfloat16* dst = p.dq + static_cast<long>(seq_start + row) * p.dq_stride_t + head * 128 + wg * 64;
-#pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
-      uint32_t ov[32];
-      tmem_ld_32x32b_x32(tmem_base + 256 + wg * 64 + c * 32 + lane_off, ov);
-      tmem_ld_wait();
-      if (row_ok) {
+    __nv_bfloat16* dst = p.dq + static_cast<long>(seq_start + row) * p.dq_stride_t + head * 128 + wg * 32;
+    uint32_t ov[32];
+    tmem_ld_32x32b_x32(tmem_base + 256 + wg * 32 + lane_off, ov);
+    tmem_ld_wait();
+    if (row_ok) {
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          uint4 o4;
-          o4.x = pack_bf16x2(__uint_as_float(ov[q4 * 8]), __uint_as_float(ov[q4 * 8 + 1]));
-          o4.y = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 2]), __uint_as_float(ov[q4 * 8 + 3]));
-          o4.z = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 4]), __uint_as_float(ov[q4 * 8 + 5]));
-          o4.w = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 6]), __uint_as_float(ov[q4 * 8 + 7]));
-          *reinterpret_cast<uint4*>(dst + c * 32 + q4 * 8) = o4;
-        }
-      }
+      for (int i = 0; i < 16; ++i) ov[i] = pack_bf16x2(__uint_as_float(ov[2 * i]) * p.scale, __uint_as_float(ov[2 * i + 1]) * p.scale);
+      stg_v8(dst, ov);
+      stg_v8(dst + 16, ov + 8);
     }
   }
   tc_fence_before();
@@ -538,7 +506,7 @@ extern "C" cudaError_t nrl_attn_bwd_tc(const CUtensorMap* maps, const void* o, c
   p.dq_stride_t = dq_stride_t; p.dkv_stride_t = dkv_stride_t;
   p.num_seqs = num_seqs; p.total_tokens = total; p.Hq = Hq; p.G = Hq / Hkv;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
-  dim3 grid_kv(total / 128 + num_seqs, Hkv), grid_q(total / 128 + num_seqs, Hq);
+  const unsigned most = total / 128 + num_seqs, grid_kv = most * Hkv, grid_q = most * Hq;
   attn_bwd_dkdv_tc_kernel<<<grid_kv, kBwdThreads, DkdvSmem::kTotal, s>>>(maps[0], maps[1], maps[2], maps[3], p);
   attn_bwd_dq_tc_kernel<<<grid_q, kBwdThreads, DqSmem::kTotal, s>>>(maps[4], maps[5], maps[6], maps[7], p);
   return cudaGetLastError();
