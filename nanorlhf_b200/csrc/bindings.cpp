@@ -318,6 +318,47 @@ torch::Tensor gemm_tc_swiglu(const torch::Tensor& a, const torch::Tensor& w_inte
   return out;
 }
 
+// act[M, F] = silu(x Wg^T + tg Bg^T) * (x Wu^T + tu Bu^T): gate and up weights [F, K] as they are stored, optional adapters (t [M, r], B [F, r])
+torch::Tensor gemm_tc_swiglu_pair(const torch::Tensor& x, const torch::Tensor& wg, const torch::Tensor& wu, const c10::optional<torch::Tensor>& tg,
+                                  const c10::optional<torch::Tensor>& tu, const c10::optional<torch::Tensor>& bg, const c10::optional<torch::Tensor>& bu) {
+  check_tc_operand(x, "x");
+  check_tc_operand(wg, "wg");
+  check_tc_operand(wu, "wu");
+  const int64_t M = x.size(0), K = x.size(1), F = wg.size(0);
+  TORCH_CHECK(wg.size(1) == K && wu.size(0) == F && wu.size(1) == K && F % 8 == 0, "gemm_tc_swiglu_pair: weights [F, K]");
+  int64_t r = 0;
+  if (tg.has_value()) {
+    TORCH_CHECK(tu.has_value() && bg.has_value() && bu.has_value(), "gemm_tc_swiglu_pair: adapters go together");
+    r = tg->size(1);
+    for (const auto* t : {&*tg, &*tu}) {
+      check_tc_operand(*t, "t");
+      TORCH_CHECK(t->size(0) == M && t->size(1) == r, "gemm_tc_swiglu_pair: t [M, r]");
+    }
+    for (const auto* t : {&*bg, &*bu}) {
+      check_tc_operand(*t, "B");
+      TORCH_CHECK(t->size(0) == F && t->size(1) == r, "gemm_tc_swiglu_pair: B [F, r]");
+    }
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  torch::Tensor out = torch::empty({M, F}, x.options());
+  if (M == 0 || F == 0) return out;
+  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  auto map = [&](const torch::Tensor& t) { return nrl::make_tma_2d(t.data_ptr(), t.size(0), t.size(1), t.stride(0) * 2, 128, 64, BF, 2); };
+  CUtensorMap maps[8];
+  maps[0] = map(x);
+  maps[1] = map(wg);
+  maps[2] = map(wu);
+  maps[3] = r > 0 ? map(*tg) : maps[0];
+  maps[4] = r > 0 ? map(*tu) : maps[0];
+  maps[5] = r > 0 ? map(*bg) : maps[1];
+  maps[6] = r > 0 ? map(*bu) : maps[1];
+  maps[7] = nrl::make_tma_2d(out.data_ptr(), M, F, out.stride(0) * 2, 32, 64, BF, 2);
+  nrl::tc::TcParams p{};
+  p.M = static_cast<int>(M); p.N = static_cast<int>(2 * F); p.K = static_cast<int>(K); p.K2 = static_cast<int>(r); p.alpha = 1.f;
+  check(nrl_gemm_tc_pair(maps, &p, num_sms(), cur_stream()), "gemm_tc_swiglu_pair");
+  return out;
+}
+
 // act[M, F] = silu(x Wg^T) * (x Wu^T) with W_gu_interleaved[2F, K] (rows: per 32 features [32 gate | 32 up])
 torch::Tensor gemm_swiglu(const torch::Tensor& a, const torch::Tensor& w_interleaved, c10::optional<torch::Tensor> out_opt) {
   check_bf16_2d(a, "a");
@@ -1071,6 +1112,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_batched", &gemm_tc_batched, py::arg("a"), py::arg("b"), py::arg("out") = py::none(), py::arg("cg") = 0, py::arg("block_n") = 0);
   m.def("gemm_tc_swiglu", &gemm_tc_swiglu, py::arg("a"), py::arg("w_interleaved"), py::arg("out") = py::none(), py::arg("cg") = 0,
         py::arg("block_n") = 0);
+  m.def("gemm_tc_swiglu_pair", &gemm_tc_swiglu_pair, py::arg("x"), py::arg("wg"), py::arg("wu"), py::arg("tg") = py::none(),
+        py::arg("tu") = py::none(), py::arg("bg") = py::none(), py::arg("bu") = py::none());
   m.def("add_layernorm", &add_layernorm);
   m.def("lmhead_logprob_fwd", &lmhead_logprob_fwd, py::arg("hidden"), py::arg("weight"), py::arg("targets"),
         py::arg("inv_temperature"), py::arg("n_splits") = 0);

@@ -186,9 +186,13 @@ NRL_DEVICE void tma_store_3d(const CUtensorMap* m, const void* smem_src, int c0,
 // FP8: A and B are e4m3 bytes, K-major (a 128-byte swizzle row = 128 contraction elements), the MMA is kind::f8f6f4
 // (K = 32 per instruction, twice the bf16 rate) and the epilogue applies the per-row (token) and per-column (output
 // channel) dequantisation scales -- the sampler's fp8 rollout GEMMs (north star: fp8 tcgen05 GEMM in the decoder).
-template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, bool BATCH = false, bool FP8 = false, bool GROUPED = false>
+// PAIR (CTA pairs, BN = 256): act = silu(x Wg^T) * (x Wu^T) from two separate weights.  The leader loads 128 rows of the gate's
+// weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
+// columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.
+template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, bool BATCH = false, bool FP8 = false, bool GROUPED = false,
+          bool PAIR = false>
 NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
-                             const CUtensorMap& tmD, const TcParams& p) {
+                             const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* tmA3 = nullptr) {
   using C = Cfg<CG, BN, B_MN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBarOff);      // CG = 2: the leader's are the live ones
@@ -204,7 +208,8 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   const int num_n = (p.N + BN - 1) / BN;
   constexpr int kElemsPerKB = FP8 ? 2 * BLOCK_K : BLOCK_K;                  // 128 bytes of contraction per k-block either way
   const int num_kb1 = (p.K + kElemsPerKB - 1) / kElemsPerKB;
-  const int num_kb = num_kb1 + (p.K2 + kElemsPerKB - 1) / kElemsPerKB;
+  const int num_kb2 = (p.K2 + kElemsPerKB - 1) / kElemsPerKB;
+  const int num_kb = num_kb1 + (PAIR ? 2 : 1) * num_kb2;
   const int splits = SPLIT ? p.splits : 1;
   const int kb_per_split = (num_kb + splits - 1) / splits;
   const int tiles_per_batch = num_m * num_n;
@@ -260,6 +265,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           m0 = __ldg(p.grp_tiles + 3 * mt + 1);
           n0 = __ldg(p.grp_tiles + 3 * mt) * p.N + c.n_blk * BN;      // the expert's block of B rows
         }
+        if (PAIR) n0 = c.n_blk * (BN / 2);
         const int kb_lo = BATCH ? 0 : (w % splits) * kb_per_split, kb_hi = BATCH ? num_kb : min(num_kb, kb_lo + kb_per_split);
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           mbar_wait(&empty_bar[stage], phase ^ 1);
@@ -270,6 +276,13 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           const CUtensorMap* ma = second ? &tmA2 : &tmA;
           const CUtensorMap* mb = second ? &tmB2 : &tmB;
           const int k0 = (second ? kb - num_kb1 : kb) * kElemsPerKB;
+          if (PAIR && second) {
+            const int which = kb - num_kb1 >= num_kb2 ? 1 : 0, k2 = k0 - which * num_kb2 * kElemsPerKB;
+            tma_load_cg<CG>(sa, which ? tmA3 : &tmA2, &full_bar[stage], k2, m0);
+            tma_load_cg<CG>(sb, &tmB2, &full_bar[stage], k2, which == static_cast<int>(rank) ? n0 : p.N);
+            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+            continue;
+          }
           if (BATCH) {
             tma_load3_cg<CG>(sa, ma, &full_bar[stage], k0, m0, bidx);
             tma_load3_cg<CG>(sb, mb, &full_bar[stage], k0, n0, bidx);
@@ -455,6 +468,26 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         continue;
       }
+      if (PAIR) {                                           // group 0 takes features 0 .. 63 of the tile, group 1 the others
+        uint32_t pk[32];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t g[32], u[32];
+          tmem_ld_32x32b_x32(t_acc + group * 64 + h * 32, g);
+          tmem_ld_32x32b_x32(t_acc + BN / 2 + group * 64 + h * 32, u);
+          tmem_ld_wait();
+          if (h == 1) release_acc();
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float g0 = __uint_as_float(g[j]), g1 = __uint_as_float(g[j + 1]);
+            pk[h * 16 + j / 2] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * __uint_as_float(u[j]), g1 / (1.f + __expf(-g1)) * __uint_as_float(u[j + 1]));
+          }
+        }
+        const int col = c.n_blk * (BN / 2) + group * 64;
+        if (col < p.N / 2 && m_blk * BLOCK_M + quad * 32 < p.M) store_slab(pk, col, m_blk * BLOCK_M + quad * 32, 0);
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        continue;
+      }
 #pragma unroll 1
       for (int it = 0;; ++it) {
         // SwiGLU: two neighbouring chunks make one output slab and stay with one warp
@@ -616,6 +649,14 @@ gemm_tc_cg2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                    const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2,
                    const __grid_constant__ CUtensorMap tmD, const TcParams p) {
   gemm_tc_body<2, BN, A_MN, B_MN, EPI>(tmA, tmB, tmA2, tmB2, tmD, p);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBg, const __grid_constant__ CUtensorMap tmBu,
+                    const __grid_constant__ CUtensorMap tmA2g, const __grid_constant__ CUtensorMap tmA2u, const __grid_constant__ CUtensorMap tmB2g,
+                    const __grid_constant__ CUtensorMap tmB2u, const __grid_constant__ CUtensorMap tmD, const TcParams p) {
+  const bool up = cluster_ctarank() != 0;
+  gemm_tc_body<2, 256, false, false, EPI_SWIGLU, false, false, false, false, true>(tmA, up ? tmBu : tmBg, tmA2g, up ? tmB2u : tmB2g, tmD, p, &tmA2u);
 }
 
 template <int BN>
@@ -791,6 +832,23 @@ extern "C" cudaError_t nrl_gemm_tc_fp8(const CUtensorMap* maps, const nrl::tc::T
   if (!swiglu && cg == 2 && bn == 192) return launch_fp8<2, 192, EPI_BF16>(maps, *p, num_sms, stream);
   if (!swiglu && cg == 1 && bn == 192) return launch_fp8<1, 192, EPI_BF16>(maps, *p, num_sms, stream);
   return cudaErrorInvalidValue;
+}
+
+extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream) {
+  using namespace nrl::tc;
+  using C = Cfg<2, 256, false>;
+  if (p->N % 16 != 0) return cudaErrorInvalidValue;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  int units = ((p->M + 255) / 256) * ((p->N + 255) / 256);
+  if (units > num_sms / 2) units = num_sms / 2;
+  if (units < 1) units = 1;
+  gemm_tc_pair_kernel<<<2 * units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], *p);
+  return cudaGetLastError();
 }
 
 extern "C" cudaError_t nrl_gemm_tc_batched(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int num_sms,

@@ -58,5 +58,8 @@ extern "C" cudaError_t nrl_gemm_tc_batched(const CUtensorMap* maps, const nrl::t
 // squared ReLU of the columns instead, out_bf16 [rows, N] = relu(row_scale * x)^2, B rows in their own order.
 extern "C" cudaError_t nrl_gemm_tc_grouped(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int max_tiles, int num_sms,
                                            cudaStream_t stream);
+// act [M, F] = silu(x Wg^T + tg Bg^T) * (x Wu^T + tu Bu^T); maps = {x box {128, 64}, Wg, Wu box {128, 64}, tg, tu box {128, 64}, Bg, Bu box
+// {128, 64}, act box {32, 64}}; p->N = 2 F, p->K2 = columns of tg and tu (0: no adapters, maps 3 .. 6 may repeat a valid one)
+extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream);
 extern "C" cudaError_t nrl_gemm_tc(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int a_mn, int b_mn,
                                    int epi, int num_sms, cudaStream_t stream);

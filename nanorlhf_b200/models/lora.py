@@ -227,6 +227,29 @@ def lora_group_forward(x, mods):
     return [m(x) for m in mods]
 
 
+def plain_module(m, cls) -> bool:
+    """``m(x)`` runs ``cls.forward`` and nothing else, so that a fused kernel may stand in for the call."""
+    return isinstance(m, cls) and type(m).forward is cls.forward and not (m._forward_hooks or m._forward_pre_hooks)
+
+
+def fused_swiglu_forward(x, gate, up):
+    """``silu(gate(x)) * up(x)`` in one GEMM outside autograd (log-probability passes); None where that GEMM does not apply."""
+    if torch.is_grad_enabled() or not ops.use_native(x) or x.dtype != torch.bfloat16:
+        return None
+    from .qwen2 import Linear
+    lora = [isinstance(m, LoraLinear) for m in (gate, up)]
+    if not all(plain_module(m, LoraLinear if is_lora else Linear) for m, is_lora in zip((gate, up), lora)):
+        return None
+    if lora[0] != lora[1] or (lora[0] and ((gate.r, gate.scaling) != (up.r, up.scaling) or not all(isinstance(m.lora_dropout, nn.Identity) for m in (gate, up)))):
+        return None
+    if any(m.bias is not None for m in (gate, up)):
+        return None
+    from ..ops import gemm as _gemm
+    if lora[0]:
+        return _gemm.swiglu_linears(x, *[(m.weight, m.lora_A.weight, m.lora_B.weight) for m in (gate, up)], scaling=gate.scaling)
+    return _gemm.swiglu_linears(x, (gate.weight, None, None), (up.weight, None, None))
+
+
 def iter_lora_layers(model: nn.Module):
     for name, mod in model.named_modules():
         if isinstance(mod, LoraLinear):

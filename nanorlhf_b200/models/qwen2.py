@@ -145,7 +145,10 @@ class Qwen2MLP(nn.Module):
         self.down_proj = Linear(cfg.intermediate_size, cfg.hidden_size, bias=False)
 
     def forward(self, x):
-        from .lora import lora_group_forward
+        from .lora import fused_swiglu_forward, lora_group_forward
+        act = fused_swiglu_forward(x, self.gate_proj, self.up_proj)
+        if act is not None:
+            return self.down_proj(act)
         gate, up = lora_group_forward(x, [self.gate_proj, self.up_proj])
         return self.down_proj(ops.swiglu_pair(gate, up))
 
@@ -159,7 +162,14 @@ class Qwen2DecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(cfg.hidden_size, cfg.rms_norm_eps)
 
     def forward(self, h, cos, sin, cu_seqlens, max_seqlen):
-        h = h + self.self_attn(self.input_layernorm(h), cos, sin, cu_seqlens, max_seqlen)
+        from .lora import plain_module
+        a = self.self_attn(self.input_layernorm(h), cos, sin, cu_seqlens, max_seqlen)
+        norm = self.post_attention_layernorm
+        if (not torch.is_grad_enabled() and ops.use_native(h) and h.dim() == 2 and plain_module(norm, RMSNorm)
+                and h.dtype == a.dtype == norm.weight.dtype == torch.bfloat16):
+            y, h = ops.add_rmsnorm(a, h, norm.weight, norm.eps)          # residual add and norm in one pass
+            return h + self.mlp(y)
+        h = h + a
         h = h + self.mlp(self.post_attention_layernorm(h))
         return h
 
