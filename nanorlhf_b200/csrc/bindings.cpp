@@ -457,12 +457,17 @@ torch::Tensor gemm_tc_fp8(const torch::Tensor& aq, const torch::Tensor& a_scale,
   return out;
 }
 
+// Vocabulary splits of the log-prob head: the (row tile, split) items are walked by one CTA per SM, so the time is the number of rounds
+// times the tiles of an item; of equals the smallest.  6001 rows (47 row tiles) x 151 936: the smallest count that covers the SMs (4, two rounds
+// of 149 tiles) took 2623 us, 22 (seven rounds of 27) 1852 us.
 int pick_splits(int64_t M, int64_t N, int bn) {
-  int64_t num_m = (M + 127) / 128, num_n = (N + bn - 1) / bn;
-  int64_t s = (num_sms() + num_m - 1) / num_m;       // enough work items to cover the SMs
-  if (num_m >= num_sms()) s = 1;
-  s = std::max<int64_t>(1, std::min<int64_t>(s, std::min<int64_t>(num_n, 64)));
-  return static_cast<int>(s);
+  const int64_t num_m = (M + 127) / 128, num_n = (N + bn - 1) / bn, sms = num_sms();
+  int64_t best = 1, least = INT64_MAX;
+  for (int64_t s = 1; s <= std::min<int64_t>(num_n, 64); ++s) {
+    const int64_t tiles = (num_m * s + sms - 1) / sms * ((num_n + s - 1) / s);
+    if (tiles < least) { least = tiles; best = s; }
+  }
+  return static_cast<int>(best);
 }
 
 // fused lm-head log-prob forward: returns (logp, entropy, lse), all fp32 [M]
