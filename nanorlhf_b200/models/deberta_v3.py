@@ -27,6 +27,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import ops
+from .lora import plain_module
 from .qwen2 import Linear
 
 
@@ -203,10 +204,9 @@ class _Intermediate(nn.Module):
         self.dense = Linear(cfg.hidden_size, cfg.intermediate_size)
 
     def forward(self, x):
-        # GEMM + bias + GELU epilogue (tcgen05 kernel, act=1).  Measured on B200 at 26.5k x 4096 x 1024 the erf in the
-        # epilogue makes the tile epilogue longer than its 16 k-block main loop (0.41 ms vs cuBLAS 0.16 + GELU 0.12),
-        # so it is opt-in until the epilogue is split across more warps.
-        if _fused_inference(x) and x.shape[-1] % 8 == 0 and os.environ.get("NANORLHF_DEBERTA_GELU_FUSED", "0") == "1":
+        # GEMM + bias + GELU epilogue (tcgen05 kernel, act=1).  24 571 x 4096 x 1024: a pass of its own costs 119 us, the epilogue
+        # 53 us: its eight warps form part of it behind the next tile's main loop
+        if _fused_inference(x) and x.shape[-1] % 8 == 0 and plain_module(self.dense, Linear):
             return ops.linear(x, self.dense.weight, self.dense.bias, act=1)
         return F.gelu(self.dense(x))
 
