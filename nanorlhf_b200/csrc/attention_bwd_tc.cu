@@ -1,7 +1,7 @@
 // tcgen05 / TMEM / TMA flash-attention BACKWARD (causal, packed varlen, GQA, head_dim 128) for sm_100a.
 //
 // Three kernels, no atomics (same decomposition as the mma.sync version in attention_varlen.cu, which stays the oracle):
-//   delta   : delta[h, t] = sum_d dO * O                                   (one warp per (token, head))
+//   delta   : delta[h, t] = sum_d dO * O                                   (half a warp per (token, head))
 //   dK / dV : one CTA per (128-key block, kv head).  K_j, V_j stay in smem; the CTA streams (q head of the group,
 //             64-row query block) pairs:   S^T = K_j Q_i^T,  dP^T = V_j dO_i^T          (tcgen05, TMEM lanes = keys)
 //             P^T = exp2(S^T*c - lse_i),  dS^T = P^T o (dP^T - delta_i)                   (softmax warps, one key row each)
@@ -88,19 +88,33 @@ NRL_DEVICE void bwd_chunk(const uint32_t (&sv)[16], const uint32_t (&dv)[16], ui
   }
 }
 
+// Half a warp per pair, sixteen bytes per lane, two pairs in flight: 12 011 tokens x 28 heads 51 -> 29 us (8 bytes per lane, one pair per warp before)
 __global__ void attn_bwd_delta_tc_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                                         float* __restrict__ delta, long o_stride_t, int total, int Hq) {
-  const long idx = blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (idx >= static_cast<long>(total) * Hq) return;
-  const int lane = threadIdx.x & 31;
-  const long t = idx / Hq;
-  const int h = idx % Hq;
-  const uint2 a = *reinterpret_cast<const uint2*>(o + t * o_stride_t + h * 128 + lane * 4);
-  const uint2 b = *reinterpret_cast<const uint2*>(dout + t * o_stride_t + h * 128 + lane * 4);
-  const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y);
-  float acc = a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
-  acc = warp_sum(acc);
-  if (lane == 0) delta[static_cast<long>(h) * total + t] = acc;
+                                         float* __restrict__ delta, long o_stride_t, int total, unsigned Hq, unsigned pairs) {
+  const int sub = threadIdx.x & 15;
+  const unsigned first = (blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4)) * 2;
+  uint4 a[2], b[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const unsigned idx = min(first + u, pairs - 1), t = idx / Hq, h = idx - t * Hq;
+    const long off = t * o_stride_t + h * 128 + sub * 8;
+    a[u] = *reinterpret_cast<const uint4*>(o + off);
+    b[u] = *reinterpret_cast<const uint4*>(dout + off);
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, bw[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = unpack_bf16x2(aw[e]), y = unpack_bf16x2(bw[e]);
+      acc = fmaf(x.x, y.x, fmaf(x.y, y.y, acc));
+    }
+#pragma unroll
+    for (int m = 8; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    const unsigned idx = first + u, t = idx / Hq, h = idx - t * Hq;
+    if (sub == 0 && idx < pairs) delta[static_cast<long>(h) * total + t] = acc;
+  }
 }
 
 // =====================================================================================================================
@@ -497,9 +511,9 @@ extern "C" cudaError_t nrl_attn_bwd_tc(const CUtensorMap* maps, const void* o, c
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  const long pairs = static_cast<long>(total) * Hq;
-  attn_bwd_delta_tc_kernel<<<static_cast<int>((pairs + 7) / 8), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), delta, o_stride_t, total, Hq);
+  const unsigned pairs = static_cast<unsigned>(total) * Hq;                   // O alone would be a terabyte at 2^32
+  attn_bwd_delta_tc_kernel<<<(pairs + 31) / 32, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), delta,
+                                                            o_stride_t, total, Hq, pairs);
   AttnBwdParams p;
   p.cu_seqlens = cu; p.lse = lse; p.delta = delta;
   p.dq = static_cast<__nv_bfloat16*>(dq); p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
