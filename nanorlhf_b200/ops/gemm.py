@@ -176,18 +176,14 @@ def lora_linear_group(x, projs, scaling: float):
     return list(_LoraGroupFn.apply(x, float(scaling), len(projs), *flat))
 
 
-# Rows from which the two projections of a SwiGLU are one GEMM: one tile of the CTA pair.  1536 -> 8960 features, two GEMMs and an activation
-# pass against one: 256 rows 27 -> 17 us (39 -> 30 with adapters), 1000 rows 57 -> 41 (73 -> 57), 32 768 rows 1602 -> 1213 (1531 -> 1295).
-# Fewer rows would leave part of every tile empty; there split-K and smaller tiles fill the GPU.
-PAIR_ROWS = 256
-
-
 def swiglu_linears(x, gate, up, scaling: float = 0.0):
-    """``silu(x Wg^T) * (x Wu^T)`` without the two projections in memory (no autograd); ``gate`` / ``up`` = (W, A | None, B | None) with a
+    """``silu(x Wg^T) * (x Wu^T)`` without the two projections in memory (no autograd), for any number of rows: two GEMMs and an activation
+    pass against one, 1536 -> 8960 features: 8 rows 32 / 19 us, 256 rows 28 / 17 (42 / 31 with adapters), 1000 rows 57 / 41 (73 / 57), 32 768
+    rows 1602 / 1213 (1531 / 1295); 4096 -> 1024 features, eight tiles only: 8 rows 29 / 25 us, 1024 rows 37 / 27. ``gate`` / ``up`` = (W, A | None, B | None) with a
     LoRA term of ``scaling`` when A and B are given.  None when the fused GEMM does not take the call."""
     (wg, ag, bg), (wu, au, bu) = gate, up
     x2 = _rows(x)
-    if x2.shape[0] < PAIR_ROWS or not (supported(x, wg) and supported(x, wu)) or wg.shape != wu.shape or (ag is None) != (au is None):
+    if x2.shape[0] == 0 or not (supported(x, wg) and supported(x, wu)) or wg.shape != wu.shape or (ag is None) != (au is None):
         return None
     if ag is None:
         _native_mod._count()
