@@ -396,6 +396,13 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       const uint32_t t_acc = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
       uint32_t sw_packed[32];
       (void)sw_packed;
+      float dl_lse = 0.f, dl_g = 0.f;
+      int dl_target = -1;
+      if (EPI == EPI_DLOGITS && row_ok) {
+        dl_lse = p.lse[row];
+        dl_g = p.grad[row] * p.alpha;                       // d logp / d logit carries the 1 / T factor
+        dl_target = p.targets[row];
+      }
       if (SPLIT) {
         // ---- split-K: park the fp32 partial tile, the last CTA of the tile reduces all partials in split order ----
         const long tile_elems = static_cast<long>(BLOCK_M) * BN;
@@ -595,7 +602,11 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
 #pragma unroll
               for (int e = 0; e < 8; ++e) x[e] *= rs * ((col + e < p.N) ? p.col_scale[col + e] : 0.f);
             }
-            if (p.bias != nullptr && col < p.N) {         // N % 8 == 0
+            if (EPI == EPI_DLOGITS) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) x[e] = ((col + e == dl_target ? 1.f : 0.f) - exp2f((x[e] - dl_lse) * 1.4426950408889634f)) * dl_g;
+            }
+            if (EPI != EPI_DLOGITS && p.bias != nullptr && col < p.N) {         // N % 8 == 0
               uint32_t bw[4];
               if (bias_vec) {
                 const uint4 bv = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
@@ -612,7 +623,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
                 x[2 * e + 1] += bf.y;
               }
             }
-            if (p.act == 1) {
+            if (EPI != EPI_DLOGITS && p.act == 1) {
 #pragma unroll
               for (int e = 0; e < 8; ++e) x[e] = gelu_erf_tc(x[e]);
             }
@@ -815,6 +826,11 @@ static cudaError_t launch(const CUtensorMap* maps, const TcParams& p, int num_sm
 
 }  // namespace tc
 }  // namespace nrl
+
+extern "C" cudaError_t nrl_gemm_tc_dlogits(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream) {
+  const CUtensorMap all[5] = {maps[0], maps[1], maps[0], maps[1], maps[2]};
+  return nrl::tc::launch<2, 256, false, false, nrl::tc::EPI_DLOGITS>(all, *p, num_sms, stream);
+}
 
 // e4m3 x e4m3 GEMM with per-row x per-column scales; maps = {A (uint8 [M,K], box {128, 128}), B (uint8 [N,K], box {bn/cg, 128}), D}
 extern "C" cudaError_t nrl_gemm_tc_fp8(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int swiglu, int num_sms,

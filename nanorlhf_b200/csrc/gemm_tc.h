@@ -10,6 +10,7 @@ namespace tc {
 enum TcEpilogue : int {
   EPI_BF16 = 0,      // D (bf16, TMA store) = alpha * acc (+ bias) (GELU)
   EPI_F32 = 1,       // out_f32 (row-major, plain stores) (+)= alpha * acc
+  EPI_DLOGITS = 3,   // D (bf16, TMA store) = (onehot(target) - exp(alpha * acc - lse)) * grad * alpha: backward of the log-prob head
   EPI_SWIGLU = 2,    // D[M, N/2] (bf16, TMA store) = silu(gate) * up; B rows interleaved per 32 features [32 gate | 32 up]
 };
 
@@ -18,6 +19,9 @@ struct TcParams {
   int K2;                       // contraction length of the second operand pair (0 = none)
   const float* row_scale;       // FP8 kernels: [M] per-token dequantisation scale of A (GROUPED: see below)
   const float* col_scale;       // FP8 kernels: [N] per-output-channel dequantisation scale of B
+  const int* targets;           // EPI_DLOGITS: [M] column of the row's target
+  const float* lse;             // EPI_DLOGITS: [M] log of the row's sum of exponentials
+  const float* grad;            // EPI_DLOGITS: [M] gradient of the row's log-probability
   int batch;                    // BATCH kernels: number of independent [M,K] x [N,K]^T problems behind 3D tensor maps (else 1)
   float alpha;                  // multiplies the accumulator
   const __nv_bfloat16* bias;    // EPI_BF16: optional [N]
@@ -46,6 +50,8 @@ struct TcParams {
 
 extern "C" cudaError_t nrl_gemm_tc_splitk(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int a_mn, int b_mn, int num_sms,
                                           cudaStream_t stream);
+// EPI_DLOGITS on CTA pairs, 256 x 256 tiles; maps = {A box {128, 64}, B box {128, 64}, D box {32, 64}}
+extern "C" cudaError_t nrl_gemm_tc_dlogits(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream);
 extern "C" cudaError_t nrl_gemm_tc_fp8(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int swiglu, int num_sms,
                                        cudaStream_t stream);
 // batched K-major x K-major GEMM, bf16 out; maps = {A, B, D} 3D (tma_host.h make_tma_3d), B box rows = bn / cg
