@@ -675,7 +675,7 @@ std::tuple<torch::Tensor, torch::Tensor> gae_scan(const torch::Tensor& rewards, 
     rptr = ret.data_ptr<float>();
   }
   check(nrl_gae_scan(rewards.data_ptr<float>(), vptr, adv.data_ptr<float>(), rptr, rewards.size(0), rewards.size(1),
-                     static_cast<float>(gamma), static_cast<float>(lam), cur_stream()), "gae_scan");
+                     gamma, lam, cur_stream()), "gae_scan");
   return {adv, ret};
 }
 

@@ -27,7 +27,7 @@ cudaError_t nrl_swiglu_bwd(const void* gate, const void* up, long in_stride, con
                            long out_stride, long T, int F, cudaStream_t s);
 
 cudaError_t nrl_gae_scan(const float* rewards, const float* values, float* adv, float* returns, int B, int T,
-                         float gamma, float lam, cudaStream_t s);
+                         double gamma, double lam, cudaStream_t s);
 cudaError_t nrl_policy_loss(const float* new_lp, const float* old_lp, const float* adv, const uint8_t* mask,
                             const float* ref_lp, float cliprange, float kl_coef, long n, float* grad_unnorm,
                             float* loss, float* stats, double* scratch, cudaStream_t s);

@@ -16,35 +16,37 @@ namespace nrl {
 // A_t = delta_t + c * A_{t+1},  delta_t = r_t + gamma * V_{t+1} - V_t  (V == nullptr -> delta = r, c = gamma*lam)
 // Block per row, kGaePer consecutive steps per thread: a thread folds its own steps, a weighted reverse scan over the warp and one over
 // the warps give every thread the advantage behind its last step, and the recurrence is then run as it is written.  4 x 1500 steps: 15 us
-// with one warp per row (47 dependent rounds of load and shuffle), 3.6 us here; longer rows go tile by tile from the end.
+// with one warp per row (47 dependent rounds of load and shuffle), 3.6 us here; longer rows go tile by tile from the end.  In double: powers of
+// a rounded c cost more than the sums themselves (error against float64 2.4e-7 -> 2.5e-8).
 constexpr int kGaeThreads = 256, kGaePer = 8, kGaeTile = kGaeThreads * kGaePer;
 
 __global__ void __launch_bounds__(kGaeThreads)
 gae_scan_kernel(const float* __restrict__ rewards, const float* __restrict__ values, float* __restrict__ adv,
-                float* __restrict__ returns, int T, float gamma, float lam) {
-  __shared__ float heads[kGaeThreads / 32 + 1];      // folded value of every warp's steps; one more: the tile's first advantage
+                float* __restrict__ returns, int T, double gamma, double lam) {
+  __shared__ double heads[kGaeThreads / 32 + 1];      // folded value of every warp's steps; one more: the tile's first advantage
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t row = static_cast<size_t>(blockIdx.x) * T;
   const float* r = rewards + row;
   const float* v = values ? values + row : nullptr;
-  const float c = gamma * lam;
-  float w[6];                                        // c^8, c^16 .. c^256: weights of a step of the scan
+  const double c = gamma * lam;
+  double w[6];                                       // c^8, c^16 .. c^256: weights of a step of the scan
   w[0] = c * c;
   w[0] *= w[0];
   w[0] *= w[0];
 #pragma unroll
   for (int k = 1; k < 6; ++k) w[k] = w[k - 1] * w[k - 1];
-  float c_lane = 1.f;                                // c^(8 * (32 - lane - 1)): from the next warp's first step to this thread's last
+  double c_lane = 1.0;                                // c^(8 * (32 - lane - 1)): from the next warp's first step to this thread's last
 #pragma unroll
   for (int k = 0; k < 5; ++k)
     if ((31 - lane) & (1 << k)) c_lane *= w[k];
-  float behind = 0.f;                                // advantage of the step behind the tile
+  double behind = 0.0;                                // advantage of the step behind the tile
   for (int tile = (T - 1) / kGaeTile; tile >= 0; --tile) {
     const int t0 = tile * kGaeTile + tid * kGaePer;
-    float d[kGaePer], vt[kGaePer];
+    double d[kGaePer];
+    float vt[kGaePer];
 #pragma unroll
     for (int j = 0; j < kGaePer; ++j) {
-      d[j] = t0 + j < T ? r[t0 + j] : 0.f;
+      d[j] = t0 + j < T ? r[t0 + j] : 0.0;
       vt[j] = v != nullptr && t0 + j < T ? v[t0 + j] : 0.f;
     }
     if (v != nullptr) {
@@ -52,27 +54,27 @@ gae_scan_kernel(const float* __restrict__ rewards, const float* __restrict__ val
 #pragma unroll
       for (int j = 0; j < kGaePer; ++j) d[j] += gamma * (j + 1 < kGaePer ? vt[j + 1] : vn) - vt[j];
     }
-    float x = 0.f;
+    double x = 0.0;
 #pragma unroll
-    for (int j = kGaePer - 1; j >= 0; --j) x = fmaf(c, x, d[j]);
+    for (int j = kGaePer - 1; j >= 0; --j) x = fma(c, x, d[j]);
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
-      const float y = __shfl_down_sync(0xffffffffu, x, 1 << k);
-      if (lane + (1 << k) < 32) x = fmaf(w[k], y, x);
+      const double y = __shfl_down_sync(0xffffffffu, x, 1 << k);
+      if (lane + (1 << k) < 32) x = fma(w[k], y, x);
     }
     __syncthreads();                                 // `heads` of the tile before has been read
     if (lane == 0) heads[warp] = x;
     __syncthreads();
-    float in = behind;                               // advantage at the first step of the next warp
-    for (int q = kGaeThreads / 32 - 1; q > warp; --q) in = fmaf(w[5], in, heads[q]);
-    const float next = __shfl_down_sync(0xffffffffu, x, 1);
-    float a = fmaf(c_lane, in, lane < 31 ? next : 0.f);
+    double in = behind;                               // advantage at the first step of the next warp
+    for (int q = kGaeThreads / 32 - 1; q > warp; --q) in = fma(w[5], in, heads[q]);
+    const double next = __shfl_down_sync(0xffffffffu, x, 1);
+    double a = fma(c_lane, in, lane < 31 ? next : 0.0);
 #pragma unroll
     for (int j = kGaePer - 1; j >= 0; --j) {
-      a = fmaf(c, a, d[j]);
+      a = fma(c, a, d[j]);
       if (t0 + j < T) {
-        adv[row + t0 + j] = a;
-        if (returns) returns[row + t0 + j] = a + vt[j];
+        adv[row + t0 + j] = static_cast<float>(a);
+        if (returns) returns[row + t0 + j] = static_cast<float>(a + vt[j]);
       }
     }
     if (tid == 0) heads[kGaeThreads / 32] = a;
@@ -304,7 +306,7 @@ __global__ void adamw_flat_kernel(__nv_bfloat16* __restrict__ param, const __nv_
 using namespace nrl;
 
 extern "C" cudaError_t nrl_gae_scan(const float* rewards, const float* values, float* adv, float* returns, int B,
-                                    int T, float gamma, float lam, cudaStream_t s) {
+                                    int T, double gamma, double lam, cudaStream_t s) {
   if (B == 0 || T == 0) return cudaSuccess;
   gae_scan_kernel<<<B, kGaeThreads, 0, s>>>(rewards, values, adv, returns, T, gamma, lam);
   return cudaGetLastError();
