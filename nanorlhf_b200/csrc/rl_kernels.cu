@@ -92,6 +92,11 @@ constexpr int kLossThreads = 512;
 constexpr long kLossClusterMax = 1 << 17;
 constexpr unsigned kLossBlocks = 148;
 
+// A block's shared memory may be written by the others of its cluster once it is known to run: every thread arrives on entry to the kernel and
+// waits in front of the first remote write, so that the pass over the tokens hides the barrier.
+__device__ __forceinline__ void cluster_started_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_started_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 template <int NS>
 __device__ bool loss_sums(double (&s)[NS], double* scratch, double (&tot)[NS]) {      // true in the one thread that has the totals
   namespace cg = cooperative_groups;
@@ -109,6 +114,7 @@ __device__ bool loss_sums(double (&s)[NS], double* scratch, double (&tot)[NS]) {
     for (int q = 0; q < kLossThreads / 32; ++q) t += red[threadIdx.x][q];
   if (scratch == nullptr) {
     cg::cluster_group cl = cg::this_cluster();
+    cluster_started_wait();
     if (threadIdx.x < NS) cl.map_shared_rank(&parts[0][0], 0)[cl.block_rank() * NS + threadIdx.x] = t;
     cl.sync();
     if (cl.block_rank() != 0 || threadIdx.x != 0) return false;
@@ -142,6 +148,7 @@ __global__ void __launch_bounds__(kLossThreads)
 policy_loss_kernel(const float* __restrict__ new_lp, const float* __restrict__ old_lp, const float* __restrict__ adv,
                    const uint8_t* __restrict__ mask, const float* __restrict__ ref_lp, float cliprange, float kl_coef, long n,
                    float* __restrict__ grad_unnorm, float* __restrict__ loss, float* __restrict__ stats, double* scratch) {
+  if (scratch == nullptr) cluster_started_arrive();
   double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -186,6 +193,7 @@ __global__ void __launch_bounds__(kLossThreads)
 value_loss_kernel(const float* __restrict__ vpred, const float* __restrict__ vold, const float* __restrict__ ret,
                   const uint8_t* __restrict__ mask, float clip, long n, float* __restrict__ grad_unnorm, float* __restrict__ loss,
                   float* __restrict__ stats, double* scratch) {
+  if (scratch == nullptr) cluster_started_arrive();
   double s[3] = {0, 0, 0};
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
