@@ -24,6 +24,7 @@ from typing import Dict, Iterable, List, Optional
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
 
@@ -87,6 +88,8 @@ class LoraLinear(nn.Module):
                                    self.lora_B.weight, self.scaling)
         y = self.base_layer(x)
         return y + self.lora_B(self.lora_A(self.lora_dropout(x))) * self.scaling
+
+    plain_forward = forward              # what a fused kernel may stand in for (plain_module)
 
     @torch.no_grad()
     def merged_weight(self) -> torch.Tensor:
@@ -228,8 +231,10 @@ def lora_group_forward(x, mods):
 
 
 def plain_module(m, cls) -> bool:
-    """``m(x)`` runs ``cls.forward`` and nothing else, so that a fused kernel may stand in for the call."""
-    return isinstance(m, cls) and type(m).forward is cls.forward and not (m._forward_hooks or m._forward_pre_hooks)
+    """``m(x)`` runs ``cls.plain_forward`` and nothing else, so that a fused kernel may stand in for the call: no forward of a subclass, of the
+    instance or put in the class's place, no call operator of its own, no hook of the module or of all modules."""
+    return (isinstance(m, cls) and type(m).forward is cls.plain_forward and "forward" not in vars(m) and type(m).__call__ is nn.Module.__call__
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) and not _has_any_global_hook())
 
 
 def fused_swiglu_forward(x, gate, up):

@@ -102,6 +102,8 @@ class Linear(nn.Linear):
     def forward(self, x):
         return ops.linear(x, self.weight, self.bias)
 
+    plain_forward = forward              # what a fused kernel may stand in for (lora.plain_module)
+
 
 class RMSNorm(nn.Module):
     def __init__(self, dim, eps):
@@ -111,6 +113,8 @@ class RMSNorm(nn.Module):
 
     def forward(self, x):
         return ops.rmsnorm(x, self.weight, self.eps)
+
+    plain_forward = forward
 
 
 class Qwen2Attention(nn.Module):
