@@ -82,7 +82,7 @@ class LoraLinear(nn.Module):
         return self.base_layer.out_features
 
     def forward(self, x):
-        if isinstance(self.lora_dropout, nn.Identity) and not self.base_layer.weight.requires_grad:
+        if _adapter_in_gemm(self):
             # one dual-source-K tcgen05 GEMM per direction on CUDA (ops/gemm.py); PyTorch oracle elsewhere
             return ops.lora_linear(x, self.base_layer.weight, self.base_layer.bias, self.lora_A.weight,
                                    self.lora_B.weight, self.scaling)
@@ -219,11 +219,17 @@ def get_peft_model(model: nn.Module, config: LoraConfig) -> PeftModel:
     return PeftModel(model, config)
 
 
+def _adapter_in_gemm(m) -> bool:
+    """The adapter rides in the base GEMM: no dropout, a frozen base.  Otherwise the base, the two factors and the sum are calls of their own, each
+    rounded, in every mode."""
+    return isinstance(m.lora_dropout, nn.Identity) and not m.base_layer.weight.requires_grad
+
+
 def lora_group_forward(x, mods):
     """``[m(x) for m in mods]`` for projections that share their input; when all of them are plain LoRA layers with the
     same rank / scaling their rank-r projections run as one launch (ops.lora_linear_group)."""
     if (len(mods) > 1 and all(isinstance(m, LoraLinear) for m in mods)
-            and all(isinstance(m.lora_dropout, nn.Identity) and not m.base_layer.weight.requires_grad for m in mods)
+            and all(_adapter_in_gemm(m) for m in mods)
             and len({(m.r, m.scaling) for m in mods}) == 1):
         return ops.lora_linear_group(x, [(m.base_layer.weight, m.base_layer.bias, m.lora_A.weight, m.lora_B.weight) for m in mods],
                                      mods[0].scaling)
@@ -245,7 +251,7 @@ def fused_swiglu_forward(x, gate, up):
     lora = [isinstance(m, LoraLinear) for m in (gate, up)]
     if not all(plain_module(m, LoraLinear if is_lora else Linear) for m, is_lora in zip((gate, up), lora)):
         return None
-    if lora[0] != lora[1] or (lora[0] and ((gate.r, gate.scaling) != (up.r, up.scaling) or not all(isinstance(m.lora_dropout, nn.Identity) for m in (gate, up)))):
+    if lora[0] != lora[1] or (lora[0] and ((gate.r, gate.scaling) != (up.r, up.scaling) or not all(_adapter_in_gemm(m) for m in (gate, up)))):
         return None
     if any(m.bias is not None for m in (gate, up)):
         return None
