@@ -245,7 +245,7 @@ def plain_module(m, cls) -> bool:
 
 def fused_swiglu_forward(x, gate, up):
     """``silu(gate(x)) * up(x)`` in one GEMM outside autograd (log-probability passes); None where that GEMM does not apply."""
-    if torch.is_grad_enabled() or not ops.use_native(x) or x.dtype != torch.bfloat16:
+    if not ops.direct_calls() or not ops.use_native(x) or x.dtype != torch.bfloat16:
         return None
     from .qwen2 import Linear
     lora = [isinstance(m, LoraLinear) for m in (gate, up)]

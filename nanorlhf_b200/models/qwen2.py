@@ -169,7 +169,7 @@ class Qwen2DecoderLayer(nn.Module):
         from .lora import plain_module
         a = self.self_attn(self.input_layernorm(h), cos, sin, cu_seqlens, max_seqlen)
         norm = self.post_attention_layernorm
-        if (not torch.is_grad_enabled() and ops.use_native(h) and h.dim() == 2 and plain_module(norm, RMSNorm)
+        if (ops.direct_calls() and ops.use_native(h) and h.dim() == 2 and plain_module(norm, RMSNorm)
                 and h.dtype == a.dtype == norm.weight.dtype == torch.bfloat16):
             y, h = ops.add_rmsnorm(a, h, norm.weight, norm.eps)          # residual add and norm in one pass
             return h + self.mlp(y)

@@ -44,6 +44,13 @@ def use_native(t: torch.Tensor) -> bool:
     return t.is_cuda
 
 
+def direct_calls() -> bool:
+    """A kernel may be called without an autograd function around it: autograd is off and nothing traces or transforms the program.  A trace would
+    keep such a call's result as a constant and forward-mode would lose the tangent, where the function is recorded or refuses."""
+    return not (torch.is_grad_enabled() or torch._C._get_tracing_state() or torch._C._are_functorch_transforms_active()
+                or torch.autograd.forward_ad._current_level >= 0)
+
+
 def backend_name(t: torch.Tensor) -> str:
     return "cuda" if use_native(t) else "torch"
 

@@ -40,3 +40,22 @@ def test_adapters_that_do_not_ride_in_the_base_gemm_stay_as_they_are(fused):
         assert fused(gate, up) is None
         assert fused(_pair(True)[0], _pair(False)[0]) is None
         assert fused(*[nn.Linear(8, 16, bias=False, dtype=torch.bfloat16) for _ in range(2)]) is None
+
+
+def _dual(f, x):
+    with torch.autograd.forward_ad.dual_level():
+        return f(x)
+
+
+@pytest.mark.parametrize("around", [
+    lambda f, x: torch.jit.trace(lambda t: (f(t), t)[1], x, check_trace=False),
+    lambda f, x: torch.vmap(lambda t: (f(t), t)[1])(x[None]),
+    lambda f, x: torch.func.jvp(lambda t: (f(t), t)[1], (x,), (x,)),
+    _dual,
+], ids=["trace", "vmap", "jvp", "dual level"])
+def test_tracing_and_transforms_keep_the_autograd_functions(fused, around):
+    seen, pair = [], _pair(False)
+    with torch.no_grad():
+        around(lambda t: seen.append((fused(*pair, t), ops.direct_calls())), torch.zeros(2, 8, dtype=torch.bfloat16))
+        assert seen == [(None, False)] and ops.direct_calls()
+    assert not ops.direct_calls()
