@@ -728,13 +728,21 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> value_loss(const torch::
 // grad_unnorm * (g_loss / denom), both scalars on the device
 torch::Tensor loss_grad(const torch::Tensor& grad_unnorm, const torch::Tensor& g_loss, const torch::Tensor& denom) {
   if (at::GradMode::is_enabled() || g_loss.scalar_type() != torch::kFloat32)      // a graph of the gradient is wanted
-    return grad_unnorm * (g_loss / denom[0]);
+    return grad_unnorm * (g_loss / denom);
   c10::cuda::CUDAGuard guard(grad_unnorm.device());
   torch::Tensor out = torch::empty_like(grad_unnorm);
   const torch::Tensor g = g_loss.contiguous();
   check(nrl_loss_grad(grad_unnorm.data_ptr<float>(), g.data_ptr<float>(), denom.data_ptr<float>(), out.numel(), out.data_ptr<float>(),
                       cur_stream()), "loss_grad");
   return out;
+}
+
+// The entries of `stats` as tensors of their own that share its memory: no views, each with its own version, so that a caller may change a
+// statistic in place before the backward.
+std::vector<torch::Tensor> own_scalars(const torch::Tensor& stats) {
+  std::vector<torch::Tensor> parts = stats.unbind();
+  for (auto& t : parts) t = t.variable_data();
+  return parts;
 }
 
 // The losses as autograd functions of the first argument.  Both run for a few thousand tokens, where Python's share of a custom function
@@ -746,7 +754,7 @@ struct PolicyLossFn : public torch::autograd::Function<PolicyLossFn> {
                                                 double kl_coef) {
     if (ref_lp.has_value()) ref_lp = ref_lp->contiguous();
     auto [loss, grad, stats] = policy_loss(new_lp.contiguous(), old_lp.contiguous(), adv.contiguous(), mask.contiguous(), ref_lp, cliprange, kl_coef);
-    ctx->save_for_backward({grad, stats});
+    ctx->save_for_backward({grad, own_scalars(stats)[0]});
     ctx->mark_non_differentiable({stats});
     return {loss, stats};
   }
@@ -760,7 +768,7 @@ struct ValueLossFn : public torch::autograd::Function<ValueLossFn> {
   static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, torch::Tensor vpred, torch::Tensor vold, torch::Tensor ret,
                                                 torch::Tensor mask, double clip) {
     auto [loss, grad, stats] = value_loss(vpred.contiguous(), vold.contiguous(), ret.contiguous(), mask.contiguous(), clip);
-    ctx->save_for_backward({grad, stats});
+    ctx->save_for_backward({grad, own_scalars(stats)[0]});
     ctx->mark_non_differentiable({stats});
     return {loss, stats};
   }
@@ -770,19 +778,19 @@ struct ValueLossFn : public torch::autograd::Function<ValueLossFn> {
   }
 };
 
-// (loss, [sum(mask), the other statistics ...]) as scalars
+// (loss, [sum(mask), the other statistics ...]), the statistics as tensors of their own
 std::tuple<torch::Tensor, std::vector<torch::Tensor>> policy_loss_fn(const torch::Tensor& new_lp, const torch::Tensor& old_lp,
                                                                      const torch::Tensor& adv, const torch::Tensor& mask,
                                                                      const c10::optional<torch::Tensor>& ref_lp, double cliprange, double kl_coef) {
   c10::optional<torch::Tensor> r;
   if (ref_lp.has_value()) r = ref_lp->to(torch::kFloat32);
   auto out = PolicyLossFn::apply(new_lp.to(torch::kFloat32), old_lp.to(torch::kFloat32), adv.to(torch::kFloat32), mask, r, cliprange, kl_coef);
-  return {out[0], out[1].unbind()};
+  return {out[0], own_scalars(out[1])};
 }
 std::tuple<torch::Tensor, std::vector<torch::Tensor>> value_loss_fn(const torch::Tensor& vpred, const torch::Tensor& vold, const torch::Tensor& ret,
                                                                     const torch::Tensor& mask, double clip) {
   auto out = ValueLossFn::apply(vpred.to(torch::kFloat32), vold.to(torch::kFloat32), ret.to(torch::kFloat32), mask, clip);
-  return {out[0], out[1].unbind()};
+  return {out[0], own_scalars(out[1])};
 }
 
 void adamw_flat(torch::Tensor param, const torch::Tensor& grad, torch::Tensor m, torch::Tensor v, double lr, double beta1,
