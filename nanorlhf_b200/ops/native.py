@@ -243,9 +243,32 @@ def _count_loss(x):
     _count(2 if x.requires_grad and torch.is_grad_enabled() else 1)          # forward and, later, backward
 
 
+class _RecordedLossFn(torch.autograd.Function):
+    """A loss in a form that a tracer records as one operation; it does not see autograd functions in C++ and would keep their results as constants."""
+
+    @staticmethod
+    def forward(ctx, parts, x, *rest):
+        loss, grad, stats = parts(x.contiguous(), *[t.contiguous() if torch.is_tensor(t) else t for t in rest])
+        ctx.save_for_backward(grad, stats[0].clone())
+        ctx.mark_non_differentiable(stats)
+        return loss, stats
+
+    @staticmethod
+    def backward(ctx, g_loss, _g_stats):
+        grad, denom = ctx.saved_tensors
+        return (None, grad * (g_loss / denom)) + (None,) * (len(ctx.needs_input_grad) - 2)
+
+
+def _loss(name, x, *rest):
+    _count_loss(x)
+    if torch._C._get_tracing_state():
+        loss, stats = _RecordedLossFn.apply(getattr(ext(), name + "_parts"), x.float(), *[t.float() if torch.is_tensor(t) and t.is_floating_point() else t for t in rest])
+        return loss, stats.unbind()
+    return getattr(ext(), name)(x, *rest)
+
+
 def policy_loss_token(new_logp, old_logp, adv, mask, cliprange, ref_logp=None, kl_coef=0.0):
-    _count_loss(new_logp)
-    loss, stats = ext().policy_loss(new_logp, old_logp, adv, mask, ref_logp, float(cliprange), float(kl_coef))
+    loss, stats = _loss("policy_loss", new_logp, old_logp, adv, mask, ref_logp, float(cliprange), float(kl_coef))
     _, clipfrac, kl_masked, kl_all, ratio_all, ratio_masked, ref_all, ref_masked = stats
     out = {"clipfrac": clipfrac, "approxkl_masked": kl_masked, "approxkl_all": kl_all, "ratio_mean_all": ratio_all,
            "ratio_mean_masked": ratio_masked}
@@ -255,8 +278,7 @@ def policy_loss_token(new_logp, old_logp, adv, mask, cliprange, ref_logp=None, k
 
 
 def value_loss(vpred, values_old, returns, mask, cliprange_value):
-    _count_loss(vpred)
-    loss, stats = ext().value_loss(vpred, values_old, returns, mask, float(cliprange_value))
+    loss, stats = _loss("value_loss", vpred, values_old, returns, mask, float(cliprange_value))
     return loss, stats[1]
 
 
