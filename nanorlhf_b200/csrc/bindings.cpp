@@ -134,6 +134,18 @@ inline void check_tc_operand(const torch::Tensor& t, const char* name) {
               name, " must have unit inner stride and 16-byte aligned rows");
 }
 
+// ---- split-K of gemm_tc: into how many ranges the contraction of a product [M, K] x [K, N] is cut unless the caller says so ----
+// measured (bench/sampler_bench.py, profiles/skinny_gemm_split_sweep_r2.json): the last CTA's reduction reads `splits` partial tiles, so
+// beyond ~4 k-ranges the fix-up costs more than the shorter main loop saves, and work items past one wave (148) cost a second wave
+// (any N: the adapter-input gradient dA = t'^T x is [r, K_in] -- 12 or 24 tiles of a 6.6 k-long contraction)
+inline int split_block_n(int64_t N) { return N <= 64 ? 64 : 128; }
+inline int64_t split_tiles(int64_t M, int64_t N) { return ((M + 127) / 128) * ((N + split_block_n(N) - 1) / split_block_n(N)); }
+int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
+  const int64_t tiles = split_tiles(M, N), sms = num_sms();
+  const int64_t splits = std::min<int64_t>(std::min<int64_t>(sms / std::max<int64_t>(tiles, 1), (K + 63) / 64 / 4), 4);
+  return tiles * 2 <= sms && splits >= 2 ? splits : 1;
+}
+
 // D[M,N] = alpha * (opA(a) opB(b)^T + opA(a2) opB(b2)^T) (+bias) (GELU).
 //   a_mn = false: a is [M, K] (contraction contiguous);  a_mn = true: a is [K, M] (contraction = rows).  Same for b / N.
 //   Output: bf16 `out` [M, N] (allocated when absent) or, when `out_f32` is given, fp32 out_f32 (+)= result.
@@ -174,14 +186,11 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
   // ---- split-K: few output tiles, long contraction (rank-r projections, LoRA weight gradients) ----
   const bool bias_ok = !bias.has_value() || ((reinterpret_cast<uintptr_t>(bias->data_ptr()) & 15) == 0 && bias->is_contiguous());
   if (cg_req <= 0 && bn_req <= 0 && K2 == 0 && !f32 && bias_ok && act == 0 && (a_mn == b_mn || !a_mn) && splitk_req != 0) {
-    const int bn = N <= 64 ? 64 : 128;
-    const int64_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), num_kb = (K + 63) / 64;
+    const int bn = split_block_n(N);
+    const int64_t tiles = split_tiles(M, N), num_kb = (K + 63) / 64;
     const int sms = num_sms();
-    // measured (bench/sampler_bench.py, profiles/skinny_gemm_split_sweep_r2.json): the last CTA's reduction reads `splits` partial tiles, so
-    // beyond ~4 k-ranges the fix-up costs more than the shorter main loop saves, and work items past one wave (148) cost a second wave
-    int64_t splits = splitk_req > 0 ? splitk_req : std::min<int64_t>(std::min<int64_t>(sms / std::max<int64_t>(tiles, 1), num_kb / 4), 4);
-    // (any N: the adapter-input gradient dA = t'^T x is [r, K_in] -- 12 or 24 tiles of a 6.6 k-long contraction)
-    if (splitk_req > 0 || (tiles * 2 <= sms && splits >= 2)) {
+    int64_t splits = splitk_req > 0 ? splitk_req : auto_splits(M, N, K);
+    if (splitk_req > 0 || splits > 1) {
       splits = std::max<int64_t>(1, std::min<int64_t>(splits, num_kb));
       const int64_t per = (num_kb + splits - 1) / splits;
       splits = (num_kb + per - 1) / per;                                 // no empty k-range
@@ -1145,6 +1154,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_batched", &gemm_tc_batched, py::arg("a"), py::arg("b"), py::arg("out") = py::none(), py::arg("cg") = 0, py::arg("block_n") = 0);
   m.def("gemm_tc_swiglu", &gemm_tc_swiglu, py::arg("a"), py::arg("w_interleaved"), py::arg("out") = py::none(), py::arg("cg") = 0,
         py::arg("block_n") = 0);
+  m.def("gemm_tc_auto_splits", &auto_splits, py::arg("M"), py::arg("N"), py::arg("K"));
   m.def("gemm_tc_swiglu_pair", &gemm_tc_swiglu_pair, py::arg("x"), py::arg("wg"), py::arg("wu"), py::arg("tg") = py::none(),
         py::arg("tu") = py::none(), py::arg("bg") = py::none(), py::arg("bu") = py::none());
   m.def("add_layernorm", &add_layernorm);

@@ -486,8 +486,11 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           if (h == 1) release_acc();
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float g0 = __uint_as_float(g[j]), g1 = __uint_as_float(g[j + 1]);
-            pk[h * 16 + j / 2] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * __uint_as_float(u[j]), g1 / (1.f + __expf(-g1)) * __uint_as_float(u[j + 1]));
+            // gate and up are rounded as the two projections' own GEMMs leave them and combined as swiglu_kernel combines them: log-probabilities
+            // taken outside autograd round as the training forward does, the ratio of an unchanged policy stays 1
+            const float2 gr = unpack_bf16x2(pack_bf16x2(__uint_as_float(g[j]), __uint_as_float(g[j + 1])));
+            const float2 ur = unpack_bf16x2(pack_bf16x2(__uint_as_float(u[j]), __uint_as_float(u[j + 1])));
+            pk[h * 16 + j / 2] = pack_bf16x2(gr.x / (1.f + __expf(-gr.x)) * ur.x, gr.y / (1.f + __expf(-gr.y)) * ur.y);
           }
         }
         const int col = c.n_blk * (BN / 2) + group * 64;

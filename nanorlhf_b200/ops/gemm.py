@@ -177,15 +177,17 @@ def lora_linear_group(x, projs, scaling: float):
 
 
 def swiglu_linears(x, gate, up, scaling: float = 0.0):
-    """``silu(x Wg^T) * (x Wu^T)`` without the two projections in memory (no autograd), for any number of rows: two GEMMs and an activation
-    pass against one, 1536 -> 8960 features: 8 rows 32 / 19 us, 256 rows 28 / 17 (42 / 31 with adapters), 1000 rows 57 / 41 (73 / 57), 32 768
-    rows 1602 / 1213 (1531 / 1295); 4096 -> 1024 features, eight tiles only: 8 rows 29 / 25 us, 1024 rows 37 / 27. ``gate`` / ``up`` = (W, A | None, B | None) with a
-    LoRA term of ``scaling`` when A and B are given.  None when the fused GEMM does not take the call."""
+    """``silu(x Wg^T) * (x Wu^T)`` without the two projections in memory (no autograd).  Gate and up are rounded to bf16 before they are combined
+    and summed in the order of their own GEMMs, so that the result is bit for bit that of ``swiglu_pair(x Wg^T, x Wu^T)``, which the training
+    forward takes: log-probabilities of an unchanged policy have to agree.  ``gate`` / ``up`` = (W, A | None, B | None) with a LoRA term of
+    ``scaling`` when A and B are given.  None when the fused GEMM does not take the call."""
     (wg, ag, bg), (wu, au, bu) = gate, up
     x2 = _rows(x)
     if x2.shape[0] == 0 or not (supported(x, wg) and supported(x, wu)) or wg.shape != wu.shape or (ag is None) != (au is None):
         return None
     if ag is None:
+        if _native_mod.ext().gemm_tc_auto_splits(x2.shape[0], *wg.shape) > 1:
+            return None                                # their own GEMMs would add up ranges of the contraction: other sums
         _native_mod._count()
         y = _native_mod.ext().gemm_tc_swiglu_pair(x2, wg, wu)
     else:
