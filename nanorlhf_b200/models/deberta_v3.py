@@ -204,9 +204,12 @@ class _Intermediate(nn.Module):
         self.dense = Linear(cfg.hidden_size, cfg.intermediate_size)
 
     def forward(self, x):
-        # GEMM + bias + GELU epilogue (tcgen05 kernel, act=1).  24 571 x 4096 x 1024: a pass of its own costs 119 us, the epilogue
-        # 53 us: its eight warps form part of it behind the next tile's main loop
-        if _fused_inference(x) and x.shape[-1] % 8 == 0 and plain_module(self.dense, Linear):
+        # GEMM + bias + GELU epilogue (tcgen05 kernel, act=1), faster than GEMM and GELU at every number of rows measured: 1024 -> 4096, in a CUDA
+        # graph, 1 row 10.1 / 13.2 us, 128 rows 9.9 / 13.7 (there the GEMM alone adds up ranges of the contraction), 300 rows 11.1 / 12.3,
+        # 1024 rows 16.4 / 19.6, 24 571 rows 201 / 268 (its eight epilogue warps form part of the GELU behind the next tile's main loop);
+        # 64 -> 128, 1 row 7.2 / 7.7.  NANORLHF_DEBERTA_GELU_FUSED=0 keeps the two apart.
+        if (_fused_inference(x) and x.shape[-1] % 8 == 0 and os.environ.get("NANORLHF_DEBERTA_GELU_FUSED", "1") != "0"
+                and plain_module(self.dense, Linear)):
             return ops.linear(x, self.dense.weight, self.dense.bias, act=1)
         return F.gelu(self.dense(x))
 
