@@ -1,4 +1,4 @@
-"""PPO entry script with value-model initialisation (reference: /root/reference/PPO/ppo.py:78-399).
+"""PPO entry script with value-model initialisation (reference: PPO/ppo.py:78-399).
 
 Run:  python PPO/ppo.py [--key=value ...]      |      torchrun --nproc-per-node 8 PPO/ppo.py
 

@@ -3,7 +3,7 @@
 Run:  python RLOO/rloo.py [--key=value ...]          (1 GPU or CPU)
       torchrun --nproc-per-node 8 RLOO/rloo.py       (data parallel, one rank per B200)
 
-Mirrors /root/reference/RLOO/rloo.py:86-155: a ``RLOOConfig`` dataclass instantiated as ``training_args``,
+Mirrors the reference's RLOO/rloo.py:86-155: a ``RLOOConfig`` dataclass instantiated as ``training_args``,
 a ``reward_func(pmt_and_responses, eos_token)`` callback and a ``__main__`` that builds tokenizer / policy /
 ref policy / dataset and calls ``RLOOTrainer(...).train()``.  Models and data come from local directories when
 present and fall back to synthetic stand-ins otherwise (nanorlhf_b200/entry.py).

@@ -1,11 +1,11 @@
 """Same-box anchors: the *reference's dependency stack* (vLLM + HF transformers/flash-attn-2 + cuBLAS + NCCL +
 torch AdamW) timed phase by phase at the shapes of the headline benchmark -- with ZERO code from this repository.
 
-Why this exists: the reference itself (``/root/reference/GRPO/grpo.py``) cannot run on the benchmark box -- it is not
+Why this exists: the reference itself (``GRPO/grpo.py``) cannot run on the benchmark box -- it is not
 an installable package, imports trl / peft / accelerate (absent from the image and the offline wheelhouse) and pulls
-its models and datasets from the HF hub (no network); ``bench.py --impl reference`` therefore reports ``unavailable``
-(DESIGN.md section 7).  What *can* be measured honestly is every library call the reference's update is made of
-(/root/reference/GRPO/grpo_trainer.py): each phase below names the reference lines it stands for and is deliberately
+its models and datasets from the HF hub (no network); ``bench.py --impl reference`` therefore reports ``unavailable``.
+What *can* be measured honestly is every library call the reference's update is made of
+(GRPO/grpo_trainer.py): each phase below names the reference lines it stands for and is deliberately
 CHARITABLE to the reference -- no CPU<->GPU model swaps, no disk round trip of the weights, no LoRA adapter GEMMs,
 no ``empty_cache()`` storms -- so the resulting per-phase times are lower bounds of what the reference would need.
 
@@ -116,7 +116,7 @@ def cuda_time(fn, iters=3, warm=3):
 
 
 # ---------------------------------------------------------------------------------------------------------
-# phase: rollout  (reference: vllm_generate, /root/reference/GRPO/grpo_trainer.py:122-166)
+# phase: rollout  (reference: vllm_generate, GRPO/grpo_trainer.py:122-166)
 # ---------------------------------------------------------------------------------------------------------
 def phase_rollout(args):
     path = model_dir()

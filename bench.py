@@ -1,13 +1,12 @@
-"""Headline benchmark: GRPO episodes/s on Qwen2.5-1.5B (BASELINE.json config 2).
+"""Headline benchmark: GRPO episodes/s on Qwen2.5-1.5B.
 
   python bench.py --gpus N --steps K --warmup W            (N > 1: launched by torchrun, one rank per GPU)
-  python bench.py --impl reference ...                      (the unmodified reference; see DESIGN.md)
+  python bench.py --impl reference ...                      (the unmodified reference)
 
 Batch: the default is ``--mini-batches 8`` = 4 x 8 x 8 = 256 prompts (x 4 samples = 1024 sequences) per rank per update
--- the reference's arithmetic with ``num_mini_batches`` halved from 16 -- so that the driver's ``--steps 20 --warmup 5`` (25 full
+-- the reference's arithmetic with ``num_mini_batches`` halved from 16 -- so that ``--steps 20 --warmup 5`` (25 full
 updates) finishes inside its per-run limit at every N; ``global_batch`` in ``config`` says what was run and is the same for
-the 1-GPU bench and the 1/2/4/8 scaling runs.  ``--mini-batches 16`` is the reference's own 512 prompts per rank
-(BASELINE.md has that number too).
+the 1-GPU bench and the 1/2/4/8 scaling runs.  ``--mini-batches 16`` is the reference's own 512 prompts per rank.
 
 One *step* = one full GRPO update through the public API (``GRPOTrainer.train_one_update``): in-process
 rollout of ``prompts_per_rank x 4`` samples with up to 1500 response tokens on the sm_100a sampler,
@@ -31,8 +30,8 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# The only throughput the reference publishes: README.md:36 "~1 s/episode" on 1 x A100-40G with real weights (BASELINE.md
-# section 1).  Different hardware, real (EOS-terminated, shorter) responses: context, not a like-for-like ratio.
+# The only throughput the reference publishes: README.md:36 "~1 s/episode" on 1 x A100-40G with real weights.
+# Different hardware, real (EOS-terminated, shorter) responses: context, not a like-for-like ratio.
 BASELINE_EPISODES_PER_S = 1.0
 
 
@@ -203,7 +202,7 @@ def main():
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": value / BASELINE_EPISODES_PER_S,
             "vs_baseline_note": "denominator = the reference README's ~1 episode/s on 1 x A100-40G with real weights (its only "
-                                "published throughput); not a same-box ratio -- see BASELINE.md section 2 for same-box anchors",
+                                "published throughput); not a same-box ratio",
             "dtype": "bf16",
             "data": "synthetic hh-rlhf-shaped token prompts; random-init weights (no network)",
             "impl": "ours",

@@ -1,5 +1,5 @@
 #!/usr/bin/env bash
-# Host ASAN + UBSAN build of the sampler's C++ runtime (SURVEY.md 5.2); CPU only.  Also run by tests/test_runtime_cpp.py.
+# Host ASAN + UBSAN build of the sampler's C++ runtime; CPU only.  Also run by tests/test_runtime_cpp.py.
 set -eu
 cd "$(dirname "$0")/../nanorlhf_b200/csrc"
 out="${TMPDIR:-/tmp}/nrl_runtime_asan_$$"

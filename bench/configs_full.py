@@ -1,4 +1,4 @@
-"""Full-size runs of the other BASELINE.json configurations (3, 4, 5) through the public trainer API.
+"""Full-size runs of the other configurations (PPO with value initialisation, 7B sparse GRPO, RLOO / ReMax / RAFT with host tiering) through the public trainer API.
 
   python bench/configs_full.py [ppo] [r1] [rloo] [remax] [raft]           (one GPU)
   torchrun --nproc-per-node N --master-addr 127.0.0.1 bench/configs_full.py ...   (data parallel)

@@ -1,4 +1,4 @@
-"""Reduced-size smoke runs of the other BASELINE.json configs on one B200 (writes gpurun_out/configs_smoke.json):
+"""Reduced-size smoke runs of the other configurations on one B200 (writes gpurun_out/configs_smoke.json):
   config 3  Qwen2.5-1.5B PPO with value-model initialisation, bf16
   config 4  Qwen2.5-7B sparse-GRPO (r1-v0 style) with rule reward, dynamic mini-batching, fp8 rollout
   config 5  Qwen2.5-1.5B RLOO / ReMax / RAFT with host-offloaded ref + optimizer state

@@ -142,7 +142,7 @@ def main():
               file=sys.stderr, flush=True)
     # one verdict for the whole job (every rank exits with the same code), then an orderly teardown: drop the symmetric
     # buffers while the process group still exists, barrier, destroy the group, and leave without running the
-    # interpreter-exit destructors of the symmetric-memory handles (round 1: ranks 1-7 exited 1 after printing results)
+    # interpreter-exit destructors of the symmetric-memory handles (ranks 1-7 exited 1 after printing results without it)
     verdict = torch.tensor([1 if all(checks.values()) else 0], device=dev)
     comm.all_reduce_(verdict, "min")
     ok = bool(verdict.item())

@@ -1,5 +1,5 @@
 #!/usr/bin/env bash
-# compute-sanitizer targets (SURVEY.md 5.2): memcheck by default, `bench/sanitize.sh racecheck|synccheck|initcheck` for the rest.
+# compute-sanitizer targets: memcheck by default, `bench/sanitize.sh racecheck|synccheck|initcheck` for the rest.
 # One tiny launch per kernel family (bench/sanitize_smoke.py); the report lands in gpurun_out/sanitizer_<tool>.log.
 set -u
 tool="${1:-memcheck}"

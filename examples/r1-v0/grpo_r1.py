@@ -1,13 +1,13 @@
 """r1-v0: "sparse GRPO" + dynamic mini-batching with a rule-based math reward and 8000-token responses.
 
-Reference: /root/reference/examples/r1-v0/grpo_r1.py (config :96-155, reward :250-273, accuracy probe
+Reference: examples/r1-v0/grpo_r1.py (config :96-155, reward :250-273, accuracy probe
 :276-341) and grpo_r1_trainer.py.  Same surface: ``GRPOConfig`` / ``training_args``,
 ``reward_func(pmt_and_responses, responses_ids, tokenizer)``, ``accuracy_func(model, args) -> float`` and
 ``GRPOTrainer(..., accuracy_func=...)``; the trainer is the data-parallel-safe ``SparseGRPOTrainer``.
 
 Run:  python examples/r1-v0/grpo_r1.py [--key=value ...]   |   torchrun --nproc-per-node 8 examples/r1-v0/grpo_r1.py
 Datasets (MetaMathQA for training, MATH-500 for the accuracy probe) are read from local directories when
-present; otherwise synthetic arithmetic problems with exact answers stand in (no network on the GPU box).
+present; otherwise synthetic arithmetic problems with exact answers stand in (no network).
 """
 import os
 import sys

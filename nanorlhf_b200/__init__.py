@@ -1,2 +1,2 @@
-"""nanoRLHF-B200: a Blackwell-native RLHF training engine (see DESIGN.md / SURVEY.md)."""
+"""nanoRLHF-B200: a Blackwell-native RLHF training engine."""
 __version__ = "0.1.0"

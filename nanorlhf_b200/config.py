@@ -2,11 +2,11 @@
 
 The reference subclasses trl's ``PPOConfig`` (itself an HF ``TrainingArguments``) once per
 algorithm and instantiates it at module import inside the entry script
-(/root/reference/GRPO/grpo.py:86-155, PPO/ppo.py:78-166).  trl / HF ``Trainer`` are not
-dependencies here, so ``RLConfig`` owns every field the reference consumes (SURVEY.md section 2.2
-``PPOConfig`` row and App. A) with the same names and defaults, promotes the constants the
+(GRPO/grpo.py:86-155, PPO/ppo.py:78-166).  trl / HF ``Trainer`` are not
+dependencies here, so ``RLConfig`` owns every field the reference consumes
+with the same names and defaults, promotes the constants the
 reference hard-codes (top-p, token budgets, scratch dirs ...) to fields, and adds
-``--key=value`` CLI / ``NANORLHF_KEY`` env overrides (the reference has neither, SURVEY.md 5.6).
+``--key=value`` CLI / ``NANORLHF_KEY`` env overrides (the reference has neither).
 """
 from __future__ import annotations
 

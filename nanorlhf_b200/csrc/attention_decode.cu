@@ -12,7 +12,7 @@
 //   * each warp streams its own pages with private online-softmax state; warps (and optional
 //     KV splits) are merged once at the end.
 // Reference path replaced: vLLM PagedAttention / FlashInfer decode inside llm.generate
-// (/root/reference/GRPO/grpo_trainer.py:142).
+// (GRPO/grpo_trainer.py:142).
 #include "common.cuh"
 #include "kernels.h"
 

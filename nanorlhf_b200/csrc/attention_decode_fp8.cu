@@ -1,8 +1,8 @@
 // fp8 (e4m3) paged KV cache: page writer + decode attention that reads HALF the bytes of the bf16 path.
 //
 // Decode attention is the dominant cost of the rollout and it is HBM-bound (attention_decode.cu runs at the copy
-// roofline), so the only way to make it faster is to move fewer bytes.  Round 1 had an fp8 variant that dequantised
-// whole pages through shared memory and was issue-bound (slower than bf16).  This version dequantises IN REGISTERS,
+// roofline), so the only way to make it faster is to move fewer bytes.  An fp8 variant that dequantised
+// whole pages through shared memory was issue-bound (slower than bf16).  This version dequantises IN REGISTERS,
 // on the operand fragments of the tensor-core instruction itself:
 //
 //   * K page  [16 tokens][128 d] e4m3 (2 KB);  V page stored TRANSPOSED [128 d][16 tokens] e4m3 (2 KB);
@@ -20,7 +20,7 @@
 //     bf16 kernel; 3 CTAs per SM (68 KB each) keep ~200 KB of loads in flight per SM.
 //
 // Reference path replaced: vLLM PagedAttention / FlashInfer decode inside llm.generate
-// (/root/reference/GRPO/grpo_trainer.py:142; SURVEY.md section 2.5 K2, "fp8 KV option").
+// (GRPO/grpo_trainer.py:142).
 #include "common.cuh"
 #include "kernels.h"
 

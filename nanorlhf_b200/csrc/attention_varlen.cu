@@ -10,8 +10,8 @@
 //   * REL_BIAS: score += A[i, c(i-j)] + B[j, c(i-j)] with c = log-bucketed relative position: the c2p and
 //     p2c terms of DeBERTa's disentangled attention, gathered from per-row / per-key tables that stay in
 //     shared memory, so the three score terms are fused in one flash-style pass
-//     (reference path: HF eager DeBERTa, /root/reference/GRPO/grpo.py:189-192).
-// These replace flash-attn-2 (attn_implementation="flash_attention_2", /root/reference/GRPO/grpo.py:219).
+//     (reference path: HF eager DeBERTa, GRPO/grpo.py:189-192).
+// These replace flash-attn-2 (attn_implementation="flash_attention_2", GRPO/grpo.py:219).
 #include "common.cuh"
 #include "kernels.h"
 

@@ -3,7 +3,7 @@
 Every ``.cu`` is compiled by nvcc for ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` (kernel
 translation units do not include torch headers, so they compile in seconds); ``bindings.cpp`` /
 ``runtime.cpp`` are compiled by g++ against the torch headers; everything is linked into
-``nanorlhf_b200/_C.so`` (git-ignored, but it travels to the GPU box with the gpurun snapshot).
+``nanorlhf_b200/_C.so`` (git-ignored, built in-tree).
 nvcc cross-compiles without a GPU, so this is also the CPU-side "does it build" check.
 """
 from __future__ import annotations

@@ -1,7 +1,7 @@
 // K-AR: data-parallel gradient all-reduce FUSED with the AdamW update, over NVLink symmetric memory.
 //
-// Baseline being replaced (SURVEY.md N3/K17/K18): DDP's bucketed NCCL all-reduce of the bf16 gradients
-// followed by a separate torch AdamW step (/root/reference/GRPO/grpo_trainer.py:690-692).
+// Baseline being replaced: DDP's bucketed NCCL all-reduce of the bf16 gradients
+// followed by a separate torch AdamW step (GRPO/grpo_trainer.py:690-692).
 //
 // Every rank keeps its flat gradient buffer and flat parameter buffer in symmetric memory (mapped into
 // all peers).  One kernel per optimizer step, rank r owns elements [lo, lo+n):

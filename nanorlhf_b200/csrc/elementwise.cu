@@ -1,8 +1,7 @@
 // Bandwidth-bound fused elementwise / row-reduce kernels (K4): RMSNorm (+residual), RoPE, SwiGLU.
 // All 128-bit vectorised, one pass over the data, fp32 math, bf16 I/O.
 // Reference equivalents: HF eager RMSNorm / rotate_half RoPE / SiLU*mul in the training path and
-// vLLM's fused_add_rms_norm / rotary_embedding / silu_and_mul in the rollout path
-// (SURVEY.md section 2.5 K4).
+// vLLM's fused_add_rms_norm / rotary_embedding / silu_and_mul in the rollout path.
 #include "common.cuh"
 #include "kernels.h"
 

@@ -17,7 +17,7 @@
 //   EPI_DLOGITS K-LP backward: dZ = (onehot(target) - softmax(z)) * g / T in bf16 via TMA store
 //
 // Reference call sites this replaces: cuBLAS GEMMs behind every nn.Linear and the
-// logits -> /T -> log_softmax -> gather chain (/root/reference/GRPO/grpo_trainer.py:543-549,652-660).
+// logits -> /T -> log_softmax -> gather chain (GRPO/grpo_trainer.py:543-549,652-660).
 #include "common.cuh"
 #include "gemm_sm100.h"
 

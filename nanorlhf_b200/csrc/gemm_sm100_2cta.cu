@@ -1,4 +1,4 @@
-// EXPERIMENTAL (opt-in: NRL_GEMM_2CTA=1; not yet validated on hardware -- written at the end of round 1 when the GPU
+// EXPERIMENTAL (opt-in: NRL_GEMM_2CTA=1; not yet validated on hardware -- written when the GPU
 // budget was spent; first item of the next round's GPU time).
 //
 // 2-CTA (cta_group::2) variant of the bf16 GEMM  D[M,N] = A[M,K] * B[N,K]^T (+bias, +GELU):

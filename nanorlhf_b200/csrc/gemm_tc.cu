@@ -3,7 +3,7 @@
 //   D[M,N] = alpha * ( opA(A) . opB(B)^T  +  A2 . B2^T )  (+ bias[N]) (GELU)          bf16 in, fp32 accumulate
 //
 // One kernel template covers what the reference gets from cuBLAS behind every nn.Linear / peft LoRA layer / torch.bmm
-// (/root/reference/GRPO/grpo_trainer.py:543-556,652-660; GRPO/grpo.py:189-192,228-243):
+// (GRPO/grpo_trainer.py:543-556,652-660; GRPO/grpo.py:189-192,228-243):
 //
 //   * CG = 1 | 2      cta_group::1 (one CTA, 128 x BN tile) or cta_group::2 (a CTA pair of one TPC computes a 256 x BN
 //                     tile; each CTA TMA-loads its own 128 rows of A and only HALF of the B tile, one elected thread of
@@ -185,7 +185,7 @@ NRL_DEVICE void tma_store_3d(const CUtensorMap* m, const void* smem_src, int c0,
 
 // FP8: A and B are e4m3 bytes, K-major (a 128-byte swizzle row = 128 contraction elements), the MMA is kind::f8f6f4
 // (K = 32 per instruction, twice the bf16 rate) and the epilogue applies the per-row (token) and per-column (output
-// channel) dequantisation scales -- the sampler's fp8 rollout GEMMs (north star: fp8 tcgen05 GEMM in the decoder).
+// channel) dequantisation scales -- the sampler's fp8 rollout GEMMs.
 // PAIR (CTA pairs, BN = 256): act = silu(x Wg^T) * (x Wu^T) from two separate weights.  The leader loads 128 rows of the gate's
 // weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
 // columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.

@@ -3,7 +3,7 @@
 //   K-LOSS policy_loss       PPO-clip (+ GRPO k3-KL) forward + gradient + all statistics in ONE pass
 //          value_loss        clipped value loss forward + gradient
 //   K18    adamw_flat        AdamW over flat bf16 parameter / gradient buffers with fp32 or bf16 moments
-// Reference: the python time-step loop (/root/reference/GRPO/grpo_trainer.py:611-617, PPO/ppo_trainer.py:
+// Reference: the python time-step loop (GRPO/grpo_trainer.py:611-617, PPO/ppo_trainer.py:
 // 688-697), ~15 elementwise launches per micro-batch (:662-688) and torch AdamW (:692).
 #include <cooperative_groups.h>
 

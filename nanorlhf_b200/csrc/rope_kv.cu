@@ -1,4 +1,4 @@
-// Decode-step fusion of RoPE(q), RoPE(k) and the KV page write ("RoPE fused on K at write").
+// Decode-step fusion of RoPE(q), RoPE(k) and the KV page write.
 //
 // The decode step used to launch three kernels per layer for this (rope on q, rope on k, page writer); at 1024 sequences
 // each moves a few MB, i.e. they are launch-latency sized.  Here ONE warp handles one (sequence, head) of the fused qkv

@@ -1,6 +1,6 @@
 // Host-side sampler runtime (C++): paged-KV block manager + continuous-batching scheduler.
 // Replaces the scheduler / block-manager half of the vLLM engine the reference boots per rollout
-// (/root/reference/GRPO/grpo_trainer.py:141-142; SURVEY.md section 2.6 first row).
+// (GRPO/grpo_trainer.py:141-142).
 #pragma once
 #include <pybind11/pybind11.h>
 

@@ -1,4 +1,4 @@
-// Host-sanitizer target (SURVEY.md 5.2): the sampler's C++ runtime (paged-KV BlockManager + continuous-batching
+// Host-sanitizer target: the sampler's C++ runtime (paged-KV BlockManager + continuous-batching
 // Scheduler) driven through a randomized admit / advance / finish / preempt workload under
 //   g++ -std=c++17 -O1 -g -fsanitize=address,undefined -DNRL_RUNTIME_NO_PYBIND runtime_asan_test.cpp
 // Invariants checked every step: no page is owned twice, free + owned == total, reference counts match the tables.

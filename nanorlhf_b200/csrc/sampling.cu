@@ -16,7 +16,7 @@
 //   sample_top_p_kernel        the streaming histogram kernel described above (fp32 logits, rows that are not 16-byte sliceable,
 //                              larger vocabularies, top_p < 0.5): one CTA per row, every pass re-reads the row through L2.
 // Reference: vLLM SamplingParams(temperature, top_p=0.95, seed=...) in vllm_generate
-// (/root/reference/GRPO/grpo_trainer.py:127) and the T=0 greedy pass of ReMax (remax_trainer.py:167).
+// (GRPO/grpo_trainer.py:127) and the T=0 greedy pass of ReMax (remax_trainer.py:167).
 #include <curand_kernel.h>
 
 #include <algorithm>

@@ -1,7 +1,7 @@
 """Shared plumbing of the per-algorithm entry scripts (GRPO/grpo.py ...).
 
 The reference's scripts download models / datasets from the HF hub at import
-(/root/reference/GRPO/grpo.py:159,209-224,247).  The GPU box has no network, so every loader here
+(GRPO/grpo.py:159,209-224,247).  There may be no network, so every loader here
 takes a local directory when one exists and otherwise falls back to a *synthetic* stand-in of the same
 shape (random-init weights of the named architecture, byte-level tokenizer, hh-rlhf-shaped prompts) and
 says so on stdout.  ``NANORLHF_MODEL_SHAPE`` (tiny | 125m | 1.5b | 7b) overrides the architecture.

@@ -2,7 +2,7 @@
 
 The reference loads ``OpenAssistant/reward-model-deberta-v3-large-v2`` through HF
 ``AutoModelForSequenceClassification`` in fp32 and swaps it GPU<->CPU around every scoring pass
-(/root/reference/GRPO/grpo.py:159-198).  This is a from-scratch module with the HF
+(GRPO/grpo.py:159-198).  This is a from-scratch module with the HF
 parameter names (``deberta.encoder.layer.N.attention.self.query_proj.weight`` ...) so the published
 checkpoint loads, running in bf16 and staying resident in HBM.
 

@@ -1,4 +1,4 @@
-"""safetensors state-dict I/O (HF checkpoint format library; SURVEY.md App. C compatibility)."""
+"""safetensors state-dict I/O (HF checkpoint format library)."""
 from __future__ import annotations
 
 import torch

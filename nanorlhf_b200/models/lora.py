@@ -2,9 +2,9 @@
 
 The reference wraps the policy with ``peft.get_peft_model(policy, LoraConfig(r=64, alpha=16,
 target_modules=[q,k,v,o,gate,up,down]_proj, modules_to_save=[embed_tokens, lm_head, score]))``
-(/root/reference/GRPO/grpo.py:228-243) and merges with ``merge_and_unload`` on the CPU before
-every rollout (/root/reference/GRPO/grpo_trainer.py:131-138).  peft is not a dependency here.
-Semantics owned by this file (SURVEY.md section 2.2):
+(GRPO/grpo.py:228-243) and merges with ``merge_and_unload`` on the CPU before
+every rollout (GRPO/grpo_trainer.py:131-138).  peft is not a dependency here.
+Semantics owned by this file:
 
 * ``y = W x + (alpha/r) * B (A x)``; A ~ kaiming-uniform, B = 0 (so step 0 equals the base model);
 * ``modules_to_save`` modules become fully trainable (tied embeddings are un-tied by copying);

@@ -1,8 +1,8 @@
 """Qwen2 / Qwen2.5 decoder, packed-varlen, built on the op layer.
 
 The reference reaches this model through ``transformers.AutoModelForCausalLM`` +
-flash-attn-2 (/root/reference/GRPO/grpo.py:218-224) and, for the PPO critic,
-``AutoModelForSequenceClassification(num_labels=1)`` (/root/reference/PPO/ppo.py:280-287).
+flash-attn-2 (GRPO/grpo.py:218-224) and, for the PPO critic,
+``AutoModelForSequenceClassification(num_labels=1)`` (PPO/ppo.py:280-287).
 This is a from-scratch module with the same parameter names as the HF checkpoint format
 (``model.layers.N.self_attn.q_proj.weight`` ...) so safetensors checkpoints round-trip, but with a
 B200-first execution model:
@@ -53,7 +53,7 @@ class Qwen2Config:
         if self.head_dim is None:
             self.head_dim = self.hidden_size // self.num_attention_heads
 
-    # ---- named shapes (SURVEY.md App. E) ---------------------------------------------------
+    # ---- named shapes ---------------------------------------------------
     @classmethod
     def qwen2_5_1_5b(cls, **kw):
         return cls(vocab_size=151936, hidden_size=1536, intermediate_size=8960, num_hidden_layers=28,
@@ -270,7 +270,7 @@ class Qwen2PreTrained(nn.Module):
 
     @classmethod
     def from_config(cls, cfg: Qwen2Config, torch_dtype=torch.bfloat16, device="cpu", seed: Optional[int] = None):
-        """Random-init (there is no network on the GPU box: SURVEY.md environment facts)."""
+        """Random-init (for machines without a network)."""
         dev = torch.device(device)
         # Billion-parameter models are initialised ON the GPU (seconds instead of ~half a minute of CPU normal_() per
         # model -- start-up time counts against the benchmark driver's per-run limit); small models keep the CPU generator
@@ -308,7 +308,7 @@ class Qwen2ForCausalLM(Qwen2PreTrained):
             self.lm_head.weight = self.model.embed_tokens.weight
 
     def untie_weights(self):
-        """Give lm_head its own storage (peft ``modules_to_save`` semantics, SURVEY.md section 2.2)."""
+        """Give lm_head its own storage (peft ``modules_to_save`` semantics)."""
         if self.lm_head.weight is self.model.embed_tokens.weight:
             self.lm_head.weight = nn.Parameter(self.model.embed_tokens.weight.detach().clone())
 

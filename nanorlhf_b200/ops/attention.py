@@ -4,7 +4,7 @@ Native kernels: ``csrc/attention_fwd_tc.cu`` / ``csrc/attention_bwd_tc.cu`` (tcg
 TMA-fed, warp-specialised; head_dim 128); other head sizes and ``NANORLHF_ATTN_TC=0`` use
 ``csrc/attention_varlen.cu`` (mma.sync flash attention, also the oracle of the tcgen05 kernels).  ``NANORLHF_ATTN=flash_attn`` runs the flash-attn
 library instead; that path is the *baseline* this framework replaces
-(reference: attn_implementation="flash_attention_2", /root/reference/GRPO/grpo.py:219).
+(reference: attn_implementation="flash_attention_2", GRPO/grpo.py:219).
 """
 from __future__ import annotations
 

@@ -1,8 +1,8 @@
 """Linear layers of the training / log-prob / reward paths on the general tcgen05 GEMM (csrc/gemm_tc.cu).
 
 What the reference runs here is cuBLAS behind ``nn.Linear`` plus peft's LoRA wrapper -- per projection and direction a base
-GEMM, two adapter GEMMs and an add over the ``[tokens, out]`` result (/root/reference/GRPO/grpo.py:228-243; call sites
-/root/reference/GRPO/grpo_trainer.py:543-556,652-660).  Here every contraction of the decoder is one launch of the same
+GEMM, two adapter GEMMs and an add over the ``[tokens, out]`` result (GRPO/grpo.py:228-243; call sites
+GRPO/grpo_trainer.py:543-556,652-660).  Here every contraction of the decoder is one launch of the same
 sm_100a kernel, with the operand "major-ness" chosen so that no transposed copy is ever made:
 
 =================  =========================================  =====================================================

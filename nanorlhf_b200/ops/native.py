@@ -1,8 +1,8 @@
 """CUDA backend of the op layer: thin autograd wrappers over ``nanorlhf_b200/_C.so``.
 
 ``load()`` imports the in-tree extension (built by ``python -m nanorlhf_b200.csrc.build``).  It is
-not JIT-compiled at import: the ``.so`` must travel with the source tree (gpurun snapshot), and a
-missing build on a GPU box is a hard error (ops/__init__.py), never a silent PyTorch fallback.
+not JIT-compiled at import: the ``.so`` must travel with the source tree, and a
+missing build on a machine with a GPU is a hard error (ops/__init__.py), never a silent PyTorch fallback.
 """
 from __future__ import annotations
 

@@ -2,7 +2,7 @@
 
 These are (a) the CPU / plumbing backend (``NANORLHF_BACKEND=torch``) and (b) the oracle the
 CUDA kernels in ``csrc/`` are tested against (tests/test_kernels_gpu.py).  Everything here is
-written from the behaviour described in SURVEY.md section 3.5; citations point at the reference
+written from the reference's behaviour; citations point at the
 call sites the semantics come from.
 """
 from __future__ import annotations
@@ -136,7 +136,7 @@ def lmhead_logprob_top_p(hidden: torch.Tensor, weight: torch.Tensor, targets: to
                          chunk: int = 1024) -> Tuple[torch.Tensor, torch.Tensor]:
     """Log-probs under the distribution the sampler actually draws from: softmax(z / T) restricted to its top-p nucleus and
     renormalised -- ``logp[t] = z_y - logsumexp_{v in nucleus(t)} z_v``.  The reference samples with top_p = 0.95 but scores
-    with the full softmax (/root/reference/GRPO/grpo_trainer.py:127 vs :547-549); this is the consistent variant
+    with the full softmax (GRPO/grpo_trainer.py:127 vs :547-549); this is the consistent variant
     (``logprob_top_p_consistent=True``).  Plain autograd over [chunk, V] logits: an experimental switch, not a fast path.  The
     nucleus is treated as a constant set; a target outside it (never produced by the sampler) gets the full-softmax value.
     Returns (logp [T], entropy of the truncated distribution [T])."""

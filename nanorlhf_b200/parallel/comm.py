@@ -1,8 +1,7 @@
 """Control-plane communicator.
 
-The reference never calls ``torch.distributed`` directly -- accelerate does (SURVEY.md section 2.4,
-call sites N1-N5).  Here one small ``Comm`` object owns the process group.  It is used for
-rendezvous, barriers, the tiny packed metrics reduction (N4 -> one all-reduce instead of ten
+The reference never calls ``torch.distributed`` directly -- accelerate does.  Here one small ``Comm`` object owns the process group.  It is used for
+rendezvous, barriers, the tiny packed metrics reduction (one all-reduce instead of ten
 all-gathers) and as the *baseline* implementation (``comm="nccl"``) of the two bandwidth paths;
 the product paths are the fused kernels in ``parallel/fused_allreduce.py`` (K-AR) and
 ``parallel/weight_sync.py`` (K-BC) which run over symmetric memory.
@@ -103,7 +102,7 @@ class Comm:
 
     def broadcast_module_(self, module, src: int = 0, only_frozen: bool = False) -> int:
         """Make a module's parameters and buffers identical to rank ``src``'s (what DDP's constructor does for everything
-        it wraps, SURVEY.md N2).  Tensors are coalesced per dtype into flat staging buffers so a 1.5B model is a handful
+        it wraps).  Tensors are coalesced per dtype into flat staging buffers so a 1.5B model is a handful
         of NCCL broadcasts.  ``only_frozen`` skips trainable parameters (the optimizer broadcasts its flat buffers itself).
         Returns the number of bytes broadcast."""
         if self.world_size == 1 or module is None:
@@ -134,7 +133,7 @@ class Comm:
         return total
 
     def reduce_scalars(self, values: Dict[str, float], op: str = "mean") -> Dict[str, float]:
-        """Pack a dict of python floats into ONE vector and all-reduce it (SURVEY.md K23)."""
+        """Pack a dict of python floats into ONE vector and all-reduce it."""
         if self.world_size == 1:
             return dict(values)
         keys = sorted(values)

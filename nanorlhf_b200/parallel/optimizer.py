@@ -1,9 +1,9 @@
 """Flat-buffer AdamW with the data-parallel gradient reduction folded into ``step()``.
 
 Reference: HF ``Trainer.create_optimizer`` -> ``torch.optim.AdamW`` over ``requires_grad`` params
-(/root/reference/GRPO/grpo_trainer.py:258), DDP's bucketed NCCL all-reduce on the accumulation
-boundary (:690, SURVEY.md N3) and a separate AdamW step (:692, K18); PPO overrides
-``create_optimizer`` for two learning rates (/root/reference/PPO/ppo_trainer.py:341-402).
+(GRPO/grpo_trainer.py:258), DDP's bucketed NCCL all-reduce on the accumulation
+boundary (:690) and a separate AdamW step (:692, K18); PPO overrides
+``create_optimizer`` for two learning rates (PPO/ppo_trainer.py:341-402).
 
 B200-first design:
 
@@ -17,7 +17,7 @@ B200-first design:
   peer's parameter buffer -- reduce-scatter + Adam + all-gather in one kernel, moments sharded
   ZeRO-1 style.  ``comm="nccl"`` keeps the baseline: ``dist.all_reduce`` then a local step.
 * moments are fp32 by default (``optimizer_state_dtype="bf16"`` reproduces the reference's
-  bf16-moment behaviour, SURVEY.md 7.4);
+  bf16-moment behaviour);
 * bf16 parameters get an **fp32 master copy of the owned shard** next to the moments (``master_weights``): at
   the shipped lr = 6e-6 an Adam step (~lr) is far below half a bf16 ulp of a typical weight (|w| ~ 0.02 ->
   ulp 1.2e-4), so without it ``round(p - lr * u)`` == p and training silently stalls.  peft keeps adapter
@@ -126,14 +126,14 @@ class FusedAdamW(torch.optim.Optimizer):
         if self._fused is not None:
             self._fused.register([f for f in self._flats if f is not None])
         if self.world > 1:
-            # replicas must start identical (DDP broadcasts rank 0's parameters at construction, SURVEY.md N2);
+            # replicas must start identical (DDP broadcasts rank 0's parameters at construction);
             # one flat broadcast per group over the bootstrap process group
             for f in self.flats:
                 comm.broadcast_(f.param, 0)
 
     # ---- comm="nccl": DDP-style bucketed all-reduce overlapped with the backward -----------------
     def enable_bucket_overlap(self, bucket_bytes: int = 25 << 20) -> bool:
-        """What DDP's reducer does for the reference (/root/reference/GRPO/grpo_trainer.py:690): gradients are
+        """What DDP's reducer does for the reference (GRPO/grpo_trainer.py:690): gradients are
         grouped into ~25 MB buckets in reverse parameter order (the order the backward produces them); on the micro-step the
         trainer arms with ``arm_overlap()`` a post-accumulate hook per parameter counts its bucket down and the bucket's
         all-reduce is issued asynchronously the moment it is complete, while the backward of the earlier layers still runs.

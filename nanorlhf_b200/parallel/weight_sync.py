@@ -1,8 +1,8 @@
 """K-BC: policy -> sampler weight refresh, on device, no filesystem.
 
-Reference (SURVEY.md N6 / K6): every rollout the reference saves the adapter, reloads the base model
+Reference: every rollout the reference saves the adapter, reloads the base model
 on the CPU, runs ``merge_and_unload`` there, writes the merged model to /data/temp_vllm_model and
-boots vLLM from it (/root/reference/GRPO/grpo_trainer.py:131-141): 3.1 GB written+read twice plus
+boots vLLM from it (GRPO/grpo_trainer.py:131-141): 3.1 GB written+read twice plus
 an engine boot per update.
 
 Here the sampler keeps a fused arena (qkv / gate_up concatenated) and ``refresh_sampler_arena``

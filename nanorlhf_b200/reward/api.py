@@ -1,9 +1,9 @@
 """Reward callback contract + simple rule rewards.
 
-Contract (reference: /root/reference/GRPO/grpo.py:162): ``reward_func(pmt_and_responses: list[str],
+Contract (reference: GRPO/grpo.py:162): ``reward_func(pmt_and_responses: list[str],
 eos_token: str) -> FloatTensor[len]`` -- the trainer hands over decoded prompt+response strings.
 A callback may set ``accepts_ids = True`` to receive ``(queries, responses, tokenizer)`` id tensors
-instead and skip the decode -> parse round trip (tokenizers row).
+instead and skip the decode -> parse round trip.
 """
 from __future__ import annotations
 
@@ -26,7 +26,7 @@ def split_prompt_response(text: str, eos_token: str):
 
 
 class ConstantReward:
-    """Plumbing reward: every sample scores ``value`` (BASELINE.json config 1)."""
+    """Plumbing reward: every sample scores ``value``."""
 
     def __init__(self, value: float = 1.0):
         self.value = value

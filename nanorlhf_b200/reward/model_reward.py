@@ -1,6 +1,6 @@
 """Model-based reward callback (DeBERTa-v3 reward model).
 
-Reference behaviour (/root/reference/GRPO/grpo.py:159-198): parse (question, response) back out of the
+Reference behaviour (GRPO/grpo.py:159-198): parse (question, response) back out of the
 decoded chat-templated string, tokenize the *pair* with the reward model's own tokenizer, score in
 batches of ``reward_batch_size`` taking ``logits.squeeze()``, moving the RM GPU<->CPU around the pass.
 Here the RM is resident in HBM in bf16 (tiering via ``TieringEngine`` when ``offload_reward=host``),
@@ -98,7 +98,7 @@ class ModelReward:
         """Id-level fast path (no RM tokenizer: synthetic / offline runs).  Policy ids are folded into the RM vocabulary and
         every row ``[CLS] question [SEP] response [SEP]`` is assembled ON THE DEVICE with index arithmetic -- no Python loop
         over the 2048 x 1500 response ids, no per-row tensors, no per-batch host read (the reference decodes to strings and
-        re-tokenizes on the CPU: /root/reference/GRPO/grpo.py:166-188).  ``queries`` are left-padded, ``responses``
+        re-tokenizes on the CPU: GRPO/grpo.py:166-188).  ``queries`` are left-padded, ``responses``
         right-padded; a response ends before its first pad / EOS."""
         cfg = self.rm.config
         dev = self.device

@@ -1,12 +1,12 @@
 """Rule-based math reward: boxed-answer extraction + answer equivalence with a *working* timeout.
 
 Reference: the r1-v0 example rewards 1/0 by comparing the ``\\boxed{}`` content of the response with the
-MetaMathQA "The answer is: X" ground truth through ``iscorrect`` (/root/reference/examples/r1-v0/
+MetaMathQA "The answer is: X" ground truth through ``iscorrect`` (examples/r1-v0/
 grpo_r1.py:194-224,250-273), backed by 2.4 kLoC of vendored graders (``utils/toolkit_for_MATH/
 latex_answer_check.py``, ``utils/eval/eval_script.py``, ``utils/eval/eval_utils.py``,
 ``utils/data_processing/answer_extraction.py``).  In the shipped reference the symbolic graders are never
 reached: every comparison is forked into a fresh process with a 15 ms join timeout and a mismatched
-argument list, so the effective rule is a whitespace-stripped exact string match (SURVEY.md 3.5 quirk 2).
+argument list, so the effective rule is a whitespace-stripped exact string match.
 
 This module implements the *intended* behaviour, re-derived from the description of those graders:
   normalise (MATH-style ``strip_string``) -> exact match -> numeric match (floats, fractions, percent,
@@ -65,7 +65,7 @@ _FEW_SHOT_STOPS = {"math": ("Problem:",), "gsm8k": ("Q: ",), "sat": ("Problem:",
 
 def extract_answer(text: str, dataset: str = "math") -> Optional[str]:
     """Final answer of a free-form solution, in the order the reference's extractors try
-    (/root/reference/examples/r1-v0/utils/data_processing/answer_extraction.py:65-338, re-derived from their behaviour):
+    (examples/r1-v0/utils/data_processing/answer_extraction.py:65-338, re-derived from their behaviour):
     a few-shot continuation is cut at the next exemplar header (``Problem:``, ``Q: ``, ...) -> last ``\\boxed{}`` -> "final
     answer is $...$" (minerva) -> "the answer is ..." / "答案是" -> ``#### x`` (gsm8k) -> the body of the last ```` ```output ````
     block (tool-integrated solutions) -> a multiple-choice letter for ``dataset in {"mmlu", "sat", "aqua"}`` -> the last

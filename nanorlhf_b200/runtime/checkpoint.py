@@ -1,6 +1,6 @@
 """HF-style checkpoint directories + real resume.
 
-On-disk layout is the reference's (writer /root/reference/GRPO/grpo_trainer.py:
+On-disk layout is the reference's (writer GRPO/grpo_trainer.py:
 321-404, PPO/ppo_trainer.py:407-418):
 
     <output_dir>/checkpoint-<global_step>/
@@ -11,7 +11,7 @@ On-disk layout is the reference's (writer /root/reference/GRPO
 including the ``_old``-suffix quirk of the best-checkpoint bookkeeping (a metric whose name ends in
 ``_old`` describes the policy *before* this update, so the previous checkpoint is the one recorded
 as best, :375-380) and rotation to ``save_total_limit`` that never deletes the best.  Unlike the
-reference (which cannot resume: SURVEY.md 5.4) ``load_checkpoint`` restores model/adapter,
+reference (which cannot resume) ``load_checkpoint`` restores model/adapter,
 optimizer moments, scheduler, every RNG incl. the sampler-seed stream, dataloader position, episode.
 """
 from __future__ import annotations

@@ -2,10 +2,10 @@
 
 The reference swaps whole models with synchronous, pageable, tensor-by-tensor ``.to('cpu')`` /
 ``.to(device)`` calls four times per update and walks the optimizer state dict doing the same
-(/root/reference/GRPO/grpo_trainer.py:124,164,168-172,475,525,622,625,728; GRPO/grpo.py:164,195),
+(GRPO/grpo_trainer.py:124,164,168-172,475,525,622,625,728; GRPO/grpo.py:164,195),
 followed by ``torch.cuda.empty_cache()`` storms.  On a 180 GB B200 every role of the 1.5B/7B
 configs fits resident, so the default residency is ``resident`` (all calls below are no-ops).
-``host`` residency is kept as a first-class capability (BASELINE.json config 5):
+``host`` residency is kept as a first-class capability:
 
 * each role owns ONE flat device buffer (params are views) and ONE pinned host mirror, so a swap is
   a single ``cudaMemcpyAsync`` at PCIe/C2C line rate instead of hundreds of small pageable copies;

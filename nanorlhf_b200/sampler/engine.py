@@ -1,6 +1,6 @@
 """In-process rollout engine: the replacement for the reference's ``vllm_generate``.
 
-Reference (/root/reference/GRPO/grpo_trainer.py:122-166): move the policy to the CPU, merge LoRA on
+Reference (GRPO/grpo_trainer.py:122-166): move the policy to the CPU, merge LoRA on
 the CPU, write the model to disk twice, boot a fresh vLLM engine from disk, generate, tear the
 engine down, move the policy back.  Here the sampler lives in the trainer's process and CUDA
 context and shares HBM with it; "weight sync" is a fused on-device kernel (parallel/weight_sync.py)
@@ -9,7 +9,7 @@ and nothing touches the host or the filesystem.
 ``generate`` keeps the reference's call shape -- ``generate([n,] model, tokenizer, prompts,
 temperature, max_tokens)`` returning a right-padded ``LongTensor[len(prompts)*n, max_tokens]`` in
 prompt-major / sample-minor order -- but takes prompt *ids* (the reference round-trips ids ->
-strings -> ids; SURVEY.md 7.4) and exposes ``top_p`` / ``seed``.
+strings -> ids) and exposes ``top_p`` / ``seed``.
 """
 from __future__ import annotations
 
@@ -102,8 +102,8 @@ def generate(n: int, model, tokenizer, prompts: Union[torch.Tensor, Sequence[Seq
 def vllm_generate(*args, **kwargs) -> torch.Tensor:
     """Drop-in name of the reference's rollout helper.  Both call shapes are accepted:
     ``vllm_generate(n, model, tokenizer, prompts, temperature, max_tokens)`` (GRPO / RLOO / RAFT,
-    /root/reference/GRPO/grpo_trainer.py:122) and ``vllm_generate(model, tokenizer, prompts, temperature, max_tokens)``
-    (PPO / REINFORCE / ReMax, /root/reference/PPO/ppo_trainer.py:132).  There is no vLLM behind it: the resident
+    GRPO/grpo_trainer.py:122) and ``vllm_generate(model, tokenizer, prompts, temperature, max_tokens)``
+    (PPO / REINFORCE / ReMax, PPO/ppo_trainer.py:132).  There is no vLLM behind it: the resident
     in-process sampler is used, nothing is written to disk and no engine is booted."""
     if args and isinstance(args[0], int) and not isinstance(args[0], bool):
         return generate(*args, **kwargs)

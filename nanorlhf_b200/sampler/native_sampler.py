@@ -1,4 +1,4 @@
-"""The sm_100a rollout engine (replaces vLLM; SURVEY.md section 2.6 first row, K1-K5).
+"""The sm_100a rollout engine (replaces vLLM, K1-K5).
 
 * lives in the trainer's process / CUDA context, constructed once per policy (no boot, no teardown);
 * weights: a fused arena (qkv / gate_up concatenated, LoRA merged) refreshed on device by
@@ -10,7 +10,7 @@
   bucket; the host only looks at the ``finished`` flags every ``sync_every`` steps;
 * sampling semantics of the reference's ``vllm_generate``: temperature, top-p 0.95, n samples per
   prompt, seeded, stop at EOS (kept), right-pad with pad_id, prompt-major / sample-minor order
-  (/root/reference/GRPO/grpo_trainer.py:122-166); temperature 0 = greedy (ReMax baseline / eval).
+  (GRPO/grpo_trainer.py:122-166); temperature 0 = greedy (ReMax baseline / eval).
 """
 from __future__ import annotations
 

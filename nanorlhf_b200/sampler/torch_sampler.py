@@ -1,6 +1,6 @@
 """Reference autoregressive sampler in plain PyTorch (CPU plumbing backend + oracle).
 
-Plays the role vLLM plays in the reference's ``vllm_generate`` (/root/reference/GRPO/
+Plays the role vLLM plays in the reference's ``vllm_generate`` (GRPO/
 grpo_trainer.py:122-166): temperature + nucleus (top-p 0.95) sampling, ``n`` samples per prompt,
 stop at EOS (kept), right-pad with ``pad_token_id`` to ``max_tokens``, output ordered prompt-major /
 sample-minor.  It runs *in process* on the live policy weights (LoRA un-merged: the adapter path is

@@ -1,6 +1,6 @@
 """The six algorithms (+ sparse GRPO) as thin subclasses of ``RLTrainer``.
 
-Semantics table: SURVEY.md section 3.5.  Reference trainers:
+Reference trainers:
 GRPO/grpo_trainer.py, PPO/ppo_trainer.py, RLOO/rloo_trainer.py, ReMax/remax_trainer.py,
 RAFT/raft_trainer.py, REINFORCE/reinforce_trainer.py, examples/r1-v0/grpo_r1_trainer.py.
 """
@@ -80,7 +80,7 @@ class SparseGRPOTrainer(GRPOTrainer):
     (examples/r1-v0/grpo_r1_trainer.py:562-591,691-791): drop rows whose normalised advantage is 0,
     strip common padding, pack the survivors into token-budget micro-buckets.
 
-    Data-parallel safety (the reference would deadlock, SURVEY.md section 2.3 (iv)): gradients are
+    Data-parallel safety (the reference would deadlock): gradients are
     accumulated locally and reduced once per optimizer step, and all ranks agree on the number of
     optimizer steps with one tiny all-reduce -- ranks that run out of rows contribute zero grads.
     """

@@ -1,8 +1,8 @@
 """The shared online-RL training loop.
 
 The reference ships seven near-identical copies of this loop, one per algorithm
-(/root/reference/GRPO/grpo_trainer.py:176-778 and siblings), each subclassing HF ``Trainer``.
-Here there is one ``RLTrainer`` that owns the six phases of an update (SURVEY.md section 0):
+(GRPO/grpo_trainer.py:176-778 and siblings), each subclassing HF ``Trainer``.
+Here there is one ``RLTrainer`` that owns the six phases of an update:
 
   1. tier optimizer state out of the way (optional)        -- runtime/offload.py   (K-OFF)
   2. rollout with the in-process sampler                   -- sampler/engine.py    (K1-K5, K-BC)
@@ -12,8 +12,8 @@ Here there is one ``RLTrainer`` that owns the six phases of an update (SURVEY.md
   6. optimisation: epochs x mini-batches x micro-batches   -- ops (K-LOSS), parallel/optimizer.py (K-AR)
 
 and thin subclasses that override only the algorithm-specific hooks (``select_samples``,
-``token_rewards``, ``advantages``, ``micro_loss``).  Public surface matches the reference
-(SURVEY.md App. D): ``XTrainer(config, processing_class, policy, ref_policy, train_dataset,
+``token_rewards``, ``advantages``, ``micro_loss``).  Public surface matches the reference:
+``XTrainer(config, processing_class, policy, ref_policy, train_dataset,
 reward_func=..., callbacks=..., [value_model])``, ``.train()``, ``.save_model()``,
 ``._save_checkpoint()``, ``.state / .control / .callback_handler``.
 """
@@ -127,7 +127,7 @@ class RLTrainer:
                 self.model.value_model.gradient_checkpointing_enable(args.gradient_checkpointing_kwargs)
 
         # Replicas must hold identical weights -- frozen ones included (base model under LoRA, reference policy, reward
-        # model): the reference gets this from DDP's constructor broadcast (SURVEY.md N2).  Seeds alone are not enough:
+        # model): the reference gets this from DDP's constructor broadcast.  Seeds alone are not enough:
         # device-side random init is not guaranteed to be bit-identical across processes.
         if self.comm.world_size > 1:
             for m in (policy, ref_policy, value_model if self.uses_value_model else None, getattr(reward_func, "rm", None)):
@@ -151,7 +151,7 @@ class RLTrainer:
         self.callback_handler = CallbackHandler(cbs, self.model, processing_class, self.optimizer, self.lr_scheduler)
         self.state.stateful_callbacks = {type(c).__name__: c.state() for c in cbs if hasattr(c, "state")}
 
-        torch.manual_seed(args.seed)       # same shuffle on every rank, then shard (SURVEY.md N5)
+        torch.manual_seed(args.seed)       # same shuffle on every rank, then shard
         self.dataloader = PromptLoader(train_dataset, args.local_batch_size, self.data_collator, seed=args.seed,
                                        rank=self.comm.rank, world_size=self.comm.world_size,
                                        drop_last=args.dataloader_drop_last)
@@ -283,7 +283,7 @@ class RLTrainer:
         pad = self.tokenizer.pad_token_id
         qr = torch.cat([queries, responses], 1)
         lens = (qr != pad).sum(1).tolist()
-        # packed layout => the budget is on real tokens, not on padded rectangles (SURVEY.md 5.7)
+        # packed layout => the budget is on real tokens, not on padded rectangles
         chunks = create_batches(lens, a.token_budget_fwd, mode="packed")
         B, T_r = responses.shape
         lp = torch.empty(B, T_r, dtype=torch.float32, device=self.device)
@@ -324,7 +324,7 @@ class RLTrainer:
             self._write_memory_log(update, metrics)
             self.lr_scheduler.step()
             self.control = self.callback_handler.on_step_end(a, self.state, self.control)
-            # state.max_steps = batches * minibatches is never reached by global_step (SURVEY.md 3.5 "Schedules"),
+            # state.max_steps = batches * minibatches is never reached by global_step,
             # so the flow callback cannot stop the loop early; a stop raised by any *other* callback (early stopping,
             # a user callback) is honoured after this update's checkpoint.
             if self.control.should_save:
@@ -370,7 +370,7 @@ class RLTrainer:
 
     def _maybe_load_best(self):
         """``load_best_model_at_end``: finish with the weights of ``state.best_model_checkpoint`` (HF semantics; the reference
-        sets the flag only to satisfy EarlyStoppingCallback and its overridden ``train`` never acts on it -- SURVEY.md 2.2)."""
+        sets the flag only to satisfy EarlyStoppingCallback and its overridden ``train`` never acts on it)."""
         a, best = self.args, self.state.best_model_checkpoint
         if not a.load_best_model_at_end or a.save_strategy == "no" or not best or not os.path.isdir(best):
             return

@@ -1,6 +1,6 @@
 """Value-model initialisation for PPO: pre-fit the critic to Monte-Carlo returns of the initial policy.
 
-Reference: ``finetuned_value_model`` (/root/reference/PPO/value_initializer.py:69-388; call site
+Reference: ``finetuned_value_model`` (PPO/value_initializer.py:69-388; call site
 PPO/ppo.py:371-380; "about 15 minutes" on an A100, PPO/ppo.py:370).  Behaviour reproduced:
 
   1. one batch of ``min(train_data_size, len(dataset))`` prompts, n = 1 rollout with the policy;

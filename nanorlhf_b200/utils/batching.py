@@ -1,10 +1,10 @@
 """Token-budget bucket batching (dynamic mini-batching of the r1-v0 example).
 
-Behaviour of the reference's ``_create_batches`` (/root/reference/examples/r1-v0/grpo_r1_trainer.py:
+Behaviour of the reference's ``_create_batches`` (examples/r1-v0/grpo_r1_trainer.py:
 410-435): sort by length ascending and greedily grow a batch while
 ``max_len_in_batch * (count + 1) <= budget`` (the padded-token footprint).  Because this engine
 packs tokens (no padding reaches a kernel) the same routine also offers ``mode="packed"`` where
-the budget is on the *sum* of lengths -- the knapsack the survey (section 5.7) asks for.
+the budget is on the *sum* of lengths.
 """
 from __future__ import annotations
 

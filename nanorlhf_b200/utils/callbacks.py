@@ -2,7 +2,7 @@
 
 The reference inherits these from HF ``Trainer`` (``TrainerState``/``OnlineTrainerState``,
 ``TrainerControl``, ``CallbackHandler``, ``DefaultFlowCallback``, ``EarlyStoppingCallback``:
-import sites /root/reference/GRPO/grpo_trainer.py:49-59, use :266-273,:462,:749-752).
+import sites GRPO/grpo_trainer.py:49-59, use :266-273,:462,:749-752).
 Events fired by the trainers: on_train_begin, on_step_end, on_log, on_save, on_evaluate,
 on_train_end -- the same set the reference reaches.
 """
@@ -97,7 +97,7 @@ class ProgressCallback(TrainerCallback):
 
 class EarlyStoppingCallback(TrainerCallback):
     """Counts non-improving evaluations; acts only in ``on_evaluate`` (so it is inert in the
-    reference's RL loops, which never fire it -- SURVEY.md section 2.2 -- but live in the value
+    reference's RL loops, which never fire it -- but live in the value
     pre-fit, PPO/ppo.py:84-110)."""
 
     def __init__(self, early_stopping_patience: int = 1, early_stopping_threshold: float = 0.0):

@@ -2,9 +2,9 @@
 
 Reference behaviour reproduced (not its code): hh-rlhf prompts are the text between the first
 ``Human: `` and the following ``Assistant: `` of the ``chosen`` field, wrapped in a fixed Qwen chat
-template and tokenized without padding into ``{"input_ids"}`` (/root/reference/GRPO/grpo.py:247-270);
+template and tokenized without padding into ``{"input_ids"}`` (GRPO/grpo.py:247-270);
 the trainer shuffles, batches ``local_batch_size`` prompts with ``drop_last`` and left-pads
-(/root/reference/GRPO/grpo_trainer.py:300-310).  There is no network on the GPU box, so
+(GRPO/grpo_trainer.py:300-310).  There may be no network, so
 ``synthetic_hh_prompts`` generates prompts with an hh-rlhf-like length distribution.
 """
 from __future__ import annotations
@@ -94,9 +94,9 @@ class PromptLoader:
     """Shuffled, drop-last, rank-sharded, resumable batch iterator.
 
     All ranks draw the same permutation (seeded) and take interleaved shards -- the behaviour of an
-    accelerate-prepared DataLoader (SURVEY.md section 2.4 N5).  ``drop_last=False`` keeps the tail of every epoch: the last
+    accelerate-prepared DataLoader.  ``drop_last=False`` keeps the tail of every epoch: the last
     global batch is completed with the first prompts of the same permutation (the update needs full batches).  ``state_dict`` makes the dataloader
-    position part of checkpoints (the reference cannot resume, SURVEY.md 5.4).
+    position part of checkpoints (the reference cannot resume).
     """
 
     def __init__(self, dataset, batch_size: int, collate_fn: Callable, seed: int, rank: int = 0,

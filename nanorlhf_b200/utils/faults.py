@@ -1,6 +1,6 @@
 """Failure detection: fault injection hooks, per-rank heartbeat, watchdog.
 
-The reference has none of this (SURVEY.md 5.3).  ``NANORLHF_FAULT=rank:phase:step`` makes the named
+The reference has none of this.  ``NANORLHF_FAULT=rank:phase:step`` makes the named
 rank raise (``:exit`` suffix -> ``os._exit(17)``) when it enters ``phase`` of update ``step`` --
 used by the distributed tests to check that surviving ranks exit non-zero within the watchdog
 timeout and that a restart resumes from the last checkpoint.

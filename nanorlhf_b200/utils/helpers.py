@@ -1,6 +1,6 @@
 """Small tensor helpers whose semantics the RLHF algorithms depend on.
 
-The reference borrows these from trl (import sites: /root/reference/GRPO/grpo_trainer.py:54-68);
+The reference borrows these from trl (import sites: GRPO/grpo_trainer.py:54-68);
 trl is not a dependency here, so the behaviour is owned and unit-tested by this package
 (tests/test_helpers.py).
 """

@@ -1,8 +1,8 @@
 """Metric sinks: stdout, JSONL (always), tensorboard, wandb (offline-capable).
 
 Reference: ``self.log(metrics)`` -> HF ``on_log`` -> Wandb/TensorBoard callbacks per ``report_to``
-(/root/reference/GRPO/grpo_trainer.py:747, GRPO/grpo.py:136); completions table printed with rich
-and logged to wandb (:712-724).  Keys are listed in SURVEY.md App. B.
+(GRPO/grpo_trainer.py:747, GRPO/grpo.py:136); completions table printed with rich
+and logged to wandb (:712-724).
 """
 from __future__ import annotations
 
@@ -59,7 +59,7 @@ class TensorBoardLogger(TrainerCallback):
 
 
 class WandbLogger(TrainerCallback):
-    """wandb in offline mode when there is no network (GPU box)."""
+    """wandb in offline mode when there is no network."""
 
     def __init__(self, run_name: Optional[str] = None, config: Optional[dict] = None):
         self.run_name, self.config, self.run = run_name, config, None

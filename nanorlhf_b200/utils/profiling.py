@@ -1,7 +1,7 @@
 """Phase timers (CUDA events), NVTX ranges, memory high-water marks -> ``time/*`` / ``mem/*`` metrics.
 
-The reference only prints wall-clock ``s/episode`` (/root/reference/GRPO/grpo_trainer.py:726) and
-imports an unused memory profiler (SURVEY.md 5.1).  Here every phase of an update (rollout, reward,
+The reference only prints wall-clock ``s/episode`` (GRPO/grpo_trainer.py:726) and
+imports an unused memory profiler.  Here every phase of an update (rollout, reward,
 logprob, advantage, train, comm, ckpt) is bracketed with CUDA events on the current stream and an
 NVTX range, with no host synchronisation until the metrics are read at the end of the update.
 """
@@ -63,7 +63,7 @@ class PhaseTimer:
 
 
 def debug_sync_enabled() -> bool:
-    """``NANORLHF_DEBUG_SYNC=1``: sync + finite-check after each phase (SURVEY.md 5.2)."""
+    """``NANORLHF_DEBUG_SYNC=1``: sync + finite-check after each phase."""
     return os.environ.get("NANORLHF_DEBUG_SYNC", "0") == "1"
 
 

@@ -1,9 +1,9 @@
-"""LR schedules (the reference gets these from HF ``get_scheduler``; SURVEY.md section 2.2).
+"""LR schedules (the reference gets these from HF ``get_scheduler``).
 
 ``cosine_with_min_lr`` with ``min_lr_rate`` is the default of every entry script
-(/root/reference/GRPO/grpo.py:119-121); ``reduce_lr_on_plateau`` is used by the value pre-fit
-(/root/reference/PPO/ppo.py:92-94).  Schedulers are stepped once per *update* with horizon
-``num_total_batches`` (/root/reference/GRPO/grpo_trainer.py:258-260,748).
+(GRPO/grpo.py:119-121); ``reduce_lr_on_plateau`` is used by the value pre-fit
+(PPO/ppo.py:92-94).  Schedulers are stepped once per *update* with horizon
+``num_total_batches`` (GRPO/grpo_trainer.py:258-260,748).
 """
 from __future__ import annotations
 

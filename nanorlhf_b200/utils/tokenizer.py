@@ -1,6 +1,6 @@
 """Offline tokenizers.
 
-The GPU box has no network, so ``AutoTokenizer.from_pretrained("Qwen/...")`` (reference:
+There may be no network, so ``AutoTokenizer.from_pretrained("Qwen/...")`` (reference:
 GRPO/grpo.py:209-216) cannot be assumed.  ``ByteTokenizer`` is a self-contained UTF-8 byte-level
 tokenizer with the Qwen chat special tokens as single ids; ``HFTokenizerAdapter`` wraps an installed
 ``tokenizer.json`` when one exists on disk.  Both expose the small surface the trainers use:

@@ -1,4 +1,4 @@
-"""Advantage estimators and losses against slow oracles written straight from SURVEY.md section 3.5."""
+"""Advantage estimators and losses against slow oracles written straight from the definitions."""
 import math
 
 import pytest

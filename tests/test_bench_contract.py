@@ -1,4 +1,4 @@
-"""The driver's bench.py contract: one JSON line on stdout with the agreed keys."""
+"""The contract of bench.py: one JSON line on stdout with the agreed keys."""
 import json
 import os
 import subprocess

@@ -51,7 +51,7 @@ def test_entry_script_runs_offline(script, extra, tmp_path):
 
 
 def test_reference_helper_names_are_importable():
-    """module-level helpers a reference user imports from the trainer module."""
+    """Module-level helpers a reference user imports from the trainer module."""
     import torch
     from nanorlhf_b200.models.qwen2 import Qwen2Config, Qwen2ForCausalLM
     from nanorlhf_b200.trainer import (INVALID_LOGPROB, PolicyAndValueWrapper, forward, state_to_device,  # noqa: F401

@@ -1,5 +1,5 @@
 """Failure detection + restart: kill one rank mid-update (fault injection), the survivor must exit non-zero,
-and a relaunch resumes from the last checkpoint (SURVEY.md section 5.3; the reference has none of this)."""
+and a relaunch resumes from the last checkpoint (the reference has none of this)."""
 import os
 import tempfile
 import time

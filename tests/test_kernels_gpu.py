@@ -535,7 +535,7 @@ def test_paged_decode_fp8_kv(Hq, Hkv, splits, max_ctx):
 
 
 def test_adamw_flat_master_weights_lr_6e6():
-    """at lr = 6e-6 bf16 parameters stall without an fp32 master copy; with it the kernel tracks
+    """At lr = 6e-6 bf16 parameters stall without an fp32 master copy; with it the kernel tracks
     torch.optim.AdamW (fp32) over 100 steps."""
     n = _native()
     torch.manual_seed(0)

@@ -1,5 +1,5 @@
 """Flat AdamW: fp32 master weights at the shipped learning rate, step-count invariance of ``train_samples_per_prompt``,
-resharding of the saved optimizer state (ADVICE round 1; reference optimizer: GRPO/grpo_trainer.py:258,692)."""
+resharding of the saved optimizer state (reference optimizer: GRPO/grpo_trainer.py:258,692)."""
 import torch
 
 from nanorlhf_b200.parallel.optimizer import FusedAdamW, shard_bounds

@@ -68,7 +68,7 @@ def test_on_demand_preemption_and_recompute():
 
 
 def test_runtime_under_address_and_ub_sanitizers():
-    """the host runtime built with -fsanitize=address,undefined survives a randomized
+    """The host runtime built with -fsanitize=address,undefined survives a randomized
     admit / advance / finish / preempt workload with page accounting checked every step."""
     import os
     import shutil

@@ -1,4 +1,4 @@
-"""T1: every algorithm end to end on CPU with the PyTorch sampler (plumbing config of BASELINE.json)."""
+"""T1: every algorithm end to end on CPU with the PyTorch sampler (the smallest configuration)."""
 import os
 
 import pytest
@@ -123,7 +123,7 @@ def test_value_initializer(tmp_path):
 
 def test_train_on_all_samples_keeps_step_count(tmp_path):
     """``train_samples_per_prompt = N`` (train on every sample): N x the rows, the same number of optimizer steps, no
-    out-of-range stats slot (ADVICE round 1)."""
+    out-of-range stats slot."""
     t = build(GRPOTrainer, tmp_path, {"grpo_sample_N": 4}, train_samples_per_prompt=4)
     steps0 = t.optimizer._step
     m = t.train()
