@@ -9,7 +9,8 @@
 //                scores, where it is the A operand of P V; O / l and LSE at the end.  The next item's queries and first keys arrive meanwhile.
 // One persistent CTA per SM (TMEM 512 columns, 193 KB of shared memory).  Items go from the most to the fewest key blocks over all
 // sequences, heads varying fastest, and are dealt to the CTAs forwards and backwards in turn, so that their shares come out even.
-// The bound is the tensor pipe and, equally, 2^x on the special-function unit (see attention_window_tc.cu).
+// Tensor pipe and special-function unit (2^x) are each 56 % busy at 4 x 4096 tokens, 12 heads over 2: what is left is the hand-over between
+// scores, softmax and P V of the two tiles (attention_tc.cuh).
 // The earlier form (blocks of 64 keys, P through swizzled shared memory, a CTA per item) spent its time on the shared-memory round trip of
 // P and between CTAs: 28 heads over 4, 2 x 6005 tokens 648 -> 467 us (1.1 PFLOP/s).
 // Backward: attention_bwd_tc.cu.  Oracle: the mma.sync kernels in attention_varlen.cu.  Together they replace flash-attn-2
@@ -175,7 +176,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
               mbar_wait(&full[k_slot], phase);
               ring_next();
             }
-            // keys behind the end of the sequence belong to another one: their P is 0, their V stays out
+            // keys behind the end of the sequence belong to another one: their P is 0, and groups of 16 of them stay out.  The last group
+            // may hold up to 15 rows of the next sequence's V times 0: an infinity or NaN there reaches this block's rows
             const int steps = min(8, (it.len - j * kAtBN + 15) / 16);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {

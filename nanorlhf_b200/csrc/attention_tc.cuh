@@ -131,8 +131,9 @@ NRL_DEVICE void attn_mask_block(uint32_t (&sv)[4][32], int lo, int hi, int keep)
 // Thread = one row of S (128 scores in registers, raw; -inf where masked).  Replaces the scores by P = 2^(s * scale - m) in TMEM
 // (bf16), updates the running maximum / sum and rescales the row of O when its maximum moved by more than 2^8 (a stale maximum is
 // harmless below that: P stays under 256 and the sum is kept in float).  `first`: O holds nothing yet.
-// A share of the 2^x on the FMA pipe (polynomial) was tried: 430 -> 438 / 454 us with 2 / 3 of 8 pairs at 16 x 2048 tokens, so the
-// special-function unit is not what limits this block.
+// Neither the tensor pipe nor the special-function unit is saturated while this runs (56 % each, 4 x 4096 tokens): what bounds it is the chain from
+// a tile's scores to its P and on to the next scores.  A share of the 2^x on the FMA pipe (polynomial) brought nothing: 430 -> 438 / 454 us with
+// 2 / 3 of 8 pairs at 16 x 2048 tokens.
 NRL_DEVICE void attn_softmax_block(uint32_t (&sv)[4][32], float scale, uint32_t t_p, uint32_t t_o, bool first, float& m_run, float& l_run) {
   float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll

@@ -16,9 +16,9 @@
 //                into TMEM over its scores; behind the last block the next item's queries (float -> bf16, swizzled), so that its first
 //                scores are formed during the epilogue: sink, gate, store
 // Tokens of different sequences that fall into one item are walked one run after the other over the same accumulators.
-// TMEM 512 columns and 197 KB of shared memory: one CTA per SM.  The bound is the tensor pipe and, equally, 2^x on the special-function
-// unit (16 per clock and SM against 4096 multiply-adds: both need 1024 clocks per 128 x 128 x 128 block and tile); 1.0 PFLOP/s at 4 x 8192
-// causal tokens.  At 16 x 2048 tokens with window 1024 the query fetch and the epilogue between items cost about a third.
+// TMEM 512 columns and 197 KB of shared memory: one CTA per SM.  Tensor pipe and 2^x on the special-function unit need 1024 clocks each per
+// 128 x 128 x 128 block and tile (16 per clock and SM against 4096 multiply-adds) and neither is saturated: the hand-over between them bounds
+// the walk (attention_tc.cuh); 1.0 PFLOP/s at 4 x 8192 causal tokens.  At 16 x 2048 tokens with window 1024 the query fetch and the epilogue between items cost about a third.
 // Compiled WITHOUT fast-math.
 #include "attention_tc.cuh"
 #include "hybrid_kernels.h"

@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
           }
           if (tok < 0) tok = last;
           s_pub[0] = __int_as_float(e0 + tok);
-          s_pub[1] = fmaf(vec_elem(load(tok >> 3), tok & 7), sc, -mx);     // octaves above the row maximum (at most 0)
+          s_pub[1] = fmaf(vec_elem(load(tok >> 3), tok & 7), sc, -mx);     // octaves above the rounded row maximum: at most half an ulp of it
         }
       }
     }
