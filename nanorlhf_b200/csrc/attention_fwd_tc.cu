@@ -252,7 +252,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int key0 = j * kAtBN;
         // only the block on the diagonal needs a mask: the others end before the tile's first row
         if (j == n - 1) attn_mask_block(sv, 0, min(row, it.len - 1) - key0, 0);
-        attn_softmax_block(sv, p.scale_log2, t_s, t_o, j == 0, m_run, l_run);
+        attn_softmax_block<false>(sv, p.scale_log2, t_s, t_o, j == 0, m_run, l_run);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready[x]);

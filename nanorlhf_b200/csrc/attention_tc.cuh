@@ -43,6 +43,11 @@ NRL_DEVICE uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 
+// lo += the pair's first element, hi += its second
+NRL_DEVICE void add_bf16x2(uint32_t pair, float& lo, float& hi) {
+  asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tadd.rn.f32.bf16 %0, a, %0;\n\tadd.rn.f32.bf16 %1, b, %1;\n\t}" : "+f"(lo), "+f"(hi) : "r"(pair));
+}
+
 // Packed sequences cut into blocks of BM rows, put in order by the number of blocks in front of (or behind) them: how many blocks have
 // `level` or more of them, and the n-th sequence that has more than `level` blocks (both by a whole warp).
 template <int BM>
@@ -131,9 +136,13 @@ NRL_DEVICE void attn_mask_block(uint32_t (&sv)[4][32], int lo, int hi, int keep)
 // Thread = one row of S (128 scores in registers, raw; -inf where masked).  Replaces the scores by P = 2^(s * scale - m) in TMEM
 // (bf16), updates the running maximum / sum and rescales the row of O when its maximum moved by more than 2^8 (a stale maximum is
 // harmless below that: P stays under 256 and the sum is kept in float).  `first`: O holds nothing yet.
+// EXACT, for results that leave no statistic of the sum: the maximum is the row's own in every block, so that its largest weight is
+// exactly 1, and the sum adds the weights as P V sees them, rounded.  Error against float64, 16 x 2048 tokens with window 1024: 2.51e-3, lazily
+// and with unrounded sums 2.56e-3, mma.sync kernel 2.52e-3; it costs 349 -> 368 us.  (A sum whose logarithm the backward forms P from adds unrounded weights.)
 // Neither the tensor pipe nor the special-function unit is saturated while this runs (56 % each, 4 x 4096 tokens): what bounds it is the chain from
 // a tile's scores to its P and on to the next scores.  A share of the 2^x on the FMA pipe (polynomial) brought nothing: 430 -> 438 / 454 us with
 // 2 / 3 of 8 pairs at 16 x 2048 tokens.
+template <bool EXACT>
 NRL_DEVICE void attn_softmax_block(uint32_t (&sv)[4][32], float scale, uint32_t t_p, uint32_t t_o, bool first, float& m_run, float& l_run) {
   float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -142,12 +151,13 @@ NRL_DEVICE void attn_softmax_block(uint32_t (&sv)[4][32], float scale, uint32_t 
     for (int i = 0; i < 32; i += 2)
       mx4[(i >> 1) & 3] = fmaxf(mx4[(i >> 1) & 3], fmaxf(__uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1])));
   const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale;
-  const bool moved = mx > m_run + 8.f;                        // false while nothing has been seen (-inf > -inf)
+  const bool moved = mx > (EXACT ? m_run : m_run + 8.f);      // false while nothing has been seen (-inf > -inf)
   const float corr = moved ? ex2_approx(m_run - mx) : 1.f;
   m_run = moved ? mx : m_run;
   const float m_sub = m_run == -INFINITY ? 0.f : m_run;       // 2^(-inf - 0) = 0 for a row without keys so far
   const uint64_t sc2 = pack_f32x2(scale, scale), nm2 = pack_f32x2(-m_sub, -m_sub);
   uint64_t sum2[2] = {0, 0};
+  float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     uint32_t pv[32];
@@ -159,24 +169,33 @@ NRL_DEVICE void attn_softmax_block(uint32_t (&sv)[4][32], float scale, uint32_t 
         unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * h + c][i]), __uint_as_float(sv[2 * h + c][i + 1])), sc2, nm2), a, b);
         a = ex2_approx(a);
         b = ex2_approx(b);
-        sum2[(i >> 1) & 1] = add_f32x2(sum2[(i >> 1) & 1], pack_f32x2(a, b));
         pv[c * 16 + i / 2] = pack_bf16x2(a, b);
+        if (EXACT) add_bf16x2(pv[c * 16 + i / 2], sum4[(i >> 1) & 1], sum4[2 + ((i >> 1) & 1)]);
+        else sum2[(i >> 1) & 1] = add_f32x2(sum2[(i >> 1) & 1], pack_f32x2(a, b));
       }
     tmem_st_32x32b_x32(t_p + h * 32, pv);
   }
   float s0, s1;
   unpack_f32x2(add_f32x2(sum2[0], sum2[1]), s0, s1);
+  if (EXACT) {
+    s0 = sum4[0] + sum4[1];
+    s1 = sum4[2] + sum4[3];
+  }
   l_run = l_run * corr + (s0 + s1);
   // the block's S was committed behind the previous P V, so O is current here
   if (__any_sync(0xffffffffu, moved && !first)) {
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-      uint32_t ov[32];
-      tmem_ld_32x32b_x32(t_o + c * 32, ov);
+    for (int c = 0; c < 2; ++c) {
+      uint32_t ov[2][32];
+      tmem_ld_32x32b_x32(t_o + c * 64, ov[0]);
+      tmem_ld_32x32b_x32(t_o + c * 64 + 32, ov[1]);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
-      tmem_st_32x32b_x32(t_o + c * 32, ov);
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) ov[h][i] = __float_as_uint(__uint_as_float(ov[h][i]) * corr);
+        tmem_st_32x32b_x32(t_o + c * 64 + h * 32, ov[h]);
+      }
     }
   }
   tmem_st_wait();

@@ -4,7 +4,7 @@
 //
 // Work item: two tiles (A, B) of 128 query rows that share one key/value head -- QT consecutive tokens x HB query heads each -- which
 // walk the keys their rows can see in blocks of 128 (eight pages).  One persistent CTA per SM takes every gridDim-th item,
-// key heads varying fastest: 16 x 2048 tokens, 16 heads over 4, window 1024: 331 to 344 us; tokens varying fastest 334 us (422 -> 624 us with 16 key
+// key heads varying fastest: 16 x 2048 tokens, 16 heads over 4, window 1024: 331 to 344 us (368 with the exact maximum of attention_tc.cuh, as all figures here are without); tokens varying fastest 334 us (422 -> 624 us with 16 key
 // heads and no window: the same few tiles of every sequence fell to the same CTAs); items handed out by a counter 365 us.
 //   warp 0       producer: eight lanes each bring one page (two 64-column panels) of K or V by TMA into a ring of four 32 KB tiles,
 //                in the order the MMAs use them (K_0, V_0, K_1, V_1, K_2 ...); keys behind the end of a sequence are zero (missing pages by an
@@ -441,7 +441,7 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid
             const int plo = first_key(wk.p0 + (trel - wk.t0), wk.window, wk.chunked) - kb;
             attn_mask_block(sv, plo, pq, wk.keep - kb);
           }
-          attn_softmax_block(sv, sl2, t_s, t_o, !any, m_run, l_run);
+          attn_softmax_block<true>(sv, sl2, t_s, t_o, !any, m_run, l_run);
           any = true;
           tc_fence_before();
           __syncwarp();
