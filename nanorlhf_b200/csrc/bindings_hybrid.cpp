@@ -153,7 +153,7 @@ void delta_scan(const Tensor& qkv, int64_t col_k, int64_t col_v, const c10::opti
   check(nrl_delta_scan(f32(qkv, "qkv"), qkv.stride(0), static_cast<int>(col_k), static_cast<int>(col_v), beta.has_value() ? f32(*beta, "beta") : nullptr,
                        f32(decay, "decay"), f32w(state, "state"), f32w(o, "o"), i32(cu, "cu"), i32(start, "start"),
                        i32(state_slot, "state_slot"), E, static_cast<int>(qkv.size(0)), heads, static_cast<int>(kv_heads), D, Dv, per_channel ? 1 : 0,
-                       static_cast<int>(impl), cur_stream()),
+                       static_cast<int>(impl), num_sms(), cur_stream()),
         "delta_scan");
 }
 
@@ -806,6 +806,8 @@ void bind_hybrid(pybind11::module_& m) {
         pybind11::arg("act") = 1);
   m.def("ssd_scan", &ssd_scan, "state-space scan with a scalar decay per head, state carried per slot");
   m.def("delta_prep", &delta_prep, "unit q / k, beta and decays of the gated delta rule");
+  m.def("delta_scan_blocked", &nrl_delta_scan_blocked, "a step goes four tokens at a time", pybind11::arg("E"), pybind11::arg("T"), pybind11::arg("D"),
+        pybind11::arg("Dv"));
   m.def("delta_scan", &delta_scan, "gated delta rule scan, state carried per slot");
   m.def("qknorm_kv_write", &qknorm_kv_write, "per-head RMS norm of q (in place) and k (into the paged cache), v into the cache");
   m.def("window_attention", &window_attention, "sliding-window attention over the paged cache", pybind11::arg("q"),

@@ -158,11 +158,12 @@ cudaError_t nrl_gla_prep(float* qkv, long sq, const float* a_raw, long sa, const
 
 // Gated delta rule scan.  Per head: S = g S (rows);  u = beta (v - S^T k);  S += k u^T;  o = S^T q.
 // beta == nullptr: plain accumulation, u = v (gated linear attention: S = diag(g) S + k v^T).
-// state float [slots, heads, D, Dv];  o float [T, heads*Dv].  `impl`: 0 picks (T >= 12 E: four tokens at a time, else column-resident),
+// state float [slots, heads, D, Dv];  o float [T, heads*Dv].  `impl`: 0 picks (nrl_delta_scan_blocked: four tokens at a time, else column-resident),
 // 1 column-resident, 2 row groups, 3 state in shared memory, 4 four tokens at a time (D <= 128).
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
                            float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
-                           int D, int Dv, int per_channel, int impl, cudaStream_t s);
+                           int D, int Dv, int per_channel, int impl, int num_sms, cudaStream_t s);
+int nrl_delta_scan_blocked(long E, long T, int D, int Dv);       // impl 0 takes a step of E entries and T tokens four tokens at a time
 
 // Per-head RMS norm (weight [D], shared by heads) of q in place and of k into the paged cache; v into the paged cache.
 // q float [T, Hq*D] (row stride sq), k float [T, Hkv*D], v float [T, Hkv*Dv] (row strides sk, sv).

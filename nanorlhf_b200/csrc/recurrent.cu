@@ -684,10 +684,11 @@ delta_scan_col_kernel(const float* __restrict__ qkv, long sq, int col_k, int col
 //   S  <- c_4 S + sum_j (G(4,j) k_j) u_j^T
 // so an element of the state costs three multiply-adds per token (and one product per chunk) and every vector value that is read from
 // shared memory serves four or eight columns.  The column-resident kernels wait for their vectors and two sums once per token: 16 x 2048
-// tokens, 16 heads of 128 x 128: 4350 us there, 2310 us here (950 us at the float32 multiply-add rate).  What bounds it now is latency: 128 rows
-// x 8 columns take 254 registers, so eight warps per SM issue 0.38 instructions per clock and scheduler, stalled on shared-memory reads,
-// shuffles and fixed latencies.  Inputs come by cp.async three chunks ahead and a chunk's vectors are prepared while the one before is
-// computed (2520 us with loads one chunk ahead); 64 registers of state per thread over twice the warps took 2730 us.
+// tokens, 16 heads of 128 x 128: 4350 us there, 2300 us here (950 us at the float32 multiply-add rate).  What bounds it now is latency and
+// registers: 128 rows x 8 columns take 254 and spill (-Xptxas -v: 870 to 950 bytes of stores and 1200 to 1350 of loads a thread; 4 columns of 128 rows and 8 of
+// 64 about 300 to 400 each), so eight warps per SM issue 0.38 instructions per clock and scheduler, stalled on shared-memory reads, shuffles and fixed latencies.
+// Inputs come by cp.async three chunks ahead and a chunk's vectors are prepared while the one before is computed (2520 us with loads one
+// chunk ahead); 64 registers of state per thread over twice the warps took 2730 us.
 //
 // Lane = (one of four column groups, one of eight row groups): a thread keeps 2 PIECES rows x CT columns of the state in registers, rows
 // 16 p + 2 rg + {0, 1}, columns in pairs for the packed multiply-add; the shared vectors are stored with every value twice, so that
@@ -785,9 +786,12 @@ delta_scan_blk_kernel(const float* __restrict__ qkv, long sq, int col_k, int col
   using Sm = BlkSmem<DP, COLS>;
   extern __shared__ __align__(16) unsigned char blk_smem[];
   Sm& sm = *reinterpret_cast<Sm*>(blk_smem);
-  const int e = blockIdx.x, h = blockIdx.y, g = h / (heads / kv_heads);
+  // Entry by entry: the blocks of one portion lie side by side and go to SMs of their own.  With the entry varying fastest a long portion among 15
+  // single tokens kept every sixteenth block, two to three to an SM: 2000 tokens, 16 heads of 128 x 128, 2269 us, 1816 in this order.
+  const unsigned parts = (Dv + COLS - 1) / COLS, eh = blockIdx.x / parts;
+  const int e = static_cast<int>(eh / heads), h = static_cast<int>(eh % heads), g = h / (heads / kv_heads);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rg = lane & 7, x = CT == 8 ? rg : rg >> 1;
-  const int cb0 = blockIdx.z * COLS, cw = warp * 4 * CT + (lane >> 3) * CT, c0 = cb0 + cw;      // first column: block, group in it, group
+  const int cb0 = static_cast<int>(blockIdx.x % parts) * COLS, cw = warp * 4 * CT + (lane >> 3) * CT, c0 = cb0 + cw;      // first column: block, group in it, group
   float* gS = state + (static_cast<long>(state_slot[e]) * heads + h) * D * Dv;
   const bool carried = start[e] > 0;
   const int t0 = cu[e], t1 = cu[e + 1];
@@ -986,6 +990,10 @@ bool pick_col_layout(int cols, int rows, int* rows_t, int* split_out, int* threa
   *split_out = split;
   *threads_out = threads;
   return true;
+}
+bool col_form_fits(int cols, int rows) {
+  int rows_t, split, threads;
+  return pick_col_layout(cols, rows, &rows_t, &split, &threads);
 }
 
 // rows per thread / row groups for a state of `rows` x `cols`: as many row groups as 512 threads allow (256 when a thread
@@ -1298,21 +1306,30 @@ cudaError_t nrl_gla_prep(float* qkv, long sq, const float* a_raw, long sa, const
   return cudaGetLastError();
 }
 
+// Steps of prompt portions take four tokens at a time.  Where the column-resident form fits (Dv <= 256) the lines are
+//   D > 32      a smaller state is padded to 64 rows here, to 16 or 32 there: 64 entries of 128 tokens, 16 heads of 32 x 32, 230 us against 83; one
+//               row more, 33 x 33, 237 / 316
+//   T >= 20 E   a thread's state is not read in whole lines, so that short portions pay more for it: 128 x 128, 64 entries of 2: 95 us against 50,
+//               of 4: 97 / 65; 16 entries of 12: 38 / 38, 8 of 16: 30 / 26, 16 of 20: 45 / 54; 64 x 128, 16 of 16: 26 / 24, of 20: 30 / 30.
+// Above: 16 entries of 2048, 128 x 128: 2300 / 4350, one of 2000: 1515 / 2119; 64 x 64, 16 of 1000: 689 / 1013; without the delta (beta == nullptr) 0.4 to 0.9
+// of the other's time; single tokens beside one portion of 2000, 128 x 128: 15 of them 1816 / 2143, 64 1909 / 2171.  Where the column form does not fit
+// (Dv > 256) the row groups take 1.1 to 10 times as long from twelve tokens an entry on, at D = 16 to 128.
+int nrl_delta_scan_blocked(long E, long T, int D, int Dv) {
+  return D <= 128 && (col_form_fits(Dv, D) ? D > 32 && T >= 20 * E : T >= 12 * E);
+}
+
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
                            float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
-                           int D, int Dv, int per_channel, int impl, cudaStream_t s) {
+                           int D, int Dv, int per_channel, int impl, int num_sms, cudaStream_t s) {
   if (E <= 0) return cudaSuccess;
   if (Dv > 512 || heads % kv_heads != 0 || impl < 0 || impl > 4) return cudaErrorInvalidValue;
-  // Steps of prompt portions: four tokens at a time.  The line lies at twelve tokens an entry because a thread's state is not read in
-  // whole lines: 64 entries x 16 heads of 128 x 128, portions of 2: 95 us against 50 (column-resident), 4: 97 / 65, 8: 111 / about 97; 16 entries of
-  // 2048: 2310 / 4350, one of 2048: 1564 / 2164, one of 70 with 8 heads of 64 x 64: 33 / 66.
-  if (D >= 1 && D <= 128 && Dv >= 1 && (impl == 4 || (impl == 0 && T >= 12L * E))) {
+  if (D >= 1 && D <= 128 && Dv >= 1 && (impl == 4 || (impl == 0 && nrl_delta_scan_blocked(E, T, D, Dv)))) {
     const bool wide = D % 4 == 0 && sq % 4 == 0 && col_k % 4 == 0 && reinterpret_cast<uintptr_t>(qkv) % 16 == 0 &&
                      reinterpret_cast<uintptr_t>(decay) % 16 == 0;
     // eight columns per thread unless that leaves SMs without a block (one entry of 2048, 16 heads: four columns 1564 us, eight 1816; 16 entries:
     // 3730 / 2310)
-    const int ct = static_cast<long>(E) * heads * ((Dv + 63) / 64) >= 148 ? 8 : 4;
-    const dim3 grid(E, heads, (Dv + 8 * ct - 1) / (8 * ct));
+    const int ct = static_cast<long>(E) * heads * ((Dv + 63) / 64) >= num_sms ? 8 : 4;
+    const dim3 grid(static_cast<unsigned>(E) * heads * ((Dv + 8 * ct - 1) / (8 * ct)));
 #define NRL_DELTAB(P_, C_, B_)                                                                                                   \
   if ((D <= 64 ? 4 : 8) == P_ && ct == C_ && (beta != nullptr) == B_)                                                              \
     return (wide ? launch_delta_blk<P_, C_, B_, true> : launch_delta_blk<P_, C_, B_, false>)(                                      \
