@@ -20,6 +20,8 @@
 // 128 x 128 x 128 block and tile (16 per clock and SM against 4096 multiply-adds) and neither is saturated: the hand-over between them bounds
 // the walk (attention_tc.cuh); 1.0 PFLOP/s at 4 x 8192 causal tokens.  At 16 x 2048 tokens with window 1024 the query fetch and the epilogue between items cost about a third.
 // Compiled WITHOUT fast-math.
+#include <algorithm>
+
 #include "attention_tc.cuh"
 #include "hybrid_kernels.h"
 
@@ -528,9 +530,23 @@ int nrl_window_attention_tc_fits(const float* q, long sq, const void* out, long 
   return T >= 1 && T < (1L << 24);
 }
 
+// Tokens of a tile.  An item walks its runs one after the other, so a step of many short portions in few items waits for a few CTAs.  There the tiles
+// take as few tokens as give every SM an item (in brackets: full tiles, mma.sync form): 64 portions of 4 tokens, 16 heads over 16, 35 us (155, 100), behind
+// 1000 keys 159 (1098, 1421); 16 over 4, 20 (49, 34); 200 single tokens behind 1000 keys beside a portion of 30, 16 over 16, 474 (3396, 5633).
+// Not where the portions are long: an item that holds one whole portion has one run, a smaller one that lies across two has two (16 portions of
+// 64 behind 1000 keys, 16 over 4: 32 us, with small tiles 57).
+int nrl_window_attention_tc_tokens(long T, long E, int Hq, int Hkv, int num_sms) {
+  const int per_g = Hq / Hkv, HB = per_g < 128 ? per_g : 128, most = 128 / HB;
+  const int heads = Hkv * ((per_g + HB - 1) / HB), share = num_sms / heads;          // items of one stretch of tokens; stretches that the SMs hold
+  if (share < 1 || E < 1) return most;
+  const long qt = (T + 2 * share - 1) / (2 * share);
+  const long runs_T = std::min(E * T, 2 * most * E);                                 // runs of a full item, times T: E, or its tokens by the mean portion
+  return qt < most && runs_T > T + 2 * qt * E ? static_cast<int>(qt) : most;
+}
+
 cudaError_t nrl_window_attention_tc(const CUtensorMap* tmK, const CUtensorMap* tmV, int oob_k, int oob_v, const float* q, long sq,
                                     const int* block_table, int max_blocks, const int* tok_entry, const int* pos, int window, float scale,
-                                    float out_scale, void* out, long so, int T, int Hq, int Hkv, const NrlAttnMods* md, int num_sms,
+                                    float out_scale, void* out, long so, int T, int E, int Hq, int Hkv, const NrlAttnMods* md, int num_sms,
                                     cudaStream_t s) {
   using namespace nrl;
   if (T <= 0) return cudaSuccess;
@@ -540,7 +556,7 @@ cudaError_t nrl_window_attention_tc(const CUtensorMap* tmK, const CUtensorMap* t
   p.scale = scale; p.out_scale = out_scale; p.out = static_cast<__nv_bfloat16*>(out); p.so = so; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
   const int per_g = Hq / Hkv;
   p.HB = per_g < 128 ? per_g : 128;
-  p.QT = 128 / p.HB;
+  p.QT = nrl_window_attention_tc_tokens(T, E, Hq, Hkv, num_sms);
   p.oob_k = oob_k; p.oob_v = oob_v; p.md = *md;
   static bool configured = false;
   if (!configured) {

@@ -239,10 +239,10 @@ void window_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
     md.out_float = out.data_ptr<float>();
     md.out_float_stride = out.stride(0);
   }
-  // Prompt portions over bf16 pages at head size 128: the tcgen05 kernel (impl 4) in every step that is not all single tokens.  It was the
-  // faster one at each size measured, 16 heads over 4: 8192 tokens in portions of 4 behind 1000 keys 1147 us against 1374 (mma.sync),
-  // portions of 32 190 against 493, 16 x 2048 tokens with window 1024 344 against 1460, one portion of 77 tokens 15 against 19, and steps
-  // that mix 64 single tokens with a 4096-token portion 1344 against 1663.
+  // Prompt portions over bf16 pages at head size 128: the tcgen05 kernel (impl 4) in every step that is not all single tokens.  Of 1332 steps measured (4 to
+  // 32 heads over 2 to 16; portions of 1 to 64 tokens, 4 to 200 of them, and single tokens beside one portion of 16 to 2000; behind 0 to 1000 keys) it took
+  // a quarter of the mma.sync form's time in the geometric mean, more than 1.03 times as long in 14, 1.15 times at most (200 portions of 16, 16 heads
+  // over 16: 100 us against 87, a second round of items that is nearly empty).  16 x 2048 tokens with window 1024: 368 against 1460.
   const int64_t rows_k = k_cache.size(0) * Hkv * 16, rows_v = v_cache.size(0) * v_cache.size(1) * 16;
   const bool tc_fits = k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.is_contiguous() &&
                        v_cache.is_contiguous() && window >= 1 && rows_k < (int64_t{1} << 31) - 16 && rows_v < (int64_t{1} << 31) - 16 &&
@@ -257,7 +257,7 @@ void window_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
     check(nrl_window_attention_tc(&tmk, &tmv, static_cast<int>(rows_k), static_cast<int>(rows_v), f32(q, "q"), q.stride(0),
                                   i32(block_table, "block_table"), static_cast<int>(block_table.size(1)), i32(tok_entry, "tok_entry"),
                                   i32(pos, "pos"), static_cast<int>(window), static_cast<float>(scale), static_cast<float>(out_scale),
-                                  out.data_ptr(), out.stride(0), T, Hq, Hkv, &md, num_sms(), cur_stream()),
+                                  out.data_ptr(), out.stride(0), T, static_cast<int>(block_table.size(0)), Hq, Hkv, &md, num_sms(), cur_stream()),
           "window_attention");
     return;
   }
@@ -810,6 +810,8 @@ void bind_hybrid(pybind11::module_& m) {
         pybind11::arg("Dv"));
   m.def("delta_scan", &delta_scan, "gated delta rule scan, state carried per slot");
   m.def("qknorm_kv_write", &qknorm_kv_write, "per-head RMS norm of q (in place) and k (into the paged cache), v into the cache");
+  m.def("window_attention_tc_tokens", &nrl_window_attention_tc_tokens, "tokens of a tile of the tcgen05 kernel", pybind11::arg("T"), pybind11::arg("E"),
+        pybind11::arg("Hq"), pybind11::arg("Hkv"), pybind11::arg("num_sms"));
   m.def("window_attention", &window_attention, "sliding-window attention over the paged cache", pybind11::arg("q"),
         pybind11::arg("k_cache"), pybind11::arg("v_cache"), pybind11::arg("block_table"), pybind11::arg("tok_entry"), pybind11::arg("pos"),
         pybind11::arg("window"), pybind11::arg("scale"), pybind11::arg("out_scale"), pybind11::arg("out"), pybind11::arg("impl") = 0,

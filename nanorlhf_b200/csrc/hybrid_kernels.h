@@ -220,8 +220,9 @@ int nrl_window_attention_tc_fits(const float* q, long sq, const void* out, long 
                                  const NrlAttnMods* md);
 cudaError_t nrl_window_attention_tc(const CUtensorMap* tmK, const CUtensorMap* tmV, int oob_k, int oob_v, const float* q, long sq,
                                     const int* block_table, int max_blocks, const int* tok_entry, const int* pos, int window, float scale,
-                                    float out_scale, void* out, long so, int T, int Hq, int Hkv, const NrlAttnMods* md, int num_sms,
+                                    float out_scale, void* out, long so, int T, int E, int Hq, int Hkv, const NrlAttnMods* md, int num_sms,
                                     cudaStream_t s);
+int nrl_window_attention_tc_tokens(long T, long E, int Hq, int Hkv, int num_sms);      // tokens of a tile in a step of E entries and T tokens
 
 // Tensor-core kernel for prompt portions over bf16 pages of 16 tokens (attention_window_mma.cu); `_fits` says whether the
 // shapes and the output's alignment allow it.

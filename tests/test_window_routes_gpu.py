@@ -40,3 +40,17 @@ def test_refused_forms_stay_on_the_general_kernel():
     with pytest.raises(RuntimeError):
         _run(small, "tc")
     assert torch.equal(_run(small, "auto"), _run(small, "mma"))
+
+
+@pytest.mark.parametrize("H,Hkv", [(16, 16), (8, 2), (3, 1), (128, 1)])
+@pytest.mark.parametrize("news,olds", [([4] * 64, [0] * 64), ([2] * 40 + [70], [100] * 40 + [0]), ([7] * 33, [13] * 33), ([1] * 90 + [5], [300] * 91)])
+def test_rows_do_not_depend_on_how_a_step_is_cut(H, Hkv, news, olds):
+    step = _step(news, olds, H, Hkv)
+    plan, kc, vc, q = step
+    got, t0 = _run(step, "tc"), 0
+    assert ((got.float() - _run(step, "mma").float()).norm() / got.float().norm()).item() < 6e-3
+    for e in (0, len(news) // 2, len(news) - 1):                # entries alone: full tiles of one run
+        t0, n = sum(news[:e]), news[e]
+        alone = _step([n], [olds[e]], H, Hkv)[0]
+        alone.block_table[0, :plan.block_table.shape[1]] = plan.block_table[e, :alone.block_table.shape[1]]
+        assert torch.equal(_run((alone, kc, vc, q[t0:t0 + n]), "tc"), got[t0:t0 + n])
