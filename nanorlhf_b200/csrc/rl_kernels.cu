@@ -18,14 +18,20 @@ namespace nrl {
 // the warps give every thread the advantage behind its last step, and the recurrence is then run as it is written.  4 x 1500 steps: 15 us
 // with one warp per row (47 dependent rounds of load and shuffle), 3.6 us here; longer rows go tile by tile from the end.  In double: powers of
 // a rounded c cost more than the sums themselves (error against float64 2.4e-7 -> 2.5e-8).
-constexpr int kGaeThreads = 256, kGaePer = 8, kGaeTile = kGaeThreads * kGaePer;
+// Rows that one warp holds (256 steps) take a warp each, four to a block, without barriers: 512 x 100 steps 2.6 us, a block per row 4.1; one row of 64
+// 2.5 us either way.
+constexpr int kGaeWarps = 8, kGaePer = 8, kGaeRows = 4;
 
-__global__ void __launch_bounds__(kGaeThreads)
+template <int WARPS>                                  // that share a row: kGaeWarps, or 1 and kGaeRows rows to a block
+__global__ void __launch_bounds__(32 * (WARPS == 1 ? kGaeRows : WARPS))
 gae_scan_kernel(const float* __restrict__ rewards, const float* __restrict__ values, float* __restrict__ adv,
-                float* __restrict__ returns, int T, double gamma, double lam) {
-  __shared__ double heads[kGaeThreads / 32 + 1];      // folded value of every warp's steps; one more: the tile's first advantage
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const size_t row = static_cast<size_t>(blockIdx.x) * T;
+                float* __restrict__ returns, int B, int T, double gamma, double lam) {
+  constexpr int kTile = 32 * WARPS * kGaePer;
+  __shared__ double heads[WARPS + 1];                 // folded value of every warp's steps; one more: the tile's first advantage
+  const int lane = threadIdx.x & 31, warp = WARPS == 1 ? 0 : threadIdx.x >> 5, tid = warp * 32 + lane;
+  const int seq = WARPS == 1 ? blockIdx.x * kGaeRows + (threadIdx.x >> 5) : blockIdx.x;
+  if (seq >= B) return;
+  const size_t row = static_cast<size_t>(seq) * T;
   const float* r = rewards + row;
   const float* v = values ? values + row : nullptr;
   const double c = gamma * lam;
@@ -40,8 +46,8 @@ gae_scan_kernel(const float* __restrict__ rewards, const float* __restrict__ val
   for (int k = 0; k < 5; ++k)
     if ((31 - lane) & (1 << k)) c_lane *= w[k];
   double behind = 0.0;                                // advantage of the step behind the tile
-  for (int tile = (T - 1) / kGaeTile; tile >= 0; --tile) {
-    const int t0 = tile * kGaeTile + tid * kGaePer;
+  for (int tile = (T - 1) / kTile; tile >= 0; --tile) {
+    const int t0 = tile * kTile + tid * kGaePer;
     double d[kGaePer];
     float vt[kGaePer];
 #pragma unroll
@@ -62,11 +68,13 @@ gae_scan_kernel(const float* __restrict__ rewards, const float* __restrict__ val
       const double y = __shfl_down_sync(0xffffffffu, x, 1 << k);
       if (lane + (1 << k) < 32) x = fma(w[k], y, x);
     }
-    __syncthreads();                                 // `heads` of the tile before has been read
-    if (lane == 0) heads[warp] = x;
-    __syncthreads();
     double in = behind;                               // advantage at the first step of the next warp
-    for (int q = kGaeThreads / 32 - 1; q > warp; --q) in = fma(w[5], in, heads[q]);
+    if (WARPS > 1) {
+      __syncthreads();                               // `heads` of the tile before has been read
+      if (lane == 0) heads[warp] = x;
+      __syncthreads();
+      for (int q = WARPS - 1; q > warp; --q) in = fma(w[5], in, heads[q]);
+    }
     const double next = __shfl_down_sync(0xffffffffu, x, 1);
     double a = fma(c_lane, in, lane < 31 ? next : 0.0);
 #pragma unroll
@@ -77,9 +85,13 @@ gae_scan_kernel(const float* __restrict__ rewards, const float* __restrict__ val
         if (returns) returns[row + t0 + j] = static_cast<float>(a + vt[j]);
       }
     }
-    if (tid == 0) heads[kGaeThreads / 32] = a;
-    __syncthreads();
-    behind = heads[kGaeThreads / 32];
+    if (WARPS > 1) {
+      if (tid == 0) heads[WARPS] = a;
+      __syncthreads();
+      behind = heads[WARPS];
+    } else {
+      behind = __shfl_sync(0xffffffffu, a, 0);
+    }
   }
 }
 
@@ -90,7 +102,7 @@ gae_scan_kernel(const float* __restrict__ rewards, const float* __restrict__ val
 // micro-step of 4 x 1500 tokens; 11 launches, 27 us of kernels and 155 us in all with these.
 constexpr int kLossThreads = 512;
 constexpr long kLossClusterMax = 1 << 17;
-constexpr unsigned kLossBlocks = 148;
+constexpr unsigned kLossBlocks = 148;               // a number of its own, so that the order of the sums does not depend on the device
 
 // A block's shared memory may be written by the others of its cluster once it is known to run: every thread arrives on entry to the kernel and
 // waits in front of the first remote write, so that the pass over the tokens hides the barrier.
@@ -316,7 +328,10 @@ using namespace nrl;
 extern "C" cudaError_t nrl_gae_scan(const float* rewards, const float* values, float* adv, float* returns, int B,
                                     int T, double gamma, double lam, cudaStream_t s) {
   if (B == 0 || T == 0) return cudaSuccess;
-  gae_scan_kernel<<<B, kGaeThreads, 0, s>>>(rewards, values, adv, returns, T, gamma, lam);
+  if (T <= 32 * kGaePer)
+    gae_scan_kernel<1><<<(B + kGaeRows - 1) / kGaeRows, 32 * kGaeRows, 0, s>>>(rewards, values, adv, returns, B, T, gamma, lam);
+  else
+    gae_scan_kernel<kGaeWarps><<<B, 32 * kGaeWarps, 0, s>>>(rewards, values, adv, returns, B, T, gamma, lam);
   return cudaGetLastError();
 }
 
