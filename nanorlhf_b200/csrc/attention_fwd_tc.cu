@@ -94,6 +94,11 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncwarp();
     tmem_alloc(tmem_ptr, 512);
   }
+  int level = 0;                                                     // warp 2: blocks of the longest sequence
+  if (warp == 2) {
+    for (int s = lane; s < p.num_seqs; s += 32) level = max(level, (p.cu_seqlens[s + 1] - p.cu_seqlens[s] + kTcBM - 1) / kTcBM);
+    level = __reduce_max_sync(0xffffffffu, level);
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -199,9 +204,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     } else if (warp == 2) {
       // ============================== items ==============================
       const int* cu = p.cu_seqlens;
-      int level = 0;
-      for (int s = lane; s < p.num_seqs; s += 32) level = max(level, (cu[s + 1] - cu[s] + kTcBM - 1) / kTcBM);
-      level = __reduce_max_sync(0xffffffffu, level);                 // blocks of the longest sequence
       int above = 0, upto = 0;                                       // row blocks with an index > level, >= level
       for (uint32_t k = 0;; ++k) {
         const int at = (k & 1) ? (k + 1) * gridDim.x - 1 - blockIdx.x : k * gridDim.x + blockIdx.x;

@@ -62,7 +62,8 @@ NRL_DEVICE int attn_nth_sequence(const int* cu, int num_seqs, int level, int n, 
     const int s = s0 + lane;
     const bool has = s < num_seqs && (cu[s + 1] - cu[s] + BM - 1) / BM > level;
     const uint32_t m = __ballot_sync(0xffffffffu, has);
-    if (n < __popc(m)) return s0 + __fns(m, 0, n + 1);
+    const uint32_t hit = __ballot_sync(0xffffffffu, has && __popc(m & ((1u << lane) - 1)) == n);
+    if (hit != 0) return s0 + __ffs(hit) - 1;
     n -= __popc(m);
   }
   return 0;                                    // not reached for n below their number
