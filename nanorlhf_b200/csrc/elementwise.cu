@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(128) rmsnorm_bwd_kernel(const __nv_bfloat16* _
 // NV 16-byte vectors per lane, all of a row's loads in flight before the first is used, no barrier; FULL: d is exactly 256 NV.  The block
 // forms above (128 threads and one barrier per row, half of them idle in the second vector of 1536 columns) reached 2.5 TB/s:
 // 32 768 x 1536 rmsnorm 79 -> 29 us, 6601 x 1536 rmsnorm_bwd 31 -> 12 us, 24 571 x 1024 add_layernorm 52 -> 24 us.
-// Wider rows keep the block forms.
+// Wider rows keep the block forms.  So that a row's sums never depend on how many rows there are (log-probability pass and training step), the
+// number of rows chooses nothing, although the block forms are 0.2 to 0.3 us faster for a few hundred rows of 2048 and more columns.
 constexpr int kNormWarps = 4;
 
 template <int NV, bool FULL>
@@ -225,7 +226,8 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   store_row<NV, FULL>(gx + off, nvec, lane, a);
 }
 
-// y = LayerNorm(x + residual) * w + b: mean, then centred variance
+// y = LayerNorm(x + residual) * w + b: mean, then centred variance.  The sum stays in float; the plain modules (NANORLHF_DEBERTA=eager) round it to
+// bf16 first.  With GELU in the GEMM's epilogue that takes a reward layer's error against float64 from 4.4e-3 to 3.2e-3.
 template <int NV, bool FULL>
 __global__ void __launch_bounds__(32 * kNormWarps)
 add_layernorm_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ w,
@@ -369,7 +371,9 @@ static inline int grid_for(long total, int threads) {
 
 using namespace nrl;
 
-// vectors per lane of a warp-per-row kernel: 1024, 1536, 2048 or 3584 columns, exact or below
+// Vectors per lane of a warp-per-row kernel: 1024, 1536, 2048 or 3584 columns, exact or below.  What exactness brings: RMS norm with the residual
+// 6601 x 1536 12.8 us (14.4 with the test of the index), 12 011 x 3584 55.4 (61.6), the others up to 4 %.  At 2048 columns it costs: 24 571 rows, RMS norm
+// with the residual 65.2 us (63.5), LayerNorm 58.2 (53.0), so that width has none.
 #define NRL_NORM_DISPATCH(d_, CALL_)                 \
   if ((d_) == 1024) { CALL_(4, true); }              \
   else if ((d_) < 1024) { CALL_(4, false); }         \
