@@ -186,6 +186,26 @@ NRL_DEVICE void tma_store_3d(const CUtensorMap* m, const void* smem_src, int c0,
 // FP8: A and B are e4m3 bytes, K-major (a 128-byte swizzle row = 128 contraction elements), the MMA is kind::f8f6f4
 // (K = 32 per instruction, twice the bf16 rate) and the epilogue applies the per-row (token) and per-column (output
 // channel) dequantisation scales -- the sampler's fp8 rollout GEMMs.
+// 32 rows of W words, one row per lane, handed out in pieces of 16 bytes so that W / 4 neighbouring lanes hold neighbouring pieces of a row:
+// put(step, row, piece, words).  The plain stores of the float and grouped epilogues go through it: a lane per row wrote 16 bytes into each of 32
+// lines at a time, which eight warps at once took longer for than four (4096 x 1536
+// -> 151 936 floats 1699 us, with eight 1893, handed out 1469; added to 3552, 1590; 16 384 tokens over 64 experts 721, 900, 563).
+template <int W, class F>
+NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F&& put) {
+  constexpr int P = W / 4;
+  __syncwarp();                                           // the slab's last rows have been read
+#pragma unroll
+  for (int q = 0; q < P; ++q)
+    *reinterpret_cast<uint4*>(slab + lane * (W * 4) + ((q ^ (lane & (P - 1))) * 16)) = make_uint4(w[q * 4], w[q * 4 + 1], w[q * 4 + 2], w[q * 4 + 3]);
+  __syncwarp();
+  const int q = lane % P;
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const int r = i * (32 / P) + lane / P;
+    put(i, r, q, *reinterpret_cast<const uint4*>(slab + r * (W * 4) + ((q ^ (r & (P - 1))) * 16)));
+  }
+}
+
 // PAIR (CTA pairs, BN = 256): act = silu(x Wg^T) * (x Wu^T) from two separate weights.  The leader loads 128 rows of the gate's
 // weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
 // columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.
@@ -384,13 +404,14 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       TileCoord c = GROUPED ? TileCoord{0, 0} : tile_coord(tile_id, num_m, num_n);
       const int m_blk = c.m_tile * CG + static_cast<int>(rank);
       int row = m_blk * BLOCK_M + row_in_tile;
-      bool row_ok = row < p.M;
+      int row_end = p.M;
       if (GROUPED) {
         const int mt = w / num_n;
         c.n_blk = w - mt * num_n;
         row = __ldg(p.grp_tiles + 3 * mt + 1) + row_in_tile;
-        row_ok = row < __ldg(p.grp_tiles + 3 * mt + 2);
+        row_end = __ldg(p.grp_tiles + 3 * mt + 2);
       }
+      const bool row_ok = row < row_end;
       mbar_wait(&tmem_full[acc], acc_phase);
       tc_fence_after();
       const uint32_t t_acc = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
@@ -514,62 +535,58 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         const int col0 = c.n_blk * BN + ch * 64;
         if (EPI == EPI_F32 && GROUPED && p.out_bf16 != nullptr && p.act == 2) {
           // grouped up projection with the squared ReLU formed here: a chunk yields 64 activations of this row
-          if (row_ok) {
-            const float rw = p.row_scale != nullptr ? p.row_scale[row] : 1.f;
-            __nv_bfloat16* orow = p.out_bf16 + static_cast<long>(row) * p.out_stride + col0;
+          const float rw = p.row_scale != nullptr && row_ok ? p.row_scale[row] : 1.f;
+          uint32_t pk[32];
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                if (col0 + h * 32 + j >= p.N) continue;     // N % 8 == 0
-                uint32_t pk[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float a0 = fmaxf(rw * __uint_as_float(v[h][j + 2 * e]), 0.f), a1 = fmaxf(rw * __uint_as_float(v[h][j + 2 * e + 1]), 0.f);
-                  pk[e] = pack_bf16x2(a0 * a0, a1 * a1);
-                }
-                *reinterpret_cast<uint4*>(orow + h * 32 + j) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-              }
+          for (int j = 0; j < 32; ++j) {
+            const float a0 = fmaxf(rw * __uint_as_float(v[j >> 4][(j & 15) * 2]), 0.f), a1 = fmaxf(rw * __uint_as_float(v[j >> 4][(j & 15) * 2 + 1]), 0.f);
+            pk[j] = pack_bf16x2(a0 * a0, a1 * a1);
           }
+          warp_rows_out(slab, pk, lane, [&](int, int r, int q, const uint4& x) {      // N % 8 == 0
+            const int rr = row - lane + r, col = col0 + q * 8;
+            if (rr < row_end && col < p.N) *reinterpret_cast<uint4*>(p.out_bf16 + static_cast<long>(rr) * p.out_stride + col) = x;
+          });
         } else if (EPI == EPI_F32 && GROUPED && p.out_bf16 != nullptr) {
           // grouped gate / up projection with the SwiGLU formed here: B rows are interleaved per 32 features ([32 gate | 32 up]
-          // in every 64-column chunk), so a chunk yields 32 activations of this row: 64 contiguous bytes, plain masked stores
+          // in every 64-column chunk), so a chunk yields 32 activations of this row: 64 contiguous bytes
           const int f0 = c.n_blk * (BN / 2) + ch * 32;
-          if (row_ok && f0 < p.N / 2) {
-            const float rw = p.row_scale != nullptr ? p.row_scale[row] : 1.f;      // a weight on the expert's input: gate and up scale with it
-            __nv_bfloat16* orow = p.out_bf16 + static_cast<long>(row) * p.out_stride + f0;
+          if (f0 < p.N / 2) {
+            const float rw = p.row_scale != nullptr && row_ok ? p.row_scale[row] : 1.f;      // a weight on the expert's input: gate and up scale with it
+            uint32_t pk[16];
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              uint32_t pk[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float g0 = rw * __uint_as_float(v[0][j + 2 * e]), g1 = rw * __uint_as_float(v[0][j + 2 * e + 1]);
-                const float u0 = rw * __uint_as_float(v[1][j + 2 * e]), u1 = rw * __uint_as_float(v[1][j + 2 * e + 1]);
-                pk[e] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
-              }
-              *reinterpret_cast<uint4*>(orow + j) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            for (int e = 0; e < 16; ++e) {
+              const float g0 = rw * __uint_as_float(v[0][2 * e]), g1 = rw * __uint_as_float(v[0][2 * e + 1]);
+              const float u0 = rw * __uint_as_float(v[1][2 * e]), u1 = rw * __uint_as_float(v[1][2 * e + 1]);
+              pk[e] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
             }
+            warp_rows_out(slab, pk, lane, [&](int, int r, int q, const uint4& x) {
+              const int rr = row - lane + r;
+              if (rr < row_end) *reinterpret_cast<uint4*>(p.out_bf16 + static_cast<long>(rr) * p.out_stride + f0 + q * 8) = x;
+            });
           }
         } else if (EPI == EPI_F32) {
-          // fp32 row-major out (+)= alpha * acc : thread = row, 2 x 128 contiguous bytes per chunk
-          if (row_ok) {
-            float* orow = p.out_f32 + static_cast<long>(row) * p.out_f32_stride + col0;
+          // fp32 row-major out (+)= alpha * acc: 128 contiguous bytes of four rows at a time; N % 4 == 0 (checked on the host)
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+          for (int h = 0; h < 2; ++h) {
+            const int cl = col0 + h * 32 + (lane & 7) * 4, r0 = row - lane + (lane >> 3);      // this lane's column and first row
+            float4* dst = reinterpret_cast<float4*>(p.out_f32 + static_cast<long>(r0) * p.out_f32_stride + cl);
+            float4 old[8];
+            if (!GROUPED && p.accumulate) {
 #pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                const int col = col0 + h * 32 + j;
-                if (col < p.N) {                        // N % 4 == 0 (checked on the host)
-                  float4 o = make_float4(__uint_as_float(v[h][j]) * p.alpha, __uint_as_float(v[h][j + 1]) * p.alpha,
-                                         __uint_as_float(v[h][j + 2]) * p.alpha, __uint_as_float(v[h][j + 3]) * p.alpha);
-                  float4* dst = reinterpret_cast<float4*>(orow + h * 32 + j);
-                  if (p.accumulate) {
-                    const float4 old = *dst;
-                    o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                  }
-                  *dst = o;
-                }
+              for (int i = 0; i < 8; ++i)
+                if (r0 + 4 * i < row_end && cl < p.N) old[i] = dst[i * p.out_f32_stride];
+            }
+            uint32_t x[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(__uint_as_float(v[h][j]) * p.alpha);
+            warp_rows_out(slab, x, lane, [&](int i, int, int, const uint4& y) {
+              if (r0 + 4 * i >= row_end || cl >= p.N) return;
+              float4 o = make_float4(__uint_as_float(y.x), __uint_as_float(y.y), __uint_as_float(y.z), __uint_as_float(y.w));
+              if (!GROUPED && p.accumulate) {
+                o.x += old[i].x; o.y += old[i].y; o.z += old[i].z; o.w += old[i].w;
               }
+              dst[i * p.out_f32_stride] = o;
+            });
           }
         } else if (EPI == EPI_SWIGLU) {
           // every 64-column chunk of the accumulator is [32 gate | 32 up] of the same 32 features (weight rows interleaved at
