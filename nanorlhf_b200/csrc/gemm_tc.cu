@@ -528,6 +528,12 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           break;
         }
         uint32_t v[2][32];
+        float gate_scale = 0.f, up_scale = 0.f;          // FP8 SwiGLU: lane l holds those of the chunk's columns l and 32 + l
+        if (FP8 && EPI == EPI_SWIGLU) {
+          const int cl = c.n_blk * BN + ch * 64 + lane;
+          if (cl < p.N) gate_scale = __ldg(p.col_scale + cl);
+          if (cl + 32 < p.N) up_scale = __ldg(p.col_scale + cl + 32);
+        }
         tmem_ld_32x32b_x32(t_acc + ch * 64, v[0]);
         tmem_ld_32x32b_x32(t_acc + ch * 64 + 32, v[1]);
         tmem_ld_wait();
@@ -599,9 +605,8 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             float g0 = __uint_as_float(v[0][j]), g1 = __uint_as_float(v[0][j + 1]);
             float u0 = __uint_as_float(v[1][j]), u1 = __uint_as_float(v[1][j + 1]);
             if (FP8) {
-              const int cg_ = min(col0 + j, p.N - 2), cu_ = min(col0 + 32 + j, p.N - 2);
-              g0 *= rs8 * p.col_scale[cg_]; g1 *= rs8 * p.col_scale[cg_ + 1];
-              u0 *= rs8 * p.col_scale[cu_]; u1 *= rs8 * p.col_scale[cu_ + 1];
+              g0 *= rs8 * __shfl_sync(0xffffffffu, gate_scale, j); g1 *= rs8 * __shfl_sync(0xffffffffu, gate_scale, j + 1);
+              u0 *= rs8 * __shfl_sync(0xffffffffu, up_scale, j); u1 *= rs8 * __shfl_sync(0xffffffffu, up_scale, j + 1);
             }
             const uint32_t pk = pack_bf16x2(g0 / (1.f + exp2f(-g0 * kLog2e)) * u0, g1 / (1.f + exp2f(-g1 * kLog2e)) * u1);
             if ((ch & 1) == 0) sw_packed[j / 2] = pk;     // static indices: the array stays in registers
