@@ -763,7 +763,7 @@ struct PolicyLossFn : public torch::autograd::Function<PolicyLossFn> {
                                                 double kl_coef) {
     if (ref_lp.has_value()) ref_lp = ref_lp->contiguous();
     auto [loss, grad, stats] = policy_loss(new_lp.contiguous(), old_lp.contiguous(), adv.contiguous(), mask.contiguous(), ref_lp, cliprange, kl_coef);
-    ctx->save_for_backward({grad, own_scalars(stats)[0]});
+    ctx->save_for_backward({grad, stats.select(0, 0).variable_data()});
     ctx->mark_non_differentiable({stats});
     return {loss, stats};
   }
@@ -777,7 +777,7 @@ struct ValueLossFn : public torch::autograd::Function<ValueLossFn> {
   static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, torch::Tensor vpred, torch::Tensor vold, torch::Tensor ret,
                                                 torch::Tensor mask, double clip) {
     auto [loss, grad, stats] = value_loss(vpred.contiguous(), vold.contiguous(), ret.contiguous(), mask.contiguous(), clip);
-    ctx->save_for_backward({grad, own_scalars(stats)[0]});
+    ctx->save_for_backward({grad, stats.select(0, 0).variable_data()});
     ctx->mark_non_differentiable({stats});
     return {loss, stats};
   }
