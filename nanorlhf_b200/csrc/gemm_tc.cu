@@ -214,6 +214,7 @@ template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, boo
 NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
                              const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* tmA3 = nullptr) {
   using C = Cfg<CG, BN, B_MN>;
+  constexpr bool kPlainStores = EPI == EPI_F32 || EPI == EPI_GRP_SWIGLU || EPI == EPI_GRP_RELU2;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBarOff);      // CG = 2: the leader's are the live ones
   uint64_t* empty_bar = full_bar + C::kStages;                              // per CTA (multicast commit)
@@ -246,7 +247,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       tma_prefetch_desc(&tmA2);
       tma_prefetch_desc(&tmB2);
     }
-    if (EPI != EPI_F32) tma_prefetch_desc(&tmD);
+    if (!kPlainStores) tma_prefetch_desc(&tmD);
   }
   if (warp == 1 && lane == 0) {
     for (int i = 0; i < C::kStages; ++i) {
@@ -539,7 +540,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         tmem_ld_wait();
         if ((EPI == EPI_SWIGLU ? ((it + 1) >> 1) * 4 + group * 2 + ((it + 1) & 1) : ch + 2) >= BN / 64) release_acc();      // its last one
         const int col0 = c.n_blk * BN + ch * 64;
-        if (EPI == EPI_F32 && GROUPED && p.out_bf16 != nullptr && p.act == 2) {
+        if (EPI == EPI_GRP_RELU2) {
           // grouped up projection with the squared ReLU formed here: a chunk yields 64 activations of this row
           const float rw = p.row_scale != nullptr && row_ok ? p.row_scale[row] : 1.f;
           uint32_t pk[32];
@@ -552,7 +553,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             const int rr = row - lane + r, col = col0 + q * 8;
             if (rr < row_end && col < p.N) *reinterpret_cast<uint4*>(p.out_bf16 + static_cast<long>(rr) * p.out_stride + col) = x;
           });
-        } else if (EPI == EPI_F32 && GROUPED && p.out_bf16 != nullptr) {
+        } else if (EPI == EPI_GRP_SWIGLU) {
           // grouped gate / up projection with the SwiGLU formed here: B rows are interleaved per 32 features ([32 gate | 32 up]
           // in every 64-column chunk), so a chunk yields 32 activations of this row: 64 contiguous bytes
           const int f0 = c.n_blk * (BN / 2) + ch * 32;
@@ -660,7 +661,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
-    if (EPI != EPI_F32 && !SPLIT && lane == 0) tma_store_wait<0>();
+    if (!kPlainStores && !SPLIT && lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -695,27 +696,34 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   gemm_tc_body<2, 256, false, false, EPI_SWIGLU, false, false, false, false, true>(tmA, up ? tmBu : tmBg, tmA2g, up ? tmB2u : tmB2g, tmD, p, &tmA2u);
 }
 
-template <int BN>
+// FORM: one kernel for each epilogue; with all three behind run-time branches in one kernel steps of 64 to 256 tokens took half a microsecond longer per GEMM
+template <int BN, int FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
-  gemm_tc_body<1, BN, false, false, EPI_F32, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
+  gemm_tc_body<1, BN, false, false, FORM, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
 }
-template <int BN>
-static cudaError_t launch_grouped(const CUtensorMap* maps, const TcParams& p, int max_tiles, int num_sms, cudaStream_t stream) {
+template <int BN, int FORM>
+static cudaError_t launch_grouped_form(const CUtensorMap* maps, const TcParams& p, int units, cudaStream_t stream) {
   using C = Cfg<1, BN, false>;
-  const int num_n = (p.N + BN - 1) / BN;
-  long units = static_cast<long>(max_tiles) * num_n;
-  if (units > num_sms) units = num_sms;
-  if (units < 1) units = 1;
-  auto kern = gemm_tc_grouped_kernel<BN>;
+  auto kern = gemm_tc_grouped_kernel<BN, FORM>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  kern<<<static_cast<int>(units), kThreads, C::kTotal, stream>>>(maps[0], maps[1], p);
+  kern<<<units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], p);
   return cudaGetLastError();
+}
+template <int BN>
+static cudaError_t launch_grouped(const CUtensorMap* maps, const TcParams& p, int max_tiles, int num_sms, cudaStream_t stream) {
+  const int num_n = (p.N + BN - 1) / BN;
+  long units = static_cast<long>(max_tiles) * num_n;
+  if (units > num_sms) units = num_sms;
+  if (units < 1) units = 1;
+  const int n = static_cast<int>(units);
+  if (p.out_bf16 == nullptr) return launch_grouped_form<BN, EPI_F32>(maps, p, n, stream);
+  return p.act == 2 ? launch_grouped_form<BN, EPI_GRP_RELU2>(maps, p, n, stream) : launch_grouped_form<BN, EPI_GRP_SWIGLU>(maps, p, n, stream);
 }
 
 template <int BN>

@@ -11,6 +11,8 @@ enum TcEpilogue : int {
   EPI_BF16 = 0,      // D (bf16, TMA store) = alpha * acc (+ bias) (GELU)
   EPI_F32 = 1,       // out_f32 (row-major, plain stores) (+)= alpha * acc
   EPI_DLOGITS = 3,   // D (bf16, TMA store) = (onehot(target) - exp(alpha * acc - lse)) * grad * alpha: backward of the log-prob head
+  EPI_GRP_SWIGLU = 4,  // GROUPED: out_bf16 [rows, N / 2] = silu(gate) * up of row_scale * acc, B rows interleaved as for EPI_SWIGLU, plain stores
+  EPI_GRP_RELU2 = 5,   // GROUPED: out_bf16 [rows, N] = relu(row_scale * acc)^2, plain stores
   EPI_SWIGLU = 2,    // D[M, N/2] (bf16, TMA store) = silu(gate) * up; B rows interleaved per 32 features [32 gate | 32 up]
 };
 
