@@ -183,13 +183,10 @@ NRL_DEVICE void tma_store_3d(const CUtensorMap* m, const void* smem_src, int c0,
                ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 
-// FP8: A and B are e4m3 bytes, K-major (a 128-byte swizzle row = 128 contraction elements), the MMA is kind::f8f6f4
-// (K = 32 per instruction, twice the bf16 rate) and the epilogue applies the per-row (token) and per-column (output
-// channel) dequantisation scales -- the sampler's fp8 rollout GEMMs.
 // 32 rows of W words, one row per lane, handed out in pieces of 16 bytes so that W / 4 neighbouring lanes hold neighbouring pieces of a row:
 // put(step, row, piece, words).  The plain stores of the float and grouped epilogues go through it: a lane per row wrote 16 bytes into each of 32
-// lines at a time, which eight warps at once took longer for than four (4096 x 1536
-// -> 151 936 floats 1699 us, with eight 1893, handed out 1469; added to 3552, 1590; 16 384 tokens over 64 experts 721, 900, 563).
+// lines at a time, which eight warps at once took longer for than four (4096 x 1536 -> 151 936
+// floats 1699 us, with eight 1893, handed out 1469; added to 3552, 1590; 16 384 tokens over 64 experts 721, 900, 563).
 template <int W, class F>
 NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F&& put) {
   constexpr int P = W / 4;
@@ -206,6 +203,9 @@ NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F
   }
 }
 
+// FP8: A and B are e4m3 bytes, K-major (a 128-byte swizzle row = 128 contraction elements), the MMA is kind::f8f6f4
+// (K = 32 per instruction, twice the bf16 rate) and the epilogue applies the per-row (token) and per-column (output
+// channel) dequantisation scales -- the sampler's fp8 rollout GEMMs.
 // PAIR (CTA pairs, BN = 256): act = silu(x Wg^T) * (x Wu^T) from two separate weights.  The leader loads 128 rows of the gate's
 // weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
 // columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.
