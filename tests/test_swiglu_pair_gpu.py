@@ -23,7 +23,7 @@ def test_swiglu_linears_against_float64(M, K, F, r):
         want.append(y)
     want = torch.nn.functional.silu(want[0]) * want[1]
     got = gemm.swiglu_linears(x, *weights, scaling=0.25)
-    # the adapters' inner product and the result are rounded to bf16 (2^-9 each)
+    # gate, up, the adapters' inner product and the result are rounded to bf16 (2^-9 at most, 1.7e-3 in the root mean square each): 3.3e-3 together
     assert ((got.double() - want).norm() / want.norm()).item() < 4e-3
 
 
