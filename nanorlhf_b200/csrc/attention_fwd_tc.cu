@@ -4,7 +4,7 @@
 //   warp 0       TMA producer : Q tiles, then K_0, V_0, K_1, V_1 ... into a ring of four 32 KB tiles (128B-swizzled panels of 64 dims)
 //   warp 1       MMA issuer   : S_X = Q_X K_j^T, then per block O_X += P_X V_j and at once the next S_X, tiles alternating, so that the
 //                               tensor pipe works on one tile while the other is in its softmax
-//   warp 2       finds the next item (which sequence, which rows) while the current one is computed
+//   warp 2       finds the next item (which sequence, which rows) while the current one is computed, the first one during the set-up
 //   warps 4..11  one thread per query row: scores from TMEM, mask, online softmax (attention_tc.cuh), P as bf16 back into TMEM over its
 //                scores, where it is the A operand of P V; O / l and LSE at the end.  The next item's queries and first keys arrive meanwhile.
 // One persistent CTA per SM (TMEM 512 columns, 193 KB of shared memory).  Items go from the most to the fewest key blocks over all
@@ -94,10 +94,26 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncwarp();
     tmem_alloc(tmem_ptr, 512);
   }
-  int level = 0;                                                     // warp 2: blocks of the longest sequence
+  // warp 2: the blocks of the longest sequence and the first item, while barriers and tensor memory are set up
+  const int* cu = p.cu_seqlens;
+  int level = 0, above = 0, upto = 0;                                // row blocks with an index > level, >= level
+  auto item_of = [&](uint32_t k) {
+    const int at = (k & 1) ? (k + 1) * gridDim.x - 1 - blockIdx.x : k * gridDim.x + blockIdx.x;
+    const int rank = at / p.Hq;
+    while (level > 0 && rank >= upto) {
+      --level;
+      above = upto;
+      upto = attn_blocks_from<kTcBM>(cu, p.num_seqs, level, lane);
+    }
+    if (rank >= upto) return make_int4(-1, 0, 0, 0);
+    const int src = attn_nth_sequence<kTcBM>(cu, p.num_seqs, level, rank - above, lane);
+    return make_int4(at - rank * p.Hq, level * kTcBM, cu[src], cu[src + 1] - cu[src]);
+  };
+  int4 next = make_int4(-1, 0, 0, 0);
   if (warp == 2) {
-    for (int s = lane; s < p.num_seqs; s += 32) level = max(level, (p.cu_seqlens[s + 1] - p.cu_seqlens[s] + kTcBM - 1) / kTcBM);
+    for (int s = lane; s < p.num_seqs; s += 32) level = max(level, (cu[s + 1] - cu[s] + kTcBM - 1) / kTcBM);
     level = __reduce_max_sync(0xffffffffu, level);
+    next = item_of(0);
   }
   tc_fence_before();
   __syncthreads();
@@ -203,21 +219,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       __syncwarp();
     } else if (warp == 2) {
       // ============================== items ==============================
-      const int* cu = p.cu_seqlens;
-      int above = 0, upto = 0;                                       // row blocks with an index > level, >= level
       for (uint32_t k = 0;; ++k) {
-        const int at = (k & 1) ? (k + 1) * gridDim.x - 1 - blockIdx.x : k * gridDim.x + blockIdx.x;
-        const int rank = at / p.Hq;
-        while (level > 0 && rank >= upto) {
-          --level;
-          above = upto;
-          upto = attn_blocks_from<kTcBM>(cu, p.num_seqs, level, lane);
-        }
-        int4 it = make_int4(-1, 0, 0, 0);
-        if (rank < upto) {
-          const int src = attn_nth_sequence<kTcBM>(cu, p.num_seqs, level, rank - above, lane);
-          it = make_int4(at - rank * p.Hq, level * kTcBM, cu[src], cu[src + 1] - cu[src]);
-        }
+        const int4 it = next;
         mbar_wait(&tab_empty[k & 1], ((k >> 1) & 1) ^ 1);
         if (lane == 0) {
           *reinterpret_cast<int4*>(smem + L::kTab + (k & 1) * 16) = it;
@@ -225,6 +228,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
         __syncwarp();
         if (it.x < 0) break;
+        next = item_of(k + 1);
       }
     }
   } else {
@@ -254,7 +258,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int key0 = j * kAtBN;
         // only the block on the diagonal needs a mask: the others end before the tile's first row
         if (j == n - 1) attn_mask_block(sv, 0, min(row, it.len - 1) - key0, 0);
-        attn_softmax_block<false>(sv, p.scale_log2, t_s, t_o, j == 0, m_run, l_run);
+        attn_softmax_block<false>(sv, p.scale_log2, t_s, t_o, j == 0, m_run, l_run, it.len - key0 <= 64);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready[x]);

@@ -136,7 +136,8 @@ NRL_DEVICE void attn_mask_block(uint32_t (&sv)[4][32], int lo, int hi, int keep)
 
 // Thread = one row of S (128 scores in registers, raw; -inf where masked).  Replaces the scores by P = 2^(s * scale - m) in TMEM
 // (bf16), updates the running maximum / sum and rescales the row of O when its maximum moved by more than 2^8 (a stale maximum is
-// harmless below that: P stays under 256 and the sum is kept in float).  `first`: O holds nothing yet.
+// harmless below that: P stays under 256 and the sum is kept in float).  `first`: O holds nothing yet.  `half`: columns 64 and up are all masked
+// and their P is not read.
 // EXACT, for results that leave no statistic of the sum: the maximum is the row's own in every block, so that its largest weight is
 // exactly 1, and the sum adds the weights as P V sees them, rounded.  Error against float64, 16 x 2048 tokens with window 1024: 2.51e-3, lazily
 // and with unrounded sums 2.56e-3, mma.sync kernel 2.52e-3; it costs 349 -> 368 us.  (A sum whose logarithm the backward forms P from adds unrounded weights.)
@@ -144,7 +145,8 @@ NRL_DEVICE void attn_mask_block(uint32_t (&sv)[4][32], int lo, int hi, int keep)
 // a tile's scores to its P and on to the next scores.  A share of the 2^x on the FMA pipe (polynomial) brought nothing: 430 -> 438 / 454 us with
 // 2 / 3 of 8 pairs at 16 x 2048 tokens.
 template <bool EXACT>
-NRL_DEVICE void attn_softmax_block(uint32_t (&sv)[4][32], float scale, uint32_t t_p, uint32_t t_o, bool first, float& m_run, float& l_run) {
+NRL_DEVICE void attn_softmax_block(uint32_t (&sv)[4][32], float scale, uint32_t t_p, uint32_t t_o, bool first, float& m_run, float& l_run,
+                                   bool half = false) {
   float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
   for (int c = 0; c < 4; ++c)
@@ -161,6 +163,7 @@ NRL_DEVICE void attn_softmax_block(uint32_t (&sv)[4][32], float scale, uint32_t 
   float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
+    if (h == 1 && half) break;
     uint32_t pv[32];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
