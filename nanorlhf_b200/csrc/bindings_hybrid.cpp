@@ -806,6 +806,8 @@ void bind_hybrid(pybind11::module_& m) {
         pybind11::arg("act") = 1);
   m.def("ssd_scan", &ssd_scan, "state-space scan with a scalar decay per head, state carried per slot");
   m.def("delta_prep", &delta_prep, "unit q / k, beta and decays of the gated delta rule");
+  m.def("delta_scan_chunked", &nrl_delta_scan_chunked, "a step goes 32 tokens at a time", pybind11::arg("E"), pybind11::arg("T"), pybind11::arg("heads"),
+        pybind11::arg("D"), pybind11::arg("Dv"), pybind11::arg("num_sms"));
   m.def("delta_scan_blocked", &nrl_delta_scan_blocked, "a step goes four tokens at a time", pybind11::arg("E"), pybind11::arg("T"), pybind11::arg("D"),
         pybind11::arg("Dv"));
   m.def("delta_scan", &delta_scan, "gated delta rule scan, state carried per slot");

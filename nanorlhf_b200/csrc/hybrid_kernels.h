@@ -158,11 +158,15 @@ cudaError_t nrl_gla_prep(float* qkv, long sq, const float* a_raw, long sa, const
 
 // Gated delta rule scan.  Per head: S = g S (rows);  u = beta (v - S^T k);  S += k u^T;  o = S^T q.
 // beta == nullptr: plain accumulation, u = v (gated linear attention: S = diag(g) S + k v^T).
-// state float [slots, heads, D, Dv];  o float [T, heads*Dv].  `impl`: 0 picks (nrl_delta_scan_blocked: four tokens at a time, else column-resident),
-// 1 column-resident, 2 row groups, 3 state in shared memory, 4 four tokens at a time (D <= 128).
+// state float [slots, heads, D, Dv];  o float [T, heads*Dv].  `impl`: 0 picks (nrl_delta_scan_chunked, nrl_delta_scan_blocked, else column-resident),
+// 1 column-resident, 2 row groups, 3 state in shared memory, 4 four tokens at a time (D <= 128), 5 32 at a time (D <= 128, one decay per head).
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
                            float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
                            int D, int Dv, int per_channel, int impl, int num_sms, cudaStream_t s);
+cudaError_t nrl_delta_chunk_tc(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state, float* o,
+                               const int* cu, const int* start, const int* state_slot, int E, int heads, int kv_heads, int D, int Dv,
+                               bool rows16, cudaStream_t s);      // rows16: rows of q, k and v start and end on 16-byte boundaries
+int nrl_delta_scan_chunked(long E, long T, int heads, int D, int Dv, int num_sms);      // one decay per head: impl 0 takes a step of E entries and T tokens 32 at a time
 int nrl_delta_scan_blocked(long E, long T, int D, int Dv);       // impl 0 takes a step of E entries and T tokens four tokens at a time
 
 // Per-head RMS norm (weight [D], shared by heads) of q in place and of k into the paged cache; v into the paged cache.

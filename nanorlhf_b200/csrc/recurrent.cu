@@ -1306,7 +1306,7 @@ cudaError_t nrl_gla_prep(float* qkv, long sq, const float* a_raw, long sa, const
   return cudaGetLastError();
 }
 
-// Steps of prompt portions take four tokens at a time.  Where the column-resident form fits (Dv <= 256) the lines are
+// Other steps of prompt portions (a decay per key channel above all) take four tokens at a time.  Where the column-resident form fits (Dv <= 256) the lines are
 //   D > 32      a smaller state is padded to 64 rows here, to 16 or 32 there: 64 entries of 128 tokens, 16 heads of 32 x 32, 230 us against 83; one
 //               row more, 33 x 33, 237 / 316
 //   T >= 20 E   a thread's state is not read in whole lines, so that short portions pay more for it: 128 x 128, 64 entries of 2: 95 us against 50,
@@ -1318,11 +1318,30 @@ int nrl_delta_scan_blocked(long E, long T, int D, int Dv) {
   return D <= 128 && (col_form_fits(Dv, D) ? D > 32 && T >= 20 * E : T >= 12 * E);
 }
 
+// One decay per head and rows of q, k and v on 16-byte boundaries: 32 tokens at a time on the tensor cores (delta_chunk_tc.cu), where a block has an SM to itself
+// and starts with 64 KB of state, so that short portions need a full state and many portions need more tokens each.  us there / the better of the others,
+// 16 heads (E x heads blocks; one to a block of 128 columns):
+//   any state, blocks <= SMs, T >= 20 E   1 x 20 tokens 64 x 64: 14 / 15, 128 x 128: 15 / 23; 1 x 2000, 128 x 128: 310 / 1450
+//   128 x 128, T >= 20 E                  16 x 20: 29 / 43; 64 x 20: 99 / 156; 16 x 2048: 630 / 2290; 64 single tokens beside a portion of 2000 take the same line
+//   64 x 128, T >= 32 E                   256 x 20: 293 / 264, x 32: 305 / 345
+//   128 x 64 (half the lanes), T >= 48 E  256 x 20: 366 / 285, x 32: 375 / 377, x 48: 517 / 497; 32 x 48: 75 / 72, x 64: 74 / 93
+//   64 x 64, T >= 128 E                   256 x 64: 445 / 331; 128 x 96: 285 / 265, x 128: 343 / 343; 64 x 128: 190 / 235
+// Rows that are not aligned come float by float: 64 x 256 tokens, 33 x 33: 531 / 456; they stay with four tokens at a time.
+int nrl_delta_scan_chunked(long E, long T, int heads, int D, int Dv, int num_sms) {
+  if (D <= 32 || D > 128 || T < 20 * E) return 0;
+  if (E * heads * ((Dv + 127) / 128) <= num_sms) return 1;
+  return T >= (Dv > 64 ? (D > 64 ? 20 : 32) : (D > 64 ? 48 : 128)) * E;
+}
+
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
                            float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
                            int D, int Dv, int per_channel, int impl, int num_sms, cudaStream_t s) {
   if (E <= 0) return cudaSuccess;
-  if (Dv > 512 || heads % kv_heads != 0 || impl < 0 || impl > 4) return cudaErrorInvalidValue;
+  if (Dv > 512 || heads % kv_heads != 0 || impl < 0 || impl > 5) return cudaErrorInvalidValue;
+  const bool rows16 = D % 4 == 0 && Dv % 4 == 0 && sq % 4 == 0 && col_k % 4 == 0 && col_v % 4 == 0 && reinterpret_cast<uintptr_t>(qkv) % 16 == 0;
+  if (!per_channel && D >= 1 && D <= 128 && Dv >= 1 && (impl == 5 || (impl == 0 && rows16 && nrl_delta_scan_chunked(E, T, heads, D, Dv, num_sms))))
+    return nrl_delta_chunk_tc(qkv, sq, col_k, col_v, beta, decay, state, o, cu, start, state_slot, E, heads, kv_heads, D, Dv, rows16, s);
+  if (impl == 5) return cudaErrorInvalidValue;
   if (D >= 1 && D <= 128 && Dv >= 1 && (impl == 4 || (impl == 0 && nrl_delta_scan_blocked(E, T, D, Dv)))) {
     const bool wide = D % 4 == 0 && sq % 4 == 0 && col_k % 4 == 0 && reinterpret_cast<uintptr_t>(qkv) % 16 == 0 &&
                      reinterpret_cast<uintptr_t>(decay) % 16 == 0;

@@ -46,7 +46,7 @@ def causal_conv(x, w, bias, state, out, plan, in_bias=None, act: str = "silu"):
                        {"none": 0, "silu": 1}[act])
 
 
-SCAN_IMPLS = {"auto": 0, "column": 1, "rows": 2, "shared": 3, "blocked": 4}        # "blocked": four tokens at a time, delta_scan only
+SCAN_IMPLS = {"auto": 0, "column": 1, "rows": 2, "shared": 3, "blocked": 4, "chunked": 5}        # four / 32 tokens at a time, delta_scan only
 
 
 def ssd_scan(xbc, col_b, col_c, dt_raw, dt_bias, A_log, D, state, y, plan, groups, impl: str = "auto"):
