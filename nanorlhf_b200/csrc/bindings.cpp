@@ -952,6 +952,38 @@ torch::Tensor deberta_attn_fwd(const torch::Tensor& q, const torch::Tensor& k, c
   return out;
 }
 
+// The same on tcgen05 for up to 512 buckets; the kernel forms content to position itself.  pos_k: [H, NB, 64] bf16 (a view of the [NB, H * 64] projection).
+torch::Tensor deberta_attn_tc(const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, const torch::Tensor& cu_seqlens, int64_t max_seqlen,
+                              double scale, const torch::Tensor& pos_k, const torch::Tensor& rel_b, const torch::Tensor& lut) {
+  check_thd(q, "q"); check_thd(k, "k"); check_thd(v, "v");
+  TORCH_CHECK(cu_seqlens.scalar_type() == torch::kInt32 && cu_seqlens.is_contiguous());
+  TORCH_CHECK(pos_k.is_cuda() && pos_k.scalar_type() == torch::kBFloat16 && pos_k.dim() == 3 && pos_k.stride(2) == 1 && pos_k.stride(0) == 64);
+  TORCH_CHECK(rel_b.is_cuda() && rel_b.is_contiguous() && rel_b.scalar_type() == torch::kBFloat16 && rel_b.dim() == 3);
+  TORCH_CHECK(lut.is_cuda() && lut.scalar_type() == torch::kInt16 && lut.is_contiguous());
+  c10::cuda::CUDAGuard guard(q.device());
+  const int T = q.size(0), H = q.size(1), D = q.size(2), NB = rel_b.size(2);
+  TORCH_CHECK(D == 64 && k.size(0) == T && k.size(1) == H && k.size(2) == 64 && v.size(0) == T && v.size(1) == H && v.size(2) == 64);
+  TORCH_CHECK(rel_b.size(0) == H && rel_b.size(1) == T && pos_k.size(0) == H && pos_k.size(1) == NB && pos_k.size(2) == 64);
+  TORCH_CHECK(NB % 8 == 0 && NB >= 8 && NB <= 512);
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(q.data_ptr()) % 16 == 0 && q.stride(0) % 8 == 0, "q must have rows on 16-byte boundaries");
+  const int center = (lut.numel() - 1) / 2;
+  TORCH_CHECK(center >= max_seqlen + 63, "bucket LUT is too short for max_seqlen (needs a 64-entry margin)");
+  torch::Tensor out = torch::empty({T, H, D}, q.options());
+  if (T == 0) return out;
+  auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const uint64_t cols = static_cast<uint64_t>(H) * D, rows_b = static_cast<uint64_t>(H) * T, pitch_b = static_cast<uint64_t>(NB) * 2;
+  const CUtensorMap maps[5] = {
+      nrl::make_tma_2d(pos_k.data_ptr(), NB, cols, pos_k.stride(1) * 2, 64, 64, bf, 2),
+      nrl::make_tma_2d(k.data_ptr(), T, cols, k.stride(0) * 2, 64, 64, bf, 2),
+      nrl::make_tma_2d(v.data_ptr(), T, cols, v.stride(0) * 2, 64, 64, bf, 2),
+      nrl::make_tma_2d_plain(rel_b.data_ptr(), rows_b, NB, pitch_b, 8, 144, bf, 2),
+      nrl::make_tma_2d_plain(rel_b.data_ptr(), rows_b, NB, pitch_b, 64, 8, bf, 2)};
+  check(nrl_deberta_attn_tc(maps, q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), cu_seqlens.data_ptr<int>(), cu_seqlens.numel() - 1, T, H,
+                            static_cast<float>(scale), reinterpret_cast<const short*>(lut.data_ptr()), center, NB, num_sms(), cur_stream()),
+        "deberta_attn_tc");
+  return out;
+}
+
 // y = LayerNorm(x + residual) (residual optional); bf16 [rows, d], d <= 2048
 torch::Tensor add_layernorm(const torch::Tensor& x, const c10::optional<torch::Tensor>& residual, const torch::Tensor& w,
                             const torch::Tensor& b, double eps) {
@@ -1195,6 +1227,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_varlen_bwd", &attn_varlen_bwd);
   m.def("attn_bwd_tc", &attn_bwd_tc);
   m.def("deberta_attn_fwd", &deberta_attn_fwd);
+  m.def("deberta_attn_tc", &deberta_attn_tc);
   m.def("attn_fwd_tc", &attn_fwd_tc, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("cu_seqlens"), py::arg("scale"));
   m.def("kv_cache_write_fp8", &kv_cache_write_fp8, py::arg("k"), py::arg("v"), py::arg("kq"), py::arg("vq"), py::arg("ks"), py::arg("vs"),
         py::arg("slot_mapping"), py::arg("src_index") = py::none());

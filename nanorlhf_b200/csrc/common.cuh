@@ -90,6 +90,22 @@ NRL_DEVICE void mbar_wait(uint64_t* bar, uint32_t parity) {
     }
   }
 }
+// The same for kernels in which many warps wait while others compute: a try lasts 20 us (the hint keeps waiting warps from taking issue slots) and the bound
+// is a count of tries, not the clock, whose code at every wait would pass through the instruction cache.
+NRL_DEVICE void mbar_wait_quiet(uint64_t* bar, uint32_t parity) {
+  for (uint32_t n = 0;;) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2, %3;\n\t"
+        "selp.b32 %0, 1, 0, P;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
+        : "memory");
+    if (ok) return;
+    if (++n == (1u << 20)) __trap();
+  }
+}
 
 // ------------------------------------------------------------------------------------------------
 // TMA (cp.async.bulk.tensor) -- descriptors are built on the host (tma_host.h)

@@ -79,23 +79,6 @@ NRL_DEVICE void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]) {
                : "memory");
 }
 
-// Bounded by a count (20 us at most per try: the hint keeps waiting warps from taking issue slots), not by the clock, whose code thirty times over
-// would pass through the instruction cache once per chunk.
-NRL_DEVICE void dc_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t n = 0;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred P;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2, %3;\n\t"
-        "selp.b32 %0, 1, 0, P;\n\t}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
-        : "memory");
-    if (ok) return;
-    if (++n == (1u << 20)) __trap();
-  }
-}
-
 // product of two numbers that are each the sum of two floats
 NRL_DEVICE float2 mul_wide(float2 a, float2 b) {
   const float p = a.x * b.x;
@@ -227,13 +210,13 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
       const uint32_t ph = n & 1, ph2 = (n >> 1) & 1;
       const float* sc = reinterpret_cast<const float*>(smem + L::kSc + st * L::kScStage);
       float u[kC], r[kC];
-      dc_wait(&raw_full[st], ph2);
+      mbar_wait_quiet(&raw_full[st], ph2);
       const float* v = reinterpret_cast<const float*>(smem + L::kRaw + st * L::kRawStage + L::kRawV) + (warp & 3) * 32 + lane;
 #pragma unroll
       for (int i = 0; i < kC; ++i) u[i] = v[i * 128];
       mbar_arrive(&raw_free[st]);
-      dc_wait(&kq_full[st], ph2);
-      dc_wait(rk_full, ph);
+      mbar_wait_quiet(&kq_full[st], ph2);
+      mbar_wait_quiet(rk_full, ph);
       tc_fence_after();
       auto read_rq = [&](int c, uint32_t (&a)[16]) {       // sixteen columns of S^T [K; Q]
         tmem_ld_32x32b_x16(tmem + Tm::kR1 + c + lane_off, a);
@@ -257,7 +240,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
             u[c + i + 3] = b4.w * (u[c + i + 3] - c4.w * __uint_as_float(x[i + 3]));
           }
         }
-        dc_wait(&lm_full[st], ph2);
+        mbar_wait_quiet(&lm_full[st], ph2);
         const float* lj = reinterpret_cast<const float*>(smem + L::kL + st * L::kLStage);
 #pragma unroll
         for (int i = 0; i < kC; ++i) r[i] = 0.f;           // a sum of its own: smaller than u, and so are its roundings
@@ -274,7 +257,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
           }
         }
       }
-      dc_wait(rq_full, ph);                                // the terms of S, which U's go over, have been read
+      mbar_wait_quiet(rq_full, ph);                                // the terms of S, which U's go over, have been read
       tc_fence_after();
       // Terms of U: scaled for the state, then as they are for the outputs.  The products of a row of U reach tokens before u_j with a weight of
       // zero: a value that is not finite would spoil them, so it is taken out in front of the second pass, and its token and all behind it
@@ -330,7 +313,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
       tc_fence_before();
       mbar_arrive(u_full);
       mbar_arrive(&sc_free[st]);
-      dc_wait(o2_full, ph);
+      mbar_wait_quiet(o2_full, ph);
       tc_fence_after();
       float* od = p.o + (static_cast<long>(t) * p.heads + h) * p.Dv + col;
       const int left = mine ? t1 - t : 0;
@@ -372,10 +355,10 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
           tc_fence_before();
           mbar_arrive(&sp_full[c]);
         }
-        dc_wait(&kq_full[n & 1], (n >> 1) & 1);
+        mbar_wait_quiet(&kq_full[n & 1], (n >> 1) & 1);
         const float c_n = reinterpret_cast<const float*>(smem + L::kSc + (n & 1) * L::kScStage)[2 * kC - 1];
         mbar_arrive(&sc_free[n & 1]);
-        dc_wait(ds_full, n & 1);
+        mbar_wait_quiet(ds_full, n & 1);
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -395,9 +378,9 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
     } else {
       for (int n = 0; n < n_chunks; ++n) {
         for (int c = 0; c < 4; ++c) mbar_arrive(&sp_full[c]);
-        dc_wait(&kq_full[n & 1], (n >> 1) & 1);
+        mbar_wait_quiet(&kq_full[n & 1], (n >> 1) & 1);
         mbar_arrive(&sc_free[n & 1]);
-        dc_wait(ds_full, n & 1);
+        mbar_wait_quiet(ds_full, n & 1);
       }
     }
   } else if (warp < 16) {
@@ -432,8 +415,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
           if (lane + m < 32) w = mul_wide(w, b);
         }
       }
-      dc_wait(&kq_free[st], ph2 ^ 1);
-      dc_wait(&sc_free[st], ph2 ^ 1);
+      mbar_wait_quiet(&kq_free[st], ph2 ^ 1);
+      mbar_wait_quiet(&sc_free[st], ph2 ^ 1);
       if (warp == 12) {
         float* sc = reinterpret_cast<float*>(smem + L::kSc + st * L::kScStage);
         sc[lane] = beta;
@@ -443,7 +426,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         sc[4 * kC + lane] = 1.f;
       }
       fetch_sc(t + kC);
-      dc_wait(&raw_full[st], ph2);
+      mbar_wait_quiet(&raw_full[st], ph2);
       uint8_t* tile = smem + L::kKQ + st * L::kKQStage;
       const float* raw = reinterpret_cast<const float*>(smem + L::kRaw + st * L::kRawStage);
 #pragma unroll 1
@@ -475,12 +458,12 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
     for (int n = 0; n < n_chunks; ++n) {
       const int st = n & 1;
       const uint32_t ph2 = (n >> 1) & 1;
-      dc_wait(&kq_full[st], ph2);
-      dc_wait(&kq_free[st], ph2 ^ 1);                      // the products that read the stage's Gram matrices
+      mbar_wait_quiet(&kq_full[st], ph2);
+      mbar_wait_quiet(&kq_free[st], ph2 ^ 1);                      // the products that read the stage's Gram matrices
       const float* sc = reinterpret_cast<const float*>(smem + L::kSc + st * L::kScStage);
       const float bi = is_q ? 1.f : sc[gi];
       float2 w = make_float2(1.f, 0.f);                    // G(gi, j)
-      dc_wait(gram_full, n & 1);
+      mbar_wait_quiet(gram_full, n & 1);
       tc_fence_after();
       uint8_t* mt = smem + L::kM + st * L::kMStage;
       float* lj = reinterpret_cast<float*>(smem + L::kL + st * L::kLStage);
@@ -538,7 +521,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
       }
       for (int n = 0; n < n_chunks && (!WIDE || warp == 21); ++n) {
         const int st = n & 1, t = t0 + n * kC;
-        dc_wait(&raw_free[st], ((n >> 1) & 1) ^ 1);
+        mbar_wait_quiet(&raw_free[st], ((n >> 1) & 1) ^ 1);
         float* raw = reinterpret_cast<float*>(smem + L::kRaw + st * L::kRawStage);
         float* rv = reinterpret_cast<float*>(smem + L::kRaw + st * L::kRawStage + L::kRawV);
         if (WIDE) {                                         // a lane per token
@@ -585,8 +568,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
       auto gram = [&](int n) {
         const int st = n & 1;
         const uint64_t d = kq0 + st * (L::kKQStage / 16);
-        dc_wait(&kq_full[st], (n >> 1) & 1);
-        if (n > 0) dc_wait(gram_free, (n - 1) & 1);
+        mbar_wait_quiet(&kq_full[st], (n >> 1) & 1);
+        if (n > 0) mbar_wait_quiet(gram_free, (n - 1) & 1);
         tc_fence_after();
 #pragma unroll 1
         for (int pr = 0; pr < 6; ++pr) {
@@ -611,7 +594,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         // K, which the solve waits for: the small pairs as the terms come
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
-          dc_wait(&sp_full[c], n & 1);
+          mbar_wait_quiet(&sp_full[c], n & 1);
           tc_fence_after();
 #pragma unroll
           for (int pr = 0; pr < 5; ++pr)
@@ -627,7 +610,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
           for (int k = 0; k < 4 * NH; ++k) rq(pr, k, 1, pr == 5 && k >= 2 * NH, (pr == 0 && k == 0) || (pr == 5 && k == 2 * NH));
         dc_commit(leader, rq_full);
         if (n + 1 < n_chunks) gram(n + 1);
-        dc_wait(uh_full, n & 1);
+        mbar_wait_quiet(uh_full, n & 1);
         tc_fence_after();
 #pragma unroll
         for (int hf = 0; hf < NH; ++hf)
@@ -638,8 +621,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
               dc_mma_ts(leader, tmem_u + Tm::kHalf * hf, tmem_u + Tm::uh(pair_a(pr)) + 8 * k, dt + pair_b(pr) * kTerm + hf * kHalfTile + k * 128, id_ds,
                           pr == 0 && k == 0 ? 0u : 1u);
         dc_commit(leader, ds_full);
-        dc_wait(u_full, n & 1);
-        dc_wait(&lm_full[st], (n >> 1) & 1);
+        mbar_wait_quiet(u_full, n & 1);
+        mbar_wait_quiet(&lm_full[st], (n >> 1) & 1);
         tc_fence_after();
 #pragma unroll 1
         for (int pr = 0; pr < 6; ++pr)

@@ -122,7 +122,7 @@ class DisentangledSelfAttention(nn.Module):
     def forward_packed(self, x, cu_seqlens, max_len, lut, rel_emb):
         """x: [T_total, hidden] packed real tokens.  c2p and p2c share the index c = bucket(i-j)+span
         (bucketing is odd in its argument), so score = (Qc.Kc + A[i,c] + B[j,c]) * scale with
-        A = Qc Kr^T and B = Kc Qr^T -- two small GEMMs feeding the fused attention kernel."""
+        A = Qc Kr^T and B = Kc Qr^T.  B is a small GEMM; A is one too where it does not fit into shared memory (more than 512 buckets)."""
         from ..ops import native
         T = x.shape[0]
         q = self.query_proj(x).view(T, self.h, self.dh)
@@ -130,12 +130,17 @@ class DisentangledSelfAttention(nn.Module):
         v = self.value_proj(x).view(T, self.h, self.dh)
         pos_k = self.key_proj(rel_emb).view(-1, self.h, self.dh).transpose(0, 1)          # [H, NB, dh]
         pos_q = self.query_proj(rel_emb).view(-1, self.h, self.dh).transpose(0, 1)
-        # the two bias tables A = Qc Kr^T and B = Kc Qr^T ([H, T, NB]): per head a [T, 64] x [NB, 64]^T product on the general
+        # the bias tables A = Qc Kr^T and B = Kc Qr^T ([H, T, NB]): per head a [T, 64] x [NB, 64]^T product on the general
         # tcgen05 GEMM; the per-head operands are column slices of the packed projections (no copies)
-        rel_a, rel_b = _bias_tables(q, pos_k), _bias_tables(k, pos_q)
+        rel_b = _bias_tables(k, pos_q)
         scale = 1.0 / math.sqrt(self.dh * self.scale_factor)
         native._count()
-        if os.environ.get("NANORLHF_DEBERTA_TMA", "1") != "0" and self.dh == 64:
+        tma = os.environ.get("NANORLHF_DEBERTA_TMA", "1") != "0" and self.dh == 64
+        if tma and pos_k.shape[1] <= 512:
+            out = native.ext().deberta_attn_tc(q, k, v, cu_seqlens, int(max_len), scale, pos_k, rel_b, lut)      # forms A itself, in shared memory
+            return out.reshape(T, -1)
+        rel_a = _bias_tables(q, pos_k)
+        if tma:
             # every tile (Q, K, V and the two sliding bias-table windows) arrives by TMA
             out = native.ext().deberta_attn_fwd(q, k, v, cu_seqlens, int(max_len), scale, rel_a, rel_b, lut)
         else:

@@ -1,0 +1,70 @@
+"""Disentangled attention on tcgen05 (csrc/attention_deberta_tc.cu) against float64, at the edges of its tiles (128 queries, 64 keys, 64 buckets)."""
+import math
+
+import pytest
+import torch
+
+from nanorlhf_b200.models.deberta_v3 import build_bucket_lut
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(lens, heads, buckets, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    T = sum(lens)
+    qkv = torch.randn(T, 3, heads, 64, generator=g, device="cuda").bfloat16()
+    pos_k, pos_q = (torch.randn(buckets, heads, 64, generator=g, device="cuda").bfloat16().transpose(0, 1) for _ in range(2))
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    return [qkv[:, i].contiguous() for i in range(3)], pos_k, pos_q, cu
+
+
+def _reference(qkv, pos_k, rel_b, lut, lens, scale):
+    q, k, v = (t.double().transpose(0, 1) for t in qkv)
+    rel_a = torch.bmm(q.float(), pos_k.float().transpose(1, 2)).bfloat16().double()          # rounded as the kernel rounds it
+    out, s0, center = [], 0, (lut.numel() - 1) // 2
+    for n in lens:
+        i, r = torch.arange(n, device="cuda"), slice(s0, s0 + n)
+        c = lut.long()[i[:, None] - i[None, :] + center][None].expand(q.shape[0], n, n)
+        s = q[:, r] @ k[:, r].transpose(1, 2) + rel_a[:, r].gather(2, c) + rel_b[:, r].double().gather(2, c.transpose(1, 2)).transpose(1, 2)
+        out.append((torch.softmax(s * scale, -1) @ v[:, r]).transpose(0, 1))
+        s0 += n
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("lens,heads,span,top", [
+    ([1], 16, 256, 512), ([64], 2, 256, 512), ([65], 1, 256, 512), ([128, 129, 1, 63], 3, 256, 512), ([700, 40, 1], 2, 256, 512),
+    ([1663, 640, 641], 2, 256, 512),                 # blocks with one bucket for all differences
+    ([1300], 2, 16, 64), ([500, 90], 2, 4, 16),      # few buckets, far fewer than the 144 columns of a window
+    ([900], 2, 100, 4000),                           # a bucket that still changes at the far end
+    ([2, 3] * 40, 16, 256, 512),                     # more items than SMs
+])
+def test_against_float64(lens, heads, span, top):
+    from nanorlhf_b200.models.deberta_v3 import _bias_tables
+    from nanorlhf_b200.ops import native
+    qkv, pos_k, pos_q, cu = _inputs(lens, heads, 2 * span)
+    lut = build_bucket_lut(max(lens), span, top, span, "cuda")
+    rel_b, scale = _bias_tables(qkv[1], pos_q), 1.0 / math.sqrt(192)
+    got = native.ext().deberta_attn_tc(*qkv, cu, max(lens), scale, pos_k, rel_b, lut)
+    want = _reference(qkv, pos_k, rel_b, lut, lens, scale)
+    # weights and results are rounded to bf16 once each: 2^-9 of every term and 2^-9 of the result.  A sum of A on the other side of a rounding boundary
+    # moves its score by 2^-8 |A| scale and one weight by that factor: below 2^-8 for |A| up to 14, six standard deviations being 48, so one in many
+    assert torch.isfinite(got).all()
+    assert (got.double() - want).norm() <= 2.0 ** -8 * want.norm()
+    assert (got.double() - want).abs().max() <= 2.0 ** -7 * (qkv[2].double().abs().max() + want.abs().max())
+    assert torch.equal(got, native.ext().deberta_attn_tc(*qkv, cu, max(lens), scale, pos_k, rel_b, lut))
+
+
+def test_rows_of_a_wider_projection_and_tables():
+    """q, k and v as columns of one product, against the kernel that reads both tables."""
+    from nanorlhf_b200.models.deberta_v3 import _bias_tables
+    from nanorlhf_b200.ops import native
+    lens, heads = [300, 77], 4
+    qkv, pos_k, pos_q, cu = _inputs(lens, heads, 512, seed=1)
+    lut = build_bucket_lut(300, 256, 512, 256, "cuda")
+    wide = torch.cat([t.reshape(-1, heads * 64) for t in qkv], 1)
+    q, k, v = (wide[:, i * heads * 64:(i + 1) * heads * 64].unflatten(1, (heads, 64)) for i in range(3))
+    got = native.ext().deberta_attn_tc(q, k, v, cu, 300, 0.07, pos_k, _bias_tables(k, pos_q), lut)
+    old = native.ext().deberta_attn_fwd(q, k, v, cu, 300, 0.07, _bias_tables(q, pos_k), _bias_tables(k, pos_q), lut)
+    assert (got.float() - old.float()).norm() <= 2.0 ** -8 * old.float().norm()
+    with pytest.raises(RuntimeError):
+        native.ext().deberta_attn_tc(q, k, v, cu, 301 + 64, 0.07, pos_k, _bias_tables(k, pos_q), lut)
