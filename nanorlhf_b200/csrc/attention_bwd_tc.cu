@@ -23,6 +23,7 @@
 // GRPO/grpo.py:219; training step GRPO/grpo_trainer.py:652).
 #include "attention_tc.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace nrl {
 
@@ -91,6 +92,8 @@ NRL_DEVICE void bwd_chunk(const uint32_t (&sv)[16], const uint32_t (&dv)[16], ui
 // Half a warp per pair, sixteen bytes per lane, two pairs in flight: 12 011 tokens x 28 heads 51 -> 29 us (8 bytes per lane, one pair per warp before)
 __global__ void attn_bwd_delta_tc_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                          float* __restrict__ delta, long o_stride_t, int total, unsigned Hq, unsigned pairs) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int sub = threadIdx.x & 15;
   const unsigned first = (blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4)) * 2;
   uint4 a[2], b[2];
@@ -144,6 +147,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done_bar + 1);
   int* info = reinterpret_cast<int*>(tmem_ptr + 4);      // its own 16-byte slot: tcgen05.alloc writes next to it
 
+  pdl_wait();
   int behind, blocks, seq_start, seq_len;
   const int rank = blockIdx.x / (p.Hq / p.G), kvh = blockIdx.x - rank * (p.Hq / p.G);
   if (!bwd_locate(p.cu_seqlens, p.num_seqs, rank, info, behind, blocks, seq_start, seq_len)) return;
@@ -169,6 +173,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
+  pdl_launch_dependents();
   // TMEM columns: S^T[parity] 0/64, dP^T[parity] 128/192, dV 256..383, dK 384..511
 
   if (warp == 0) {
@@ -348,6 +353,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done_bar + 1);
   int* info = reinterpret_cast<int*>(tmem_ptr + 4);      // its own 16-byte slot: tcgen05.alloc writes next to it
 
+  pdl_wait();
   int mb, blocks, seq_start, seq_len;
   const int rank = blockIdx.x / p.Hq, head = blockIdx.x - rank * p.Hq, kvh = head / p.G;
   if (!bwd_locate(p.cu_seqlens, p.num_seqs, rank, info, mb, blocks, seq_start, seq_len)) return;
@@ -370,6 +376,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
+  pdl_launch_dependents();
   // TMEM columns: S[parity] 0/64, dP[parity] 128/192, dQ 256..383
 
   if (warp == 0) {
@@ -512,8 +519,8 @@ extern "C" cudaError_t nrl_attn_bwd_tc(const CUtensorMap* maps, const void* o, c
     configured = true;
   }
   const unsigned pairs = static_cast<unsigned>(total) * Hq;                   // O alone would be a terabyte at 2^32
-  attn_bwd_delta_tc_kernel<<<(pairs + 31) / 32, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), delta,
-                                                            o_stride_t, total, Hq, pairs);
+  launch_dependent(attn_bwd_delta_tc_kernel, (pairs + 31) / 32, 256, 0, s, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), delta,
+                   o_stride_t, total, Hq, pairs);
   AttnBwdParams p;
   p.cu_seqlens = cu; p.lse = lse; p.delta = delta;
   p.dq = static_cast<__nv_bfloat16*>(dq); p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
@@ -521,7 +528,7 @@ extern "C" cudaError_t nrl_attn_bwd_tc(const CUtensorMap* maps, const void* o, c
   p.num_seqs = num_seqs; p.total_tokens = total; p.Hq = Hq; p.G = Hq / Hkv;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   const unsigned most = total / 128 + num_seqs, grid_kv = most * Hkv, grid_q = most * Hq;
-  attn_bwd_dkdv_tc_kernel<<<grid_kv, kBwdThreads, DkdvSmem::kTotal, s>>>(maps[0], maps[1], maps[2], maps[3], p);
-  attn_bwd_dq_tc_kernel<<<grid_q, kBwdThreads, DqSmem::kTotal, s>>>(maps[4], maps[5], maps[6], maps[7], p);
+  launch_dependent(attn_bwd_dkdv_tc_kernel, grid_kv, kBwdThreads, DkdvSmem::kTotal, s, maps[0], maps[1], maps[2], maps[3], p);
+  launch_dependent(attn_bwd_dq_tc_kernel, grid_q, kBwdThreads, DqSmem::kTotal, s, maps[4], maps[5], maps[6], maps[7], p);
   return cudaGetLastError();
 }

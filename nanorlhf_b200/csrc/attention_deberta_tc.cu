@@ -21,6 +21,7 @@
 // 54 + 24, 4 x 700 48 / 59 + 15, 16 x 40 11.5 / 6.7 + 8.8, so that it is left only where A does not fit (more than 512 buckets).
 #include "attention_tc.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace nrl {
 namespace {
@@ -201,6 +202,8 @@ deberta_attn_tc_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
+  pdl_wait();
+  pdl_launch_dependents();
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
@@ -589,6 +592,7 @@ extern "C" cudaError_t nrl_deberta_attn_tc(const CUtensorMap* maps, const void* 
   const cudaError_t e = cudaFuncSetAttribute(deberta_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DbSmem::kTotal);
   if (e != cudaSuccess) return e;
   const long most = static_cast<long>(total / kDbBM + num_seqs) * heads;
-  deberta_attn_tc_kernel<<<static_cast<int>(most < num_sms ? most : num_sms), kDbThreads, DbSmem::kTotal, s>>>(maps[0], maps[1], maps[2], maps[3], maps[4], p);
+  launch_dependent(deberta_attn_tc_kernel, static_cast<int>(most < num_sms ? most : num_sms), kDbThreads, DbSmem::kTotal, s, maps[0], maps[1], maps[2], maps[3],
+                   maps[4], p);
   return cudaGetLastError();
 }

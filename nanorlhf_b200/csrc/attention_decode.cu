@@ -15,6 +15,7 @@
 // (GRPO/grpo_trainer.py:142).
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace nrl {
 
@@ -48,6 +49,8 @@ __global__ void kv_cache_write_kernel(const __nv_bfloat16* __restrict__ k, const
                                       long k_stride_t, long v_stride_t, __nv_bfloat16* __restrict__ k_cache,
                                       __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ slot_mapping,
                                       const int* __restrict__ src_index, int T, int Hkv) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int vec_per_tok = Hkv * (kHeadDim / 8);
   const long total = static_cast<long>(T) * vec_per_tok;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
@@ -81,6 +84,8 @@ struct DecodeParams {
 };
 
 __global__ void __launch_bounds__(kDecWarps * 32, 2) paged_decode_kernel(DecodeParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(1024) uint8_t smem[];
   // layout: [warp][stage][K page | V page] , then Q tile [16][128] bf16 (4 KB)
   uint8_t* q_tile = smem + kDecWarps * kDecStages * 2 * kPageBytes;
@@ -254,6 +259,8 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2) paged_decode_kernel(DecodeP
 }
 
 __global__ void decode_merge_splits_kernel(DecodeParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int seq = blockIdx.x, kvh = blockIdx.y;
   for (int i = threadIdx.x; i < p.G * kHeadDim; i += blockDim.x) {
     const int r = i / kHeadDim, d = i % kHeadDim;
@@ -283,8 +290,7 @@ extern "C" cudaError_t nrl_kv_cache_write(const void* k, const void* v, long k_s
   long total = static_cast<long>(T) * Hkv * (kHeadDim / 8);
   long blocks = (total + 255) / 256;
   if (blocks > 148L * 8) blocks = 148L * 8;
-  kv_cache_write_kernel<<<static_cast<int>(blocks), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), k_stride_t, v_stride_t,
+  launch_dependent(kv_cache_write_kernel, static_cast<int>(blocks), 256, 0, s, static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), k_stride_t, v_stride_t,
       static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), slot_mapping, src_index, T, Hkv);
   return cudaGetLastError();
 }
@@ -319,11 +325,11 @@ extern "C" cudaError_t nrl_paged_decode(const void* q, long q_stride_s, const vo
     configured = true;
   }
   dim3 grid(S, Hkv, splits);
-  paged_decode_kernel<<<grid, kDecWarps * 32, smem, s>>>(p);
+  launch_dependent(paged_decode_kernel, grid, kDecWarps * 32, smem, s, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (splits > 1) {
-    decode_merge_splits_kernel<<<dim3(S, Hkv), 128, 0, s>>>(p);
+    launch_dependent(decode_merge_splits_kernel, dim3(S, Hkv), 128, 0, s, p);
     e = cudaGetLastError();
   }
   return e;

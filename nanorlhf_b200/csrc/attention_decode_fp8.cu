@@ -23,6 +23,7 @@
 // (GRPO/grpo_trainer.py:142).
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace nrl {
 
@@ -66,6 +67,8 @@ __global__ void kv_cache_write_fp8_kernel(const __nv_bfloat16* __restrict__ k, c
                                           uint8_t* __restrict__ vq, float* __restrict__ ks, float* __restrict__ vs,
                                           const int* __restrict__ slot_mapping, const int* __restrict__ src_index,
                                           int pairs, int Hkv) {
+  pdl_wait();
+  pdl_launch_dependents();
   const long widx = blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (widx >= static_cast<long>(pairs) * Hkv) return;
   const int lane = threadIdx.x & 31;
@@ -114,6 +117,8 @@ struct Decode8Params {
 };
 
 __global__ void __launch_bounds__(kWarps8 * 32, 3) paged_decode_fp8_kernel(Decode8Params p) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(128) uint8_t smem[];
   const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -283,6 +288,8 @@ __global__ void __launch_bounds__(kWarps8 * 32, 3) paged_decode_fp8_kernel(Decod
 }
 
 __global__ void decode8_merge_splits_kernel(Decode8Params p) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int seq = blockIdx.x, kvh = blockIdx.y;
   for (int i = threadIdx.x; i < p.G * kHd; i += blockDim.x) {
     const int r = i / kHd, d = i % kHd;
@@ -310,8 +317,7 @@ extern "C" cudaError_t nrl_kv_cache_write_fp8(const void* k, const void* v, long
   if (head_dim != kHd || page != kPg) return cudaErrorInvalidValue;
   if (pairs == 0) return cudaSuccess;
   const long warps = static_cast<long>(pairs) * Hkv;
-  kv_cache_write_fp8_kernel<<<static_cast<int>((warps + 7) / 8), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), k_stride_t, v_stride_t,
+  launch_dependent(kv_cache_write_fp8_kernel, static_cast<int>((warps + 7) / 8), 256, 0, s, static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), k_stride_t, v_stride_t,
       static_cast<uint8_t*>(kq), static_cast<uint8_t*>(vq), ks, vs, slot_mapping, src_index, pairs, Hkv);
   return cudaGetLastError();
 }
@@ -340,11 +346,11 @@ extern "C" cudaError_t nrl_paged_decode_fp8(const void* q, long q_stride_s, cons
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  paged_decode_fp8_kernel<<<dim3(S, Hkv, splits), kWarps8 * 32, smem, s>>>(p);
+  launch_dependent(paged_decode_fp8_kernel, dim3(S, Hkv, splits), kWarps8 * 32, smem, s, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (splits > 1) {
-    decode8_merge_splits_kernel<<<dim3(S, Hkv), 128, 0, s>>>(p);
+    launch_dependent(decode8_merge_splits_kernel, dim3(S, Hkv), 128, 0, s, p);
     e = cudaGetLastError();
   }
   return e;

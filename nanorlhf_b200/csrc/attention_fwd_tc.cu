@@ -17,6 +17,7 @@
 // (attn_implementation="flash_attention_2", GRPO/grpo.py:219) on the training, log-prob and prefill paths.
 #include "attention_tc.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace nrl {
 
@@ -94,6 +95,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncwarp();
     tmem_alloc(tmem_ptr, 512);
   }
+  pdl_wait();
   // warp 2: the blocks of the longest sequence and the first item, while barriers and tensor memory are set up
   const int* cu = p.cu_seqlens;
   int level = 0, above = 0, upto = 0;                                // row blocks with an index > level, >= level
@@ -119,6 +121,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
+  pdl_launch_dependents();
 
   if (warp < 4) {
     attn_regs_issue();
@@ -314,6 +317,6 @@ extern "C" cudaError_t nrl_attn_fwd_tc(const CUtensorMap* tmQ, const CUtensorMap
     configured = true;
   }
   const long most = static_cast<long>(total / kTcBM + num_seqs) * Hq;
-  attn_fwd_tc_kernel<<<static_cast<int>(most < num_sms ? most : num_sms), kAtThreads, AttnTcSmem::kTotal, s>>>(*tmQ, *tmK, *tmV, p);
+  launch_dependent(attn_fwd_tc_kernel, static_cast<int>(most < num_sms ? most : num_sms), kAtThreads, AttnTcSmem::kTotal, s, *tmQ, *tmK, *tmV, p);
   return cudaGetLastError();
 }

@@ -29,6 +29,10 @@ NRL_DEVICE bool elect_one() {
   return pred != 0;
 }
 
+// Launches that overlap the end of the kernel in front (launch.h)
+NRL_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+NRL_DEVICE void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename T>
 NRL_DEVICE T warp_sum(T v) {
 #pragma unroll

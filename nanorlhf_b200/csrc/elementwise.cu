@@ -4,6 +4,7 @@
 // vLLM's fused_add_rms_norm / rotary_embedding / silu_and_mul in the rollout path.
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace nrl {
 
@@ -17,6 +18,8 @@ __global__ void __launch_bounds__(128) rmsnorm_kernel(const __nv_bfloat16* __res
                                                       __nv_bfloat16* __restrict__ y,
                                                       __nv_bfloat16* __restrict__ residual_out,
                                                       float* __restrict__ rstd_out, int d, float eps) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int row = blockIdx.x;
   const int nvec = d / 8;
   const uint4* xv = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * d);
@@ -85,6 +88,8 @@ __global__ void __launch_bounds__(128) rmsnorm_bwd_kernel(const __nv_bfloat16* _
                                                           const __nv_bfloat16* __restrict__ gy,
                                                           const float* __restrict__ rstd_in,
                                                           __nv_bfloat16* __restrict__ gx, int d) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int row = blockIdx.x;
   const int nvec = d / 8;
   const float rstd = rstd_in[row];
@@ -162,6 +167,8 @@ template <int NV, bool FULL, bool RES>
 __global__ void __launch_bounds__(32 * kNormWarps)
 rmsnorm_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ w,
                     __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ residual_out, float* __restrict__ rstd_out, int rows, int d, float eps) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int row = blockIdx.x * kNormWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31, nvec = d / 8;
   if (row >= rows) return;
   const size_t off = static_cast<size_t>(row) * d;
@@ -199,6 +206,8 @@ template <int NV, bool FULL>
 __global__ void __launch_bounds__(32 * kNormWarps)
 rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ gy,
                         const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ gx, int rows, int d) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int row = blockIdx.x * kNormWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31, nvec = d / 8;
   if (row >= rows) return;
   const size_t off = static_cast<size_t>(row) * d;
@@ -232,6 +241,8 @@ template <int NV, bool FULL>
 __global__ void __launch_bounds__(32 * kNormWarps)
 add_layernorm_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ w,
                           const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y, int rows, int d, float eps) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int row = blockIdx.x * kNormWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31, nvec = d / 8;
   if (row >= rows) return;
   const size_t off = static_cast<size_t>(row) * d;
@@ -279,6 +290,8 @@ add_layernorm_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t, int T, int H, int D,
                             long x_stride_t, long y_stride_t, float sin_sign) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int half = D / 2;
   const int vec_per_head = half / 8;                 // 8 pairs per thread-iteration
   const long total = static_cast<long>(T) * H * vec_per_head;
@@ -314,6 +327,8 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* 
 // gate_up: [T, 2F] = [gate | up]; out[T, F] = silu(gate) * up
 __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up, long in_stride,
                               __nv_bfloat16* __restrict__ out, long T, int F) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int vecs = F / 8;
   const long total = T * vecs;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
@@ -338,6 +353,8 @@ __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gate, const __nv
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up, long in_stride,
                                   const __nv_bfloat16* __restrict__ gout, __nv_bfloat16* __restrict__ dgate,
                                   __nv_bfloat16* __restrict__ dup, long out_stride, long T, int F) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int vecs = F / 8;
   const long total = T * vecs;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
@@ -395,16 +412,16 @@ extern "C" cudaError_t nrl_rmsnorm(const void* x, const void* residual, const vo
   if (d <= 3584) {
     const int blocks = (rows + kNormWarps - 1) / kNormWarps;
 #define NRL_CALL(NV_, FULL_)                                                                                                           \
-  if (residual != nullptr) rmsnorm_warp_kernel<NV_, FULL_, true><<<blocks, 32 * kNormWarps, 0, s>>>(X, R, W, Y, RO, rstd, rows, d, eps); \
-  else rmsnorm_warp_kernel<NV_, FULL_, false><<<blocks, 32 * kNormWarps, 0, s>>>(X, nullptr, W, Y, nullptr, rstd, rows, d, eps)
+  if (residual != nullptr) launch_dependent(rmsnorm_warp_kernel<NV_, FULL_, true>, blocks, 32 * kNormWarps, 0, s, X, R, W, Y, RO, rstd, rows, d, eps); \
+  else launch_dependent(rmsnorm_warp_kernel<NV_, FULL_, false>, blocks, 32 * kNormWarps, 0, s, X, nullptr, W, Y, nullptr, rstd, rows, d, eps)
     NRL_NORM_DISPATCH(d, NRL_CALL)
 #undef NRL_CALL
     return cudaGetLastError();
   }
   if (residual != nullptr)
-    rmsnorm_kernel<true><<<rows, 128, 0, s>>>(X, R, W, Y, RO, rstd, d, eps);
+    launch_dependent(rmsnorm_kernel<true>, rows, 128, 0, s, X, R, W, Y, RO, rstd, d, eps);
   else
-    rmsnorm_kernel<false><<<rows, 128, 0, s>>>(X, nullptr, W, Y, nullptr, rstd, d, eps);
+    launch_dependent(rmsnorm_kernel<false>, rows, 128, 0, s, X, nullptr, W, Y, nullptr, rstd, d, eps);
   return cudaGetLastError();
 }
 
@@ -413,8 +430,7 @@ extern "C" cudaError_t nrl_add_layernorm(const void* x, const void* residual, co
   if (d % 8 != 0 || d > 2048) return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
 #define NRL_CALL(NV_, FULL_)                                                                                                              \
-  add_layernorm_warp_kernel<NV_, FULL_><<<(rows + kNormWarps - 1) / kNormWarps, 32 * kNormWarps, 0, s>>>(                                  \
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual), static_cast<const __nv_bfloat16*>(w),            \
+  launch_dependent(add_layernorm_warp_kernel<NV_, FULL_>, (rows + kNormWarps - 1) / kNormWarps, 32 * kNormWarps, 0, s, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual), static_cast<const __nv_bfloat16*>(w),            \
       static_cast<const __nv_bfloat16*>(b), static_cast<__nv_bfloat16*>(y), rows, d, eps)
   if (d == 1024) NRL_CALL(4, true);
   else if (d < 1024) NRL_CALL(4, false);
@@ -429,14 +445,13 @@ extern "C" cudaError_t nrl_rmsnorm_bwd(const void* x, const void* w, const void*
   if (rows == 0) return cudaSuccess;
   if (d <= 3584) {
 #define NRL_CALL(NV_, FULL_)                                                                                                          \
-  rmsnorm_bwd_warp_kernel<NV_, FULL_><<<(rows + kNormWarps - 1) / kNormWarps, 32 * kNormWarps, 0, s>>>(                                \
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(gy), rstd,        \
+  launch_dependent(rmsnorm_bwd_warp_kernel<NV_, FULL_>, (rows + kNormWarps - 1) / kNormWarps, 32 * kNormWarps, 0, s, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(gy), rstd,        \
       static_cast<__nv_bfloat16*>(gx), rows, d)
     NRL_NORM_DISPATCH(d, NRL_CALL)
 #undef NRL_CALL
     return cudaGetLastError();
   }
-  rmsnorm_bwd_kernel<<<rows, 128, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
+  launch_dependent(rmsnorm_bwd_kernel, rows, 128, 0, s, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
                                           static_cast<const __nv_bfloat16*>(gy), rstd,
                                           static_cast<__nv_bfloat16*>(gx), d);
   return cudaGetLastError();
@@ -447,7 +462,7 @@ extern "C" cudaError_t nrl_rope(const void* x, void* y, const float* cos_t, cons
   if (D % 16 != 0) return cudaErrorInvalidValue;
   long total = static_cast<long>(T) * H * (D / 16);
   if (total == 0) return cudaSuccess;
-  rope_kernel<<<grid_for(total, 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x),
+  launch_dependent(rope_kernel, grid_for(total, 256), 256, 0, s, static_cast<const __nv_bfloat16*>(x),
                                                    static_cast<__nv_bfloat16*>(y), cos_t, sin_t, T, H, D, x_stride_t,
                                                    y_stride_t, sin_sign);
   return cudaGetLastError();
@@ -457,7 +472,7 @@ extern "C" cudaError_t nrl_swiglu(const void* gate, const void* up, long in_stri
                                   cudaStream_t s) {
   if (F % 8 != 0 || in_stride % 8 != 0) return cudaErrorInvalidValue;
   if (T == 0) return cudaSuccess;
-  swiglu_kernel<<<grid_for(T * (F / 8), 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(gate),
+  launch_dependent(swiglu_kernel, grid_for(T * (F / 8), 256), 256, 0, s, static_cast<const __nv_bfloat16*>(gate),
                                                           static_cast<const __nv_bfloat16*>(up), in_stride,
                                                           static_cast<__nv_bfloat16*>(out), T, F);
   return cudaGetLastError();
@@ -467,8 +482,7 @@ extern "C" cudaError_t nrl_swiglu_bwd(const void* gate, const void* up, long in_
                                       void* dup, long out_stride, long T, int F, cudaStream_t s) {
   if (F % 8 != 0 || in_stride % 8 != 0 || out_stride % 8 != 0) return cudaErrorInvalidValue;
   if (T == 0) return cudaSuccess;
-  swiglu_bwd_kernel<<<grid_for(T * (F / 8), 256), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up), in_stride,
+  launch_dependent(swiglu_bwd_kernel, grid_for(T * (F / 8), 256), 256, 0, s, static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up), in_stride,
       static_cast<const __nv_bfloat16*>(gout), static_cast<__nv_bfloat16*>(dgate), static_cast<__nv_bfloat16*>(dup),
       out_stride, T, F);
   return cudaGetLastError();

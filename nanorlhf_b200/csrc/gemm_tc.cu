@@ -31,6 +31,7 @@
 // (K = 64) 235 -> 92 us each; nothing changes above K = 4096.
 #include "common.cuh"
 #include "gemm_tc.h"
+#include "launch.h"
 
 namespace nrl {
 namespace tc {
@@ -234,9 +235,6 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   const int splits = SPLIT ? p.splits : 1;
   const int kb_per_split = (num_kb + splits - 1) / splits;
   const int tiles_per_batch = num_m * num_n;
-  // SPLIT: work item = (tile, k-range), splits of a tile adjacent.  BATCH: work item = (batch, tile), third TMA coordinate
-  // GROUPED: work item = (row tile of the device-side table, column block); the column blocks of a row tile are adjacent
-  const int num_work = GROUPED ? __ldg(p.grp_num_tiles) * num_n : tiles_per_batch * (BATCH ? p.batch : splits);
   const int unit = blockIdx.x / CG, num_units = gridDim.x / CG;
   volatile int* s_last = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
@@ -269,6 +267,11 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
+  pdl_wait();
+  pdl_launch_dependents();
+  // SPLIT: work item = (tile, k-range), splits of a tile adjacent.  BATCH: work item = (batch, tile), third TMA coordinate
+  // GROUPED: work item = (row tile of the device-side table, column block); the column blocks of a row tile are adjacent
+  const int num_work = GROUPED ? __ldg(p.grp_num_tiles) * num_n : tiles_per_batch * (BATCH ? p.batch : splits);
 
   if (warp == 0) {
     // ================================ TMA producer (every CTA) ================================
@@ -712,7 +715,7 @@ static cudaError_t launch_grouped_form(const CUtensorMap* maps, const TcParams& 
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  kern<<<units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], p);
+  launch_dependent(kern, units, kThreads, C::kTotal, stream, maps[0], maps[1], p);
   return cudaGetLastError();
 }
 template <int BN>
@@ -765,7 +768,7 @@ static cudaError_t launch_fp8(const CUtensorMap* maps, const TcParams& p, int nu
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    kern<<<units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], p);
+    launch_dependent(kern, units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   } else {
     auto kern = gemm_tc_fp8_cg2_kernel<BN, EPI>;
     if (!configured) {
@@ -773,7 +776,7 @@ static cudaError_t launch_fp8(const CUtensorMap* maps, const TcParams& p, int nu
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    kern<<<2 * units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], p);
+    launch_dependent(kern, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   }
   return cudaGetLastError();
 }
@@ -793,7 +796,7 @@ static cudaError_t launch_batched(const CUtensorMap* maps, const TcParams& p, in
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    kern<<<static_cast<int>(units), kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], p);
+    launch_dependent(kern, static_cast<int>(units), kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   } else {
     auto kern = gemm_tc_batched_cg2_kernel<BN>;
     if (!configured) {
@@ -801,7 +804,7 @@ static cudaError_t launch_batched(const CUtensorMap* maps, const TcParams& p, in
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    kern<<<static_cast<int>(2 * units), kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], p);
+    launch_dependent(kern, static_cast<int>(2 * units), kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   }
   return cudaGetLastError();
 }
@@ -825,7 +828,7 @@ static cudaError_t launch_splitk(const CUtensorMap* maps, const TcParams& p, int
   const int tiles = ((p.M + BLOCK_M - 1) / BLOCK_M) * ((p.N + BN - 1) / BN);
   int grid = tiles * p.splits;
   if (grid > num_sms) grid = num_sms;
-  kern<<<grid, kThreads, C::kTotal, stream>>>(maps[0], maps[1], p);
+  launch_dependent(kern, grid, kThreads, C::kTotal, stream, maps[0], maps[1], p);
   return cudaGetLastError();
 }
 
@@ -844,7 +847,7 @@ static cudaError_t launch(const CUtensorMap* maps, const TcParams& p, int num_sm
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    kern<<<units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], p);
+    launch_dependent(kern, units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[4], p);
   } else {
     auto kern = gemm_tc_cg2_kernel<BN, A_MN, B_MN, EPI>;
     if (!configured) {
@@ -852,7 +855,7 @@ static cudaError_t launch(const CUtensorMap* maps, const TcParams& p, int num_sm
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    kern<<<2 * units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], p);   // consecutive CTAs pair up
+    launch_dependent(kern, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[4], p);   // consecutive CTAs pair up
   }
   return cudaGetLastError();
 }
@@ -896,7 +899,7 @@ extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::
   int units = ((p->M + 255) / 256) * ((p->N + 255) / 256);
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;
-  gemm_tc_pair_kernel<<<2 * units, kThreads, C::kTotal, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], *p);
+  nrl::launch_dependent(gemm_tc_pair_kernel, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], *p);
   return cudaGetLastError();
 }
 
