@@ -23,6 +23,7 @@
 // (GRPO/grpo_trainer.py:142).
 #include "common.cuh"
 #include "kernels.h"
+#include "decode_merge.cuh"
 #include "launch.h"
 
 namespace nrl {
@@ -287,24 +288,10 @@ __global__ void __launch_bounds__(kWarps8 * 32, 3) paged_decode_fp8_kernel(Decod
   }
 }
 
-__global__ void decode8_merge_splits_kernel(Decode8Params p) {
+__global__ void __launch_bounds__(kMergeD) decode8_merge_splits_kernel(const MergeParams p) {
   pdl_wait();
   pdl_launch_dependents();
-  const int seq = blockIdx.x, kvh = blockIdx.y;
-  for (int i = threadIdx.x; i < p.G * kHd; i += blockDim.x) {
-    const int r = i / kHd, d = i % kHd;
-    const long base = ((static_cast<long>(seq) * p.Hkv + kvh) * p.splits) * 8 + r;
-    float M = -INFINITY;
-    for (int s = 0; s < p.splits; ++s) M = fmaxf(M, p.part_ml[(base + s * 8) * 2]);
-    float L = 0.f, acc = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-      const float ms = p.part_ml[(base + s * 8) * 2];
-      const float c = (ms == -INFINITY) ? 0.f : exp2f(ms - M);
-      L += p.part_ml[(base + s * 8) * 2 + 1] * c;
-      acc += p.part_o[(base + s * 8) * kHd + d] * c;
-    }
-    p.out[(static_cast<long>(seq) * p.Hq + kvh * p.G + r) * kHd + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
-  }
+  merge_decode_parts(p);
 }
 
 }  // namespace nrl
@@ -350,7 +337,8 @@ extern "C" cudaError_t nrl_paged_decode_fp8(const void* q, long q_stride_s, cons
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (splits > 1) {
-    launch_dependent(decode8_merge_splits_kernel, dim3(S, Hkv), 128, 0, s, p);
+    const MergeParams m = {part_o, part_ml, static_cast<__nv_bfloat16*>(out), Hq, Hkv, Hq / Hkv, splits};
+    launch_dependent(decode8_merge_splits_kernel, dim3(S, Hq), kMergeD, 0, s, m);
     e = cudaGetLastError();
   }
   return e;
