@@ -135,20 +135,29 @@ inline void check_tc_operand(const torch::Tensor& t, const char* name) {
 }
 
 // ---- split-K of gemm_tc: into how many ranges the contraction of a product [M, K] x [K, N] is cut unless the caller says so ----
-// measured (bench/sampler_bench.py, profiles/skinny_gemm_split_sweep_r2.json): the last CTA's reduction reads `splits` partial tiles, so
-// beyond ~4 k-ranges the fix-up costs more than the shorter main loop saves, and work items past one wave (148) cost a second wave
-// (any N: the adapter-input gradient dA = t'^T x is [r, K_in] -- 12 or 24 tiles of a 6.6 k-long contraction)
-// A block of 64 contraction columns takes 0.172 us in a CTA, the fix-up of 128 columns 5.5 us and that of 64 about 2.5, which the blocks saved have to
-// outweigh.  us whole / cut: 128 x 1536 with 1536 columns 8.1 / 11.2, 2560 11.5 / 12.0, 3072 13.3 / 12.6, 8960 31.9 / 18.4; 512 x 1536 (three
-// ranges) 2560 12.5 / 13.4, 3072 14.3 / 13.9; 3300 x 192 (two) 2560 12.6 / 13.6, 3584 16.1 / 15.6; 16 x 64 1024 6.1 / 6.1, 1536 7.7 / 6.5;
-// 6601 x 64 (two) 1536 9.0 / 9.6, 2560 12.5 / 11.7; 8960 x 64 (two) 1500 9.1 / 10.4, 2500 12.7 / 12.7, 3300 15.1 / 14.8.
+// (any N: the adapter-input gradient dA = t'^T x is [r, K_in] -- 12 or 24 tiles of a 6.6 k-long contraction).
+// The number of ranges is the one for which this estimate (us) is least: 0.172 for each block of 64 contraction columns of a range, and for the sum of the parts
+// 1.2 + 0.2 a range where clusters form it (tiles 128 wide; 64 wide 1.0 + 0.1), 5 (2.5) through the workspace, where beyond four ranges it costs more
+// than it saves.  Half a microsecond is left to the uncut product, which takes every tile shape.  us uncut / cut (clusters): 128 x 1536 with 1024
+// columns 6.6 / 6.6 (four), 1536 8.2 / 7.1, 8960 31.9 / 12.8 (eight; through the workspace 18.4 with four); 16 x 1536, 8960 31.6 / 10.3; 3300 x 192 (two) 1536 8.9 / 9.3,
+// 2560 12.3 / 11.4; 6601 x 64 (two) 1536 9.0 / 8.6; 600 x 64, 8960 31.6 / 9.0; dA 64 x 1536, 6601 tokens 24.5 / 9.9; 512 x 1536, 8960
+// 33.8 / 21.1 (three, workspace).
 inline int split_block_n(int64_t N) { return N <= 64 ? 64 : 128; }
 inline int64_t split_tiles(int64_t M, int64_t N) { return ((M + 127) / 128) * ((N + split_block_n(N) - 1) / split_block_n(N)); }
 int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
-  const int64_t tiles = split_tiles(M, N), sms = num_sms();
-  const int64_t blocks = (K + 63) / 64, splits = std::min<int64_t>(std::min<int64_t>(sms / std::max<int64_t>(tiles, 1), blocks / 4), 4);
-  const int64_t worth = split_block_n(N) == 64 ? 16 : 32;                    // blocks saved that pay for the fix-up
-  return tiles * 2 <= sms && splits >= 2 && blocks * (splits - 1) >= worth * splits ? splits : 1;
+  const int64_t tiles = split_tiles(M, N), blocks = (K + 63) / 64;
+  if (tiles < 1 || tiles * 2 > num_sms()) return 1;
+  const bool narrow = split_block_n(N) == 64;
+  double least = 0.172 * blocks - 0.5;
+  int64_t best = 1;
+  for (int64_t s = 2; s <= 8 && tiles * s <= num_sms() && blocks >= 4 * s; ++s) {
+    if (s > 4 && s < 8) continue;                        // 3300 x 64 with 1536 columns: four 6.7 us, five 7.1
+    const bool clusters = tiles <= nrl_gemm_tc_split_clusters(split_block_n(N), static_cast<int>(s));
+    if (!clusters && s > 4) break;
+    const double t = 0.172 * ((blocks + s - 1) / s) + (clusters ? (narrow ? 1.0 + 0.1 * s : 1.2 + 0.2 * s) : narrow ? 2.5 : 5.0);
+    if (t < least) { least = t; best = s; }
+  }
+  return best;
 }
 
 // D[M,N] = alpha * (opA(a) opB(b)^T + opA(a2) opB(b2)^T) (+bias) (GELU).

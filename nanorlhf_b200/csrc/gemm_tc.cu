@@ -49,6 +49,7 @@ constexpr int kStagingBytes = kEpiWarps * kSlabBytes;
 constexpr int kSmemBudget = 227 * 1024;
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;         // clears the CTA-pair peer bit of a shared::cluster address
 constexpr int GROUP_M = 8;                          // tile rows per L2 super-row
+constexpr int kMaxClusterSplits = 8;                // blocks of a portable cluster
 
 template <int CG, int BN, bool B_MN = false>
 struct Cfg {
@@ -75,6 +76,13 @@ NRL_DEVICE uint32_t cluster_ctarank() {
 NRL_DEVICE void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// four floats at the same place of the shared memory of the cluster's block `rank`
+NRL_DEVICE float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+  return v;
 }
 template <int CG>
 NRL_DEVICE void tmem_alloc_cg(uint32_t* smem_dst, uint32_t ncols) {
@@ -211,7 +219,7 @@ NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F
 // weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
 // columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.
 template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, bool BATCH = false, bool FP8 = false, bool GROUPED = false,
-          bool PAIR = false>
+          bool PAIR = false, bool CLUSTER = false>
 NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
                              const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* tmA3 = nullptr) {
   using C = Cfg<CG, BN, B_MN>;
@@ -427,6 +435,21 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         dl_lse = p.lse[row];
         dl_g = p.grad[row] * p.alpha;                       // d logp / d logit carries the 1 / T factor
         dl_target = p.targets[row];
+      }
+      if (CLUSTER) {
+        // ---- split-K by a cluster: the partial tile takes the place of the operands, all of which have been read, in the workspace's layout below ----
+        float* mine = reinterpret_cast<float*>(smem) + row_in_tile * 4;
+#pragma unroll 1
+        for (int ch = group; ch < BN / 32; ch += 2) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(t_acc + ch * 32, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(mine + (ch * 8 + (j >> 2)) * (BLOCK_M * 4)) =
+                make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+        }
+        break;                                             // one tile per block
       }
       if (SPLIT) {
         // ---- split-K: park the fp32 partial tile, the last CTA of the tile reduces all partials in split order ----
@@ -667,8 +690,56 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     if (!kPlainStores && !SPLIT && lane == 0) tma_store_wait<0>();
   }
 
+  if (CLUSTER) {
+    // every block sums a share of the tile over the cluster's parts, in split order
+    __syncwarp();
+    cluster_sync_all();
+    const TileCoord c = tile_coord(unit / splits, num_m, num_n);
+    const int me = unit % splits, units = BLOCK_M * BN / 8;                  // a unit: eight columns of a row
+    const uint32_t part = smem_u32(smem);
+    for (int u = units * me / splits + threadIdx.x; u < units * (me + 1) / splits; u += kThreads) {
+      const int row = c.m_tile * BLOCK_M + (u & (BLOCK_M - 1)), g8 = u / BLOCK_M, col = c.n_blk * BN + g8 * 8;
+      if (row >= p.M || col >= p.N) continue;              // N % 8 == 0
+      const uint32_t at = part + (g8 * 2 * BLOCK_M + (u & (BLOCK_M - 1))) * 16;
+      float acc[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+#pragma unroll 1
+      for (int s0 = 0; s0 < splits; s0 += 4) {
+        float4 x[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (s0 + i < splits) {
+            x[i][0] = ld_cluster_f4(at, s0 + i);
+            x[i][1] = ld_cluster_f4(at + BLOCK_M * 16, s0 + i);
+          }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (s0 + i < splits) {
+            acc[0] += x[i][0].x; acc[1] += x[i][0].y; acc[2] += x[i][0].z; acc[3] += x[i][0].w;
+            acc[4] += x[i][1].x; acc[5] += x[i][1].y; acc[6] += x[i][1].z; acc[7] += x[i][1].w;
+          }
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] *= p.alpha;
+      if (p.bias != nullptr) {
+        const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);      // bias 16-byte aligned
+        const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 bf = unpack_bf16x2(bw[e]);
+          acc[2 * e] += bf.x;
+          acc[2 * e + 1] += bf.y;
+        }
+      }
+      *reinterpret_cast<uint4*>(p.out_bf16 + static_cast<long>(row) * p.out_stride + col) =
+          make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
+    }
+    __syncwarp();
+  }
   tc_fence_before();
-  if (CG == 2) cluster_sync_all();     // nobody leaves (or frees TMEM) while the peer can still signal / read it
+  if (CLUSTER) cluster_sync_all();          // nobody leaves while others read its part
+  else if (CG == 2) cluster_sync_all();     // nobody leaves (or frees TMEM) while the peer can still signal / read it
   else __syncthreads();
   if (warp == 1) {
     tc_fence_after();
@@ -815,6 +886,28 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   gemm_tc_body<1, BN, A_MN, B_MN, EPI_BF16, true>(tmA, tmB, tmA, tmB, tmA, p);
 }
 
+// The same with a tile's ranges in one cluster, which sums its parts through distributed shared memory: the workspace form passes them through L2, and its
+// last block sums them alone while the others have left.  As many clusters as the GPU holds at a time; larger products keep that form.
+template <int BN, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_tc_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
+  gemm_tc_body<1, BN, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
+}
+
+// clusters of `splits` blocks that run at a time
+template <int BN, bool A_MN, bool B_MN>
+static int splitk_clusters(int splits) {
+  using C = Cfg<1, BN, B_MN>;
+  if (splits < 2 || splits > kMaxClusterSplits) return 0;
+  static int fits[kMaxClusterSplits + 1] = {};                               // plus one
+  if (fits[splits] == 0) {
+    auto kern = gemm_tc_splitk_cluster_kernel<BN, A_MN, B_MN>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
+    fits[splits] = 1 + (e == cudaSuccess ? clusters_at_a_time(kern, kThreads, C::kTotal, splits) : 0);
+  }
+  return fits[splits] - 1;
+}
+
 template <int BN, bool A_MN, bool B_MN>
 static cudaError_t launch_splitk(const CUtensorMap* maps, const TcParams& p, int num_sms, cudaStream_t stream) {
   using C = Cfg<1, BN, B_MN>;
@@ -827,6 +920,10 @@ static cudaError_t launch_splitk(const CUtensorMap* maps, const TcParams& p, int
   }
   const int tiles = ((p.M + BLOCK_M - 1) / BLOCK_M) * ((p.N + BN - 1) / BN);
   int grid = tiles * p.splits;
+  if (grid <= num_sms && tiles <= splitk_clusters<BN, A_MN, B_MN>(p.splits)) {
+    launch_dependent_clusters(gemm_tc_splitk_cluster_kernel<BN, A_MN, B_MN>, grid, kThreads, C::kTotal, stream, p.splits, maps[0], maps[1], p);
+    return cudaGetLastError();
+  }
   if (grid > num_sms) grid = num_sms;
   launch_dependent(kern, grid, kThreads, C::kTotal, stream, maps[0], maps[1], p);
   return cudaGetLastError();
@@ -923,6 +1020,10 @@ extern "C" cudaError_t nrl_gemm_tc_grouped(const CUtensorMap* maps, const nrl::t
   if (bn == 128) return launch_grouped<128>(maps, *p, max_tiles, num_sms, stream);
   if (bn == 256) return launch_grouped<256>(maps, *p, max_tiles, num_sms, stream);
   return cudaErrorInvalidValue;
+}
+
+extern "C" int nrl_gemm_tc_split_clusters(int bn, int splits) {
+  return bn == 64 ? nrl::tc::splitk_clusters<64, false, false>(splits) : nrl::tc::splitk_clusters<128, false, false>(splits);
 }
 
 // split-K variant (cta_group::1, bf16 output with plain stores, no second operand pair); maps = {A, B}

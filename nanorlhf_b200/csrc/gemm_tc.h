@@ -32,8 +32,9 @@ struct TcParams {
   long out_f32_stride;
   int accumulate;               // EPI_F32: 1 = add to what is there
   // split-K (SPLIT kernels; small outputs with a long contraction -- LoRA wgrads, rank-r projections): every tile is
-  // computed by `splits` CTAs over disjoint k-ranges; partial tiles go to `ws` (fp32), the last CTA to arrive on the
-  // tile's counter sums them in split order (deterministic) and stores the bf16 result.  Counters reset themselves.
+  // computed by `splits` CTAs over disjoint k-ranges; where they fit they are a cluster that sums its partial tiles through distributed shared memory,
+  // else partial tiles go to `ws` (fp32) and the last CTA to arrive on the tile's counter sums them.  Either way in split order
+  // (deterministic), bf16 result.  Counters reset themselves.
   int splits;
   float* ws;                    // [splits, tiles, 128, BN] fp32
   int* counters;                // [tiles] int32, zero between launches
@@ -50,6 +51,8 @@ struct TcParams {
 }  // namespace tc
 }  // namespace nrl
 
+// how many tiles' ranges clusters of `splits` blocks hold at a time (0: none); the launch decides by its own kernel's figure
+extern "C" int nrl_gemm_tc_split_clusters(int bn, int splits);
 extern "C" cudaError_t nrl_gemm_tc_splitk(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int a_mn, int b_mn, int num_sms,
                                           cudaStream_t stream);
 // EPI_DLOGITS on CTA pairs, 256 x 256 tiles; maps = {A box {128, 64}, B box {128, 64}, D box {32, 64}}
