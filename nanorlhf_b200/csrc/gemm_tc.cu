@@ -29,6 +29,7 @@
 // barrier joins the warps.  With four warps that met at two barriers per chunk and read the bias value by value, a 128 x 256 tile's
 // epilogue took longer than a main loop of K = 1024: the six linears of a reward layer (24 571 tokens) 742 -> 429 us, its bias tables
 // (K = 64) 235 -> 92 us each; nothing changes above K = 4096.
+#include "cluster_read.h"
 #include "common.cuh"
 #include "gemm_tc.h"
 #include "launch.h"
@@ -76,13 +77,6 @@ NRL_DEVICE uint32_t cluster_ctarank() {
 NRL_DEVICE void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// four floats at the same place of the shared memory of the cluster's block `rank`
-NRL_DEVICE float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
-  float4 v;
-  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
-  return v;
 }
 template <int CG>
 NRL_DEVICE void tmem_alloc_cg(uint32_t* smem_dst, uint32_t ncols) {
