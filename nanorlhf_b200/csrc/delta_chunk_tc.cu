@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         float* all = reinterpret_cast<float*>(smem + L::kRaw);
         if (p.D < DP || vcols < 128)                        // columns that no copy reaches
           for (int x = tid; x < 2 * L::kRawStage / 4; x += kDcLoaders) all[x] = 0.f;
+        fence_proxy_async_smem();                           // the zeros lie under what the copies bring: in front of them for the asynchronous proxy too
         named_barrier_sync(1, kDcLoaders);
       }
       for (int n = 0; n < n_chunks && (!WIDE || warp == 21); ++n) {
