@@ -1,6 +1,6 @@
 // tcgen05 / TMEM / TMA flash-attention BACKWARD (causal, packed varlen, GQA, head_dim 128) for sm_100a.
 //
-// Three kernels, no atomics (same decomposition as the mma.sync version in attention_varlen.cu, which stays the oracle):
+// Two kernels, no atomics (same decomposition as the mma.sync version in attention_varlen.cu, which stays the oracle); dK / dV and dQ are blocks of one:
 //   delta   : delta[h, t] = sum_d dO * O                                   (half a warp per (token, head))
 //   dK / dV : one CTA per (128-key block, kv head).  K_j, V_j stay in smem; the CTA streams (q head of the group,
 //             64-row query block) pairs:   S^T = K_j Q_i^T,  dP^T = V_j dO_i^T          (tcgen05, TMEM lanes = keys)
@@ -133,11 +133,9 @@ struct DkdvSmem {
   static constexpr int kTotal = kBar + 256;
 };
 
-__global__ void __launch_bounds__(kBwdThreads, 1)
-attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
-                        const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, AttnBwdParams p) {
+NRL_DEVICE void bwd_dkdv(uint8_t* smem, unsigned block, const CUtensorMap& tmQ, const CUtensorMap& tmDO, const CUtensorMap& tmK,
+                         const CUtensorMap& tmV, const AttnBwdParams& p) {
   using L = DkdvSmem;
-  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* kv_full = reinterpret_cast<uint64_t*>(smem + L::kBar);
   uint64_t* qdo_full = kv_full + 1;            // [kRing]
   uint64_t* qdo_empty = qdo_full + kRing;      // [kRing]
@@ -147,9 +145,8 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done_bar + 1);
   int* info = reinterpret_cast<int*>(tmem_ptr + 4);      // its own 16-byte slot: tcgen05.alloc writes next to it
 
-  pdl_wait();
   int behind, blocks, seq_start, seq_len;
-  const int rank = blockIdx.x / (p.Hq / p.G), kvh = blockIdx.x - rank * (p.Hq / p.G);
+  const int rank = block / (p.Hq / p.G), kvh = block - rank * (p.Hq / p.G);
   if (!bwd_locate(p.cu_seqlens, p.num_seqs, rank, info, behind, blocks, seq_start, seq_len)) return;
   const int kb = blocks - 1 - behind;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -339,11 +336,9 @@ struct DqSmem {
   static constexpr int kTotal = kBar + 256;
 };
 
-__global__ void __launch_bounds__(kBwdThreads, 1)
-attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
-                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, AttnBwdParams p) {
+NRL_DEVICE void bwd_dq(uint8_t* smem, unsigned block, const CUtensorMap& tmQ, const CUtensorMap& tmDO, const CUtensorMap& tmK,
+                       const CUtensorMap& tmV, const AttnBwdParams& p) {
   using L = DqSmem;
-  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + L::kBar);
   uint64_t* kv_full = q_full + 1;              // [kRing]
   uint64_t* kv_empty = kv_full + kRing;        // [kRing]
@@ -353,17 +348,9 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done_bar + 1);
   int* info = reinterpret_cast<int*>(tmem_ptr + 4);      // its own 16-byte slot: tcgen05.alloc writes next to it
 
-  // dQ takes nothing from dK / dV, the kernel in front, whose blocks have all waited for everything before them when the first of these starts (it lets the
-  // next kernel start behind that wait).  So these blocks do not wait and fill the SMs that dK / dV leaves idle: with two key heads it has a block
-  // for two SMs in three (backward of 4 sequences, 6601 tokens, 12 heads over 2: 262 -> 184 us; 6 of 500, 28 over 4: 157 -> 104; 2 of 6005: 1659 -> 1589;
-  // 4 of 6000: 3644 / 3652).  The last block waits before it ends, so that this kernel does not end before that one, for the sake of the next.
-  const bool last = blockIdx.x == gridDim.x - 1;
   int mb, blocks, seq_start, seq_len;
-  const int rank = blockIdx.x / p.Hq, head = blockIdx.x - rank * p.Hq, kvh = head / p.G;
-  if (!bwd_locate(p.cu_seqlens, p.num_seqs, rank, info, mb, blocks, seq_start, seq_len)) {
-    if (last) pdl_wait();
-    return;
-  }
+  const int rank = block / p.Hq, head = block - rank * p.Hq, kvh = head / p.G;
+  if (!bwd_locate(p.cu_seqlens, p.num_seqs, rank, info, mb, blocks, seq_start, seq_len)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q0 = mb * 128;
   const int n_kb = min((seq_len + 63) / 64, (q0 + 128 + 63) / 64);
@@ -505,24 +492,36 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_before();
   __syncthreads();
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
-  if (last) pdl_wait();
+}
+
+// Both in one launch, dQ's blocks behind those of dK / dV: neither takes anything from the other, and with two key heads dK / dV has a block for two SMs in
+// three only, so that dQ starts on the SMs that it leaves idle.  us of the whole backward as launches one after the other / so: 4 sequences, 6601 tokens, 12
+// heads over 2 250 / 164; 6 of 500, 28 over 4 116 / 76; 2 of 6005 1755 / 1582 to 1688; 4 of 6000 3529 / 3400; one of 300, 12 over 2 58 / 40.
+__global__ void __launch_bounds__(kBwdThreads, 1)
+attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ64, const __grid_constant__ CUtensorMap tmDO64, const __grid_constant__ CUtensorMap tmK128,
+                   const __grid_constant__ CUtensorMap tmV128, const __grid_constant__ CUtensorMap tmQ128, const __grid_constant__ CUtensorMap tmDO128,
+                   const __grid_constant__ CUtensorMap tmK64, const __grid_constant__ CUtensorMap tmV64, const __grid_constant__ AttnBwdParams p,
+                   const unsigned dkdv_blocks) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  pdl_wait();
+  if (blockIdx.x < dkdv_blocks) bwd_dkdv(smem, blockIdx.x, tmQ64, tmDO64, tmK128, tmV128, p);
+  else bwd_dq(smem, blockIdx.x - dkdv_blocks, tmQ128, tmDO128, tmK64, tmV64, p);
 }
 
 }  // namespace nrl
 
-// maps: [0] Q box 64 rows, [1] dO box 64 rows, [2] K box 128 rows, [3] V box 128 rows  (dK/dV kernel)
-//       [4] Q box 128 rows, [5] dO box 128 rows, [6] K box 64 rows, [7] V box 64 rows  (dQ kernel)
+// maps: [0] Q box 64 rows, [1] dO box 64 rows, [2] K box 128 rows, [3] V box 128 rows  (dK / dV)
+//       [4] Q box 128 rows, [5] dO box 128 rows, [6] K box 64 rows, [7] V box 64 rows  (dQ)
 extern "C" cudaError_t nrl_attn_bwd_tc(const CUtensorMap* maps, const void* o, const void* dout, const float* lse,
                                        float* delta, void* dq, void* dk, void* dv, long o_stride_t, long dq_stride_t,
                                        long dkv_stride_t, const int* cu, int num_seqs, int total, int Hq, int Hkv,
                                        float scale, cudaStream_t s) {
   using namespace nrl;
   if (total == 0) return cudaSuccess;
+  constexpr int smem = DkdvSmem::kTotal > DqSmem::kTotal ? DkdvSmem::kTotal : DqSmem::kTotal;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DkdvSmem::kTotal);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(attn_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem::kTotal);
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured = true;
   }
@@ -536,7 +535,7 @@ extern "C" cudaError_t nrl_attn_bwd_tc(const CUtensorMap* maps, const void* o, c
   p.num_seqs = num_seqs; p.total_tokens = total; p.Hq = Hq; p.G = Hq / Hkv;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   const unsigned most = total / 128 + num_seqs, grid_kv = most * Hkv, grid_q = most * Hq;
-  launch_dependent(attn_bwd_dkdv_tc_kernel, grid_kv, kBwdThreads, DkdvSmem::kTotal, s, maps[0], maps[1], maps[2], maps[3], p);
-  launch_dependent(attn_bwd_dq_tc_kernel, grid_q, kBwdThreads, DqSmem::kTotal, s, maps[4], maps[5], maps[6], maps[7], p);
+  launch_dependent(attn_bwd_tc_kernel, grid_kv + grid_q, kBwdThreads, smem, s, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], p,
+                   grid_kv);
   return cudaGetLastError();
 }

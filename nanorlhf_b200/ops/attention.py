@@ -39,10 +39,11 @@ class _NativeAttn(torch.autograd.Function):
     def backward(ctx, do):
         from . import native
         q, k, v, o, lse, cu = ctx.saved_tensors
-        native._count(3)
         if _USE_TC and q.shape[-1] == 128 and q.is_contiguous() and k.is_contiguous() and v.is_contiguous():
+            native._count(2)
             dq, dk, dv = native.ext().attn_bwd_tc(do.contiguous(), q, k, v, o, lse, cu, ctx.scale)
         else:
+            native._count(3)
             dq, dk, dv = native.ext().attn_varlen_bwd(do.contiguous(), q, k, v, o, lse, cu, ctx.max_seqlen, ctx.scale)
         return dq, dk, dv, None, None, None
 
