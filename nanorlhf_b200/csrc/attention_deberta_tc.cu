@@ -43,7 +43,7 @@ struct DbSmem {
   static constexpr int kMeta = kLut + 2 * kLutCopy;
   static constexpr int kStage = kMeta + 128;                     // a multiple of 128
   static constexpr int kA = kB + kDbStages * kStage;
-  static constexpr int kMax = kA + kDbBM * kDbAPitch;            // [tile stream][half] maxima of 128 rows, bf16
+  static constexpr int kMax = kA + kDbBM * kDbAPitch;            // [tile stream][half] 16 bits of the maxima of 128 rows
   static constexpr int kBar = kMax + 4 * 128 * 2;
   static constexpr int kTab = kBar + 320;                        // two items of 8 ints
   static constexpr int kTotal = kTab + 2 * 32;
@@ -98,6 +98,11 @@ NRL_DEVICE DbItem db_item(const uint8_t* smem, uint64_t* tab_full, uint32_t k) {
 
 NRL_DEVICE void sts_u16(uint32_t addr, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(v)) : "memory"); }
 NRL_DEVICE void sts_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+NRL_DEVICE uint32_t lds_u16(uint32_t addr) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+  return v;
+}
 // f + the bf16 at a shared address
 template <int OFFSET = 0>
 NRL_DEVICE float add_lds_bf16(float f, uint32_t addr) {
@@ -419,10 +424,15 @@ deberta_attn_tc_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_con
         const float mx = (fmaxf(mx2[0], mx2[1]) + a0) * p.scale_log2;
         float corr = 1.f;
         if (barrier_any(pair, mx > m_run + 8.f)) {             // also orders both halves' reads of the scores before the first P over them
-          sts_u16(mx_own, pack_bf16x2(mx, 0.f));
+          // The larger of both halves, exact: half a bf16 step of a score of 2^16 would be a factor of 2^128 here.  Shared memory has no room for a float each, and
+          // forms with one slot for both or through tensor memory spill registers (16 x 1536 tokens 485 -> 510 us): the upper 16 bits, then the lower
+          sts_u16(mx_own, __float_as_uint(mx) >> 16);
           named_barrier_sync(pair, 64);
-          const float both = fmaxf(add_lds_bf16(0.f, mx_own), add_lds_bf16(0.f, mx_oth));      // rounded: any number near the maximum will do
+          const uint32_t upper = lds_u16(mx_oth) << 16;
           named_barrier_sync(pair, 64);
+          sts_u16(mx_own, __float_as_uint(mx));
+          named_barrier_sync(pair, 64);
+          const float both = fmaxf(mx, __uint_as_float(upper | lds_u16(mx_oth)));      // read before the next barrier_any
           if (both > m_run) {
             corr = ex2_approx(m_run - both);
             m_run = both;

@@ -54,6 +54,28 @@ def test_against_float64(lens, heads, span, top):
     assert torch.equal(got, native.ext().deberta_attn_tc(*qkv, cu, max(lens), scale, pos_k, rel_b, lut))
 
 
+@pytest.mark.parametrize("lens", [[300, 129], [40], [64]])
+def test_large_scores(lens):
+    """Scores of 2^17 and more in front of the softmax, a different size in every row: what is subtracted from them has to be as exact as they are."""
+    from nanorlhf_b200.models.deberta_v3 import _bias_tables
+    from nanorlhf_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(2)
+    T, heads, buckets, scale = sum(lens), 2, 512, 0.75
+    small = lambda *shape: torch.randint(-2, 3, shape, generator=g, device="cuda").to(torch.bfloat16) / 2  # noqa: E731
+    q, k, v = small(T, heads, 64), small(T, heads, 64), torch.randn(T, heads, 64, generator=g, device="cuda").bfloat16()
+    pos_k, pos_q = (small(buckets, heads, 64).transpose(0, 1) for _ in range(2))
+    q[:, :, 0], k[:, :, 0] = 256.0 + 2.0 * torch.arange(T, device="cuda")[:, None] % 200, 512.0
+    pos_k[:, :, 0], pos_q[:, :, 0] = 0.0, 0.0
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    lut = build_bucket_lut(max(lens), 256, 512, 256, "cuda")
+    rel_b = _bias_tables(k, pos_q)
+    got = native.ext().deberta_attn_tc(q, k, v, cu, max(lens), scale, pos_k, rel_b, lut)
+    want = _reference([q, k, v], pos_k, rel_b, lut, lens, scale)
+    # every product is a multiple of a quarter and every sum below 2^18, so that scores are exact; scaled they are rounded to 2^-7 once, the same for all keys
+    assert torch.isfinite(got).all()
+    assert (got.double() - want).norm() <= 2.0 ** -8 * want.norm()
+
+
 def test_rows_of_a_wider_projection_and_tables():
     """q, k and v as columns of one product, against the kernel that reads both tables."""
     from nanorlhf_b200.models.deberta_v3 import _bias_tables
