@@ -136,28 +136,42 @@ inline void check_tc_operand(const torch::Tensor& t, const char* name) {
 
 // ---- split-K of gemm_tc: into how many ranges the contraction of a product [M, K] x [K, N] is cut unless the caller says so ----
 // (any N: the adapter-input gradient dA = t'^T x is [r, K_in] -- 12 or 24 tiles of a 6.6 k-long contraction).
-// The number of ranges is the one for which this estimate (us) is least: 0.172 for each block of 64 contraction columns of a range, and for the sum of the parts
-// 1.2 + 0.2 a range where clusters form it (tiles 128 wide; 64 wide 1.0 + 0.1), 5 (2.5) through the workspace, where beyond four ranges it costs more
-// than it saves.  Half a microsecond is left to the uncut product, which takes every tile shape.  us uncut / cut (clusters): 128 x 1536 with 1024
-// columns 6.6 / 6.6 (four), 1536 8.2 / 7.1, 8960 31.9 / 12.8 (eight; through the workspace 18.4 with four); 16 x 1536, 8960 31.6 / 10.3; 3300 x 192 (two) 1536 8.9 / 9.3,
-// 2560 12.3 / 11.4; 6601 x 64 (two) 1536 9.0 / 8.6; 600 x 64, 8960 31.6 / 9.0; dA 64 x 1536, 6601 tokens 24.5 / 9.9; 512 x 1536, 8960
-// 33.8 / 21.1 (three, workspace).
+// The number of ranges is the one for which this estimate (us) is least, over the numbers that leave no range empty, since those are launched: 0.2 for each
+// block of 64 contraction columns of a range, 0.008 for each block of the grid, and for the sum of the parts 2.5 where clusters form it (tiles 64 wide:
+// 1.0), 0.8 (0.6) more above four parts, which are read four at a time, and 6 (2.5) through the workspace, where beyond four ranges it costs more than it saves.
+// us uncut / cut, in a graph (tiles; clusters unless said): 128 x 1536 (12) with 1024 columns 6.4 / four 6.7; 1536 8.0 / 7.1, five 7.8; 2624 11.5 / four 8.1, seven 8.4;
+// 3136 13.0 / 8.5, 8.6; 4096 16.0 / 9.1, eight 8.8; 8960 31.2 / 13.1, 11.0.  1024 x 256 (16) 8960 31.3 / four 13.3, six 12.7, seven (workspace) 16.6.
+// 512 x 1536 (48) 1536 8.5 / two 9.1; 2112 10.4 / 10.2; 8960 32.5 / two 22.5, three (workspace) 19.9.  1664 x 64 (13) 1024 6.4 / four 5.3; 2112 9.7 / four 6.35, seven
+// 6.46; 4096 16.2 / four 7.8, eight 7.1.  3300 x 64 (26) 1536 8.2 / four 6.3, five 6.7; 8960 31.3 / 12.3, 11.8.  4700 x 64 (37) 4096 16.0 / three 9.7, four (workspace) 10.0;
+// 8960 31.2 / 15.3, 14.4.  Over 18 outputs with 11 contractions of 1024 to 8960 columns each the choice is within 0.35 us of the fastest, but for 8 rows, which
+// read less (1024 columns 6.1 / four 5.1; 3584 eight 8.6, seven 7.6), 16 x 4096 with 1024 (7.6 / two 6.9) and 512 x 1536 with 6656 (two 18.5, three 17.6).
 inline int split_block_n(int64_t N) { return N <= 64 ? 64 : 128; }
 inline int64_t split_tiles(int64_t M, int64_t N) { return ((M + 127) / 128) * ((N + split_block_n(N) - 1) / split_block_n(N)); }
-int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
+// how many of `splits` ranges of a contraction of `blocks` are launched: none is empty
+inline int64_t split_ranges(int64_t blocks, int64_t splits) {
+  const int64_t per = (blocks + splits - 1) / splits;
+  return (blocks + per - 1) / per;
+}
+// fits(s): clusters of s blocks that run at a time
+template <class Fits>
+int64_t split_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits) {
   const int64_t tiles = split_tiles(M, N), blocks = (K + 63) / 64;
-  if (tiles < 1 || tiles * 2 > num_sms()) return 1;
+  if (tiles < 1 || tiles * 2 > sms) return 1;
   const bool narrow = split_block_n(N) == 64;
-  double least = 0.172 * blocks - 0.5;
+  auto loop = [&](int64_t s) { return 0.2 * ((blocks + s - 1) / s) + 0.008 * (tiles * s); };
+  double least = loop(1);
   int64_t best = 1;
-  for (int64_t s = 2; s <= 8 && tiles * s <= num_sms() && blocks >= 4 * s; ++s) {
-    if (s > 4 && s < 8) continue;                        // 3300 x 64 with 1536 columns: four 6.7 us, five 7.1
-    const bool clusters = tiles <= nrl_gemm_tc_split_clusters(split_block_n(N), static_cast<int>(s));
-    if (!clusters && s > 4) break;
-    const double t = 0.172 * ((blocks + s - 1) / s) + (clusters ? (narrow ? 1.0 + 0.1 * s : 1.2 + 0.2 * s) : narrow ? 2.5 : 5.0);
+  for (int64_t s = 2; s <= 8 && tiles * s <= sms && blocks >= 4 * s; ++s) {
+    if (split_ranges(blocks, s) != s) continue;            // comes as a smaller number
+    const bool clusters = tiles <= fits(static_cast<int>(s));
+    if (!clusters && s > 4) continue;
+    const double t = loop(s) + (clusters ? (narrow ? 1.0 : 2.5) + (s > 4 ? (narrow ? 0.6 : 0.8) : 0.0) : narrow ? 2.5 : 6.0);
     if (t < least) { least = t; best = s; }
   }
   return best;
+}
+int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
+  return split_choice(M, N, K, num_sms(), [&](int s) { return nrl_gemm_tc_split_clusters(split_block_n(N), s); });
 }
 
 // D[M,N] = alpha * (opA(a) opB(b)^T + opA(a2) opB(b2)^T) (+bias) (GELU).
@@ -206,8 +220,7 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
     int64_t splits = splitk_req > 0 ? splitk_req : auto_splits(M, N, K);
     if (splitk_req > 0 || splits > 1) {
       splits = std::max<int64_t>(1, std::min<int64_t>(splits, num_kb));
-      const int64_t per = (num_kb + splits - 1) / splits;
-      splits = (num_kb + per - 1) / per;                                 // no empty k-range
+      splits = split_ranges(num_kb, splits);
       // Captured CUDA graphs (decode step, training micro-step) hold these addresses: a workspace that is outgrown is
       // retired, never freed.  (Automatic dispatch needs at most num_sms tiles of 128 x 128 floats = 9.7 MB < the 16 MB minimum.)
       static thread_local torch::Tensor ws, counters;
@@ -1201,6 +1214,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_swiglu", &gemm_tc_swiglu, py::arg("a"), py::arg("w_interleaved"), py::arg("out") = py::none(), py::arg("cg") = 0,
         py::arg("block_n") = 0);
   m.def("gemm_tc_auto_splits", &auto_splits, py::arg("M"), py::arg("N"), py::arg("K"));
+  m.def("gemm_tc_split_choice", [](int64_t M, int64_t N, int64_t K, int64_t sms, const std::vector<int>& fits) {
+    return split_choice(M, N, K, sms, [&](int s) { return fits.at(s); });
+  }, "auto_splits for a GPU of `sms` SMs that runs fits[s] clusters of s blocks at a time");
+  m.def("gemm_tc_split_clusters", &nrl_gemm_tc_split_clusters, py::arg("block_n"), py::arg("splits"));
   m.def("gemm_tc_swiglu_pair", &gemm_tc_swiglu_pair, py::arg("x"), py::arg("wg"), py::arg("wu"), py::arg("tg") = py::none(),
         py::arg("tu") = py::none(), py::arg("bg") = py::none(), py::arg("bu") = py::none());
   m.def("add_layernorm", &add_layernorm);

@@ -888,7 +888,9 @@ gemm_tc_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   gemm_tc_body<1, BN, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
 }
 
-// clusters of `splits` blocks that run at a time
+// clusters of `splits` blocks that run at a time: one block per SM, so the same for all forms of the operands, whose blocks are alike
+static_assert(Cfg<1, 64, true>::kTotal == Cfg<1, 64, false>::kTotal && Cfg<1, 128, true>::kTotal == Cfg<1, 128, false>::kTotal && Cfg<1, 64>::kTotal > kSmemBudget / 2 &&
+              Cfg<1, 128>::kTotal > kSmemBudget / 2, "auto_splits asks for one form");
 template <int BN, bool A_MN, bool B_MN>
 static int splitk_clusters(int splits) {
   using C = Cfg<1, BN, B_MN>;

@@ -51,7 +51,7 @@ struct TcParams {
 }  // namespace tc
 }  // namespace nrl
 
-// how many tiles' ranges clusters of `splits` blocks hold at a time (0: none); the launch decides by its own kernel's figure
+// clusters of `splits` blocks that run at a time (0: none), whichever form the operands have
 extern "C" int nrl_gemm_tc_split_clusters(int bn, int splits);
 extern "C" cudaError_t nrl_gemm_tc_splitk(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int a_mn, int b_mn, int num_sms,
                                           cudaStream_t stream);
