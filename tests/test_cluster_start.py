@@ -1,5 +1,6 @@
 """A block's shared memory may be written by its cluster's other blocks only once it is known to have started.  The order of start-up is not
-ours to choose, so this is read from the sources: every remote write follows a cluster barrier that all blocks arrive at on entry."""
+ours to choose, so this is read from the sources: every remote write follows a cluster barrier that all blocks arrive at on entry.  Remote reads have a
+header of their own (test_cluster_read.py)."""
 import os
 import re
 
@@ -25,7 +26,8 @@ def _function(src, name):
 
 
 def test_no_other_file_writes_remote_shared_memory():
-    assert {f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")) and REMOTE.search(_source(f))} == {"rl_kernels.cu", "sampling.cu"}
+    reach = {f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h", ".cpp")) and REMOTE.search(_source(f))}
+    assert reach == {"rl_kernels.cu", "sampling.cu", "cluster_read.h"}
 
 
 @pytest.mark.parametrize("kernel", ["policy_loss_kernel", "value_loss_kernel"])
