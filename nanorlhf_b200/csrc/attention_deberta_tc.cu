@@ -133,10 +133,6 @@ NRL_DEVICE void db_add_column(uint32_t (&sv)[32], uint32_t b_col) {
 NRL_DEVICE void tmem_st_x2(uint32_t taddr, uint32_t a, uint32_t b) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
 }
-NRL_DEVICE void tmem_ld_x8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
-}
 // does any thread of two warps say so
 NRL_DEVICE bool barrier_any(uint32_t id, bool pred) {
   uint32_t any;
@@ -481,7 +477,7 @@ deberta_attn_tc_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_con
       tc_fence_after();
       const uint32_t col = w * 32 + h * 16;
       uint32_t ml[8], o0[16], o1[16];
-      tmem_ld_x8(t_lane + kDbTmemML, ml);
+      tmem_ld_32x32b_x8(t_lane + kDbTmemML, ml);
       tmem_ld_32x32b_x16(t_lane + kDbTmemO + col, o0);
       tmem_ld_32x32b_x16(t_lane + kDbTmemO + 64 + col, o1);
       tmem_ld_wait();
