@@ -14,11 +14,14 @@
 // A block whose differences all fall into one bucket (from 511 positions on) needs no lookup: A is a number per row and B one per key.
 // One persistent CTA per SM; items go from the longest to the shortest sequence, dealt to the CTAs forwards and backwards in turn.
 //
-// What bounds it: the chain of one tile, above all its lookups (two and a half reads of shared memory a score; 16 x 1536 tokens with 16 heads 530 us, 365 with
-// the lookups left out, 294 without P V and 2^x too).  The streams take turns at them (542 -> 530 us); all loads in front of the first sum, sums of A and B
-// before the scores are there and longer sleeps of the waiting warps changed nothing or cost up to 8 %.  The mma.sync form with both tables in global memory
-// takes 835 us and 92 more for the second table, and is bound by the windows that it fetches (5 GB through the L2, 1.1 here): 16 x 300 tokens 55 against
-// 54 + 24, 4 x 700 48 / 59 + 15, 16 x 40 11.5 / 6.7 + 8.8, so that it is left only where A does not fit (more than 512 buckets).
+// What bounds it: the chain of one tile, above all its lookups (two and a half reads of shared memory a score; without them it took 0.69 of its time, without
+// P V and 2^x too 0.55).  The streams take turns at them (2 %); all loads in front of the first sum, sums of A and B before the scores are there and longer
+// sleeps of the waiting warps changed nothing or cost up to 8 %.  The maximum is the row's own in every block, which both halves of a row agree on through tensor
+// memory: 16 x 1536 tokens with 16 heads 524 us in a graph, 486 with one that may be stale by 2^8, whose error against float64 was up to 1.21 times that of the
+// mma.sync form (operands of standard deviation 1.5; now 0.98); asking first whether any row moved 562.
+// The mma.sync form with both tables in global memory takes 767 us and 90 more for the second table, and is bound by the windows that it fetches (5 GB through
+// the L2, 1.1 here): 16 x 300 tokens 55 against 54 + 23, 4 x 700 49 / 59 + 14, 16 x 40 10.7 / 6.7 + 7.9, so that it is left only where A does not fit (more than 512
+// buckets).
 #include "attention_tc.cuh"
 #include "kernels.h"
 #include "launch.h"
@@ -26,7 +29,7 @@
 namespace nrl {
 namespace {
 
-constexpr int kDbThreads = 768;            // registers: 768 x 80 at launch = 128 x (64 + 4 x 88 + 64)
+constexpr int kDbThreads = 768;            // registers: 768 x 80 at launch = 128 x (56 + 4 x 88 + 72)
 constexpr int kDbBM = 128, kDbBN = 64;     // query rows per item, keys per block
 constexpr int kDbTile = 64 * 128;          // [64 rows][64 x bf16], 128B-swizzled
 constexpr int kDbWin = 144;                // columns of B staged per 8 keys
@@ -43,15 +46,14 @@ struct DbSmem {
   static constexpr int kMeta = kLut + 2 * kLutCopy;
   static constexpr int kStage = kMeta + 128;                     // a multiple of 128
   static constexpr int kA = kB + kDbStages * kStage;
-  static constexpr int kMax = kA + kDbBM * kDbAPitch;            // [tile stream][half] 16 bits of the maxima of 128 rows
-  static constexpr int kBar = kMax + 4 * 128 * 2;
+  static constexpr int kBar = kA + kDbBM * kDbAPitch;
   static constexpr int kTab = kBar + 320;                        // two items of 8 ints
   static constexpr int kTotal = kTab + 2 * 32;
 };
-static_assert(DbSmem::kStage % 128 == 0 && DbSmem::kMax % 16 == 0 && DbSmem::kTotal <= 227 * 1024, "shared memory");
+static_assert(DbSmem::kStage % 128 == 0 && DbSmem::kBar % 16 == 0 && DbSmem::kTotal <= 227 * 1024, "shared memory");
 
-// TMEM columns: scores [stream][2] (P over the first 32 of them) | O [stream] | Q [2] | maximum and sum
-constexpr int kDbTmemO = 256, kDbTmemQ = 384, kDbTmemML = 448;      // ... | [stream][half]
+// TMEM columns: scores [stream][2] (P over the first 32 of them) | O [stream] | Q [2] | maximum and sum | maxima of a tile
+constexpr int kDbTmemO = 256, kDbTmemQ = 384, kDbTmemML = 448, kDbTmemMax = 456;      // ... | [stream][half] | [stream][tile & 1][half]
 
 struct DbParams {
   const int* cu_seqlens;
@@ -98,11 +100,6 @@ NRL_DEVICE DbItem db_item(const uint8_t* smem, uint64_t* tab_full, uint32_t k) {
 
 NRL_DEVICE void sts_u16(uint32_t addr, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(v)) : "memory"); }
 NRL_DEVICE void sts_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
-NRL_DEVICE uint32_t lds_u16(uint32_t addr) {
-  unsigned short v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
-  return v;
-}
 // f + the bf16 at a shared address
 template <int OFFSET = 0>
 NRL_DEVICE float add_lds_bf16(float f, uint32_t addr) {
@@ -130,15 +127,16 @@ NRL_DEVICE void db_add_column(uint32_t (&sv)[32], uint32_t b_col) {
     db_add_column<I + 1>(sv, b_col);
   }
 }
+NRL_DEVICE void tmem_st_x1(uint32_t taddr, uint32_t a) { asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(a) : "memory"); }
+// the larger of two columns
+NRL_DEVICE float tmem_max_x2(uint32_t taddr) {
+  uint32_t a, b;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(taddr) : "memory");
+  tmem_ld_wait();
+  return fmaxf(__uint_as_float(a), __uint_as_float(b));
+}
 NRL_DEVICE void tmem_st_x2(uint32_t taddr, uint32_t a, uint32_t b) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
-}
-// does any thread of two warps say so
-NRL_DEVICE bool barrier_any(uint32_t id, bool pred) {
-  uint32_t any;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\tbar.red.or.pred q, %1, 64, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
-               : "=r"(any) : "r"(id), "r"(static_cast<uint32_t>(pred)) : "memory");
-  return any != 0;
 }
 
 __global__ void __launch_bounds__(kDbThreads, 1)
@@ -207,7 +205,7 @@ deberta_attn_tc_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_con
   pdl_launch_dependents();
 
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0) {
       // ============================== position keys, K and V ==============================
       if (elect_one()) {
@@ -349,7 +347,6 @@ deberta_attn_tc_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_con
     const int quad = warp & 3, r = quad * 32 + lane;           // row of the item == TMEM lane
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     const uint32_t a_row = smem_u32(smem + L::kA) + r * kDbAPitch;
-    const uint32_t mx_own = smem_u32(smem + L::kMax) + ((w * 2 + h) * 128 + r) * 2, mx_oth = smem_u32(smem + L::kMax) + ((w * 2 + (h ^ 1)) * 128 + r) * 2;
     const uint32_t pair = 2 + w * 4 + quad;                    // barrier of the two warps that hold the same rows of a tile
     const int y0 = 127 - r;
     const uint32_t lut_off = L::kLut + (y0 & 1) * L::kLutCopy + (y0 & ~1) * 2 + h * 64;
@@ -413,36 +410,35 @@ deberta_attn_tc_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_con
           for (int i = 0; i < 32; ++i)
             if (i >= see) sv[i] = 0xff800000u;
         }
-        // ---- online softmax: a maximum that is stale by less than 2^8 does no harm, so that the halves seldom have to agree on another ----
+        // ---- online softmax ----
         float mx2[2] = {-INFINITY, -INFINITY};
 #pragma unroll
         for (int i = 0; i < 32; i += 2) mx2[(i >> 1) & 1] = fmaxf(mx2[(i >> 1) & 1], fmaxf(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])));
         const float mx = (fmaxf(mx2[0], mx2[1]) + a0) * p.scale_log2;
+        // The row's own maximum: the larger of both halves, which also orders their reads of the scores before the first P over them.  A stale one would do for the
+        // range (a weight below 2^8 is harmless), but a row's largest weight has to be exactly 1 to pass the rounding of P whole
+        const uint32_t t_mx = t_lane + kDbTmemMax + w * 4 + (n_pv & 1) * 2;
+        tmem_st_x1(t_mx + h, __float_as_uint(mx));
+        tmem_st_wait();
+        tc_fence_before();
+        named_barrier_sync(pair, 64);
+        tc_fence_after();
+        const float both = tmem_max_x2(t_mx);
+        const bool moved = both > m_run;
         float corr = 1.f;
-        if (barrier_any(pair, mx > m_run + 8.f)) {             // also orders both halves' reads of the scores before the first P over them
-          // The larger of both halves, exact: half a bf16 step of a score of 2^16 would be a factor of 2^128 here.  Shared memory has no room for a float each, and
-          // forms with one slot for both or through tensor memory spill registers (16 x 1536 tokens 485 -> 510 us): the upper 16 bits, then the lower
-          sts_u16(mx_own, __float_as_uint(mx) >> 16);
-          named_barrier_sync(pair, 64);
-          const uint32_t upper = lds_u16(mx_oth) << 16;
-          named_barrier_sync(pair, 64);
-          sts_u16(mx_own, __float_as_uint(mx));
-          named_barrier_sync(pair, 64);
-          const float both = fmaxf(mx, __uint_as_float(upper | lds_u16(mx_oth)));      // read before the next barrier_any
-          if (both > m_run) {
-            corr = ex2_approx(m_run - both);
-            m_run = both;
-          }
-          if (!first) {
-            mbar_wait_quiet(&pv_done[w], (n_pv - 1) & 1);
-            tc_fence_after();
-            uint32_t ov[32];
-            tmem_ld_32x32b_x32(t_lane + kDbTmemO + w * 64 + h * 32, ov);
-            tmem_ld_wait();
+        if (moved) {
+          corr = ex2_approx(m_run - both);
+          m_run = both;
+        }
+        if (__any_sync(0xffffffffu, moved && !first)) {
+          mbar_wait_quiet(&pv_done[w], (n_pv - 1) & 1);
+          tc_fence_after();
+          uint32_t ov[32];
+          tmem_ld_32x32b_x32(t_lane + kDbTmemO + w * 64 + h * 32, ov);
+          tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
-            tmem_st_32x32b_x32(t_lane + kDbTmemO + w * 64 + h * 32, ov);
-          }
+          for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+          tmem_st_32x32b_x32(t_lane + kDbTmemO + w * 64 + h * 32, ov);
         }
         const float m_sub = m_run == -INFINITY ? 0.f : m_run, off = fmaf(a0, p.scale_log2, -m_sub);
         const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), off2 = pack_f32x2(off, off);
@@ -506,7 +502,7 @@ deberta_attn_tc_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_con
     }
   } else {
     // ============================== queries, buckets, B ==============================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     const int quad = warp & 3, r = quad * 32 + lane;
     auto queries = [&](uint32_t k) {
       const DbItem it = db_item(smem, tab_full, k);

@@ -76,6 +76,24 @@ def test_large_scores(lens):
     assert (got.double() - want).norm() <= 2.0 ** -8 * want.norm()
 
 
+@pytest.mark.parametrize("std", [0.5, 1.0, 1.5, 2.0])           # of the operands: flat rows to single weights
+@pytest.mark.parametrize("lens", [[1536], [300, 300], [40] * 8, [700, 90]])
+def test_no_further_from_float64_than_the_kernel_with_two_tables(lens, std):
+    from nanorlhf_b200.models.deberta_v3 import _bias_tables
+    from nanorlhf_b200.ops import native
+    (q, k, v), pos_k, pos_q, cu = _inputs(lens, 8, 512, seed=4)
+    q, k, pos_k, pos_q = ((t.float() * std).bfloat16() for t in (q, k, pos_k.transpose(0, 1), pos_q.transpose(0, 1)))
+    pos_k, pos_q = pos_k.transpose(0, 1), pos_q.transpose(0, 1)
+    lut, scale = build_bucket_lut(max(lens), 256, 512, 256, "cuda"), 1.0 / math.sqrt(192)
+    rel_b = _bias_tables(k, pos_q)
+    want = _reference([q, k, v], pos_k, rel_b, lut, lens, scale)
+    new = native.ext().deberta_attn_tc(q, k, v, cu, max(lens), scale, pos_k, rel_b, lut)
+    old = native.ext().deberta_attn_fwd(q, k, v, cu, max(lens), scale, _bias_tables(q, pos_k), rel_b, lut)
+    # both round each weight and each result once, a row's largest weight being 1; how often it is another block's that is rounded differs by a share of
+    # a per cent either way, and so does the rounding of A
+    assert (new.double() - want).norm() <= 1.005 * (old.double() - want).norm()
+
+
 def test_rows_of_a_wider_projection_and_tables():
     """q, k and v as columns of one product, against the kernel that reads both tables."""
     from nanorlhf_b200.models.deberta_v3 import _bias_tables
