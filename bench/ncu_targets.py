@@ -101,6 +101,32 @@ if which in ("all", "deberta_tma"):
     lut = build_bucket_lut(1660, 256, 512, 256, dev)
     for _ in range(3):
         native.ext().deberta_attn_fwd(q, k, v, cu, 1660, 1 / math.sqrt(192), ra, rb, lut)
+if which in ("all", "deberta_tc"):
+    from nanorlhf_b200.models.deberta_v3 import build_bucket_lut
+    lens = [1536] * 4
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), device=dev, dtype=torch.int32)
+    T = sum(lens)
+    q, k, v = (torch.randn(T, 16, 64, device=dev, dtype=torch.bfloat16) for _ in range(3))
+    pos_k = torch.randn(512, 16, 64, device=dev, dtype=torch.bfloat16).transpose(0, 1)
+    rb = torch.randn(16, T, 512, device=dev, dtype=torch.bfloat16)
+    lut = build_bucket_lut(1536, 256, 512, 256, dev)
+    for _ in range(3):
+        native.ext().deberta_attn_tc(q, k, v, cu, 1536, 1 / math.sqrt(192), pos_k, rb, lut)
+if which in ("all", "gemm_tc_cut"):
+    a, b = torch.randn(128, 8960, device=dev, dtype=torch.bfloat16), torch.randn(1536, 8960, device=dev, dtype=torch.bfloat16)
+    for _ in range(3):                       # the ranges of a tile are a cluster
+        native.ext().gemm_tc(a, b, False, False)
+if which in ("all", "delta_chunk"):
+    from types import SimpleNamespace
+    from nanorlhf_b200.ops import hybrid
+    E, n, H, D = 16, 512, 16, 128
+    qkv = torch.randn(E * n, 3 * H * D, device=dev) * 0.1
+    beta, decay = torch.rand(E * n, H, device=dev), torch.rand(E * n, H, device=dev) * 0.1 + 0.9
+    plan = SimpleNamespace(cu=torch.arange(E + 1, device=dev, dtype=torch.int32) * n, start=torch.zeros(E, device=dev, dtype=torch.int32),
+                           state_slot=torch.arange(E, device=dev, dtype=torch.int32))
+    state, o = torch.zeros(E, H, D, D, device=dev), torch.empty(E * n, H * D, device=dev)
+    for _ in range(3):
+        hybrid.delta_scan(qkv, H * D, 2 * H * D, beta, decay, state, o, plan, H, False, impl="chunked")
 if which in ("all", "dlogits"):
     h = torch.randn(8192, 1536, device=dev, dtype=torch.bfloat16)
     w = (torch.randn(151936, 1536, device=dev) * 0.02).bfloat16()

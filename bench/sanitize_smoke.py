@@ -32,6 +32,16 @@ ext.attn_bwd_tc(torch.randn_like(o), q, k, v, o, lse, cu, 1 / math.sqrt(128))
 qd, kd, vd = (torch.randn(T, 2, 64, device=dev, dtype=bf) for _ in range(3))
 ra, rb = (torch.randn(2, T, 512, device=dev, dtype=bf) for _ in range(2))
 ext.deberta_attn_fwd(qd, kd, vd, cu, max(lens), 1 / math.sqrt(192), ra, rb, build_bucket_lut(max(lens), 256, 512, 256, dev))
+ext.deberta_attn_tc(qd, kd, vd, cu, max(lens), 1 / math.sqrt(192), torch.randn(512, 2, 64, device=dev, dtype=bf).transpose(0, 1), rb,
+                    build_bucket_lut(max(lens), 256, 512, 256, dev))
+# delta-rule scan, 32 tokens at a time: rows by bulk copies (64 columns beside zeroed ones) and float by float
+from types import SimpleNamespace  # noqa: E402
+from nanorlhf_b200.ops import hybrid  # noqa: E402
+plan = SimpleNamespace(cu=cu, start=torch.zeros(3, dtype=torch.int32, device=dev), state_slot=torch.arange(3, dtype=torch.int32, device=dev))
+for Dd in (64, 33):
+    qkvd, od = torch.randn(T, 6 * Dd, device=dev) * 0.1, torch.empty(T, 2 * Dd, device=dev)
+    hybrid.delta_scan(qkvd, 2 * Dd, 4 * Dd, torch.rand(T, 2, device=dev), torch.rand(T, 2, device=dev), torch.zeros(3, 2, Dd, Dd, device=dev), od, plan, 2,
+                      False, impl="chunked")
 # elementwise / RL kernels
 x = torch.randn(64, 256, device=dev, dtype=bf)
 native.rmsnorm(x, torch.ones(256, device=dev, dtype=bf), 1e-6)
@@ -106,6 +116,11 @@ lgw = torch.randn(6, 151936, device=dev, dtype=bf)
 for impl in (21, 22, 24):                                # cluster kernel: 1 / 2 / 4 CTAs per row (bulk loads, DSMEM exchange)
     native.sample(lg if impl == 21 else lgw, 0.9, 0.95, 7, 0, impl=impl)
 native.sample(lgw, 1.0, 0.5, 7, 0, impl=2)               # many redraws
+# a cut contraction summed by clusters of eight, and through the workspace (20 tiles: more than clusters of seven fit)
+ext.gemm_tc(torch.randn(64, 2048, device=dev, dtype=bf), torch.randn(264, 2048, device=dev, dtype=bf), False, False, None, None, None, 0, 1.0, None, None, False,
+            0, 0, 8)
+ext.gemm_tc(torch.randn(1280, 2048, device=dev, dtype=bf), torch.randn(256, 2048, device=dev, dtype=bf), False, False, None, None, None, 0, 1.0, None, None, False,
+            0, 0, 7)
 # split-K with bias in the fix-up, and the fused decode-step RoPE + KV page write
 ext.gemm_tc(torch.randn(64, 2048, device=dev, dtype=bf), torch.randn(264, 2048, device=dev, dtype=bf), False, False, None, None,
             torch.randn(264, device=dev, dtype=bf))
