@@ -4,7 +4,8 @@
 //
 // Work item: two tiles (A, B) of 128 query rows that share one key/value head -- QT consecutive tokens x HB query heads each -- which
 // walk the keys their rows can see in blocks of 128 (eight pages).  One persistent CTA per SM takes every gridDim-th item,
-// key heads varying fastest: 16 x 2048 tokens, 16 heads over 4, window 1024: 331 to 344 us (368 with the exact maximum of attention_tc.cuh, as all figures here are without); tokens varying fastest 334 us (422 -> 624 us with 16 key
+// key heads varying fastest: 16 x 2048 tokens, 16 heads over 4, window 1024: 363 to 368 us.  The row's maximum is exact in every block (attention_tc.cuh); the other
+// figures here were taken with one that could be stale by 2^8, 331 to 344 us for the same: tokens varying fastest 334 us (422 -> 624 us with 16 key
 // heads and no window: the same few tiles of every sequence fell to the same CTAs); items handed out by a counter 365 us.
 //   warp 0       producer: eight lanes each bring one page (two 64-column panels) of K or V by TMA into a ring of four 32 KB tiles,
 //                in the order the MMAs use them (K_0, V_0, K_1, V_1, K_2 ...); keys behind the end of a sequence are zero (missing pages by an
@@ -12,7 +13,7 @@
 //   warp 1       MMA issuer: S_X = Q_X K^T, then per block O_X += P_X V and at once the next S_X, tiles alternating, so that the tensor
 //                pipe works on one tile while the other is in its softmax
 //   warp 2       finds the next item's runs (tokens of one entry) while the current one is computed; warp 3 prefetches its queries to L2
-//   warps 4..11  one thread per row: scores from TMEM, cap, mask, online softmax in float with lazy rescaling (attention_tc.cuh), P back
+//   warps 4..11  one thread per row: scores from TMEM, cap, mask, online softmax in float with the exact maximum, O rescaled where it moved, P back
 //                into TMEM over its scores; behind the last block the next item's queries (float -> bf16, swizzled), so that its first
 //                scores are formed during the epilogue: sink, gate, store
 // Tokens of different sequences that fall into one item are walked one run after the other over the same accumulators.
