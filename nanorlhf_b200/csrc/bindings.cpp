@@ -163,7 +163,7 @@ int64_t split_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits) {
   int64_t best = 1;
   for (int64_t s = 2; s <= 8 && tiles * s <= sms && blocks >= 4 * s; ++s) {
     if (split_ranges(blocks, s) != s) continue;            // comes as a smaller number
-    const bool clusters = tiles <= fits(static_cast<int>(s));
+    const bool clusters = nrl::tc::split_by_clusters(static_cast<int>(s), blocks) && tiles <= fits(static_cast<int>(s));
     if (!clusters && s > 4) continue;
     const double t = loop(s) + (clusters ? (narrow ? 1.0 : 2.5) + (s > 4 ? (narrow ? 0.6 : 0.8) : 0.0) : narrow ? 2.5 : 6.0);
     if (t < least) { least = t; best = s; }

@@ -881,7 +881,7 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 }
 
 // The same with a tile's ranges in one cluster, which sums its parts through distributed shared memory: the workspace form passes them through L2, and its
-// last block sums them alone while the others have left.  As many clusters as the GPU holds at a time; larger products keep that form.
+// last block sums them alone while the others have left.  As many clusters as the GPU holds at a time; larger products and pairs of long ranges keep that form.
 template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
@@ -916,7 +916,7 @@ static cudaError_t launch_splitk(const CUtensorMap* maps, const TcParams& p, int
   }
   const int tiles = ((p.M + BLOCK_M - 1) / BLOCK_M) * ((p.N + BN - 1) / BN);
   int grid = tiles * p.splits;
-  if (grid <= num_sms && tiles <= splitk_clusters<BN, A_MN, B_MN>(p.splits)) {
+  if (grid <= num_sms && split_by_clusters(p.splits, (p.K + BLOCK_K - 1) / BLOCK_K) && tiles <= splitk_clusters<BN, A_MN, B_MN>(p.splits)) {
     launch_dependent_clusters(gemm_tc_splitk_cluster_kernel<BN, A_MN, B_MN>, grid, kThreads, C::kTotal, stream, p.splits, maps[0], maps[1], p);
     return cudaGetLastError();
   }

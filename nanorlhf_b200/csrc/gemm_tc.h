@@ -48,6 +48,12 @@ struct TcParams {
   const int* grp_num_tiles;     // [1]: row tiles in use
 };
 
+// Is a contraction of `blocks` times 64 columns in `splits` ranges summed by clusters (where they fit)?  Not two long ranges: a cluster of two takes both SMs of a
+// pair that share their way to the L2 and leaves other pairs idle, which costs more than the sum through the workspace from 32 768 columns on.  us, clusters /
+// workspace: 400 x 1536 over 32 768 columns 67.0 / 66.9, 65 536 127.5 / 118.2, 151 936 272 / 263; 554 x 1536 over 16 384 35.7 / 36.8, 32 768 66.7 / 67.1, 65 536 128.6 /
+// 126.9, 151 936 296 / 290; three ranges of 300 x 1536 over 65 536 85.3 / 85.5, eight of 100 x 1536 41.5 / 48.4.
+inline bool split_by_clusters(int splits, long blocks) { return splits > 2 || blocks <= 512; }
+
 }  // namespace tc
 }  // namespace nrl
 

@@ -24,3 +24,16 @@ def test_against_float64(M, N, K, a_mn, b_mn, splits):
     bound = 2.0 ** -8 * want.abs() + K ** 0.5 * 2.0 ** -22 * (A.norm(dim=1)[:, None] * B.norm(dim=0)[None])
     assert ((got.double() - want).abs() <= bound).all()
     assert torch.equal(got, run(splits))
+
+
+@pytest.mark.parametrize("K", [32768, 32832])                # the last pair of ranges that a cluster sums, the first through the workspace
+@pytest.mark.parametrize("M,N", [(129, 72), (16, 64)])
+def test_pairs_of_long_ranges_against_float64(M, N, K):
+    from nanorlhf_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a, b = (torch.randn(r, K, generator=g, device="cuda").bfloat16() for r in (M, N))
+    run = lambda: native.ext().gemm_tc(a, b, False, False, None, None, None, 0, 0.5, None, None, False, 0, 0, 2)  # noqa: E731
+    got, want = run(), 0.5 * (a.double() @ b.double().T)
+    bound = 2.0 ** -8 * want.abs() + K ** 0.5 * 2.0 ** -22 * (a.double().norm(dim=1)[:, None] * b.double().norm(dim=1)[None])
+    assert ((got.double() - want).abs() <= bound).all()
+    assert torch.equal(got, run())
