@@ -8,11 +8,12 @@
 
 namespace nrl {
 
+// early false: behind the end of the kernel in front, where pdl_wait() finds nothing to wait for; cluster 0: as the kernel itself says
 template <class... Params, class... Args>
-inline void launch_dependent_clusters(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+inline void launch_early_if(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = cluster;
   attr[1].val.clusterDim.y = 1;
@@ -23,12 +24,16 @@ inline void launch_dependent_clusters(void (*kernel)(Params...), dim3 grid, dim3
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 0 ? 2 : 1;                  // 0: as the kernel itself says
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 template <class... Params, class... Args>
+inline void launch_dependent_clusters(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+  launch_early_if(true, kernel, grid, block, smem, stream, cluster, std::forward<Args>(args)...);
+}
+template <class... Params, class... Args>
 inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-  launch_dependent_clusters(kernel, grid, block, smem, stream, 0, std::forward<Args>(args)...);
+  launch_early_if(true, kernel, grid, block, smem, stream, 0, std::forward<Args>(args)...);
 }
 
 // how many clusters of `cluster` blocks the GPU runs at a time

@@ -37,7 +37,7 @@ def _unconditional(body):
 def _launched(src):
     """Kernels that a file launches this way, by name or through a variable."""
     names = set()
-    for a in re.findall(r"launch_dependent(?:_clusters)?\(\s*(\w+)", src):
+    for a in re.findall(r"launch_(?:dependent(?:_clusters)?\(|early_if\(early,)\s*(\w+)", src):
         names |= set(re.findall(r"\b" + a + r"\s*=\s*(\w+_kernel)\b", src)) or {a}
     return names
 
