@@ -293,27 +293,14 @@ NRL_DEVICE void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, u
 }
 
 constexpr int kMaxCluster = 4;
-constexpr int kSmemThreads = 512;                                 // 16 warps; two CTAs per SM when the slice is <= ~100 KB
-constexpr int kSmemPerLane = kSmemThreads / 32;
+constexpr int kSmemOrder = 512;                                   // threads of the order in which a slice's masses are summed and drawn from
 constexpr int kSliceBytesMax = 216 * 1024;
 constexpr int kMaxAttempts = 32;                                  // P(32 rejections) <= (1 - top_p)^32; dispatch keeps top_p >= 0.5
 constexpr int kXSlots = 6;                                        // max, mass, and (candidate, mass above) x attempt parity
-constexpr int kPieceVecs = 2 * kSmemThreads;                      // a slice arrives in pieces of two vectors per thread (16 KB)
+constexpr int kPieceVecs = 2 * kSmemOrder;                        // a slice arrives in pieces of 16 KB
 constexpr int kPiecesMax = (kSliceBytesMax / 16 + kPieceVecs - 1) / kPieceVecs;
-constexpr int kWalkMax = (kSliceBytesMax / 16 + kSmemThreads - 1) / kSmemThreads;      // vectors of one thread at most
+constexpr int kWalkMax = (kSliceBytesMax / 16 + kSmemOrder - 1) / kSmemOrder;      // vectors of one thread of the order at most
 static_assert(kWalkMax <= 32, "a lane per vector of the drawn thread");
-
-// every CTA of the cluster publishes `n` floats into slot [my rank] of `dst` in every CTA; after the cluster barrier all CTAs hold
-// all contributions and combine them in rank order (identical result everywhere).  A CTA can run at most one cluster barrier
-// ahead of its peers, and a slot is reused four barriers later at the earliest, so it is never rewritten while still being read.
-NRL_DEVICE void cluster_publish(float (*dst)[2], const float* src, int n, uint32_t my_rank, uint32_t nrank) {
-  if (threadIdx.x < static_cast<unsigned>(n) * nrank) {
-    const uint32_t peer = threadIdx.x / n;
-    const int k = threadIdx.x % n;
-    st_cluster_f32(map_to_rank(&dst[my_rank][k], peer), src[k]);
-  }
-  cluster_sync_all();
-}
 
 NRL_DEVICE uint4 lds_v4(uint32_t saddr) {
   uint4 r;
@@ -362,10 +349,13 @@ NRL_DEVICE float vec_elem(const uint4& raw, int j) {
 // decides a draw is formed in that order from the row's maximum, so that a (seed, row, step) names one token for good.
 // The maximum is taken piece by piece as the bulk copies arrive and the first uniform number is drawn meanwhile; the drawn thread's
 // exponentials are formed by a warp and only added in turn; the verification skips vectors without a more probable token.
-// 1024 x 151 936: 201 us (230 with a maximum pass behind the whole copy and a one-thread walk); the floors are 47 us of reads and about
-// 70 us of 2^x on the special-function unit, the rest waits at the row's exchanges.  One pass for maximum and mass (189 us) and half
-// slices on top of it (180 us) change the sums' last bits and with them 1 to 3 tokens in 1024.
-__global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(const __nv_bfloat16* __restrict__ logits, long row_stride,
+// What bounds it is the chain of a row -- copy, maximum, mass, draw, verification, with an exchange between four blocks behind each -- so rows in flight
+// count: the registers (40) and the shared memory (640 bytes beside the slice; masses pass between threads by shuffles and every thread ends up with a
+// block's sums, one barrier each) leave room for three blocks per SM.  1024 x 151 936: 201 us with two blocks, 3.4 KB and four barriers per sum, 189 with
+// two of this form, 159 with three; 128 rows 34.8 -> 31.6, 1024 x 32 000 51.7 -> 43.3.  256 threads with two vectors each in the same order 162 and slower for
+// few rows.  The floors are 47 us of reads and about 70 us of 2^x on the special-function unit.  One pass for maximum and mass, and half slices on top of
+// it, change the sums' last bits and with them 1 to 3 tokens in 1024.
+__global__ void __launch_bounds__(kSmemOrder, 3) sample_top_p_smem_kernel(const __nv_bfloat16* __restrict__ logits, long row_stride,
                                                                             int V, int slice, float inv_temp, float top_p,
                                                                             unsigned long long seed, unsigned long long step,
                                                                             const int* __restrict__ row_ids,
@@ -373,16 +363,13 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
                                                                             int* __restrict__ out_tokens) {
   extern __shared__ __align__(128) unsigned char s_dyn[];
   __shared__ __align__(8) uint64_t s_bar[kPiecesMax];
-  __shared__ float red[32];
-  __shared__ float s_pub[2];
+  __shared__ float red[2][kSmemOrder / 32];
   __shared__ float s_x[kXSlots][kMaxCluster][2];           // exchange slots, written by the peers
-  __shared__ float chunk_sum[kSmemThreads];
-  __shared__ __align__(16) float s_walk[kWalkMax][8];
-  __shared__ float s_resid, s_u;
-  __shared__ int s_owner;
+  __shared__ float s_part[kSmemOrder / 16];                // masses of sixteen neighbouring threads of the order
+  __shared__ float s_u;
   const uint32_t crank = cluster_ctarank(), csize = cluster_nctarank();
   const int row = blockIdx.x / static_cast<int>(csize);
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int e0 = static_cast<int>(crank) * slice;                                // first token of this CTA's slice
   const int Vl = max(0, min(slice, V - e0));                                     // tokens in the slice (multiple of 8)
   const int nvec = Vl / 8;
@@ -421,35 +408,49 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
     mbar_wait(&s_bar[piece], 0);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int v = v0 + k * kSmemThreads;
+      const int v = v0 + k * kSmemOrder;
       if (v < nvec) {
         const uint4 raw = load(v);
         mx = fmaxf(mx, (sc >= 0.f ? vec_max(raw) : vec_min(raw)) * sc);
       }
     }
   }
-  mx = block_reduce_max(mx, red);
-  if (tid == 0) s_pub[0] = mx;
+  mx = warp_max(mx);
+  if (lane == 0) red[0][warp] = mx;
   __syncthreads();
+  mx = warp_max(lane < kSmemOrder / 32 ? red[0][lane] : -INFINITY);
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster has started
-  cluster_publish(s_x[0], s_pub, 1, crank, csize);
+  auto cluster_publish = [&](int slot, float x) {          // thread r writes the peer of rank r
+    if (tid < static_cast<int>(csize)) st_cluster_f32(map_to_rank(&s_x[slot][crank][0], tid), x);
+    __syncwarp();
+    cluster_sync_all();
+  };
+  cluster_publish(0, mx);
   mx = s_x[0][0][0];
   for (uint32_t r = 1; r < csize; ++r) mx = fmaxf(mx, s_x[0][r][0]);
 
+  // sums of the block in the order: a warp's threads, then the warps; every thread gets the result
+  auto block_sum = [&](float x, float* out) {
+    x = warp_sum(x);
+    if (lane == 0) out[warp] = x;
+    __syncthreads();
+    return warp_sum(lane < kSmemOrder / 32 ? out[lane] : 0.f);
+  };
   // ---- pass 2: un-normalised probability mass per thread, per CTA, per row ----
   float mine = 0.f;
 #pragma unroll 4
-  for (int v = tid; v < nvec; v += kSmemThreads) {
+  for (int v = tid; v < nvec; v += kSmemOrder) {
     float e[8];
     vec_affine(load(v), sc, -mx, e);
 #pragma unroll
     for (int j = 0; j < 8; ++j) mine += exp2f(e[j]);
   }
-  chunk_sum[tid] = mine;
-  const float cta_mass = block_reduce_sum(mine, red);      // (its barriers also publish chunk_sum)
-  if (tid == 0) s_pub[0] = cta_mass;
-  __syncthreads();
-  cluster_publish(s_x[1], s_pub, 1, crank, csize);
+  float part = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) part += __shfl_sync(0xffffffffu, mine, (lane & 16) + i);
+  if ((lane & 15) == 0) s_part[tid >> 4] = part;
+  const float cta_mass = block_sum(mine, red[1]);          // (its barrier also publishes s_part)
+  cluster_publish(1, cta_mass);
   float Z = 0.f, excl_cta = 0.f;
   int last_with_mass = 0;
   for (uint32_t r = 0; r < csize; ++r) {
@@ -472,84 +473,75 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
         acc += s_x[1][r][0];
       }
     }
+    const int cand = 2 + 2 * (attempt & 1);
     if (owner_cta == static_cast<int>(crank)) {            // CTA-uniform branch
       const float ul = fminf(fmaxf(u - excl_cta, 0.f), cta_mass);     // the draw, local to this CTA's mass
-      if (tid < 32) {
-        float local[kSmemPerLane];
-        float tsum = 0.f;
+      // sixteen threads of the order whose mass holds the draw: every warp finds them, the warp that has them goes on
+      const float tsum = s_part[lane];
+      float incl = tsum;
 #pragma unroll
-        for (int i = 0; i < kSmemPerLane; ++i) { local[i] = chunk_sum[tid * kSmemPerLane + i]; tsum += local[i]; }
-        float incl = tsum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          float y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (tid >= o) incl += y;
-        }
-        const float excl = incl - tsum;
-        const unsigned has = __ballot_sync(0xffffffffu, tsum > 0.f);
-        const unsigned ball = __ballot_sync(0xffffffffu, (incl >= ul) && (tsum > 0.f));
-        const int wl = ball ? (__ffs(ball) - 1) : (has ? 31 - __clz(has) : 31);      // numerical slack: the last lane with mass
-        if (tid == wl) {
-          float acc2 = excl;
-          int owner = tid * kSmemPerLane + kSmemPerLane - 1;
-          float resid = 0.f;
-          bool hit = false;
-#pragma unroll
-          for (int i = 0; i < kSmemPerLane; ++i) {
-            if (!hit && local[i] > 0.f && acc2 + local[i] >= ul) { owner = tid * kSmemPerLane + i; resid = ul - acc2; hit = true; }
-            if (!hit) acc2 += local[i];
-          }
-          if (!hit) {   // numerical slack: the last thread with mass takes it
-#pragma unroll
-            for (int i = kSmemPerLane - 1; i >= 0; --i)
-              if (!hit && local[i] > 0.f) { owner = tid * kSmemPerLane + i; resid = local[i]; hit = true; }
-          }
-          s_owner = owner;
-          s_resid = resid;
-        }
+      for (int o = 1; o < 32; o <<= 1) {
+        float y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
       }
-      if (tid < 32) {
-        __syncwarp();
-        // the owner's elements in the order pass 2 summed them: lane k forms the exponentials of its k-th vector, lane 0 adds them up
-        const int owner = s_owner, vk = owner + tid * kSmemThreads;
+      const unsigned has = __ballot_sync(0xffffffffu, tsum > 0.f);
+      const unsigned ball = __ballot_sync(0xffffffffu, (incl >= ul) && (tsum > 0.f));
+      const int wl = ball ? (__ffs(ball) - 1) : (has ? 31 - __clz(has) : 31);      // numerical slack: the last with mass
+      float acc2 = __shfl_sync(0xffffffffu, incl - tsum, wl);
+      if (warp == wl >> 1) {
+        int owner = wl * 16 + 15, last = -1;
+        float resid = 0.f, last_mass = 0.f;
+        bool hit = false;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float x = __shfl_sync(0xffffffffu, mine, (wl & 1) * 16 + i);
+          if (!hit && x > 0.f && acc2 + x >= ul) { owner = wl * 16 + i; resid = ul - acc2; hit = true; }
+          if (!hit) acc2 += x;
+          if (x > 0.f) { last = wl * 16 + i; last_mass = x; }
+        }
+        if (!hit && last >= 0) { owner = last; resid = last_mass; }      // numerical slack: the last thread with mass takes it
+        // the owner's elements in the order pass 2 summed them: lane k forms the exponentials of its k-th vector and adds them to the lanes' before it
+        const int vk = owner + lane * kSmemOrder;
+        float e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (vk < nvec) {
-          float e[8];
           vec_affine(load(vk), sc, -mx, e);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) s_walk[tid][j] = exp2f(e[j]);
+          for (int j = 0; j < 8; ++j) e[j] = exp2f(e[j]);
         }
-        __syncwarp();
-        if (tid == 0) {
-          const float resid = s_resid;
-          float acc2 = 0.f;
-          int tok = -1, last = 0;
-          for (int k = 0; tok < 0 && owner + k * kSmemThreads < nvec; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(&s_walk[k][0]), c = *reinterpret_cast<const float4*>(&s_walk[k][4]);
-            const float e[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-            last = (owner + k * kSmemThreads) * 8 + 7;
+        acc2 = 0.f;
+        int tok = -1;
+        last = 0;
+        for (int k = 0; tok < 0 && owner + k * kSmemOrder < nvec; ++k) {
+          float a = acc2;
+          int at = -1;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              acc2 += e[j];
-              if (tok < 0 && acc2 >= resid) tok = last - 7 + j;
-            }
+          for (int j = 0; j < 8; ++j) {
+            a += e[j];
+            if (at < 0 && a >= resid) at = j;
           }
-          if (tok < 0) tok = last;
-          s_pub[0] = __int_as_float(e0 + tok);
-          s_pub[1] = fmaf(vec_elem(load(tok >> 3), tok & 7), sc, -mx);     // octaves above the rounded row maximum: at most half an ulp of it
+          acc2 = __shfl_sync(0xffffffffu, a, k);
+          at = __shfl_sync(0xffffffffu, at, k);
+          last = (owner + k * kSmemOrder) * 8 + 7;
+          if (at >= 0) tok = last - 7 + at;
+        }
+        if (tok < 0) tok = last;
+        if (lane < static_cast<int>(csize)) {
+          const uint32_t dst = map_to_rank(&s_x[cand][crank][0], lane);
+          st_cluster_f32(dst, __int_as_float(e0 + tok));
+          st_cluster_f32(dst + 4, fmaf(vec_elem(load(tok >> 3), tok & 7), sc, -mx));     // octaves above the rounded row maximum: at most half an ulp of it
         }
       }
     }
-    __syncthreads();
-    float (*slot)[2] = s_x[2 + 2 * (attempt & 1)];
-    cluster_publish(slot, s_pub, 2, crank, csize);         // only the owner's entry is read
-    const int tok = __float_as_int(slot[owner_cta][0]);
-    const float e_tok = slot[owner_cta][1];
+    __syncwarp();
+    cluster_sync_all();                                    // the owner's entry is there
+    const int tok = __float_as_int(s_x[cand][owner_cta][0]);
+    const float e_tok = s_x[cand][owner_cta][1];
     bool accept = top_p >= 1.f || attempt == kMaxAttempts - 1;
     if (!accept) {
       // ---- verification pass: mass of the strictly more probable tokens ----
       float above = 0.f;
 #pragma unroll 4
-      for (int v = tid; v < nvec; v += kSmemThreads) {
+      for (int v = tid; v < nvec; v += kSmemOrder) {
         const uint4 raw = load(v);
         if (fmaf(sc >= 0.f ? vec_max(raw) : vec_min(raw), sc, -mx) > e_tok) {
           float e[8];
@@ -559,13 +551,9 @@ __global__ void __launch_bounds__(kSmemThreads, 2) sample_top_p_smem_kernel(cons
             if (e[j] > e_tok) above += exp2f(e[j]);
         }
       }
-      above = block_reduce_sum(above, red);
-      if (tid == 0) s_pub[0] = above;
-      __syncthreads();
-      float (*slot2)[2] = s_x[3 + 2 * (attempt & 1)];
-      cluster_publish(slot2, s_pub, 1, crank, csize);
+      cluster_publish(cand + 1, block_sum(above, red[attempt & 1]));
       float tot = 0.f;
-      for (uint32_t r = 0; r < csize; ++r) tot += slot2[r][0];
+      for (uint32_t r = 0; r < csize; ++r) tot += s_x[cand + 1][r][0];
       accept = tot < top_p * Z;                            // identical on every CTA
     }
     if (accept) {
@@ -645,7 +633,7 @@ extern "C" cudaError_t nrl_sample(const void* logits, int is_bf16, long row_stri
     static const int env_impl = [] { const char* e = std::getenv("NANORLHF_SAMPLER_KERNEL"); return e && std::string(e) == "stream" ? 1 : 0; }();
     // (21 / 22 / 24: the cluster kernel with 1 / 2 / 4 CTAs per row, for benchmarking)
     int impl = impl_req != 0 ? impl_req : env_impl;
-    // slices of <= 100 KB let two CTAs share an SM (one row's load overlaps another row's passes: 235 vs 254 us at 1024 x 151 936)
+    // slices of <= 100 KB let two CTAs share an SM, of <= 76 160 bytes three (one row's load overlaps other rows' passes)
     int cmin = 1;
     while (cmin < kMaxCluster && (static_cast<long>(V) * 2 + cmin - 1) / cmin > kSliceBytesMax) cmin *= 2;
     int csize = cmin;
@@ -660,12 +648,13 @@ extern "C" cudaError_t nrl_sample(const void* logits, int is_bf16, long row_stri
       static bool smem_configured = false;
       if (!smem_configured) {
         cudaError_t e = cudaFuncSetAttribute(sample_top_p_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSliceBytesMax);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_top_p_smem_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
         smem_configured = true;
       }
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3(static_cast<unsigned>(rows) * csize, 1, 1);
-      cfg.blockDim = dim3(kSmemThreads, 1, 1);
+      cfg.blockDim = dim3(kSmemOrder, 1, 1);
       cfg.dynamicSmemBytes = smem;
       cfg.stream = s;
       cudaLaunchAttribute attr[1];
