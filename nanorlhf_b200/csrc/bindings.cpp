@@ -355,8 +355,10 @@ torch::Tensor gemm_tc_swiglu(const torch::Tensor& a, const torch::Tensor& w_inte
 }
 
 // act[M, F] = silu(x Wg^T + tg Bg^T) * (x Wu^T + tu Bu^T): gate and up weights [F, K] as they are stored, optional adapters (t [M, r], B [F, r])
-torch::Tensor gemm_tc_swiglu_pair(const torch::Tensor& x, const torch::Tensor& wg, const torch::Tensor& wu, const c10::optional<torch::Tensor>& tg,
-                                  const c10::optional<torch::Tensor>& tu, const c10::optional<torch::Tensor>& bg, const c10::optional<torch::Tensor>& bu) {
+// (and, with `keep`, the two projections)
+std::vector<torch::Tensor> gemm_pair(const torch::Tensor& x, const torch::Tensor& wg, const torch::Tensor& wu, const c10::optional<torch::Tensor>& tg,
+                                     const c10::optional<torch::Tensor>& tu, const c10::optional<torch::Tensor>& bg, const c10::optional<torch::Tensor>& bu,
+                                     bool keep) {
   check_tc_operand(x, "x");
   check_tc_operand(wg, "wg");
   check_tc_operand(wu, "wu");
@@ -376,11 +378,12 @@ torch::Tensor gemm_tc_swiglu_pair(const torch::Tensor& x, const torch::Tensor& w
     }
   }
   c10::cuda::CUDAGuard guard(x.device());
-  torch::Tensor out = torch::empty({M, F}, x.options());
-  if (M == 0 || F == 0) return out;
+  std::vector<torch::Tensor> outs;
+  for (int i = 0; i < (keep ? 3 : 1); ++i) outs.push_back(torch::empty({M, F}, x.options()));
+  if (M == 0 || F == 0) return outs;
   const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   auto map = [&](const torch::Tensor& t) { return nrl::make_tma_2d(t.data_ptr(), t.size(0), t.size(1), t.stride(0) * 2, 128, 64, BF, 2); };
-  CUtensorMap maps[8];
+  CUtensorMap maps[10];
   maps[0] = map(x);
   maps[1] = map(wg);
   maps[2] = map(wu);
@@ -388,10 +391,73 @@ torch::Tensor gemm_tc_swiglu_pair(const torch::Tensor& x, const torch::Tensor& w
   maps[4] = r > 0 ? map(*tu) : maps[0];
   maps[5] = r > 0 ? map(*bg) : maps[1];
   maps[6] = r > 0 ? map(*bu) : maps[1];
-  maps[7] = nrl::make_tma_2d(out.data_ptr(), M, F, out.stride(0) * 2, 32, 64, BF, 2);
+  for (size_t i = 0; i < outs.size(); ++i) maps[7 + i] = nrl::make_tma_2d(outs[i].data_ptr(), M, F, outs[i].stride(0) * 2, 32, 64, BF, 2);
   nrl::tc::TcParams p{};
   p.M = static_cast<int>(M); p.N = static_cast<int>(2 * F); p.K = static_cast<int>(K); p.K2 = static_cast<int>(r); p.alpha = 1.f;
-  check(nrl_gemm_tc_pair(maps, &p, num_sms(), cur_stream()), "gemm_tc_swiglu_pair");
+  check(nrl_gemm_tc_pair(maps, &p, keep ? 1 : 0, num_sms(), cur_stream()), "gemm_tc_swiglu_pair");
+  return outs;
+}
+torch::Tensor gemm_tc_swiglu_pair(const torch::Tensor& x, const torch::Tensor& wg, const torch::Tensor& wu, const c10::optional<torch::Tensor>& tg,
+                                  const c10::optional<torch::Tensor>& tu, const c10::optional<torch::Tensor>& bg, const c10::optional<torch::Tensor>& bu) {
+  return gemm_pair(x, wg, wu, tg, tu, bg, bu, false)[0];
+}
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> gemm_tc_swiglu_pair_keep(const torch::Tensor& x, const torch::Tensor& wg, const torch::Tensor& wu,
+                                                                                 const torch::Tensor& tg, const torch::Tensor& tu, const torch::Tensor& bg,
+                                                                                 const torch::Tensor& bu) {
+  const auto o = gemm_pair(x, wg, wu, tg, tu, bg, bu, true);
+  return {o[0], o[1], o[2]};
+}
+
+// (d gate, d up) [M, F] of act = silu(gate) * up, from the gradient behind a projection of act: d act = dy W + t A with W [K, F], A [r, F]
+std::tuple<torch::Tensor, torch::Tensor> gemm_tc_dswiglu(const torch::Tensor& dy, const torch::Tensor& w, const torch::Tensor& t, const torch::Tensor& a,
+                                                         const torch::Tensor& gate, const torch::Tensor& up) {
+  const torch::Tensor* ops[6] = {&dy, &w, &t, &a, &gate, &up};
+  const char* names[6] = {"dy", "w", "t", "a", "gate", "up"};
+  for (int i = 0; i < 6; ++i) check_tc_operand(*ops[i], names[i]);
+  const int64_t M = dy.size(0), K = dy.size(1), F = w.size(1), r = t.size(1);
+  TORCH_CHECK(w.size(0) == K && t.size(0) == M && a.size(0) == r && a.size(1) == F && gate.size(0) == M && gate.size(1) == F && up.sizes() == gate.sizes() &&
+              F % 8 == 0, "gemm_tc_dswiglu: shapes differ");
+  c10::cuda::CUDAGuard guard(dy.device());
+  torch::Tensor dg = torch::empty({M, F}, dy.options()), du = torch::empty({M, F}, dy.options());
+  if (M == 0 || F == 0) return {dg, du};
+  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  auto map = [&](const torch::Tensor& x, int rows) { return nrl::make_tma_2d(x.data_ptr(), x.size(0), x.size(1), x.stride(0) * 2, rows, 64, BF, 2); };
+  const CUtensorMap maps[8] = {map(dy, 128), map(w, 64), map(t, 128), map(a, 64), map(gate, 32), map(up, 32), map(dg, 32), map(du, 32)};
+  nrl::tc::TcParams p{};
+  p.M = static_cast<int>(M); p.N = static_cast<int>(F); p.K = static_cast<int>(K); p.K2 = static_cast<int>(r); p.alpha = 1.f;
+  check(nrl_gemm_tc_dswiglu(maps, &p, num_sms(), cur_stream()), "gemm_tc_dswiglu");
+  return {dg, du};
+}
+
+// sum_i a[i] [M, K_i] . b[i] [K_i, N], summed in one float accumulator
+torch::Tensor gemm_tc_sum(const std::vector<torch::Tensor>& a, const std::vector<torch::Tensor>& b) {
+  const size_t n = a.size();
+  TORCH_CHECK(n >= 1 && n <= nrl::tc::kSumPairs && b.size() == n, "gemm_tc_sum: one to four pairs");
+  for (size_t i = 0; i < n; ++i) {
+    check_tc_operand(a[i], "a");
+    check_tc_operand(b[i], "b");
+    TORCH_CHECK(a[i].size(0) == a[0].size(0) && b[i].size(1) == b[0].size(1) && a[i].size(1) == b[i].size(0), "gemm_tc_sum: shapes differ");
+  }
+  const int64_t M = a[0].size(0), N = b[0].size(1);
+  TORCH_CHECK(N % 8 == 0, "gemm_tc_sum: N must be a multiple of 8");
+  c10::cuda::CUDAGuard guard(a[0].device());
+  torch::Tensor out = torch::empty({M, N}, a[0].options());
+  if (M == 0 || N == 0) return out;
+  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  CUtensorMap maps[2 * nrl::tc::kSumPairs + 1];
+  nrl::tc::TcParams p{};
+  p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.alpha = 1.f;
+  int blocks = 0;
+  for (size_t i = 0; i < nrl::tc::kSumPairs; ++i) {
+    const torch::Tensor &x = a[std::min(i, n - 1)], &y = b[std::min(i, n - 1)];
+    maps[i] = nrl::make_tma_2d(x.data_ptr(), x.size(0), x.size(1), x.stride(0) * 2, 128, 64, BF, 2);
+    maps[nrl::tc::kSumPairs + i] = nrl::make_tma_2d(y.data_ptr(), y.size(0), y.size(1), y.stride(0) * 2, 64, 64, BF, 2);
+    if (i < n) blocks += static_cast<int>((x.size(1) + 63) / 64);
+    p.sum_end[i] = blocks;
+  }
+  maps[2 * nrl::tc::kSumPairs] = nrl::make_tma_2d(out.data_ptr(), M, N, out.stride(0) * 2, 32, 64, BF, 2);
+  const TcChoice ch = pick_tc_tile(M, N, false, true, false);
+  check(nrl_gemm_tc_sum(maps, &p, ch.bn == 64 ? 128 : ch.bn, num_sms(), cur_stream()), "gemm_tc_sum");
   return out;
 }
 
@@ -1218,6 +1284,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return split_choice(M, N, K, sms, [&](int s) { return fits.at(s); });
   }, "auto_splits for a GPU of `sms` SMs that runs fits[s] clusters of s blocks at a time");
   m.def("gemm_tc_split_clusters", &nrl_gemm_tc_split_clusters, py::arg("block_n"), py::arg("splits"));
+  m.def("gemm_tc_swiglu_pair_keep", &gemm_tc_swiglu_pair_keep, "(act, gate, up) of gemm_tc_swiglu_pair with adapters");
+  m.def("gemm_tc_dswiglu", &gemm_tc_dswiglu, "(d gate, d up) of silu(gate) * up behind a projection's backward");
+  m.def("gemm_tc_sum", &gemm_tc_sum, "sum_i a[i] b[i] in one accumulator", py::arg("a"), py::arg("b"));
   m.def("gemm_tc_swiglu_pair", &gemm_tc_swiglu_pair, py::arg("x"), py::arg("wg"), py::arg("wu"), py::arg("tg") = py::none(),
         py::arg("tu") = py::none(), py::arg("bg") = py::none(), py::arg("bu") = py::none());
   m.def("add_layernorm", &add_layernorm);

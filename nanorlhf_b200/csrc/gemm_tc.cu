@@ -52,7 +52,7 @@ constexpr uint32_t kPeerMask = 0xFEFFFFFFu;         // clears the CTA-pair peer 
 constexpr int GROUP_M = 8;                          // tile rows per L2 super-row
 constexpr int kMaxClusterSplits = 8;                // blocks of a portable cluster
 
-template <int CG, int BN, bool B_MN = false>
+template <int CG, int BN, bool B_MN = false, int SLABS = 1>      // SLABS: output slabs of an epilogue warp
 struct Cfg {
   static constexpr int kBRows = BN / CG;                                  // B rows (n) this CTA contributes per k-block
   // an MN-major B tile is made of whole [64 k x 64 n] panels: 96 columns (BN = 192 on a CTA pair) load two panels, the
@@ -60,10 +60,11 @@ struct Cfg {
   static constexpr int kBPanels = (kBRows + 63) / 64;
   static constexpr int kBBytes = B_MN ? kBPanels * kPanelBytes : kBRows * BLOCK_K * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStagesFit = (kSmemBudget - kStagingBytes - 1024) / kStageBytes;
+  static constexpr int kStaging = SLABS * kStagingBytes;
+  static constexpr int kStagesFit = (kSmemBudget - kStaging - 1024) / kStageBytes;
   static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
   static constexpr int kStagingOff = kStages * kStageBytes;
-  static constexpr int kBarOff = kStagingOff + kStagingBytes;
+  static constexpr int kBarOff = kStagingOff + kStaging;
   static constexpr int kTotal = kBarOff + 512;
   static constexpr uint32_t kTmemCols = (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;
   static_assert(kStageBytes % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
@@ -213,10 +214,11 @@ NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F
 // weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
 // columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.
 template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, bool BATCH = false, bool FP8 = false, bool GROUPED = false,
-          bool PAIR = false, bool CLUSTER = false>
+          bool PAIR = false, bool CLUSTER = false, bool SUM = false>
 NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
-                             const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* tmA3 = nullptr) {
-  using C = Cfg<CG, BN, B_MN>;
+                             const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* more = nullptr) {
+  // more: PAIR the up adapter's columns, then (EPI_SWIGLU_KEEP) gate and up; EPI_DSWIGLU gate, up, d up; SUM kSumPairs maps of A and as many of B
+  using C = Cfg<CG, BN, B_MN, EPI == EPI_DSWIGLU ? 2 : 1>;
   constexpr bool kPlainStores = EPI == EPI_F32 || EPI == EPI_GRP_SWIGLU || EPI == EPI_GRP_RELU2;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBarOff);      // CG = 2: the leader's are the live ones
@@ -233,7 +235,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   constexpr int kElemsPerKB = FP8 ? 2 * BLOCK_K : BLOCK_K;                  // 128 bytes of contraction per k-block either way
   const int num_kb1 = (p.K + kElemsPerKB - 1) / kElemsPerKB;
   const int num_kb2 = (p.K2 + kElemsPerKB - 1) / kElemsPerKB;
-  const int num_kb = num_kb1 + (PAIR ? 2 : 1) * num_kb2;
+  const int num_kb = SUM ? p.sum_end[kSumPairs - 1] : num_kb1 + (PAIR ? 2 : 1) * num_kb2;
   const int splits = SPLIT ? p.splits : 1;
   const int kb_per_split = (num_kb + splits - 1) / splits;
   const int tiles_per_batch = num_m * num_n;
@@ -241,9 +243,11 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   volatile int* s_last = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
   if (warp == 0 && lane == 0) {
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
-    if (p.K2 > 0) {
+    if (SUM)
+      for (int i = 0; i < 2 * kSumPairs; ++i) tma_prefetch_desc(more + i);
+    else tma_prefetch_desc(&tmA);
+    if (!SUM) tma_prefetch_desc(&tmB);
+    if (!SUM && p.K2 > 0) {
       tma_prefetch_desc(&tmA2);
       tma_prefetch_desc(&tmB2);
     }
@@ -258,6 +262,8 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       mbar_init(&tmem_full[i], 1);                      // one (multicast) commit
       mbar_init(&tmem_empty[i], CG * kEpiWarps); // the epilogue warps (of both CTAs)
     }
+    if (EPI == EPI_DSWIGLU)
+      for (int i = 0; i < kEpiWarps; ++i) mbar_init(reinterpret_cast<uint64_t*>(smem + C::kBarOff + 256) + i, 1);
     fence_mbar_init();
   }
   if (CG == 2) cluster_sync_all();                      // the peer's barriers exist before anything remote is signalled
@@ -301,10 +307,17 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           const bool second = kb >= num_kb1;
           const CUtensorMap* ma = second ? &tmA2 : &tmA;
           const CUtensorMap* mb = second ? &tmB2 : &tmB;
-          const int k0 = (second ? kb - num_kb1 : kb) * kElemsPerKB;
+          int k0 = (second ? kb - num_kb1 : kb) * kElemsPerKB;
+          if (SUM) {
+            int i = 0;
+            while (kb >= p.sum_end[i]) ++i;              // kb < sum_end[kSumPairs - 1]
+            ma = more + i;
+            mb = more + kSumPairs + i;
+            k0 = (i > 0 ? kb - p.sum_end[i - 1] : kb) * kElemsPerKB;
+          }
           if (PAIR && second) {
             const int which = kb - num_kb1 >= num_kb2 ? 1 : 0, k2 = k0 - which * num_kb2 * kElemsPerKB;
-            tma_load_cg<CG>(sa, which ? tmA3 : &tmA2, &full_bar[stage], k2, m0);
+            tma_load_cg<CG>(sa, which ? more : &tmA2, &full_bar[stage], k2, m0);
             tma_load_cg<CG>(sb, &tmB2, &full_bar[stage], k2, which == static_cast<int>(rank) ? n0 : p.N);
             if (++stage == C::kStages) { stage = 0; phase ^= 1; }
             continue;
@@ -376,7 +389,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     const int epi_tid = threadIdx.x - 64, group = (warp - 2) >> 2;      // the two warps of a quadrant take alternate chunks
     int acc = 0;
     uint32_t acc_phase = 0;
-    uint8_t* slab = smem + C::kStagingOff + (warp - 2) * kSlabBytes;
+    uint8_t* slab = smem + C::kStagingOff + (warp - 2) * (EPI == EPI_DSWIGLU ? 2 : 1) * kSlabBytes;
     const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
     // the accumulator has been read by this warp
     auto release_acc = [&]() {
@@ -388,7 +401,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       }
     };
     // 64 packed columns of this thread's row -> slab -> global
-    auto store_slab = [&](const uint32_t (&pk)[32], int col, int row0, int b) {
+    auto store_slab_to = [&](const CUtensorMap* to, const uint32_t (&pk)[32], int col, int row0, int b) {
       if (lane == 0) tma_store_wait_read<0>();                          // the warp's previous store has drained
       __syncwarp();
       uint8_t* rowp = slab + lane * 128;
@@ -398,11 +411,31 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        if (BATCH) tma_store_3d(&tmD, slab, col, row0, b);
-        else tma_store_2d(&tmD, slab, col, row0);
+        if (BATCH) tma_store_3d(to, slab, col, row0, b);
+        else tma_store_2d(to, slab, col, row0);
         tma_store_commit();
       }
     };
+    auto store_slab = [&](const uint32_t (&pk)[32], int col, int row0, int b) { store_slab_to(&tmD, pk, col, row0, b); };
+    // EPI_DSWIGLU: gate and up of a chunk arrive in the warp's two slabs ahead of its sums and leave as their gradients
+    uint64_t* in_bar = reinterpret_cast<uint64_t*>(smem + C::kBarOff + 256) + (warp - 2);
+    uint32_t in_phase = 0;
+    auto chunk_at = [&](int w, int it, int& col0, int& row0) {
+      const TileCoord c = tile_coord(w, num_m, num_n);
+      col0 = c.n_blk * BN + (it * 2 + group) * 64;
+      row0 = (c.m_tile * CG + static_cast<int>(rank)) * BLOCK_M + quad * 32;
+      return col0 < p.N && row0 < p.M;
+    };
+    auto fetch = [&](int w, int it) {
+      int col0, row0;
+      if (w < num_work && chunk_at(w, it, col0, row0) && lane == 0) {
+        tma_store_wait_read<0>();                          // the slabs' last contents have left
+        mbar_arrive_expect_tx(in_bar, 2 * kSlabBytes);
+        tma_load_2d(slab, more, in_bar, col0, row0);
+        tma_load_2d(slab + kSlabBytes, more + 1, in_bar, col0, row0);
+      }
+    };
+    if (EPI == EPI_DSWIGLU) fetch(unit, 0);
     for (int w = unit; w < num_work; w += num_units) {
       const int tile_id = BATCH ? w % tiles_per_batch : w / splits;
       const int bidx = BATCH ? w / tiles_per_batch : 0;
@@ -517,8 +550,57 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         continue;
       }
+      if (EPI == EPI_DSWIGLU) {
+        // the gradient of the activation is rounded as its own GEMM would leave it, then d gate = g * up * (s + gate s (1 - s)), d up = g * gate * s
+#pragma unroll 1
+        for (int it = 0; it < BN / 128; ++it) {
+          int col0, row0;
+          const bool ok = chunk_at(w, it, col0, row0);
+          uint32_t v[2][32];
+          tmem_ld_32x32b_x32(t_acc + (it * 2 + group) * 64, v[0]);
+          tmem_ld_32x32b_x32(t_acc + (it * 2 + group) * 64 + 32, v[1]);
+          tmem_ld_wait();
+          if (it == BN / 128 - 1) release_acc();
+          if (ok) {
+            mbar_wait(in_bar, in_phase);
+            in_phase ^= 1;
+            uint8_t* rg = slab + lane * 128;
+#pragma unroll
+            for (int q8 = 0; q8 < 8; ++q8) {
+              uint4* pg = reinterpret_cast<uint4*>(rg + ((q8 ^ (lane & 7)) * 16));
+              uint4* pu = reinterpret_cast<uint4*>(rg + kSlabBytes + ((q8 ^ (lane & 7)) * 16));
+              const uint4 g4 = *pg, u4 = *pu;
+              const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
+              uint32_t dg[4], du[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int j = q8 * 8 + 2 * e;
+                const float2 o = unpack_bf16x2(pack_bf16x2(__uint_as_float(v[j >> 5][j & 31]), __uint_as_float(v[j >> 5][(j & 31) + 1])));
+                const float2 a = unpack_bf16x2(gw[e]), b = unpack_bf16x2(uw[e]);
+                const float s0 = 1.f / (1.f + __expf(-a.x)), s1 = 1.f / (1.f + __expf(-a.y));
+                dg[e] = pack_bf16x2(o.x * b.x * (s0 + a.x * s0 * (1.f - s0)), o.y * b.y * (s1 + a.y * s1 * (1.f - s1)));
+                du[e] = pack_bf16x2(o.x * a.x * s0, o.y * a.y * s1);
+              }
+              *pg = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+              *pu = make_uint4(du[0], du[1], du[2], du[3]);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(&tmD, slab, col0, row0);
+              tma_store_2d(more + 2, slab + kSlabBytes, col0, row0);
+              tma_store_commit();
+            }
+          }
+          if (it + 1 < BN / 128) fetch(w, it + 1);
+          else fetch(w + num_units, 0);
+        }
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        continue;
+      }
       if (PAIR) {                                           // group 0 takes features 0 .. 63 of the tile, group 1 the others
-        uint32_t pk[32];
+        constexpr int kKeep = EPI == EPI_SWIGLU_KEEP ? 32 : 1;
+        uint32_t pk[32], gk[kKeep], uk[kKeep];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t g[32], u[32];
@@ -530,13 +612,23 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           for (int j = 0; j < 32; j += 2) {
             // gate and up are rounded as the two projections' own GEMMs leave them and combined as swiglu_kernel combines them: log-probabilities
             // taken outside autograd round as the training forward does, the ratio of an unchanged policy stays 1
-            const float2 gr = unpack_bf16x2(pack_bf16x2(__uint_as_float(g[j]), __uint_as_float(g[j + 1])));
-            const float2 ur = unpack_bf16x2(pack_bf16x2(__uint_as_float(u[j]), __uint_as_float(u[j + 1])));
+            const uint32_t g2 = pack_bf16x2(__uint_as_float(g[j]), __uint_as_float(g[j + 1])), u2 = pack_bf16x2(__uint_as_float(u[j]), __uint_as_float(u[j + 1]));
+            const float2 gr = unpack_bf16x2(g2), ur = unpack_bf16x2(u2);
+            if (EPI == EPI_SWIGLU_KEEP) {
+              gk[(h * 16 + j / 2) % kKeep] = g2;
+              uk[(h * 16 + j / 2) % kKeep] = u2;
+            }
             pk[h * 16 + j / 2] = pack_bf16x2(gr.x / (1.f + __expf(-gr.x)) * ur.x, gr.y / (1.f + __expf(-gr.y)) * ur.y);
           }
         }
         const int col = c.n_blk * (BN / 2) + group * 64;
-        if (col < p.N / 2 && m_blk * BLOCK_M + quad * 32 < p.M) store_slab(pk, col, m_blk * BLOCK_M + quad * 32, 0);
+        if (col < p.N / 2 && m_blk * BLOCK_M + quad * 32 < p.M) {
+          store_slab(pk, col, m_blk * BLOCK_M + quad * 32, 0);
+          if constexpr (EPI == EPI_SWIGLU_KEEP) {
+            store_slab_to(more + 1, gk, col, m_blk * BLOCK_M + quad * 32, 0);
+            store_slab_to(more + 2, uk, col, m_blk * BLOCK_M + quad * 32, 0);
+          }
+        }
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         continue;
       }
@@ -756,12 +848,53 @@ gemm_tc_cg2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   gemm_tc_body<2, BN, A_MN, B_MN, EPI>(tmA, tmB, tmA2, tmB2, tmD, p);
 }
 
+struct TcMaps3 { CUtensorMap m[3]; };
+struct TcMaps8 { CUtensorMap m[2 * kSumPairs]; };
+
+// EPI: EPI_SWIGLU, or EPI_SWIGLU_KEEP where gate and up are wanted too (training); more = {the up adapter's columns, gate, up}.  Two GEMMs and an activation
+// pass move 2.4 times as much memory, the pass alone 54 us of traffic at 6601 x 8960; three stores a tile hide behind its 26 blocks of contraction.
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBg, const __grid_constant__ CUtensorMap tmBu,
-                    const __grid_constant__ CUtensorMap tmA2g, const __grid_constant__ CUtensorMap tmA2u, const __grid_constant__ CUtensorMap tmB2g,
-                    const __grid_constant__ CUtensorMap tmB2u, const __grid_constant__ CUtensorMap tmD, const TcParams p) {
+                    const __grid_constant__ CUtensorMap tmA2g, const __grid_constant__ CUtensorMap tmB2g, const __grid_constant__ CUtensorMap tmB2u,
+                    const __grid_constant__ CUtensorMap tmD, const __grid_constant__ TcMaps3 more, const TcParams p) {
   const bool up = cluster_ctarank() != 0;
-  gemm_tc_body<2, 256, false, false, EPI_SWIGLU, false, false, false, false, true>(tmA, up ? tmBu : tmBg, tmA2g, up ? tmB2u : tmB2g, tmD, p, &tmA2u);
+  gemm_tc_body<2, 256, false, false, EPI, false, false, false, false, true>(tmA, up ? tmBu : tmBg, tmA2g, up ? tmB2u : tmB2g, tmD, p, more.m);
+}
+
+// (d gate, d up) of the SwiGLU from d y of the projection behind it: d act = dY W + T A, which never is in memory; more = {gate, up, d up}.
+// Gate and up of a chunk (32 rows x 64 columns of each, a warp's own) are fetched while its sums are formed and overwritten by their gradients, so that the
+// epilogue holds two slabs a warp and waits for nothing of another warp; one stage of the ring less pays for the second slab.
+// With this, the kept gate and up and sums in one accumulator a decoder layer's forward and backward over 6601 tokens takes 1724 us, 1862 before.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_tc_dswiglu_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA2,
+                       const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmD, const __grid_constant__ TcMaps3 more,
+                       const TcParams p) {
+  gemm_tc_body<2, 256, false, true, EPI_DSWIGLU>(tmA, tmB, tmA2, tmB2, tmD, p, more.m);
+}
+
+// D = the sum of up to kSumPairs products A_i [M, K_i] B_i [K_i, N] in one accumulator: the gradient of an input that several projections share, without a
+// result, an addition and a rounding per projection (6601 x 1536: 60 MB each time)
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_tc_sum_kernel(const __grid_constant__ TcMaps8 maps, const __grid_constant__ CUtensorMap tmD, const TcParams p) {
+  gemm_tc_body<2, BN, false, true, EPI_BF16, false, false, false, false, false, false, true>(tmD, tmD, tmD, tmD, tmD, p, maps.m);
+}
+template <int BN>
+static cudaError_t launch_sum(const TcMaps8& maps, const CUtensorMap& tmD, const TcParams& p, int num_sms, cudaStream_t stream) {
+  using C = Cfg<2, BN, true>;
+  auto kern = gemm_tc_sum_kernel<BN>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  int units = ((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
+  if (units > num_sms / 2) units = num_sms / 2;
+  if (units < 1) units = 1;
+  launch_dependent(kern, 2 * units, kThreads, C::kTotal, stream, maps, tmD, p);
+  return cudaGetLastError();
 }
 
 // FORM: one kernel for each epilogue; with all three behind run-time branches in one kernel steps of 64 to 256 tokens took half a microsecond longer per GEMM
@@ -984,21 +1117,55 @@ extern "C" cudaError_t nrl_gemm_tc_fp8(const CUtensorMap* maps, const nrl::tc::T
   return cudaErrorInvalidValue;
 }
 
-extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream) {
+template <int EPI>
+static cudaError_t launch_pair(const CUtensorMap* maps, const nrl::tc::TcParams& p, int num_sms, cudaStream_t stream) {
   using namespace nrl::tc;
   using C = Cfg<2, 256, false>;
-  if (p->N % 16 != 0) return cudaErrorInvalidValue;
+  auto kern = gemm_tc_pair_kernel<EPI>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  int units = ((p.M + 255) / 256) * ((p.N + 255) / 256);
+  if (units > num_sms / 2) units = num_sms / 2;
+  if (units < 1) units = 1;
+  const TcMaps3 more{{maps[4], EPI == EPI_SWIGLU_KEEP ? maps[8] : maps[7], EPI == EPI_SWIGLU_KEEP ? maps[9] : maps[7]}};
+  nrl::launch_dependent(kern, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[5], maps[6], maps[7], more, p);
+  return cudaGetLastError();
+}
+extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::TcParams* p, int keep, int num_sms, cudaStream_t stream) {
+  if (p->N % 16 != 0) return cudaErrorInvalidValue;
+  return keep ? launch_pair<nrl::tc::EPI_SWIGLU_KEEP>(maps, *p, num_sms, stream) : launch_pair<nrl::tc::EPI_SWIGLU>(maps, *p, num_sms, stream);
+}
+
+extern "C" cudaError_t nrl_gemm_tc_dswiglu(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream) {
+  using namespace nrl::tc;
+  using C = Cfg<2, 256, true, 2>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_dswiglu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
     if (e != cudaSuccess) return e;
     configured = true;
   }
   int units = ((p->M + 255) / 256) * ((p->N + 255) / 256);
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;
-  nrl::launch_dependent(gemm_tc_pair_kernel, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], *p);
+  const TcMaps3 more{{maps[4], maps[5], maps[7]}};
+  nrl::launch_dependent(gemm_tc_dswiglu_kernel, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[6], more, *p);
   return cudaGetLastError();
+}
+
+extern "C" cudaError_t nrl_gemm_tc_sum(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int num_sms, cudaStream_t stream) {
+  using namespace nrl::tc;
+  TcMaps8 all;
+  for (int i = 0; i < 2 * kSumPairs; ++i) all.m[i] = maps[i];
+  const CUtensorMap& d = maps[2 * kSumPairs];
+  if (bn == 256) return launch_sum<256>(all, d, *p, num_sms, stream);
+  if (bn == 192) return launch_sum<192>(all, d, *p, num_sms, stream);
+  if (bn == 128) return launch_sum<128>(all, d, *p, num_sms, stream);
+  return cudaErrorInvalidValue;
 }
 
 extern "C" cudaError_t nrl_gemm_tc_batched(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int num_sms,

@@ -13,8 +13,12 @@ enum TcEpilogue : int {
   EPI_DLOGITS = 3,   // D (bf16, TMA store) = (onehot(target) - exp(alpha * acc - lse)) * grad * alpha: backward of the log-prob head
   EPI_GRP_SWIGLU = 4,  // GROUPED: out_bf16 [rows, N / 2] = silu(gate) * up of row_scale * acc, B rows interleaved as for EPI_SWIGLU, plain stores
   EPI_GRP_RELU2 = 5,   // GROUPED: out_bf16 [rows, N] = relu(row_scale * acc)^2, plain stores
+  EPI_SWIGLU_KEEP = 6,  // PAIR kernels: as EPI_SWIGLU, and gate and up (bf16, TMA store)
+  EPI_DSWIGLU = 7,   // D, D2 (bf16, TMA store) = gradients of gate and up, acc being that of silu(gate) * up
   EPI_SWIGLU = 2,    // D[M, N/2] (bf16, TMA store) = silu(gate) * up; B rows interleaved per 32 features [32 gate | 32 up]
 };
+
+constexpr int kSumPairs = 4;    // products that one accumulator takes (nrl_gemm_tc_sum)
 
 struct TcParams {
   int M, N, K;                  // D is [M, N]; K = contraction length of the first operand pair
@@ -46,6 +50,7 @@ struct TcParams {
   // routing kernels of the same stream), so no launch parameter depends on the routing.
   const int* grp_tiles;         // [max tiles, 3]: expert, first row, end row (exclusive) of the expert's rows
   const int* grp_num_tiles;     // [1]: row tiles in use
+  int sum_end[kSumPairs];       // SUM kernels: k-blocks of the products up to and with the i-th (of those behind the last: as many)
 };
 
 // Is a contraction of `blocks` times 64 columns in `splits` ranges summed by clusters (where they fit)?  Not two long ranges: a cluster of two takes both SMs of a
@@ -76,7 +81,14 @@ extern "C" cudaError_t nrl_gemm_tc_batched(const CUtensorMap* maps, const nrl::t
 extern "C" cudaError_t nrl_gemm_tc_grouped(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int max_tiles, int num_sms,
                                            cudaStream_t stream);
 // act [M, F] = silu(x Wg^T + tg Bg^T) * (x Wu^T + tu Bu^T); maps = {x box {128, 64}, Wg, Wu box {128, 64}, tg, tu box {128, 64}, Bg, Bu box
-// {128, 64}, act box {32, 64}}; p->N = 2 F, p->K2 = columns of tg and tu (0: no adapters, maps 3 .. 6 may repeat a valid one)
-extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream);
+// {128, 64}, act box {32, 64}}; p->N = 2 F, p->K2 = columns of tg and tu (0: no adapters, maps 3 .. 6 may repeat a valid one); keep: x Wg^T + tg Bg^T
+// and x Wu^T + tu Bu^T too, through maps 8 and 9, box {32, 64}
+extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::TcParams* p, int keep, int num_sms, cudaStream_t stream);
+// gradients of gate and up [M, N] from dY [M, K], W [K, N], T [M, K2], A [K2, N] (K2 may be 0): maps = {dY box {128, 64}, W box {64, 64}, T box {128, 64},
+// A box {64, 64}, gate, up, d gate, d up, box {32, 64}}
+extern "C" cudaError_t nrl_gemm_tc_dswiglu(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream);
+// D [M, N] = sum of A_i [M, K_i] B_i [K_i, N] on CTA pairs; maps = {A_0 .. A_3 box {128, 64}, B_0 .. B_3 box {64, 64}, D box {32, 64}}, unused ones repeat a
+// valid one; p->sum_end as there
+extern "C" cudaError_t nrl_gemm_tc_sum(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int num_sms, cudaStream_t stream);
 extern "C" cudaError_t nrl_gemm_tc(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int a_mn, int b_mn,
                                    int epi, int num_sms, cudaStream_t stream);

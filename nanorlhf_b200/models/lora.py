@@ -261,6 +261,19 @@ def fused_swiglu_forward(x, gate, up):
     return _gemm.swiglu_linears(x, (gate.weight, None, None), (up.weight, None, None))
 
 
+def fused_mlp_forward(x, gate, up, down):
+    """``down(silu(gate(x)) * up(x))`` in autograd, for plain LoRA projections without biases; None where the fused form does not apply."""
+    if not torch.is_grad_enabled() or not ops.use_native(x) or x.dtype != torch.bfloat16:
+        return None
+    mods = (gate, up, down)
+    if not all(plain_module(m, LoraLinear) and _adapter_in_gemm(m) and m.bias is None for m in mods):
+        return None
+    if len({(m.r, m.scaling) for m in mods}) != 1:
+        return None
+    from ..ops import gemm as _gemm
+    return _gemm.lora_mlp(x, *[(m.weight, m.lora_A.weight, m.lora_B.weight) for m in mods], scaling=gate.scaling)
+
+
 def iter_lora_layers(model: nn.Module):
     for name, mod in model.named_modules():
         if isinstance(mod, LoraLinear):

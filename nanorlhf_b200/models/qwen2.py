@@ -149,7 +149,10 @@ class Qwen2MLP(nn.Module):
         self.down_proj = Linear(cfg.intermediate_size, cfg.hidden_size, bias=False)
 
     def forward(self, x):
-        from .lora import fused_swiglu_forward, lora_group_forward
+        from .lora import fused_mlp_forward, fused_swiglu_forward, lora_group_forward
+        y = fused_mlp_forward(x, self.gate_proj, self.up_proj, self.down_proj)
+        if y is not None:
+            return y
         act = fused_swiglu_forward(x, self.gate_proj, self.up_proj)
         if act is not None:
             return self.down_proj(act)

@@ -125,12 +125,35 @@ def lora_linear(x, w, bias, a, b, scaling: float):
     return _LoraLinearFn.apply(x, w, bias, a, b, float(scaling))
 
 
+def sum_gemms(a, b):
+    """``sum_i a[i] b[i]`` for the gradient of an input that several projections share: one launch with one float accumulator where none of the
+    products would be cut into ranges of its contraction, else product by product, added in bf16."""
+    pick = _native_mod.ext().gemm_tc_auto_splits
+    if len(a) <= 4 and all(pick(x.shape[0], y.shape[1], x.shape[1]) == 1 for x, y in zip(a, b)):
+        _native_mod._count()
+        return _native_mod.ext().gemm_tc_sum(a, b)
+    out = gemm(a[0], b[0], b_mn=True, a2=a[-1], b2=b[-1])
+    for x, y in zip(a[1:-1], b[1:-1]):
+        out = out + gemm(x, y, b_mn=True)
+    return out
+
+
+def _group_backward(gs, x2, t_cat, a_cat, ws, Bs, s, need_x):
+    """Gradients of a group of LoRA projections of ``x2``: (d x | None, d [A_1; ..; A_n], [d B_i])."""
+    n, r = len(gs), t_cat.shape[1] // len(gs)
+    tp_cat = torch.empty(x2.shape[0], n * r, dtype=x2.dtype, device=x2.device)
+    for i in range(n):
+        gemm(gs[i], Bs[i], b_mn=True, alpha=s, out=tp_cat[:, i * r:(i + 1) * r])               # t'_i = s dy_i B_i
+    gx = sum_gemms([*gs, tp_cat], [*ws, a_cat]) if need_x else None                           # sum_i dy_i W_i + [t'_1 .. t'_n] [A_1; ..; A_n]
+    ga_cat = gemm(tp_cat, x2, a_mn=True, b_mn=True)                                            # [n r, K]
+    return gx, ga_cat, [gemm(gs[i], t_cat[:, i * r:(i + 1) * r], a_mn=True, b_mn=True) for i in range(n)]
+
+
 class _LoraGroupFn(torch.autograd.Function):
     """Several LoRA projections of ONE input (q / k / v, gate / up): the rank-r down-projections share a launch
     (``t = s x [A_1; ...; A_n]^T``), each base GEMM takes its slice of ``t`` as dual-source-K operand, and in the backward the
-    adapter-input gradients ``dA_i`` come out of one GEMM over the concatenated ``t'`` while the whole LoRA term of ``dx`` rides
-    in the first dgrad GEMM (K2 = n r).  Compared with n independent ``_LoraLinearFn``: n - 1 fewer skinny launches per
-    direction, ``x`` is re-read once instead of n times."""
+    adapter-input gradients ``dA_i`` come out of one GEMM over the concatenated ``t'`` and ``dx`` out of one over all projections and the
+    LoRA term.  Compared with n independent ``_LoraLinearFn``: n - 1 fewer skinny launches per direction, ``x`` is re-read once instead of n times."""
 
     @staticmethod
     def forward(ctx, x, scaling, n, *flat):
@@ -150,22 +173,52 @@ class _LoraGroupFn(torch.autograd.Function):
         saved = ctx.saved_tensors
         x2, t_cat, a_cat = saved[:3]
         ws, Bs = saved[3:3 + n], saved[3 + n:3 + 2 * n]
-        gs = [_rows(g) for g in gys]
-        tp_cat = torch.empty(x2.shape[0], n * r, dtype=x2.dtype, device=x2.device)
+        gx, ga_cat, gbs = _group_backward([_rows(g) for g in gys], x2, t_cat, a_cat, ws, Bs, s, ctx.needs_input_grad[0])
+        grads = [gx.view(xshape) if gx is not None else None, None, None]
         for i in range(n):
-            gemm(gs[i], Bs[i], b_mn=True, alpha=s, out=tp_cat[:, i * r:(i + 1) * r])       # t'_i = s dy_i B_i
-        gx = None
-        if ctx.needs_input_grad[0]:
-            gx = gemm(gs[0], ws[0], b_mn=True, a2=tp_cat, b2=a_cat)                          # dy_0 W_0 + [t'_1 .. t'_n] [A_1; ..; A_n]
-            for i in range(1, n):
-                gx = gx + gemm(gs[i], ws[i], b_mn=True)
-            gx = gx.view(xshape)
-        ga_cat = gemm(tp_cat, x2, a_mn=True, b_mn=True)                                       # [n r, K]
-        grads = [gx, None, None]
-        for i in range(n):
-            gb = gemm(gs[i], t_cat[:, i * r:(i + 1) * r], a_mn=True, b_mn=True)             # [N_i, r]
-            grads += [None, None, ga_cat[i * r:(i + 1) * r], gb]
+            grads += [None, None, ga_cat[i * r:(i + 1) * r], gbs[i]]
         return tuple(grads)
+
+
+class _LoraMlpFn(torch.autograd.Function):
+    """``(silu(gate) * up) Wd^T`` with LoRA on all three projections, frozen bases without biases.  Forward: one GEMM leaves gate, up and their
+    product.  Backward: the product's gradient is formed and taken apart into those of gate and up in one GEMM's epilogue and never stored."""
+
+    @staticmethod
+    def forward(ctx, x, scaling, wg, ag, bg, wu, au, bu, wd, ad, bd):
+        x2, r, ext = _rows(x), ag.shape[0], _native_mod.ext()
+        a_cat = torch.cat([ag, au], 0)
+        t_cat = gemm(x2, a_cat, alpha=scaling)
+        _native_mod._count()
+        act, gate, up = ext.gemm_tc_swiglu_pair_keep(x2, wg, wu, t_cat[:, :r], t_cat[:, r:], bg, bu)
+        td = gemm(act, ad, alpha=scaling)
+        y = gemm(act, wd, a2=td, b2=bd)
+        ctx.save_for_backward(x2, t_cat, a_cat, wg, wu, bg, bu, gate, up, act, wd, ad, bd, td)
+        ctx.meta = (scaling, r, x.shape)
+        return y.view(*x.shape[:-1], y.shape[-1])
+
+    @staticmethod
+    def backward(ctx, gy):
+        s, r, xshape = ctx.meta
+        x2, t_cat, a_cat, wg, wu, bg, bu, gate, up, act, wd, ad, bd, td = ctx.saved_tensors
+        g2 = _rows(gy)
+        tpd = gemm(g2, bd, b_mn=True, alpha=s)                                                 # s dy Bd
+        _native_mod._count()
+        dgate, dup = _native_mod.ext().gemm_tc_dswiglu(g2, wd, tpd, ad, gate, up)
+        gad = gemm(tpd, act, a_mn=True, b_mn=True)
+        gbd = gemm(g2, td, a_mn=True, b_mn=True)
+        gx, ga_cat, (gbg, gbu) = _group_backward([dgate, dup], x2, t_cat, a_cat, [wg, wu], [bg, bu], s, ctx.needs_input_grad[0])
+        return (gx.view(xshape) if gx is not None else None, None, None, ga_cat[:r], gbg, None, ga_cat[r:], gbu, None, gad, gbd)
+
+
+def lora_mlp(x, gate, up, down, scaling: float):
+    """``gate`` / ``up`` / ``down`` = (W, A, B); None when the fused form does not take the call."""
+    (wg, ag, bg), (wu, au, bu), (wd, ad, bd) = gate, up, down
+    if (x.numel() == 0 or wg.shape != wu.shape or wd.shape[1] != wg.shape[0] or ag.shape != au.shape or x.shape[-1] != wg.shape[1]
+            or not (lora_supported(x, wg, ag, bg) and lora_supported(x, wu, au, bu)) or ad.shape[1] != wg.shape[0]
+            or any(w.dtype != torch.bfloat16 or not w.is_contiguous() or any(n % 8 for n in w.shape) for w in (wd, ad, bd))):
+        return None
+    return _LoraMlpFn.apply(x, float(scaling), *gate, *up, *down)
 
 
 def lora_linear_group(x, projs, scaling: float):
