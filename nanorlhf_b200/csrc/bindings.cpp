@@ -170,7 +170,65 @@ int64_t split_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits) {
   }
   return best;
 }
+
+// ---- the same on pairs of CTAs (tiles of 256 rows): which form a product with a K-major A takes ----
+// A pair copies half as much of B per product as a block of its own, and copies bound these loops (65 bytes a clock and SM).  The time (us) of a block of 64 columns
+// in a tile `bn` wide grows with the share of the chip in use, up to the power cap.  With it and what the sums of the parts cost, each fitted to the sweep below, a
+// cut on pairs is taken where its estimate is 4 % below that of the form that is taken otherwise: by clusters, where those run at a time, or through a workspace, which
+// costs 5 to 9 us a round of the tiles, for contractions of more than 32 768 columns only (8960: 768 x 1536 22.8 / 22.9, 1024 30.1 / 31.0).
+// us without / with (rows x columns; contraction): 8960, 512 x 1536 21.2 / 20.4 (256 wide, four); 900 29.9 / 24.7 (192, two), 1024 30.1 / 24.8; 768 22.9 / 24.5 not
+// taken; 256 15.0 / 14.1 not taken.  18 944, 256 x 3584 42.9 / 34.7 (256, four), 512 61.0 / 58.3.  4096, 1024 x 1024 14.1 / 13.8; 1536, 1024 x 1536 9.5 / 11.1 not taken.  151 936
+// (through a workspace, 256 wide): 300 x 1536 160 / 175 not taken; 400 206 / 182 (five), 768 305 / 251 (four), 1000 484 / 327 (three), 1300 514 / 482 (four), 1600 698 / 586
+// (five), 2000 777 / 635 (three), 3000 958 uncut, 3800 1549 / 1271 (four), 5000 1911 / 1734 (three).
+struct PairCut { int bn, splits; bool clusters; };       // splits 1: not taken
+inline double pair_block_us(int bn, double load) {
+  const double light = bn == 128 ? 0.2 : bn == 192 ? 0.26 : 0.314, full = bn == 128 ? 0.23 : bn == 192 ? 0.33 : 0.41;
+  return light + (full - light) * std::min(1.0, load);
+}
+constexpr int64_t kPairWorkspaceMax = 128 << 20;         // bytes
+// fits(s) as for split_choice, pair_fits(bn, s): clusters of s pairs that run at a time
+template <class Fits, class PairFits>
+PairCut pair_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits, PairFits pair_fits) {
+  const int64_t blocks = (K + 63) / 64, units = sms / 2, num_m = (M + 255) / 256;
+  PairCut best{0, 1, false};
+  if (N <= 64 || blocks < 16 || units < 1) return best;
+  // the form that is taken otherwise
+  const int64_t tiles1 = split_tiles(M, N), s1 = split_choice(M, N, K, sms, fits);
+  double other;
+  if (s1 > 1) {
+    const bool clusters = nrl::tc::split_by_clusters(static_cast<int>(s1), blocks) && tiles1 <= fits(static_cast<int>(s1));
+    other = (0.2 + 0.07 * std::min(1.0, static_cast<double>(tiles1 * s1) / sms)) * ((blocks + s1 - 1) / s1) + 0.008 * (tiles1 * s1) +
+            (clusters ? 2.5 + (s1 > 4 ? 0.8 : 0.0) : 6.0) + 4.0;
+  } else {
+    other = 1e30;
+    for (int bn : {128, 192, 256}) {
+      const int64_t tiles = num_m * ((N + bn - 1) / bn), waves = (tiles + units - 1) / units;
+      other = std::min(other, waves * blocks * pair_block_us(bn, static_cast<double>(tiles) / (waves * units)) + (bn == 256 ? 4.5 : 4.0));
+    }
+  }
+  double least = 0.96 * other;
+  for (int bn : {128, 192, 256}) {
+    const int64_t tiles = num_m * ((N + bn - 1) / bn);
+    for (int64_t s = 2; s <= 8 && blocks >= 4 * s; ++s) {
+      if (split_ranges(blocks, s) != s) continue;
+      const bool clusters = s <= 4 && tiles <= pair_fits(bn, static_cast<int>(s));
+      if (!clusters && (blocks <= 512 || s * tiles * 256 * bn * 4 > kPairWorkspaceMax)) continue;
+      const int64_t waves = (tiles * s + units - 1) / units;
+      const double loop = pair_block_us(bn, static_cast<double>(tiles * s) / (waves * units)) * ((blocks + s - 1) / s), start = bn == 256 ? 4.5 : 4.0;
+      const double t = clusters ? loop + start + (s == 2 ? 1.8 : s == 3 ? 3.1 : 3.4) : waves * (loop + (bn == 128 ? 5.0 : bn == 192 ? 7.0 : 9.0)) + start;
+      if (t < least) { least = t; best = {bn, static_cast<int>(s), clusters}; }
+    }
+  }
+  return best;
+}
+PairCut auto_pairs(int64_t M, int64_t N, int64_t K) {
+  return pair_choice(M, N, K, num_sms(), [&](int s) { return nrl_gemm_tc_split_clusters(split_block_n(N), s); },
+                     [](int bn, int s) { return nrl_gemm_tc_pair_clusters(bn, s); });
+}
+// ranges of the contraction that gemm_tc adds up for a product with a K-major A, 1: none
 int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
+  const PairCut pc = auto_pairs(M, N, K);
+  if (pc.splits > 1) return pc.splits;
   return split_choice(M, N, K, num_sms(), [&](int s) { return nrl_gemm_tc_split_clusters(split_block_n(N), s); });
 }
 
@@ -213,11 +271,44 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
   if (M == 0 || N == 0) return out;
   // ---- split-K: few output tiles, long contraction (rank-r projections, LoRA weight gradients) ----
   const bool bias_ok = !bias.has_value() || ((reinterpret_cast<uintptr_t>(bias->data_ptr()) & 15) == 0 && bias->is_contiguous());
+  if (K2 == 0 && !f32 && bias_ok && act == 0 && !a_mn && splitk_req != 0 && (cg_req == 2 ? bn_req > 0 && splitk_req > 1 : cg_req <= 0 && bn_req <= 0 && splitk_req < 0)) {
+    PairCut pc = auto_pairs(M, N, K);
+    if (cg_req == 2) {                                     // asked for: by clusters where they fit
+      pc.bn = static_cast<int>(bn_req);
+      pc.splits = static_cast<int>(split_ranges((K + 63) / 64, std::min<int64_t>(splitk_req, (K + 63) / 64)));
+      pc.clusters = ((M + 255) / 256) * ((N + pc.bn - 1) / pc.bn) <= nrl_gemm_tc_pair_clusters(pc.bn, pc.splits);
+    }
+    if (pc.splits > 1) {
+      const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+      const CUtensorMap maps2[2] = {nrl::make_tma_2d(a.data_ptr(), a.size(0), a.size(1), a.stride(0) * 2, 128, 64, BF, 2),
+                                    nrl::make_tma_2d(b.data_ptr(), b.size(0), b.size(1), b.stride(0) * 2, b_mn ? 64 : pc.bn / 2, 64, BF, 2)};
+      nrl::tc::TcParams ps{};
+      ps.M = static_cast<int>(M); ps.N = static_cast<int>(N); ps.K = static_cast<int>(K);
+      ps.alpha = static_cast<float>(alpha);
+      if (bias.has_value()) {
+        TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == torch::kBFloat16 && bias->numel() == N, "gemm_tc: bias must be bf16 [N]");
+        ps.bias = reinterpret_cast<const __nv_bfloat16*>(bias->data_ptr());
+      }
+      ps.splits = pc.splits;
+      ps.out_bf16 = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+      ps.out_stride = out.stride(0);
+      torch::Tensor ws, counters;                          // of this call: products on other streams have their own
+      if (!pc.clusters) {
+        const int64_t tiles = ((M + 255) / 256) * ((N + pc.bn - 1) / pc.bn);
+        ws = torch::empty({pc.splits * tiles * 256 * pc.bn}, a.options().dtype(torch::kFloat32));
+        counters = torch::zeros({2 * tiles}, a.options().dtype(torch::kInt32));
+        ps.ws = ws.data_ptr<float>();
+        ps.counters = counters.data_ptr<int>();
+      }
+      check(nrl_gemm_tc_split_pairs(maps2, &ps, pc.bn, b_mn ? 1 : 0, pc.clusters ? 1 : 0, num_sms(), cur_stream()), "gemm_tc_split_pairs");
+      return out;
+    }
+  }
   if (cg_req <= 0 && bn_req <= 0 && K2 == 0 && !f32 && bias_ok && act == 0 && (a_mn == b_mn || !a_mn) && splitk_req != 0) {
     const int bn = split_block_n(N);
     const int64_t tiles = split_tiles(M, N), num_kb = (K + 63) / 64;
     const int sms = num_sms();
-    int64_t splits = splitk_req > 0 ? splitk_req : auto_splits(M, N, K);
+    int64_t splits = splitk_req > 0 ? splitk_req : split_choice(M, N, K, sms, [&](int s) { return nrl_gemm_tc_split_clusters(bn, s); });
     if (splitk_req > 0 || splits > 1) {
       splits = std::max<int64_t>(1, std::min<int64_t>(splits, num_kb));
       splits = split_ranges(num_kb, splits);
@@ -1282,7 +1373,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_auto_splits", &auto_splits, py::arg("M"), py::arg("N"), py::arg("K"));
   m.def("gemm_tc_split_choice", [](int64_t M, int64_t N, int64_t K, int64_t sms, const std::vector<int>& fits) {
     return split_choice(M, N, K, sms, [&](int s) { return fits.at(s); });
-  }, "auto_splits for a GPU of `sms` SMs that runs fits[s] clusters of s blocks at a time");
+  }, "split_choice for a GPU of `sms` SMs that runs fits[s] clusters of s blocks at a time");
+  m.def("gemm_tc_pair_choice", [](int64_t M, int64_t N, int64_t K, int64_t sms, const std::vector<int>& fits) {
+    const PairCut c = pair_choice(M, N, K, sms, [&](int s) { return fits.at(s); }, [&](int, int s) { return 2 * s <= 8 ? fits.at(2 * s) : 0; });
+    return std::make_tuple(c.bn, c.splits, c.clusters);
+  }, "(tile width, ranges, by clusters) of a cut on pairs of blocks, ranges 1 where it is not taken");
+  m.def("gemm_tc_pair_clusters", &nrl_gemm_tc_pair_clusters);
   m.def("gemm_tc_split_clusters", &nrl_gemm_tc_split_clusters, py::arg("block_n"), py::arg("splits"));
   m.def("gemm_tc_swiglu_pair_keep", &gemm_tc_swiglu_pair_keep, "(act, gate, up) of gemm_tc_swiglu_pair with adapters");
   m.def("gemm_tc_dswiglu", &gemm_tc_dswiglu, "(d gate, d up) of silu(gate) * up behind a projection's backward");

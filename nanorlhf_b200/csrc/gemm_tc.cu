@@ -120,13 +120,14 @@ NRL_DEVICE void umma_fp8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint
 }
 // all MMAs issued so far by this thread arrive on `bar` when they retire (CG = 2: on the barrier at the same offset in
 // BOTH CTAs of the pair)
+// (`pair`: the two blocks' bits among the cluster's)
 template <int CG>
-NRL_DEVICE void umma_commit_cg(uint64_t* bar) {
+NRL_DEVICE void umma_commit_cg(uint64_t* bar, uint32_t pair = 3) {
   if (CG == 1) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
   } else {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3)) : "memory");
+                 ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(pair)) : "memory");
   }
 }
 // TMA tile load; CG = 2: the transaction bytes are credited to the LEADER CTA's barrier (peer bit cleared)
@@ -228,7 +229,8 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = (CG == 2) ? cluster_ctarank() : 0u;
+  const uint32_t rank = (CG == 2) ? cluster_ctarank() & 1u : 0u;
+  const uint32_t pair = (CG == 2 && CLUSTER) ? 3u << (cluster_ctarank() & ~1u) : 3u;
   const bool leader = rank == 0;
   const int num_m = (p.M + CG * BLOCK_M - 1) / (CG * BLOCK_M);
   const int num_n = (p.N + BN - 1) / BN;
@@ -374,10 +376,10 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             if (FP8) umma_fp8<CG>(d_tmem, adesc, bdesc, idesc, ((kb - kb_lo) | k) != 0 ? 1u : 0u);
             else umma_bf16<CG>(d_tmem, adesc, bdesc, idesc, ((kb - kb_lo) | k) != 0 ? 1u : 0u);
           }
-          umma_commit_cg<CG>(&empty_bar[stage]);        // smem stage reusable once these MMAs retire
+          umma_commit_cg<CG>(&empty_bar[stage], pair);  // smem stage reusable once these MMAs retire
           if (++stage == C::kStages) { stage = 0; phase ^= 1; }
         }
-        umma_commit_cg<CG>(&tmem_full[acc]);            // accumulator complete -> epilogue (of both CTAs)
+        umma_commit_cg<CG>(&tmem_full[acc], pair);      // accumulator complete -> epilogue (of both CTAs)
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
@@ -483,7 +485,8 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         const long tile_elems = static_cast<long>(BLOCK_M) * BN;
         // workspace tile layout [BN / 4 column groups][128 rows][4]: a warp's 32 rows of one column group are 512 contiguous
         // bytes, for the partial stores here and for the reduction's loads below
-        float* mine = p.ws + (static_cast<long>(w % splits) * (num_m * num_n) + tile_id) * tile_elems + row_in_tile * 4;
+        const int part_id = tile_id * CG + static_cast<int>(rank), num_parts = num_m * num_n * CG;      // a block's half of a pair's tile
+        float* mine = p.ws + (static_cast<long>(w % splits) * num_parts + part_id) * tile_elems + row_in_tile * 4;
 #pragma unroll 1
         for (int ch = group; ch < BN / 32; ch += 2) {
           uint32_t v[32];
@@ -498,16 +501,16 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         __threadfence();                                   // this thread's partial is visible device-wide ...
         named_barrier_sync(1, kEpiThreads);                // ... and so is every other epilogue thread's
         if (epi_tid == 0) {
-          const int old = atomicAdd(p.counters + tile_id, 1);
+          const int old = atomicAdd(p.counters + part_id, 1);
           const int last = (old == splits - 1) ? 1 : 0;
-          if (last) p.counters[tile_id] = 0;               // self-reset for the next launch
+          if (last) p.counters[part_id] = 0;               // self-reset for the next launch
           __threadfence();
           *s_last = last;
         }
         named_barrier_sync(2, kEpiThreads);
         if (*s_last && row_ok) {
-          const float* base = p.ws + static_cast<long>(tile_id) * tile_elems + row_in_tile * 4;
-          const long split_stride = static_cast<long>(num_m * num_n) * tile_elems;
+          const float* base = p.ws + static_cast<long>(part_id) * tile_elems + row_in_tile * 4;
+          const long split_stride = static_cast<long>(num_parts) * tile_elems;
           __nv_bfloat16* orow = p.out_bf16 + static_cast<long>(row) * p.out_stride + c.n_blk * BN;
 #pragma unroll 1
           for (int c0 = group * 32; c0 < BN; c0 += 64) {
@@ -784,7 +787,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     const int me = unit % splits, units = BLOCK_M * BN / 8;                  // a unit: eight columns of a row
     const uint32_t part = smem_u32(smem);
     for (int u = units * me / splits + threadIdx.x; u < units * (me + 1) / splits; u += kThreads) {
-      const int row = c.m_tile * BLOCK_M + (u & (BLOCK_M - 1)), g8 = u / BLOCK_M, col = c.n_blk * BN + g8 * 8;
+      const int row = (c.m_tile * CG + static_cast<int>(rank)) * BLOCK_M + (u & (BLOCK_M - 1)), g8 = u / BLOCK_M, col = c.n_blk * BN + g8 * 8;
       if (row >= p.M || col >= p.N) continue;              // N % 8 == 0
       const uint32_t at = part + (g8 * 2 * BLOCK_M + (u & (BLOCK_M - 1))) * 16;
       float acc[8];
@@ -796,8 +799,8 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           if (s0 + i < splits) {
-            x[i][0] = ld_cluster_f4(at, s0 + i);
-            x[i][1] = ld_cluster_f4(at + BLOCK_M * 16, s0 + i);
+            x[i][0] = ld_cluster_f4(at, (s0 + i) * CG + rank);
+            x[i][1] = ld_cluster_f4(at + BLOCK_M * 16, (s0 + i) * CG + rank);
           }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -1021,6 +1024,54 @@ gemm_tc_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   gemm_tc_body<1, BN, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
 }
 
+// The same with pairs of blocks on a tile of 256 rows: a cluster is `splits` pairs, and each block sums rows of its own half.
+template <int BN, bool B_MN>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_tc_split_pairs_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
+  static_assert(Cfg<2, BN, B_MN>::kStagingOff >= BLOCK_M * BN * 4, "a part takes the place of the operands");
+  gemm_tc_body<2, BN, false, B_MN, EPI_BF16, true, false, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
+}
+template <int BN, bool B_MN>
+static int split_pairs_clusters(int splits) {
+  if (splits < 2 || 2 * splits > kMaxClusterSplits) return 0;
+  static int fits[kMaxClusterSplits / 2 + 1] = {};                           // plus one
+  if (fits[splits] == 0) {
+    auto kern = gemm_tc_split_pairs_kernel<BN, B_MN>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2, BN, B_MN>::kTotal);
+    fits[splits] = 1 + (e == cudaSuccess ? clusters_at_a_time(kern, kThreads, Cfg<2, BN, B_MN>::kTotal, 2 * splits) : 0);
+  }
+  return fits[splits] - 1;
+}
+// ... or passed through the workspace
+template <int BN, bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_tc_split_pairs_ws_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
+  gemm_tc_body<2, BN, false, B_MN, EPI_BF16, true>(tmA, tmB, tmA, tmB, tmA, p);
+}
+template <int BN, bool B_MN>
+static cudaError_t launch_split_pairs(const CUtensorMap* maps, const TcParams& p, bool clusters, int num_sms, cudaStream_t stream) {
+  using C = Cfg<2, BN, B_MN>;
+  const int tiles = ((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
+  if (clusters) {
+    if (tiles > split_pairs_clusters<BN, B_MN>(p.splits)) return cudaErrorInvalidConfiguration;
+    launch_dependent_clusters(gemm_tc_split_pairs_kernel<BN, B_MN>, tiles * p.splits * 2, kThreads, C::kTotal, stream, 2 * p.splits, maps[0], maps[1], p);
+    return cudaGetLastError();
+  }
+  if (p.ws == nullptr || p.counters == nullptr) return cudaErrorInvalidValue;
+  auto kern = gemm_tc_split_pairs_ws_kernel<BN, B_MN>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  int units = tiles * p.splits;
+  if (units > num_sms / 2) units = num_sms / 2;
+  const bool early = p.K <= 32768;                         // as in launch()
+  launch_early_if(early, kern, 2 * units, kThreads, C::kTotal, stream, 0, maps[0], maps[1], p);
+  return cudaGetLastError();
+}
+
 // clusters of `splits` blocks that run at a time: one block per SM, so the same for all forms of the operands, whose blocks are alike
 static_assert(Cfg<1, 64, true>::kTotal == Cfg<1, 64, false>::kTotal && Cfg<1, 128, true>::kTotal == Cfg<1, 128, false>::kTotal && Cfg<1, 64>::kTotal > kSmemBudget / 2 &&
               Cfg<1, 128>::kTotal > kSmemBudget / 2, "auto_splits asks for one form");
@@ -1187,6 +1238,26 @@ extern "C" cudaError_t nrl_gemm_tc_grouped(const CUtensorMap* maps, const nrl::t
   if (bn == 64) return launch_grouped<64>(maps, *p, max_tiles, num_sms, stream);
   if (bn == 128) return launch_grouped<128>(maps, *p, max_tiles, num_sms, stream);
   if (bn == 256) return launch_grouped<256>(maps, *p, max_tiles, num_sms, stream);
+  return cudaErrorInvalidValue;
+}
+
+extern "C" int nrl_gemm_tc_pair_clusters(int bn, int splits) {
+  using namespace nrl::tc;
+  return bn == 128 ? split_pairs_clusters<128, false>(splits) : bn == 192 ? split_pairs_clusters<192, false>(splits) : split_pairs_clusters<256, false>(splits);
+}
+extern "C" cudaError_t nrl_gemm_tc_split_pairs(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int b_mn, int clusters, int num_sms,
+                                               cudaStream_t stream) {
+  using namespace nrl::tc;
+  if (p->splits < 2 || p->out_bf16 == nullptr || p->K2 != 0) return cudaErrorInvalidValue;
+#define NRL_TC_PAIRS(BN_, BMN_) \
+  if (bn == BN_ && b_mn == (BMN_ ? 1 : 0)) return launch_split_pairs<BN_, BMN_>(maps, *p, clusters != 0, num_sms, stream);
+  NRL_TC_PAIRS(128, false)
+  NRL_TC_PAIRS(128, true)
+  NRL_TC_PAIRS(192, false)
+  NRL_TC_PAIRS(192, true)
+  NRL_TC_PAIRS(256, false)
+  NRL_TC_PAIRS(256, true)
+#undef NRL_TC_PAIRS
   return cudaErrorInvalidValue;
 }
 

@@ -64,6 +64,11 @@ inline bool split_by_clusters(int splits, long blocks) { return splits > 2 || bl
 
 // clusters of `splits` blocks that run at a time (0: none), whichever form the operands have
 extern "C" int nrl_gemm_tc_split_clusters(int bn, int splits);
+// the same for clusters of `splits` pairs of blocks (tiles of 256 x bn), and the GEMM that they run: A K-major (box {128, 64}), B box {bn / 2, 64} or, MN-major,
+// {64, 64}; bf16 output with plain stores; p->splits ranges, none empty
+extern "C" int nrl_gemm_tc_pair_clusters(int bn, int splits);
+extern "C" cudaError_t nrl_gemm_tc_split_pairs(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int b_mn, int clusters, int num_sms,
+                                               cudaStream_t stream);
 extern "C" cudaError_t nrl_gemm_tc_splitk(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int a_mn, int b_mn, int num_sms,
                                           cudaStream_t stream);
 // EPI_DLOGITS on CTA pairs, 256 x 256 tiles; maps = {A box {128, 64}, B box {128, 64}, D box {32, 64}}
