@@ -653,8 +653,8 @@ torch::Tensor gemm_tc_fp8(const torch::Tensor& aq, const torch::Tensor& a_scale,
 // Vocabulary splits of the log-prob head: the (row tile, split) items are walked by one CTA per SM, so the time is the number of rounds
 // times the tiles of an item; of equals the smallest.  6001 rows (47 row tiles) x 151 936: the smallest count that covers the SMs (4, two rounds
 // of 149 tiles) took 2623 us, 22 (seven rounds of 27) 1852 us.
-int pick_splits(int64_t M, int64_t N, int bn) {
-  const int64_t num_m = (M + 127) / 128, num_n = (N + bn - 1) / bn, sms = num_sms();
+int pick_splits(int64_t M, int64_t N, int bn, bool pairs) {
+  const int64_t num_m = (M + (pairs ? 255 : 127)) / (pairs ? 256 : 128), num_n = (N + bn - 1) / bn, sms = num_sms() / (pairs ? 2 : 1);
   int64_t best = 1, least = INT64_MAX;
   for (int64_t s = 1; s <= std::min<int64_t>(num_n, 64); ++s) {
     const int64_t tiles = (num_m * s + sms - 1) / sms * ((num_n + s - 1) / s);
@@ -662,6 +662,12 @@ int pick_splits(int64_t M, int64_t N, int bn) {
   }
   return static_cast<int>(best);
 }
+
+// The head's log-probabilities and the logits' gradient on CTA pairs (256-row tiles, a seventh less time per row) unless the last tile's idle half costs more.
+// 151 936 columns, single CTAs against pairs, the gradient: 128 rows 105 us (pairs not run), 256 rows 123 / 111, 300 rows 143 / 154, 384 rows 148 / 160,
+// 512 rows 195 / 168, 640 rows 225 / 229, 1024 rows 348 / 313, 6001 rows 2009 / 1822; log-probabilities: 256 rows 119 / 109, 512 rows 186 / 174,
+// 1000 rows 339 / 316, 2500 rows 806 / 762, 6001 rows 1839 / 1794, under the power cap 2124 / 2043.
+bool head_pairs(int64_t M) { return 12 * ((M + 255) / 256) <= 7 * ((M + 127) / 128); }
 
 // fused lm-head log-prob forward: returns (logp, entropy, lse), all fp32 [M]
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> lmhead_logprob_fwd(const torch::Tensor& hidden,
@@ -679,7 +685,24 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> lmhead_logprob_fwd(const
   torch::Tensor logp = torch::empty({M}, fopt), ent = torch::empty({M}, fopt), lse = torch::empty({M}, fopt);
   if (M == 0) return {logp, ent, lse};
   const int bn = 256;
-  const int splits = n_splits > 0 ? static_cast<int>(n_splits) : pick_splits(M, V, bn);
+  const bool pairs = head_pairs(M);
+  const int splits = n_splits > 0 ? static_cast<int>(n_splits) : pick_splits(M, V, bn, pairs);
+  if (pairs) {
+    torch::Tensor partials = torch::empty({2 * splits, M, 4}, fopt);
+    const CUtensorMap maps[2] = {nrl::make_tma_2d(hidden.data_ptr(), M, K, hidden.stride(0) * 2, 128, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2),
+                                 nrl::make_tma_2d(weight.data_ptr(), V, K, weight.stride(0) * 2, 128, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2)};
+    nrl::tc::TcParams p{};
+    p.M = M; p.N = V; p.K = K; p.alpha = static_cast<float>(inv_temperature);
+    p.batch = 1;
+    p.splits = 1;
+    p.col_ranges = splits;
+    p.targets = targets.data_ptr<int>();
+    p.out_f32 = partials.data_ptr<float>();
+    check(nrl_gemm_tc_logprob(maps, &p, num_sms(), cur_stream()), "lmhead_logprob_fwd");
+    check(nrl_lmhead_combine(partials.data_ptr<float>(), M, 2 * splits, logp.data_ptr<float>(), ent.data_ptr<float>(), lse.data_ptr<float>(), cur_stream()),
+          "lmhead_combine");
+    return {logp, ent, lse};
+  }
   torch::Tensor partials = torch::empty({splits, M, 4}, fopt);
   CUtensorMap tmA = nrl::make_tma_2d(hidden.data_ptr(), M, K, hidden.stride(0) * 2, 128, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
   CUtensorMap tmB = nrl::make_tma_2d(weight.data_ptr(), V, K, weight.stride(0) * 2, bn, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
@@ -693,11 +716,6 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> lmhead_logprob_fwd(const
   return {logp, ent, lse};
 }
 
-// The logits' gradient on CTA pairs (256-row tiles, a seventh less time per row) unless the last tile's idle half costs more than that.
-// 151 936 columns, single CTAs against pairs: 128 rows 105 us (pairs not run), 256 rows 123 / 111, 300 rows 143 / 154, 384 rows 148 / 160,
-// 512 rows 195 / 168, 640 rows 225 / 229, 1024 rows 348 / 313, 6001 rows 2009 / 1822.
-bool dlogits_pairs(int64_t M) { return 12 * ((M + 255) / 256) <= 7 * ((M + 127) / 128); }
-
 // K-LP backward, stage 1: dZ[M,V] = (onehot - softmax) * grad_logp / T, recomputed through the tensor cores
 torch::Tensor lmhead_dlogits(const torch::Tensor& hidden, const torch::Tensor& weight, const torch::Tensor& targets,
                              const torch::Tensor& lse, const torch::Tensor& grad_logp, double inv_temperature) {
@@ -710,7 +728,7 @@ torch::Tensor lmhead_dlogits(const torch::Tensor& hidden, const torch::Tensor& w
   c10::cuda::CUDAGuard guard(hidden.device());
   torch::Tensor dz = torch::empty({M, V}, hidden.options());
   if (M == 0) return dz;
-  if (dlogits_pairs(M)) {
+  if (head_pairs(M)) {
     auto map_of = [&](const torch::Tensor& t, int64_t rows, int64_t cols, int box) {
       return nrl::make_tma_2d(t.data_ptr(), rows, cols, t.stride(0) * 2, box, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
     };

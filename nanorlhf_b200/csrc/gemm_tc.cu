@@ -220,7 +220,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
                              const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* more = nullptr) {
   // more: PAIR the up adapter's columns, then (EPI_SWIGLU_KEEP) gate and up; EPI_DSWIGLU gate, up, d up; SUM kSumPairs maps of A and as many of B
   using C = Cfg<CG, BN, B_MN, EPI == EPI_DSWIGLU ? 2 : 1>;
-  constexpr bool kPlainStores = EPI == EPI_F32 || EPI == EPI_GRP_SWIGLU || EPI == EPI_GRP_RELU2;
+  constexpr bool kPlainStores = EPI == EPI_F32 || EPI == EPI_LOGPROB || EPI == EPI_GRP_SWIGLU || EPI == EPI_GRP_RELU2;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBarOff);      // CG = 2: the leader's are the live ones
   uint64_t* empty_bar = full_bar + C::kStages;                              // per CTA (multicast commit)
@@ -281,7 +281,17 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   pdl_launch_dependents();
   // SPLIT: work item = (tile, k-range), splits of a tile adjacent.  BATCH: work item = (batch, tile), third TMA coordinate
   // GROUPED: work item = (row tile of the device-side table, column block); the column blocks of a row tile are adjacent
-  const int num_work = GROUPED ? __ldg(p.grp_num_tiles) * num_n : tiles_per_batch * (BATCH ? p.batch : splits);
+  // EPI_LOGPROB: work item = (row tile, range of column tiles), row tiles varying fastest: blocks that share a range walk its weight together
+  constexpr bool kRanges = EPI == EPI_LOGPROB;
+  const int n_per_range = kRanges ? (num_n + p.col_ranges - 1) / p.col_ranges : 1;
+  auto range_of = [&](int w, TileCoord& c) {               // first column tile in c, returns the end
+    if (!kRanges) return c.n_blk + 1;
+    const int g = w / num_m;
+    c.m_tile = w - g * num_m;
+    c.n_blk = g * n_per_range;
+    return min(num_n, c.n_blk + n_per_range);
+  };
+  const int num_work = GROUPED ? __ldg(p.grp_num_tiles) * num_n : kRanges ? num_m * p.col_ranges : tiles_per_batch * (BATCH ? p.batch : splits);
 
   if (warp == 0) {
     // ================================ TMA producer (every CTA) ================================
@@ -290,60 +300,64 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       uint32_t phase = 0;
       for (int w = unit; w < num_work; w += num_units) {
         const int bidx = BATCH ? w / tiles_per_batch : 0;
-        TileCoord c = GROUPED ? TileCoord{0, 0} : tile_coord(BATCH ? w % tiles_per_batch : w / splits, num_m, num_n);
-        int m0 = (c.m_tile * CG + static_cast<int>(rank)) * BLOCK_M;
-        int n0 = c.n_blk * BN + static_cast<int>(rank) * C::kBRows;
-        if (GROUPED) {
-          const int mt = w / num_n;
-          c.n_blk = w - mt * num_n;
-          m0 = __ldg(p.grp_tiles + 3 * mt + 1);
-          n0 = __ldg(p.grp_tiles + 3 * mt) * p.N + c.n_blk * BN;      // the expert's block of B rows
-        }
-        if (PAIR) n0 = c.n_blk * (BN / 2);
-        const int kb_lo = BATCH ? 0 : (w % splits) * kb_per_split, kb_hi = BATCH ? num_kb : min(num_kb, kb_lo + kb_per_split);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          mbar_wait(&empty_bar[stage], phase ^ 1);
-          uint8_t* sa = smem + stage * C::kStageBytes;
-          uint8_t* sb = sa + kABytes;
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], CG * C::kStageBytes);
-          const bool second = kb >= num_kb1;
-          const CUtensorMap* ma = second ? &tmA2 : &tmA;
-          const CUtensorMap* mb = second ? &tmB2 : &tmB;
-          int k0 = (second ? kb - num_kb1 : kb) * kElemsPerKB;
-          if (SUM) {
-            int i = 0;
-            while (kb >= p.sum_end[i]) ++i;              // kb < sum_end[kSumPairs - 1]
-            ma = more + i;
-            mb = more + kSumPairs + i;
-            k0 = (i > 0 ? kb - p.sum_end[i - 1] : kb) * kElemsPerKB;
+        TileCoord c = GROUPED || kRanges ? TileCoord{0, 0} : tile_coord(BATCH ? w % tiles_per_batch : w / splits, num_m, num_n);
+        const int n_end = range_of(w, c);
+        for (; c.n_blk < n_end; ++c.n_blk) {
+          int m0 = (c.m_tile * CG + static_cast<int>(rank)) * BLOCK_M;
+          int n0 = c.n_blk * BN + static_cast<int>(rank) * C::kBRows;
+          if (GROUPED) {
+            const int mt = w / num_n;
+            c.n_blk = w - mt * num_n;
+            m0 = __ldg(p.grp_tiles + 3 * mt + 1);
+            n0 = __ldg(p.grp_tiles + 3 * mt) * p.N + c.n_blk * BN;      // the expert's block of B rows
           }
-          if (PAIR && second) {
-            const int which = kb - num_kb1 >= num_kb2 ? 1 : 0, k2 = k0 - which * num_kb2 * kElemsPerKB;
-            tma_load_cg<CG>(sa, which ? more : &tmA2, &full_bar[stage], k2, m0);
-            tma_load_cg<CG>(sb, &tmB2, &full_bar[stage], k2, which == static_cast<int>(rank) ? n0 : p.N);
-            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-            continue;
-          }
-          if (BATCH) {
-            tma_load3_cg<CG>(sa, ma, &full_bar[stage], k0, m0, bidx);
-            tma_load3_cg<CG>(sb, mb, &full_bar[stage], k0, n0, bidx);
-            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-            continue;
-          }
-          if (A_MN) {          // stored [K rows][M cols]: two [64 k x 64 m] panels
-            tma_load_cg<CG>(sa, ma, &full_bar[stage], m0, k0);
-            tma_load_cg<CG>(sa + kPanelBytes, ma, &full_bar[stage], m0 + 64, k0);
-          } else {
-            tma_load_cg<CG>(sa, ma, &full_bar[stage], k0, m0);
-          }
-          if (B_MN) {
+          if (PAIR) n0 = c.n_blk * (BN / 2);
+          const int kb_lo = BATCH ? 0 : (w % splits) * kb_per_split, kb_hi = BATCH ? num_kb : min(num_kb, kb_lo + kb_per_split);
+          for (int kb = kb_lo; kb < kb_hi; ++kb) {
+            mbar_wait(&empty_bar[stage], phase ^ 1);
+            uint8_t* sa = smem + stage * C::kStageBytes;
+            uint8_t* sb = sa + kABytes;
+            if (leader) mbar_arrive_expect_tx(&full_bar[stage], CG * C::kStageBytes);
+            const bool second = kb >= num_kb1;
+            const CUtensorMap* ma = second ? &tmA2 : &tmA;
+            const CUtensorMap* mb = second ? &tmB2 : &tmB;
+            int k0 = (second ? kb - num_kb1 : kb) * kElemsPerKB;
+            if (SUM) {
+              int i = 0;
+              while (kb >= p.sum_end[i]) ++i;              // kb < sum_end[kSumPairs - 1]
+              ma = more + i;
+              mb = more + kSumPairs + i;
+              k0 = (i > 0 ? kb - p.sum_end[i - 1] : kb) * kElemsPerKB;
+            }
+            if (PAIR && second) {
+              const int which = kb - num_kb1 >= num_kb2 ? 1 : 0, k2 = k0 - which * num_kb2 * kElemsPerKB;
+              tma_load_cg<CG>(sa, which ? more : &tmA2, &full_bar[stage], k2, m0);
+              tma_load_cg<CG>(sb, &tmB2, &full_bar[stage], k2, which == static_cast<int>(rank) ? n0 : p.N);
+              if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+              continue;
+            }
+            if (BATCH) {
+              tma_load3_cg<CG>(sa, ma, &full_bar[stage], k0, m0, bidx);
+              tma_load3_cg<CG>(sb, mb, &full_bar[stage], k0, n0, bidx);
+              if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+              continue;
+            }
+            if (A_MN) {          // stored [K rows][M cols]: two [64 k x 64 m] panels
+              tma_load_cg<CG>(sa, ma, &full_bar[stage], m0, k0);
+              tma_load_cg<CG>(sa + kPanelBytes, ma, &full_bar[stage], m0 + 64, k0);
+            } else {
+              tma_load_cg<CG>(sa, ma, &full_bar[stage], k0, m0);
+            }
+            if (B_MN) {
 #pragma unroll
-            for (int pn = 0; pn < C::kBPanels; ++pn)
-              tma_load_cg<CG>(sb + pn * kPanelBytes, mb, &full_bar[stage], n0 + pn * 64, k0);
-          } else {
-            tma_load_cg<CG>(sb, mb, &full_bar[stage], k0, n0);
+              for (int pn = 0; pn < C::kBPanels; ++pn)
+                tma_load_cg<CG>(sb + pn * kPanelBytes, mb, &full_bar[stage], n0 + pn * 64, k0);
+            } else {
+              tma_load_cg<CG>(sb, mb, &full_bar[stage], k0, n0);
+            }
+            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
           }
-          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          if (!kRanges) break;
         }
       }
     }
@@ -357,30 +371,34 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       int acc = 0;
       uint32_t acc_phase = 0;
       for (int w = unit; w < num_work; w += num_units) {
-        mbar_wait(&tmem_empty[acc], acc_phase ^ 1);
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        const int kb_lo = BATCH ? 0 : (w % splits) * kb_per_split, kb_hi = BATCH ? num_kb : min(num_kb, kb_lo + kb_per_split);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          mbar_wait(&full_bar[stage], phase);
+        TileCoord c{0, 0};
+        const int n_end = range_of(w, c);
+        for (; c.n_blk < n_end; ++c.n_blk) {
+          mbar_wait(&tmem_empty[acc], acc_phase ^ 1);
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * C::kStageBytes);
-          const uint32_t b_addr = a_addr + kABytes;
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          const int kb_lo = BATCH ? 0 : (w % splits) * kb_per_split, kb_hi = BATCH ? num_kb : min(num_kb, kb_lo + kb_per_split);
+          for (int kb = kb_lo; kb < kb_hi; ++kb) {
+            mbar_wait(&full_bar[stage], phase);
+            tc_fence_after();
+            const uint32_t a_addr = smem_u32(smem + stage * C::kStageBytes);
+            const uint32_t b_addr = a_addr + kABytes;
 #pragma unroll
-          for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-            // K-major: 16 contraction elements = 32 bytes along the swizzled row; MN-major: 16 contraction rows = 2048 B
-            const uint64_t adesc = A_MN ? make_smem_desc_sw128_mn(a_addr + k * UMMA_K * 128, kPanelBytes)
-                                        : make_smem_desc_sw128(a_addr + k * UMMA_K * 2);
-            const uint64_t bdesc = B_MN ? make_smem_desc_sw128_mn(b_addr + k * UMMA_K * 128, kPanelBytes)
-                                        : make_smem_desc_sw128(b_addr + k * UMMA_K * 2);
-            if (FP8) umma_fp8<CG>(d_tmem, adesc, bdesc, idesc, ((kb - kb_lo) | k) != 0 ? 1u : 0u);
-            else umma_bf16<CG>(d_tmem, adesc, bdesc, idesc, ((kb - kb_lo) | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+              // K-major: 16 contraction elements = 32 bytes along the swizzled row; MN-major: 16 contraction rows = 2048 B
+              const uint64_t adesc = A_MN ? make_smem_desc_sw128_mn(a_addr + k * UMMA_K * 128, kPanelBytes)
+                                          : make_smem_desc_sw128(a_addr + k * UMMA_K * 2);
+              const uint64_t bdesc = B_MN ? make_smem_desc_sw128_mn(b_addr + k * UMMA_K * 128, kPanelBytes)
+                                          : make_smem_desc_sw128(b_addr + k * UMMA_K * 2);
+              if (FP8) umma_fp8<CG>(d_tmem, adesc, bdesc, idesc, ((kb - kb_lo) | k) != 0 ? 1u : 0u);
+              else umma_bf16<CG>(d_tmem, adesc, bdesc, idesc, ((kb - kb_lo) | k) != 0 ? 1u : 0u);
+            }
+            umma_commit_cg<CG>(&empty_bar[stage], pair);  // smem stage reusable once these MMAs retire
+            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
           }
-          umma_commit_cg<CG>(&empty_bar[stage], pair);  // smem stage reusable once these MMAs retire
-          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          umma_commit_cg<CG>(&tmem_full[acc], pair);      // accumulator complete -> epilogue (of both CTAs)
+          if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
-        umma_commit_cg<CG>(&tmem_full[acc], pair);      // accumulator complete -> epilogue (of both CTAs)
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
     __syncwarp();
@@ -442,7 +460,8 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       const int tile_id = BATCH ? w % tiles_per_batch : w / splits;
       const int bidx = BATCH ? w / tiles_per_batch : 0;
       (void)bidx;
-      TileCoord c = GROUPED ? TileCoord{0, 0} : tile_coord(tile_id, num_m, num_n);
+      TileCoord c = GROUPED || kRanges ? TileCoord{0, 0} : tile_coord(tile_id, num_m, num_n);
+      const int n_end = range_of(w, c);
       const int m_blk = c.m_tile * CG + static_cast<int>(rank);
       int row = m_blk * BLOCK_M + row_in_tile;
       int row_end = p.M;
@@ -453,6 +472,52 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
         row_end = __ldg(p.grp_tiles + 3 * mt + 2);
       }
       const bool row_ok = row < row_end;
+      if (EPI == EPI_LOGPROB) {
+        // per row and warp group: largest logit, sum of exponentials, sum of exponential times logit and the target's logit over the item's columns
+        constexpr float kLog2e = 1.4426950408889634f;
+        const int target = row_ok ? p.targets[row] : -1;
+        float run_max = -INFINITY, run_sum = 0.f, run_ez = 0.f, tgt = -INFINITY;
+        for (; c.n_blk < n_end; ++c.n_blk) {
+          mbar_wait(&tmem_full[acc], acc_phase);
+          tc_fence_after();
+          const uint32_t t_acc = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
+#pragma unroll 1
+          for (int it = 0; it < BN / 128; ++it) {
+            uint32_t v[2][32];
+            tmem_ld_32x32b_x32(t_acc + (it * 2 + group) * 64, v[0]);
+            tmem_ld_32x32b_x32(t_acc + (it * 2 + group) * 64 + 32, v[1]);
+            tmem_ld_wait();
+            if (it == BN / 128 - 1) release_acc();
+            const int col0 = c.n_blk * BN + (it * 2 + group) * 64;
+            float cmax = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 64; ++j) {
+              float z = __uint_as_float(v[j >> 5][j & 31]) * p.alpha;
+              z = col0 + j < p.N ? z : -INFINITY;
+              v[j >> 5][j & 31] = __float_as_uint(z);
+              cmax = fmaxf(cmax, z);
+              if (col0 + j == target) tgt = z;
+            }
+            const float new_max = fmaxf(run_max, cmax);
+            if (new_max > -INFINITY) {
+              const float corr = exp2f((run_max - new_max) * kLog2e), mb = new_max * kLog2e;      // exp2(-inf) = 0 on the first chunk
+              run_sum *= corr;
+              run_ez *= corr;
+#pragma unroll
+              for (int j = 0; j < 64; ++j) {
+                const float z = __uint_as_float(v[j >> 5][j & 31]), e = exp2f(fmaf(z, kLog2e, -mb));
+                run_sum += e;
+                run_ez = fmaf(e, z == -INFINITY ? 0.f : z, run_ez);
+              }
+              run_max = new_max;
+            }
+          }
+          if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        }
+        if (row_ok)
+          reinterpret_cast<float4*>(p.out_f32)[static_cast<size_t>((w / num_m) * 2 + group) * p.M + row] = make_float4(run_max, run_sum, run_ez, tgt);
+        continue;
+      }
       mbar_wait(&tmem_full[acc], acc_phase);
       tc_fence_after();
       const uint32_t t_acc = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
@@ -1113,7 +1178,7 @@ template <int CG, int BN, bool A_MN, bool B_MN, int EPI>
 static cudaError_t launch(const CUtensorMap* maps, const TcParams& p, int num_sms, cudaStream_t stream) {
   using C = Cfg<CG, BN, B_MN>;
   const int num_m = (p.M + CG * BLOCK_M - 1) / (CG * BLOCK_M), num_n = (p.N + BN - 1) / BN;
-  int units = num_m * num_n;
+  int units = num_m * (EPI == EPI_LOGPROB ? p.col_ranges : num_n);
   if (units > num_sms / CG) units = num_sms / CG;
   if (units < 1) units = 1;
   // Blocks that start early take the SMs that the kernel in front leaves first, side by side rather than spread over the chip, and share what those have of the way
@@ -1166,6 +1231,11 @@ extern "C" cudaError_t nrl_gemm_tc_fp8(const CUtensorMap* maps, const nrl::tc::T
   if (!swiglu && cg == 2 && bn == 192) return launch_fp8<2, 192, EPI_BF16>(maps, *p, num_sms, stream);
   if (!swiglu && cg == 1 && bn == 192) return launch_fp8<1, 192, EPI_BF16>(maps, *p, num_sms, stream);
   return cudaErrorInvalidValue;
+}
+
+extern "C" cudaError_t nrl_gemm_tc_logprob(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream) {
+  const CUtensorMap all[5] = {maps[0], maps[1], maps[0], maps[1], maps[0]};
+  return nrl::tc::launch<2, 256, false, false, nrl::tc::EPI_LOGPROB>(all, *p, num_sms, stream);
 }
 
 template <int EPI>

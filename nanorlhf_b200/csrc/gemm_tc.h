@@ -15,6 +15,7 @@ enum TcEpilogue : int {
   EPI_GRP_RELU2 = 5,   // GROUPED: out_bf16 [rows, N] = relu(row_scale * acc)^2, plain stores
   EPI_SWIGLU_KEEP = 6,  // PAIR kernels: as EPI_SWIGLU, and gate and up (bf16, TMA store)
   EPI_DSWIGLU = 7,   // D, D2 (bf16, TMA store) = gradients of gate and up, acc being that of silu(gate) * up
+  EPI_LOGPROB = 8,   // out_f32 [2 col_ranges, M, 4] = statistics of a row over half a range's columns: max, sum of exp, sum of exp * logit, target's logit
   EPI_SWIGLU = 2,    // D[M, N/2] (bf16, TMA store) = silu(gate) * up; B rows interleaved per 32 features [32 gate | 32 up]
 };
 
@@ -25,7 +26,8 @@ struct TcParams {
   int K2;                       // contraction length of the second operand pair (0 = none)
   const float* row_scale;       // FP8 kernels: [M] per-token dequantisation scale of A (GROUPED: see below)
   const float* col_scale;       // FP8 kernels: [N] per-output-channel dequantisation scale of B
-  const int* targets;           // EPI_DLOGITS: [M] column of the row's target
+  int col_ranges;               // EPI_LOGPROB: into how many ranges the column tiles are cut (work items = row tiles x ranges)
+  const int* targets;           // EPI_LOGPROB, EPI_DLOGITS: [M] column of the row's target
   const float* lse;             // EPI_DLOGITS: [M] log of the row's sum of exponentials
   const float* grad;            // EPI_DLOGITS: [M] gradient of the row's log-probability
   int batch;                    // BATCH kernels: number of independent [M,K] x [N,K]^T problems behind 3D tensor maps (else 1)
@@ -73,6 +75,8 @@ extern "C" cudaError_t nrl_gemm_tc_splitk(const CUtensorMap* maps, const nrl::tc
                                           cudaStream_t stream);
 // EPI_DLOGITS on CTA pairs, 256 x 256 tiles; maps = {A box {128, 64}, B box {128, 64}, D box {32, 64}}
 extern "C" cudaError_t nrl_gemm_tc_dlogits(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream);
+// EPI_LOGPROB likewise; maps = {A box {128, 64}, B box {128, 64}}
+extern "C" cudaError_t nrl_gemm_tc_logprob(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream);
 extern "C" cudaError_t nrl_gemm_tc_fp8(const CUtensorMap* maps, const nrl::tc::TcParams* p, int cg, int bn, int swiglu, int num_sms,
                                        cudaStream_t stream);
 // batched K-major x K-major GEMM, bf16 out; maps = {A, B, D} 3D (tma_host.h make_tma_3d), B box rows = bn / cg
