@@ -150,10 +150,14 @@ void delta_scan(const Tensor& qkv, int64_t col_k, int64_t col_v, const c10::opti
   const int heads = static_cast<int>(state.size(1)), D = static_cast<int>(state.size(2)), Dv = static_cast<int>(state.size(3));
   const int E = static_cast<int>(start.numel());
   TORCH_CHECK(qkv.dim() == 2 && col_v + heads * Dv <= qkv.size(1) && o.is_contiguous() && o.size(-1) == heads * Dv, "delta_scan: shapes");
+  const long bytes = nrl_delta_scan_scratch(f32(qkv, "qkv"), qkv.stride(0), static_cast<int>(col_k), static_cast<int>(col_v), E, qkv.size(0), heads, D, Dv,
+                                            per_channel ? 1 : 0, static_cast<int>(impl), num_sms());
+  torch::Tensor scratch;                                     // of this call: steps on other streams have their own
+  if (bytes > 0) scratch = torch::empty({bytes}, qkv.options().dtype(torch::kUInt8));
   check(nrl_delta_scan(f32(qkv, "qkv"), qkv.stride(0), static_cast<int>(col_k), static_cast<int>(col_v), beta.has_value() ? f32(*beta, "beta") : nullptr,
                        f32(decay, "decay"), f32w(state, "state"), f32w(o, "o"), i32(cu, "cu"), i32(start, "start"),
                        i32(state_slot, "state_slot"), E, static_cast<int>(qkv.size(0)), heads, static_cast<int>(kv_heads), D, Dv, per_channel ? 1 : 0,
-                       static_cast<int>(impl), num_sms(), cur_stream()),
+                       static_cast<int>(impl), num_sms(), bytes > 0 ? scratch.data_ptr() : nullptr, cur_stream()),
         "delta_scan");
 }
 
@@ -808,6 +812,8 @@ void bind_hybrid(pybind11::module_& m) {
   m.def("delta_prep", &delta_prep, "unit q / k, beta and decays of the gated delta rule");
   m.def("delta_scan_chunked", &nrl_delta_scan_chunked, "a step goes 32 tokens at a time", pybind11::arg("E"), pybind11::arg("T"), pybind11::arg("heads"),
         pybind11::arg("D"), pybind11::arg("Dv"), pybind11::arg("num_sms"));
+  m.def("delta_scan_shared", &nrl_delta_scan_shared, "blocks of a step taken 32 tokens at a time share its chunks", pybind11::arg("E"), pybind11::arg("T"),
+        pybind11::arg("heads"), pybind11::arg("Dv"), pybind11::arg("num_sms"));
   m.def("delta_scan_blocked", &nrl_delta_scan_blocked, "a step goes four tokens at a time", pybind11::arg("E"), pybind11::arg("T"), pybind11::arg("D"),
         pybind11::arg("Dv"));
   m.def("delta_scan", &delta_scan, "gated delta rule scan, state carried per slot");

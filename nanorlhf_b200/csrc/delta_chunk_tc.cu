@@ -126,15 +126,90 @@ NRL_DEVICE void bulk_load(float* dst, const float* src, uint32_t bytes, uint64_t
 NRL_DEVICE int pair_a(int pr) { return (0x010210 >> (4 * pr)) & 3; }
 NRL_DEVICE int pair_b(int pr) { return (0x001012 >> (4 * pr)) & 3; }
 
+// More items (entry, head, 128 columns) than SMs: their chunks lie on a line, entry by entry, and block j takes the `per` chunks of it from j per on, an even share or
+// the longest item.  An item that a block's end cuts is computed first by the block behind, at that block's start (its first chunks, as many as lie there
+// on the line), and then by this block, at its end, from the state that the other has left: no item is longer than `per`, so that state is there by then.
+// Blocks start from the line's end, so that none waits for one that starts later; should the wait run out all the same, the state becomes NaN.
+// The segments are laid out by a kernel of their own, and between two segments the block starts anew (barriers and all): code that every warp runs through is
+// dear here.  With phases that run on over the segments a chunk took 19 % longer, so 13 % (92 KB of code, 78 for whole items).
+// 10 x 2048 tokens, 16 heads of 128 x 128 (160 items of 64 chunks on 148 SMs): two rounds of 64 chunks 625 us, 70 chunks in a row 381 us.  When it is taken: recurrent.cu.
+struct DcSegment {
+  int t0, n, t1;              // first token, chunks, end of the entry's tokens
+  int h, cb0, e;              // head, first column, entry
+  int in, out;                // the state comes from the block behind / goes to the block in front
+};
+struct DcLine {
+  DcSegment* segments;        // [items + blocks]; null: a block per item
+  int *first, *last;          // [blocks] a block's segments
+  int* handed;                // [blocks] 1 once the state that the block hands on is there
+  float* carry;               // [blocks][128][128]
+};
+constexpr int kDcMaxEntries = 4096;
+
+__global__ void __launch_bounds__(1024) delta_line_kernel(const int* __restrict__ cu, int E, int heads, int parts, int blocks, const DcLine l) {
+  __shared__ int from[kDcMaxEntries + 1];                  // chunks of an item of the entries in front
+  __shared__ int most[32];
+  const int tid = threadIdx.x, items = heads * parts;
+  for (int b = tid; b < blocks; b += blockDim.x) l.first[b] = l.last[b] = l.handed[b] = 0;
+  auto chunks = [&](int e) { return max(1, (cu[e + 1] - cu[e] + kC - 1) / kC); };      // an entry without tokens keeps its state: one empty chunk
+  int m = 0;
+  for (int e = tid; e < E; e += blockDim.x) m = max(m, chunks(e));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((tid & 31) == 0) most[tid >> 5] = m;
+  if (tid < 32) {
+    int base = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      int upto = e0 + tid < E ? chunks(e0 + tid) : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, upto, d);
+        if (tid >= d) upto += y;
+      }
+      if (e0 + tid < E) from[e0 + tid + 1] = base + upto;
+      base += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (tid == 0) from[0] = 0;
+  }
+  __syncthreads();
+  m = most[tid & 31];
+  const int total = from[E] * items, per = max(__reduce_max_sync(0xffffffffu, m), (total + blocks - 1) / blocks);
+  for (int q = tid; q < E * items; q += blockDim.x) {
+    const int e = q / items, k = q - e * items, n = from[e + 1] - from[e], s = from[e] * items + k * n, t0 = cu[e], t1 = cu[e + 1];
+    const int h = k / parts, cb0 = (k - h * parts) * 128, a = s / per, here = min(n, (a + 1) * per - s);      // chunks that lie in block a
+    l.segments[q + a] = DcSegment{t0 + (n - here) * kC, here, t1, h, cb0, e, here < n, 0};
+    if (s == a * per) l.first[a] = q + a;
+    if (s + n >= (a + 1) * per || q == E * items - 1) l.last[a] = q + a + 1;
+    if (here < n) {                                        // the rest, which is computed first
+      l.segments[q + a + 1] = DcSegment{t0, n - here, t1, h, cb0, e, 0, 1};
+      l.first[a + 1] = q + a + 1;
+      if (s + n >= (a + 2) * per || q == E * items - 1) l.last[a + 1] = q + a + 2;
+    }
+  }
+}
+
+// has the state been handed on (by a whole warp); false after some seconds
+NRL_DEVICE bool dc_handed(const int* flag) {
+  int ok = 0;
+  for (int n = 0; ok == 0 && n < (1 << 22); ++n) {
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(ok) : "l"(flag) : "memory");
+    if (ok == 0) __nanosleep(500);
+  }
+  return __all_sync(0xffffffffu, ok != 0);
+}
+
 struct DcParams {
   const float *qkv, *beta, *decay;
   float *state, *o;
   const int *cu, *start, *state_slot;
   long sq;
   int col_k, col_v, heads, kv_heads, D, Dv;
+  DcLine line;
 };
 
-template <int DP, bool DELTA, bool WIDE>      // DP: padded rows of S; WIDE: rows of q, k and v are 16-byte aligned
+NRL_DEVICE void mbar_inval(uint64_t* bar) { asm volatile("mbarrier.inval.shared.b64 [%0];" ::"r"(smem_u32(bar)) : "memory"); }
+
+// DP: padded rows of S; WIDE: rows of q, k and v are 16-byte aligned; LINE: a block takes its share of the line instead of an item
+template <int DP, bool DELTA, bool WIDE, bool LINE>
 __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcParams p) {
   using L = DcSmem<DP>;
   using Tm = DcTmem<DP>;
@@ -158,27 +233,28 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o2_full + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 20) {
-    if (lane == 0) {
-      for (int i = 0; i < 2; ++i) {
-        mbar_init(&kq_full[i], 128);
-        mbar_init(&kq_free[i], 1);
-        mbar_init(&lm_full[i], 128);
-        mbar_init(&sc_free[i], 512);
-        mbar_init(&raw_full[i], WIDE ? 32 : kDcLoaders);
-        mbar_init(&raw_free[i], 256);
-      }
-      for (int i = 0; i < 4; ++i) mbar_init(&sp_full[i], 256);
-      mbar_init(gram_full, 1);
-      mbar_init(gram_free, 128);
-      mbar_init(rk_full, 1);
-      mbar_init(rq_full, 1);
-      mbar_init(uh_full, 128);
-      mbar_init(u_full, 128);
-      mbar_init(ds_full, 1);
-      mbar_init(o2_full, 1);
-      fence_mbar_init();
+  auto init_barriers = [&]() {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&kq_full[i], 128);
+      mbar_init(&kq_free[i], 1);
+      mbar_init(&lm_full[i], 128);
+      mbar_init(&sc_free[i], 512);
+      mbar_init(&raw_full[i], WIDE ? 32 : kDcLoaders);
+      mbar_init(&raw_free[i], 256);
     }
+    for (int i = 0; i < 4; ++i) mbar_init(&sp_full[i], 256);
+    mbar_init(gram_full, 1);
+    mbar_init(gram_free, 128);
+    mbar_init(rk_full, 1);
+    mbar_init(rq_full, 1);
+    mbar_init(uh_full, 128);
+    mbar_init(u_full, 128);
+    mbar_init(ds_full, 1);
+    mbar_init(o2_full, 1);
+    fence_mbar_init();
+  };
+  if (warp == 20) {
+    if (lane == 0) init_barriers();
     __syncwarp();
     tmem_alloc(tmem_ptr, 512);
   }
@@ -187,193 +263,252 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
   tc_fence_after();
   const uint32_t tmem = *tmem_ptr;
 
-  const unsigned parts = (p.Dv + 127) / 128, eh = blockIdx.x / parts;
-  const int e = static_cast<int>(eh / p.heads), h = static_cast<int>(eh % p.heads), g = h / (p.heads / p.kv_heads);
-  const int cb0 = static_cast<int>(blockIdx.x % parts) * 128;
-  const int t0 = p.cu[e], n_chunks = (p.cu[e + 1] - t0 + kC - 1) / kC, t1 = p.cu[e + 1];
   const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  const int col = cb0 + (warp & 3) * 32 + lane;            // column of S of a thread of the solve and the state
+  const int line = gridDim.x - 1 - blockIdx.x;
+  const int first = LINE ? p.line.first[line] : 0, last = LINE ? p.line.last[line] : 1;      // segments of this block
+  int e, h, cb0, t0, n_chunks, t1;
+  auto take = [&](int i) {
+    if (LINE) {
+      const DcSegment& sg = p.line.segments[i];
+      e = sg.e; h = sg.h; cb0 = sg.cb0; t0 = sg.t0; n_chunks = sg.n; t1 = sg.t1;
+    } else {
+      const unsigned parts = (p.Dv + 127) / 128, eh = blockIdx.x / parts;
+      e = static_cast<int>(eh / p.heads);
+      h = static_cast<int>(eh % p.heads);
+      cb0 = static_cast<int>(blockIdx.x % parts) * 128;
+      t0 = p.cu[e];
+      t1 = p.cu[e + 1];
+      n_chunks = (t1 - t0 + kC - 1) / kC;
+    }
+  };
+  if (!LINE) take(0);
+  // between two segments: everybody has done with the barriers, then they start anew
+  auto turn = [&]() {
+    if (!LINE) return;
+    __syncwarp();
+    tc_fence_before();
+    named_barrier_sync(3, kDcThreads);
+    if (warp == 20 && lane == 0) {
+      for (uint64_t* b = kq_full; b <= o2_full; ++b) mbar_inval(b);
+      init_barriers();
+    }
+    named_barrier_sync(3, kDcThreads);
+    tc_fence_after();
+  };
 
   if (warp < 4) {
     // ============================== solve and outputs ==============================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
-    const bool mine = col < p.Dv;
-    for (int n = 0; n < n_chunks; ++n) {
-      const int st = n & 1, t = t0 + n * kC;
-      const uint32_t ph = n & 1, ph2 = (n >> 1) & 1;
-      const float* sc = reinterpret_cast<const float*>(smem + L::kSc + st * L::kScStage);
-      float u[kC], r[kC];
-      mbar_wait_quiet(&raw_full[st], ph2);
-      const float* v = reinterpret_cast<const float*>(smem + L::kRaw + st * L::kRawStage + L::kRawV) + (warp & 3) * 32 + lane;
+#pragma unroll 1
+    for (int i = first; i < last; ++i, turn()) {
+      if (LINE) take(i);
+      for (int n = 0; n < n_chunks; ++n) {
+        const int st = n & 1;
+        const uint32_t ph = n & 1, ph2 = (n >> 1) & 1;
+        const float* sc = reinterpret_cast<const float*>(smem + L::kSc + st * L::kScStage);
+        float u[kC], r[kC];
+        mbar_wait_quiet(&raw_full[st], ph2);
+        const float* v = reinterpret_cast<const float*>(smem + L::kRaw + st * L::kRawStage + L::kRawV) + (warp & 3) * 32 + lane;
 #pragma unroll
-      for (int i = 0; i < kC; ++i) u[i] = v[i * 128];
-      mbar_arrive(&raw_free[st]);
-      mbar_wait_quiet(&kq_full[st], ph2);
-      mbar_wait_quiet(rk_full, ph);
-      tc_fence_after();
-      auto read_rq = [&](int c, uint32_t (&a)[16]) {       // sixteen columns of S^T [K; Q]
-        tmem_ld_32x32b_x16(tmem + Tm::kR1 + c + lane_off, a);
-        uint32_t b[16];
-        tmem_ld_32x32b_x16(tmem + Tm::kR2 + c + lane_off, b);
-        tmem_ld_wait();
+        for (int i = 0; i < kC; ++i) u[i] = v[i * 128];
+        mbar_arrive(&raw_free[st]);
+        mbar_wait_quiet(&kq_full[st], ph2);
+        mbar_wait_quiet(rk_full, ph);
+        tc_fence_after();
+        auto read_rq = [&](int c, uint32_t (&a)[16]) {       // sixteen columns of S^T [K; Q]
+          tmem_ld_32x32b_x16(tmem + Tm::kR1 + c + lane_off, a);
+          uint32_t b[16];
+          tmem_ld_32x32b_x16(tmem + Tm::kR2 + c + lane_off, b);
+          tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) a[i] = __float_as_uint(__uint_as_float(a[i]) + __uint_as_float(b[i]));
-      };
-      if (DELTA) {
+          for (int i = 0; i < 16; ++i) a[i] = __float_as_uint(__uint_as_float(a[i]) + __uint_as_float(b[i]));
+        };
+        if (DELTA) {
+#pragma unroll
+          for (int c = 0; c < kC; c += 16) {
+            uint32_t x[16];
+            read_rq(c, x);
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 b4 = *reinterpret_cast<const float4*>(sc + c + i), c4 = *reinterpret_cast<const float4*>(sc + kC + c + i);
+              u[c + i] = b4.x * (u[c + i] - c4.x * __uint_as_float(x[i]));
+              u[c + i + 1] = b4.y * (u[c + i + 1] - c4.y * __uint_as_float(x[i + 1]));
+              u[c + i + 2] = b4.z * (u[c + i + 2] - c4.z * __uint_as_float(x[i + 2]));
+              u[c + i + 3] = b4.w * (u[c + i + 3] - c4.w * __uint_as_float(x[i + 3]));
+            }
+          }
+          mbar_wait_quiet(&lm_full[st], ph2);
+          const float* lj = reinterpret_cast<const float*>(smem + L::kL + st * L::kLStage);
+#pragma unroll
+          for (int i = 0; i < kC; ++i) r[i] = 0.f;           // a sum of its own: smaller than u, and so are its roundings
+#pragma unroll
+          for (int j = 0; j < kC; ++j) {
+            u[j] -= r[j];
+#pragma unroll
+            for (int i4 = (j + 1) / 4; i4 < kC / 4; ++i4) {
+              const float4 w = *reinterpret_cast<const float4*>(lj + j * kC + i4 * 4);
+              if (i4 * 4 + 0 > j) r[i4 * 4 + 0] = fmaf(w.x, u[j], r[i4 * 4 + 0]);
+              if (i4 * 4 + 1 > j) r[i4 * 4 + 1] = fmaf(w.y, u[j], r[i4 * 4 + 1]);
+              if (i4 * 4 + 2 > j) r[i4 * 4 + 2] = fmaf(w.z, u[j], r[i4 * 4 + 2]);
+              if (i4 * 4 + 3 > j) r[i4 * 4 + 3] = fmaf(w.w, u[j], r[i4 * 4 + 3]);
+            }
+          }
+        }
+        mbar_wait_quiet(rq_full, ph);                                // the terms of S, which U's go over, have been read
+        tc_fence_after();
+        // Terms of U: scaled for the state, then as they are for the outputs.  The products of a row of U reach tokens before u_j with a weight of
+        // zero: a value that is not finite would spoil them, so it is taken out in front of the second pass, and its token and all behind it
+        // are made NaN at the output.
+        int bad = kC;
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+          if (pass == 1) {
+            float probe = 0.f;
+#pragma unroll
+            for (int i = 0; i < kC; ++i) probe = fmaf(u[i], 0.f, probe);
+            if (probe != probe) {
+#pragma unroll
+              for (int i = kC - 1; i >= 0; --i)
+                if (!(fabsf(u[i]) < INFINITY)) {
+                  bad = i;
+                  u[i] = 0.f;
+                }
+            }
+          }
+          const float* ws = sc + (pass == 0 ? 2 : 4) * kC;   // G(n, .) or ones
+          const uint32_t to = tmem + lane_off + (pass == 0 ? Tm::uh(0) : Tm::kU), third = pass == 0 ? Tm::uh(2) - Tm::uh(0) : 32;
+#pragma unroll
+          for (int c = 0; c < kC; c += 16) {
+            uint32_t s0[8], s1[8], s2[8];
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 w = *reinterpret_cast<const float4*>(ws + c + i);
+              split3(w.x * u[c + i], w.y * u[c + i + 1], s0[i / 2], s1[i / 2], s2[i / 2]);
+              split3(w.z * u[c + i + 2], w.w * u[c + i + 3], s0[i / 2 + 1], s1[i / 2 + 1], s2[i / 2 + 1]);
+            }
+            tmem_st_32x32b_x8(to + c / 2, s0);
+            tmem_st_32x32b_x8(to + 16 + c / 2, s1);
+            tmem_st_32x32b_x8(to + third + c / 2, s2);
+          }
+          tmem_st_wait();
+          tc_fence_before();
+          if (pass == 0) mbar_arrive(uh_full);
+        }
 #pragma unroll
         for (int c = 0; c < kC; c += 16) {
           uint32_t x[16];
-          read_rq(c, x);
+          read_rq(kC + c, x);
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
-            const float4 b4 = *reinterpret_cast<const float4*>(sc + c + i), c4 = *reinterpret_cast<const float4*>(sc + kC + c + i);
-            u[c + i] = b4.x * (u[c + i] - c4.x * __uint_as_float(x[i]));
-            u[c + i + 1] = b4.y * (u[c + i + 1] - c4.y * __uint_as_float(x[i + 1]));
-            u[c + i + 2] = b4.z * (u[c + i + 2] - c4.z * __uint_as_float(x[i + 2]));
-            u[c + i + 3] = b4.w * (u[c + i + 3] - c4.w * __uint_as_float(x[i + 3]));
+            const float4 w = *reinterpret_cast<const float4*>(sc + kC + c + i);
+            r[c + i] = w.x * __uint_as_float(x[i]);
+            r[c + i + 1] = w.y * __uint_as_float(x[i + 1]);
+            r[c + i + 2] = w.z * __uint_as_float(x[i + 2]);
+            r[c + i + 3] = w.w * __uint_as_float(x[i + 3]);
           }
         }
-        mbar_wait_quiet(&lm_full[st], ph2);
-        const float* lj = reinterpret_cast<const float*>(smem + L::kL + st * L::kLStage);
-#pragma unroll
-        for (int i = 0; i < kC; ++i) r[i] = 0.f;           // a sum of its own: smaller than u, and so are its roundings
-#pragma unroll
-        for (int j = 0; j < kC; ++j) {
-          u[j] -= r[j];
-#pragma unroll
-          for (int i4 = (j + 1) / 4; i4 < kC / 4; ++i4) {
-            const float4 w = *reinterpret_cast<const float4*>(lj + j * kC + i4 * 4);
-            if (i4 * 4 + 0 > j) r[i4 * 4 + 0] = fmaf(w.x, u[j], r[i4 * 4 + 0]);
-            if (i4 * 4 + 1 > j) r[i4 * 4 + 1] = fmaf(w.y, u[j], r[i4 * 4 + 1]);
-            if (i4 * 4 + 2 > j) r[i4 * 4 + 2] = fmaf(w.z, u[j], r[i4 * 4 + 2]);
-            if (i4 * 4 + 3 > j) r[i4 * 4 + 3] = fmaf(w.w, u[j], r[i4 * 4 + 3]);
-          }
-        }
-      }
-      mbar_wait_quiet(rq_full, ph);                                // the terms of S, which U's go over, have been read
-      tc_fence_after();
-      // Terms of U: scaled for the state, then as they are for the outputs.  The products of a row of U reach tokens before u_j with a weight of
-      // zero: a value that is not finite would spoil them, so it is taken out in front of the second pass, and its token and all behind it
-      // are made NaN at the output.
-      int bad = kC;
-#pragma unroll 1
-      for (int pass = 0; pass < 2; ++pass) {
-        if (pass == 1) {
-          float probe = 0.f;
-#pragma unroll
-          for (int i = 0; i < kC; ++i) probe = fmaf(u[i], 0.f, probe);
-          if (probe != probe) {
-#pragma unroll
-            for (int i = kC - 1; i >= 0; --i)
-              if (!(fabsf(u[i]) < INFINITY)) {
-                bad = i;
-                u[i] = 0.f;
-              }
-          }
-        }
-        const float* ws = sc + (pass == 0 ? 2 : 4) * kC;   // G(n, .) or ones
-        const uint32_t to = tmem + lane_off + (pass == 0 ? Tm::uh(0) : Tm::kU), third = pass == 0 ? Tm::uh(2) - Tm::uh(0) : 32;
+        tc_fence_before();
+        mbar_arrive(u_full);
+        mbar_arrive(&sc_free[st]);
+        if (LINE) take(i);                                     // looked up in every chunk, not kept
+        const int t = t0 + n * kC, col = cb0 + (warp & 3) * 32 + lane;      // of S
+        mbar_wait_quiet(o2_full, ph);
+        tc_fence_after();
+        float* od = p.o + (static_cast<long>(t) * p.heads + h) * p.Dv + col;
+        const int left = col < p.Dv ? t1 - t : 0;
 #pragma unroll
         for (int c = 0; c < kC; c += 16) {
-          uint32_t s0[8], s1[8], s2[8];
+          uint32_t x[16];
+          tmem_ld_32x32b_x16(tmem + Tm::kO2 + c + lane_off, x);
+          tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            const float4 w = *reinterpret_cast<const float4*>(ws + c + i);
-            split3(w.x * u[c + i], w.y * u[c + i + 1], s0[i / 2], s1[i / 2], s2[i / 2]);
-            split3(w.z * u[c + i + 2], w.w * u[c + i + 3], s0[i / 2 + 1], s1[i / 2 + 1], s2[i / 2 + 1]);
+          for (int i = 0; i < 16; ++i) {
+            if (c + i < left) *od = c + i >= bad ? NAN : r[c + i] + __uint_as_float(x[i]);
+            od += static_cast<long>(p.heads) * p.Dv;
           }
-          tmem_st_32x32b_x8(to + c / 2, s0);
-          tmem_st_32x32b_x8(to + 16 + c / 2, s1);
-          tmem_st_32x32b_x8(to + third + c / 2, s2);
         }
-        tmem_st_wait();
         tc_fence_before();
-        if (pass == 0) mbar_arrive(uh_full);
       }
-#pragma unroll
-      for (int c = 0; c < kC; c += 16) {
-        uint32_t x[16];
-        read_rq(kC + c, x);
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-          const float4 w = *reinterpret_cast<const float4*>(sc + kC + c + i);
-          r[c + i] = w.x * __uint_as_float(x[i]);
-          r[c + i + 1] = w.y * __uint_as_float(x[i + 1]);
-          r[c + i + 2] = w.z * __uint_as_float(x[i + 2]);
-          r[c + i + 3] = w.w * __uint_as_float(x[i + 3]);
-        }
-      }
-      tc_fence_before();
-      mbar_arrive(u_full);
-      mbar_arrive(&sc_free[st]);
-      mbar_wait_quiet(o2_full, ph);
-      tc_fence_after();
-      float* od = p.o + (static_cast<long>(t) * p.heads + h) * p.Dv + col;
-      const int left = mine ? t1 - t : 0;
-#pragma unroll
-      for (int c = 0; c < kC; c += 16) {
-        uint32_t x[16];
-        tmem_ld_32x32b_x16(tmem + Tm::kO2 + c + lane_off, x);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          if (c + i < left) *od = c + i >= bad ? NAN : r[c + i] + __uint_as_float(x[i]);
-          od += static_cast<long>(p.heads) * p.Dv;
-        }
-      }
-      tc_fence_before();
     }
   } else if (warp < 12) {
     // ============================== state ==============================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     const int half = (warp - 4) >> 2;
-    if (half < NH) {
-      float* gS = p.state + ((static_cast<long>(p.state_slot[e]) * p.heads + h) * p.D + half * 64) * p.Dv + col;
-      const int rows = col < p.Dv ? p.D - half * 64 : 0, from = p.start[e] > 0 ? rows : 0;      // rows of S here, rows that are carried
-      float S[64];
-      const float* ld = gS;
+#pragma unroll 1
+    for (int i = first; i < last; ++i, turn()) {
+      if (LINE) take(i);
+      if (half < NH) {
+        const int col = cb0 + (warp & 3) * 32 + lane;
+        float* gS = p.state + ((static_cast<long>(p.state_slot[e]) * p.heads + h) * p.D + half * 64) * p.Dv + col;
+        int rows = col < p.Dv ? p.D - half * 64 : 0;                                              // rows of S here
+        int from = p.start[e] > 0 ? rows : 0;                                                     // rows that are carried
+        float S[64];
+        const float* ld = gS;
+        long step = p.Dv;
+        bool there = true;
+        if (LINE && p.line.segments[i].in) {
+          there = dc_handed(p.line.handed + line + 1);
+          ld = p.line.carry + (static_cast<long>(line + 1) * 128 + half * 64) * 128 + (warp & 3) * 32 + lane;
+          step = 128;
+          from = rows;
+        }
 #pragma unroll
-      for (int d = 0; d < 64; ++d, ld += p.Dv) S[d] = d < from ? *ld : 0.f;
-      const uint32_t base = tmem + Tm::kHalf * half + lane_off;
-      for (int n = 0; n < n_chunks; ++n) {
+        for (int d = 0; d < 64; ++d, ld += step) S[d] = d < from ? __ldcg(ld) : 0.f;
+        if (!there) S[0] = NAN;
+        const uint32_t base = tmem + Tm::kHalf * half + lane_off;
+        for (int n = 0; n < n_chunks; ++n) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t s0[8], s1[8], s2[8];
+          for (int c = 0; c < 4; ++c) {
+            uint32_t s0[8], s1[8], s2[8];
 #pragma unroll
-          for (int i = 0; i < 16; i += 2) split3(S[c * 16 + i], S[c * 16 + i + 1], s0[i / 2], s1[i / 2], s2[i / 2]);
-          tmem_st_32x32b_x8(base + c * 8, s0);
-          tmem_st_32x32b_x8(base + 32 + c * 8, s1);
-          tmem_st_32x32b_x8(base + 64 + c * 8, s2);
-          tmem_st_wait();
+            for (int i = 0; i < 16; i += 2) split3(S[c * 16 + i], S[c * 16 + i + 1], s0[i / 2], s1[i / 2], s2[i / 2]);
+            tmem_st_32x32b_x8(base + c * 8, s0);
+            tmem_st_32x32b_x8(base + 32 + c * 8, s1);
+            tmem_st_32x32b_x8(base + 64 + c * 8, s2);
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(&sp_full[c]);
+          }
+          mbar_wait_quiet(&kq_full[n & 1], (n >> 1) & 1);
+          const float c_n = reinterpret_cast<const float*>(smem + L::kSc + (n & 1) * L::kScStage)[2 * kC - 1];
+          mbar_arrive(&sc_free[n & 1]);
+          mbar_wait_quiet(ds_full, n & 1);
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t x[16];
+            tmem_ld_32x32b_x16(base + c * 16, x);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) S[c * 16 + i] = fmaf(c_n, S[c * 16 + i], __uint_as_float(x[i]));
+          }
           tc_fence_before();
-          mbar_arrive(&sp_full[c]);
         }
-        mbar_wait_quiet(&kq_full[n & 1], (n >> 1) & 1);
-        const float c_n = reinterpret_cast<const float*>(smem + L::kSc + (n & 1) * L::kScStage)[2 * kC - 1];
-        mbar_arrive(&sc_free[n & 1]);
-        mbar_wait_quiet(ds_full, n & 1);
-        tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t x[16];
-          tmem_ld_32x32b_x16(base + c * 16, x);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) S[c * 16 + i] = fmaf(c_n, S[c * 16 + i], __uint_as_float(x[i]));
+        step = p.Dv;
+        const bool out = LINE && p.line.segments[i].out;
+        if (LINE) {                                          // the segment is looked up again: nothing of it is kept over the loop
+          take(i);
+          rows = cb0 + (warp & 3) * 32 + lane < p.Dv ? p.D - half * 64 : 0;
+          gS = out ? p.line.carry + (static_cast<long>(line) * 128 + half * 64) * 128 + (warp & 3) * 32 + lane
+                   : p.state + ((static_cast<long>(p.state_slot[e]) * p.heads + h) * p.D + half * 64) * p.Dv + cb0 + (warp & 3) * 32 + lane;
+          if (out) step = 128;
         }
-        tc_fence_before();
-      }
-      long step = p.Dv;
-      asm volatile("" : "+l"(gS), "+l"(step));             // the addresses are not kept from the load to here: 128 registers
+        asm volatile("" : "+l"(gS), "+l"(step));             // the addresses are not kept from the load to here: 128 registers
 #pragma unroll
-      for (int d = 0; d < 64; ++d, gS += step)
-        if (d < rows) *gS = S[d];
-    } else {
-      for (int n = 0; n < n_chunks; ++n) {
-        for (int c = 0; c < 4; ++c) mbar_arrive(&sp_full[c]);
-        mbar_wait_quiet(&kq_full[n & 1], (n >> 1) & 1);
-        mbar_arrive(&sc_free[n & 1]);
-        mbar_wait_quiet(ds_full, n & 1);
+        for (int d = 0; d < 64; ++d, gS += step)
+          if (d < rows) *gS = S[d];
+        if (out) {
+          __threadfence();
+          named_barrier_sync(2, NH * 128);
+          if (threadIdx.x == 4 * 32) asm volatile("st.release.gpu.global.b32 [%0], 1;" ::"l"(p.line.handed + line) : "memory");
+        }
+      } else {
+        for (int n = 0; n < n_chunks; ++n) {
+          for (int c = 0; c < 4; ++c) mbar_arrive(&sp_full[c]);
+          mbar_wait_quiet(&kq_full[n & 1], (n >> 1) & 1);
+          mbar_arrive(&sc_free[n & 1]);
+          mbar_wait_quiet(ds_full, n & 1);
+        }
       }
     }
   } else if (warp < 16) {
@@ -392,55 +527,59 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         gd = p.decay[static_cast<long>(t + tid) * p.heads + h];
       }
     };
-    fetch_sc(t0);
-    for (int n = 0; n < n_chunks; ++n) {
-      const int st = n & 1, t = t0 + n * kC;
-      const uint32_t ph2 = (n >> 1) & 1;
-      float2 c = make_float2(gd, 0.f), w = make_float2(1.f, 0.f);      // g_1 .. g_i and g_{i+1} .. g_n
-      if (warp == 12) {
-        w.x = __shfl_down_sync(0xffffffffu, gd, 1);
-        if (lane == 31) w.x = 1.f;
 #pragma unroll 1
-        for (int m = 1; m < 32; m <<= 1) {
-          const float2 a = make_float2(__shfl_up_sync(0xffffffffu, c.x, m), __shfl_up_sync(0xffffffffu, c.y, m));
-          const float2 b = make_float2(__shfl_down_sync(0xffffffffu, w.x, m), __shfl_down_sync(0xffffffffu, w.y, m));
-          if (lane >= m) c = mul_wide(c, a);
-          if (lane + m < 32) w = mul_wide(w, b);
+    for (int i = first; i < last; ++i, turn()) {
+      if (LINE) take(i);
+      fetch_sc(t0);
+      for (int n = 0; n < n_chunks; ++n) {
+        const int st = n & 1, t = t0 + n * kC;
+        const uint32_t ph2 = (n >> 1) & 1;
+        float2 c = make_float2(gd, 0.f), w = make_float2(1.f, 0.f);      // g_1 .. g_i and g_{i+1} .. g_n
+        if (warp == 12) {
+          w.x = __shfl_down_sync(0xffffffffu, gd, 1);
+          if (lane == 31) w.x = 1.f;
+#pragma unroll 1
+          for (int m = 1; m < 32; m <<= 1) {
+            const float2 a = make_float2(__shfl_up_sync(0xffffffffu, c.x, m), __shfl_up_sync(0xffffffffu, c.y, m));
+            const float2 b = make_float2(__shfl_down_sync(0xffffffffu, w.x, m), __shfl_down_sync(0xffffffffu, w.y, m));
+            if (lane >= m) c = mul_wide(c, a);
+            if (lane + m < 32) w = mul_wide(w, b);
+          }
         }
-      }
-      mbar_wait_quiet(&kq_free[st], ph2 ^ 1);
-      mbar_wait_quiet(&sc_free[st], ph2 ^ 1);
-      if (warp == 12) {
-        float* sc = reinterpret_cast<float*>(smem + L::kSc + st * L::kScStage);
-        sc[lane] = beta;
-        sc[kC + lane] = c.x + c.y;
-        sc[2 * kC + lane] = w.x + w.y;
-        sc[3 * kC + lane] = gd;
-        sc[4 * kC + lane] = 1.f;
-      }
-      fetch_sc(t + kC);
-      mbar_wait_quiet(&raw_full[st], ph2);
-      uint8_t* tile = smem + L::kKQ + st * L::kKQStage;
-      const float* raw = reinterpret_cast<const float*>(smem + L::kRaw + st * L::kRawStage);
+        mbar_wait_quiet(&kq_free[st], ph2 ^ 1);
+        mbar_wait_quiet(&sc_free[st], ph2 ^ 1);
+        if (warp == 12) {
+          float* sc = reinterpret_cast<float*>(smem + L::kSc + st * L::kScStage);
+          sc[lane] = beta;
+          sc[kC + lane] = c.x + c.y;
+          sc[2 * kC + lane] = w.x + w.y;
+          sc[3 * kC + lane] = gd;
+          sc[4 * kC + lane] = 1.f;
+        }
+        fetch_sc(t + kC);
+        mbar_wait_quiet(&raw_full[st], ph2);
+        uint8_t* tile = smem + L::kKQ + st * L::kKQStage;
+        const float* raw = reinterpret_cast<const float*>(smem + L::kRaw + st * L::kRawStage);
 #pragma unroll 1
-      for (int s = 0; s < NR; ++s)
+        for (int s = 0; s < NR; ++s)
 #pragma unroll 1
-        for (int q = 0; q < 2; ++q) {
-          const int row = s * RW + r0, d = d0 + q * (DP / 2), chunk = (d & 63) >> 3;
-          const float4 a = *reinterpret_cast<const float4*>(raw + row * DP + d), b = *reinterpret_cast<const float4*>(raw + row * DP + d + 4);
-          uint32_t y[3][4];
-          split3(a.x, a.y, y[0][0], y[1][0], y[2][0]);
-          split3(a.z, a.w, y[0][1], y[1][1], y[2][1]);
-          split3(b.x, b.y, y[0][2], y[1][2], y[2][2]);
-          split3(b.z, b.w, y[0][3], y[1][3], y[2][3]);
+          for (int q = 0; q < 2; ++q) {
+            const int row = s * RW + r0, d = d0 + q * (DP / 2), chunk = (d & 63) >> 3;
+            const float4 a = *reinterpret_cast<const float4*>(raw + row * DP + d), b = *reinterpret_cast<const float4*>(raw + row * DP + d + 4);
+            uint32_t y[3][4];
+            split3(a.x, a.y, y[0][0], y[1][0], y[2][0]);
+            split3(a.z, a.w, y[0][1], y[1][1], y[2][1]);
+            split3(b.x, b.y, y[0][2], y[1][2], y[2][2]);
+            split3(b.z, b.w, y[0][3], y[1][3], y[2][3]);
 #pragma unroll
-          for (int m = 0; m < 3; ++m)
-            *reinterpret_cast<uint4*>(tile + (m * NH + (d >> 6)) * kDcTile + row * 128 + ((chunk ^ (row & 7)) << 4)) =
-                make_uint4(y[m][0], y[m][1], y[m][2], y[m][3]);
-        }
-      mbar_arrive(&raw_free[st]);
-      fence_proxy_async_smem();
-      mbar_arrive(&kq_full[st]);
+            for (int m = 0; m < 3; ++m)
+              *reinterpret_cast<uint4*>(tile + (m * NH + (d >> 6)) * kDcTile + row * 128 + ((chunk ^ (row & 7)) << 4)) =
+                  make_uint4(y[m][0], y[m][1], y[m][2], y[m][3]);
+          }
+        mbar_arrive(&raw_free[st]);
+        fence_proxy_async_smem();
+        mbar_arrive(&kq_full[st]);
+      }
     }
   } else if (warp < 20) {
     // ============================== Gram matrices ==============================
@@ -448,108 +587,116 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
     // rows of this thread: those of a 64-row accumulator are sixteen lanes of each warp's quarter
     const int gi = ((warp & 3) * 16 + (lane & 15)) & (kC - 1);
     const bool is_q = (warp & 3) >= 2, have = lane < 16;
-    for (int n = 0; n < n_chunks; ++n) {
-      const int st = n & 1;
-      const uint32_t ph2 = (n >> 1) & 1;
-      mbar_wait_quiet(&kq_full[st], ph2);
-      mbar_wait_quiet(&kq_free[st], ph2 ^ 1);                      // the products that read the stage's Gram matrices
-      const float* sc = reinterpret_cast<const float*>(smem + L::kSc + st * L::kScStage);
-      const float bi = is_q ? 1.f : sc[gi];
-      float2 w = make_float2(1.f, 0.f);                    // G(gi, j)
-      mbar_wait_quiet(gram_full, n & 1);
-      tc_fence_after();
-      uint8_t* mt = smem + L::kM + st * L::kMStage;
-      float* lj = reinterpret_cast<float*>(smem + L::kL + st * L::kLStage);
 #pragma unroll 1
-      for (int c = kC - 8; c >= 0; c -= 8) {
-        uint32_t ga[8], gb[8];
-        tmem_ld_32x32b_x8(tmem + Tm::kG1 + c + lane_off, ga);
-        tmem_ld_32x32b_x8(tmem + Tm::kG2 + c + lane_off, gb);
-        float m[8];
+    for (int i = first; i < last; ++i, turn()) {
+      if (LINE) take(i);
+      for (int n = 0; n < n_chunks; ++n) {
+        const int st = n & 1;
+        const uint32_t ph2 = (n >> 1) & 1;
+        mbar_wait_quiet(&kq_full[st], ph2);
+        mbar_wait_quiet(&kq_free[st], ph2 ^ 1);                      // the products that read the stage's Gram matrices
+        const float* sc = reinterpret_cast<const float*>(smem + L::kSc + st * L::kScStage);
+        const float bi = is_q ? 1.f : sc[gi];
+        float2 w = make_float2(1.f, 0.f);                    // G(gi, j)
+        mbar_wait_quiet(gram_full, n & 1);
+        tc_fence_after();
+        uint8_t* mt = smem + L::kM + st * L::kMStage;
+        float* lj = reinterpret_cast<float*>(smem + L::kL + st * L::kLStage);
+#pragma unroll 1
+        for (int c = kC - 8; c >= 0; c -= 8) {
+          uint32_t ga[8], gb[8];
+          tmem_ld_32x32b_x8(tmem + Tm::kG1 + c + lane_off, ga);
+          tmem_ld_32x32b_x8(tmem + Tm::kG2 + c + lane_off, gb);
+          float m[8];
 #pragma unroll
-        for (int a = 7; a >= 0; --a) {
-          const int j = c + a;
-          const float gj = j < gi ? sc[3 * kC + j + 1] : 1.f;
-          w = mul_wide(w, make_float2(gj, 0.f));
-          m[a] = bi * (w.x + w.y);
-        }
-        tmem_ld_wait();
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-          m[a] = c + a < gi || (is_q && c + a == gi) ? m[a] * (__uint_as_float(ga[a]) + __uint_as_float(gb[a])) : 0.f;
-        if (have && is_q) {
-          uint32_t y[3][4];
-#pragma unroll
-          for (int a = 0; a < 8; a += 2) split3(m[a], m[a + 1], y[0][a / 2], y[1][a / 2], y[2][a / 2]);
-#pragma unroll
-          for (int b = 0; b < 3; ++b) {
-            const int chunk = (b == 1 ? 4 : 0) + c / 8;
-            *reinterpret_cast<uint4*>(mt + (b == 2 ? kC * 128 : 0) + gi * 128 + ((chunk ^ (gi & 7)) << 4)) =
-                make_uint4(y[b][0], y[b][1], y[b][2], y[b][3]);
+          for (int a = 7; a >= 0; --a) {
+            const int j = c + a;
+            const float gj = j < gi ? sc[3 * kC + j + 1] : 1.f;
+            w = mul_wide(w, make_float2(gj, 0.f));
+            m[a] = bi * (w.x + w.y);
           }
-        } else if (have && DELTA) {
+          tmem_ld_wait();
 #pragma unroll
-          for (int a = 0; a < 8; ++a) lj[(c + a) * kC + gi] = m[a];
+          for (int a = 0; a < 8; ++a)
+            m[a] = c + a < gi || (is_q && c + a == gi) ? m[a] * (__uint_as_float(ga[a]) + __uint_as_float(gb[a])) : 0.f;
+          if (have && is_q) {
+            uint32_t y[3][4];
+#pragma unroll
+            for (int a = 0; a < 8; a += 2) split3(m[a], m[a + 1], y[0][a / 2], y[1][a / 2], y[2][a / 2]);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+              const int chunk = (b == 1 ? 4 : 0) + c / 8;
+              *reinterpret_cast<uint4*>(mt + (b == 2 ? kC * 128 : 0) + gi * 128 + ((chunk ^ (gi & 7)) << 4)) =
+                  make_uint4(y[b][0], y[b][1], y[b][2], y[b][3]);
+            }
+          } else if (have && DELTA) {
+#pragma unroll
+            for (int a = 0; a < 8; ++a) lj[(c + a) * kC + gi] = m[a];
+          }
         }
+        tc_fence_before();
+        mbar_arrive(gram_free);
+        mbar_arrive(&sc_free[st]);
+        fence_proxy_async_smem();
+        mbar_arrive(&lm_full[st]);
       }
-      tc_fence_before();
-      mbar_arrive(gram_free);
-      mbar_arrive(&sc_free[st]);
-      fence_proxy_async_smem();
-      mbar_arrive(&lm_full[st]);
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp > 20) {
       // ============================== q, k and v ==============================
       const int tid = threadIdx.x - 21 * 32;
-      const float* src = p.qkv + static_cast<long>(g) * p.D;
-      const float* vsrc = p.qkv + p.col_v + static_cast<long>(h) * p.Dv + cb0;
-      const int vcols = min(p.Dv - cb0, 128);
       if (WIDE) {
         float* all = reinterpret_cast<float*>(smem + L::kRaw);
-        if (p.D < DP || vcols < 128)                        // columns that no copy reaches
+        if (p.D < DP || p.Dv % 128 != 0)                    // columns that no copy reaches
           for (int x = tid; x < 2 * L::kRawStage / 4; x += kDcLoaders) all[x] = 0.f;
         fence_proxy_async_smem();                           // the zeros lie under what the copies bring: in front of them for the asynchronous proxy too
         named_barrier_sync(1, kDcLoaders);
       }
-      for (int n = 0; n < n_chunks && (!WIDE || warp == 21); ++n) {
-        const int st = n & 1, t = t0 + n * kC;
-        mbar_wait_quiet(&raw_free[st], ((n >> 1) & 1) ^ 1);
-        float* raw = reinterpret_cast<float*>(smem + L::kRaw + st * L::kRawStage);
-        float* rv = reinterpret_cast<float*>(smem + L::kRaw + st * L::kRawStage + L::kRawV);
-        if (WIDE) {                                         // a lane per token
-          if (t + lane < t1) {
-            const long row = static_cast<long>(t + lane) * p.sq;
-            mbar_arrive_expect_tx(&raw_full[st], (2 * p.D + vcols) * 4);
-            bulk_load(raw + lane * DP, src + p.col_k + row, p.D * 4, &raw_full[st]);
-            bulk_load(raw + (kC + lane) * DP, src + row, p.D * 4, &raw_full[st]);
-            bulk_load(rv + lane * 128, vsrc + row, vcols * 4, &raw_full[st]);
-          } else {
-            for (int d = 0; d < DP; d += 4) {
-              *reinterpret_cast<float4*>(raw + lane * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
-              *reinterpret_cast<float4*>(raw + (kC + lane) * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+      for (int i = first; i < last; ++i, turn()) {
+        if (LINE) take(i);
+        const float* src = p.qkv + static_cast<long>(h / (p.heads / p.kv_heads)) * p.D;
+        const float* vsrc = p.qkv + p.col_v + static_cast<long>(h) * p.Dv + cb0;
+        const int vcols = min(p.Dv - cb0, 128);
+        for (int n = 0; n < n_chunks && (!WIDE || warp == 21); ++n) {
+          const int st = n & 1, t = t0 + n * kC;
+          mbar_wait_quiet(&raw_free[st], ((n >> 1) & 1) ^ 1);
+          float* raw = reinterpret_cast<float*>(smem + L::kRaw + st * L::kRawStage);
+          float* rv = reinterpret_cast<float*>(smem + L::kRaw + st * L::kRawStage + L::kRawV);
+          if (WIDE) {                                         // a lane per token
+            if (t + lane < t1) {
+              const long row = static_cast<long>(t + lane) * p.sq;
+              mbar_arrive_expect_tx(&raw_full[st], (2 * p.D + vcols) * 4);
+              bulk_load(raw + lane * DP, src + p.col_k + row, p.D * 4, &raw_full[st]);
+              bulk_load(raw + (kC + lane) * DP, src + row, p.D * 4, &raw_full[st]);
+              bulk_load(rv + lane * 128, vsrc + row, vcols * 4, &raw_full[st]);
+            } else {
+              for (int d = 0; d < DP; d += 4) {
+                *reinterpret_cast<float4*>(raw + lane * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(raw + (kC + lane) * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+              }
+              for (int c = 0; c < 128; c += 4) *reinterpret_cast<float4*>(rv + lane * 128 + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+              mbar_arrive(&raw_full[st]);
             }
-            for (int c = 0; c < 128; c += 4) *reinterpret_cast<float4*>(rv + lane * 128 + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-            mbar_arrive(&raw_full[st]);
-          }
-        } else {
+          } else {
 #pragma unroll 1
-          for (int x = tid; x < 2 * kC * DP; x += kDcLoaders) {              // rows 0..31 are K, 32..63 Q
-            const int row = x / DP, d = x % DP, i = row & (kC - 1);
-            const bool ok = t + i < t1 && d < p.D;
-            cp_async_zfill(raw + row * DP + d, ok ? src + static_cast<long>(t + i) * p.sq + (row < kC ? p.col_k : 0) + d : p.qkv, ok);
-          }
+            for (int x = tid; x < 2 * kC * DP; x += kDcLoaders) {              // rows 0..31 are K, 32..63 Q
+              const int row = x / DP, d = x % DP, i = row & (kC - 1);
+              const bool ok = t + i < t1 && d < p.D;
+              cp_async_zfill(raw + row * DP + d, ok ? src + static_cast<long>(t + i) * p.sq + (row < kC ? p.col_k : 0) + d : p.qkv, ok);
+            }
 #pragma unroll 1
-          for (int x = tid; x < kC * 128; x += kDcLoaders) {
-            const int i = x / 128, c = x % 128;
-            const bool ok = t + i < t1 && c < vcols;
-            cp_async_zfill(rv + i * 128 + c, ok ? vsrc + static_cast<long>(t + i) * p.sq + c : p.qkv, ok);
+            for (int x = tid; x < kC * 128; x += kDcLoaders) {
+              const int i = x / 128, c = x % 128;
+              const bool ok = t + i < t1 && c < vcols;
+              cp_async_zfill(rv + i * 128 + c, ok ? vsrc + static_cast<long>(t + i) * p.sq + c : p.qkv, ok);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[st])) : "memory");
           }
-          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[st])) : "memory");
         }
       }
-    } else if (n_chunks > 0) {
+    } else {
       // ============================== MMA issuer ==============================
       // the whole warp runs the loops, one lane issues: what is the same in all lanes stays in uniform registers
       const uint32_t leader = elect_one(), tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
@@ -576,56 +723,63 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         }
         dc_commit(leader, gram_full);
       };
-      gram(0);
 #pragma unroll 1
-      for (int n = 0; n < n_chunks; ++n) {
-        const int st = n & 1;
-        const uint64_t d = kq0 + st * (L::kKQStage / 16), dt = kt0 + st * (L::kKQStage / 16), dm = m0 + st * (L::kMStage / 16);
-        auto rq = [&](int pr, int k, int kq, bool second, bool first) {      // kq: 0 K, 1 Q, 32 rows further and 32 columns
-          dc_mma_ts(leader, tmem_u + (second ? Tm::kR2 : Tm::kR1) + kq * kC, tmem_u + Tm::kHalf * (k >> 2) + 32 * pair_a(pr) + 8 * (k & 3),
-                      d + pair_b(pr) * kTerm + (k >> 2) * kHalfTile + (k & 3) * kStep + kq * (kC * 8), id_rq, first ? 0u : 1u);
-        };
-        // K, which the solve waits for: the small pairs as the terms come
+      for (int i = first; i < last; ++i, turn()) {
+        if (LINE) take(i);
+        if (n_chunks > 0) gram(0);
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          mbar_wait_quiet(&sp_full[c], n & 1);
-          tc_fence_after();
-#pragma unroll
-          for (int pr = 0; pr < 5; ++pr)
-#pragma unroll
-            for (int hf = 0; hf < NH; ++hf) rq(pr, 4 * hf + c, 0, false, c == 0 && pr == 0 && hf == 0);
-        }
-#pragma unroll
-        for (int k = 0; k < 4 * NH; ++k) rq(5, k, 0, k >= 2 * NH, k == 2 * NH);
-        dc_commit(leader, rk_full);
+        for (int n = 0; n < n_chunks; ++n) {
+          const int st = n & 1;
+          const uint64_t d = kq0 + st * (L::kKQStage / 16), dt = kt0 + st * (L::kKQStage / 16), dm = m0 + st * (L::kMStage / 16);
+          auto rq = [&](int pr, int k, int kq, bool second, bool first) {      // kq: 0 K, 1 Q, 32 rows further and 32 columns
+            dc_mma_ts(leader, tmem_u + (second ? Tm::kR2 : Tm::kR1) + kq * kC, tmem_u + Tm::kHalf * (k >> 2) + 32 * pair_a(pr) + 8 * (k & 3),
+                        d + pair_b(pr) * kTerm + (k >> 2) * kHalfTile + (k & 3) * kStep + kq * (kC * 8), id_rq, first ? 0u : 1u);
+          };
+          // K, which the solve waits for: the small pairs as the terms come
 #pragma unroll 1
-        for (int pr = 0; pr < 6; ++pr)
+          for (int c = 0; c < 4; ++c) {
+            mbar_wait_quiet(&sp_full[c], n & 1);
+            tc_fence_after();
 #pragma unroll
-          for (int k = 0; k < 4 * NH; ++k) rq(pr, k, 1, pr == 5 && k >= 2 * NH, (pr == 0 && k == 0) || (pr == 5 && k == 2 * NH));
-        dc_commit(leader, rq_full);
-        if (n + 1 < n_chunks) gram(n + 1);
-        mbar_wait_quiet(uh_full, n & 1);
-        tc_fence_after();
+            for (int pr = 0; pr < 5; ++pr)
 #pragma unroll
-        for (int hf = 0; hf < NH; ++hf)
+              for (int hf = 0; hf < NH; ++hf) rq(pr, 4 * hf + c, 0, false, c == 0 && pr == 0 && hf == 0);
+          }
 #pragma unroll
+          for (int k = 0; k < 4 * NH; ++k) rq(5, k, 0, k >= 2 * NH, k == 2 * NH);
+          dc_commit(leader, rk_full);
+#pragma unroll 1
           for (int pr = 0; pr < 6; ++pr)
 #pragma unroll
-            for (int k = 0; k < kC / 16; ++k)               // 16 tokens: 16 rows of 128 bytes
-              dc_mma_ts(leader, tmem_u + Tm::kHalf * hf, tmem_u + Tm::uh(pair_a(pr)) + 8 * k, dt + pair_b(pr) * kTerm + hf * kHalfTile + k * 128, id_ds,
-                          pr == 0 && k == 0 ? 0u : 1u);
-        dc_commit(leader, ds_full);
-        mbar_wait_quiet(u_full, n & 1);
-        mbar_wait_quiet(&lm_full[st], (n >> 1) & 1);
-        tc_fence_after();
-#pragma unroll 1
-        for (int pr = 0; pr < 6; ++pr)
+            for (int k = 0; k < 4 * NH; ++k) rq(pr, k, 1, pr == 5 && k >= 2 * NH, (pr == 0 && k == 0) || (pr == 5 && k == 2 * NH));
+          dc_commit(leader, rq_full);
+          if (n + 1 < n_chunks) gram(n + 1);
+          mbar_wait_quiet(uh_full, n & 1);
+          tc_fence_after();
 #pragma unroll
-          for (int k = 0; k < kC / 16; ++k)                 // terms 0 and 1 side by side, 2 in a tile of its own
-            dc_mma_ts(leader, tmem_u + Tm::kO2, tmem_u + Tm::kU + 16 * pair_a(pr) + 8 * k,
-                        dm + (pair_b(pr) == 2 ? kC * 128 / 16 : pair_b(pr) * 4) + k * kStep, id_o2, pr == 0 && k == 0 ? 0u : 1u);
-        dc_commit(leader, o2_full);
-        dc_commit(leader, &kq_free[st]);
+          for (int hf = 0; hf < NH; ++hf)
+#pragma unroll
+            for (int pr = 0; pr < 6; ++pr)
+#pragma unroll
+              for (int k = 0; k < kC / 16; ++k)               // 16 tokens: 16 rows of 128 bytes
+                dc_mma_ts(leader, tmem_u + Tm::kHalf * hf, tmem_u + Tm::uh(pair_a(pr)) + 8 * k, dt + pair_b(pr) * kTerm + hf * kHalfTile + k * 128, id_ds,
+                            pr == 0 && k == 0 ? 0u : 1u);
+          dc_commit(leader, ds_full);
+          mbar_wait_quiet(u_full, n & 1);
+          mbar_wait_quiet(&lm_full[st], (n >> 1) & 1);
+          tc_fence_after();
+#pragma unroll 1
+          for (int pr = 0; pr < 6; ++pr)
+#pragma unroll
+            for (int k = 0; k < kC / 16; ++k)                 // terms 0 and 1 side by side, 2 in a tile of its own
+              dc_mma_ts(leader, tmem_u + Tm::kO2, tmem_u + Tm::kU + 16 * pair_a(pr) + 8 * k,
+                          dm + (pair_b(pr) == 2 ? kC * 128 / 16 : pair_b(pr) * 4) + k * kStep, id_o2, pr == 0 && k == 0 ? 0u : 1u);
+          dc_commit(leader, o2_full);
+          dc_commit(leader, &kq_free[st]);
+        }
+        // nothing that is still under way arrives at a barrier that starts anew
+        if (LINE)
+          for (int n = max(0, n_chunks - 2); n < n_chunks; ++n) mbar_wait_quiet(&kq_free[n & 1], (n >> 1) & 1);
       }
     }
   }
@@ -638,9 +792,9 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
   }
 }
 
-template <int DP, bool DELTA, bool WIDE>
+template <int DP, bool DELTA, bool WIDE, bool LINE>
 cudaError_t launch_delta_chunk(unsigned grid, const DcParams& p, cudaStream_t s) {
-  auto kern = delta_chunk_tc_kernel<DP, DELTA, WIDE>;
+  auto kern = delta_chunk_tc_kernel<DP, DELTA, WIDE, LINE>;
   constexpr int smem = DcSmem<DP>::kTotal;
   static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (configured != cudaSuccess) return configured;
@@ -651,15 +805,31 @@ cudaError_t launch_delta_chunk(unsigned grid, const DcParams& p, cudaStream_t s)
 }  // namespace
 }  // namespace nrl
 
-// D <= 128, one decay per head; beta == nullptr: plain accumulation; rows16: rows of q, k and v start and end on 16-byte boundaries
+// D <= 128, one decay per head; beta == nullptr: plain accumulation; rows16: rows of q, k and v start and end on 16-byte boundaries; line: null, or (rows16)
+// nrl_delta_line_bytes() of scratch with which `blocks` blocks share the chunks of all items
+extern "C" long nrl_delta_line_bytes(long E, int heads, int Dv, int blocks) {
+  return blocks * (128l * 128 * 4 + 16) + (E * heads * ((Dv + 127) / 128) + blocks) * static_cast<long>(sizeof(nrl::DcSegment));
+}
 extern "C" cudaError_t nrl_delta_chunk_tc(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state, float* o,
                                           const int* cu, const int* start, const int* state_slot, int E, int heads, int kv_heads, int D, int Dv,
-                                          bool rows16, cudaStream_t s) {
-  const nrl::DcParams p{qkv, beta, decay, state, o, cu, start, state_slot, sq, col_k, col_v, heads, kv_heads, D, Dv};
-  const unsigned grid = static_cast<unsigned>(E) * heads * ((Dv + 127) / 128);
+                                          bool rows16, void* line, int blocks, cudaStream_t s) {
+  nrl::DcParams p{qkv, beta, decay, state, o, cu, start, state_slot, sq, col_k, col_v, heads, kv_heads, D, Dv, {}};
+  const int parts = (Dv + 127) / 128;
+  unsigned grid = static_cast<unsigned>(E) * heads * parts;
+  if (line != nullptr) {
+    if (E > nrl::kDcMaxEntries || !rows16) return cudaErrorInvalidValue;
+    p.line.carry = static_cast<float*>(line);
+    p.line.first = reinterpret_cast<int*>(p.line.carry + blocks * 128l * 128);
+    p.line.last = p.line.first + blocks;
+    p.line.handed = p.line.last + blocks;
+    p.line.segments = reinterpret_cast<nrl::DcSegment*>(p.line.handed + 2 * blocks);
+    nrl::delta_line_kernel<<<1, 1024, 0, s>>>(cu, E, heads, parts, blocks, p.line);
+    grid = static_cast<unsigned>(blocks);
+  }
 #define NRL_DC(P_, B_)                                                 \
   if ((D <= 64 ? 64 : 128) == P_ && (beta != nullptr) == B_)             \
-    return (rows16 ? nrl::launch_delta_chunk<P_, B_, true> : nrl::launch_delta_chunk<P_, B_, false>)(grid, p, s);
+    return (line != nullptr ? nrl::launch_delta_chunk<P_, B_, true, true>                                                       \
+                            : rows16 ? nrl::launch_delta_chunk<P_, B_, true, false> : nrl::launch_delta_chunk<P_, B_, false, false>)(grid, p, s);
   NRL_DC(64, true) NRL_DC(64, false) NRL_DC(128, true) NRL_DC(128, false)
 #undef NRL_DC
   return cudaErrorInvalidValue;

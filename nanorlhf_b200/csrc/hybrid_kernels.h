@@ -162,10 +162,14 @@ cudaError_t nrl_gla_prep(float* qkv, long sq, const float* a_raw, long sa, const
 // 1 column-resident, 2 row groups, 3 state in shared memory, 4 four tokens at a time (D <= 128), 5 32 at a time (D <= 128, one decay per head).
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
                            float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
-                           int D, int Dv, int per_channel, int impl, int num_sms, cudaStream_t s);
+                           int D, int Dv, int per_channel, int impl, int num_sms, void* scratch, cudaStream_t s);
+// bytes of scratch that such a call wants (0: null)
+long nrl_delta_scan_scratch(const float* qkv, long sq, int col_k, int col_v, long E, long T, int heads, int D, int Dv, int per_channel, int impl, int num_sms);
+long nrl_delta_line_bytes(long E, int heads, int Dv, int blocks);
+int nrl_delta_scan_shared(long E, long T, int heads, int Dv, int num_sms);      // a step taken 32 tokens at a time: its blocks share the chunks of all items
 cudaError_t nrl_delta_chunk_tc(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state, float* o,
                                const int* cu, const int* start, const int* state_slot, int E, int heads, int kv_heads, int D, int Dv,
-                               bool rows16, cudaStream_t s);      // rows16: rows of q, k and v start and end on 16-byte boundaries
+                               bool rows16, void* line, int blocks, cudaStream_t s);      // rows16: rows of q, k and v start and end on 16-byte boundaries
 int nrl_delta_scan_chunked(long E, long T, int heads, int D, int Dv, int num_sms);      // one decay per head: impl 0 takes a step of E entries and T tokens 32 at a time
 int nrl_delta_scan_blocked(long E, long T, int D, int Dv);       // impl 0 takes a step of E entries and T tokens four tokens at a time
 
