@@ -8,16 +8,21 @@
 //   * K page  [16 tokens][128 d] e4m3 (2 KB);  V page stored TRANSPOSED [128 d][16 tokens] e4m3 (2 KB);
 //     one fp32 scale per (token, kv head) for K and for V (64 + 64 B)   ->  4.1 KB per page instead of 8 KB.
 //   * both MMAs are mma.sync m16n8k16 f16 (e4m3 values are exact in f16).  The B fragment of that instruction wants, per
-//     thread, the pairs k = {2t, 2t+1} and {2t+8, 2t+9} of one column.  The contraction index is a dummy, so it is RENUMBERED:
-//     virtual k {2t, 2t+1, 2t+8, 2t+9} := physical {4t, 4t+1, 4t+2, 4t+3}.  One 32-bit shared-memory load then holds exactly
-//     the four e4m3 values a thread needs, and two `cvt.rn.f16x2.e4m3x2` turn it into the two B registers -- no unpacking,
-//     no ldmatrix, no shuffles.  Q (the A operand of S = Q K^T) is loaded with the same renumbering of d; for O = P V the
+//     thread, the pairs k = {2t, 2t+1} and {2t+8, 2t+9} of one column.  The contraction index is a dummy, so it is RENUMBERED: a thread's
+//     four virtual k are four neighbouring physical ones.  One 32-bit word then holds exactly the four e4m3 values that a thread needs, and two
+//     `cvt.rn.f16x2.e4m3x2` turn it into the two B registers -- no unpacking, no ldmatrix, no shuffles.  For S = Q K^T thread t takes d = 64 h + 16 t .. + 15,
+//     so that one 16-byte load feeds four MMAs; Q (the A operand) is loaded with the same numbers.  For O = P V the
 //     renumbered index is the token, which fixes which physical key each score column must hold: lane group g of score tile
 //     j loads key 4 (g >> 1) + 2 j + (g & 1), so the accumulator registers of S already sit where the A fragment of P needs them.
 //   * per-token scales: S[:, tok] *= k_scale[tok] after the first MMA, P[:, tok] *= v_scale[tok] * 2^10 before the second
 //     (the 2^10 keeps small probabilities out of the f16 subnormal range; it is divided out with the softmax denominator).
 //   * per-warp 4-stage cp.async page pipeline, all G = Hq / Hkv query heads per KV read, split-KV merge -- as in the
-//     bf16 kernel; 3 CTAs per SM (68 KB each) keep ~200 KB of loads in flight per SM.
+//     bf16 kernel; 3 CTAs per SM (68 KB each) keep 100 to 200 KB of loads in flight per SM.
+//   * two pages a step: one maximum, one rescaling of O and half the bookkeeping per page; page numbers wait in the lanes, 32 at a time, and the sum of the
+//     weights is joined over the lanes at the end.  What bounds it is the copy rate, and under the power cap the energy of what is issued beside it: a fifth
+//     fewer instructions per page take 1024 sequences of 1000 tokens from 103 to 97 us (0.87 of the copy rate), kept up for seconds from 111 to 105;
+//     256 sequences 37.4 -> 35.5.  Six stages with two CTAs per SM 110; an odd last page inside the step of two, by predicates 108, as a page of zeros 104 and
+//     a microsecond more for short contexts.
 //
 // Reference path replaced: vLLM PagedAttention / FlashInfer decode inside llm.generate
 // (GRPO/grpo_trainer.py:142).
@@ -25,6 +30,8 @@
 #include "kernels.h"
 #include "decode_merge.cuh"
 #include "launch.h"
+
+#include <type_traits>
 
 namespace nrl {
 
@@ -57,9 +64,14 @@ NRL_DEVICE uint32_t lds32(uint32_t addr) {
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(r) : "r"(addr));
   return r;
 }
-// K rows are 128 B = 8 chunks of 16 B; chunk c of token row r lives at chunk (c ^ sigma(r)), sigma(r) = 2 (r >> 2) + (r & 1):
-// the 8 rows a warp reads together (4 (g >> 1) + 2 j + (g & 1), g = 0..7) have sigma = g, i.e. 8 distinct chunks -> 32 banks.
-NRL_DEVICE int k_sigma(int r) { return ((r >> 2) << 1) | (r & 1); }
+NRL_DEVICE uint4 lds128(uint32_t addr) {
+  uint4 r;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(addr));
+  return r;
+}
+// K rows are 128 B = 8 chunks of 16 B; chunk c of token row r lives at chunk c ^ 4 (r & 1): the eight lanes that are served together read chunks t = 0..3
+// (or 4..7) of an even and an odd row, which are all eight chunks' banks.
+NRL_DEVICE int k_sigma(int r) { return (r & 1) << 2; }
 
 // ---- page writer: one warp per (token, kv head) ----------------------------------------------------------------
 // kq [num_blocks, Hkv, 16, 128]   vq [num_blocks, Hkv, 128, 16] (transposed)   ks, vs [num_blocks, Hkv, 16]
@@ -131,14 +143,14 @@ __global__ void __launch_bounds__(kWarps8 * 32, 3) paged_decode_fp8_kernel(Decod
   const int page_hi = min(n_pages, page_lo + pages_per_split);
   const int* bt = p.block_tables + static_cast<long>(seq) * p.max_blocks;
 
-  // ---- Q fragments straight from global: row g (query head g of this kv head), d = 16 ks + 4 t .. + 3, as f16 ----
+  // ---- Q fragments straight from global: row g (query head g of this kv head), d = 64 (ks >> 2) + 16 t + 4 (ks & 3) .. + 3, as f16 ----
   uint32_t qa0[8], qa2[8];
   {
     const bool real = g < p.G;
     const __nv_bfloat16* qrow = p.q + seq * p.q_stride_s + (kvh * p.G + (real ? g : 0)) * kHd;
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(qrow + ks * 16 + t4 * 4);
+      const uint2 raw = *reinterpret_cast<const uint2*>(qrow + (ks >> 2) * 64 + t4 * 16 + (ks & 3) * 4);
       const float2 a = unpack_bf16x2(raw.x), b = unpack_bf16x2(raw.y);
       qa0[ks] = real ? pack_f16x2(a.x, a.y) : 0u;
       qa2[ks] = real ? pack_f16x2(b.x, b.y) : 0u;
@@ -149,10 +161,12 @@ __global__ void __launch_bounds__(kWarps8 * 32, 3) paged_decode_fp8_kernel(Decod
   const int my_first = page_lo + warp;
   const int my_count = (my_first < page_hi) ? (page_hi - my_first + kWarps8 - 1) / kWarps8 : 0;
 
+  // the warp's pages, 32 at a time in its lanes: a look-up per page would stand in front of every page's copies
+  int ids = 0;
   auto issue = [&](int it) {
+    if ((it & 31) == 0) ids = it + lane < my_count ? bt[my_first + (it + lane) * kWarps8] : 0;
+    const long pg = static_cast<long>(__shfl_sync(0xffffffffu, ids, it & 31)) * p.Hkv + kvh;
     if (it < my_count) {
-      const int page = my_first + it * kWarps8;
-      const long pg = static_cast<long>(bt[page]) * p.Hkv + kvh;
       const uint8_t* ksrc = p.kq + pg * kRawPage;
       const uint8_t* vsrc = p.vq + pg * kRawPage;
       uint8_t* kd = my_smem + (it % kStages8) * kStage8;
@@ -175,76 +189,96 @@ __global__ void __launch_bounds__(kWarps8 * 32, 3) paged_decode_fp8_kernel(Decod
   float o[16][4];
 #pragma unroll
   for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float m_run = -INFINITY, l_run = 0.f;     // row g
+  float m_run = -INFINITY, l_run = 0.f;     // row g; the sum over this thread's tokens
 
-#pragma unroll
-  for (int s = 0; s < kStages8 - 1; ++s) issue(s);
-  for (int it = 0; it < my_count; ++it) {
-    issue(it + kStages8 - 1);
-    cp_async_wait<kStages8 - 1>();
+#pragma unroll 1
+  for (int s = 0; s < kStages8; ++s) issue(s);
+  auto step = [&](auto pages, int it) {             // pages it and, of two, it + 1: one rescaling of O
+    constexpr int U = decltype(pages)::value;
+    cp_async_wait<kStages8 - U>();
     __syncwarp();
-    const uint32_t kb = smem_u32(my_smem + (it % kStages8) * kStage8);
-    const uint32_t vb = kb + kRawPage;
-    const uint32_t sb = vb + kRawPage;
-    const int tok0 = (my_first + it * kWarps8) * kPg;
-
-    // ---- S = Q K^T : score tile j holds physical keys 4 t + 2 j + {0, 1} in its columns {2t, 2t+1} ----
-    float s[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    const int tok0 = (my_first + it * kWarps8) * kPg;      // of the first; the second's lie 16 kWarps8 further
+    // ---- S = Q K^T : score tile j of a page holds its keys 4 t + 2 j + {0, 1} in columns {2t, 2t+1} ----
+    float s[U][2][4];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int krow = ((g >> 1) << 2) + 2 * j + (g & 1);            // sigma(krow) == g
-      const uint32_t rbase = kb + krow * 128 + t4 * 4;
+    for (int u = 0; u < U; ++u) {
+      const uint32_t kb = smem_u32(my_smem + ((it + u) % kStages8) * kStage8);
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const uint32_t w = lds32(rbase + ((ks ^ g) << 4));
-        mma_f16_16816(s[j], qa0[ks], qa2[ks], e4m3x2_to_f16x2(w & 0xFFFFu), e4m3x2_to_f16x2(w >> 16));
+      for (int j = 0; j < 2; ++j) {
+        s[u][j][0] = s[u][j][1] = s[u][j][2] = s[u][j][3] = 0.f;
+        const int krow = ((g >> 1) << 2) + 2 * j + (g & 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 w4 = lds128(kb + krow * 128 + (((4 * h + t4) ^ k_sigma(g)) << 4));      // sigma(krow) == sigma(g)
+          const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            mma_f16_16816(s[u][j], qa0[4 * h + i], qa2[4 * h + i], e4m3x2_to_f16x2(w[i] & 0xFFFFu), e4m3x2_to_f16x2(w[i] >> 16));
+        }
       }
     }
     // ---- scale, mask, online softmax on row g ----
-    float4 ksc, vsc;
-    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(ksc.x), "=f"(ksc.y), "=f"(ksc.z), "=f"(ksc.w) : "r"(sb + t4 * 16));
-    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(vsc.x), "=f"(vsc.y), "=f"(vsc.z), "=f"(vsc.w) : "r"(sb + 64 + t4 * 16));
-    const float kscale[2][2] = {{ksc.x, ksc.y}, {ksc.z, ksc.w}};
-    const float vscale[2][2] = {{vsc.x, vsc.y}, {vsc.z, vsc.w}};
+    float vscale[U][4];
     float tmax = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int u = 0; u < U; ++u) {
+      const uint32_t sb = smem_u32(my_smem + ((it + u) % kStages8) * kStage8) + 2 * kRawPage;
+      const uint4 kr = lds128(sb + t4 * 16), vr = lds128(sb + 64 + t4 * 16);
+      const float kscale[4] = {__uint_as_float(kr.x), __uint_as_float(kr.y), __uint_as_float(kr.z), __uint_as_float(kr.w)};
+      vscale[u][0] = __uint_as_float(vr.x); vscale[u][1] = __uint_as_float(vr.y); vscale[u][2] = __uint_as_float(vr.z); vscale[u][3] = __uint_as_float(vr.w);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int tok = tok0 + t4 * 4 + 2 * j + e;
-        s[j][e] = (tok >= ctx) ? -INFINITY : s[j][e] * kscale[j][e] * p.scale_log2;
-        tmax = fmaxf(tmax, s[j][e]);
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) s[u][j][e] *= kscale[2 * j + e] * p.scale_log2;
+      if (tok0 + u * kWarps8 * kPg + kPg > ctx) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (tok0 + u * kWarps8 * kPg + t4 * 4 + 2 * j + e >= ctx) s[u][j][e] = -INFINITY;
       }
+      tmax = fmaxf(tmax, fmaxf(fmaxf(s[u][0][0], s[u][0][1]), fmaxf(s[u][1][0], s[u][1][1])));
+    }
     tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
     tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-    const float m_new = fmaxf(m_run, tmax);
-    const float corr = (m_new == -INFINITY) ? 1.f : exp2f(m_run - m_new);
+    const float m_new = fmaxf(m_run, tmax), m_sub = m_new == -INFINITY ? 0.f : m_new;
+    const float corr = exp2f(m_run - m_sub);        // 0 while nothing has been seen
+    uint32_t pa[U][2];
     float psum = 0.f;
-    float pr[2][2];
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int u = 0; u < U; ++u) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        pr[j][e] = (m_new == -INFINITY) ? 0.f : exp2f(s[j][e] - m_new);
-        psum += pr[j][e];
+      for (int j = 0; j < 2; ++j) {
+        const float p0 = exp2f(s[u][j][0] - m_sub), p1 = exp2f(s[u][j][1] - m_sub);
+        psum += p0 + p1;
+        // tokens 4 t + 2 j, + 1: the A fragment is this thread's own score registers
+        pa[u][j] = pack_f16x2(p0 * (vscale[u][2 * j] * kPScale), p1 * (vscale[u][2 * j + 1] * kPScale));
       }
-    psum += __shfl_xor_sync(0xffffffffu, psum, 1);
-    psum += __shfl_xor_sync(0xffffffffu, psum, 2);
+    }
     l_run = l_run * corr + psum;
     m_run = m_new;
 #pragma unroll
     for (int i = 0; i < 16; ++i) { o[i][0] *= corr; o[i][1] *= corr; }
-    // ---- O += (P * v_scale) V : A fragment = this thread's own score registers ----
-    const uint32_t pa0 = pack_f16x2(pr[0][0] * vscale[0][0] * kPScale, pr[0][1] * vscale[0][1] * kPScale);   // tokens 4t, 4t+1
-    const uint32_t pa2 = pack_f16x2(pr[1][0] * vscale[1][0] * kPScale, pr[1][1] * vscale[1][1] * kPScale);   // tokens 4t+2, 4t+3
-    const uint32_t vrow = vb + g * kPg + t4 * 4;                          // V^T[d = 8 nd + g][tokens 4t .. 4t+3]
+    // ---- O += (P * v_scale) V ----
 #pragma unroll
-    for (int nd = 0; nd < 16; ++nd) {
-      const uint32_t w = lds32(vrow + nd * 8 * kPg);
-      mma_f16_16816(o[nd], pa0, pa2, e4m3x2_to_f16x2(w & 0xFFFFu), e4m3x2_to_f16x2(w >> 16));
+    for (int u = 0; u < U; ++u) {
+      const uint32_t vrow = smem_u32(my_smem + ((it + u) % kStages8) * kStage8) + kRawPage + g * kPg + t4 * 4;      // V^T[d = 8 nd + g][tokens 4t .. 4t+3]
+#pragma unroll
+      for (int nd = 0; nd < 16; ++nd) {
+        const uint32_t w = lds32(vrow + nd * 8 * kPg);
+        mma_f16_16816(o[nd], pa[u][0], pa[u][1], e4m3x2_to_f16x2(w & 0xFFFFu), e4m3x2_to_f16x2(w >> 16));
+      }
     }
     __syncwarp();
-  }
+#pragma unroll 1
+    for (int u = 0; u < U; ++u) issue(it + kStages8 + u);
+  };
+  int it = 0;
+#pragma unroll 1
+  for (; it + 1 < my_count; it += 2) step(std::integral_constant<int, 2>{}, it);
+  if (it < my_count) step(std::integral_constant<int, 1>{}, it);
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
   cp_async_wait<0>();
   __syncthreads();
 
