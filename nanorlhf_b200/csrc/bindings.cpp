@@ -1,6 +1,7 @@
 // Python bindings (pybind11 via torch extension headers) for the sm_100a kernels.
 // Kernels live in plain .cu translation units with a C launch API (kernels.h, gemm_sm100.h); this file
 // only validates tensors, builds TMA descriptors and forwards the current CUDA stream.
+#include <functional>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
@@ -382,6 +383,62 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
   check(nrl_gemm_tc(maps, &p, ch.cg, ch.bn, a_mn ? 1 : 0, b_mn ? 1 : 0, f32 ? nrl::tc::EPI_F32 : nrl::tc::EPI_BF16, num_sms(),
                     cur_stream()), "gemm_tc (no kernel instantiated for this cg / block_n / operand-major combination?)");
   return out;
+}
+
+// Several products a[i] [K_i, M_i]^T (a_mn) or [M_i, K_i] times b[i] [K_i, N_i] in one launch, into out[i] [M_i, N_i] or, transposed[i], [N_i, M_i].
+// The number of ranges of every contraction is the one for which this estimate (us) is least: 0.2 for each block of 64 contraction columns of a range and 3 for a
+// tile's start and end, by rounds of the grid, and 1.0 (1.6 above four) for the sum of the parts.
+// The factors' gradients of rank-64 adapters of a 1536 / 8960 wide layer, us, a launch for each product -> one launch (the best number of ranges where it is another):
+//   tokens                          200           700           1650          3300          6601
+//   gate, up and down               19.8 -> 12.0  27.8 -> 15.0  41.0 -> 23.9  58.6 -> 40.6  87.4 -> 68.7
+//   query, key and value            15.6 -> 5.9   21.2 -> 7.4   24.2 -> 8.0   27.2 -> 10.9  33.9 -> 16.3
+//   output                          7.9 -> 5.9    10.8 -> 7.4   12.5 -> 6.9   14.4 -> 8.1   17.0 -> 10.5
+//   dt of gate and up               16.9 -> 9.0   17.4 -> 9.7   18.9 -> 12.5  30.2 -> 24.6  48.2 -> 42.2
+//   dt of query, key and value      13.3 -> 9.7   13.5 -> 9.7   14.1 -> 10.0  14.6 -> 10.0  16.3 -> 11.4   (four ranges, up to 700 tokens: 6.1)
+// 3584 / 18944 wide, the five together: 60 tokens 76 -> 54, 250 85 -> 59, 1000 124 -> 85, 6601 338 -> 292, 16 384 700 -> 664; single ones lose up to 0.7 us below 300
+// tokens and 4 us at 16 384.
+// What bounds the large ones is the copy of the 8960-wide operand, 118 MB (18 us) a product, which each product reads once.
+int64_t multi_splits(const std::vector<int64_t>& tiles, const std::vector<int64_t>& blocks, int64_t sms, const std::function<int(int)>& fits) {
+  int64_t total = 0, longest = 0, best = 1;
+  for (size_t i = 0; i < tiles.size(); ++i) {
+    total += tiles[i];
+    longest = std::max(longest, blocks[i]);
+  }
+  double least = 1e30;
+  for (int64_t s = 1; s <= 8; ++s) {
+    bool ok = s == 1 || (total * s <= sms && total <= fits(static_cast<int>(s)));
+    for (int64_t b : blocks) ok = ok && (s == 1 || (b >= 4 * s && split_ranges(b, s) == s));
+    if (!ok) continue;
+    const double t = static_cast<double>((total * s + sms - 1) / sms) * (0.2 * ((longest + s - 1) / s) + 3.0) + (s == 1 ? 0.0 : s > 4 ? 1.6 : 1.0);
+    if (t < least) { least = t; best = s; }
+  }
+  return best;
+}
+void gemm_tc_multi(const std::vector<torch::Tensor>& a, const std::vector<torch::Tensor>& b, std::vector<torch::Tensor> out, const std::vector<bool>& transposed,
+                   const std::vector<double>& alpha, bool a_mn, int64_t splits_req) {
+  const size_t n = a.size();
+  TORCH_CHECK(n >= 1 && n <= nrl::tc::kMultiMax && b.size() == n && out.size() == n && transposed.size() == n && alpha.size() == n, "gemm_tc_multi: one to six products");
+  c10::cuda::CUDAGuard guard(a[0].device());
+  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  CUtensorMap maps[2 * nrl::tc::kMultiMax];
+  nrl::tc::TcMultiProduct q[nrl::tc::kMultiMax];
+  std::vector<int64_t> tiles, blocks;
+  for (size_t i = 0; i < n; ++i) {
+    check_tc_operand(a[i], "a");
+    check_tc_operand(b[i], "b");
+    check_tc_operand(out[i], "out");
+    const int64_t M = a_mn ? a[i].size(1) : a[i].size(0), K = a_mn ? a[i].size(0) : a[i].size(1), N = b[i].size(1);
+    TORCH_CHECK(b[i].size(0) == K && N % 8 == 0 && M > 0 && N > 0 && K > 0, "gemm_tc_multi: shapes differ");
+    TORCH_CHECK(out[i].size(transposed[i] ? 1 : 0) == M && out[i].size(transposed[i] ? 0 : 1) == N, "gemm_tc_multi: out has the wrong shape");
+    maps[2 * i] = nrl::make_tma_2d(a[i].data_ptr(), a[i].size(0), a[i].size(1), a[i].stride(0) * 2, a_mn ? 64 : 128, 64, BF, 2);
+    maps[2 * i + 1] = nrl::make_tma_2d(b[i].data_ptr(), K, N, b[i].stride(0) * 2, 64, 64, BF, 2);
+    q[i] = {static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<float>(alpha[i]), out[i].data_ptr(), out[i].stride(0), transposed[i] ? 1 : 0};
+    tiles.push_back(((M + 127) / 128) * ((N + 63) / 64));
+    blocks.push_back((K + 63) / 64);
+  }
+  const int64_t splits = splits_req > 0 ? splits_req : multi_splits(tiles, blocks, num_sms(), [&](int s) { return nrl_gemm_tc_multi_clusters(a_mn ? 1 : 0, s); });
+  for (int64_t x : blocks) TORCH_CHECK(split_ranges(x, splits) == splits, "gemm_tc_multi: an empty range");
+  check(nrl_gemm_tc_multi(maps, q, static_cast<int>(n), a_mn ? 1 : 0, static_cast<int>(splits), cur_stream()), "gemm_tc_multi");
 }
 
 // out[b] = a[b] . b[b]^T for b < B: a [B, M, K], b [B, N, K], out [B, M, N]; any batch / row strides (inner stride 1), e.g. the
@@ -1400,6 +1457,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_split_clusters", &nrl_gemm_tc_split_clusters, py::arg("block_n"), py::arg("splits"));
   m.def("gemm_tc_swiglu_pair_keep", &gemm_tc_swiglu_pair_keep, "(act, gate, up) of gemm_tc_swiglu_pair with adapters");
   m.def("gemm_tc_dswiglu", &gemm_tc_dswiglu, "(d gate, d up) of silu(gate) * up behind a projection's backward");
+  m.def("gemm_tc_multi", &gemm_tc_multi, "several products with narrow results in one launch", py::arg("a"), py::arg("b"), py::arg("out"), py::arg("transposed"),
+        py::arg("alpha"), py::arg("a_mn"), py::arg("splits") = 0);
+  m.def("gemm_tc_multi_splits", [](const std::vector<int64_t>& tiles, const std::vector<int64_t>& blocks, int64_t sms, const std::vector<int>& fits) {
+    return multi_splits(tiles, blocks, sms, [&](int s) { return fits.at(s); });
+  });
   m.def("gemm_tc_sum", &gemm_tc_sum, "sum_i a[i] b[i] in one accumulator", py::arg("a"), py::arg("b"));
   m.def("gemm_tc_swiglu_pair", &gemm_tc_swiglu_pair, py::arg("x"), py::arg("wg"), py::arg("wu"), py::arg("tg") = py::none(),
         py::arg("tu") = py::none(), py::arg("bg") = py::none(), py::arg("bu") = py::none());

@@ -217,7 +217,7 @@ NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F
 template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, bool BATCH = false, bool FP8 = false, bool GROUPED = false,
           bool PAIR = false, bool CLUSTER = false, bool SUM = false>
 NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
-                             const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* more = nullptr) {
+                             const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* more = nullptr, int unit0 = 0) {
   // more: PAIR the up adapter's columns, then (EPI_SWIGLU_KEEP) gate and up; EPI_DSWIGLU gate, up, d up; SUM kSumPairs maps of A and as many of B
   using C = Cfg<CG, BN, B_MN, EPI == EPI_DSWIGLU ? 2 : 1>;
   constexpr bool kPlainStores = EPI == EPI_F32 || EPI == EPI_LOGPROB || EPI == EPI_GRP_SWIGLU || EPI == EPI_GRP_RELU2;
@@ -241,7 +241,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   const int splits = SPLIT ? p.splits : 1;
   const int kb_per_split = (num_kb + splits - 1) / splits;
   const int tiles_per_batch = num_m * num_n;
-  const int unit = blockIdx.x / CG, num_units = gridDim.x / CG;
+  const int unit = blockIdx.x / CG - unit0, num_units = gridDim.x / CG;      // unit0: blocks that work on other products
   volatile int* s_last = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
   if (warp == 0 && lane == 0) {
@@ -886,6 +886,11 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           acc[2 * e + 1] += bf.y;
         }
       }
+      if (p.transposed) {                                  // neighbouring threads hold neighbouring rows
+#pragma unroll
+        for (int e = 0; e < 8; ++e) p.out_bf16[static_cast<long>(col + e) * p.out_stride + row] = __float2bfloat16(acc[e]);
+        continue;
+      }
       *reinterpret_cast<uint4*>(p.out_bf16 + static_cast<long>(row) * p.out_stride + col) =
           make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
     }
@@ -1087,6 +1092,49 @@ template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
   gemm_tc_body<1, BN, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
+}
+
+// Several products with results at most a few tiles wide (the adapters' factors and inputs) in one launch: each of them alone leaves SMs idle and starts and
+// ends for 5 us, as long as it works.  The products' tiles lie one after the other over the grid, every tile cut into the same number of ranges.
+struct TcMulti {
+  CUtensorMap a[kMultiMax], b[kMultiMax];
+  int tiles[kMultiMax];                                    // up to and with the i-th product
+  int M[kMultiMax], N[kMultiMax], K[kMultiMax];
+  float alpha[kMultiMax];
+  __nv_bfloat16* out[kMultiMax];
+  long stride[kMultiMax];
+  int transposed[kMultiMax];
+};
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(kThreads, 1) gemm_tc_multi_kernel(const __grid_constant__ TcMulti m, const int splits) {
+  int i = 0;
+  while (static_cast<int>(blockIdx.x) >= m.tiles[i] * splits) ++i;      // the grid ends with the last product
+  TcParams p{};
+  p.M = m.M[i]; p.N = m.N[i]; p.K = m.K[i];
+  p.alpha = m.alpha[i];
+  p.splits = splits;
+  p.out_bf16 = m.out[i];
+  p.out_stride = m.stride[i];
+  p.transposed = m.transposed[i];
+  gemm_tc_body<1, 64, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true>(m.a[i], m.b[i], m.a[i], m.b[i], m.a[i], p, nullptr,
+                                                                                   i > 0 ? m.tiles[i - 1] * splits : 0);
+}
+template <bool A_MN, bool B_MN>
+static int multi_clusters(int splits) {
+  if (splits < 1 || splits > kMaxClusterSplits) return 0;
+  static int fits[kMaxClusterSplits + 1] = {};             // plus one
+  if (fits[splits] == 0) {
+    auto kern = gemm_tc_multi_kernel<A_MN, B_MN>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1, 64, B_MN>::kTotal);
+    fits[splits] = 1 + (e == cudaSuccess ? clusters_at_a_time(kern, kThreads, Cfg<1, 64, B_MN>::kTotal, splits) : 0);
+  }
+  return fits[splits] - 1;
+}
+template <bool A_MN, bool B_MN>
+static cudaError_t launch_multi(const TcMulti& m, int n, int splits, cudaStream_t stream) {
+  if (multi_clusters<A_MN, B_MN>(splits) < 1) return cudaErrorInvalidConfiguration;
+  launch_dependent_clusters(gemm_tc_multi_kernel<A_MN, B_MN>, m.tiles[n - 1] * splits, kThreads, Cfg<1, 64, B_MN>::kTotal, stream, splits, m, splits);
+  return cudaGetLastError();
 }
 
 // The same with pairs of blocks on a tile of 256 rows: a cluster is `splits` pairs, and each block sums rows of its own half.
@@ -1309,6 +1357,30 @@ extern "C" cudaError_t nrl_gemm_tc_grouped(const CUtensorMap* maps, const nrl::t
   if (bn == 128) return launch_grouped<128>(maps, *p, max_tiles, num_sms, stream);
   if (bn == 256) return launch_grouped<256>(maps, *p, max_tiles, num_sms, stream);
   return cudaErrorInvalidValue;
+}
+
+extern "C" int nrl_gemm_tc_multi_clusters(int a_mn, int splits) {
+  return a_mn ? nrl::tc::multi_clusters<true, true>(splits) : nrl::tc::multi_clusters<false, true>(splits);
+}
+extern "C" cudaError_t nrl_gemm_tc_multi(const CUtensorMap* maps, const nrl::tc::TcMultiProduct* products, int n, int a_mn, int splits, cudaStream_t stream) {
+  using namespace nrl::tc;
+  if (n < 1 || n > kMultiMax || splits < 1) return cudaErrorInvalidValue;
+  TcMulti m;
+  int tiles = 0;
+  for (int i = 0; i < n; ++i) {
+    const TcMultiProduct& q = products[i];
+    if (q.M < 1 || q.N < 1 || q.K < 1 || q.out == nullptr) return cudaErrorInvalidValue;
+    tiles += ((q.M + BLOCK_M - 1) / BLOCK_M) * ((q.N + 63) / 64);
+    m.a[i] = maps[2 * i];
+    m.b[i] = maps[2 * i + 1];
+    m.tiles[i] = tiles;
+    m.M[i] = q.M; m.N[i] = q.N; m.K[i] = q.K;
+    m.alpha[i] = q.alpha;
+    m.out[i] = static_cast<__nv_bfloat16*>(q.out);
+    m.stride[i] = q.stride;
+    m.transposed[i] = q.transposed;
+  }
+  return a_mn ? launch_multi<true, true>(m, n, splits, stream) : launch_multi<false, true>(m, n, splits, stream);
 }
 
 extern "C" int nrl_gemm_tc_pair_clusters(int bn, int splits) {

@@ -20,6 +20,14 @@ enum TcEpilogue : int {
 };
 
 constexpr int kSumPairs = 4;    // products that one accumulator takes (nrl_gemm_tc_sum)
+constexpr int kMultiMax = 6;    // products of one launch (nrl_gemm_tc_multi)
+struct TcMultiProduct {         // out [M, N] (row stride `stride`) or, transposed, [N, M] = alpha A B
+  int M, N, K;
+  float alpha;
+  void* out;
+  long stride;
+  int transposed;
+};
 
 struct TcParams {
   int M, N, K;                  // D is [M, N]; K = contraction length of the first operand pair
@@ -46,6 +54,7 @@ struct TcParams {
   int* counters;                // [tiles] int32, zero between launches
   __nv_bfloat16* out_bf16;      // SPLIT: D written with plain stores (row stride out_stride elements)
   long out_stride;
+  int transposed;               // CLUSTER kernels: D^T [N, M] is written
   // GROUPED kernels (mixture of experts): the rows of A are sorted by expert and B holds every expert's [N, K] matrix one after
   // the other.  A row tile belongs to one expert; it may start at any row and is cut off at the end of the expert's rows
   // (the tile's further rows are computed and dropped).  The table and its length live on the device (written by the
@@ -64,6 +73,10 @@ inline bool split_by_clusters(int splits, long blocks) { return splits > 2 || bl
 }  // namespace tc
 }  // namespace nrl
 
+// n products in one launch, B MN-major [K, N] (box {64, 64}), A MN-major [K, M] (a_mn, box {64, 64}) or K-major [M, K] (box {128, 64}); maps = {A_0, B_0, A_1 ..}; bf16
+// results with plain stores, N and, transposed, the stride multiples of 8; every contraction cut into `splits` ranges, none empty, summed by clusters
+extern "C" int nrl_gemm_tc_multi_clusters(int a_mn, int splits);
+extern "C" cudaError_t nrl_gemm_tc_multi(const CUtensorMap* maps, const nrl::tc::TcMultiProduct* products, int n, int a_mn, int splits, cudaStream_t stream);
 // clusters of `splits` blocks that run at a time (0: none), whichever form the operands have
 extern "C" int nrl_gemm_tc_split_clusters(int bn, int splits);
 // the same for clusters of `splits` pairs of blocks (tiles of 256 x bn), and the GEMM that they run: A K-major (box {128, 64}), B box {bn / 2, 64} or, MN-major,

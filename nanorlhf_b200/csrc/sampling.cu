@@ -364,7 +364,8 @@ __global__ void __launch_bounds__(kSmemOrder, 3) sample_top_p_smem_kernel(const 
   extern __shared__ __align__(128) unsigned char s_dyn[];
   __shared__ __align__(8) uint64_t s_bar[kPiecesMax];
   __shared__ float red[2][kSmemOrder / 32];
-  __shared__ float s_x[kXSlots][kMaxCluster][2];           // exchange slots, written by the peers
+  __shared__ float s_x[kXSlots][kMaxCluster][2];           // exchange slots, written by the peers; a slot is written again four
+                                                           // cluster barriers later at the earliest and a block runs at most one ahead
   __shared__ float s_part[kSmemOrder / 16];                // masses of sixteen neighbouring threads of the order
   __shared__ float s_u;
   const uint32_t crank = cluster_ctarank(), csize = cluster_nctarank();
