@@ -3,6 +3,8 @@
 // only validates tensors, builds TMA descriptors and forwards the current CUDA stream.
 #include <functional>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/SavedTensorHooks.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -395,7 +397,7 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
 //   output                          7.9 -> 5.9    10.8 -> 7.4   12.5 -> 6.9   14.4 -> 8.1   17.0 -> 10.5
 //   dt of gate and up               16.9 -> 9.0   17.4 -> 9.7   18.9 -> 12.5  30.2 -> 24.6  48.2 -> 42.2
 //   dt of query, key and value      13.3 -> 9.7   13.5 -> 9.7   14.1 -> 10.0  14.6 -> 10.0  16.3 -> 11.4   (four ranges, up to 700 tokens: 6.1)
-// 3584 / 18944 wide, the five together: 60 tokens 76 -> 54, 250 85 -> 59, 1000 124 -> 85, 6601 338 -> 292, 16 384 700 -> 664; single ones lose up to 0.7 us below 300
+// 3584 / 18944 wide, the five together: 60 tokens 76 -> 54, 250 86 -> 59, 1000 124 -> 85, 6601 338 -> 292, 16 384 700 -> 664; single ones lose up to 1.9 us below 300
 // tokens and 4 us at 16 384.
 // What bounds the large ones is the copy of the 8960-wide operand, 118 MB (18 us) a product, which each product reads once.
 int64_t multi_splits(const std::vector<int64_t>& tiles, const std::vector<int64_t>& blocks, int64_t sms, const std::function<int(int)>& fits) {
@@ -726,11 +728,33 @@ int pick_splits(int64_t M, int64_t N, int bn, bool pairs) {
 // 1000 rows 339 / 316, 2500 rows 806 / 762, 6001 rows 1839 / 1794, under the power cap 2124 / 2043.
 bool head_pairs(int64_t M) { return 12 * ((M + 255) / 256) <= 7 * ((M + 127) / 128); }
 
-// fused lm-head log-prob forward: returns (logp, entropy, lse), all fp32 [M]
+// A [M, V] float buffer in which the head's forward leaves its logits for the backward, which then reads them instead of forming the product once more; none where
+// that is not wanted: above 4 GiB, where allocations of twice the size would leave less than a quarter of the device's memory unallocated, under hooks that would carry
+// the saved tensor elsewhere, and where the allocator does not say what it has handed out.  The gradients are the same bits either way.
+// 151 936 columns, forward and backward in a row (us), the product formed again / logits kept: 100 rows 441 / 375, 300 rows 714 / 606, 1000 rows 1560 / 1357,
+// 2000 rows 2990 / 2634, 6001 rows 8515 / 7440, for 3.6 GB of float more from the forward to the end of the backward.  The stores cost the forward 20 us up to 512
+// rows, 270 of 1759 at 6001.
+constexpr int64_t kKeptLogitsMax = 4ll << 30;
+c10::optional<torch::Tensor> lmhead_logits_buffer(const torch::Tensor& hidden, int64_t V) {
+  const int64_t M = hidden.size(0);
+  if (M == 0 || V % 8 != 0 || M > kKeptLogitsMax / 4 / V || at::SavedTensorDefaultHooks::get_hooks().has_value()) return c10::nullopt;
+  c10::cuda::CUDAGuard guard(hidden.device());
+  try {
+    const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(hidden.device().index());
+    const int64_t total = at::cuda::getCurrentDeviceProperties()->totalGlobalMem;
+    if (stats.allocated_bytes[0].current + 8 * M * V > total / 4 * 3) return c10::nullopt;
+    return torch::empty({M, V}, hidden.options().dtype(torch::kFloat32));
+  } catch (const c10::Error&) {
+    return c10::nullopt;
+  }
+}
+
+// fused lm-head log-prob forward: returns (logp, entropy, lse), all fp32 [M]; logits: lmhead_logits_buffer()'s
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> lmhead_logprob_fwd(const torch::Tensor& hidden,
                                                                           const torch::Tensor& weight,
                                                                           const torch::Tensor& targets,
-                                                                          double inv_temperature, int64_t n_splits) {
+                                                                          double inv_temperature, int64_t n_splits,
+                                                                          const c10::optional<torch::Tensor>& logits) {
   check_bf16_2d(hidden, "hidden");
   check_bf16_2d(weight, "weight");
   const int64_t M = hidden.size(0), K = hidden.size(1), V = weight.size(0);
@@ -739,6 +763,9 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> lmhead_logprob_fwd(const
               "targets must be contiguous CUDA int32 [M]");
   c10::cuda::CUDAGuard guard(hidden.device());
   auto fopt = hidden.options().dtype(torch::kFloat32);
+  if (logits.has_value())
+    TORCH_CHECK(V % 8 == 0 && logits->is_cuda() && logits->scalar_type() == torch::kFloat32 && logits->is_contiguous() && logits->dim() == 2 && logits->size(0) == M &&
+                    logits->size(1) == V && (reinterpret_cast<uintptr_t>(logits->data_ptr()) & 31) == 0, "logits must be contiguous, 32-byte aligned float32 [M, V], V a multiple of 8");
   torch::Tensor logp = torch::empty({M}, fopt), ent = torch::empty({M}, fopt), lse = torch::empty({M}, fopt);
   if (M == 0) return {logp, ent, lse};
   const int bn = 256;
@@ -755,6 +782,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> lmhead_logprob_fwd(const
     p.col_ranges = splits;
     p.targets = targets.data_ptr<int>();
     p.out_f32 = partials.data_ptr<float>();
+    p.logits = logits.has_value() ? logits->data_ptr<float>() : nullptr;
     check(nrl_gemm_tc_logprob(maps, &p, num_sms(), cur_stream()), "lmhead_logprob_fwd");
     check(nrl_lmhead_combine(partials.data_ptr<float>(), M, 2 * splits, logp.data_ptr<float>(), ent.data_ptr<float>(), lse.data_ptr<float>(), cur_stream()),
           "lmhead_combine");
@@ -767,10 +795,26 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> lmhead_logprob_fwd(const
   p.M = M; p.N = V; p.K = K; p.n_splits = splits; p.scale = static_cast<float>(inv_temperature);
   p.targets = targets.data_ptr<int>();
   p.partials = partials.data_ptr<float>();
+  p.logits = logits.has_value() ? logits->data_ptr<float>() : nullptr;
   check(nrl_gemm_bf16_tn(&tmA, &tmB, &tmA, &p, bn, nrl::EPI_LOGPROB, num_sms(), cur_stream()), "lmhead_logprob_fwd");
   check(nrl_lmhead_combine(partials.data_ptr<float>(), M, splits, logp.data_ptr<float>(), ent.data_ptr<float>(),
                            lse.data_ptr<float>(), cur_stream()), "lmhead_combine");
   return {logp, ent, lse};
+}
+
+// K-LP backward, stage 1, from the logits that the forward left
+torch::Tensor logits_grad(const torch::Tensor& logits, const torch::Tensor& targets, const torch::Tensor& lse, const torch::Tensor& grad_logp, double inv_temperature) {
+  const int64_t M = logits.size(0), V = logits.size(1);
+  TORCH_CHECK(logits.is_cuda() && logits.scalar_type() == torch::kFloat32 && logits.is_contiguous() && V % 8 == 0 &&
+              (reinterpret_cast<uintptr_t>(logits.data_ptr()) & 31) == 0, "logits must be contiguous, 32-byte aligned float32 [M, V], V a multiple of 8");
+  TORCH_CHECK(targets.scalar_type() == torch::kInt32 && lse.scalar_type() == torch::kFloat32 && grad_logp.scalar_type() == torch::kFloat32 &&
+              targets.is_contiguous() && lse.is_contiguous() && grad_logp.is_contiguous() && targets.numel() == M && lse.numel() == M && grad_logp.numel() == M);
+  c10::cuda::CUDAGuard guard(logits.device());
+  torch::Tensor dz = torch::empty({M, V}, logits.options().dtype(torch::kBFloat16));
+  if (M == 0) return dz;
+  check(nrl_logits_grad(logits.data_ptr<float>(), targets.data_ptr<int>(), lse.data_ptr<float>(), grad_logp.data_ptr<float>(), static_cast<float>(inv_temperature), M, V,
+                        dz.data_ptr(), cur_stream()), "logits_grad");
+  return dz;
 }
 
 // K-LP backward, stage 1: dZ[M,V] = (onehot - softmax) * grad_logp / T, recomputed through the tensor cores
@@ -1467,8 +1511,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("tu") = py::none(), py::arg("bg") = py::none(), py::arg("bu") = py::none());
   m.def("add_layernorm", &add_layernorm);
   m.def("lmhead_logprob_fwd", &lmhead_logprob_fwd, py::arg("hidden"), py::arg("weight"), py::arg("targets"),
-        py::arg("inv_temperature"), py::arg("n_splits") = 0);
+        py::arg("inv_temperature"), py::arg("n_splits") = 0, py::arg("logits") = py::none());
   m.def("lmhead_dlogits", &lmhead_dlogits);
+  m.def("lmhead_logits_buffer", &lmhead_logits_buffer);
+  m.def("logits_grad", &logits_grad);
   m.def("lora_merge", &lora_merge, py::arg("w"), py::arg("lora_a"), py::arg("lora_b"), py::arg("scale"), py::arg("out"),
         py::arg("mc_out_ptr") = 0);
   m.def("quant_rows_e4m3", &quant_rows_e4m3);

@@ -489,6 +489,12 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             tmem_ld_wait();
             if (it == BN / 128 - 1) release_acc();
             const int col0 = c.n_blk * BN + (it * 2 + group) * 64;
+            if (p.logits != nullptr && row_ok) {
+              float* to = p.logits + static_cast<size_t>(row) * p.N + col0;
+#pragma unroll
+              for (int j = 0; j < 64; j += 8)
+                if (col0 + j < p.N) stg_v8(to + j, &v[j >> 5][j & 31]);
+            }
             float cmax = -INFINITY;
 #pragma unroll
             for (int j = 0; j < 64; ++j) {

@@ -42,6 +42,7 @@ struct TcParams {
   float alpha;                  // multiplies the accumulator
   const __nv_bfloat16* bias;    // EPI_BF16: optional [N]
   int act;                      // EPI_BF16: 0 = none, 1 = exact (erf) GELU after the bias (GROUPED: see below)
+  float* logits;                // EPI_LOGPROB: null, or [M, N] for the accumulator
   float* out_f32;               // EPI_F32: [M, N] fp32, row stride out_f32_stride elements
   long out_f32_stride;
   int accumulate;               // EPI_F32: 1 = add to what is there

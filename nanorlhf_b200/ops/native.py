@@ -178,27 +178,29 @@ def attention_varlen(q, k, v, cu_seqlens, max_seqlen=None, causal=True, scale=No
 # fused lm-head log-prob (K-LP)
 # --------------------------------------------------------------------------------------------
 class _LmHeadLogprobFn(torch.autograd.Function):
-    """Forward: tcgen05 GEMM with an online-softmax epilogue (no [T,V] tensor).
-    Backward: the same mainloop recomputes the logits and its epilogue emits dZ in bf16 (one 8192-row chunk at a
+    """Forward: tcgen05 GEMM with an online-softmax epilogue, which for a backward also leaves the float32 logits where they take up to 4 GiB of plenty
+    (``lmhead_logits_buffer``; no [T, V] tensor otherwise).
+    Backward: dZ in bf16 from those logits, or from the same mainloop, which forms them again (one 8192-row chunk at a
     time); dH = dZ W (K-major x MN-major) and dW += dZ^T H (MN-major x MN-major, fp32 accumulate across chunks in the
     epilogue) run on the general tcgen05 GEMM -- W and H are consumed as stored, nothing is transposed."""
 
     CHUNK = 8192      # rows of dZ materialised at a time in backward (8192 x 152k bf16 = 2.5 GB)
 
     @staticmethod
-    def forward(ctx, hidden, weight, targets, temperature, want_entropy):
+    def forward(ctx, hidden, weight, targets, temperature, want_entropy, keep):
         h = hidden.contiguous()
         t32 = targets.to(torch.int32).contiguous()
         _count(2)
-        logp, ent, lse = ext().lmhead_logprob_fwd(h, weight, t32, 1.0 / temperature, 0)
-        ctx.save_for_backward(h, weight, t32, lse)
+        z = ext().lmhead_logits_buffer(h, weight.shape[0]) if keep else None
+        logp, ent, lse = ext().lmhead_logprob_fwd(h, weight, t32, 1.0 / temperature, 0, z)
+        ctx.save_for_backward(h, weight, t32, lse, z)
         ctx.temperature = temperature
         ctx.mark_non_differentiable(ent)
         return logp, ent
 
     @staticmethod
     def backward(ctx, g_logp, _g_ent):
-        h, weight, t32, lse = ctx.saved_tensors
+        h, weight, t32, lse, z = ctx.saved_tensors
         inv_t = 1.0 / ctx.temperature
         g = g_logp.float().contiguous()
         need_h, need_w = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
@@ -212,21 +214,25 @@ class _LmHeadLogprobFn(torch.autograd.Function):
         for s in range(0, T, _LmHeadLogprobFn.CHUNK):
             e = min(T, s + _LmHeadLogprobFn.CHUNK)
             _count()
-            dz = ext().lmhead_dlogits(h[s:e], weight, t32[s:e], lse[s:e], g[s:e], inv_t)
+            if z is not None:
+                dz = ext().logits_grad(z[s:e], t32[s:e], lse[s:e], g[s:e], inv_t)
+            else:
+                dz = ext().lmhead_dlogits(h[s:e], weight, t32[s:e], lse[s:e], g[s:e], inv_t)
             if need_h:
                 _lin.gemm(dz, weight, b_mn=True, out=dh[s:e])
             if need_w and whole:
                 dw = _lin.gemm(dz, h, a_mn=True, b_mn=True, split_k=0)
             elif need_w:
                 _lin.gemm(dz, h[s:e], a_mn=True, b_mn=True, out_f32=dw, accumulate=True)
-        return dh, (dw.to(weight.dtype) if need_w else None), None, None, None
+        return dh, (dw.to(weight.dtype) if need_w else None), None, None, None, None
 
 
 def lmhead_logprob(hidden, weight, targets, temperature=1.0, want_entropy=True):
     if hidden.dtype != torch.bfloat16 or hidden.shape[0] == 0:
         logp, ent, _ = ref.lmhead_logprob(hidden, weight, targets, temperature, want_entropy=want_entropy)
         return logp, ent
-    return _LmHeadLogprobFn.apply(hidden, weight, targets, float(temperature), bool(want_entropy))
+    keep = torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)
+    return _LmHeadLogprobFn.apply(hidden, weight, targets, float(temperature), bool(want_entropy), keep)
 
 
 # --------------------------------------------------------------------------------------------
