@@ -712,10 +712,11 @@ torch::Tensor gemm_tc_fp8(const torch::Tensor& aq, const torch::Tensor& a_scale,
 // Vocabulary splits of the log-prob head: the (row tile, split) items are walked by one CTA per SM, so the time is the number of rounds
 // times the tiles of an item; of equals the smallest.  6001 rows (47 row tiles) x 151 936: the smallest count that covers the SMs (4, two rounds
 // of 149 tiles) took 2623 us, 22 (seven rounds of 27) 1852 us.
+// Up to one split per SM (pair): 100 rows 126 us with 64 splits of ten tiles, 103 with 119 of five, 256 rows 124 / 109.
 int pick_splits(int64_t M, int64_t N, int bn, bool pairs) {
   const int64_t num_m = (M + (pairs ? 255 : 127)) / (pairs ? 256 : 128), num_n = (N + bn - 1) / bn, sms = num_sms() / (pairs ? 2 : 1);
   int64_t best = 1, least = INT64_MAX;
-  for (int64_t s = 1; s <= std::min<int64_t>(num_n, 64); ++s) {
+  for (int64_t s = 1; s <= std::min(num_n, sms); ++s) {
     const int64_t tiles = (num_m * s + sms - 1) / sms * ((num_n + s - 1) / s);
     if (tiles < least) { least = tiles; best = s; }
   }

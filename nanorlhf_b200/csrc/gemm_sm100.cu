@@ -454,23 +454,44 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
 }
 
-// Combine the per-split partials of the fused log-prob GEMM into logp / entropy / lse.
-__global__ void lmhead_combine_kernel(const float4* __restrict__ partials, int M, int n_splits,
-                                      float* __restrict__ logp, float* __restrict__ entropy,
-                                      float* __restrict__ lse_out) {
-  int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= M) return;
+// Combine the per-split partials of the fused log-prob GEMM into logp / entropy / lse: a block per 32 rows, eight threads a row with every eighth part each, so that a
+// row's up to 148 parts are not read one behind the other (256 rows of 128 parts 14.8 us with a thread a row).
+constexpr int kCombineRows = 32, kCombineParts = 8;
+__global__ void __launch_bounds__(kCombineRows * kCombineParts) lmhead_combine_kernel(const float4* __restrict__ partials, int M, int n_splits,
+                                                                                      float* __restrict__ logp, float* __restrict__ entropy,
+                                                                                      float* __restrict__ lse_out) {
+  __shared__ float red[4][kCombineParts][kCombineRows];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5, row = blockIdx.x * kCombineRows + lane;
   float mx = -INFINITY;
-  for (int s = 0; s < n_splits; ++s) mx = fmaxf(mx, partials[static_cast<size_t>(s) * M + row].x);
+  if (row < M)
+#pragma unroll 4
+    for (int s = part; s < n_splits; s += kCombineParts) mx = fmaxf(mx, partials[static_cast<size_t>(s) * M + row].x);
+  red[0][part][lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kCombineParts; ++i) mx = fmaxf(mx, red[0][i][lane]);
   float sum = 0.f, ez = 0.f, tgt = -INFINITY;
-  for (int s = 0; s < n_splits; ++s) {
-    float4 q = partials[static_cast<size_t>(s) * M + row];
-    float c = (q.x == -INFINITY) ? 0.f : __expf(q.x - mx);
-    sum += q.y * c;
-    ez += q.z * c;
-    tgt = fmaxf(tgt, q.w);
+  if (row < M)
+#pragma unroll 4
+    for (int s = part; s < n_splits; s += kCombineParts) {
+      const float4 q = partials[static_cast<size_t>(s) * M + row];
+      const float c = (q.x == -INFINITY) ? 0.f : __expf(q.x - mx);
+      sum += q.y * c;
+      ez += q.z * c;
+      tgt = fmaxf(tgt, q.w);
+    }
+  red[1][part][lane] = sum;
+  red[2][part][lane] = ez;
+  red[3][part][lane] = tgt;
+  __syncthreads();
+  if (part != 0 || row >= M) return;
+#pragma unroll
+  for (int i = 1; i < kCombineParts; ++i) {
+    sum += red[1][i][lane];
+    ez += red[2][i][lane];
+    tgt = fmaxf(tgt, red[3][i][lane]);
   }
-  float lse = mx + __logf(sum);
+  const float lse = mx + __logf(sum);
   logp[row] = tgt - lse;
   if (entropy != nullptr) entropy[row] = lse - ez / sum;
   if (lse_out != nullptr) lse_out[row] = lse;
@@ -579,9 +600,8 @@ extern "C" cudaError_t nrl_logits_grad(const float* z, const int* targets, const
 }
 extern "C" cudaError_t nrl_lmhead_combine(const float* partials, int M, int n_splits, float* logp, float* entropy,
                                           float* lse, cudaStream_t stream) {
-  int threads = 256;
-  int blocks = (M + threads - 1) / threads;
-  nrl::lmhead_combine_kernel<<<blocks, threads, 0, stream>>>(reinterpret_cast<const float4*>(partials), M, n_splits,
-                                                             logp, entropy, lse);
+  const int blocks = (M + nrl::kCombineRows - 1) / nrl::kCombineRows;
+  nrl::lmhead_combine_kernel<<<blocks, nrl::kCombineRows * nrl::kCombineParts, 0, stream>>>(reinterpret_cast<const float4*>(partials), M, n_splits,
+                                                                                            logp, entropy, lse);
   return cudaGetLastError();
 }
