@@ -12,7 +12,7 @@
 // Epilogues (template EPI):
 //   EPI_STORE   bf16 store (+ optional bias[N]) through swizzled smem + TMA store           (K3: linear layers)
 //   EPI_LOGPROB fused lm-head log-prob (K-LP fwd): per-row online (max, sum-exp, sum exp*z) over the vocab
-//               range of the work item + target logit; nothing of size [M,V] is ever written
+//               range of the work item + target logit; where the backward wants them the accumulators [M,V] too
 //   EPI_SWIGLU  gate_up projection with silu(gate)*up applied in the epilogue (interleaved weight rows)
 //   EPI_DLOGITS K-LP backward: dZ = (onehot(target) - softmax(z)) * g / T in bf16 via TMA store
 //
