@@ -611,6 +611,76 @@ torch::Tensor gemm_tc_sum(const std::vector<torch::Tensor>& a, const std::vector
   return out;
 }
 
+// x W_i^T + t_i b_i^T (+ bias_i) for up to four i in one launch: x [M, K], w[i] [N_i, K], t[i] [M, r] and b[i] [N_i, r] of one r, or none of them
+std::vector<torch::Tensor> gemm_tc_cat(const torch::Tensor& x, const std::vector<torch::Tensor>& w, const std::vector<c10::optional<torch::Tensor>>& bias,
+                                       const std::vector<torch::Tensor>& t, const std::vector<torch::Tensor>& b, int64_t cg_req, int64_t bn_req) {
+  const size_t n = w.size();
+  TORCH_CHECK(n >= 1 && n <= nrl::tc::kCatMax && bias.size() == n && t.size() == b.size() && (t.empty() || t.size() == n), "gemm_tc_cat: one to four products");
+  check_tc_operand(x, "x");
+  const int64_t M = x.size(0), K = x.size(1), K2 = t.empty() ? 0 : t[0].size(1);
+  c10::cuda::CUDAGuard guard(x.device());
+  std::vector<torch::Tensor> out;
+  for (size_t i = 0; i < n; ++i) {
+    check_tc_operand(w[i], "w");
+    const int64_t N = w[i].size(0);
+    TORCH_CHECK(w[i].size(1) == K && N > 0 && N % 8 == 0, "gemm_tc_cat: shapes differ");
+    if (K2 > 0) {
+      check_tc_operand(t[i], "t");
+      check_tc_operand(b[i], "b");
+      TORCH_CHECK(t[i].size(0) == M && t[i].size(1) == K2 && b[i].size(0) == N && b[i].size(1) == K2, "gemm_tc_cat: second operands have the wrong shape");
+    }
+    if (bias[i].has_value())
+      TORCH_CHECK(bias[i]->is_cuda() && bias[i]->scalar_type() == torch::kBFloat16 && bias[i]->numel() == N && bias[i]->is_contiguous() &&
+                  (reinterpret_cast<uintptr_t>(bias[i]->data_ptr()) & 15) == 0, "bias must be a contiguous, 16-byte aligned CUDA bf16 [N] tensor");
+    out.push_back(torch::empty({M, N}, x.options()));
+  }
+  if (M == 0) return out;
+  // the tile of the best use of the SMs, as pick_tc_tile
+  struct Cand { int cg, bn; double eff; };
+  int cg = 2, bn = 256;
+  double best = -1.0;
+  for (const Cand& c : {Cand{2, 256, 1.00}, Cand{2, 192, 0.95}, Cand{2, 128, 0.82}, Cand{1, 128, 0.72}, Cand{1, 64, 0.45}}) {
+    const int64_t tm = c.cg * 128, num_m = (M + tm - 1) / tm, units = num_sms() / c.cg;
+    int64_t tiles = 0, cols = 0;
+    for (const auto& y : w) { tiles += (y.size(0) + c.bn - 1) / c.bn; cols += y.size(0); }
+    tiles *= num_m;
+    const int64_t waves = (tiles + units - 1) / units;
+    const double s = c.eff * static_cast<double>(M) * cols / (static_cast<double>(waves) * units * tm * c.bn);
+    if (s > best) { best = s; cg = c.cg; bn = c.bn; }
+  }
+  if (cg_req > 0) cg = static_cast<int>(cg_req);
+  if (bn_req > 0) bn = static_cast<int>(bn_req);
+  auto map_of = [&](const torch::Tensor& y, int box) {
+    return nrl::make_tma_2d(y.data_ptr(), y.size(0), y.size(1), y.stride(0) * 2, box, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
+  };
+  constexpr int Q = nrl::tc::kCatMax;
+  CUtensorMap maps[1 + 4 * Q];
+  nrl::tc::TcCat cat{};
+  maps[0] = map_of(x, 128);
+  int tiles = 0;
+  for (size_t i = 0; i < Q; ++i) {
+    const size_t j = std::min(i, n - 1);
+    if (i < n) {
+      tiles += static_cast<int>((w[i].size(0) + bn - 1) / bn);
+      maps[1 + i] = map_of(w[i], bn / cg);
+      maps[1 + Q + i] = K2 > 0 ? map_of(t[i], 128) : maps[0];
+      maps[1 + 2 * Q + i] = K2 > 0 ? map_of(b[i], bn / cg) : maps[1 + i];
+      maps[1 + 3 * Q + i] = map_of(out[i], 32);
+      cat.n[i] = static_cast<int>(w[i].size(0));
+      if (bias[i].has_value()) cat.bias[i] = reinterpret_cast<const __nv_bfloat16*>(bias[i]->data_ptr());
+    } else {
+      for (int k = 0; k < 4; ++k) maps[1 + k * Q + i] = maps[1 + k * Q + j];
+    }
+    cat.end[i] = tiles;
+  }
+  nrl::tc::TcParams p{};
+  p.M = static_cast<int>(M); p.K = static_cast<int>(K); p.K2 = static_cast<int>(K2); p.alpha = 1.f;
+  p.batch = 1;
+  p.splits = 1;
+  check(nrl_gemm_tc_cat(maps, &p, &cat, cg, bn, num_sms(), cur_stream()), "gemm_tc_cat");
+  return out;
+}
+
 // act[M, F] = silu(x Wg^T) * (x Wu^T) with W_gu_interleaved[2F, K] (rows: per 32 features [32 gate | 32 up])
 torch::Tensor gemm_swiglu(const torch::Tensor& a, const torch::Tensor& w_interleaved, c10::optional<torch::Tensor> out_opt) {
   check_bf16_2d(a, "a");
@@ -1507,6 +1577,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_multi_splits", [](const std::vector<int64_t>& tiles, const std::vector<int64_t>& blocks, int64_t sms, const std::vector<int>& fits) {
     return multi_splits(tiles, blocks, sms, [&](int s) { return fits.at(s); });
   });
+  m.def("gemm_tc_cat", &gemm_tc_cat, "projections of one input in one launch", py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("t"), py::arg("b"), py::arg("cg") = 0,
+        py::arg("block_n") = 0);
   m.def("gemm_tc_sum", &gemm_tc_sum, "sum_i a[i] b[i] in one accumulator", py::arg("a"), py::arg("b"));
   m.def("gemm_tc_swiglu_pair", &gemm_tc_swiglu_pair, py::arg("x"), py::arg("wg"), py::arg("wu"), py::arg("tg") = py::none(),
         py::arg("tu") = py::none(), py::arg("bg") = py::none(), py::arg("bu") = py::none());

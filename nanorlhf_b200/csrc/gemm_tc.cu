@@ -215,10 +215,11 @@ NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F
 // weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
 // columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.
 template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, bool BATCH = false, bool FP8 = false, bool GROUPED = false,
-          bool PAIR = false, bool CLUSTER = false, bool SUM = false>
+          bool PAIR = false, bool CLUSTER = false, bool SUM = false, bool CAT = false>
 NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
-                             const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* more = nullptr, int unit0 = 0) {
-  // more: PAIR the up adapter's columns, then (EPI_SWIGLU_KEEP) gate and up; EPI_DSWIGLU gate, up, d up; SUM kSumPairs maps of A and as many of B
+                             const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* more = nullptr, int unit0 = 0, const TcCat* cat = nullptr) {
+  // more: PAIR the up adapter's columns, then (EPI_SWIGLU_KEEP) gate and up; EPI_DSWIGLU gate, up, d up; SUM kSumPairs maps of A and as many of B;
+  // CAT kCatMax each of B, A2, B2, D
   using C = Cfg<CG, BN, B_MN, EPI == EPI_DSWIGLU ? 2 : 1>;
   constexpr bool kPlainStores = EPI == EPI_F32 || EPI == EPI_LOGPROB || EPI == EPI_GRP_SWIGLU || EPI == EPI_GRP_RELU2;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -233,7 +234,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   const uint32_t pair = (CG == 2 && CLUSTER) ? 3u << (cluster_ctarank() & ~1u) : 3u;
   const bool leader = rank == 0;
   const int num_m = (p.M + CG * BLOCK_M - 1) / (CG * BLOCK_M);
-  const int num_n = (p.N + BN - 1) / BN;
+  const int num_n = CAT ? cat->end[kCatMax - 1] : (p.N + BN - 1) / BN;
   constexpr int kElemsPerKB = FP8 ? 2 * BLOCK_K : BLOCK_K;                  // 128 bytes of contraction per k-block either way
   const int num_kb1 = (p.K + kElemsPerKB - 1) / kElemsPerKB;
   const int num_kb2 = (p.K2 + kElemsPerKB - 1) / kElemsPerKB;
@@ -248,12 +249,14 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     if (SUM)
       for (int i = 0; i < 2 * kSumPairs; ++i) tma_prefetch_desc(more + i);
     else tma_prefetch_desc(&tmA);
-    if (!SUM) tma_prefetch_desc(&tmB);
-    if (!SUM && p.K2 > 0) {
+    if (CAT)
+      for (int i = 0; i < 4 * kCatMax; ++i) tma_prefetch_desc(more + i);
+    if (!SUM && !CAT) tma_prefetch_desc(&tmB);
+    if (!SUM && !CAT && p.K2 > 0) {
       tma_prefetch_desc(&tmA2);
       tma_prefetch_desc(&tmB2);
     }
-    if (!kPlainStores) tma_prefetch_desc(&tmD);
+    if (!kPlainStores && !CAT) tma_prefetch_desc(&tmD);
   }
   if (warp == 1 && lane == 0) {
     for (int i = 0; i < C::kStages; ++i) {
@@ -291,6 +294,12 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     c.n_blk = g * n_per_range;
     return min(num_n, c.n_blk + n_per_range);
   };
+  auto product_of = [&](int& n_blk) {                      // CAT: the product of a column tile, which becomes one of that product
+    int i = 0;
+    while (n_blk >= cat->end[i]) ++i;                      // n_blk < end[kCatMax - 1]
+    if (i > 0) n_blk -= cat->end[i - 1];
+    return i;
+  };
   const int num_work = GROUPED ? __ldg(p.grp_num_tiles) * num_n : kRanges ? num_m * p.col_ranges : tiles_per_batch * (BATCH ? p.batch : splits);
 
   if (warp == 0) {
@@ -312,6 +321,12 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             n0 = __ldg(p.grp_tiles + 3 * mt) * p.N + c.n_blk * BN;      // the expert's block of B rows
           }
           if (PAIR) n0 = c.n_blk * (BN / 2);
+          int which = 0;
+          if (CAT) {
+            int blk = c.n_blk;
+            which = product_of(blk);
+            n0 = blk * BN + static_cast<int>(rank) * C::kBRows;
+          }
           const int kb_lo = BATCH ? 0 : (w % splits) * kb_per_split, kb_hi = BATCH ? num_kb : min(num_kb, kb_lo + kb_per_split);
           for (int kb = kb_lo; kb < kb_hi; ++kb) {
             mbar_wait(&empty_bar[stage], phase ^ 1);
@@ -322,6 +337,10 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             const CUtensorMap* ma = second ? &tmA2 : &tmA;
             const CUtensorMap* mb = second ? &tmB2 : &tmB;
             int k0 = (second ? kb - num_kb1 : kb) * kElemsPerKB;
+            if (CAT) {
+              if (second) ma = more + kCatMax + which;
+              mb = more + (second ? 2 * kCatMax : 0) + which;
+            }
             if (SUM) {
               int i = 0;
               while (kb >= p.sum_end[i]) ++i;              // kb < sum_end[kSumPairs - 1]
@@ -330,9 +349,9 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
               k0 = (i > 0 ? kb - p.sum_end[i - 1] : kb) * kElemsPerKB;
             }
             if (PAIR && second) {
-              const int which = kb - num_kb1 >= num_kb2 ? 1 : 0, k2 = k0 - which * num_kb2 * kElemsPerKB;
-              tma_load_cg<CG>(sa, which ? more : &tmA2, &full_bar[stage], k2, m0);
-              tma_load_cg<CG>(sb, &tmB2, &full_bar[stage], k2, which == static_cast<int>(rank) ? n0 : p.N);
+              const int half = kb - num_kb1 >= num_kb2 ? 1 : 0, k2 = k0 - half * num_kb2 * kElemsPerKB;
+              tma_load_cg<CG>(sa, half ? more : &tmA2, &full_bar[stage], k2, m0);
+              tma_load_cg<CG>(sb, &tmB2, &full_bar[stage], k2, half == static_cast<int>(rank) ? n0 : p.N);
               if (++stage == C::kStages) { stage = 0; phase ^= 1; }
               continue;
             }
@@ -410,7 +429,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     int acc = 0;
     uint32_t acc_phase = 0;
     uint8_t* slab = smem + C::kStagingOff + (warp - 2) * (EPI == EPI_DSWIGLU ? 2 : 1) * kSlabBytes;
-    const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+    const bool bias_vec = CAT || (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
     // the accumulator has been read by this warp
     auto release_acc = [&]() {
       tc_fence_before();
@@ -462,6 +481,9 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
       (void)bidx;
       TileCoord c = GROUPED || kRanges ? TileCoord{0, 0} : tile_coord(tile_id, num_m, num_n);
       const int n_end = range_of(w, c);
+      const int which = CAT ? product_of(c.n_blk) : 0;
+      const int n_cols = CAT ? cat->n[which] : p.N;
+      const __nv_bfloat16* bias = CAT ? cat->bias[which] : p.bias;
       const int m_blk = c.m_tile * CG + static_cast<int>(rank);
       int row = m_blk * BLOCK_M + row_in_tile;
       int row_end = p.M;
@@ -818,13 +840,13 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
 #pragma unroll
               for (int e = 0; e < 8; ++e) x[e] = ((col + e == dl_target ? 1.f : 0.f) - exp2f((x[e] - dl_lse) * 1.4426950408889634f)) * dl_g;
             }
-            if (EPI != EPI_DLOGITS && p.bias != nullptr && col < p.N) {         // N % 8 == 0
+            if (EPI != EPI_DLOGITS && bias != nullptr && col < n_cols) {        // N % 8 == 0
               uint32_t bw[4];
               if (bias_vec) {
-                const uint4 bv = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
+                const uint4 bv = __ldg(reinterpret_cast<const uint4*>(bias + col));
                 bw[0] = bv.x; bw[1] = bv.y; bw[2] = bv.z; bw[3] = bv.w;
               } else {
-                const uint16_t* b16 = reinterpret_cast<const uint16_t*>(p.bias + col);
+                const uint16_t* b16 = reinterpret_cast<const uint16_t*>(bias + col);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) bw[e] = b16[2 * e] | (static_cast<uint32_t>(b16[2 * e + 1]) << 16);
               }
@@ -842,7 +864,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
 #pragma unroll
             for (int e = 0; e < 4; ++e) packed[j / 2 + e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
           }
-          if (col0 < p.N && m_blk * BLOCK_M + quad * 32 < p.M) store_slab(packed, col0, m_blk * BLOCK_M + quad * 32, bidx);
+          if (col0 < n_cols && m_blk * BLOCK_M + quad * 32 < p.M) store_slab_to(CAT ? more + 3 * kCatMax + which : &tmD, packed, col0, m_blk * BLOCK_M + quad * 32, bidx);
         }
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
@@ -973,6 +995,38 @@ static cudaError_t launch_sum(const TcMaps8& maps, const CUtensorMap& tmD, const
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;
   launch_dependent(kern, 2 * units, kThreads, C::kTotal, stream, maps, tmD, p);
+  return cudaGetLastError();
+}
+
+// D_i = A B_i^T + A2_i B2_i^T (+ bias_i): the projections of one input (query, key, value) in one launch, whose column tiles lie side by side: one start and one
+// last wave for all.  us, a launch each -> one (rows 250, 800, 3300, 6601, 24 571, 32 768): 3 x 1024 features of 1024: 23 -> 7.4, 24 -> 10, 39 -> 21, 47 -> 31, 127 -> 106, 156 -> 138;
+// 1536 + 256 + 256 of 1536 with adapters of rank 64: 31 -> 10, 30 -> 10, 39 -> 20, 47 -> 30, 131 -> 108, 164 -> 141; 3584 + 512 + 512 of 3584: 65 -> 17, 54 -> 24, 92 -> 81,
+// 165 -> 146, 626 -> 608, 788 -> 759.
+struct TcMaps16 { CUtensorMap m[4 * kCatMax]; };
+template <int BN>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_tc_cat_cg1_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ TcMaps16 maps, const TcParams p, const __grid_constant__ TcCat cat) {
+  gemm_tc_body<1, BN, false, false, EPI_BF16, false, false, false, false, false, false, false, true>(tmA, tmA, tmA, tmA, tmA, p, maps.m, 0, &cat);
+}
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_tc_cat_cg2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ TcMaps16 maps, const TcParams p, const __grid_constant__ TcCat cat) {
+  gemm_tc_body<2, BN, false, false, EPI_BF16, false, false, false, false, false, false, false, true>(tmA, tmA, tmA, tmA, tmA, p, maps.m, 0, &cat);
+}
+template <int CG, int BN>
+static cudaError_t launch_cat(const CUtensorMap& tmA, const TcMaps16& maps, const TcParams& p, const TcCat& cat, int num_sms, cudaStream_t stream) {
+  using C = Cfg<CG, BN>;
+  auto kern = CG == 2 ? gemm_tc_cat_cg2_kernel<BN> : gemm_tc_cat_cg1_kernel<BN>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  int units = (p.M + CG * BLOCK_M - 1) / (CG * BLOCK_M) * cat.end[kCatMax - 1];
+  if (units > num_sms / CG) units = num_sms / CG;
+  if (units < 1) units = 1;
+  launch_dependent(kern, CG * units, kThreads, C::kTotal, stream, tmA, maps, p, cat);
   return cudaGetLastError();
 }
 
@@ -1340,6 +1394,17 @@ extern "C" cudaError_t nrl_gemm_tc_sum(const CUtensorMap* maps, const nrl::tc::T
   if (bn == 256) return launch_sum<256>(all, d, *p, num_sms, stream);
   if (bn == 192) return launch_sum<192>(all, d, *p, num_sms, stream);
   if (bn == 128) return launch_sum<128>(all, d, *p, num_sms, stream);
+  return cudaErrorInvalidValue;
+}
+
+extern "C" cudaError_t nrl_gemm_tc_cat(const CUtensorMap* maps, const nrl::tc::TcParams* p, const nrl::tc::TcCat* cat, int cg, int bn, int num_sms, cudaStream_t stream) {
+  using namespace nrl::tc;
+  TcMaps16 all;
+  for (int i = 0; i < 4 * kCatMax; ++i) all.m[i] = maps[1 + i];
+#define NRL_TC_CAT(CG_, BN_) \
+  if (cg == CG_ && bn == BN_) return launch_cat<CG_, BN_>(maps[0], all, *p, *cat, num_sms, stream);
+  NRL_TC_CAT(1, 64) NRL_TC_CAT(1, 128) NRL_TC_CAT(2, 128) NRL_TC_CAT(2, 192) NRL_TC_CAT(2, 256)
+#undef NRL_TC_CAT
   return cudaErrorInvalidValue;
 }
 

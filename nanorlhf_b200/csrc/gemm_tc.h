@@ -29,6 +29,13 @@ struct TcMultiProduct {         // out [M, N] (row stride `stride`) or, transpos
   int transposed;
 };
 
+constexpr int kCatMax = 4;      // products of one input side by side (nrl_gemm_tc_cat)
+struct TcCat {
+  int end[kCatMax];             // column tiles of the products up to and with the i-th (of those behind the last: as many)
+  int n[kCatMax];               // its columns
+  const __nv_bfloat16* bias[kCatMax];
+};
+
 struct TcParams {
   int M, N, K;                  // D is [M, N]; K = contraction length of the first operand pair
   int K2;                       // contraction length of the second operand pair (0 = none)
@@ -110,6 +117,9 @@ extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::
 // gradients of gate and up [M, N] from dY [M, K], W [K, N], T [M, K2], A [K2, N] (K2 may be 0): maps = {dY box {128, 64}, W box {64, 64}, T box {128, 64},
 // A box {64, 64}, gate, up, d gate, d up, box {32, 64}}
 extern "C" cudaError_t nrl_gemm_tc_dswiglu(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream);
+// D_i = x W_i^T + T_i B_i^T (+ bias_i) for up to kCatMax i with one x and equal K and K2; maps = {x box {128, 64}, then kCatMax each of W box {bn / cg, 64},
+// T box {128, 64}, B box {bn / cg, 64}, D box {32, 64}}
+extern "C" cudaError_t nrl_gemm_tc_cat(const CUtensorMap* maps, const nrl::tc::TcParams* p, const nrl::tc::TcCat* cat, int cg, int bn, int num_sms, cudaStream_t stream);
 // D [M, N] = sum of A_i [M, K_i] B_i [K_i, N] on CTA pairs; maps = {A_0 .. A_3 box {128, 64}, B_0 .. B_3 box {64, 64}, D box {32, 64}}, unused ones repeat a
 // valid one; p->sum_end as there
 extern "C" cudaError_t nrl_gemm_tc_sum(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int num_sms, cudaStream_t stream);

@@ -124,12 +124,10 @@ class DisentangledSelfAttention(nn.Module):
         (bucketing is odd in its argument), so score = (Qc.Kc + A[i,c] + B[j,c]) * scale with
         A = Qc Kr^T and B = Kc Qr^T.  B is a small GEMM; A is one too where it does not fit into shared memory (more than 512 buckets)."""
         from ..ops import native
+        from .lora import lora_group_forward
         T = x.shape[0]
-        q = self.query_proj(x).view(T, self.h, self.dh)
-        k = self.key_proj(x).view(T, self.h, self.dh)
-        v = self.value_proj(x).view(T, self.h, self.dh)
-        pos_k = self.key_proj(rel_emb).view(-1, self.h, self.dh).transpose(0, 1)          # [H, NB, dh]
-        pos_q = self.query_proj(rel_emb).view(-1, self.h, self.dh).transpose(0, 1)
+        q, k, v = (y.view(T, self.h, self.dh) for y in lora_group_forward(x, [self.query_proj, self.key_proj, self.value_proj]))
+        pos_k, pos_q = (y.view(-1, self.h, self.dh).transpose(0, 1) for y in lora_group_forward(rel_emb, [self.key_proj, self.query_proj]))      # [H, NB, dh]
         # the bias tables A = Qc Kr^T and B = Kc Qr^T ([H, T, NB]): per head a [T, 64] x [NB, 64]^T product on the general
         # tcgen05 GEMM; the per-head operands are column slices of the packed projections (no copies)
         rel_b = _bias_tables(k, pos_q)

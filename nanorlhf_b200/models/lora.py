@@ -227,12 +227,18 @@ def _adapter_in_gemm(m) -> bool:
 
 def lora_group_forward(x, mods):
     """``[m(x) for m in mods]`` for projections that share their input; when all of them are plain LoRA layers with the
-    same rank / scaling their rank-r projections run as one launch (ops.lora_linear_group)."""
+    same rank / scaling their rank-r projections run as one launch (ops.lora_linear_group), and their own as another; so do plain layers outside autograd."""
     if (len(mods) > 1 and all(isinstance(m, LoraLinear) for m in mods)
             and all(_adapter_in_gemm(m) for m in mods)
             and len({(m.r, m.scaling) for m in mods}) == 1):
         return ops.lora_linear_group(x, [(m.base_layer.weight, m.base_layer.bias, m.lora_A.weight, m.lora_B.weight) for m in mods],
                                      mods[0].scaling)
+    from .qwen2 import Linear
+    if len(mods) > 1 and ops.direct_calls() and ops.use_native(x) and x.dtype == torch.bfloat16 and all(plain_module(m, Linear) for m in mods):
+        from ..ops import gemm as _gemm
+        ys = _gemm.linears(x, [m.weight for m in mods], [m.bias for m in mods])
+        if ys is not None:
+            return ys
     return [m(x) for m in mods]
 
 

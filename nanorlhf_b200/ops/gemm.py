@@ -79,6 +79,16 @@ class _LinearFn(torch.autograd.Function):
         return gx, gw, gb, None
 
 
+def linears(x, ws, bs):
+    """``[F.linear(x, w, b) ...]`` of one input without autograd; None where the native GEMMs do not apply or add up ranges of a contraction."""
+    if x.numel() == 0 or not all(supported(x, w) for w in ws):
+        return None
+    x2 = _rows(x)
+    if any(_native_mod.ext().gemm_tc_auto_splits(x2.shape[0], *w.shape) > 1 for w in ws):
+        return None
+    return [y.view(*x.shape[:-1], y.shape[-1]) for y in _projections(x2, ws, bs)]
+
+
 def linear(x, w, b=None, act: int = 0):
     """``F.linear`` on the native GEMM (``act=1``: exact GELU fused into the epilogue, no-grad use only)."""
     if supported(x, w):
@@ -177,6 +187,14 @@ def _group_backward(gs, x2, t_cat, a_cat, ws, Bs, s, need_x, more_factors=(), mo
     return gx, gas[0], gbs[:n], gbs[n:] + gas[1:]
 
 
+def _projections(x2, ws, bs, ts=(), Bs=()):
+    """``x2 W_i^T + t_i B_i^T + b_i`` for every i, in one launch where four or fewer of them have aligned biases; their sums are those of their own GEMMs."""
+    if 1 < len(ws) <= 4 and all(b is None or (b.is_contiguous() and b.dtype == torch.bfloat16 and b.data_ptr() % 16 == 0) for b in bs):
+        _native_mod._count()
+        return _native_mod.ext().gemm_tc_cat(x2, list(ws), list(bs), list(ts), list(Bs))
+    return [gemm(x2, w, a2=ts[i] if ts else None, b2=Bs[i] if Bs else None, bias=bs[i]) for i, w in enumerate(ws)]
+
+
 class _LoraGroupFn(torch.autograd.Function):
     """Several LoRA projections of ONE input (q / k / v, gate / up): the rank-r down-projections share a launch
     (``t = s x [A_1; ...; A_n]^T``), each base GEMM takes its slice of ``t`` as dual-source-K operand, and in the backward the
@@ -190,7 +208,7 @@ class _LoraGroupFn(torch.autograd.Function):
         r = As[0].shape[0]
         a_cat = torch.cat(As, 0)                                             # [n r, K]
         t_cat = gemm(x2, a_cat, alpha=scaling)                               # [T, n r]
-        ys = [gemm(x2, ws[i], a2=t_cat[:, i * r:(i + 1) * r], b2=Bs[i], bias=bs[i]) for i in range(n)]
+        ys = _projections(x2, ws, bs, [t_cat[:, i * r:(i + 1) * r] for i in range(n)], Bs)
         ctx.save_for_backward(x2, t_cat, a_cat, *ws, *Bs)
         ctx.meta = (scaling, n, r, x.shape)
         return tuple(y.view(*x.shape[:-1], y.shape[-1]) for y in ys)
