@@ -241,7 +241,7 @@ int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
 torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn, bool b_mn, const c10::optional<torch::Tensor>& a2,
                       const c10::optional<torch::Tensor>& b2, const c10::optional<torch::Tensor>& bias, int64_t act, double alpha,
                       c10::optional<torch::Tensor> out_opt, c10::optional<torch::Tensor> out_f32, bool accumulate, int64_t cg_req,
-                      int64_t bn_req, int64_t splitk_req) {
+                      int64_t bn_req, int64_t splitk_req, const c10::optional<torch::Tensor>& residual) {
   check_tc_operand(a, "a");
   check_tc_operand(b, "b");
   const int64_t M = a_mn ? a.size(1) : a.size(0), K = a_mn ? a.size(0) : a.size(1);
@@ -259,6 +259,10 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
   }
   c10::cuda::CUDAGuard guard(a.device());
   const bool f32 = out_f32.has_value();
+  if (residual.has_value()) {
+    check_tc_operand(*residual, "residual");
+    TORCH_CHECK(!f32 && !a_mn && !b_mn && residual->size(0) == M && residual->size(1) == N, "gemm_tc: residual must be [M, N], of a bf16 result of K-major operands");
+  }
   torch::Tensor out;
   if (f32) {
     TORCH_CHECK(out_f32->is_cuda() && out_f32->scalar_type() == torch::kFloat32 && out_f32->dim() == 2 && out_f32->size(0) == M &&
@@ -304,7 +308,7 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
         ps.counters = counters.data_ptr<int>();
       }
       check(nrl_gemm_tc_split_pairs(maps2, &ps, pc.bn, b_mn ? 1 : 0, pc.clusters ? 1 : 0, num_sms(), cur_stream()), "gemm_tc_split_pairs");
-      return out;
+      return residual.has_value() ? out.add_(*residual) : out;
     }
   }
   if (cg_req <= 0 && bn_req <= 0 && K2 == 0 && !f32 && bias_ok && act == 0 && (a_mn == b_mn || !a_mn) && splitk_req != 0) {
@@ -347,7 +351,7 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
       ps.out_bf16 = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
       ps.out_stride = out.stride(0);
       check(nrl_gemm_tc_splitk(maps2, &ps, bn, a_mn ? 1 : 0, b_mn ? 1 : 0, sms, cur_stream()), "gemm_tc_splitk");
-      return out;
+      return residual.has_value() ? out.add_(*residual) : out;
     }
   }
   TcChoice ch = pick_tc_tile(M, N, a_mn, b_mn, f32);
@@ -377,12 +381,16 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
                 "bias must be a contiguous CUDA bf16 [N] tensor");
     p.bias = reinterpret_cast<const __nv_bfloat16*>(bias->data_ptr());
   }
+  if (residual.has_value()) {
+    p.residual = reinterpret_cast<const __nv_bfloat16*>(residual->data_ptr());
+    p.residual_stride = residual->stride(0);
+  }
   if (f32) {
     p.out_f32 = out.data_ptr<float>();
     p.out_f32_stride = out.stride(0);
     p.accumulate = accumulate ? 1 : 0;
   }
-  check(nrl_gemm_tc(maps, &p, ch.cg, ch.bn, a_mn ? 1 : 0, b_mn ? 1 : 0, f32 ? nrl::tc::EPI_F32 : nrl::tc::EPI_BF16, num_sms(),
+  check(nrl_gemm_tc(maps, &p, ch.cg, ch.bn, a_mn ? 1 : 0, b_mn ? 1 : 0, f32 ? nrl::tc::EPI_F32 : residual.has_value() ? nrl::tc::EPI_RESIDUAL : nrl::tc::EPI_BF16, num_sms(),
                     cur_stream()), "gemm_tc (no kernel instantiated for this cg / block_n / operand-major combination?)");
   return out;
 }
@@ -1554,7 +1562,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc", &gemm_tc, py::arg("a"), py::arg("b"), py::arg("a_mn") = false, py::arg("b_mn") = false, py::arg("a2") = py::none(),
         py::arg("b2") = py::none(), py::arg("bias") = py::none(), py::arg("act") = 0, py::arg("alpha") = 1.0, py::arg("out") = py::none(),
         py::arg("out_f32") = py::none(), py::arg("accumulate") = false, py::arg("cg") = 0, py::arg("block_n") = 0,
-        py::arg("split_k") = -1);      // -1 = automatic, 0 = never, n = exactly n k-ranges
+        py::arg("split_k") = -1, py::arg("residual") = py::none());      // split_k: -1 = automatic, 0 = never, n = exactly n k-ranges
   m.def("gemm_tc_fp8", &gemm_tc_fp8, py::arg("aq"), py::arg("a_scale"), py::arg("bq"), py::arg("b_scale"), py::arg("bias") = py::none(),
         py::arg("swiglu") = false, py::arg("cg") = 0, py::arg("block_n") = 0);
   m.def("gemm_tc_batched", &gemm_tc_batched, py::arg("a"), py::arg("b"), py::arg("out") = py::none(), py::arg("cg") = 0, py::arg("block_n") = 0);

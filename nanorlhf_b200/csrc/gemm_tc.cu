@@ -743,6 +743,17 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           if (cl < p.N) gate_scale = __ldg(p.col_scale + cl);
           if (cl + 32 < p.N) up_scale = __ldg(p.col_scale + cl + 32);
         }
+        // A residual is read a row per thread as whole sectors, ahead of the sums: 128 bytes in 0.4 us that a tile's epilogue
+        // has to spare.  A form of its own: behind a run-time branch of the plain one it cost other GEMMs 2 %.
+        constexpr bool kResidual = EPI == EPI_RESIDUAL;
+        uint4 rs[8];
+        if (kResidual && row_ok) {
+          const int cl = c.n_blk * BN + ch * 64;
+          const uint4* from = reinterpret_cast<const uint4*>(p.residual + static_cast<long>(row) * p.residual_stride + cl);
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (cl + q * 8 < p.N) rs[q] = __ldg(from + q);
+        }
         tmem_ld_32x32b_x32(t_acc + ch * 64, v[0]);
         tmem_ld_32x32b_x32(t_acc + ch * 64 + 32, v[1]);
         tmem_ld_wait();
@@ -863,6 +874,14 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) packed[j / 2 + e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
+            if (kResidual) {       // rounded, then added and rounded, as by a kernel of its own
+              const uint32_t r[4] = {rs[j / 8].x, rs[j / 8].y, rs[j / 8].z, rs[j / 8].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 y = unpack_bf16x2(packed[j / 2 + e]), z = unpack_bf16x2(r[e]);
+                packed[j / 2 + e] = pack_bf16x2(y.x + z.x, y.y + z.y);
+              }
+            }
           }
           if (col0 < n_cols && m_blk * BLOCK_M + quad * 32 < p.M) store_slab_to(CAT ? more + 3 * kCatMax + which : &tmD, packed, col0, m_blk * BLOCK_M + quad * 32, bidx);
         }
@@ -1511,6 +1530,13 @@ extern "C" cudaError_t nrl_gemm_tc(const CUtensorMap* maps, const nrl::tc::TcPar
   NRL_TC_CASE(2, 128, false, false, EPI_BF16)
   NRL_TC_CASE(2, 192, false, false, EPI_BF16)
   NRL_TC_CASE(2, 256, false, false, EPI_BF16)
+  NRL_TC_CASE(1, 64, false, false, EPI_RESIDUAL)
+  NRL_TC_CASE(1, 128, false, false, EPI_RESIDUAL)
+  NRL_TC_CASE(1, 192, false, false, EPI_RESIDUAL)
+  NRL_TC_CASE(1, 256, false, false, EPI_RESIDUAL)
+  NRL_TC_CASE(2, 128, false, false, EPI_RESIDUAL)
+  NRL_TC_CASE(2, 192, false, false, EPI_RESIDUAL)
+  NRL_TC_CASE(2, 256, false, false, EPI_RESIDUAL)
   NRL_TC_CASE(1, 128, false, false, EPI_SWIGLU)
   NRL_TC_CASE(1, 256, false, false, EPI_SWIGLU)
   NRL_TC_CASE(2, 128, false, false, EPI_SWIGLU)

@@ -16,6 +16,7 @@ enum TcEpilogue : int {
   EPI_SWIGLU_KEEP = 6,  // PAIR kernels: as EPI_SWIGLU, and gate and up (bf16, TMA store)
   EPI_DSWIGLU = 7,   // D, D2 (bf16, TMA store) = gradients of gate and up, acc being that of silu(gate) * up
   EPI_LOGPROB = 8,   // out_f32 [2 col_ranges, M, 4] = statistics of a row over half a range's columns: max, sum of exp, sum of exp * logit, target's logit
+  EPI_RESIDUAL = 9,  // EPI_BF16 and a residual [M, N] added to the rounded result, K-major operands
   EPI_SWIGLU = 2,    // D[M, N/2] (bf16, TMA store) = silu(gate) * up; B rows interleaved per 32 features [32 gate | 32 up]
 };
 
@@ -48,6 +49,8 @@ struct TcParams {
   int batch;                    // BATCH kernels: number of independent [M,K] x [N,K]^T problems behind 3D tensor maps (else 1)
   float alpha;                  // multiplies the accumulator
   const __nv_bfloat16* bias;    // EPI_BF16: optional [N]
+  const __nv_bfloat16* residual;      // EPI_RESIDUAL: [M, N], row stride residual_stride
+  long residual_stride;
   int act;                      // EPI_BF16: 0 = none, 1 = exact (erf) GELU after the bias (GROUPED: see below)
   float* logits;                // EPI_LOGPROB: null, or [M, N] for the accumulator
   float* out_f32;               // EPI_F32: [M, N] fp32, row stride out_f32_stride elements

@@ -148,16 +148,21 @@ class Qwen2MLP(nn.Module):
         self.up_proj = Linear(cfg.hidden_size, cfg.intermediate_size, bias=False)
         self.down_proj = Linear(cfg.intermediate_size, cfg.hidden_size, bias=False)
 
-    def forward(self, x):
-        from .lora import fused_mlp_forward, fused_swiglu_forward, lora_group_forward
+    def forward(self, x, residual=None):
+        from .lora import add_linear_forward, fused_mlp_forward, fused_swiglu_forward, lora_group_forward
         y = fused_mlp_forward(x, self.gate_proj, self.up_proj, self.down_proj)
         if y is not None:
-            return y
+            return y if residual is None else residual + y
         act = fused_swiglu_forward(x, self.gate_proj, self.up_proj)
-        if act is not None:
+        if act is None:
+            gate, up = lora_group_forward(x, [self.gate_proj, self.up_proj])
+            act = ops.swiglu_pair(gate, up)
+        if residual is None:
             return self.down_proj(act)
-        gate, up = lora_group_forward(x, [self.gate_proj, self.up_proj])
-        return self.down_proj(ops.swiglu_pair(gate, up))
+        y = add_linear_forward(act, self.down_proj, residual)
+        return residual + self.down_proj(act) if y is None else y
+
+    plain_forward = forward              # what a call with the residual may stand in for (lora.plain_module)
 
 
 class Qwen2DecoderLayer(nn.Module):
@@ -175,7 +180,7 @@ class Qwen2DecoderLayer(nn.Module):
         if (ops.direct_calls() and ops.use_native(h) and h.dim() == 2 and plain_module(norm, RMSNorm)
                 and h.dtype == a.dtype == norm.weight.dtype == torch.bfloat16):
             y, h = ops.add_rmsnorm(a, h, norm.weight, norm.eps)          # residual add and norm in one pass
-            return h + self.mlp(y)
+            return self.mlp(y, h) if plain_module(self.mlp, Qwen2MLP) else h + self.mlp(y)
         h = h + a
         h = h + self.mlp(self.post_attention_layernorm(h))
         return h

@@ -44,11 +44,11 @@ def _rows(x: torch.Tensor) -> torch.Tensor:
 
 
 def gemm(a, b, a_mn=False, b_mn=False, a2=None, b2=None, bias=None, act=0, alpha=1.0, out=None, out_f32=None,
-         accumulate=False, cg=0, block_n=0, split_k=-1):
+         accumulate=False, cg=0, block_n=0, split_k=-1, residual=None):
     """Thin wrapper over ``_C.gemm_tc`` (see csrc/bindings.cpp) that counts the launch."""
     _native_mod._count()
     return _native_mod.ext().gemm_tc(a, b, a_mn, b_mn, a2, b2, bias, act, alpha, out, out_f32, accumulate, cg, block_n,
-                                     split_k)
+                                     split_k, residual)
 
 
 class _LinearFn(torch.autograd.Function):
@@ -253,6 +253,17 @@ class _LoraMlpFn(torch.autograd.Function):
         dgate, dup = _native_mod.ext().gemm_tc_dswiglu(g2, wd, tpd, ad, gate, up)
         gx, ga_cat, (gbg, gbu), (gbd, gad) = _group_backward([dgate, dup], x2, t_cat, a_cat, [wg, wu], [bg, bu], s, ctx.needs_input_grad[0], [(g2, td)], [(tpd, act)])
         return (gx.view(xshape) if gx is not None else None, None, None, ga_cat[:r], gbg, None, ga_cat[r:], gbu, None, gad, gbd)
+
+
+def linear_add(x, w, residual, a=None, b=None, scaling: float = 0.0):
+    """``residual + (x W^T + scaling (x A^T) B^T)`` without autograd, the sum in brackets rounded to bf16 as by its own GEMM; None where that GEMM does
+    not apply."""
+    if (x.numel() == 0 or not (supported(x, w) if a is None else lora_supported(x, w, a, b))
+            or residual.dtype != torch.bfloat16 or residual.shape != (*x.shape[:-1], w.shape[0]) or residual.device != x.device):
+        return None
+    x2 = _rows(x)
+    t = None if a is None else gemm(x2, a, alpha=scaling)
+    return gemm(x2, w, a2=t, b2=b, residual=_rows(residual)).view(residual.shape)
 
 
 def lora_mlp(x, gate, up, down, scaling: float):
