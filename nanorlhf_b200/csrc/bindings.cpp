@@ -183,7 +183,7 @@ int64_t split_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits) {
 // taken; 256 15.0 / 14.1 not taken.  18 944, 256 x 3584 42.9 / 34.7 (256, four), 512 61.0 / 58.3.  4096, 1024 x 1024 14.1 / 13.8; 1536, 1024 x 1536 9.5 / 11.1 not taken.  151 936
 // (through a workspace, 256 wide): 300 x 1536 160 / 175 not taken; 400 206 / 182 (five), 768 305 / 251 (four), 1000 484 / 327 (three), 1300 514 / 482 (four), 1600 698 / 586
 // (five), 2000 777 / 635 (three), 3000 958 uncut, 3800 1549 / 1271 (four), 5000 1911 / 1734 (three).
-struct PairCut { int bn, splits; bool clusters; };       // splits 1: not taken
+struct PairCut { int bn, splits; bool clusters; int64_t single; };       // splits 1: not taken; single: split_choice, 0 where it was not asked
 inline double pair_block_us(int bn, double load) {
   const double light = bn == 128 ? 0.2 : bn == 192 ? 0.26 : 0.314, full = bn == 128 ? 0.23 : bn == 192 ? 0.33 : 0.41;
   return light + (full - light) * std::min(1.0, load);
@@ -193,10 +193,12 @@ constexpr int64_t kPairWorkspaceMax = 128 << 20;         // bytes
 template <class Fits, class PairFits>
 PairCut pair_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits, PairFits pair_fits) {
   const int64_t blocks = (K + 63) / 64, units = sms / 2, num_m = (M + 255) / 256;
-  PairCut best{0, 1, false};
+  PairCut best{0, 1, false, 0};
   if (N <= 64 || blocks < 16 || units < 1) return best;
   // the form that is taken otherwise
+  auto column_tiles = [&](int bn) { return static_cast<int>(bn == 128 ? (N + 127) >> 7 : bn == 256 ? (N + 255) >> 8 : (N + 191) / 192); };
   const int64_t tiles1 = split_tiles(M, N), s1 = split_choice(M, N, K, sms, fits);
+  best.single = s1;
   double other;
   if (s1 > 1) {
     const bool clusters = nrl::tc::split_by_clusters(static_cast<int>(s1), blocks) && tiles1 <= fits(static_cast<int>(s1));
@@ -210,16 +212,21 @@ PairCut pair_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits, Pai
     }
   }
   double least = 0.96 * other;
-  for (int bn : {128, 192, 256}) {
-    const int64_t tiles = num_m * ((N + bn - 1) / bn);
-    for (int64_t s = 2; s <= 8 && blocks >= 4 * s; ++s) {
-      if (split_ranges(blocks, s) != s) continue;
-      const bool clusters = s <= 4 && tiles <= pair_fits(bn, static_cast<int>(s));
-      if (!clusters && (blocks <= 512 || s * tiles * 256 * bn * 4 > kPairWorkspaceMax)) continue;
-      const int64_t waves = (tiles * s + units - 1) / units;
-      const double loop = pair_block_us(bn, static_cast<double>(tiles * s) / (waves * units)) * ((blocks + s - 1) / s), start = bn == 256 ? 4.5 : 4.0;
+  // by number of ranges outside, so that its divisions are made once, and of int; this is run for every product.  Short contractions are cut by clusters only.
+  const int nb = static_cast<int>(blocks), nu = static_cast<int>(units), top = nb <= 512 ? 4 : 8;
+  int tiles_of[3], n = 0;
+  for (int bn : {128, 192, 256}) tiles_of[n++] = static_cast<int>(num_m) * column_tiles(bn);
+  for (int s = 2; s <= top && nb >= 4 * s; ++s) {
+    const int per = (nb + s - 1) / s;
+    if ((nb + per - 1) / per != s) continue;               // comes as a smaller number
+    for (int i = 0; i < 3; ++i) {
+      const int bn = 128 + 64 * i, tiles = tiles_of[i];
+      const bool clusters = s <= 4 && tiles <= pair_fits(bn, s);
+      if (!clusters && (nb <= 512 || static_cast<int64_t>(s) * tiles * 256 * bn * 4 > kPairWorkspaceMax)) continue;
+      const int waves = (tiles * s + nu - 1) / nu;
+      const double loop = pair_block_us(bn, static_cast<double>(tiles * s) / (waves * nu)) * per, start = bn == 256 ? 4.5 : 4.0;
       const double t = clusters ? loop + start + (s == 2 ? 1.8 : s == 3 ? 3.1 : 3.4) : waves * (loop + (bn == 128 ? 5.0 : bn == 192 ? 7.0 : 9.0)) + start;
-      if (t < least) { least = t; best = {bn, static_cast<int>(s), clusters}; }
+      if (t < least) { least = t; best = {bn, s, clusters, s1}; }
     }
   }
   return best;
@@ -232,7 +239,7 @@ PairCut auto_pairs(int64_t M, int64_t N, int64_t K) {
 int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
   const PairCut pc = auto_pairs(M, N, K);
   if (pc.splits > 1) return pc.splits;
-  return split_choice(M, N, K, num_sms(), [&](int s) { return nrl_gemm_tc_split_clusters(split_block_n(N), s); });
+  return pc.single > 0 ? pc.single : split_choice(M, N, K, num_sms(), [&](int s) { return nrl_gemm_tc_split_clusters(split_block_n(N), s); });
 }
 
 // D[M,N] = alpha * (opA(a) opB(b)^T + opA(a2) opB(b2)^T) (+bias) (GELU).
@@ -277,9 +284,11 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
   }
   if (M == 0 || N == 0) return out;
   // ---- split-K: few output tiles, long contraction (rank-r projections, LoRA weight gradients) ----
+  int64_t single = 0;                                      // split_choice, where auto_pairs has asked it
   const bool bias_ok = !bias.has_value() || ((reinterpret_cast<uintptr_t>(bias->data_ptr()) & 15) == 0 && bias->is_contiguous());
   if (K2 == 0 && !f32 && bias_ok && act == 0 && !a_mn && splitk_req != 0 && (cg_req == 2 ? bn_req > 0 && splitk_req > 1 : cg_req <= 0 && bn_req <= 0 && splitk_req < 0)) {
     PairCut pc = auto_pairs(M, N, K);
+    single = pc.single;
     if (cg_req == 2) {                                     // asked for: by clusters where they fit
       pc.bn = static_cast<int>(bn_req);
       pc.splits = static_cast<int>(split_ranges((K + 63) / 64, std::min<int64_t>(splitk_req, (K + 63) / 64)));
@@ -315,7 +324,7 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
     const int bn = split_block_n(N);
     const int64_t tiles = split_tiles(M, N), num_kb = (K + 63) / 64;
     const int sms = num_sms();
-    int64_t splits = splitk_req > 0 ? splitk_req : split_choice(M, N, K, sms, [&](int s) { return nrl_gemm_tc_split_clusters(bn, s); });
+    int64_t splits = splitk_req > 0 ? splitk_req : single > 0 ? single : split_choice(M, N, K, sms, [&](int s) { return nrl_gemm_tc_split_clusters(bn, s); });
     if (splitk_req > 0 || splits > 1) {
       splits = std::max<int64_t>(1, std::min<int64_t>(splits, num_kb));
       splits = split_ranges(num_kb, splits);

@@ -215,7 +215,7 @@ NRL_DEVICE void warp_rows_out(uint8_t* slab, const uint32_t (&w)[W], int lane, F
 // weight, its peer the same 128 rows of the up weight, so the accumulator's halves are gate and up of the same features; the adapters'
 // columns follow (first the gate's, then the up's), each weight taking zeros (rows behind its end) for the other's.
 template <int CG, int BN, bool A_MN, bool B_MN, int EPI, bool SPLIT = false, bool BATCH = false, bool FP8 = false, bool GROUPED = false,
-          bool PAIR = false, bool CLUSTER = false, bool SUM = false, bool CAT = false>
+          bool PAIR = false, bool CLUSTER = false, bool SUM = false, bool CAT = false, bool MULTI = false>
 NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
                              const CUtensorMap& tmD, const TcParams& p, const CUtensorMap* more = nullptr, int unit0 = 0, const TcCat* cat = nullptr) {
   // more: PAIR the up adapter's columns, then (EPI_SWIGLU_KEEP) gate and up; EPI_DSWIGLU gate, up, d up; SUM kSumPairs maps of A and as many of B;
@@ -933,7 +933,7 @@ NRL_DEVICE void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB, con
           acc[2 * e + 1] += bf.y;
         }
       }
-      if (p.transposed) {                                  // neighbouring threads hold neighbouring rows
+      if (MULTI && p.transposed) {                         // neighbouring threads hold neighbouring rows
 #pragma unroll
         for (int e = 0; e < 8; ++e) p.out_bf16[static_cast<long>(col + e) * p.out_stride + row] = __float2bfloat16(acc[e]);
         continue;
@@ -1195,7 +1195,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_multi_kernel(const __grid
   p.out_bf16 = m.out[i];
   p.out_stride = m.stride[i];
   p.transposed = m.transposed[i];
-  gemm_tc_body<1, 64, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true>(m.a[i], m.b[i], m.a[i], m.b[i], m.a[i], p, nullptr,
+  gemm_tc_body<1, 64, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true, false, false, true>(m.a[i], m.b[i], m.a[i], m.b[i], m.a[i], p, nullptr,
                                                                                    i > 0 ? m.tiles[i - 1] * splits : 0);
 }
 template <bool A_MN, bool B_MN>

@@ -16,6 +16,9 @@ sm_100a kernel, with the operand "major-ness" chosen so that no transposed copy 
  LoRA wgrad         dA = t'^T x,  dB = dy^T t                  MN-major x MN-major (rank-r outputs)
 =================  =========================================  =====================================================
 
+Projections of one input share a launch (``_projections``), so do the products whose sum is that input's gradient (``sum_gemms``) and the narrow
+gradients of a group's factors (``_adapter_grads``).
+
 Tensors whose shape the kernel cannot address (inner extents not multiples of 8, mis-aligned rows) and non-bf16 /
 non-CUDA tensors take the PyTorch path; a bf16 CUDA tensor of a supported shape never falls back silently.
 """
@@ -197,9 +200,8 @@ def _projections(x2, ws, bs, ts=(), Bs=()):
 
 class _LoraGroupFn(torch.autograd.Function):
     """Several LoRA projections of ONE input (q / k / v, gate / up): the rank-r down-projections share a launch
-    (``t = s x [A_1; ...; A_n]^T``), each base GEMM takes its slice of ``t`` as dual-source-K operand, and in the backward the
-    adapter-input gradients ``dA_i`` come out of one GEMM over the concatenated ``t'`` and ``dx`` out of one over all projections and the
-    LoRA term.  Compared with n independent ``_LoraLinearFn``: n - 1 fewer skinny launches per direction, ``x`` is re-read once instead of n times."""
+    (``t = s x [A_1; ...; A_n]^T``), the base GEMMs share another and take their slices of ``t`` as dual-source-K operands, and in the backward the
+    gradients of all factors come out of one launch and ``dx`` out of one over all projections and the LoRA term.  Compared with n independent ``_LoraLinearFn``: n - 1 fewer skinny launches per direction, ``x`` is re-read once instead of n times."""
 
     @staticmethod
     def forward(ctx, x, scaling, n, *flat):
