@@ -226,10 +226,9 @@ def _adapter_in_gemm(m) -> bool:
 
 
 def lora_group_forward(x, mods):
-    """``[m(x) for m in mods]`` for projections that share their input; when all of them are plain LoRA layers with the
+    """``[m(x) for m in mods]`` for projections that share their input; when all of them are plain LoRA layers (``plain_module``) with the
     same rank / scaling their rank-r projections run as one launch (ops.lora_linear_group), and their own as another; so do plain layers outside autograd."""
-    if (len(mods) > 1 and all(isinstance(m, LoraLinear) for m in mods)
-            and all(_adapter_in_gemm(m) for m in mods)
+    if (len(mods) > 1 and all(plain_module(m, LoraLinear) and _adapter_in_gemm(m) for m in mods)
             and len({(m.r, m.scaling) for m in mods}) == 1):
         return ops.lora_linear_group(x, [(m.base_layer.weight, m.base_layer.bias, m.lora_A.weight, m.lora_B.weight) for m in mods],
                                      mods[0].scaling)
