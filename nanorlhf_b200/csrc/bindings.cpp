@@ -5,6 +5,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/SavedTensorHooks.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -817,20 +818,36 @@ int pick_splits(int64_t M, int64_t N, int bn, bool pairs) {
 bool head_pairs(int64_t M) { return 12 * ((M + 255) / 256) <= 7 * ((M + 127) / 128); }
 
 // A [M, V] float buffer in which the head's forward leaves its logits for the backward, which then reads them instead of forming the product once more; none where
-// that is not wanted: above 4 GiB, where allocations of twice the size would leave less than a quarter of the device's memory unallocated, under hooks that would carry
-// the saved tensor elsewhere, and where the allocator does not say what it has handed out.  The gradients are the same bits either way.
+// that is not wanted: above 4 GiB, where it would take memory that the rest of a step may need (keeps_logits), and under hooks that would carry the saved tensor
+// elsewhere.  The gradients are the same bits either way.
 // 151 936 columns, forward and backward in a row (us), the product formed again / logits kept: 100 rows 441 / 375, 300 rows 714 / 606, 1000 rows 1560 / 1357,
-// 2000 rows 2990 / 2634, 6001 rows 8515 / 7440, for 3.6 GB of float more from the forward to the end of the backward.  The stores cost the forward 20 us up to 512
-// rows, 270 of 1759 at 6001.
+// 2000 rows 2990 / 2634, 6001 rows 8515 / 7440.  The stores cost the forward 20 us up to 512 rows, 270 of 1759 at 6001.  The price is 3.6 GB of float at 6001 rows
+// from the forward to the end of the backward; of a step that is captured into a graph, the graph's pool keeps them for as long as the graph lives.  The 4 GiB bound
+// that price, not the gain, which grows with the rows.
 constexpr int64_t kKeptLogitsMax = 4ll << 30;
+// `taken` bytes of the device's `total` are held by somebody: a quarter stays beside the logits and the backward's bf16 gradient of them, with as much again to spare
+bool keeps_logits(int64_t M, int64_t V, int64_t taken, int64_t total) {
+  return M > 0 && V > 0 && V % 8 == 0 && M <= kKeptLogitsMax / 4 / V && taken <= total / 4 * 3 - 8 * M * V;
+}
 c10::optional<torch::Tensor> lmhead_logits_buffer(const torch::Tensor& hidden, int64_t V) {
   const int64_t M = hidden.size(0);
-  if (M == 0 || V % 8 != 0 || M > kKeptLogitsMax / 4 / V || at::SavedTensorDefaultHooks::get_hooks().has_value()) return c10::nullopt;
+  if (!keeps_logits(M, V, 0, INT64_MAX) || at::SavedTensorDefaultHooks::get_hooks().has_value()) return c10::nullopt;
   c10::cuda::CUDAGuard guard(hidden.device());
   try {
-    const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(hidden.device().index());
-    const int64_t total = at::cuda::getCurrentDeviceProperties()->totalGlobalMem;
-    if (stats.allocated_bytes[0].current + 8 * M * V > total / 4 * 3) return c10::nullopt;
+    // What the allocator has reserved counts as taken, handed out or not: blocks that wait in a captured graph's pool serve nobody else.
+    int64_t total = at::cuda::getCurrentDeviceProperties()->totalGlobalMem;
+    int64_t taken = c10::cuda::CUDACachingAllocator::getDeviceStats(hidden.device().index()).reserved_bytes[0].current;
+    if (4 * M * V >= (256 << 20)) {      // worth the 73 us in which the driver tells what others hold too: other processes, communicators, the context
+      c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};
+      size_t free_bytes = 0, all = 0;
+      if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) {
+        cudaGetLastError();
+        return c10::nullopt;
+      }
+      total = static_cast<int64_t>(all);
+      taken = total - static_cast<int64_t>(free_bytes);
+    }
+    if (!keeps_logits(M, V, taken, total)) return c10::nullopt;
     return torch::empty({M, V}, hidden.options().dtype(torch::kFloat32));
   } catch (const c10::Error&) {
     return c10::nullopt;
@@ -1604,6 +1621,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("inv_temperature"), py::arg("n_splits") = 0, py::arg("logits") = py::none());
   m.def("lmhead_dlogits", &lmhead_dlogits);
   m.def("lmhead_logits_buffer", &lmhead_logits_buffer);
+  m.def("lmhead_keeps_logits", &keeps_logits, py::arg("M"), py::arg("V"), py::arg("taken"), py::arg("total"));
   m.def("logits_grad", &logits_grad);
   m.def("lora_merge", &lora_merge, py::arg("w"), py::arg("lora_a"), py::arg("lora_b"), py::arg("scale"), py::arg("out"),
         py::arg("mc_out_ptr") = 0);

@@ -178,7 +178,7 @@ def attention_varlen(q, k, v, cu_seqlens, max_seqlen=None, causal=True, scale=No
 # fused lm-head log-prob (K-LP)
 # --------------------------------------------------------------------------------------------
 class _LmHeadLogprobFn(torch.autograd.Function):
-    """Forward: tcgen05 GEMM with an online-softmax epilogue, which for a backward also leaves the float32 logits where they take up to 4 GiB of plenty
+    """Forward: tcgen05 GEMM with an online-softmax epilogue, which for a backward also leaves the float32 logits where they take up to 4 GiB and plenty is free
     (``lmhead_logits_buffer``; no [T, V] tensor otherwise).
     Backward: dZ in bf16 from those logits, or from the same mainloop, which forms them again (one 8192-row chunk at a
     time); dH = dZ W (K-major x MN-major) and dW += dZ^T H (MN-major x MN-major, fp32 accumulate across chunks in the
