@@ -15,6 +15,7 @@
 
 #include "gemm_sm100.h"
 #include "gemm_tc.h"
+#include "per_device.h"
 #include "kernels.h"
 #include "runtime.h"
 #include "bindings_hybrid.h"
@@ -232,15 +233,44 @@ PairCut pair_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits, Pai
   }
   return best;
 }
-PairCut auto_pairs(int64_t M, int64_t N, int64_t K) {
-  return pair_choice(M, N, K, num_sms(), [&](int s) { return nrl_gemm_tc_split_clusters(split_block_n(N), s); },
-                     [](int bn, int s) { return nrl_gemm_tc_pair_clusters(bn, s); });
+// clusters that the current device runs at a time, asked once: blocks by themselves (64, 128 columns; up to eight), pairs (128, 192, 256; up to four), blocks of the
+// grouped kernel (A K-major, MN-major)
+struct ClusterFits {
+  bool known;
+  int single[2][9], pairs[3][5], multi[2][9];
+  int blocks(int bn, int s) const { return single[bn == 64 ? 0 : 1][s]; }
+  int of_pairs(int bn, int s) const { return s <= 4 ? pairs[(bn - 128) / 64][s] : 0; }
+};
+const ClusterFits& cluster_fits() {
+  static nrl::PerDevice<ClusterFits> all;
+  ClusterFits& f = all.here();
+  if (!f.known) {
+    for (int s = 2; s <= 8; ++s)
+      for (int i = 0; i < 2; ++i) f.single[i][s] = nrl_gemm_tc_split_clusters(64 << i, s);
+    for (int s = 2; s <= 4; ++s)
+      for (int i = 0; i < 3; ++i) f.pairs[i][s] = nrl_gemm_tc_pair_clusters(128 + 64 * i, s);
+    for (int s = 1; s <= 8; ++s)
+      for (int i = 0; i < 2; ++i) f.multi[i][s] = nrl_gemm_tc_multi_clusters(i, s);
+    f.known = true;
+  }
+  return f;
 }
-// ranges of the contraction that gemm_tc adds up for a product with a K-major A, 1: none
-int64_t auto_splits(int64_t M, int64_t N, int64_t K) {
+int64_t auto_single(int64_t M, int64_t N, int64_t K) {
+  const ClusterFits& f = cluster_fits();
+  const int bn = split_block_n(N);
+  return split_choice(M, N, K, num_sms(), [&](int s) { return f.blocks(bn, s); });
+}
+PairCut auto_pairs(int64_t M, int64_t N, int64_t K) {
+  const ClusterFits& f = cluster_fits();
+  const int bn = split_block_n(N);
+  return pair_choice(M, N, K, num_sms(), [&](int s) { return f.blocks(bn, s); }, [&](int w, int s) { return f.of_pairs(w, s); });
+}
+// ranges of the contraction that gemm_tc adds up on `device` (-1: the current one) for a product with a K-major A, 1: none
+int64_t auto_splits(int64_t M, int64_t N, int64_t K, int64_t device) {
+  const c10::cuda::OptionalCUDAGuard guard(device >= 0 ? c10::optional<c10::DeviceIndex>(static_cast<c10::DeviceIndex>(device)) : c10::nullopt);
   const PairCut pc = auto_pairs(M, N, K);
   if (pc.splits > 1) return pc.splits;
-  return pc.single > 0 ? pc.single : split_choice(M, N, K, num_sms(), [&](int s) { return nrl_gemm_tc_split_clusters(split_block_n(N), s); });
+  return pc.single > 0 ? pc.single : auto_single(M, N, K);
 }
 
 // D[M,N] = alpha * (opA(a) opB(b)^T + opA(a2) opB(b2)^T) (+bias) (GELU).
@@ -325,7 +355,7 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
     const int bn = split_block_n(N);
     const int64_t tiles = split_tiles(M, N), num_kb = (K + 63) / 64;
     const int sms = num_sms();
-    int64_t splits = splitk_req > 0 ? splitk_req : single > 0 ? single : split_choice(M, N, K, sms, [&](int s) { return nrl_gemm_tc_split_clusters(bn, s); });
+    int64_t splits = splitk_req > 0 ? splitk_req : single > 0 ? single : auto_single(M, N, K);
     if (splitk_req > 0 || splits > 1) {
       splits = std::max<int64_t>(1, std::min<int64_t>(splits, num_kb));
       splits = split_ranges(num_kb, splits);
@@ -456,7 +486,7 @@ void gemm_tc_multi(const std::vector<torch::Tensor>& a, const std::vector<torch:
     tiles.push_back(((M + 127) / 128) * ((N + 63) / 64));
     blocks.push_back((K + 63) / 64);
   }
-  const int64_t splits = splits_req > 0 ? splits_req : multi_splits(tiles, blocks, num_sms(), [&](int s) { return nrl_gemm_tc_multi_clusters(a_mn ? 1 : 0, s); });
+  const int64_t splits = splits_req > 0 ? splits_req : multi_splits(tiles, blocks, num_sms(), [&](int s) { return cluster_fits().multi[a_mn ? 1 : 0][s]; });
   for (int64_t x : blocks) TORCH_CHECK(split_ranges(x, splits) == splits, "gemm_tc_multi: an empty range");
   check(nrl_gemm_tc_multi(maps, q, static_cast<int>(n), a_mn ? 1 : 0, static_cast<int>(splits), cur_stream()), "gemm_tc_multi");
 }
@@ -1594,7 +1624,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_batched", &gemm_tc_batched, py::arg("a"), py::arg("b"), py::arg("out") = py::none(), py::arg("cg") = 0, py::arg("block_n") = 0);
   m.def("gemm_tc_swiglu", &gemm_tc_swiglu, py::arg("a"), py::arg("w_interleaved"), py::arg("out") = py::none(), py::arg("cg") = 0,
         py::arg("block_n") = 0);
-  m.def("gemm_tc_auto_splits", &auto_splits, py::arg("M"), py::arg("N"), py::arg("K"));
+  m.def("gemm_tc_auto_splits", &auto_splits, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("device") = -1);
   m.def("gemm_tc_split_choice", [](int64_t M, int64_t N, int64_t K, int64_t sms, const std::vector<int>& fits) {
     return split_choice(M, N, K, sms, [&](int s) { return fits.at(s); });
   }, "split_choice for a GPU of `sms` SMs that runs fits[s] clusters of s blocks at a time");

@@ -33,6 +33,7 @@
 #include "common.cuh"
 #include "gemm_tc.h"
 #include "launch.h"
+#include "per_device.h"
 
 namespace nrl {
 namespace tc {
@@ -1004,12 +1005,8 @@ template <int BN>
 static cudaError_t launch_sum(const TcMaps8& maps, const CUtensorMap& tmD, const TcParams& p, int num_sms, cudaStream_t stream) {
   using C = Cfg<2, BN, true>;
   auto kern = gemm_tc_sum_kernel<BN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   int units = ((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;
@@ -1036,12 +1033,8 @@ template <int CG, int BN>
 static cudaError_t launch_cat(const CUtensorMap& tmA, const TcMaps16& maps, const TcParams& p, const TcCat& cat, int num_sms, cudaStream_t stream) {
   using C = Cfg<CG, BN>;
   auto kern = CG == 2 ? gemm_tc_cat_cg2_kernel<BN> : gemm_tc_cat_cg1_kernel<BN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   int units = (p.M + CG * BLOCK_M - 1) / (CG * BLOCK_M) * cat.end[kCatMax - 1];
   if (units > num_sms / CG) units = num_sms / CG;
   if (units < 1) units = 1;
@@ -1059,12 +1052,8 @@ template <int BN, int FORM>
 static cudaError_t launch_grouped_form(const CUtensorMap* maps, const TcParams& p, int units, cudaStream_t stream) {
   using C = Cfg<1, BN, false>;
   auto kern = gemm_tc_grouped_kernel<BN, FORM>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   launch_dependent(kern, units, kThreads, C::kTotal, stream, maps[0], maps[1], p);
   return cudaGetLastError();
 }
@@ -1110,22 +1099,14 @@ static cudaError_t launch_fp8(const CUtensorMap* maps, const TcParams& p, int nu
   int units = num_m * num_n;
   if (units > num_sms / CG) units = num_sms / CG;
   if (units < 1) units = 1;
-  static bool configured = false;
+  static nrl::PerDevice<bool> configured;
   if (CG == 1) {
     auto kern = gemm_tc_fp8_cg1_kernel<BN, EPI>;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
     launch_dependent(kern, units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   } else {
     auto kern = gemm_tc_fp8_cg2_kernel<BN, EPI>;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
     launch_dependent(kern, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   }
   return cudaGetLastError();
@@ -1138,22 +1119,14 @@ static cudaError_t launch_batched(const CUtensorMap* maps, const TcParams& p, in
   long units = static_cast<long>(num_m) * num_n * p.batch;
   if (units > num_sms / CG) units = num_sms / CG;
   if (units < 1) units = 1;
-  static bool configured = false;
+  static nrl::PerDevice<bool> configured;
   if (CG == 1) {
     auto kern = gemm_tc_batched_cg1_kernel<BN>;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
     launch_dependent(kern, static_cast<int>(units), kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   } else {
     auto kern = gemm_tc_batched_cg2_kernel<BN>;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
     launch_dependent(kern, static_cast<int>(2 * units), kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], p);
   }
   return cudaGetLastError();
@@ -1171,6 +1144,18 @@ template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
   gemm_tc_body<1, BN, A_MN, B_MN, EPI_BF16, true, false, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
+}
+
+struct ClusterCounts { int plus_one[kMaxClusterSplits + 1]; };               // 0: not asked yet
+// clusters of `blocks` blocks of a kernel that the current device runs at a time; the kernel may then use its shared memory there
+template <class Kernel>
+static int clusters_of(nrl::PerDevice<ClusterCounts>& counts, Kernel kernel, int smem, int blocks) {
+  int& n = counts.here().plus_one[blocks];
+  if (n == 0) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    n = 1 + (e == cudaSuccess ? clusters_at_a_time(kernel, kThreads, smem, blocks) : 0);
+  }
+  return n - 1;
 }
 
 // Several products with results at most a few tiles wide (the adapters' factors and inputs) in one launch: each of them alone leaves SMs idle and starts and
@@ -1201,13 +1186,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_multi_kernel(const __grid
 template <bool A_MN, bool B_MN>
 static int multi_clusters(int splits) {
   if (splits < 1 || splits > kMaxClusterSplits) return 0;
-  static int fits[kMaxClusterSplits + 1] = {};             // plus one
-  if (fits[splits] == 0) {
-    auto kern = gemm_tc_multi_kernel<A_MN, B_MN>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1, 64, B_MN>::kTotal);
-    fits[splits] = 1 + (e == cudaSuccess ? clusters_at_a_time(kern, kThreads, Cfg<1, 64, B_MN>::kTotal, splits) : 0);
-  }
-  return fits[splits] - 1;
+  static nrl::PerDevice<ClusterCounts> counts;
+  return clusters_of(counts, gemm_tc_multi_kernel<A_MN, B_MN>, Cfg<1, 64, B_MN>::kTotal, splits);
 }
 template <bool A_MN, bool B_MN>
 static cudaError_t launch_multi(const TcMulti& m, int n, int splits, cudaStream_t stream) {
@@ -1223,16 +1203,14 @@ gemm_tc_split_pairs_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
   static_assert(Cfg<2, BN, B_MN>::kStagingOff >= BLOCK_M * BN * 4, "a part takes the place of the operands");
   gemm_tc_body<2, BN, false, B_MN, EPI_BF16, true, false, false, false, false, true>(tmA, tmB, tmA, tmB, tmA, p);
 }
+static_assert(Cfg<2, 128, true>::kTotal > kSmemBudget / 2 && Cfg<2, 128, false>::kTotal > kSmemBudget / 2 && Cfg<2, 192, true>::kTotal > kSmemBudget / 2 &&
+              Cfg<2, 192, false>::kTotal > kSmemBudget / 2 && Cfg<2, 256, true>::kTotal > kSmemBudget / 2 && Cfg<2, 256, false>::kTotal > kSmemBudget / 2,
+              "one block per SM in either form of B: nrl_gemm_tc_pair_clusters asks for one");
 template <int BN, bool B_MN>
 static int split_pairs_clusters(int splits) {
   if (splits < 2 || 2 * splits > kMaxClusterSplits) return 0;
-  static int fits[kMaxClusterSplits / 2 + 1] = {};                           // plus one
-  if (fits[splits] == 0) {
-    auto kern = gemm_tc_split_pairs_kernel<BN, B_MN>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2, BN, B_MN>::kTotal);
-    fits[splits] = 1 + (e == cudaSuccess ? clusters_at_a_time(kern, kThreads, Cfg<2, BN, B_MN>::kTotal, 2 * splits) : 0);
-  }
-  return fits[splits] - 1;
+  static nrl::PerDevice<ClusterCounts> counts;
+  return clusters_of(counts, gemm_tc_split_pairs_kernel<BN, B_MN>, Cfg<2, BN, B_MN>::kTotal, 2 * splits);
 }
 // ... or passed through the workspace
 template <int BN, bool B_MN>
@@ -1251,12 +1229,8 @@ static cudaError_t launch_split_pairs(const CUtensorMap* maps, const TcParams& p
   }
   if (p.ws == nullptr || p.counters == nullptr) return cudaErrorInvalidValue;
   auto kern = gemm_tc_split_pairs_ws_kernel<BN, B_MN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   int units = tiles * p.splits;
   if (units > num_sms / 2) units = num_sms / 2;
   const bool early = p.K <= 32768;                         // as in launch()
@@ -1271,25 +1245,16 @@ template <int BN, bool A_MN, bool B_MN>
 static int splitk_clusters(int splits) {
   using C = Cfg<1, BN, B_MN>;
   if (splits < 2 || splits > kMaxClusterSplits) return 0;
-  static int fits[kMaxClusterSplits + 1] = {};                               // plus one
-  if (fits[splits] == 0) {
-    auto kern = gemm_tc_splitk_cluster_kernel<BN, A_MN, B_MN>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    fits[splits] = 1 + (e == cudaSuccess ? clusters_at_a_time(kern, kThreads, C::kTotal, splits) : 0);
-  }
-  return fits[splits] - 1;
+  static nrl::PerDevice<ClusterCounts> counts;
+  return clusters_of(counts, gemm_tc_splitk_cluster_kernel<BN, A_MN, B_MN>, C::kTotal, splits);
 }
 
 template <int BN, bool A_MN, bool B_MN>
 static cudaError_t launch_splitk(const CUtensorMap* maps, const TcParams& p, int num_sms, cudaStream_t stream) {
   using C = Cfg<1, BN, B_MN>;
   auto kern = gemm_tc_splitk_kernel<BN, A_MN, B_MN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   const int tiles = ((p.M + BLOCK_M - 1) / BLOCK_M) * ((p.N + BN - 1) / BN);
   int grid = tiles * p.splits;
   if (grid <= num_sms && split_by_clusters(p.splits, (p.K + BLOCK_K - 1) / BLOCK_K) && tiles <= splitk_clusters<BN, A_MN, B_MN>(p.splits)) {
@@ -1313,22 +1278,14 @@ static cudaError_t launch(const CUtensorMap* maps, const TcParams& p, int num_sm
   // backward (151 936 columns, 48 pairs of blocks) 1325 / 1309 us early / in order, 1000 rows 1470 / 1453, before overlapping launches 1310 / 1450; the line is
   // that of split_by_clusters, far from both sides' sizes (8960 columns, 18 to 74 pairs, gain).
   const bool early = p.K <= 32768;
-  static bool configured = false;
+  static nrl::PerDevice<bool> configured;
   if (CG == 1) {
     auto kern = gemm_tc_cg1_kernel<BN, A_MN, B_MN, EPI>;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
     launch_early_if(early, kern, units, kThreads, C::kTotal, stream, 0, maps[0], maps[1], maps[2], maps[3], maps[4], p);
   } else {
     auto kern = gemm_tc_cg2_kernel<BN, A_MN, B_MN, EPI>;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
     launch_early_if(early, kern, 2 * units, kThreads, C::kTotal, stream, 0, maps[0], maps[1], maps[2], maps[3], maps[4], p);   // consecutive CTAs pair up
   }
   return cudaGetLastError();
@@ -1370,12 +1327,8 @@ static cudaError_t launch_pair(const CUtensorMap* maps, const nrl::tc::TcParams&
   using namespace nrl::tc;
   using C = Cfg<2, 256, false>;
   auto kern = gemm_tc_pair_kernel<EPI>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   int units = ((p.M + 255) / 256) * ((p.N + 255) / 256);
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;
@@ -1391,12 +1344,8 @@ extern "C" cudaError_t nrl_gemm_tc_pair(const CUtensorMap* maps, const nrl::tc::
 extern "C" cudaError_t nrl_gemm_tc_dswiglu(const CUtensorMap* maps, const nrl::tc::TcParams* p, int num_sms, cudaStream_t stream) {
   using namespace nrl::tc;
   using C = Cfg<2, 256, true, 2>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_dswiglu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, gemm_tc_dswiglu_kernel, C::kTotal); e != cudaSuccess) return e;
   int units = ((p->M + 255) / 256) * ((p->N + 255) / 256);
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;

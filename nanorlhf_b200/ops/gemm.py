@@ -87,7 +87,7 @@ def linears(x, ws, bs):
     if x.numel() == 0 or not all(supported(x, w) for w in ws):
         return None
     x2 = _rows(x)
-    if any(_native_mod.ext().gemm_tc_auto_splits(x2.shape[0], *w.shape) > 1 for w in ws):
+    if any(_native_mod.ext().gemm_tc_auto_splits(x2.shape[0], *w.shape, x2.get_device()) > 1 for w in ws):
         return None
     return [y.view(*x.shape[:-1], y.shape[-1]) for y in _projections(x2, ws, bs)]
 
@@ -141,7 +141,7 @@ def sum_gemms(a, b):
     """``sum_i a[i] b[i]`` for the gradient of an input that several projections share: one launch with one float accumulator where none of the
     products would be cut into ranges of its contraction, else product by product, added in bf16."""
     pick = _native_mod.ext().gemm_tc_auto_splits
-    if len(a) <= 4 and all(pick(x.shape[0], y.shape[1], x.shape[1]) == 1 for x, y in zip(a, b)):
+    if len(a) <= 4 and all(pick(x.shape[0], y.shape[1], x.shape[1], x.get_device()) == 1 for x, y in zip(a, b)):
         _native_mod._count()
         return _native_mod.ext().gemm_tc_sum(a, b)
     out = gemm(a[0], b[0], b_mn=True, a2=a[-1], b2=b[-1])
@@ -297,7 +297,7 @@ def swiglu_linears(x, gate, up, scaling: float = 0.0):
     if x2.shape[0] == 0 or not (supported(x, wg) and supported(x, wu)) or wg.shape != wu.shape or (ag is None) != (au is None):
         return None
     if ag is None:
-        if _native_mod.ext().gemm_tc_auto_splits(x2.shape[0], *wg.shape) > 1:
+        if _native_mod.ext().gemm_tc_auto_splits(x2.shape[0], *wg.shape, x2.get_device()) > 1:
             return None                                # their own GEMMs would add up ranges of the contraction: other sums
         _native_mod._count()
         y = _native_mod.ext().gemm_tc_swiglu_pair(x2, wg, wu)
