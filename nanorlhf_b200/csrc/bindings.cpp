@@ -178,25 +178,27 @@ int64_t split_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits) {
 
 // ---- the same on pairs of CTAs (tiles of 256 rows): which form a product with a K-major A takes ----
 // A pair copies half as much of B per product as a block of its own, and copies bound these loops (65 bytes a clock and SM).  The time (us) of a block of 64 columns
-// in a tile `bn` wide grows with the share of the chip in use, up to the power cap.  With it and what the sums of the parts cost, each fitted to the sweep below, a
-// cut on pairs is taken where its estimate is 4 % below that of the form that is taken otherwise: by clusters, where those run at a time, or through a workspace, which
-// costs 5 to 9 us a round of the tiles, for contractions of more than 32 768 columns only (8960: 768 x 1536 22.8 / 22.9, 1024 30.1 / 31.0).
-// us without / with (rows x columns; contraction): 8960, 512 x 1536 21.2 / 20.4 (256 wide, four); 900 29.9 / 24.7 (192, two), 1024 30.1 / 24.8; 768 22.9 / 24.5 not
-// taken; 256 15.0 / 14.1 not taken.  18 944, 256 x 3584 42.9 / 34.7 (256, four), 512 61.0 / 58.3.  4096, 1024 x 1024 14.1 / 13.8; 1536, 1024 x 1536 9.5 / 11.1 not taken.  151 936
-// (through a workspace, 256 wide): 300 x 1536 160 / 175 not taken; 400 206 / 182 (five), 768 305 / 251 (four), 1000 484 / 327 (three), 1300 514 / 482 (four), 1600 698 / 586
-// (five), 2000 777 / 635 (three), 3000 958 uncut, 3800 1549 / 1271 (four), 5000 1911 / 1734 (three).
+// in a tile `bn` wide grows with the share of the chip in use, up to the power cap.  With it and what the sums of the parts cost, each fitted to sweeps, a cut on
+// pairs is taken where its estimate is 2 % below that of the form that is taken otherwise, which is up to 0.8 us too high: by clusters, where those run at a time,
+// or through a workspace for contractions of more than 32 768 columns, where all ranges run at once.  Ranges of a second round walk operands that the first no
+// longer holds in L2: 2000 x 896 over 151 936 columns 479 us uncut / 665 (128 wide, five, four rounds), 5000 x 1536 1817 / 2142.  Up to 128 rows half of a pair has
+// no work: 39 x 3584 over 1536 columns 8.2 / 9.1, 128 rows 8.5 / 9.3.
+// us without / with, weights from memory (rows x columns; contraction): 1536, 493 x 1536 8.8 / 9.0 and 2048, 545 x 1536 10.2 / 11.4 not taken; 2560, 212 x 3072
+// 11.5 / 10.8; 3584, 205 x 3072 13.7 / 12.5; 5120, 228 x 3584 17.1 / 15.5; 8960, 501 x 2048 23.8 / 21.7, 1024 x 1536 30.1 / 24.8 (192, two); 768 x 1536 22.9 / 24.5
+// not taken; 14 336, 995 x 1536 47.7 / 37.1; 18 944, 236 x 5120 60.7 / 45.6 (256, three).  151 936 (through a workspace): 200 x 1536 133 / 113 (128, six),
+// 400 218 / 177 (256, six), 768 318 / 255 (256, four), 1000 463 / 336 (three), 1300 521 / 461 (two).
 struct PairCut { int bn, splits; bool clusters; int64_t single; };       // splits 1: not taken; single: split_choice, 0 where it was not asked
 inline double pair_block_us(int bn, double load) {
   const double light = bn == 128 ? 0.2 : bn == 192 ? 0.26 : 0.314, full = bn == 128 ? 0.23 : bn == 192 ? 0.33 : 0.41;
   return light + (full - light) * std::min(1.0, load);
 }
-constexpr int64_t kPairWorkspaceMax = 128 << 20;         // bytes
+inline bool pairs_come_into_question(int64_t M, int64_t N, int64_t K) { return M > 128 && N > 64 && K > 15 * 64; }
 // fits(s) as for split_choice, pair_fits(bn, s): clusters of s pairs that run at a time
 template <class Fits, class PairFits>
 PairCut pair_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits, PairFits pair_fits) {
   const int64_t blocks = (K + 63) / 64, units = sms / 2, num_m = (M + 255) / 256;
   PairCut best{0, 1, false, 0};
-  if (N <= 64 || blocks < 16 || units < 1) return best;
+  if (!pairs_come_into_question(M, N, K) || units < 1) return best;
   // the form that is taken otherwise
   auto column_tiles = [&](int bn) { return static_cast<int>(bn == 128 ? (N + 127) >> 7 : bn == 256 ? (N + 255) >> 8 : (N + 191) / 192); };
   const int64_t tiles1 = split_tiles(M, N), s1 = split_choice(M, N, K, sms, fits);
@@ -213,7 +215,7 @@ PairCut pair_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits, Pai
       other = std::min(other, waves * blocks * pair_block_us(bn, static_cast<double>(tiles) / (waves * units)) + (bn == 256 ? 4.5 : 4.0));
     }
   }
-  double least = 0.96 * other;
+  double least = 0.98 * (other - 0.8);
   // by number of ranges outside, so that its divisions are made once, and of int; this is run for every product.  Short contractions are cut by clusters only.
   const int nb = static_cast<int>(blocks), nu = static_cast<int>(units), top = nb <= 512 ? 4 : 8;
   int tiles_of[3], n = 0;
@@ -224,10 +226,10 @@ PairCut pair_choice(int64_t M, int64_t N, int64_t K, int64_t sms, Fits fits, Pai
     for (int i = 0; i < 3; ++i) {
       const int bn = 128 + 64 * i, tiles = tiles_of[i];
       const bool clusters = s <= 4 && tiles <= pair_fits(bn, s);
-      if (!clusters && (nb <= 512 || static_cast<int64_t>(s) * tiles * 256 * bn * 4 > kPairWorkspaceMax)) continue;
-      const int waves = (tiles * s + nu - 1) / nu;
-      const double loop = pair_block_us(bn, static_cast<double>(tiles * s) / (waves * nu)) * per, start = bn == 256 ? 4.5 : 4.0;
-      const double t = clusters ? loop + start + (s == 2 ? 1.8 : s == 3 ? 3.1 : 3.4) : waves * (loop + (bn == 128 ? 5.0 : bn == 192 ? 7.0 : 9.0)) + start;
+      if (!clusters && (nb <= 512 || tiles * s > nu)) continue;
+      const double loop = pair_block_us(bn, static_cast<double>(tiles * s) / nu) * per, start = bn == 256 ? 4.5 : 4.0;
+      const double sums = clusters ? (s == 2 ? 2.2 : s == 3 ? 3.1 : 3.4) + (bn == 192 ? 0.5 : 0.0) : (bn == 128 ? 5.0 : bn == 192 ? 7.0 : 9.0) + 1.6 * std::max(0, s - 3);
+      const double t = loop + sums + start;
       if (t < least) { least = t; best = {bn, s, clusters, s1}; }
     }
   }
@@ -261,6 +263,7 @@ int64_t auto_single(int64_t M, int64_t N, int64_t K) {
   return split_choice(M, N, K, num_sms(), [&](int s) { return f.blocks(bn, s); });
 }
 PairCut auto_pairs(int64_t M, int64_t N, int64_t K) {
+  if (!pairs_come_into_question(M, N, K)) return {0, 1, false, 0};
   const ClusterFits& f = cluster_fits();
   const int bn = split_block_n(N);
   return pair_choice(M, N, K, num_sms(), [&](int s) { return f.blocks(bn, s); }, [&](int w, int s) { return f.of_pairs(w, s); });
