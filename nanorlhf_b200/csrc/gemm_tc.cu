@@ -969,8 +969,8 @@ gemm_tc_cg2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   gemm_tc_body<2, BN, A_MN, B_MN, EPI>(tmA, tmB, tmA2, tmB2, tmD, p);
 }
 
-struct TcMaps3 { CUtensorMap m[3]; };
-struct TcMaps8 { CUtensorMap m[2 * kSumPairs]; };
+template <int N>
+struct TcMaps { CUtensorMap m[N]; };      // as many as a kernel reads: they are launch parameters too
 
 // EPI: EPI_SWIGLU, or EPI_SWIGLU_KEEP where gate and up are wanted too (training); more = {the up adapter's columns, gate, up}.  Two GEMMs and an activation
 // pass move 2.4 times as much memory, the pass alone 54 us of traffic at 6601 x 8960; three stores a tile hide behind its 26 blocks of contraction.
@@ -978,7 +978,7 @@ template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBg, const __grid_constant__ CUtensorMap tmBu,
                     const __grid_constant__ CUtensorMap tmA2g, const __grid_constant__ CUtensorMap tmB2g, const __grid_constant__ CUtensorMap tmB2u,
-                    const __grid_constant__ CUtensorMap tmD, const __grid_constant__ TcMaps3 more, const TcParams p) {
+                    const __grid_constant__ CUtensorMap tmD, const __grid_constant__ TcMaps<EPI == EPI_SWIGLU_KEEP ? 3 : 1> more, const TcParams p) {
   const bool up = cluster_ctarank() != 0;
   gemm_tc_body<2, 256, false, false, EPI, false, false, false, false, true>(tmA, up ? tmBu : tmBg, tmA2g, up ? tmB2u : tmB2g, tmD, p, more.m);
 }
@@ -989,7 +989,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // With this, the kept gate and up and sums in one accumulator a decoder layer's forward and backward over 6601 tokens takes 1724 us, 1862 before.
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_tc_dswiglu_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA2,
-                       const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmD, const __grid_constant__ TcMaps3 more,
+                       const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmD, const __grid_constant__ TcMaps<3> more,
                        const TcParams p) {
   gemm_tc_body<2, 256, false, true, EPI_DSWIGLU>(tmA, tmB, tmA2, tmB2, tmD, p, more.m);
 }
@@ -998,11 +998,11 @@ gemm_tc_dswiglu_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 // result, an addition and a rounding per projection (6601 x 1536: 60 MB each time)
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-gemm_tc_sum_kernel(const __grid_constant__ TcMaps8 maps, const __grid_constant__ CUtensorMap tmD, const TcParams p) {
+gemm_tc_sum_kernel(const __grid_constant__ TcMaps<2 * kSumPairs> maps, const __grid_constant__ CUtensorMap tmD, const TcParams p) {
   gemm_tc_body<2, BN, false, true, EPI_BF16, false, false, false, false, false, false, true>(tmD, tmD, tmD, tmD, tmD, p, maps.m);
 }
 template <int BN>
-static cudaError_t launch_sum(const TcMaps8& maps, const CUtensorMap& tmD, const TcParams& p, int num_sms, cudaStream_t stream) {
+static cudaError_t launch_sum(const TcMaps<2 * kSumPairs>& maps, const CUtensorMap& tmD, const TcParams& p, int num_sms, cudaStream_t stream) {
   using C = Cfg<2, BN, true>;
   auto kern = gemm_tc_sum_kernel<BN>;
   static nrl::PerDevice<bool> configured;
@@ -1018,19 +1018,18 @@ static cudaError_t launch_sum(const TcMaps8& maps, const CUtensorMap& tmD, const
 // last wave for all.  us, a launch each -> one (rows 250, 800, 3300, 6601, 24 571, 32 768): 3 x 1024 features of 1024: 23 -> 7.4, 24 -> 10, 39 -> 21, 47 -> 31, 127 -> 106, 156 -> 138;
 // 1536 + 256 + 256 of 1536 with adapters of rank 64: 31 -> 10, 30 -> 10, 39 -> 20, 47 -> 30, 131 -> 108, 164 -> 141; 3584 + 512 + 512 of 3584: 65 -> 17, 54 -> 24, 92 -> 81,
 // 165 -> 146, 626 -> 608, 788 -> 759.
-struct TcMaps16 { CUtensorMap m[4 * kCatMax]; };
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_cat_cg1_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ TcMaps16 maps, const TcParams p, const __grid_constant__ TcCat cat) {
+gemm_tc_cat_cg1_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ TcMaps<4 * kCatMax> maps, const TcParams p, const __grid_constant__ TcCat cat) {
   gemm_tc_body<1, BN, false, false, EPI_BF16, false, false, false, false, false, false, false, true>(tmA, tmA, tmA, tmA, tmA, p, maps.m, 0, &cat);
 }
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-gemm_tc_cat_cg2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ TcMaps16 maps, const TcParams p, const __grid_constant__ TcCat cat) {
+gemm_tc_cat_cg2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ TcMaps<4 * kCatMax> maps, const TcParams p, const __grid_constant__ TcCat cat) {
   gemm_tc_body<2, BN, false, false, EPI_BF16, false, false, false, false, false, false, false, true>(tmA, tmA, tmA, tmA, tmA, p, maps.m, 0, &cat);
 }
 template <int CG, int BN>
-static cudaError_t launch_cat(const CUtensorMap& tmA, const TcMaps16& maps, const TcParams& p, const TcCat& cat, int num_sms, cudaStream_t stream) {
+static cudaError_t launch_cat(const CUtensorMap& tmA, const TcMaps<4 * kCatMax>& maps, const TcParams& p, const TcCat& cat, int num_sms, cudaStream_t stream) {
   using C = Cfg<CG, BN>;
   auto kern = CG == 2 ? gemm_tc_cat_cg2_kernel<BN> : gemm_tc_cat_cg1_kernel<BN>;
   static nrl::PerDevice<bool> configured;
@@ -1252,15 +1251,15 @@ static int splitk_clusters(int splits) {
 template <int BN, bool A_MN, bool B_MN>
 static cudaError_t launch_splitk(const CUtensorMap* maps, const TcParams& p, int num_sms, cudaStream_t stream) {
   using C = Cfg<1, BN, B_MN>;
-  auto kern = gemm_tc_splitk_kernel<BN, A_MN, B_MN>;
-  static nrl::PerDevice<bool> configured;
-  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   const int tiles = ((p.M + BLOCK_M - 1) / BLOCK_M) * ((p.N + BN - 1) / BN);
   int grid = tiles * p.splits;
   if (grid <= num_sms && split_by_clusters(p.splits, (p.K + BLOCK_K - 1) / BLOCK_K) && tiles <= splitk_clusters<BN, A_MN, B_MN>(p.splits)) {
     launch_dependent_clusters(gemm_tc_splitk_cluster_kernel<BN, A_MN, B_MN>, grid, kThreads, C::kTotal, stream, p.splits, maps[0], maps[1], p);
     return cudaGetLastError();
   }
+  auto kern = gemm_tc_splitk_kernel<BN, A_MN, B_MN>;
+  static nrl::PerDevice<bool> configured;
+  if (const cudaError_t e = nrl::allow_smem(configured, kern, C::kTotal); e != cudaSuccess) return e;
   if (grid > num_sms) grid = num_sms;
   launch_dependent(kern, grid, kThreads, C::kTotal, stream, maps[0], maps[1], p);
   return cudaGetLastError();
@@ -1332,7 +1331,12 @@ static cudaError_t launch_pair(const CUtensorMap* maps, const nrl::tc::TcParams&
   int units = ((p.M + 255) / 256) * ((p.N + 255) / 256);
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;
-  const TcMaps3 more{{maps[4], EPI == EPI_SWIGLU_KEEP ? maps[8] : maps[7], EPI == EPI_SWIGLU_KEEP ? maps[9] : maps[7]}};
+  TcMaps<EPI == EPI_SWIGLU_KEEP ? 3 : 1> more;
+  more.m[0] = maps[4];
+  if constexpr (EPI == EPI_SWIGLU_KEEP) {
+    more.m[1] = maps[8];
+    more.m[2] = maps[9];
+  }
   nrl::launch_dependent(kern, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[5], maps[6], maps[7], more, p);
   return cudaGetLastError();
 }
@@ -1349,14 +1353,14 @@ extern "C" cudaError_t nrl_gemm_tc_dswiglu(const CUtensorMap* maps, const nrl::t
   int units = ((p->M + 255) / 256) * ((p->N + 255) / 256);
   if (units > num_sms / 2) units = num_sms / 2;
   if (units < 1) units = 1;
-  const TcMaps3 more{{maps[4], maps[5], maps[7]}};
+  const TcMaps<3> more{{maps[4], maps[5], maps[7]}};
   nrl::launch_dependent(gemm_tc_dswiglu_kernel, 2 * units, kThreads, C::kTotal, stream, maps[0], maps[1], maps[2], maps[3], maps[6], more, *p);
   return cudaGetLastError();
 }
 
 extern "C" cudaError_t nrl_gemm_tc_sum(const CUtensorMap* maps, const nrl::tc::TcParams* p, int bn, int num_sms, cudaStream_t stream) {
   using namespace nrl::tc;
-  TcMaps8 all;
+  TcMaps<2 * kSumPairs> all;
   for (int i = 0; i < 2 * kSumPairs; ++i) all.m[i] = maps[i];
   const CUtensorMap& d = maps[2 * kSumPairs];
   if (bn == 256) return launch_sum<256>(all, d, *p, num_sms, stream);
@@ -1367,7 +1371,7 @@ extern "C" cudaError_t nrl_gemm_tc_sum(const CUtensorMap* maps, const nrl::tc::T
 
 extern "C" cudaError_t nrl_gemm_tc_cat(const CUtensorMap* maps, const nrl::tc::TcParams* p, const nrl::tc::TcCat* cat, int cg, int bn, int num_sms, cudaStream_t stream) {
   using namespace nrl::tc;
-  TcMaps16 all;
+  TcMaps<4 * kCatMax> all;
   for (int i = 0; i < 4 * kCatMax; ++i) all.m[i] = maps[1 + i];
 #define NRL_TC_CAT(CG_, BN_) \
   if (cg == CG_ && bn == BN_) return launch_cat<CG_, BN_>(maps[0], all, *p, *cat, num_sms, stream);

@@ -40,22 +40,35 @@ struct TcCat {
 struct TcParams {
   int M, N, K;                  // D is [M, N]; K = contraction length of the first operand pair
   int K2;                       // contraction length of the second operand pair (0 = none)
-  const float* row_scale;       // FP8 kernels: [M] per-token dequantisation scale of A (GROUPED: see below)
-  const float* col_scale;       // FP8 kernels: [N] per-output-channel dequantisation scale of B
-  int col_ranges;               // EPI_LOGPROB: into how many ranges the column tiles are cut (work items = row tiles x ranges)
+  // of one kernel at most; the parameters travel with every launch
+  union {
+    struct {
+      const float* row_scale;   // FP8 kernels: [M] per-token dequantisation scale of A (GROUPED: see below)
+      const float* col_scale;   // FP8 kernels: [N] per-output-channel dequantisation scale of B
+    };
+    struct {
+      const __nv_bfloat16* residual;      // EPI_RESIDUAL: [M, N], row stride residual_stride
+      long residual_stride;
+    };
+    float* logits;              // EPI_LOGPROB: null, or [M, N] for the accumulator
+    int sum_end[kSumPairs];     // SUM kernels: k-blocks of the products up to and with the i-th (of those behind the last: as many)
+  };
   const int* targets;           // EPI_LOGPROB, EPI_DLOGITS: [M] column of the row's target
   const float* lse;             // EPI_DLOGITS: [M] log of the row's sum of exponentials
   const float* grad;            // EPI_DLOGITS: [M] gradient of the row's log-probability
   int batch;                    // BATCH kernels: number of independent [M,K] x [N,K]^T problems behind 3D tensor maps (else 1)
   float alpha;                  // multiplies the accumulator
   const __nv_bfloat16* bias;    // EPI_BF16: optional [N]
-  const __nv_bfloat16* residual;      // EPI_RESIDUAL: [M, N], row stride residual_stride
-  long residual_stride;
-  int act;                      // EPI_BF16: 0 = none, 1 = exact (erf) GELU after the bias (GROUPED: see below)
-  float* logits;                // EPI_LOGPROB: null, or [M, N] for the accumulator
+  union {
+    int act;                    // EPI_BF16: 0 = none, 1 = exact (erf) GELU after the bias (GROUPED: see below)
+    int col_ranges;             // EPI_LOGPROB: into how many ranges the column tiles are cut (work items = row tiles x ranges)
+  };
   float* out_f32;               // EPI_F32: [M, N] fp32, row stride out_f32_stride elements
   long out_f32_stride;
-  int accumulate;               // EPI_F32: 1 = add to what is there
+  union {
+    int accumulate;             // EPI_F32: 1 = add to what is there
+    int transposed;             // MULTI kernels: D^T [N, M] is written
+  };
   // split-K (SPLIT kernels; small outputs with a long contraction -- LoRA wgrads, rank-r projections): every tile is
   // computed by `splits` CTAs over disjoint k-ranges; where they fit they are a cluster that sums its partial tiles through distributed shared memory,
   // else partial tiles go to `ws` (fp32) and the last CTA to arrive on the tile's counter sums them.  Either way in split order
@@ -65,15 +78,16 @@ struct TcParams {
   int* counters;                // [tiles] int32, zero between launches
   __nv_bfloat16* out_bf16;      // SPLIT: D written with plain stores (row stride out_stride elements)
   long out_stride;
-  int transposed;               // CLUSTER kernels: D^T [N, M] is written
   // GROUPED kernels (mixture of experts): the rows of A are sorted by expert and B holds every expert's [N, K] matrix one after
   // the other.  A row tile belongs to one expert; it may start at any row and is cut off at the end of the expert's rows
   // (the tile's further rows are computed and dropped).  The table and its length live on the device (written by the
   // routing kernels of the same stream), so no launch parameter depends on the routing.
   const int* grp_tiles;         // [max tiles, 3]: expert, first row, end row (exclusive) of the expert's rows
   const int* grp_num_tiles;     // [1]: row tiles in use
-  int sum_end[kSumPairs];       // SUM kernels: k-blocks of the products up to and with the i-th (of those behind the last: as many)
 };
+
+// 56 bytes more made four projections in a row 0.4 of 43 us slower (39 and 81 rows; in a graph as fast): the device reads them launch by launch
+static_assert(sizeof(TcParams) <= 152, "launch parameters of every GEMM");
 
 // Is a contraction of `blocks` times 64 columns in `splits` ranges summed by clusters (where they fit)?  Not two long ranges: a cluster of two takes both SMs of a
 // pair that share their way to the L2 and leaves other pairs idle, which costs more than the sum through the workspace from 32 768 columns on.  us, clusters /
