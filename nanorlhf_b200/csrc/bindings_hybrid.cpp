@@ -144,20 +144,24 @@ void delta_prep(Tensor qkv, int64_t col_k, const Tensor& b_raw, const Tensor& a_
 }
 
 void delta_scan(const Tensor& qkv, int64_t col_k, int64_t col_v, const c10::optional<Tensor>& beta, const Tensor& decay, Tensor state, Tensor o,
-                const Tensor& cu, const Tensor& start, const Tensor& state_slot, int64_t kv_heads, bool per_channel, int64_t impl) {
+                const Tensor& cu, const Tensor& start, const Tensor& state_slot, int64_t kv_heads, bool per_channel, int64_t impl,
+                const c10::optional<std::vector<int64_t>>& lengths) {
   c10::cuda::CUDAGuard guard(o.device());
   TORCH_CHECK(state.dim() == 4 && state.is_contiguous(), "delta_scan: state [slots, heads, D, Dv]");
   const int heads = static_cast<int>(state.size(1)), D = static_cast<int>(state.size(2)), Dv = static_cast<int>(state.size(3));
   const int E = static_cast<int>(start.numel());
   TORCH_CHECK(qkv.dim() == 2 && col_v + heads * Dv <= qkv.size(1) && o.is_contiguous() && o.size(-1) == heads * Dv, "delta_scan: shapes");
+  TORCH_CHECK(!lengths.has_value() || static_cast<int64_t>(lengths->size()) == E, "delta_scan: a length per entry");
+  const std::vector<long> tokens = lengths.has_value() ? std::vector<long>(lengths->begin(), lengths->end()) : std::vector<long>();
+  const int line = nrl_delta_line_mode(tokens.empty() ? nullptr : tokens.data(), E, qkv.size(0), heads, Dv, static_cast<int>(impl), num_sms());
   const long bytes = nrl_delta_scan_scratch(f32(qkv, "qkv"), qkv.stride(0), static_cast<int>(col_k), static_cast<int>(col_v), E, qkv.size(0), heads, D, Dv,
-                                            per_channel ? 1 : 0, static_cast<int>(impl), num_sms());
+                                            per_channel ? 1 : 0, static_cast<int>(impl), line, num_sms());
   torch::Tensor scratch;                                     // of this call: steps on other streams have their own
   if (bytes > 0) scratch = torch::empty({bytes}, qkv.options().dtype(torch::kUInt8));
   check(nrl_delta_scan(f32(qkv, "qkv"), qkv.stride(0), static_cast<int>(col_k), static_cast<int>(col_v), beta.has_value() ? f32(*beta, "beta") : nullptr,
                        f32(decay, "decay"), f32w(state, "state"), f32w(o, "o"), i32(cu, "cu"), i32(start, "start"),
                        i32(state_slot, "state_slot"), E, static_cast<int>(qkv.size(0)), heads, static_cast<int>(kv_heads), D, Dv, per_channel ? 1 : 0,
-                       static_cast<int>(impl), num_sms(), bytes > 0 ? scratch.data_ptr() : nullptr, cur_stream()),
+                       static_cast<int>(impl), line, num_sms(), bytes > 0 ? scratch.data_ptr() : nullptr, cur_stream()),
         "delta_scan");
 }
 
@@ -772,6 +776,19 @@ void gemm_tc_grouped(const Tensor& a, const Tensor& b, const c10::optional<Tenso
   check(nrl_gemm_tc_grouped(maps, &p, bn, static_cast<int>(tiles.size(0)), sms, cur_stream()), "gemm_tc_grouped");
 }
 
+// how the blocks share the chunks of a step (delta_chunk_tc.cu): (taken, [first, last] segment of each block, segments of eight numbers)
+std::tuple<int64_t, Tensor, Tensor> delta_line_plan(const Tensor& cu, int64_t heads, int64_t Dv, int64_t blocks, bool forced) {
+  i32(cu, "cu");
+  TORCH_CHECK(cu.is_cuda() && cu.is_contiguous() && cu.numel() >= 2 && cu.numel() <= 4097 && heads > 0 && Dv > 0 && blocks > 0, "delta_line_plan: up to 4096 entries");
+  c10::cuda::CUDAGuard guard(cu.device());
+  const int64_t E = cu.numel() - 1, bytes = nrl_delta_line_bytes(E, static_cast<int>(heads), static_cast<int>(Dv), static_cast<int>(blocks)), n = E * heads * ((Dv + 127) / 128) + blocks;
+  Tensor scratch = torch::zeros({bytes}, cu.options().dtype(torch::kUInt8));
+  check(nrl_delta_line(i32(cu, "cu"), static_cast<int>(E), static_cast<int>(heads), static_cast<int>(Dv), forced, scratch.data_ptr(), static_cast<int>(blocks), cur_stream()),
+        "delta_line_plan");
+  const Tensor ints = scratch.slice(0, blocks * 128 * 128 * 4).view(torch::kInt32);
+  return {ints[3 * blocks].item<int64_t>(), ints.slice(0, 0, 2 * blocks).view({2, blocks}).clone(), ints.slice(0, 4 * blocks, 4 * blocks + 8 * n).view({n, 8}).clone()};
+}
+
 }  // namespace
 
 namespace nrl {
@@ -812,11 +829,18 @@ void bind_hybrid(pybind11::module_& m) {
   m.def("delta_prep", &delta_prep, "unit q / k, beta and decays of the gated delta rule");
   m.def("delta_scan_chunked", &nrl_delta_scan_chunked, "a step goes 32 tokens at a time", pybind11::arg("E"), pybind11::arg("T"), pybind11::arg("heads"),
         pybind11::arg("D"), pybind11::arg("Dv"), pybind11::arg("num_sms"));
-  m.def("delta_scan_shared", &nrl_delta_scan_shared, "blocks of a step taken 32 tokens at a time share its chunks", pybind11::arg("E"), pybind11::arg("T"),
+  m.def("delta_line_pays", [](const std::vector<int64_t>& lengths, int64_t heads, int64_t Dv, int64_t blocks) {
+    const std::vector<long> tokens(lengths.begin(), lengths.end());
+    return nrl_delta_line_pays(tokens.data(), static_cast<long>(tokens.size()), static_cast<int>(heads), static_cast<int>(Dv), static_cast<int>(blocks)) != 0;
+  }, "what delta_line_plan decides, from lengths on the host");
+  m.def("delta_line_plan", &delta_line_plan, pybind11::arg("cu"), pybind11::arg("heads"), pybind11::arg("Dv"), pybind11::arg("blocks"), pybind11::arg("forced") = false);
+  m.def("delta_scan_shared", &nrl_delta_scan_shared, "blocks of a step taken 32 tokens at a time may share its chunks", pybind11::arg("E"), pybind11::arg("T"),
         pybind11::arg("heads"), pybind11::arg("Dv"), pybind11::arg("num_sms"));
   m.def("delta_scan_blocked", &nrl_delta_scan_blocked, "a step goes four tokens at a time", pybind11::arg("E"), pybind11::arg("T"), pybind11::arg("D"),
         pybind11::arg("Dv"));
-  m.def("delta_scan", &delta_scan, "gated delta rule scan, state carried per slot");
+  m.def("delta_scan", &delta_scan, "gated delta rule scan, state carried per slot", pybind11::arg("qkv"), pybind11::arg("col_k"), pybind11::arg("col_v"),
+        pybind11::arg("beta"), pybind11::arg("decay"), pybind11::arg("state"), pybind11::arg("o"), pybind11::arg("cu"), pybind11::arg("start"),
+        pybind11::arg("state_slot"), pybind11::arg("kv_heads"), pybind11::arg("per_channel"), pybind11::arg("impl"), pybind11::arg("lengths") = pybind11::none());
   m.def("qknorm_kv_write", &qknorm_kv_write, "per-head RMS norm of q (in place) and k (into the paged cache), v into the cache");
   m.def("window_attention_tc_tokens", &nrl_window_attention_tc_tokens, "tokens of a tile of the tcgen05 kernel", pybind11::arg("T"), pybind11::arg("E"),
         pybind11::arg("Hq"), pybind11::arg("Hkv"), pybind11::arg("num_sms"));

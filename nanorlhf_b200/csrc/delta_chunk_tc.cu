@@ -28,6 +28,10 @@
 #include "attention_tc.cuh"
 #include "hybrid_kernels.h"
 
+#include <algorithm>
+#include <functional>
+#include <vector>
+
 namespace nrl {
 namespace {
 
@@ -132,23 +136,31 @@ NRL_DEVICE int pair_b(int pr) { return (0x001012 >> (4 * pr)) & 3; }
 // Blocks start from the line's end, so that none waits for one that starts later; should the wait run out all the same, the state becomes NaN.
 // The segments are laid out by a kernel of their own, and between two segments the block starts anew (barriers and all): code that every warp runs through is
 // dear here.  With phases that run on over the segments a chunk took 19 % longer, so 13 % (92 KB of code, 78 for whole items).
-// 10 x 2048 tokens, 16 heads of 128 x 128 (160 items of 64 chunks on 148 SMs): two rounds of 64 chunks 625 us, 70 chunks in a row 381 us.  When it is taken: recurrent.cu.
+// 10 x 2048 tokens, 16 heads of 128 x 128 (160 items of 64 chunks on 148 SMs): two rounds of 64 chunks 625 us, 70 chunks in a row 381 us.
+// Whether it pays depends on the lengths: no block gets less than the longest item, and whole items of unequal lengths do not run in rounds.  The line is taken where
+// it is estimated a tenth below the least that whole items can take: an SM has r items of length l and more wherever more than (r - 1) SMs' worth of them exist.  A
+// caller who has the lengths on the host asks there (nrl_delta_line_pays); for others the kernel that lays the segments out decides.  16 heads, one entry of 4000
+// tokens and nine of 400: whole 600 us, line 768; 8 heads of 64, 20 entries of 33 to 700: 100 / 181.
 struct DcSegment {
   int t0, n, t1;              // first token, chunks, end of the entry's tokens
   int h, cb0, e;              // head, first column, entry
   int in, out;                // the state comes from the block behind / goes to the block in front
 };
 struct DcLine {
-  DcSegment* segments;        // [items + blocks]; null: a block per item
+  DcSegment* segments;        // [items + blocks]
   int *first, *last;          // [blocks] a block's segments
   int* handed;                // [blocks] 1 once the state that the block hands on is there
   float* carry;               // [blocks][128][128]
+  int* taken;                 // [1] the line is taken, else a block has an item
 };
 constexpr int kDcMaxEntries = 4096;
 
-__global__ void __launch_bounds__(1024) delta_line_kernel(const int* __restrict__ cu, int E, int heads, int parts, int blocks, const DcLine l) {
+// chunks in a row of the line against those of whole items; a chunk costs 13 % more there, starting anew between segments about four chunks
+__host__ NRL_DEVICE bool line_pays(long line, long whole) { return 113 * line + 400 < 90 * whole; }
+
+__global__ void __launch_bounds__(1024) delta_line_kernel(const int* __restrict__ cu, int E, int heads, int parts, int blocks, bool forced, const DcLine l) {
   __shared__ int from[kDcMaxEntries + 1];                  // chunks of an item of the entries in front
-  __shared__ int most[32];
+  __shared__ int most[32], least[32];
   const int tid = threadIdx.x, items = heads * parts;
   for (int b = tid; b < blocks; b += blockDim.x) l.first[b] = l.last[b] = l.handed[b] = 0;
   auto chunks = [&](int e) { return max(1, (cu[e + 1] - cu[e] + kC - 1) / kC); };      // an entry without tokens keeps its state: one empty chunk
@@ -172,7 +184,21 @@ __global__ void __launch_bounds__(1024) delta_line_kernel(const int* __restrict_
   }
   __syncthreads();
   m = most[tid & 31];
-  const int total = from[E] * items, per = max(__reduce_max_sync(0xffffffffu, m), (total + blocks - 1) / blocks);
+  const int total = from[E] * items, share = (total + blocks - 1) / blocks, per = max(__reduce_max_sync(0xffffffffu, m), share);
+  int whole = share;
+  for (int e = tid; e < E && !forced; e += blockDim.x) {   // at most a few hundred entries where the line comes into question
+    const int n = from[e + 1] - from[e];
+    int as_long = 0;
+    for (int k = 0; k < E; ++k) as_long += from[k + 1] - from[k] >= n ? 1 : 0;
+    whole = max(whole, (as_long * items + blocks - 1) / blocks * n);
+  }
+  whole = __reduce_max_sync(0xffffffffu, whole);
+  if ((tid & 31) == 0) least[tid >> 5] = whole;
+  __syncthreads();
+  whole = __reduce_max_sync(0xffffffffu, least[tid & 31]);
+  const bool taken = forced || line_pays(per, whole);
+  if (tid == 0) *l.taken = taken ? 1 : 0;
+  if (!taken) return;
   for (int q = tid; q < E * items; q += blockDim.x) {
     const int e = q / items, k = q - e * items, n = from[e + 1] - from[e], s = from[e] * items + k * n, t0 = cu[e], t1 = cu[e + 1];
     const int h = k / parts, cb0 = (k - h * parts) * 128, a = s / per, here = min(n, (a + 1) * per - s);      // chunks that lie in block a
@@ -208,9 +234,12 @@ struct DcParams {
 
 NRL_DEVICE void mbar_inval(uint64_t* bar) { asm volatile("mbarrier.inval.shared.b64 [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 
-// DP: padded rows of S; WIDE: rows of q, k and v are 16-byte aligned; LINE: a block takes its share of the line instead of an item
+// DP: padded rows of S; WIDE: rows of q, k and v are 16-byte aligned; LINE: a block takes its share of the line instead of an item.  Where the GPU decides, both
+// kernels are launched and one of them finds nothing to do: 10 entries of 2048 tokens 396 us (388 with the lengths on the host), 20 of 33 to 700 110 us (100).  Both
+// forms in one kernel spill: 401 and 105.
 template <int DP, bool DELTA, bool WIDE, bool LINE>
 __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcParams p) {
+  if (!LINE && p.line.taken != nullptr && *p.line.taken != 0) return;
   using L = DcSmem<DP>;
   using Tm = DcTmem<DP>;
   constexpr int NH = L::kHalves;
@@ -806,30 +835,55 @@ cudaError_t launch_delta_chunk(unsigned grid, const DcParams& p, cudaStream_t s)
 }  // namespace nrl
 
 // D <= 128, one decay per head; beta == nullptr: plain accumulation; rows16: rows of q, k and v start and end on 16-byte boundaries; line: null, or (rows16)
-// nrl_delta_line_bytes() of scratch with which `blocks` blocks share the chunks of all items
+// nrl_delta_line_bytes() of scratch with which `blocks` blocks share the chunks of all items, where that pays or it is forced
 extern "C" long nrl_delta_line_bytes(long E, int heads, int Dv, int blocks) {
   return blocks * (128l * 128 * 4 + 16) + (E * heads * ((Dv + 127) / 128) + blocks) * static_cast<long>(sizeof(nrl::DcSegment));
 }
+static nrl::DcLine line_in(void* scratch, int blocks) {
+  nrl::DcLine l{};
+  l.carry = static_cast<float*>(scratch);
+  l.first = reinterpret_cast<int*>(l.carry + blocks * 128l * 128);
+  l.last = l.first + blocks;
+  l.handed = l.last + blocks;
+  l.taken = l.handed + blocks;                             // of the fourth run of `blocks` numbers
+  l.segments = reinterpret_cast<nrl::DcSegment*>(l.handed + 2 * blocks);
+  return l;
+}
+extern "C" int nrl_delta_line_pays(const long* tokens, long E, int heads, int Dv, int blocks) {
+  const long items = static_cast<long>(heads) * ((Dv + 127) / 128);
+  std::vector<long> n(E);
+  long total = 0;
+  for (long e = 0; e < E; ++e) total += n[e] = std::max(1l, (tokens[e] + nrl::kC - 1) / nrl::kC);
+  std::sort(n.begin(), n.end(), std::greater<long>());
+  const long share = (total * items + blocks - 1) / blocks;
+  long whole = share;
+  for (long e = 0; e < E; ++e) whole = std::max(whole, ((e + 1) * items + blocks - 1) / blocks * n[e]);
+  return E > 0 && nrl::line_pays(std::max(n[0], share), whole);
+}
+extern "C" cudaError_t nrl_delta_line(const int* cu, int E, int heads, int Dv, bool forced, void* line, int blocks, cudaStream_t s) {
+  if (E > nrl::kDcMaxEntries) return cudaErrorInvalidValue;
+  nrl::delta_line_kernel<<<1, 1024, 0, s>>>(cu, E, heads, (Dv + 127) / 128, blocks, forced, line_in(line, blocks));
+  return cudaGetLastError();
+}
 extern "C" cudaError_t nrl_delta_chunk_tc(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state, float* o,
                                           const int* cu, const int* start, const int* state_slot, int E, int heads, int kv_heads, int D, int Dv,
-                                          bool rows16, void* line, int blocks, cudaStream_t s) {
+                                          bool rows16, void* line, int blocks, bool forced, cudaStream_t s) {
   nrl::DcParams p{qkv, beta, decay, state, o, cu, start, state_slot, sq, col_k, col_v, heads, kv_heads, D, Dv, {}};
   const int parts = (Dv + 127) / 128;
-  unsigned grid = static_cast<unsigned>(E) * heads * parts;
+  const unsigned grid = static_cast<unsigned>(E) * heads * parts;
   if (line != nullptr) {
-    if (E > nrl::kDcMaxEntries || !rows16) return cudaErrorInvalidValue;
-    p.line.carry = static_cast<float*>(line);
-    p.line.first = reinterpret_cast<int*>(p.line.carry + blocks * 128l * 128);
-    p.line.last = p.line.first + blocks;
-    p.line.handed = p.line.last + blocks;
-    p.line.segments = reinterpret_cast<nrl::DcSegment*>(p.line.handed + 2 * blocks);
-    nrl::delta_line_kernel<<<1, 1024, 0, s>>>(cu, E, heads, parts, blocks, p.line);
-    grid = static_cast<unsigned>(blocks);
+    if (!rows16) return cudaErrorInvalidValue;
+    p.line = line_in(line, blocks);
+    if (const cudaError_t e = nrl_delta_line(cu, E, heads, Dv, forced, line, blocks, s); e != cudaSuccess) return e;
   }
 #define NRL_DC(P_, B_)                                                 \
-  if ((D <= 64 ? 64 : 128) == P_ && (beta != nullptr) == B_)             \
-    return (line != nullptr ? nrl::launch_delta_chunk<P_, B_, true, true>                                                       \
-                            : rows16 ? nrl::launch_delta_chunk<P_, B_, true, false> : nrl::launch_delta_chunk<P_, B_, false, false>)(grid, p, s);
+  if ((D <= 64 ? 64 : 128) == P_ && (beta != nullptr) == B_) {           \
+    if (line != nullptr) {                                               \
+      const cudaError_t e = nrl::launch_delta_chunk<P_, B_, true, true>(static_cast<unsigned>(blocks), p, s);       \
+      if (e != cudaSuccess || forced) return e;                          \
+    }                                                                    \
+    return (rows16 ? nrl::launch_delta_chunk<P_, B_, true, false> : nrl::launch_delta_chunk<P_, B_, false, false>)(grid, p, s); \
+  }
   NRL_DC(64, true) NRL_DC(64, false) NRL_DC(128, true) NRL_DC(128, false)
 #undef NRL_DC
   return cudaErrorInvalidValue;

@@ -159,17 +159,23 @@ cudaError_t nrl_gla_prep(float* qkv, long sq, const float* a_raw, long sa, const
 // Gated delta rule scan.  Per head: S = g S (rows);  u = beta (v - S^T k);  S += k u^T;  o = S^T q.
 // beta == nullptr: plain accumulation, u = v (gated linear attention: S = diag(g) S + k v^T).
 // state float [slots, heads, D, Dv];  o float [T, heads*Dv].  `impl`: 0 picks (nrl_delta_scan_chunked, nrl_delta_scan_blocked, else column-resident),
-// 1 column-resident, 2 row groups, 3 state in shared memory, 4 four tokens at a time (D <= 128), 5 32 at a time (D <= 128, one decay per head).
+// 1 column-resident, 2 row groups, 3 state in shared memory, 4 four tokens at a time (D <= 128), 5 32 at a time (D <= 128, one decay per head), 6 the same and blocks share the chunks whatever that costs.
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
                            float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
-                           int D, int Dv, int per_channel, int impl, int num_sms, void* scratch, cudaStream_t s);
+                           int D, int Dv, int per_channel, int impl, int line, int num_sms, void* scratch, cudaStream_t s);
+// line: do the blocks of a step taken 32 tokens at a time share the chunks of all items (delta_chunk_tc.cu)?  0 no, 1 as the GPU finds the lengths, 2 yes.
+// tokens: the entries' lengths, or null where the host does not have them
+int nrl_delta_line_mode(const long* tokens, long E, long T, int heads, int Dv, int impl, int num_sms);
 // bytes of scratch that such a call wants (0: null)
-long nrl_delta_scan_scratch(const float* qkv, long sq, int col_k, int col_v, long E, long T, int heads, int D, int Dv, int per_channel, int impl, int num_sms);
+long nrl_delta_scan_scratch(const float* qkv, long sq, int col_k, int col_v, long E, long T, int heads, int D, int Dv, int per_channel, int impl, int line, int num_sms);
+int nrl_delta_line_pays(const long* tokens, long E, int heads, int Dv, int blocks);
 long nrl_delta_line_bytes(long E, int heads, int Dv, int blocks);
-int nrl_delta_scan_shared(long E, long T, int heads, int Dv, int num_sms);      // a step taken 32 tokens at a time: its blocks share the chunks of all items
+cudaError_t nrl_delta_line(const int* cu, int E, int heads, int Dv, bool forced, void* line, int blocks, cudaStream_t s);      // lays the line out, where it is taken
+// whether that comes into question
+int nrl_delta_scan_shared(long E, long T, int heads, int Dv, int num_sms);
 cudaError_t nrl_delta_chunk_tc(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state, float* o,
                                const int* cu, const int* start, const int* state_slot, int E, int heads, int kv_heads, int D, int Dv,
-                               bool rows16, void* line, int blocks, cudaStream_t s);      // rows16: rows of q, k and v start and end on 16-byte boundaries
+                               bool rows16, void* line, int blocks, bool forced, cudaStream_t s);      // rows16: rows of q, k and v start and end on 16-byte boundaries
 int nrl_delta_scan_chunked(long E, long T, int heads, int D, int Dv, int num_sms);      // one decay per head: impl 0 takes a step of E entries and T tokens 32 at a time
 int nrl_delta_scan_blocked(long E, long T, int D, int Dv);       // impl 0 takes a step of E entries and T tokens four tokens at a time
 

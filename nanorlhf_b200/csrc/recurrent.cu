@@ -1337,32 +1337,40 @@ static bool delta_rows16(const float* qkv, long sq, int col_k, int col_v, int D,
   return D % 4 == 0 && Dv % 4 == 0 && sq % 4 == 0 && col_k % 4 == 0 && col_v % 4 == 0 && reinterpret_cast<uintptr_t>(qkv) % 16 == 0;
 }
 static bool delta_takes_chunks(bool rows16, long E, long T, int heads, int D, int Dv, int per_channel, int impl, int num_sms) {
-  return !per_channel && D >= 1 && D <= 128 && Dv >= 1 && (impl == 5 || (impl == 0 && rows16 && nrl_delta_scan_chunked(E, T, heads, D, Dv, num_sms)));
+  return !per_channel && D >= 1 && D <= 128 && Dv >= 1 && (impl >= 5 || (impl == 0 && rows16 && nrl_delta_scan_chunked(E, T, heads, D, Dv, num_sms)));
 }
 // Blocks share the chunks of all items (delta_chunk_tc.cu) where rounds of whole items leave many SMs without one in the last: a chunk costs an eighth more
-// there, and starting anew between segments about four chunks, so it is taken for a gain of a tenth by that estimate.  us, items whole / shared (entries
-// of tokens, 16 heads): 128 x 128, 10 of 2048 625 / 381, 12 of 700 228 / 210; 64 x 64, 11 of 300 98 / 88; not taken: 16 of 2048 630 / 617, 32 of 1000 647 / 688,
-// 16 of 256 98 / 121, 64 of 200 309 / 318.
+// there, and starting anew between segments about four chunks, so it comes into question for a gain of a tenth by that estimate with entries of equal lengths, for
+// which the gain is largest; the lengths decide (nrl_delta_line_mode).  us, items whole / shared (entries of tokens, 16 heads): 128 x 128, 10 of 2048 625 / 381,
+// 12 of 700 228 / 210; 64 x 64, 11 of 300 98 / 88; not taken: 16 of 2048 630 / 617, 32 of 1000 647 / 688, 16 of 256 98 / 121, 64 of 200 309 / 318.
+static bool delta_line_fits(long E, long T, int heads, int Dv) {
+  return E <= 4096 && T / 32 + E < (1l << 30) / (heads * ((Dv + 127) / 128));
+}
 int nrl_delta_scan_shared(long E, long T, int heads, int Dv, int num_sms) {
   const long items = E * heads * ((Dv + 127) / 128), rounds = (items + num_sms - 1) / num_sms;
-  if (items <= num_sms || E > 4096 || T / 32 + E >= (1l << 30) / (heads * ((Dv + 127) / 128))) return 0;
+  if (items <= num_sms || !delta_line_fits(E, T, heads, Dv)) return 0;
   const double chunks = static_cast<double>(T) / (32.0 * E);
   return 1.13 * items * chunks / num_sms + 4.0 < 0.9 * rounds * chunks;
 }
-long nrl_delta_scan_scratch(const float* qkv, long sq, int col_k, int col_v, long E, long T, int heads, int D, int Dv, int per_channel, int impl, int num_sms) {
-  if (E <= 0 || !delta_rows16(qkv, sq, col_k, col_v, D, Dv) || !delta_takes_chunks(true, E, T, heads, D, Dv, per_channel, impl, num_sms)) return 0;
-  return nrl_delta_scan_shared(E, T, heads, Dv, num_sms) ? nrl_delta_line_bytes(E, heads, Dv, num_sms) : 0;
+int nrl_delta_line_mode(const long* tokens, long E, long T, int heads, int Dv, int impl, int num_sms) {
+  if (impl == 6) return delta_line_fits(E, T, heads, Dv) ? 2 : 0;
+  if (!nrl_delta_scan_shared(E, T, heads, Dv, num_sms)) return 0;
+  return tokens == nullptr ? 1 : nrl_delta_line_pays(tokens, E, heads, Dv, num_sms) ? 2 : 0;
+}
+long nrl_delta_scan_scratch(const float* qkv, long sq, int col_k, int col_v, long E, long T, int heads, int D, int Dv, int per_channel, int impl, int line, int num_sms) {
+  if (line == 0 || E <= 0 || !delta_rows16(qkv, sq, col_k, col_v, D, Dv) || !delta_takes_chunks(true, E, T, heads, D, Dv, per_channel, impl, num_sms)) return 0;
+  return nrl_delta_line_bytes(E, heads, Dv, num_sms);
 }
 
 cudaError_t nrl_delta_scan(const float* qkv, long sq, int col_k, int col_v, const float* beta, const float* decay, float* state,
                            float* o, const int* cu, const int* start, const int* state_slot, int E, int T, int heads, int kv_heads,
-                           int D, int Dv, int per_channel, int impl, int num_sms, void* scratch, cudaStream_t s) {
+                           int D, int Dv, int per_channel, int impl, int line, int num_sms, void* scratch, cudaStream_t s) {
   if (E <= 0) return cudaSuccess;
-  if (Dv > 512 || heads % kv_heads != 0 || impl < 0 || impl > 5) return cudaErrorInvalidValue;
+  if (Dv > 512 || heads % kv_heads != 0 || impl < 0 || impl > 6 || (impl == 6 && scratch == nullptr)) return cudaErrorInvalidValue;
   const bool rows16 = delta_rows16(qkv, sq, col_k, col_v, D, Dv);
   if (delta_takes_chunks(rows16, E, T, heads, D, Dv, per_channel, impl, num_sms))
-    return nrl_delta_chunk_tc(qkv, sq, col_k, col_v, beta, decay, state, o, cu, start, state_slot, E, heads, kv_heads, D, Dv, rows16, scratch, num_sms, s);
-  if (impl == 5) return cudaErrorInvalidValue;
+    return nrl_delta_chunk_tc(qkv, sq, col_k, col_v, beta, decay, state, o, cu, start, state_slot, E, heads, kv_heads, D, Dv, rows16, scratch, num_sms, line == 2, s);
+  if (impl >= 5) return cudaErrorInvalidValue;
   if (D >= 1 && D <= 128 && Dv >= 1 && (impl == 4 || (impl == 0 && nrl_delta_scan_blocked(E, T, D, Dv)))) {
     const bool wide = D % 4 == 0 && sq % 4 == 0 && col_k % 4 == 0 && reinterpret_cast<uintptr_t>(qkv) % 16 == 0 &&
                      reinterpret_cast<uintptr_t>(decay) % 16 == 0;

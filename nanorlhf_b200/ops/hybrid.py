@@ -46,7 +46,7 @@ def causal_conv(x, w, bias, state, out, plan, in_bias=None, act: str = "silu"):
                        {"none": 0, "silu": 1}[act])
 
 
-SCAN_IMPLS = {"auto": 0, "column": 1, "rows": 2, "shared": 3, "blocked": 4, "chunked": 5}        # four / 32 tokens at a time, delta_scan only
+SCAN_IMPLS = {"auto": 0, "column": 1, "rows": 2, "shared": 3, "blocked": 4, "chunked": 5, "line": 6}        # four / 32 tokens at a time, the same with shared chunks: delta_scan only
 
 
 def ssd_scan(xbc, col_b, col_c, dt_raw, dt_bias, A_log, D, state, y, plan, groups, impl: str = "auto"):
@@ -64,7 +64,7 @@ def delta_scan(qkv, col_k, col_v, beta, decay, state, o, plan, kv_heads, per_cha
     """``beta`` None: plain accumulation ``S = diag(decay) S + k v^T`` (gated linear attention) instead of the delta rule."""
     native._count()
     _ext().delta_scan(qkv, col_k, col_v, beta, decay, state, o, plan.cu, plan.start, plan.state_slot, kv_heads, per_channel,
-                      SCAN_IMPLS[impl])
+                      SCAN_IMPLS[impl], getattr(plan, "lengths", None))
 
 
 def qknorm_kv_write(q, k, v, qw, kw, eps, k_cache, v_cache, plan):

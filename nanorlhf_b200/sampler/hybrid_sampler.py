@@ -59,11 +59,12 @@ def _unwrap(model):
 
 
 class StepPlan:
-    """Device views of one step's packed plan (layout fixed by ``StepScheduler.plan``)."""
-    __slots__ = ("E", "T", "max_blocks", "tokens", "cu", "tok_entry", "pos", "kv_slot", "start", "state_slot", "block_table")
+    """Device views of one step's packed plan (layout fixed by ``StepScheduler.plan``).  ``lengths``: the entries' tokens, where the host has them: kernels
+    are then chosen by them before anything is launched."""
+    __slots__ = ("E", "T", "max_blocks", "tokens", "cu", "tok_entry", "pos", "kv_slot", "start", "state_slot", "block_table", "lengths")
 
-    def __init__(self, buf: torch.Tensor, E: int, T: int, MB: int):
-        self.E, self.T, self.max_blocks = E, T, MB
+    def __init__(self, buf: torch.Tensor, E: int, T: int, MB: int, lengths: Optional[Sequence[int]] = None):
+        self.E, self.T, self.max_blocks, self.lengths = E, T, MB, lengths
         o = 0
 
         def take(n):
@@ -612,7 +613,7 @@ class HybridSampler:
         self.stats["tokens"] += T
         if self.use_cuda_graph and self._bt_width and T == E and len(rows) == T:
             return self._decode_step_graphed(data, E, MB)
-        plan = StepPlan(torch.from_numpy(data).to(self.device), E, T, MB)
+        plan = StepPlan(torch.from_numpy(data).to(self.device), E, T, MB, counts)
         return self._forward(plan, rows)
 
     def _decode_step_graphed(self, data, E: int, MB: int) -> torch.Tensor:

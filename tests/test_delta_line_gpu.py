@@ -1,4 +1,8 @@
-"""The chunked delta-rule scan whose blocks share the chunks of all items: bit for bit what blocks with one item each give, and when it is taken."""
+"""The chunked delta-rule scan whose blocks share the chunks of all items: bit for bit what blocks with one item each give, when it comes into question by the number of
+items, and when the lengths say that it pays."""
+import heapq
+import random
+
 import pytest
 import torch
 
@@ -40,10 +44,13 @@ def _inputs(news, olds, H, KH, D, Dv, gla, seed):
 ])
 def test_the_bits_of_whole_items(news, olds, H, KH, D, Dv, gla):
     from nanorlhf_b200.ops import hybrid as hy
-    assert _C.delta_scan_shared(len(news), sum(news), H, Dv, SMS)
     plan, qkv, beta, decay, state = _inputs(news, olds, H, KH, D, Dv, gla, len(news) + D)
     o, s = torch.empty(sum(news), H * Dv, device="cuda"), state.clone()
-    hy.delta_scan(qkv, KH * D, 2 * KH * D, beta, decay, s, o, plan, KH, False, impl="chunked")
+    hy.delta_scan(qkv, KH * D, 2 * KH * D, beta, decay, s, o, plan, KH, False, impl="line")
+    for plan.lengths in (None, news):                                      # as the lengths say, found by the GPU or by the host
+        o0, s0 = torch.empty_like(o), state.clone()
+        hy.delta_scan(qkv, KH * D, 2 * KH * D, beta, decay, s0, o0, plan, KH, False, impl="chunked")
+        assert torch.equal(o, o0) and torch.equal(s, s0)
     # entry by entry there are fewer items than SMs
     o1, s1, cu = torch.empty_like(o), state.clone(), plan.cu.tolist()
     for e in range(len(news)):
@@ -52,3 +59,79 @@ def test_the_bits_of_whole_items(news, olds, H, KH, D, Dv, gla):
                       torch.tensor([0, news[e]], dtype=torch.int32, device="cuda"), plan.start[e:e + 1].contiguous(), plan.state_slot[e:e + 1].contiguous(),
                       KH, False, 5)
     assert torch.equal(o, o1) and torch.equal(s, s1)
+
+
+def test_hosts_with_the_lengths_decide_without_the_gpu():
+    assert _C.delta_line_pays([2048] * 10, 16, 128, SMS) and not _C.delta_line_pays([4000] + [400] * 9, 16, 128, SMS)
+    rng = random.Random(1)
+    for _ in range(300):
+        news, heads = [rng.randint(0, 2000) for _ in range(rng.randint(1, 40))], rng.choice([4, 16, 40])
+        if _C.delta_line_pays(news, heads, 128, SMS):
+            chunks = _chunks(news)
+            assert 1.13 * max(max(chunks), -(-sum(chunks) * heads // SMS)) + 4 < 0.9 * _whole(chunks, heads, SMS)
+
+
+def _chunks(news):
+    return [max(1, -(-n // 32)) for n in news]
+
+
+def _cu(news):
+    return torch.tensor([0, *torch.tensor(news).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+
+
+def _whole(chunks, items, sms):
+    """chunks in a row when whole items go to the SM that is free first"""
+    free = [0] * sms
+    for n in chunks:
+        for _ in range(items):
+            heapq.heappush(free, heapq.heappop(free) + n)
+    return max(free)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("news,heads,Dv,taken", [
+    ([2048] * 10, 16, 128, True), ([700] * 12, 16, 128, True), ([300] * 11, 16, 64, True), ([900] * 5, 16, 200, True), ([2048] * 16, 16, 128, False),
+    ([4000] + [400] * 9, 16, 128, False), ([700] + [33] * 9 + [350] * 10, 8, 64, False),      # by the mean length they were taken, and slower for it
+])
+def test_lengths_decide(news, heads, Dv, taken):
+    assert bool(_C.delta_line_plan(_cu(news), heads, Dv, SMS)[0]) == taken == _C.delta_line_pays(news, heads, Dv, SMS)
+
+
+@pytest.mark.gpu
+def test_never_taken_where_whole_items_are_as_fast():
+    rng, taken = random.Random(4), 0
+    for i in range(300):
+        heads, E, lo = rng.choice([4, 8, 16, 32]), rng.randint(2, 60), rng.choice([30, 300, 900])
+        news = [int(lo * (2000 / lo) ** rng.random()) if i % 2 else rng.randint(900, 1000) for _ in range(E)]
+        chunks = _chunks(news)
+        pays = _C.delta_line_pays(news, heads, 128, SMS)
+        assert bool(_C.delta_line_plan(_cu(news), heads, 128, SMS)[0]) == pays
+        if pays:
+            taken += 1
+            line = max(max(chunks), -(-sum(chunks) * heads // SMS))
+            assert 1.13 * line + 4 < 0.9 * _whole(chunks, heads, SMS)
+    assert taken >= 10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("news,heads,Dv,blocks", [([400] * 10, 16, 128, 148), ([700] + [33] * 9 + [0, 350, 1] * 5, 8, 300, 148), ([5, 90], 3, 64, 7), ([64] * 40, 4, 128, 13)])
+def test_every_chunk_lies_in_one_segment(news, heads, Dv, blocks):
+    taken, ends, segments = _C.delta_line_plan(_cu(news), heads, Dv, blocks, True)
+    assert taken
+    ends, segments, chunks, parts = ends.tolist(), segments.tolist(), _chunks(news), -(-Dv // 128)
+    per, seen, cu = max(max(chunks), -(-sum(chunks) * heads * parts // blocks)), {}, _cu(news).tolist()
+    for b in range(blocks):
+        mine = segments[ends[0][b]:ends[1][b]]
+        assert sum(s[1] for s in mine) <= per
+        for i, (t0, n, t1, h, cb0, e, came, goes) in enumerate(mine):
+            assert n > 0 and t1 == cu[e + 1] and (t0 - cu[e]) % 32 == 0
+            assert not goes or i == 0                                    # what another block waits for is computed first
+            assert not came or i == len(mine) - 1                        # what waits for another block is computed last
+            if came:
+                nxt = segments[ends[0][b + 1]]
+                assert nxt[7] and nxt[3:6] == [h, cb0, e] and nxt[0] + 32 * nxt[1] == t0
+            seen.setdefault((e, h, cb0), []).append(((t0 - cu[e]) // 32, n))
+    assert len(seen) == len(news) * heads * parts
+    for (e, _, _), runs in seen.items():
+        runs.sort()
+        assert runs[0][0] == 0 and all(a + n == b for (a, n), (b, _) in zip(runs, runs[1:])) and runs[-1][0] + runs[-1][1] == chunks[e]
