@@ -786,7 +786,7 @@ std::tuple<int64_t, Tensor, Tensor> delta_line_plan(const Tensor& cu, int64_t he
   check(nrl_delta_line(i32(cu, "cu"), static_cast<int>(E), static_cast<int>(heads), static_cast<int>(Dv), forced, scratch.data_ptr(), static_cast<int>(blocks), cur_stream()),
         "delta_line_plan");
   const Tensor ints = scratch.slice(0, blocks * 128 * 128 * 4).view(torch::kInt32);
-  return {ints[3 * blocks].item<int64_t>(), ints.slice(0, 0, 2 * blocks).view({2, blocks}).clone(), ints.slice(0, 4 * blocks, 4 * blocks + 8 * n).view({n, 8}).clone()};
+  return {ints[3 * blocks].item<int64_t>(), ints.slice(0, 0, 2 * blocks).view({2, blocks}).clone(), ints.slice(0, 3 * blocks + 4, 3 * blocks + 4 + 8 * n).view({n, 8}).clone()};
 }
 
 }  // namespace

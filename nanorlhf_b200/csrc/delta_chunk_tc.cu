@@ -133,7 +133,8 @@ NRL_DEVICE int pair_b(int pr) { return (0x001012 >> (4 * pr)) & 3; }
 // More items (entry, head, 128 columns) than SMs: their chunks lie on a line, entry by entry, and block j takes the `per` chunks of it from j per on, an even share or
 // the longest item.  An item that a block's end cuts is computed first by the block behind, at that block's start (its first chunks, as many as lie there
 // on the line), and then by this block, at its end, from the state that the other has left: no item is longer than `per`, so that state is there by then.
-// Blocks start from the line's end, so that none waits for one that starts later; should the wait run out all the same, the state becomes NaN.
+// Blocks take their places from the line's end in the order in which they start (a ticket), so that none waits for one that has not started; should the wait run out
+// all the same, the state becomes NaN.
 // The segments are laid out by a kernel of their own, and between two segments the block starts anew (barriers and all): code that every warp runs through is
 // dear here.  With phases that run on over the segments a chunk took 19 % longer, so 13 % (92 KB of code, 78 for whole items).
 // 10 x 2048 tokens, 16 heads of 128 x 128 (160 items of 64 chunks on 148 SMs): two rounds of 64 chunks 625 us, 70 chunks in a row 381 us.
@@ -152,6 +153,7 @@ struct DcLine {
   int* handed;                // [blocks] 1 once the state that the block hands on is there
   float* carry;               // [blocks][128][128]
   int* taken;                 // [1] the line is taken, else a block has an item
+  int* ticket;                // [1] blocks that have started
 };
 constexpr int kDcMaxEntries = 4096;
 
@@ -197,7 +199,10 @@ __global__ void __launch_bounds__(1024) delta_line_kernel(const int* __restrict_
   __syncthreads();
   whole = __reduce_max_sync(0xffffffffu, least[tid & 31]);
   const bool taken = forced || line_pays(per, whole);
-  if (tid == 0) *l.taken = taken ? 1 : 0;
+  if (tid == 0) {
+    *l.taken = taken ? 1 : 0;
+    *l.ticket = 0;
+  }
   if (!taken) return;
   for (int q = tid; q < E * items; q += blockDim.x) {
     const int e = q / items, k = q - e * items, n = from[e + 1] - from[e], s = from[e] * items + k * n, t0 = cu[e], t1 = cu[e + 1];
@@ -282,8 +287,12 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
     mbar_init(o2_full, 1);
     fence_mbar_init();
   };
+  volatile int* ticket = reinterpret_cast<volatile int*>(tmem_ptr + 1);
   if (warp == 20) {
-    if (lane == 0) init_barriers();
+    if (lane == 0) {
+      init_barriers();
+      if (LINE) *ticket = atomicAdd(p.line.ticket, 1);
+    }
     __syncwarp();
     tmem_alloc(tmem_ptr, 512);
   }
@@ -293,8 +302,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
   const uint32_t tmem = *tmem_ptr;
 
   const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  const int line = gridDim.x - 1 - blockIdx.x;
-  const int first = LINE ? p.line.first[line] : 0, last = LINE ? p.line.last[line] : 1;      // segments of this block
+  auto line = [&]() { return static_cast<int>(gridDim.x) - 1 - *ticket; };      // this block's place, read again rather than kept
+  const int first = LINE ? p.line.first[line()] : 0, last = LINE ? p.line.last[line()] : 1;      // segments of this block
   int e, h, cb0, t0, n_chunks, t1;
   auto take = [&](int i) {
     if (LINE) {
@@ -476,8 +485,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         long step = p.Dv;
         bool there = true;
         if (LINE && p.line.segments[i].in) {
-          there = dc_handed(p.line.handed + line + 1);
-          ld = p.line.carry + (static_cast<long>(line + 1) * 128 + half * 64) * 128 + (warp & 3) * 32 + lane;
+          there = dc_handed(p.line.handed + line() + 1);
+          ld = p.line.carry + (static_cast<long>(line() + 1) * 128 + half * 64) * 128 + (warp & 3) * 32 + lane;
           step = 128;
           from = rows;
         }
@@ -518,7 +527,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         if (LINE) {                                          // the segment is looked up again: nothing of it is kept over the loop
           take(i);
           rows = cb0 + (warp & 3) * 32 + lane < p.Dv ? p.D - half * 64 : 0;
-          gS = out ? p.line.carry + (static_cast<long>(line) * 128 + half * 64) * 128 + (warp & 3) * 32 + lane
+          gS = out ? p.line.carry + (static_cast<long>(line()) * 128 + half * 64) * 128 + (warp & 3) * 32 + lane
                    : p.state + ((static_cast<long>(p.state_slot[e]) * p.heads + h) * p.D + half * 64) * p.Dv + cb0 + (warp & 3) * 32 + lane;
           if (out) step = 128;
         }
@@ -529,7 +538,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_tc_kernel(const DcP
         if (out) {
           __threadfence();
           named_barrier_sync(2, NH * 128);
-          if (threadIdx.x == 4 * 32) asm volatile("st.release.gpu.global.b32 [%0], 1;" ::"l"(p.line.handed + line) : "memory");
+          if (threadIdx.x == 4 * 32) asm volatile("st.release.gpu.global.b32 [%0], 1;" ::"l"(p.line.handed + line()) : "memory");
         }
       } else {
         for (int n = 0; n < n_chunks; ++n) {
@@ -837,7 +846,7 @@ cudaError_t launch_delta_chunk(unsigned grid, const DcParams& p, cudaStream_t s)
 // D <= 128, one decay per head; beta == nullptr: plain accumulation; rows16: rows of q, k and v start and end on 16-byte boundaries; line: null, or (rows16)
 // nrl_delta_line_bytes() of scratch with which `blocks` blocks share the chunks of all items, where that pays or it is forced
 extern "C" long nrl_delta_line_bytes(long E, int heads, int Dv, int blocks) {
-  return blocks * (128l * 128 * 4 + 16) + (E * heads * ((Dv + 127) / 128) + blocks) * static_cast<long>(sizeof(nrl::DcSegment));
+  return blocks * (128l * 128 * 4 + 12) + 16 + (E * heads * ((Dv + 127) / 128) + blocks) * static_cast<long>(sizeof(nrl::DcSegment));
 }
 static nrl::DcLine line_in(void* scratch, int blocks) {
   nrl::DcLine l{};
@@ -845,8 +854,9 @@ static nrl::DcLine line_in(void* scratch, int blocks) {
   l.first = reinterpret_cast<int*>(l.carry + blocks * 128l * 128);
   l.last = l.first + blocks;
   l.handed = l.last + blocks;
-  l.taken = l.handed + blocks;                             // of the fourth run of `blocks` numbers
-  l.segments = reinterpret_cast<nrl::DcSegment*>(l.handed + 2 * blocks);
+  l.taken = l.handed + blocks;
+  l.ticket = l.taken + 1;
+  l.segments = reinterpret_cast<nrl::DcSegment*>(l.taken + 4);
   return l;
 }
 extern "C" int nrl_delta_line_pays(const long* tokens, long E, int heads, int Dv, int blocks) {

@@ -13,3 +13,11 @@ def test_zeros_are_fenced_before_the_copies():
     between = src[zeros:copies]
     # statements of all the storing threads, in this order: fence, then the barrier behind which one warp issues the copies
     assert re.match(r"\s*fence_proxy_async_smem\(\);\s*named_barrier_sync\(1, kDcLoaders\);", between)
+
+
+def test_a_blocks_place_on_the_line_is_the_order_of_its_start():
+    """A block waits for its neighbour's state.  CUDA does not say in which order blocks start, so the place comes from a counter that each takes when it runs."""
+    with open(os.path.join(CSRC, "delta_chunk_tc.cu")) as f:
+        src = re.sub(r"//[^\n]*", "", f.read())
+    assert re.search(r"\*ticket = atomicAdd\(p\.line\.ticket, 1\);", src) and re.search(r"auto line = \[&\]\(\) \{[^}]*\*ticket; \};", src)
+    assert not re.search(r"blockIdx[^;]*line|line[^;]*blockIdx", src) and src.count("*l.ticket = 0;") == 1
