@@ -1635,7 +1635,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     const PairCut c = pair_choice(M, N, K, sms, [&](int s) { return fits.at(s); }, [&](int, int s) { return 2 * s <= 8 ? fits.at(2 * s) : 0; });
     return std::make_tuple(c.bn, c.splits, c.clusters);
   }, "(tile width, ranges, by clusters) of a cut on pairs of blocks, ranges 1 where it is not taken");
-  m.def("gemm_tc_pair_clusters", &nrl_gemm_tc_pair_clusters);
   m.def("gemm_tc_split_clusters", &nrl_gemm_tc_split_clusters, py::arg("block_n"), py::arg("splits"));
   m.def("gemm_tc_swiglu_pair_keep", &gemm_tc_swiglu_pair_keep, "(act, gate, up) of gemm_tc_swiglu_pair with adapters");
   m.def("gemm_tc_dswiglu", &gemm_tc_dswiglu, "(d gate, d up) of silu(gate) * up behind a projection's backward");
