@@ -448,8 +448,6 @@ torch::Tensor gemm_tc(const torch::Tensor& a, const torch::Tensor& b, bool a_mn,
 //   output                          7.9 -> 5.9    10.8 -> 7.4   12.5 -> 6.9   14.4 -> 8.1   17.0 -> 10.5
 //   dt of gate and up               16.9 -> 9.0   17.4 -> 9.7   18.9 -> 12.5  30.2 -> 24.6  48.2 -> 42.2
 //   dt of query, key and value      13.3 -> 9.7   13.5 -> 9.7   14.1 -> 10.0  14.6 -> 10.0  16.3 -> 11.4   (four ranges, up to 700 tokens: 6.1)
-// 3584 / 18944 wide, the five together: 60 tokens 76 -> 54, 250 86 -> 59, 1000 124 -> 85, 6601 338 -> 292, 16 384 700 -> 664; single ones lose up to 1.9 us below 300
-// tokens and 4 us at 16 384.
 // What bounds the large ones is the copy of the 8960-wide operand, 118 MB (18 us) a product, which each product reads once.
 int64_t multi_splits(const std::vector<int64_t>& tiles, const std::vector<int64_t>& blocks, int64_t sms, const std::function<int(int)>& fits) {
   int64_t total = 0, longest = 0, best = 1;
@@ -466,6 +464,37 @@ int64_t multi_splits(const std::vector<int64_t>& tiles, const std::vector<int64_
     if (t < least) { least = t; best = s; }
   }
   return best;
+}
+// Narrow products [wide, K] x [K, narrow] in one launch or a GEMM each, by this estimate (us): a round of the grid's tiles starts and ends in 3.9 and 0.018 for each
+// column of a factor; a launch of its own, which begins while the one in front ends, in 3.1 and 0.5 a round; a block of 64 contraction columns takes 0.2, in a full
+// round 0.38, when its tiles wait for memory; a cut product's blocks fill the SMs that it leaves; below 32 columns GEMMs of their own take 0.8 more and a quarter
+// more of contraction.  The line lies at 0.92, where the estimate's errors end.
+// us, one launch / own.  Factors' gradients of one 18 944 x 3584 wide projection: rank 64, 60 tokens 10.4 / 8.6, 1000 16.6 / 15.5, 4000 45 / 36, 16 384 146 / 114; rank
+// 32, 4000 43.6 / 39.9; rank 16, 60 tokens 8.8 / 9.9 (one), 4000 42 / 49 (one).  Of gate, up and down of that width, rank 64: 8 tokens 21.7 / 19.4, 1000 42.0 / 46.8
+// (one), 16 384 313 / 323 (one); 28 672 x 8192: 8 tokens 31.4 / 22.1, 1000 62.9 / 58.4, 16 384 498 / 540 (one); up to 14 336 x 4096 one launch always.  Inputs dY B of
+// two 8960 wide projections: 9000 tokens 55 / 59 (one), 12 000 87 / 78, 16 384 99 / 97 (one); of query, key and value 1536 wide: 9000 12.5 / 17.0 (one), 16 384 22.7 /
+// 18.1, 32 768 49 / 35.
+bool multi_pays(const std::vector<int64_t>& wide, const std::vector<int64_t>& narrow, const std::vector<int64_t>& contraction, int64_t sms) {
+  auto run = [&](int64_t tiles, double blocks) {
+    const int64_t rest = tiles % sms;
+    return blocks * (0.38 * (tiles / sms) + (rest > 0 ? std::max(0.2, 0.38 * rest / sms) : 0.0));
+  };
+  int64_t total = 0, rank = 64;
+  double own = 0.0, work = 0.0, mean = 0.0;                // mean: blocks of contraction of a tile
+  for (size_t i = 0; i < wide.size(); ++i) {
+    const int64_t tiles = ((wide[i] + 127) / 128) * ((narrow[i] + 63) / 64), blocks = (contraction[i] + 63) / 64;
+    if (tiles < 1) return true;                            // refused there
+    const int64_t s = std::max<int64_t>(1, std::min<int64_t>({8, sms / tiles, blocks / 4}));
+    work += run(tiles * s, static_cast<double>(blocks) / s);
+    own += (s > 1 ? 1.0 : 0.0) + 0.5 * ((tiles + sms - 1) / sms);
+    total += tiles;
+    mean += static_cast<double>(tiles * blocks);
+    rank = std::min(rank, narrow[i]);
+  }
+  if (total <= sms) return true;
+  mean /= total;
+  own += rank < 32 ? 1.25 * work + 3.9 * wide.size() : work + 3.1 * wide.size();
+  return own >= 0.92 * (run(total, mean) + ((total + sms - 1) / sms) * (3.9 + 0.018 * rank));
 }
 void gemm_tc_multi(const std::vector<torch::Tensor>& a, const std::vector<torch::Tensor>& b, std::vector<torch::Tensor> out, const std::vector<bool>& transposed,
                    const std::vector<double>& alpha, bool a_mn, int64_t splits_req) {
@@ -1640,6 +1669,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_dswiglu", &gemm_tc_dswiglu, "(d gate, d up) of silu(gate) * up behind a projection's backward");
   m.def("gemm_tc_multi", &gemm_tc_multi, "several products with narrow results in one launch", py::arg("a"), py::arg("b"), py::arg("out"), py::arg("transposed"),
         py::arg("alpha"), py::arg("a_mn"), py::arg("splits") = 0);
+  m.def("gemm_tc_multi_pays", [](const std::vector<int64_t>& wide, const std::vector<int64_t>& narrow, const std::vector<int64_t>& contraction, int64_t sms) {
+    return multi_pays(wide, narrow, contraction, sms > 0 ? sms : num_sms());
+  }, "narrow products share a launch", py::arg("wide"), py::arg("narrow"), py::arg("contraction"), py::arg("sms") = 0);
   m.def("gemm_tc_multi_splits", [](const std::vector<int64_t>& tiles, const std::vector<int64_t>& blocks, int64_t sms, const std::vector<int>& fits) {
     return multi_splits(tiles, blocks, sms, [&](int s) { return fits.at(s); });
   });

@@ -150,24 +150,28 @@ def sum_gemms(a, b):
     return out
 
 
-def _narrow(r: int) -> bool:
-    """Whether an adapter's products share launches of up to six, in tiles 64 wide.  Wider factors fill wider tiles by themselves: rank 32 at 6601 tokens of a
-    1536 / 8960 wide MLP 88 -> 66 us in one launch, rank 64 87 -> 69, rank 128 95 -> 107, rank 256 121 -> 187."""
-    return r <= 64
+def _share(wide, narrow, contraction, r: int) -> bool:
+    """Whether an adapter's products [wide, contraction] x [contraction, narrow] share a launch, in tiles 64 wide: where an estimate says so
+    (csrc/bindings.cpp: multi_pays) and up to rank 64.  Wider factors fill wider tiles by themselves: rank 32 at 6601 tokens of a 1536 / 8960 wide MLP 88 -> 66 us
+    in one launch, rank 64 87 -> 69, rank 128 95 -> 107, rank 256 121 -> 187."""
+    return r <= 64 and _native_mod.ext().gemm_tc_multi_pays(wide, narrow, contraction)
 
 
 def _adapter_grads(factors, inputs, r):
     """``dy_i^T t_i`` [N_i, r_i] for every (dy_i, t_i) of ``factors`` and ``t'_j^T x_j`` [r_j, K_j] for every (t'_j, x_j) of ``inputs``, of adapters
     whose largest rank is ``r``."""
-    if not _narrow(r):
-        return [gemm(dy, t, a_mn=True, b_mn=True) for dy, t in factors], [gemm(t, x, a_mn=True, b_mn=True) for t, x in inputs]
-    a, b = [dy for dy, _ in factors] + [x for _, x in inputs], [t for _, t in factors] + [t for t, _ in inputs]
-    out = [dy.new_empty(dy.shape[1], t.shape[1]) for dy, t in factors] + [x.new_empty(t.shape[1], x.shape[1]) for t, x in inputs]
-    flip = [False] * len(factors) + [True] * len(inputs)
-    for i in range(0, len(a), 6):
-        j = slice(i, i + 6)
-        _native_mod._count()
-        _native_mod.ext().gemm_tc_multi(a[j], b[j], out[j], flip[j], [1.0] * len(a[j]), True)
+    own = lambda dy, t, flip: gemm(t, dy, a_mn=True, b_mn=True) if flip else gemm(dy, t, a_mn=True, b_mn=True)      # noqa: E731
+    wide = [(dy, t, False) for dy, t in factors] + [(x, t, True) for t, x in inputs]
+    out, ext = [], _native_mod.ext()
+    for i in range(0, len(wide), 6):
+        part = wide[i:i + 6]
+        if _share([y.shape[1] for y, _, _ in part], [t.shape[1] for _, t, _ in part], [y.shape[0] for y, _, _ in part], r):
+            to = [y.new_empty(*((t.shape[1], y.shape[1]) if flip else (y.shape[1], t.shape[1]))) for y, t, flip in part]
+            _native_mod._count()
+            ext.gemm_tc_multi([y for y, _, _ in part], [t for _, t, _ in part], to, [flip for _, _, flip in part], [1.0] * len(part), True)
+            out += to
+        else:
+            out += [own(*p) for p in part]
     return out[:len(factors)], out[len(factors):]
 
 
@@ -176,14 +180,14 @@ def _group_backward(gs, x2, t_cat, a_cat, ws, Bs, s, need_x, more_factors=(), mo
     n, r = len(gs), t_cat.shape[1] // len(gs)
     tp_cat = torch.empty(x2.shape[0], n * r, dtype=x2.dtype, device=x2.device)
     tps = [tp_cat[:, i * r:(i + 1) * r] for i in range(n)]                                      # t'_i = s dy_i B_i
-    if _narrow(r):
-        for i in range(0, n, 6):
-            j = slice(i, i + 6)
+    for i in range(0, n, 6):
+        part = list(zip(gs, Bs, tps))[i:i + 6]
+        if _share([g.shape[0] for g, _, _ in part], [r] * len(part), [g.shape[1] for g, _, _ in part], r):
             _native_mod._count()
-            _native_mod.ext().gemm_tc_multi(list(gs[j]), list(Bs[j]), tps[j], [False] * len(tps[j]), [s] * len(tps[j]), False)
-    else:
-        for g, b, tp in zip(gs, Bs, tps):
-            gemm(g, b, b_mn=True, alpha=s, out=tp)
+            _native_mod.ext().gemm_tc_multi(*(list(x) for x in zip(*part)), [False] * len(part), [s] * len(part), False)
+        else:
+            for g, b, tp in part:
+                gemm(g, b, b_mn=True, alpha=s, out=tp)
     gx = sum_gemms([*gs, tp_cat], [*ws, a_cat]) if need_x else None                           # sum_i dy_i W_i + [t'_1 .. t'_n] [A_1; ..; A_n]
     gbs, gas = _adapter_grads([(gs[i], t_cat[:, i * r:(i + 1) * r]) for i in range(n)] + list(more_factors), [(tp_cat, x2)] + list(more_inputs),
                               max([r] + [t.shape[1] for _, t in more_factors]))
@@ -201,7 +205,8 @@ def _projections(x2, ws, bs, ts=(), Bs=()):
 class _LoraGroupFn(torch.autograd.Function):
     """Several LoRA projections of ONE input (q / k / v, gate / up): the rank-r down-projections share a launch
     (``t = s x [A_1; ...; A_n]^T``), the base GEMMs share another and take their slices of ``t`` as dual-source-K operands, and in the backward the
-    gradients of all factors come out of one launch and ``dx`` out of one over all projections and the LoRA term.  Compared with n independent ``_LoraLinearFn``: n - 1 fewer skinny launches per direction, ``x`` is re-read once instead of n times."""
+    gradients of all factors come out of one launch and ``dx`` out of one over all projections and the LoRA term.  Compared with
+    n independent ``_LoraLinearFn``: n - 1 fewer skinny launches per direction, ``x`` is re-read once instead of n times."""
 
     @staticmethod
     def forward(ctx, x, scaling, n, *flat):
