@@ -2,6 +2,7 @@
 // Kernels live in plain .cu translation units with a C launch API (kernels.h, gemm_sm100.h); this file
 // only validates tensors, builds TMA descriptors and forwards the current CUDA stream.
 #include <functional>
+#include <mutex>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/SavedTensorHooks.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -891,25 +892,37 @@ constexpr int64_t kKeptLogitsMax = 4ll << 30;
 bool keeps_logits(int64_t M, int64_t V, int64_t taken, int64_t total) {
   return M > 0 && V > 0 && V % 8 == 0 && M <= kKeptLogitsMax / 4 / V && taken <= total / 4 * 3 - 8 * M * V;
 }
+// What others than this process's allocator hold of the current device: other processes, communicators, the context.  The driver is asked the first time and where the
+// allocator has reserved or given back 1 GiB since: it answers in 70 us at best and, on a machine that others use too, in up to 50 ms.  While nothing is reserved, logits
+// that are kept take memory that this process holds already.
+struct HeldByOthers { int64_t reserved = -1, bytes = 0, total = 0; };
+HeldByOthers held_by_others(int64_t reserved) {
+  static std::mutex mutex;
+  static nrl::PerDevice<HeldByOthers> known;
+  const std::lock_guard<std::mutex> lock(mutex);
+  HeldByOthers& h = known.here();
+  if (h.reserved < 0 || std::abs(reserved - h.reserved) >= (1ll << 30)) {
+    c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};
+    size_t free_bytes = 0, all = 0;
+    if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) {
+      cudaGetLastError();
+      return {-1, 0, 0};
+    }
+    h.reserved = reserved;
+    h.total = static_cast<int64_t>(all);
+    h.bytes = std::max<int64_t>(0, h.total - static_cast<int64_t>(free_bytes) - reserved);
+  }
+  return h;
+}
 c10::optional<torch::Tensor> lmhead_logits_buffer(const torch::Tensor& hidden, int64_t V) {
   const int64_t M = hidden.size(0);
   if (!keeps_logits(M, V, 0, INT64_MAX) || at::SavedTensorDefaultHooks::get_hooks().has_value()) return c10::nullopt;
   c10::cuda::CUDAGuard guard(hidden.device());
   try {
     // What the allocator has reserved counts as taken, handed out or not: blocks that wait in a captured graph's pool serve nobody else.
-    int64_t total = at::cuda::getCurrentDeviceProperties()->totalGlobalMem;
-    int64_t taken = c10::cuda::CUDACachingAllocator::getDeviceStats(hidden.device().index()).reserved_bytes[0].current;
-    if (4 * M * V >= (256 << 20)) {      // worth the 73 us in which the driver tells what others hold too: other processes, communicators, the context
-      c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};
-      size_t free_bytes = 0, all = 0;
-      if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) {
-        cudaGetLastError();
-        return c10::nullopt;
-      }
-      total = static_cast<int64_t>(all);
-      taken = total - static_cast<int64_t>(free_bytes);
-    }
-    if (!keeps_logits(M, V, taken, total)) return c10::nullopt;
+    const int64_t reserved = c10::cuda::CUDACachingAllocator::getDeviceStats(hidden.device().index()).reserved_bytes[0].current;
+    const HeldByOthers others = held_by_others(reserved);
+    if (others.reserved < 0 || !keeps_logits(M, V, others.bytes + reserved, others.total)) return c10::nullopt;
     return torch::empty({M, V}, hidden.options().dtype(torch::kFloat32));
   } catch (const c10::Error&) {
     return c10::nullopt;

@@ -20,7 +20,7 @@ def test_sizes_that_keep_nothing(M, V):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows", [64, 600])                      # 39 MB, and 365 MB, for which the driver is asked
+@pytest.mark.parametrize("rows", [64, 600])
 def test_memory_that_is_only_reserved_counts(rows):
     import torch
     V = 151936
@@ -51,3 +51,29 @@ def test_a_captured_step_asks_too():
         got = step()
     graph.replay()
     assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+def test_the_driver_is_not_asked_while_nothing_is_reserved():
+    """It may take milliseconds to answer."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    from nanorlhf_b200 import ops
+    h = torch.randn(600, 64, device="cuda").bfloat16().requires_grad_()
+    w, t = torch.randn(151936, 64, device="cuda").bfloat16(), torch.zeros(600, dtype=torch.long, device="cuda")
+
+    def step():
+        lp, _ = ops.lmhead_logprob(h, w, t, 1.0, False)
+        return torch.autograd.grad(lp.sum(), h)[0]
+
+    def asked(f):
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+            f()
+            torch.cuda.synchronize()
+        return sum(e.name == "cudaMemGetInfo" for e in p.events())
+    step()
+    step()
+    if asked(torch.cuda.mem_get_info) == 0:
+        pytest.skip("the profiler does not show such calls")
+    assert asked(lambda: [step() for _ in range(3)]) == 0
