@@ -247,14 +247,14 @@ struct ClusterFits {
 const ClusterFits& cluster_fits() {
   static nrl::PerDevice<ClusterFits> all;
   ClusterFits& f = all.here();
-  if (!f.known) {
+  if (!__atomic_load_n(&f.known, __ATOMIC_ACQUIRE)) {        // threads that come at once ask for the same numbers
     for (int s = 2; s <= 8; ++s)
       for (int i = 0; i < 2; ++i) f.single[i][s] = nrl_gemm_tc_split_clusters(64 << i, s);
     for (int s = 2; s <= 4; ++s)
       for (int i = 0; i < 3; ++i) f.pairs[i][s] = nrl_gemm_tc_pair_clusters(128 + 64 * i, s);
     for (int s = 1; s <= 8; ++s)
       for (int i = 0; i < 2; ++i) f.multi[i][s] = nrl_gemm_tc_multi_clusters(i, s);
-    f.known = true;
+    __atomic_store_n(&f.known, true, __ATOMIC_RELEASE);
   }
   return f;
 }
