@@ -87,7 +87,8 @@ def linears(x, ws, bs):
     if x.numel() == 0 or not all(supported(x, w) for w in ws):
         return None
     x2 = _rows(x)
-    if any(_native_mod.ext().gemm_tc_auto_splits(x2.shape[0], *w.shape, x2.get_device()) > 1 for w in ws):
+    pick, dev = _native_mod.ext().gemm_tc_auto_splits, x2.get_device()
+    if any(pick(x2.shape[0], *shape, dev) > 1 for shape in {w.shape for w in ws}):
         return None
     return [y.view(*x.shape[:-1], y.shape[-1]) for y in _projections(x2, ws, bs)]
 

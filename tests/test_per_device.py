@@ -50,7 +50,7 @@ def test_choices_are_asked_for_the_operands_device(monkeypatch):
     monkeypatch.setattr(torch.Tensor, "get_device", lambda t: 3)
     monkeypatch.setattr(gemm, "gemm", lambda a, b, **kw: torch.zeros(a.shape[0], b.shape[1]))
     x, w = torch.zeros(16, 8, dtype=torch.bfloat16), torch.zeros(8, 8, dtype=torch.bfloat16)
-    assert gemm.linears(x, [w, w], [None, None]) is None
+    assert gemm.linears(x, [w, torch.zeros(16, 8, dtype=torch.bfloat16)], [None, None]) is None
     assert gemm.swiglu_linears(x, (w, None, None), (w, None, None)) is None
     gemm.sum_gemms([x, x], [w, w])
     assert len(asked) == 4 and set(asked) == {3}
