@@ -484,7 +484,7 @@ bool multi_pays(const std::vector<int64_t>& wide, const std::vector<int64_t>& na
   double own = 0.0, work = 0.0, mean = 0.0;                // mean: blocks of contraction of a tile
   for (size_t i = 0; i < wide.size(); ++i) {
     const int64_t tiles = ((wide[i] + 127) / 128) * ((narrow[i] + 63) / 64), blocks = (contraction[i] + 63) / 64;
-    if (tiles < 1) return true;                            // refused there
+    if (tiles < 1) return true;
     const int64_t s = std::max<int64_t>(1, std::min<int64_t>({8, sms / tiles, blocks / 4}));
     work += run(tiles * s, static_cast<double>(blocks) / s);
     own += (s > 1 ? 1.0 : 0.0) + 0.5 * ((tiles + sms - 1) / sms);
@@ -497,15 +497,12 @@ bool multi_pays(const std::vector<int64_t>& wide, const std::vector<int64_t>& na
   own += rank < 32 ? 1.25 * work + 3.9 * wide.size() : work + 3.1 * wide.size();
   return own >= 0.92 * (run(total, mean) + ((total + sms - 1) / sms) * (3.9 + 0.018 * rank));
 }
-void gemm_tc_multi(const std::vector<torch::Tensor>& a, const std::vector<torch::Tensor>& b, std::vector<torch::Tensor> out, const std::vector<bool>& transposed,
-                   const std::vector<double>& alpha, bool a_mn, int64_t splits_req) {
+// if_faster: false, and nothing done, where GEMMs of their own are
+bool gemm_tc_multi(const std::vector<torch::Tensor>& a, const std::vector<torch::Tensor>& b, std::vector<torch::Tensor> out, const std::vector<bool>& transposed,
+                   const std::vector<double>& alpha, bool a_mn, int64_t splits_req, bool if_faster) {
   const size_t n = a.size();
   TORCH_CHECK(n >= 1 && n <= nrl::tc::kMultiMax && b.size() == n && out.size() == n && transposed.size() == n && alpha.size() == n, "gemm_tc_multi: one to six products");
-  c10::cuda::CUDAGuard guard(a[0].device());
-  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  CUtensorMap maps[2 * nrl::tc::kMultiMax];
-  nrl::tc::TcMultiProduct q[nrl::tc::kMultiMax];
-  std::vector<int64_t> tiles, blocks;
+  std::vector<int64_t> tiles, blocks, wide, narrow, contraction;
   for (size_t i = 0; i < n; ++i) {
     check_tc_operand(a[i], "a");
     check_tc_operand(b[i], "b");
@@ -513,15 +510,27 @@ void gemm_tc_multi(const std::vector<torch::Tensor>& a, const std::vector<torch:
     const int64_t M = a_mn ? a[i].size(1) : a[i].size(0), K = a_mn ? a[i].size(0) : a[i].size(1), N = b[i].size(1);
     TORCH_CHECK(b[i].size(0) == K && N % 8 == 0 && M > 0 && N > 0 && K > 0, "gemm_tc_multi: shapes differ");
     TORCH_CHECK(out[i].size(transposed[i] ? 1 : 0) == M && out[i].size(transposed[i] ? 0 : 1) == N, "gemm_tc_multi: out has the wrong shape");
-    maps[2 * i] = nrl::make_tma_2d(a[i].data_ptr(), a[i].size(0), a[i].size(1), a[i].stride(0) * 2, a_mn ? 64 : 128, 64, BF, 2);
-    maps[2 * i + 1] = nrl::make_tma_2d(b[i].data_ptr(), K, N, b[i].stride(0) * 2, 64, 64, BF, 2);
-    q[i] = {static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<float>(alpha[i]), out[i].data_ptr(), out[i].stride(0), transposed[i] ? 1 : 0};
+    wide.push_back(M);
+    narrow.push_back(N);
+    contraction.push_back(K);
     tiles.push_back(((M + 127) / 128) * ((N + 63) / 64));
     blocks.push_back((K + 63) / 64);
+  }
+  if (if_faster && !multi_pays(wide, narrow, contraction, num_sms())) return false;
+  c10::cuda::CUDAGuard guard(a[0].device());
+  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  CUtensorMap maps[2 * nrl::tc::kMultiMax];
+  nrl::tc::TcMultiProduct q[nrl::tc::kMultiMax];
+  for (size_t i = 0; i < n; ++i) {
+    maps[2 * i] = nrl::make_tma_2d(a[i].data_ptr(), a[i].size(0), a[i].size(1), a[i].stride(0) * 2, a_mn ? 64 : 128, 64, BF, 2);
+    maps[2 * i + 1] = nrl::make_tma_2d(b[i].data_ptr(), contraction[i], narrow[i], b[i].stride(0) * 2, 64, 64, BF, 2);
+    q[i] = {static_cast<int>(wide[i]), static_cast<int>(narrow[i]), static_cast<int>(contraction[i]), static_cast<float>(alpha[i]), out[i].data_ptr(), out[i].stride(0),
+            transposed[i] ? 1 : 0};
   }
   const int64_t splits = splits_req > 0 ? splits_req : multi_splits(tiles, blocks, num_sms(), [&](int s) { return cluster_fits().multi[a_mn ? 1 : 0][s]; });
   for (int64_t x : blocks) TORCH_CHECK(split_ranges(x, splits) == splits, "gemm_tc_multi: an empty range");
   check(nrl_gemm_tc_multi(maps, q, static_cast<int>(n), a_mn ? 1 : 0, static_cast<int>(splits), cur_stream()), "gemm_tc_multi");
+  return true;
 }
 
 // out[b] = a[b] . b[b]^T for b < B: a [B, M, K], b [B, N, K], out [B, M, N]; any batch / row strides (inner stride 1), e.g. the
@@ -1681,10 +1690,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tc_swiglu_pair_keep", &gemm_tc_swiglu_pair_keep, "(act, gate, up) of gemm_tc_swiglu_pair with adapters");
   m.def("gemm_tc_dswiglu", &gemm_tc_dswiglu, "(d gate, d up) of silu(gate) * up behind a projection's backward");
   m.def("gemm_tc_multi", &gemm_tc_multi, "several products with narrow results in one launch", py::arg("a"), py::arg("b"), py::arg("out"), py::arg("transposed"),
-        py::arg("alpha"), py::arg("a_mn"), py::arg("splits") = 0);
+        py::arg("alpha"), py::arg("a_mn"), py::arg("splits") = 0, py::arg("if_faster") = false);
   m.def("gemm_tc_multi_pays", [](const std::vector<int64_t>& wide, const std::vector<int64_t>& narrow, const std::vector<int64_t>& contraction, int64_t sms) {
-    return multi_pays(wide, narrow, contraction, sms > 0 ? sms : num_sms());
-  }, "narrow products share a launch", py::arg("wide"), py::arg("narrow"), py::arg("contraction"), py::arg("sms") = 0);
+    return multi_pays(wide, narrow, contraction, sms);
+  }, "narrow products share a launch", py::arg("wide"), py::arg("narrow"), py::arg("contraction"), py::arg("sms"));
   m.def("gemm_tc_multi_splits", [](const std::vector<int64_t>& tiles, const std::vector<int64_t>& blocks, int64_t sms, const std::vector<int>& fits) {
     return multi_splits(tiles, blocks, sms, [&](int s) { return fits.at(s); });
   });

@@ -141,8 +141,8 @@ def lora_linear(x, w, bias, a, b, scaling: float):
 def sum_gemms(a, b):
     """``sum_i a[i] b[i]`` for the gradient of an input that several projections share: one launch with one float accumulator where none of the
     products would be cut into ranges of its contraction, else product by product, added in bf16."""
-    pick = _native_mod.ext().gemm_tc_auto_splits
-    if len(a) <= 4 and all(pick(x.shape[0], y.shape[1], x.shape[1], x.get_device()) == 1 for x, y in zip(a, b)):
+    pick, rows, cols, dev = _native_mod.ext().gemm_tc_auto_splits, a[0].shape[0], b[0].shape[1], a[0].get_device()
+    if len(a) <= 4 and all(pick(rows, cols, k, dev) == 1 for k in {x.shape[1] for x in a}):
         _native_mod._count()
         return _native_mod.ext().gemm_tc_sum(a, b)
     out = gemm(a[0], b[0], b_mn=True, a2=a[-1], b2=b[-1])
@@ -151,28 +151,32 @@ def sum_gemms(a, b):
     return out
 
 
-def _share(wide, narrow, contraction, r: int) -> bool:
-    """Whether an adapter's products [wide, contraction] x [contraction, narrow] share a launch, in tiles 64 wide: where an estimate says so
-    (csrc/bindings.cpp: multi_pays) and up to rank 64.  Wider factors fill wider tiles by themselves: rank 32 at 6601 tokens of a 1536 / 8960 wide MLP 88 -> 66 us
-    in one launch, rank 64 87 -> 69, rank 128 95 -> 107, rank 256 121 -> 187."""
-    return r <= 64 and _native_mod.ext().gemm_tc_multi_pays(wide, narrow, contraction)
+def _narrow(r: int) -> bool:
+    """Whether an adapter's products may share launches, in tiles 64 wide.  Wider factors fill wider tiles by themselves: rank 32 at 6601 tokens of a
+    1536 / 8960 wide MLP 88 -> 66 us in one launch, rank 64 87 -> 69, rank 128 95 -> 107, rank 256 121 -> 187."""
+    return r <= 64
+
+
+def _multi(a, b, out, flip, alpha: float, a_mn: bool):
+    """``out_i = alpha a_i b_i`` (``a_mn``: ``alpha a_i^T b_i``, the transpose of it where ``flip`` says so), up to six in a launch where that is faster than a GEMM each."""
+    ext = _native_mod.ext()
+    for i in range(0, len(a), 6):
+        j = slice(i, i + 6)
+        if ext.gemm_tc_multi(a[j], b[j], out[j], flip[j], [alpha] * len(a[j]), a_mn, 0, True):
+            _native_mod._count()
+            continue
+        for x, y, o, t in zip(a[j], b[j], out[j], flip[j]):
+            gemm(y, x, a_mn=True, b_mn=True, alpha=alpha, out=o) if t else gemm(x, y, a_mn=a_mn, b_mn=True, alpha=alpha, out=o)
 
 
 def _adapter_grads(factors, inputs, r):
     """``dy_i^T t_i`` [N_i, r_i] for every (dy_i, t_i) of ``factors`` and ``t'_j^T x_j`` [r_j, K_j] for every (t'_j, x_j) of ``inputs``, of adapters
     whose largest rank is ``r``."""
-    own = lambda dy, t, flip: gemm(t, dy, a_mn=True, b_mn=True) if flip else gemm(dy, t, a_mn=True, b_mn=True)      # noqa: E731
-    wide = [(dy, t, False) for dy, t in factors] + [(x, t, True) for t, x in inputs]
-    out, ext = [], _native_mod.ext()
-    for i in range(0, len(wide), 6):
-        part = wide[i:i + 6]
-        if _share([y.shape[1] for y, _, _ in part], [t.shape[1] for _, t, _ in part], [y.shape[0] for y, _, _ in part], r):
-            to = [y.new_empty(*((t.shape[1], y.shape[1]) if flip else (y.shape[1], t.shape[1]))) for y, t, flip in part]
-            _native_mod._count()
-            ext.gemm_tc_multi([y for y, _, _ in part], [t for _, t, _ in part], to, [flip for _, _, flip in part], [1.0] * len(part), True)
-            out += to
-        else:
-            out += [own(*p) for p in part]
+    if not _narrow(r):
+        return [gemm(dy, t, a_mn=True, b_mn=True) for dy, t in factors], [gemm(t, x, a_mn=True, b_mn=True) for t, x in inputs]
+    a, b = [dy for dy, _ in factors] + [x for _, x in inputs], [t for _, t in factors] + [t for t, _ in inputs]
+    out = [dy.new_empty(dy.shape[1], t.shape[1]) for dy, t in factors] + [x.new_empty(t.shape[1], x.shape[1]) for t, x in inputs]
+    _multi(a, b, out, [False] * len(factors) + [True] * len(inputs), 1.0, True)
     return out[:len(factors)], out[len(factors):]
 
 
@@ -181,14 +185,11 @@ def _group_backward(gs, x2, t_cat, a_cat, ws, Bs, s, need_x, more_factors=(), mo
     n, r = len(gs), t_cat.shape[1] // len(gs)
     tp_cat = torch.empty(x2.shape[0], n * r, dtype=x2.dtype, device=x2.device)
     tps = [tp_cat[:, i * r:(i + 1) * r] for i in range(n)]                                      # t'_i = s dy_i B_i
-    for i in range(0, n, 6):
-        part = list(zip(gs, Bs, tps))[i:i + 6]
-        if _share([g.shape[0] for g, _, _ in part], [r] * len(part), [g.shape[1] for g, _, _ in part], r):
-            _native_mod._count()
-            _native_mod.ext().gemm_tc_multi(*(list(x) for x in zip(*part)), [False] * len(part), [s] * len(part), False)
-        else:
-            for g, b, tp in part:
-                gemm(g, b, b_mn=True, alpha=s, out=tp)
+    if _narrow(r):
+        _multi(list(gs), list(Bs), tps, [False] * n, s, False)
+    else:
+        for g, b, tp in zip(gs, Bs, tps):
+            gemm(g, b, b_mn=True, alpha=s, out=tp)
     gx = sum_gemms([*gs, tp_cat], [*ws, a_cat]) if need_x else None                           # sum_i dy_i W_i + [t'_1 .. t'_n] [A_1; ..; A_n]
     gbs, gas = _adapter_grads([(gs[i], t_cat[:, i * r:(i + 1) * r]) for i in range(n)] + list(more_factors), [(tp_cat, x2)] + list(more_inputs),
                               max([r] + [t.shape[1] for _, t in more_factors]))
